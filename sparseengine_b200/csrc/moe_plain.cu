@@ -291,6 +291,204 @@ __global__ void grouped_gemm_plain_kernel(const T* __restrict__ a, const T* __re
     }
 }
 
+// ---- the same in 32-bit, for widths that are a multiple of 4 ------------------------------------
+// 32-bit operands stay on the CUDA cores (a tensor-core split would lose digits), so a step with many rows is
+// bound by the FMA rate and one with few by streaming the experts' weights.  The kernel above keeps 2 x 4 outputs per
+// thread: one shared-memory read per 1.3 FMAs, which set its pace.
+//
+// Many rows: 128 rows x 128 weight rows per block, 8 x 8 outputs per thread (four 16-byte reads per 64 FMAs), operands
+// transposed in two shared-memory stages, the next stage's loads in registers while this one is multiplied; two blocks per
+// SM.  A warp owns 32 rows of the tile and skips the arithmetic of rows an expert does not have.  In mode 0 a warp's 64
+// columns are 32 gate rows and the up rows of the same features, so a thread ends with both.  Neighbouring blocks share
+// an expert's rows (from L2) and read its weights once.  Measured at MiniMax M2's sizes, 3,372 tokens over 256 experts
+// (a hundred rows each): 13.4 ms for gate/up and 6.7 ms for down (38 TFLOP/s, 46 counting the rows of full tiles, of 62 that
+// FMAs of three registers reach); a pass of such a prompt step and eight decode steps over two layers spends 42 ms in
+// these products and the ones below, 119 ms with the kernel above.
+constexpr int kFM = 128, kFN = 128, kFK = 16, kFPitch = kFM + 4;
+
+template <int MODE>
+__global__ void __launch_bounds__(256, 2)
+grouped_gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w, const int* __restrict__ sorted,
+                        const int* __restrict__ offsets, const int* __restrict__ tile_expert,
+                        const int* __restrict__ tile_row0, const int* __restrict__ num_tiles,
+                        const float* __restrict__ route_w, float* __restrict__ out, int n_out, int k_dim, int top_k,
+                        int n_blocks, int act_kind, float act_limit, float act_alpha) {
+    const int tile = blockIdx.x / n_blocks;
+    if (tile >= num_tiles[0]) return;
+    constexpr int kFeatures = MODE == 0 ? kFN / 2 : kFN;         // output columns per block
+    const int e = tile_expert[tile], row0 = tile_row0[tile];
+    const int n0 = (blockIdx.x - tile * n_blocks) * kFeatures;
+    const int rows = min(kFM, offsets[e + 1] - row0);
+    __shared__ __align__(16) float as[2][kFK][kFPitch];
+    __shared__ __align__(16) float ws[2][kFK][kFPitch];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 64;
+    const int lm = (lane >> 3) * 4, ln = (lane & 7) * 4;
+    const float* we = w + (size_t)e * (MODE == 0 ? 2 : 1) * n_out * k_dim;
+    // this thread's loads: rows r and r + 64 of either operand, 4 floats from k = 4 * (tid % 4) on
+    const int r = tid >> 2, kq = (tid & 3) * 4;
+    const float* pa[2];
+    const float* pw[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int row = r + 64 * i;
+        pa[i] = row < rows ? a + (size_t)(MODE == 0 ? sorted[row0 + row] / top_k : row0 + row) * k_dim + kq : nullptr;
+        int n = n0 + row, half = 0;
+        if (MODE == 0) {                       // 32 gate rows, then the up rows of the same features, per warp column
+            n = n0 + (row >> 6) * 32 + (row & 31);
+            half = (row >> 5) & 1;
+        }
+        pw[i] = n < n_out ? we + ((size_t)half * n_out + n) * k_dim + kq : nullptr;
+    }
+    float4 ra[2], rw[2];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const bool in = k0 + kq < k_dim;
+            ra[i] = in && pa[i] != nullptr ? *reinterpret_cast<const float4*>(pa[i] + k0) : make_float4(0.f, 0.f, 0.f, 0.f);
+            rw[i] = in && pw[i] != nullptr ? *reinterpret_cast<const float4*>(pw[i] + k0) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    auto put = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int row = r + 64 * i;
+            as[buf][kq][row] = ra[i].x; as[buf][kq + 1][row] = ra[i].y; as[buf][kq + 2][row] = ra[i].z; as[buf][kq + 3][row] = ra[i].w;
+            ws[buf][kq][row] = rw[i].x; ws[buf][kq + 1][row] = rw[i].y; ws[buf][kq + 2][row] = rw[i].z; ws[buf][kq + 3][row] = rw[i].w;
+        }
+    };
+    float acc[8][8] = {};
+    fetch(0);
+    put(0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = 0; k0 < k_dim; k0 += kFK, buf ^= 1) {
+        const bool more = k0 + kFK < k_dim;
+        if (more) fetch(k0 + kFK);
+        if (wm < rows) {
+#pragma unroll
+            for (int k = 0; k < kFK; ++k) {
+                float av[8], wv[8];
+                *reinterpret_cast<float4*>(av) = *reinterpret_cast<const float4*>(&as[buf][k][wm + lm]);
+                *reinterpret_cast<float4*>(av + 4) = *reinterpret_cast<const float4*>(&as[buf][k][wm + 16 + lm]);
+                *reinterpret_cast<float4*>(wv) = *reinterpret_cast<const float4*>(&ws[buf][k][wn + ln]);
+                *reinterpret_cast<float4*>(wv + 4) = *reinterpret_cast<const float4*>(&ws[buf][k][wn + 32 + ln]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+            }
+        }
+        if (more) {
+            put(buf ^ 1);                      // the other stage: the barrier below separates its readers
+            __syncthreads();
+        }
+    }
+    const bool vec = (n_out & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int row = wm + lm + (i & 3) + (i >> 2) * 16;
+        if (row >= rows) continue;
+        float* o = out + (size_t)(row0 + row) * n_out;
+        const float scale = MODE == 1 ? route_w[sorted[row0 + row]] : 1.f;
+#pragma unroll
+        for (int h = 0; h < (MODE == 0 ? 1 : 2); ++h) {
+            const int n = MODE == 0 ? n0 + (wn >> 1) + ln : n0 + wn + h * 32 + ln;
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                v[j] = MODE == 0 ? glu_value<float>(acc[i][j], acc[i][4 + j], act_kind, act_limit, act_alpha) : acc[i][4 * h + j] * scale;
+            if (vec && n + 3 < n_out) {
+                *reinterpret_cast<float4*>(o + n) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (n + j < n_out) o[n + j] = v[j];
+            }
+        }
+    }
+}
+
+// Few rows per expert (decode steps): up to 8 rows of an expert lie in shared memory, a warp streams four weight rows at a
+// time past them, 16 bytes per lane and load, sums over the lanes at the end.  A block takes 32 features (64 weight rows
+// in mode 0), so that its rows are staged once for many weights.  Measured with 4 tokens (32 experts of one row): 158 and
+// 82 us for the two products, 7.6 and 7.4 TB/s of weights.
+constexpr int kStreamRows = 8, kStreamFeatures = 32;
+
+template <int MODE, int R>
+__device__ __forceinline__ void stream_weights(const float* xs, const float* we, const int* sorted, int row0, int rows,
+                                               const float* route_w, float* out, int n_out, int k_dim, int n0, int act_kind,
+                                               float act_limit, float act_alpha) {
+    constexpr int kPer = MODE == 0 ? 2 : 4;                      // features per pass of a warp (four weight rows)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int f = n0 + warp * kPer; f < min(n_out, n0 + kStreamFeatures); f += 8 * kPer) {
+        const float* pw[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int n = min(f + (MODE == 0 ? (i & 1) : i), n_out - 1);          // beyond the last feature: read, not stored
+            pw[i] = we + ((size_t)(MODE == 0 ? (i >> 1) : 0) * n_out + n) * k_dim;
+        }
+        float acc[4][R] = {};
+#pragma unroll 4
+        for (int k = lane * 4; k < k_dim; k += 128) {
+            float4 wv[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) wv[i] = __ldcs(reinterpret_cast<const float4*>(pw[i] + k));
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+                const float4 xv = *reinterpret_cast<const float4*>(xs + (size_t)j * k_dim + k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    acc[i][j] = fmaf(wv[i].w, xv.w, fmaf(wv[i].z, xv.z, fmaf(wv[i].y, xv.y, fmaf(wv[i].x, xv.x, acc[i][j]))));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < R; ++j) acc[i][j] = warp_sum(acc[i][j]);
+        if (lane != 0) continue;
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            if (j >= rows) continue;
+            const float scale = MODE == 1 ? route_w[sorted[row0 + j]] : 1.f;
+#pragma unroll
+            for (int i = 0; i < kPer; ++i)
+                if (f + i < n_out)
+                    out[(size_t)(row0 + j) * n_out + f + i] =
+                        MODE == 0 ? glu_value<float>(acc[i][j], acc[(i + 2) & 3][j], act_kind, act_limit, act_alpha) : acc[i][j] * scale;
+        }
+    }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(256)
+grouped_stream_f32_kernel(const float* __restrict__ a, const float* __restrict__ w, const int* __restrict__ sorted,
+                          const int* __restrict__ offsets, const int* __restrict__ tile_expert,
+                          const int* __restrict__ tile_row0, const int* __restrict__ num_tiles,
+                          const float* __restrict__ route_w, float* __restrict__ out, int n_out, int k_dim, int top_k,
+                          int n_blocks, int act_kind, float act_limit, float act_alpha) {
+    extern __shared__ __align__(16) float xs[];                  // [rows, rounded up to 1, 2, 4 or 8][k_dim]
+    const int tile = blockIdx.x / n_blocks;
+    if (tile >= num_tiles[0]) return;
+    const int e = tile_expert[tile], row0 = tile_row0[tile];
+    const int n0 = (blockIdx.x - tile * n_blocks) * kStreamFeatures;
+    const int rows = min(kStreamRows, offsets[e + 1] - row0);
+    const int padded = rows > 4 ? 8 : rows > 2 ? 4 : rows;
+    for (int j = 0; j < padded; ++j) {
+        const float* src = a + (size_t)(MODE == 0 ? sorted[row0 + min(j, rows - 1)] / top_k : row0 + min(j, rows - 1)) * k_dim;
+        for (int k = threadIdx.x * 4; k < k_dim; k += 1024)
+            *reinterpret_cast<float4*>(xs + (size_t)j * k_dim + k) = *reinterpret_cast<const float4*>(src + k);
+    }
+    __syncthreads();
+    const float* we = w + (size_t)e * (MODE == 0 ? 2 : 1) * n_out * k_dim;
+#define SE_STREAM(R) stream_weights<MODE, R>(xs, we, sorted, row0, rows, route_w, out, n_out, k_dim, n0, act_kind, act_limit, act_alpha)
+    if (padded == 1) SE_STREAM(1);
+    else if (padded == 2) SE_STREAM(2);
+    else if (padded == 4) SE_STREAM(4);
+    else SE_STREAM(8);
+#undef SE_STREAM
+}
+
 // out[t, :] = cast(sum over slots (32-bit, slot order) of y[inv_pos[t * top_k + slot], :] (+ add[t, :], last)).
 // A slot without a row (inv_pos < 0) stands for an expert whose output is its input: with `x` and `weights`
 // it adds weights[t * top_k + slot] * x[t, :], without them nothing.
@@ -399,16 +597,49 @@ extern "C" int se_moe_route_build(const int* ids, int assignments, int experts, 
 
 extern "C" int se_moe_plain_tile_rows() { return se::kBM; }
 
+// Rows per tile that the 32-bit grouped products take for a step of `assignments` rows over `experts` experts, whose
+// products have inner dimensions k0 and k1: 8 (weights streamed past a few rows) while an expert has about four rows or
+// fewer and eight rows of the wider operand fit in shared memory, 128 beyond; 0: widths that only the general kernel takes.
+extern "C" int se_moe_f32_tile_rows(int assignments, int experts, int k0, int k1) {
+    if (k0 <= 0 || k1 <= 0 || (k0 & 3) || (k1 & 3)) return 0;
+    const int k = k0 > k1 ? k0 : k1;
+    if ((long long)assignments <= 4ll * experts && (long long)k * se::kStreamRows * 4 <= 200 * 1024) return se::kStreamRows;
+    return se::kFM;
+}
+
 // mode 0: gate/up + SwiGLU (a = x [tokens, k_dim], w = w13 [E, 2*n_out, k_dim]);
 // mode 1: down * routing weight (a = act [assignments, k_dim], w = w2 [E, n_out, k_dim]).
 // act_kind, act_limit, act_alpha: the gated activation of mode 0 (glu.cuh).
+// tile_rows: the rows per tile that the tile list was built with: se_moe_plain_tile_rows (any type and width), or what
+// se_moe_f32_tile_rows returned (float32).
 extern "C" int se_moe_grouped_gemm_plain(int mode, const void* a, const void* w, const int* sorted, const int* offsets,
                                          const int* tile_expert, const int* tile_row0, const int* num_tiles,
                                          const float* route_w, void* out, int max_tiles, int n_out, int k_dim,
-                                         int top_k, int act_kind, float act_limit, float act_alpha, int dtype,
+                                         int top_k, int act_kind, float act_limit, float act_alpha, int tile_rows, int dtype,
                                          cudaStream_t stream) {
     if (max_tiles <= 0) return 0;
     if (act_kind < SE_GLU_SILU || act_kind > SE_GLU_GELU) return SE_ERR_ARGUMENT;
+    if (tile_rows != se::kBM) {
+        const bool few = tile_rows == se::kStreamRows;
+        if (dtype != SE_DTYPE_F32 || (!few && tile_rows != se::kFM)) return SE_ERR_ARGUMENT;
+        if ((k_dim & 3) || ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15)) return SE_ERR_UNSUPPORTED;
+        const int per = few ? se::kStreamFeatures : mode == 0 ? se::kFN / 2 : se::kFN;
+        const int n_blocks = se::ceil_div(n_out, per);
+        if ((long long)max_tiles * n_blocks > 0x7fffffffLL) return SE_ERR_UNSUPPORTED;
+        const size_t smem = few ? (size_t)se::kStreamRows * k_dim * sizeof(float) : 0;
+        auto launch = [&](auto* kernel) {
+            if (smem > 40 * 1024) {
+                const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                if (err != cudaSuccess) return (int)err;
+            }
+            kernel<<<max_tiles * n_blocks, 256, smem, stream>>>((const float*)a, (const float*)w, sorted, offsets, tile_expert,
+                                                                tile_row0, num_tiles, route_w, (float*)out, n_out, k_dim, top_k,
+                                                                n_blocks, act_kind, act_limit, act_alpha);
+            return (int)cudaGetLastError();
+        };
+        if (few) return mode == 0 ? launch(se::grouped_stream_f32_kernel<0>) : launch(se::grouped_stream_f32_kernel<1>);
+        return mode == 0 ? launch(se::grouped_gemm_f32_kernel<0>) : launch(se::grouped_gemm_f32_kernel<1>);
+    }
     dim3 grid(max_tiles, se::ceil_div(n_out, se::kBN));
     SE_DISPATCH_DTYPE(dtype, T, {
         if (mode == 0)

@@ -968,13 +968,25 @@ def _glu_args(activation):
     return GLU_KINDS[name], float(limit), float(alpha)
 
 
-def moe_grouped_gemm_plain(mode: int, a, w, ws: dict, route_w, out, *, max_tiles, n_out, k_dim, top_k, activation=None):
+def moe_f32_tile_rows(assignments: int, experts: int, k0: int, k1: int) -> int:
+    """Rows per tile for the 32-bit grouped products of a step (csrc/moe_plain.cu), or 0 where the widths need the
+    general kernel's (:func:`moe_plain_tile_rows`)."""
+    f = library().se_moe_f32_tile_rows
+    f.restype = _I
+    f.argtypes = [_I] * 4
+    return int(f(assignments, experts, k0, k1))
+
+
+def moe_grouped_gemm_plain(mode: int, a, w, ws: dict, route_w, out, *, max_tiles, n_out, k_dim, top_k, activation=None,
+                           tile_rows: Optional[int] = None):
+    """``tile_rows``: what the tile list was built with (default: :func:`moe_plain_tile_rows`)."""
     dt = a.dtype
-    _check(_fn("se_moe_grouped_gemm_plain", "i" "ppppppppp" "iiii" "iff" "ip")(
+    _check(_fn("se_moe_grouped_gemm_plain", "i" "ppppppppp" "iiii" "iff" "iip")(
         mode, _ptr(a, None, "a"), _ptr(w, dt, "w"), _ptr(ws["sorted"]), _ptr(ws["offsets"]),
         _ptr(ws["tile_expert"]), _ptr(ws["tile_row0"]), _ptr(ws["num_tiles"]),
         _ptr(route_w, torch.float32, "route_w"), _ptr(out, dt, "out"), max_tiles, n_out, k_dim, top_k,
-        *_glu_args(activation), dtype_code(dt), _stream()), "moe_grouped_gemm_plain")
+        *_glu_args(activation), moe_plain_tile_rows() if tile_rows is None else int(tile_rows), dtype_code(dt), _stream()),
+        "moe_grouped_gemm_plain")
     return out
 
 
@@ -1235,6 +1247,28 @@ def attn_prefill(q, cache, table, seq_rows, cu_q, kv_len, out, *, entries, max_q
         num_kv_heads, head_dim, dv, page_size, float(scale), _visible_arg(window, chunk),
         cache.shape[0] if num_pages is None else int(num_pages), _ptr(error_word(q.device)),
         *_softmax_options(q, gate, num_heads, dv, softcap, sink, keep_first or 0, slopes), _stream()), "attn_prefill")
+    return out
+
+
+def attn_prefill_f32_supported(head_dim: int, v_head_dim: int, num_heads: int, num_kv_heads: int) -> bool:
+    """What ``se_attn_prefill_f32_supported`` answers (restated, as :func:`attn_decode_supported`)."""
+    return (0 < head_dim <= 128 and head_dim % 4 == 0 and 0 < v_head_dim <= 128 and v_head_dim % 4 == 0
+            and 0 < num_kv_heads <= LIMITS["grid_dim_yz"] and num_heads % num_kv_heads == 0)
+
+
+def attn_prefill_f32(q, cache, table, seq_rows, cu_q, kv_len, out, *, entries, max_q_len, num_heads, num_kv_heads,
+                     head_dim, page_size, scale, window=None, num_pages=None, v_head_dim=None, softcap=None,
+                     sink=False, gate=None, keep_first: int = 0, slopes=None, chunk=None):
+    """Prompt-portion attention in 32-bit (csrc/attention_f32.cu); arguments as :func:`attn_prefill`'s."""
+    dv = int(v_head_dim or head_dim)
+    f32 = torch.float32
+    _check(_fn("se_attn_prefill_f32", "pppipppp" "iiiiiii" "f" "i" "ip" "fipi" "pipi" "p")(
+        _ptr(q, f32, "q"), _ptr(cache, f32, "cache"), _ptr(table, torch.int32, "table"),
+        table.shape[1], _ptr(seq_rows, torch.int32, "seq_rows"), _ptr(cu_q, torch.int32, "cu_q"),
+        _ptr(kv_len, torch.int32, "kv_len"), _ptr(out, f32, "out"), entries, max_q_len, num_heads,
+        num_kv_heads, head_dim, dv, page_size, float(scale), _visible_arg(window, chunk),
+        cache.shape[0] if num_pages is None else int(num_pages), _ptr(error_word(q.device)),
+        *_softmax_options(q, gate, num_heads, dv, softcap, sink, keep_first or 0, slopes), _stream()), "attn_prefill_f32")
     return out
 
 

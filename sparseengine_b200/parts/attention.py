@@ -251,6 +251,13 @@ class PagedAttention(Mixer):
                    max_q_len=step.max_q_len, num_heads=s.num_heads, num_kv_heads=s.num_kv_heads,
                    head_dim=s.head_dim, page_size=slot.page_size, scale=s.scale, window=s.window, **options)
             return
+        # 32-bit prompt portions: the same hand-over as in 16-bit (a step of single tokens leaves the tiles' rows empty)
+        if (self.use_tensor_cores is not False and q.dtype == torch.float32 and self.takes_portion_kernel(step)
+                and ops.attn_prefill_f32_supported(s.head_dim, s.value_dim, s.num_heads, s.num_kv_heads)):
+            ops.attn_prefill_f32(q, slot.kv, slot.table, step.seq_rows, step.cu_q, step.kv_len, out, entries=step.num_seqs,
+                                 max_q_len=step.max_q_len, num_heads=s.num_heads, num_kv_heads=s.num_kv_heads,
+                                 head_dim=s.head_dim, page_size=slot.page_size, scale=s.scale, window=s.window, **options)
+            return
         ops.paged_attention_plain(q, slot.kv, slot.table, step.seq_rows, step.token_seq, step.positions, out,
                                   num_heads=s.num_heads, num_kv_heads=s.num_kv_heads, head_dim=s.head_dim,
                                   page_size=slot.page_size, scale=s.scale, window=s.window, **options)

@@ -83,6 +83,14 @@ class _RoutedSwiGLU(FeedForward):
             return False
         return ops.gemm_tc_supported(self.hidden, self.inter) and ops.gemm_tc_supported(self.inter, self.hidden)
 
+    def plain_tile_rows(self, x, assignments: int) -> int:
+        """Rows per tile of the CUDA-core products: by the step's size in float32 (widths that are multiples of 4,
+        16-byte-aligned operands), the general kernel's otherwise."""
+        rows = 0
+        if x.dtype == torch.float32 and not any(t.data_ptr() & 15 for t in (x, self.w13, self.w2)):
+            rows = ops.moe_f32_tile_rows(assignments, self.num_experts, self.hidden, self.inter)
+        return rows or ops.moe_plain_tile_rows()
+
     # Two 64-bit counters on the device, created with the first step: [0] the experts that got at
     # least one row, summed over routing builds, [1] the routing builds.  The routing build
     # counts them where its per-expert counts already are (no launch of its own, also inside
@@ -101,7 +109,10 @@ class _RoutedSwiGLU(FeedForward):
         dev = x.device
         tc = self.tensor_cores_usable(x)
         pair = tc and self.takes_pair_kernel(a)
-        tile_rows = (ops.PAIR_TILE_ROWS if pair else ops.moe_tile_rows_tc(a, self.num_experts)) if tc else ops.moe_plain_tile_rows()
+        if tc:
+            tile_rows = ops.PAIR_TILE_ROWS if pair else ops.moe_tile_rows_tc(a, self.num_experts)
+        else:
+            tile_rows = self.plain_tile_rows(x, a)
         max_tiles = ops.moe_max_tiles(a, self.num_experts, tile_rows)
         i32 = dict(dtype=torch.int32, device=dev)
         ws = {"counts": torch.empty(self.num_experts, **i32), "rank": torch.empty(a, **i32),
@@ -138,9 +149,10 @@ class _RoutedSwiGLU(FeedForward):
                                     n_out=self.hidden, k_dim=self.inter, nt=tile_rows, lists_settled=True)
         else:
             ops.moe_grouped_gemm_plain(0, x, self.w13, ws, None, act, max_tiles=max_tiles, n_out=self.inter,
-                                       k_dim=self.hidden, top_k=self.top_k, activation=self.activation_args)
+                                       k_dim=self.hidden, top_k=self.top_k, activation=self.activation_args,
+                                       tile_rows=tile_rows)
             ops.moe_grouped_gemm_plain(1, act, self.w2, ws, weights, y, max_tiles=max_tiles, n_out=self.hidden,
-                                       k_dim=self.inter, top_k=self.top_k)
+                                       k_dim=self.inter, top_k=self.top_k, tile_rows=tile_rows)
         out = torch.empty(tokens, self.hidden, dtype=x.dtype, device=dev)
         ops.moe_combine(y, ws["inv_pos"], out, self.top_k, add=add,
                         identity=(x, weights) if self.identity_experts else None)

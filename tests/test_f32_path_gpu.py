@@ -1,0 +1,111 @@
+"""The 32-bit path's kernels for prompt portions and routed experts against the general ones (one block per token and head;
+tiles of 32 rows) and against 64-bit sums, at the edges of their tiles."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _batch(q_lens, kv_lens, page, seed):
+    g = torch.Generator().manual_seed(seed)
+    most = -(-max(kv_lens) // page)
+    n = len(q_lens)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    cu = [0]
+    for t in q_lens:
+        cu.append(cu[-1] + t)
+    return dict(table=torch.randperm(n * most, generator=g).to(torch.int32).view(n, most).to(DEV), rows=torch.randperm(n, generator=g).to(torch.int32).to(DEV),
+                cu=torch.tensor(cu, **i32), kv=torch.tensor(kv_lens, **i32), pages=n * most, tokens=cu[-1],
+                seq=torch.tensor([j for j, t in enumerate(q_lens) for _ in range(t)], **i32),
+                pos=torch.tensor([k - t + i for t, k in zip(q_lens, kv_lens) for i in range(t)], **i32))
+
+
+OPTIONS = {"plain": {}, "window": dict(window=37), "wide window": dict(window=129, keep_first=70), "chunk": dict(chunk=50),
+           "cap, sink": dict(softcap=3.0, sink=True), "kept, learned sink": dict(window=20, keep_first=5, sink="learned"),
+           "slopes": dict(slopes=True, gate="head"), "gate": dict(gate="element", window=64)}
+
+
+@pytest.mark.parametrize("options", list(OPTIONS))
+@pytest.mark.parametrize("d,dv,heads,kv_heads,page", [(128, 128, 6, 1, 16), (64, 64, 4, 2, 8), (20, 12, 5, 5, 4), (100, 68, 3, 1, 16), (32, 128, 64, 1, 5)])
+def test_portion_attention(d, dv, heads, kv_heads, page, options):
+    """Tiles of 128 rows and 64 keys: entries that end on, before and behind tile edges, single tokens among them, every
+    option; and values that are not finite where a row does not see them."""
+    from sparseengine_b200.csrc import ops
+    b = _batch([64, 1, 130, 2, 63], [64, 129, 209, 17, 191], page, d + heads)
+    g = torch.Generator(device=DEV).manual_seed(d)
+    cache = torch.randn(b["pages"], page * kv_heads * (d + dv), generator=g, device=DEV) * 0.7
+    q = torch.randn(b["tokens"], heads * d, generator=g, device=DEV)
+    opt = dict(OPTIONS[options])
+    if opt.get("gate"):
+        cols = heads * (dv if opt["gate"] == "element" else 1)
+        opt["gate"] = torch.randn(b["tokens"], cols + 5, generator=g, device=DEV)[:, 2:2 + cols]
+    if opt.get("sink") == "learned":
+        opt["sink"] = torch.randn(heads, generator=g, device=DEV)
+    if opt.get("slopes"):
+        opt["slopes"] = torch.rand(heads, generator=g, device=DEV)
+    common = dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=d, v_head_dim=dv, page_size=page, scale=d ** -0.5, **opt)
+
+    def both():
+        want, got = (torch.full((b["tokens"], heads * dv), float("nan"), device=DEV) for _ in range(2))
+        ops.paged_attention_plain(q, cache, b["table"], b["rows"], b["seq"], b["pos"], want, **common)
+        ops.attn_prefill_f32(q, cache, b["table"], b["rows"], b["cu"], b["kv"], got, entries=5, max_q_len=130, **common)
+        ops.error_check(DEV)
+        return want, got
+
+    want, got = both()
+    # two orders of the same 32-bit sums over at most 209 keys of products of size one
+    assert bool(torch.isfinite(got).all()) and float((got - want).abs().max()) < 4e-6 * max(1.0, float(want.abs().max()))
+    # the last token of the first entry has a value of infinity: only rows that see it change
+    if page * kv_heads * (d + dv) and options in ("plain", "window", "chunk"):
+        where = int(b["table"][int(b["rows"][0]), 63 // page])
+        cache[where, page * kv_heads * d + (63 % page) * dv:page * kv_heads * d + (63 % page) * dv + dv] = float("inf")
+        want2, got2 = both()
+        assert torch.equal(torch.isfinite(got2), torch.isfinite(want2)) and bool(torch.isfinite(got2[:63]).all())
+        assert torch.equal(got2[:63], got[:63])
+
+
+def test_portion_attention_leaves_bad_pages_out():
+    from sparseengine_b200.csrc import ops
+    b = _batch([40], [200], 16, 1)
+    cache = torch.randn(b["pages"], 16 * 2 * 128, device=DEV)
+    q = torch.randn(40, 4 * 64, device=DEV)
+    b["table"][0, 3] = 10 ** 6
+    common = dict(num_heads=4, num_kv_heads=2, head_dim=64, page_size=16, scale=0.2)
+    want, got = torch.empty_like(q), torch.empty_like(q)
+    for fn in (lambda: ops.paged_attention_plain(q, cache, b["table"], b["rows"], b["seq"], b["pos"], want, **common),
+               lambda: ops.attn_prefill_f32(q, cache, b["table"], b["rows"], b["cu"], b["kv"], got, entries=1, max_q_len=40, **common)):
+        fn()
+        with pytest.raises(Exception):
+            ops.error_check(DEV)
+    assert float((got - want).abs().max()) < 4e-6
+
+
+@pytest.mark.parametrize("activation", [None, ("clamped_swiglu", 1.0, 1.7)])
+@pytest.mark.parametrize("counts,hidden,inter", [
+    ([1, 0, 2, 3, 4, 5, 8, 1, 9, 0, 0, 0, 0, 0, 0, 0], 64, 36),         # streamed: one to eight rows, nine in two tiles
+    ([1, 1, 0, 0], 132, 100), ([1], 4, 4),
+    ([127, 128, 129, 0, 1, 31, 33, 97], 64, 36), ([300, 5], 132, 100), ([64], 20, 260)])        # tiles of 128 rows
+def test_routed_products(counts, hidden, inter, activation):
+    """Both products of the experts, tiles of 8 and of 128 rows against the general kernel's, at their edges in rows, features
+    and inner dimension."""
+    from sparseengine_b200.config.specs import MoESpec
+    from sparseengine_b200.csrc import ops
+    from sparseengine_b200.parts.moe import SparseMoE
+    g = torch.Generator(device=DEV).manual_seed(sum(counts))
+    experts, tokens = len(counts), sum(counts)
+    spec = MoESpec(hidden_size=hidden, num_experts=experts, top_k=1, intermediate_size=inter,
+                   **({} if activation is None else dict(activation=activation[0], activation_limit=activation[1], activation_alpha=activation[2])))
+    part = SparseMoE(spec, torch.float32)
+    part.bind({"w13": torch.randn(experts, 2 * inter, hidden, generator=g, device=DEV) * hidden ** -0.5,
+               "w2": torch.randn(experts, hidden, inter, generator=g, device=DEV) * inter ** -0.5})
+    x = torch.randn(tokens, hidden, generator=g, device=DEV)
+    ids = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts))[torch.randperm(tokens, generator=torch.Generator().manual_seed(3))]
+    ids = ids.view(-1, 1).to(torch.int32).to(DEV)
+    weights = torch.rand(tokens, 1, generator=g, device=DEV)
+    assert part.plain_tile_rows(x, tokens) == (8 if tokens <= 4 * experts else 128)
+    got = part.run_experts(x, ids, weights)
+    part.plain_tile_rows = lambda x, a: ops.moe_plain_tile_rows()
+    want = part.run_experts(x, ids, weights)
+    # sums of at most 260 products of size one in another order
+    assert float((got - want).abs().max()) < 4e-6 * max(1.0, float(want.abs().max()))
