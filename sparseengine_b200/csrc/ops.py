@@ -26,7 +26,7 @@ _fns: dict = {}
 
 # Kernels launched through these bindings since the process started (a launcher that
 # starts two kernels counts two).  Benchmarks read the difference around a timed region.
-KERNELS_PER_CALL = {"se_attn_decode": 2, "se_router": 2, "se_causal_conv": 2, "se_ssm_scan": 2}   # upper bounds per call
+KERNELS_PER_CALL = {"se_attn_decode": 2, "se_router": 2, "se_causal_conv": 2, "se_ssm_scan": 2, "se_retention_chunk": 2, "se_ssm_walk": 2, "se_delta_walk": 2}   # upper bounds per call
 launch_count = 0
 calls: dict = {}     # launcher name -> times called (tests check which kernels a path took)
 
@@ -604,20 +604,26 @@ def retention_segment_plan(entries: int, heads: int, v_head_dim: int, max_q_len:
 def retention_chunk(q32, k32, proj, v_off: int, decay, state, step, o, *, heads, head_dim, v_head_dim, segments=None,
                     silu: bool = False):
     """The same recurrence as :func:`retention_scan` in chunks of 64 tokens (closed form per chunk, 32-bit
-    FMA arithmetic): for steps that bring prompt portions.  ``segments``: ``(per entry, tokens each)``, default
-    by :func:`retention_segment_plan`."""
+    FMA arithmetic): for steps that bring prompt portions.  By default the chunks are prepared side by side and walked
+    (csrc/chunk_walk.cuh) where the sizes allow it; else, or with ``segments`` (``(per entry, tokens each)``, default by
+    :func:`retention_segment_plan`), one kernel does a chunk at a time."""
     global launch_count
-    max_seg, seg_len = segments if segments is not None else retention_segment_plan(
-        step.num_seqs, heads, v_head_dim, step.max_q_len, sm_count(q32.device))
-    seg_state = None
-    if max_seg > 1:
-        seg_state = torch.empty(step.num_seqs * max_seg * heads * head_dim * v_head_dim, dtype=torch.float32, device=q32.device)
-        launch_count += 2
-    _check(_fn("se_retention_chunk", "pp" "pii" "p" "pl" "pp" "p" "iiii" "iipi" "ip")(
+    seg_state = work = None
+    max_seg, seg_len = 1, 0
+    if segments is None and chunk_walk_supported(head_dim, v_head_dim, proj.stride(0), int(v_off)) and proj.data_ptr() % 16 == 0:
+        work = _walk_work(q32.shape[0] * heads * 66, q32.device)
+    else:
+        max_seg, seg_len = segments if segments is not None else retention_segment_plan(
+            step.num_seqs, heads, v_head_dim, step.max_q_len, sm_count(q32.device))
+        if max_seg > 1:
+            seg_state = torch.empty(step.num_seqs * max_seg * heads * head_dim * v_head_dim, dtype=torch.float32, device=q32.device)
+            launch_count += 1
+    _check(_fn("se_retention_chunk", "pp" "pii" "p" "pl" "pp" "p" "iiii" "iipi" "pii" "ip")(
         _ptr(q32, torch.float32, "q32"), _ptr(k32, torch.float32, "k32"), proj.data_ptr(), proj.stride(0), int(v_off),
         _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), state.stride(0), _ptr(step.cu_q),
         _ptr(step.seq_rows), _ptr(o, torch.float32, "o"), step.num_seqs, heads, head_dim, v_head_dim, int(max_seg),
-        int(seg_len), _ptr(seg_state), int(silu), dtype_code(proj.dtype), _stream()), "retention_chunk")
+        int(seg_len), _ptr(seg_state), int(silu), _ptr(work), q32.shape[0], sm_count(q32.device), dtype_code(proj.dtype),
+        _stream()), "retention_chunk")
     return o
 
 
@@ -639,6 +645,46 @@ def retention_out_joint(o, proj, g_off: int, w, out, *, eps):
         _ptr(o, torch.float32, "o"), _rows_ptr(proj, "proj"), proj.stride(0), int(g_off), _ptr(w, proj.dtype, "w"),
         _ptr(out, proj.dtype, "out"), tokens, width, float(eps), dtype_code(proj.dtype), _stream()), "retention_out_joint")
     return out
+
+
+# ---- linear recurrences in chunks, prepared side by side and walked (csrc/chunk_walk.cu) ----------
+
+def chunk_walk_supported(d: int, dv: int, *strides: int) -> bool:
+    """Whether the chunked recurrences take a head's state of ``d`` rows and ``dv`` columns (what ``se_chunk_walk_supported``
+    answers, restated); ``strides``: pitches and offsets (in elements) of what is read four elements at a time."""
+    return 8 <= d <= 128 and d % 4 == 0 and dv >= 4 and dv % 4 == 0 and not any(n % 4 for n in strides)
+
+
+def _walk_work(n: int, device) -> torch.Tensor:
+    return torch.empty(n, dtype=torch.float32, device=device)
+
+
+def ssm_walk(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, step, y, *, heads, head_dim, state_size, groups):
+    """The recurrence of :func:`ssm_scan` over prompt portions, in chunks of 64 tokens."""
+    tokens = xbc.shape[0]
+    work = _walk_work(tokens * heads * 67, xbc.device)
+    _check(_fn("se_ssm_walk", "ppii" "ppp" "pl" "pp" "pp" "iiiiiiii" "p")(
+        _ptr(xbc, torch.float32, "xbc"), _rows_ptr(proj, "proj"), proj.stride(0), int(dt_off),
+        _ptr(dt_bias, torch.float32, "dt_bias"), _ptr(a_log, torch.float32, "a_log"), _ptr(d_skip, torch.float32, "d_skip"),
+        _ptr(state, torch.float32, "state"), state.stride(0), _ptr(step.cu_q), _ptr(step.seq_rows), _ptr(y, torch.float32, "y"),
+        work.data_ptr(), tokens, step.num_seqs, heads, head_dim, state_size, groups, sm_count(xbc.device), dtype_code(proj.dtype),
+        _stream()), "ssm_walk")
+    return y
+
+
+def delta_walk(qkv, dec, log_dec, beta, state, step, o, *, heads, kv_heads, head_dim, v_head_dim):
+    """The recurrence of :func:`delta_scan` over prompt portions: one decay per head (``log_dec``, ``dec`` None; chunks of 64
+    tokens) or per head and key channel (``dec``, ``log_dec`` None; chunks of 32)."""
+    tokens = qkv.shape[0]
+    per = 66 + head_dim + v_head_dim if dec is None else 32 + 3 * head_dim + v_head_dim
+    places = 0 if dec is None else (tokens // 32 + step.num_seqs) * heads * head_dim
+    work = _walk_work(tokens * heads * per + places, qkv.device)
+    _check(_fn("se_delta_walk", "pppp" "pl" "pp" "pp" "iiiiiii" "p")(
+        _ptr(qkv, torch.float32, "qkv"), _ptr(dec, torch.float32, "dec"), _ptr(log_dec, torch.float32, "log_dec"),
+        _ptr(beta, torch.float32, "beta"), _ptr(state, torch.float32, "state"), state.stride(0), _ptr(step.cu_q),
+        _ptr(step.seq_rows), _ptr(o, torch.float32, "o"), work.data_ptr(), tokens, step.num_seqs, heads, kv_heads, head_dim,
+        v_head_dim, sm_count(qkv.device), _stream()), "delta_walk")
+    return o
 
 
 # ---- mixers with a recurrent state (csrc/recurrent.cu) -------------------------------------------

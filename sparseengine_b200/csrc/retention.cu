@@ -13,7 +13,7 @@
 //
 // A step brings any mix of prompt portions and single tokens: entry s owns the tokens
 // cu_q[s] .. cu_q[s+1]-1 and the state row seq_rows[s].
-#include "common.cuh"
+#include "chunk_walk.cuh"
 
 namespace se {
 
@@ -392,6 +392,52 @@ retention_seg_fix_kernel(const float* __restrict__ q32, const float* __restrict_
     }
 }
 
+// ---- prompt portions, chunks prepared side by side (chunk_walk.cuh) --------------------------------
+namespace walk {
+
+// Retention: P[t][s] = decay^(t - s) q_t . k_s, rs = decay^(t + 1), ts = decay^(n - 1 - t).
+template <int DP>
+__global__ void __launch_bounds__(kThreads, 3)
+retention_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ decay,
+                         const int* __restrict__ cu_q, int entries, float* __restrict__ p, float* __restrict__ rs,
+                         float* __restrict__ ts, int H, int d) {
+    constexpr int T = 64, QP = DP + 4;
+    extern __shared__ __align__(16) float sm[];
+    float* qs = sm;
+    float* ks = qs + T * QP;
+    __shared__ float power[T + 1];
+    int first, n;
+    chunk_of<T>(blockIdx.x, cu_q, entries, first, n);
+    if (n <= 0) return;
+    const int h = blockIdx.y;
+    load_tile<T, DP>(qs, q + (size_t)h * d, H * d, first, n, d);
+    load_tile<T, DP>(ks, k + (size_t)h * d, H * d, first, n, d);
+    cp_commit();
+    const double g = (double)decay[h];
+    if (threadIdx.x <= T) power[threadIdx.x] = (float)pow(g, (double)threadIdx.x);
+    cp_wait<0>();
+    __syncthreads();
+    if (threadIdx.x < n) {
+        rs[(size_t)(first + threadIdx.x) * H + h] = power[threadIdx.x + 1];
+        ts[(size_t)(first + threadIdx.x) * H + h] = power[n - 1 - threadIdx.x];
+    }
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    float acc[4][4] = {};
+    row_products<DP, 4>(qs, ks, ty, tx, acc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = ty + 16 * i;
+        if (t >= n) continue;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int s = tx + 16 * b;
+            p[((size_t)(first + t) * H + h) * T + s] = s <= t ? acc[i][b] * power[t - s] : 0.f;
+        }
+    }
+}
+
+}  // namespace walk
+
 // out[t, h, :] = o[t, h, :] / sqrt(mean(o[t, h, :]^2) + eps) * silu(gate[t, h, :]); a warp per (token, head).
 template <typename T>
 __global__ void retention_out_kernel(const float* __restrict__ o, const T* proj, int proj_stride, int g_off,
@@ -528,13 +574,47 @@ extern "C" int se_retention_scan(const float* q32, const float* k32, const void*
     SE_LAUNCH_CHECK();
 }
 
+static int launch_retention_walk(const float* q32, const float* k32, const void* proj, int proj_stride, int v_off,
+                                 const float* decay, float* state, long long state_stride, const int* cu_q, const int* seq_rows,
+                                 float* o, float* work, int tokens, int entries, int heads, int d, int dv, int sms, int silu,
+                                 int dtype, cudaStream_t stream) {
+    using namespace se::walk;
+    if (entries <= 0 || tokens <= 0) return 0;
+    if (!takes(d, dv) || heads <= 0 || heads > 65535 || dv / 16 >= 65535) return SE_ERR_UNSUPPORTED;
+    if (proj_stride % 4 || v_off % 4 || !aligned(q32) || !aligned(k32) || !aligned(o) || !aligned(work) || (reinterpret_cast<uintptr_t>(proj) & 15))
+        return SE_ERR_UNSUPPORTED;
+    float* p = work;
+    float* rs = p + (size_t)tokens * heads * 64;
+    float* ts = rs + (size_t)tokens * heads;
+    const dim3 grid(tokens / 64 + entries, heads);
+    SE_WALK_DIMS(d, {
+        const int rc = launch(retention_prepare_kernel<DP>, grid, 2 * 64 * (DP + 4) * sizeof(float), stream, q32, k32, decay, cu_q,
+                              entries, p, rs, ts, heads, d);
+        if (rc != 0) return rc;
+        WalkArgs a = {};
+        a.q = q32; a.k = k32; a.qk_stride = heads * d; a.rep = 1; a.v_stride = proj_stride; a.silu = silu;
+        a.p = p; a.rs = rs; a.ts = ts; a.state = state; a.state_stride = state_stride; a.s_row = dv; a.s_col = 1; a.o = o;
+        a.cu_q = cu_q; a.seq_rows = seq_rows; a.H = heads; a.d = d; a.dv = dv;
+        const int cols = walk_columns(entries, heads, dv, sms);
+        SE_DISPATCH_DTYPE(dtype, T_, {
+            a.v = static_cast<const T_*>(proj) + v_off;
+            return launch_walk<64, DP, false, false, T_>(a, entries, cols, stream);
+        });
+    });
+}
+
 // The same recurrence in chunks of 64 tokens (closed form per chunk): for steps with prompt portions.
 extern "C" int se_retention_chunk_supported(int d) { return d > 0 && d <= 256; }
 
 extern "C" int se_retention_chunk(const float* q32, const float* k32, const void* proj, int proj_stride, int v_off,
                                   const float* decay, float* state, long long state_stride, const int* cu_q,
                                   const int* seq_rows, float* o, int entries, int heads, int d, int dv, int max_seg,
-                                  int seg_len, float* seg_state, int silu, int dtype, cudaStream_t stream) {
+                                  int seg_len, float* seg_state, int silu, float* work, int tokens, int sms, int dtype,
+                                  cudaStream_t stream) {
+    // work (float [tokens * heads * (64 + 2)]): chunks prepared side by side and walked; else the forms below.
+    if (work != nullptr)
+        return launch_retention_walk(q32, k32, proj, proj_stride, v_off, decay, state, state_stride, cu_q, seq_rows, o, work, tokens,
+                                     entries, heads, d, dv, sms, silu, dtype, stream);
     // max_seg > 1: the entries' tokens in segments of seg_len (a multiple of 64) that run side by side, joined by
     // the decay's powers (three launches); seg_state: float [entries, max_seg, heads, d, dv].
     if (entries <= 0) return 0;

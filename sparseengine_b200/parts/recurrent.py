@@ -25,12 +25,25 @@ def _check_state_rows(rows: int, what: str) -> None:
                          "column's rows live in the registers of one warp's lanes)")
 
 
+def takes_chunks(mixer, step, heads: int, columns: int, device) -> bool:
+    """Whether a step's recurrence runs in chunks: its longest entry has ``chunk_min_tokens`` tokens, and its entries average
+    ``chunk_min_average`` (a chunk costs a short entry as much as a full one) or do not fill the device.  Measured at a width
+    of 2,048, both mixers of the hybrid design: 64 prompts of 24 to 48 tokens take 0.9 ms more in chunks, four of 750 to 1,500
+    tokens 0.1 (decays per channel) and 0.8 ms (state space) less."""
+    if mixer.chunk_min_tokens is None or step.max_q_len < mixer.chunk_min_tokens:
+        return False
+    return (step.num_tokens >= mixer.chunk_min_average * step.num_seqs
+            or step.num_seqs * heads * -(-columns // 32) <= ops.sm_count(device))
+
+
 class StateSpaceMixer(Mixer):
     """``[z | x | B | C | dt] = in_proj(h)``; x, B, C through a causal convolution (bias) and silu;
     ``dt = softplus(dt + dt_bias)``; per head ``S <- exp(-exp(A_log) dt) S + dt B x^T``,
     ``y = S^T C + D x``; ``y * silu(z)`` RMS-normed in ``norm_groups`` parts, times a weight; out
     projection."""
     graph_safe = True
+    chunk_min_tokens = 16        # the longest entry of a step from which the recurrence runs in chunks; None: never
+    chunk_min_average = 64       # ... if the step's entries average this many tokens, or do not fill the device
 
     def __init__(self, spec, dtype):
         super().__init__(spec, dtype)
@@ -69,8 +82,11 @@ class StateSpaceMixer(Mixer):
         xbc = torch.empty(tokens, self.conv_channels, dtype=torch.float32, device=x.device)
         ops.causal_conv(proj, self.inner, self.conv_w, self.conv_b, slot.state, self.conv_off, step, xbc)
         y = torch.empty(tokens, self.inner, dtype=torch.float32, device=x.device)
-        ops.ssm_scan(xbc, proj, self.inner + self.conv_channels, self.dt_bias, self.a_log, self.d_skip, slot.state, step, y,
-                     heads=s.num_heads, head_dim=s.head_dim, state_size=s.state_size, groups=s.groups)
+        walk = (takes_chunks(self, step, s.num_heads, s.head_dim, x.device)
+                and ops.chunk_walk_supported(s.state_size, s.head_dim))
+        (ops.ssm_walk if walk else ops.ssm_scan)(
+            xbc, proj, self.inner + self.conv_channels, self.dt_bias, self.a_log, self.d_skip, slot.state, step, y,
+            heads=s.num_heads, head_dim=s.head_dim, state_size=s.state_size, groups=s.groups)
         gated = torch.empty(tokens, self.inner, dtype=x.dtype, device=x.device)
         ops.gated_group_norm(y, proj, 0, self.norm_w, gated, parts=s.norm_groups, eps=s.norm_eps)
         return linear(gated, self.o)
@@ -86,7 +102,8 @@ class GatedDeltaMixer(Mixer):
     with ``a`` a column of the input projection, and the gate ``gate_activation(g)`` with ``g`` columns of
     the input projection (no low ranks)."""
     graph_safe = True
-    chunk_min_tokens = 16        # (one decay per head) the longest entry of a step from which the chunked kernel runs; None: never
+    chunk_min_tokens = 16        # the longest entry of a step from which the recurrence runs in chunks; None: never
+    chunk_min_average = 64       # ... if the step's entries average this many tokens, or do not fill the device
 
     def __init__(self, spec, dtype):
         super().__init__(spec, dtype)
@@ -138,27 +155,29 @@ class GatedDeltaMixer(Mixer):
         a, gate = proj[:, self.a_off:self.a_off + self.a_cols], proj[:, self.g_off:self.g_off + self.g_cols]
         if not self.per_head:       # through the low ranks
             a, gate = linear(a, self.a2), linear(gate, self.g2)
-        dec = torch.empty(tokens, s.num_heads * s.head_dim, dtype=torch.float32, device=dev)
-        beta = torch.empty(tokens, s.num_heads, dtype=torch.float32, device=dev)
-        # One decay per head: a step with a prompt portion whose (entry, head, 32 columns) blocks do not fill the device
-        # takes the recurrence in chunks of 64 tokens.  The chunked form does about twice the 32-bit multiply-adds of the
-        # walk token by token (the keys' products with one another, the triangular system, the products with the state at
-        # the chunk's start), so it is ahead only while the walk leaves SMs idle (measured at 16 heads of 128 x 128: one
-        # 2,048-token prompt 930 against 1,010 us; four of them about 1,500 against 1,220 us).
-        chunked = (self.per_head and self.chunk_min_tokens is not None and step.max_q_len >= self.chunk_min_tokens
-                   and s.head_dim <= ops.LIMITS["delta_chunk_max_head_dim"]
+        # Steps with prompt portions run the recurrence in chunks, prepared side by side and walked (csrc/chunk_walk.cuh); so do
+        # not: steps of single tokens and short pieces, and head sizes the chunks do not take.
+        sizes = dict(heads=s.num_heads, kv_heads=s.num_kv_heads, head_dim=s.head_dim, v_head_dim=s.v_head_dim)
+        long = takes_chunks(self, step, s.num_heads, s.v_head_dim, dev)
+        walk = long and ops.chunk_walk_supported(s.head_dim, s.v_head_dim)
+        # One decay per head and a head size beyond that: chunks of 64 tokens in one kernel, while its (entry, head, 32
+        # columns) blocks do not fill the device (it does about twice the multiply-adds of the walk token by token).
+        chunked = (long and not walk and self.per_head and s.head_dim <= ops.LIMITS["delta_chunk_max_head_dim"]
                    and step.num_seqs * s.num_heads * (-(-s.v_head_dim // 32)) <= ops.sm_count(dev))
-        log_dec = torch.empty(tokens, s.num_heads, dtype=torch.float32, device=dev) if chunked else None
-        ops.delta_prep(qkv, a, proj, self.b_off, self.dt_bias, self.a_log, dec, beta, heads=s.num_heads,
-                       kv_heads=s.num_kv_heads, head_dim=s.head_dim, v_head_dim=s.v_head_dim, unit_eps=s.unit_eps,
+        log_dec = torch.empty(tokens, s.num_heads, dtype=torch.float32, device=dev) if self.per_head and long else None
+        dec = None
+        if not (self.per_head and (walk or chunked)):
+            dec = torch.empty(tokens, s.num_heads * s.head_dim, dtype=torch.float32, device=dev)
+        beta = torch.empty(tokens, s.num_heads, dtype=torch.float32, device=dev)
+        ops.delta_prep(qkv, a, proj, self.b_off, self.dt_bias, self.a_log, dec, beta, **sizes, unit_eps=s.unit_eps,
                        q_scale=s.head_dim ** -0.5, per_head=self.per_head, log_dec=log_dec)
         o = torch.empty(tokens, self.vv, dtype=torch.float32, device=dev)
-        if chunked:
-            ops.delta_chunk(qkv, log_dec, beta, slot.state, step, o, heads=s.num_heads, kv_heads=s.num_kv_heads,
-                            head_dim=s.head_dim, v_head_dim=s.v_head_dim)
+        if walk:
+            ops.delta_walk(qkv, dec, log_dec if self.per_head else None, beta, slot.state, step, o, **sizes)
+        elif chunked:
+            ops.delta_chunk(qkv, log_dec, beta, slot.state, step, o, **sizes)
         else:
-            ops.delta_scan(qkv, dec, beta, slot.state, step, o, heads=s.num_heads, kv_heads=s.num_kv_heads,
-                           head_dim=s.head_dim, v_head_dim=s.v_head_dim)
+            ops.delta_scan(qkv, dec, beta, slot.state, step, o, **sizes)
         out = torch.empty(tokens, self.vv, dtype=x.dtype, device=dev)
         ops.delta_out(o, gate, self.norm_w, out, heads=s.num_heads, v_head_dim=s.v_head_dim, eps=s.norm_eps,
                       silu=s.gate_activation == "silu")

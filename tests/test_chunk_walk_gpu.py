@@ -1,0 +1,130 @@
+"""The linear recurrences over prompt portions in chunks (csrc/chunk_walk.cuh) against 64-bit walks token by token, from
+non-zero states, with entries that end on, before and behind the chunks' edges."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+LENS = [1, 63, 64, 65, 200, 0, 31, 32, 33, 17]
+# two orders of the same 32-bit sums over at most 200 tokens and 128 rows, as a share of the largest value
+BOUND = 5e-6
+
+
+def _step(rows):
+    cu = [0]
+    for n in LENS:
+        cu.append(cu[-1] + n)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    return SimpleNamespace(cu_q=torch.tensor(cu, **i32), seq_rows=torch.tensor(rows, **i32), num_seqs=len(LENS), num_tokens=cu[-1],
+                           max_q_len=max(LENS), cu=cu, rows=rows,
+                           token_seq=torch.tensor([e for e, n in enumerate(LENS) for _ in range(n)], **i32))
+
+
+def _walk64(q, k, v, keep, S, beta=None):
+    """q, k [T, H, d], v [T, H, dv], keep [T, H, 1 or d], S [H, d, dv]; the delta rule with ``beta`` [T, H]."""
+    out = []
+    for t in range(q.shape[0]):
+        S = keep[t][..., None] * S
+        u = v[t]
+        if beta is not None:
+            u = beta[t][:, None] * (v[t] - torch.einsum("hd,hdv->hv", k[t], S))
+        S = S + k[t][..., None] * u[:, None]
+        out.append(torch.einsum("hd,hdv->hv", q[t], S))
+    return (torch.stack(out) if out else v), S
+
+
+def _close(got, want, what):
+    worst, most = float((got.double() - want).abs().max()), float(want.abs().max())
+    assert worst < BOUND * most, f"{what}: {worst:.3e} of {most:.3e}"
+
+
+SIZES = [(128, 128, 3, 3), (64, 64, 4, 2), (8, 4, 2, 1), (100, 36, 3, 3), (128, 20, 40, 10), (44, 132, 2, 2)]
+
+
+@pytest.mark.parametrize("decay", ["slow", "fast"])
+@pytest.mark.parametrize("d,dv,heads,kv_heads", SIZES)
+@pytest.mark.parametrize("kind", ["retention", "state space", "delta, per head", "delta, per channel"])
+def test_chunks_against_the_walk(kind, d, dv, heads, kv_heads, decay):
+    """``fast``: decays down to e^-30 per token, whose products underflow within a chunk."""
+    from sparseengine_b200.csrc import ops
+    step = _step([3, 0, 11, 1, 7, 2, 5, 4, 9, 6])
+    T, g = step.num_tokens, torch.Generator(device=DEV).manual_seed(d + heads)
+
+    def rnd(*shape):
+        return torch.randn(*shape, generator=g, device=DEV)
+
+    state = rnd(12, heads * d * dv + 5)
+    first = state.double().clone()
+    logs = -(torch.rand(T, heads, d, generator=g, device=DEV) * (30.0 if decay == "fast" else 0.2))
+    o = torch.full((T, heads, dv), float("nan"), device=DEV)
+    rep, beta = heads // kv_heads, torch.rand(T, heads, generator=g, device=DEV)
+    sizes = dict(heads=heads, head_dim=d, v_head_dim=dv)
+    column_major = kind != "retention"          # [head][column][row], retention [head][row][column]
+    skip = None
+    if kind == "retention":
+        q, k, v = rnd(T, heads, d), rnd(T, heads, d) * d ** -0.5, rnd(T, heads * dv + 8).to(torch.bfloat16)
+        decays = torch.exp(logs[0, :, 0])
+        ops.retention_chunk(q.view(T, -1), k.view(T, -1), v, 4, decays, state, step, o.view(T, -1), silu=True, **sizes)
+        v = torch.nn.functional.silu(v[:, 4:4 + heads * dv].double()).view(T, heads, dv)
+        keep = decays.double().view(1, heads, 1).expand(T, -1, -1)
+        beta = None
+    elif kind == "state space":
+        width = heads * dv + 2 * kv_heads * d
+        xbc, proj = rnd(T, width), rnd(T, heads + 3)
+        bias, a_log, skip = rnd(heads) - 2.0, torch.log(torch.rand(heads, generator=g, device=DEV) * (30 if decay == "fast" else 1) + 0.1), rnd(heads)
+        ops.ssm_walk(xbc, proj, 2, bias, a_log, skip, state, step, o.view(T, -1), heads=heads, head_dim=dv, state_size=d, groups=kv_heads)
+        dt = torch.nn.functional.softplus(proj[:, 2:2 + heads].double() + bias.double())
+        x = xbc[:, :heads * dv].double().view(T, heads, dv)
+        k = xbc[:, heads * dv:heads * dv + kv_heads * d].view(T, kv_heads, d).repeat_interleave(rep, 1)
+        q = xbc[:, heads * dv + kv_heads * d:].view(T, kv_heads, d).repeat_interleave(rep, 1)
+        v, keep, beta = x * dt[..., None], torch.exp(-torch.exp(a_log.double()) * dt)[..., None], None
+    else:
+        qk = torch.nn.functional.normalize(rnd(T, 2 * kv_heads, d), dim=-1)
+        qkv = torch.cat([qk.reshape(T, -1), rnd(T, heads * dv)], 1)
+        per_head = kind == "delta, per head"
+        if per_head:
+            logs = logs[..., 0].contiguous()
+        dec = None if per_head else torch.exp(logs).view(T, -1)
+        ops.delta_walk(qkv, dec, logs if per_head else None, beta, state, step, o.view(T, -1), heads=heads, kv_heads=kv_heads, head_dim=d, v_head_dim=dv)
+        q, k = (t.repeat_interleave(rep, 1) for t in (qk[:, :kv_heads], qk[:, kv_heads:]))
+        v = qkv[:, 2 * kv_heads * d:].double().view(T, heads, dv)
+        keep = torch.exp(logs.double())[..., None] if per_head else dec.double().view(T, heads, d)
+        beta = beta.double()
+    assert bool(torch.isfinite(o).all())
+    for e, n in enumerate(LENS):
+        a, b, row = step.cu[e], step.cu[e + 1], step.rows[e]
+        S = first[row, :heads * d * dv].view(heads, *((dv, d) if column_major else (d, dv)))
+        S = S.transpose(1, 2) if column_major else S
+        want, S = _walk64(q[a:b].double(), k[a:b].double(), v[a:b], keep[a:b], S, None if beta is None else beta[a:b])
+        if n == 0:
+            assert torch.equal(state[row].double(), first[row])
+            continue
+        if skip is not None:
+            want = want + skip.double()[:, None] * x[a:b]
+        _close(o[a:b], want, f"outputs of {n} tokens")
+        got = state[row, :heads * d * dv].view(heads, *((dv, d) if column_major else (d, dv)))
+        _close(got.transpose(1, 2) if column_major else got, S, f"state after {n} tokens")
+    others = [r for r in range(12) if r not in step.rows]
+    assert torch.equal(state[others].double(), first[others]) and torch.equal(state[:, heads * d * dv:].double(), first[:, heads * d * dv:])
+
+
+@pytest.mark.parametrize("kind", ["per head", "per channel"])
+def test_later_tokens_do_not_touch_earlier_ones(kind):
+    """A value that is not finite reaches the outputs of its own token and of later ones only."""
+    from sparseengine_b200.csrc import ops
+    H, d, T = 2, 64, 70
+    step = SimpleNamespace(cu_q=torch.tensor([0, T], dtype=torch.int32, device=DEV), seq_rows=torch.zeros(1, dtype=torch.int32, device=DEV), num_seqs=1)
+    g = torch.Generator(device=DEV).manual_seed(1)
+    qkv = torch.randn(T, 3 * H * d, generator=g, device=DEV) * 0.1
+    logs, beta = -torch.rand(T, H, generator=g, device=DEV), torch.rand(T, H, generator=g, device=DEV)
+    dec = torch.rand(T, H * d, generator=g, device=DEV) if kind == "per channel" else None
+    outs = []
+    for bad in (False, True):
+        if bad:
+            qkv[41, 2 * H * d + 3] = float("inf")
+        o = torch.empty(T, H * d, device=DEV)
+        ops.delta_walk(qkv, dec, logs if dec is None else None, beta, torch.zeros(1, H * d * d, device=DEV), step, o, heads=H, kv_heads=H, head_dim=d, v_head_dim=d)
+        outs.append(o)
+    assert torch.equal(outs[0][:41], outs[1][:41]) and not bool(torch.isfinite(outs[1][41:]).all())
