@@ -86,206 +86,167 @@ struct WalkArgs {
     int H, d, dv;
 };
 
+// Two groups of four warps share a chunk's products.  Without a system to solve, group 0 makes the outputs (q S_0, then P u, sums
+// over the slices, stores) while group 1 updates the state into a second buffer and brings the next values: one barrier for
+// all per chunk.  With one, group 0 makes u = U - W S_0 and then the state's update while group 1 makes q S_0 and then the
+// outputs: two barriers.  A thread holds T / 8 rows x C / 4 columns of its warp's slice (8 x 8 at best: an FMA costs a quarter of
+// a shared-memory wavefront then, and both units are as busy).  q, k, P and W of the next chunk are copied as soon as the last
+// reader of this one's has passed.
 template <int T, int DP, int C, bool SOLVE, bool CHANNEL>
 struct WalkShape {
-    static constexpr int kRowSplit = T == 64 && C == 32 ? 2 : 1;      // row halves of the products with the state ...
-    static constexpr int kSlices = 8 / kRowSplit;                     // ... and slices of their inner dimension, per warp
-    static constexpr int kTimeSplit = 8 / (DP / 32);                  // slices of the tokens in the state's update
+    static constexpr int kSlices = 4;                                 // of the inner dimension (or the tokens), a warp each
+    static constexpr int kRowGroups = DP / 64;                        // 64 rows of the state per warp ...
+    static constexpr int kTimeSplit = 4 / kRowGroups;                 // ... and a slice of the tokens
     static constexpr int kQP = DP + 4, kPP = T + 4;
-    static constexpr int kFloats = (SOLVE ? 3 : 2) * T * kQP + T * kPP + 2 * T * C + DP * C + kSlices * T * C +
-                                   (kTimeSplit - 1) * DP * C + 2 * T + (CHANNEL ? DP : 0);
+    static constexpr int kFloats = 3 * T * kQP + T * kPP + (SOLVE ? 2 : 3) * T * C + (SOLVE ? 1 : 2) * DP * C +
+                                   kSlices * T * C + (kTimeSplit - 1) * DP * C + 2 * T + (CHANNEL ? DP : 0);
 };
+
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory"); }
 
 template <int T, int DP, int C, bool SOLVE, bool CHANNEL, typename TV>
 __global__ void __launch_bounds__(kThreads, 1)
 chunk_walk_kernel(const WalkArgs a) {
     using Shape = WalkShape<T, DP, C, SOLVE, CHANNEL>;
-    constexpr int QP = Shape::kQP, PP = Shape::kPP, KS = Shape::kSlices, TS = Shape::kTimeSplit;
-    constexpr int RM = T / 8 / Shape::kRowSplit, RC = C / 4;           // rows and columns of a thread's output tile
-    constexpr int NV = (T * C / 4 + kThreads - 1) / kThreads;          // value quads per thread
+    constexpr int QP = Shape::kQP, PP = Shape::kPP, KS = Shape::kSlices, TS = Shape::kTimeSplit, RG = Shape::kRowGroups;
+    constexpr int RM = T / 8, RC = C / 4;            // rows and columns of a thread's output tile
+    constexpr int NQ = T * C / 4 / 128;              // quads of the chunk's value columns per thread of a group
     extern __shared__ __align__(16) float sm[];
     float* qs = sm;                                  // [T][QP]
-    float* ks = qs + T * QP;                         // [T][QP]
-    float* ws = ks + T * QP;                         // [T][QP]
-    float* ps = ws + (SOLVE ? T * QP : 0);           // [T][PP]
-    float* us = ps + T * PP;                         // [T][C]: u
-    float* u2 = us + T * C;                          // [T][C]: e^(B_n - B_t) u (decays per head)
-    float* Ss = u2 + T * C;                          // [DP][C]
-    float* part = Ss + DP * C;                       // [KS][T][C]
+    float* ks = qs + T * QP;                         // [T][QP], twice without a system to solve
+    float* ws = ks + T * QP;                         // [T][QP]: W, or the second k
+    float* ps = ws + T * QP;                         // [T][PP]
+    float* us = ps + T * PP;                         // [T][C]: u; twice without a system to solve
+    float* u2 = us + (SOLVE ? 1 : 2) * T * C;        // [T][C]: e^(B_n - B_t) u (decays per head)
+    float* Ss = u2 + T * C;                          // [DP][C]; twice without a system to solve
+    float* part = Ss + (SOLVE ? 1 : 2) * DP * C;     // [KS][T][C]
     float* part2 = part + KS * T * C;                // [TS - 1][DP][C]
-    float* rss = part2 + (TS - 1) * DP * C;          // [T]
-    float* tss = rss + T;                            // [T]
-    float* tots = tss + T;                           // [DP]
+    float* rss = part2 + (TS - 1) * DP * C;          // [2][T]
+    float* tots = rss + 2 * T;                       // [DP]
     const int e = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * C;
     const int t_first = a.cu_q[e], t_last = a.cu_q[e + 1];
     if (t_last <= t_first) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lc = lane & 3;
+    const int group = warp >> 2, gw = warp & 3, gt = tid & 127;          // the group, and this thread's place in it
     const int d = a.d, dv = a.dv;
-    const int d4 = d / 4;
 
-    // columns of q, k and w beyond d, once; the loads below never touch them
-    if (d < DP)
-        for (int i = tid; i < (SOLVE ? 3 : 2) * T * (DP - d); i += kThreads) {
-            const int r = i / (DP - d);
-            qs[r * QP + d + i - r * (DP - d)] = 0.f;
-        }
     float* S0 = a.state + (size_t)a.seq_rows[e] * a.state_stride + (size_t)h * d * dv;
     for (int i = tid; i < DP * C; i += kThreads) {   // the faster index in memory runs over neighbouring threads
         const int row = a.s_row == 1 ? i % DP : i / C, c = a.s_row == 1 ? i / DP : i % C;
         Ss[row * C + c] = row < d && c0 + c < dv ? S0[(size_t)row * a.s_row + (size_t)(c0 + c) * a.s_col] : 0.f;
     }
 
-    const float* qb = a.q + (size_t)(h / a.rep) * d;
-    const float* kb = a.k + (size_t)(h / a.rep) * d;
-    auto load_qw = [&](int t0, int n) {
-        for (int i = tid; i < T * d4; i += kThreads) {
-            const int t = i / d4, c = (i - t * d4) * 4;
-            const size_t row = (size_t)(t0 + (t < n ? t : 0));
-            cp16(qs + t * QP + c, qb + row * a.qk_stride + c, t < n);
-            if (SOLVE) cp16(ws + t * QP + c, a.w + (row * a.H + h) * d + c, t < n);
+    // T rows of d columns to shared memory by one group; rows from n on and columns from d on are zeros
+    auto load_rows = [&](float* tile, const float* src, size_t stride, int t0, int n) {
+#pragma unroll 4
+        for (int i = gt; i < T * (DP / 4); i += 128) {
+            const int t = i / (DP / 4), c = (i % (DP / 4)) * 4;
+            const bool in = t < n && c < d;
+            cp16(tile + t * QP + c, src + (size_t)(t0 + (in ? t : 0)) * stride + (in ? c : 0), in);
         }
-        cp_commit();
     };
-    auto load_kp = [&](int t0, int n) {
-        for (int i = tid; i < T * d4; i += kThreads) {
-            const int t = i / d4, c = (i - t * d4) * 4;
-            cp16(ks + t * QP + c, kb + (size_t)(t0 + (t < n ? t : 0)) * a.qk_stride + c, t < n);
-        }
-        for (int i = tid; i < T * (T / 4); i += kThreads) {
-            const int t = i / (T / 4), c = (i - t * (T / 4)) * 4;
+    auto load_p = [&](int t0, int n) {
+#pragma unroll 4
+        for (int i = gt; i < T * (T / 4); i += 128) {
+            const int t = i / (T / 4), c = (i % (T / 4)) * 4;
             cp16(ps + t * PP + c, a.p + ((size_t)(t0 + (t < n ? t : 0)) * a.H + h) * T + c, t < n);
         }
-        cp_commit();
     };
-    // values (a quad per place i * kThreads + tid) and per-token factors of a chunk, in registers until they are wanted
+    const float* qb = a.q + (size_t)(h / a.rep) * d;
+    const float* kb = a.k + (size_t)(h / a.rep) * d;
+    const float* wb = SOLVE ? a.w + (size_t)h * d : nullptr;
     const TV* vb = static_cast<const TV*>(a.v) + (size_t)h * dv + c0;
-    float4 vreg[NV];
-    float fac = 0.f, vfac[NV];
+    // value rows (or U) of a chunk, quad by quad, with the factors that go with their tokens
+    float4 vreg[NQ];
+    float vfac[NQ], tfac[NQ], rfac = 0.f;
     auto load_v = [&](int t0, int n) {
 #pragma unroll
-        for (int x = 0; x < NV; ++x) {
-            const int i = x * kThreads + tid, t = i / (C / 4), c = (i - t * (C / 4)) * 4;
-            const bool in = i < T * C / 4 && t < n && c0 + c < dv;
+        for (int x = 0; x < NQ; ++x) {
+            const int i = x * 128 + gt, t = i / (C / 4), c = (i % (C / 4)) * 4;
+            const bool in = t < n && c0 + c < dv;
+            const size_t at = (size_t)(t0 + t) * a.H + h;
             vreg[x] = in ? load4(vb + (size_t)(t0 + t) * a.v_stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-            vfac[x] = in && a.v_scale != nullptr ? a.v_scale[(size_t)(t0 + t) * a.H + h] : 1.f;
+            vfac[x] = !SOLVE && in && a.v_scale != nullptr ? a.v_scale[at] : 1.f;
+            tfac[x] = !CHANNEL && in ? a.ts[at] : 1.f;
         }
-        if (!CHANNEL && tid < 2 * T) {
-            const int t = tid < T ? tid : tid - T;
-            fac = t < n ? (tid < T ? a.rs : a.ts)[(size_t)(t0 + t) * a.H + h] : 0.f;
-        }
-        if (CHANNEL && tid < d) fac = a.tot[((size_t)(t_first / T + e + (t0 - t_first) / T) * a.H + h) * d + tid];
     };
-    const float skip = a.skip != nullptr ? a.skip[h] : 0.f;
-
-    const int first_n = min(T, t_last - t_first);
-    load_qw(t_first, first_n);
-    load_kp(t_first, first_n);
-    load_v(t_first, first_n);
-    const int slice = warp / Shape::kRowSplit, r0 = (warp % Shape::kRowSplit) * (T / Shape::kRowSplit);
-    for (int t0 = t_first; t0 < t_last; t0 += T) {
-        const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
-        float4 raw[NV];                              // the value rows as they are (or the solved U)
+    auto load_factors = [&](int t0, int n) {         // e^(B_t) of the chunk's tokens, or e^(B_n) of the channels
+        if (!CHANNEL && gt < T) rfac = gt < n ? a.rs[(size_t)(t0 + gt) * a.H + h] : 0.f;
+        if (CHANNEL) rfac = gt < d ? a.tot[((size_t)(t_first / T + e + (t0 - t_first) / T) * a.H + h) * d + gt] : 0.f;
+    };
+    int odd = 0;                                     // a value that is not finite
+    auto put_u = [&](int x, float4 u, float* to) {   // u and e^(B_n - B_t) u of one quad
+        const int i = x * 128 + gt;
+        odd |= !(isfinite(u.x) && isfinite(u.y) && isfinite(u.z) && isfinite(u.w));
+        st4(to + i * 4, u);
+        if (!CHANNEL) st4(u2 + i * 4, make_float4(u.x * tfac[x], u.y * tfac[x], u.z * tfac[x], u.w * tfac[x]));
+    };
+    auto put_values = [&](float* to) {
 #pragma unroll
-        for (int x = 0; x < NV; ++x) {
-            raw[x] = vreg[x];
-            if (a.silu) raw[x] = make_float4(value_silu<TV>(raw[x].x), value_silu<TV>(raw[x].y), value_silu<TV>(raw[x].z), value_silu<TV>(raw[x].w));
+        for (int x = 0; x < NQ; ++x) {
+            float4 v = vreg[x];
+            if (a.silu) v = make_float4(value_silu<TV>(v.x), value_silu<TV>(v.y), value_silu<TV>(v.z), value_silu<TV>(v.w));
+            put_u(x, make_float4(v.x * vfac[x], v.y * vfac[x], v.z * vfac[x], v.w * vfac[x]), to);
         }
-        int odd = 0;                                 // a value that is not finite
-        if (!CHANNEL && tid < 2 * T) (tid < T ? rss : tss - T)[tid] = fac;
-        if (CHANNEL && tid < DP) tots[tid] = tid < d ? fac : 0.f;
-        auto put_u = [&](int x, float4 u, float after) {     // u and e^(B_n - B_t) u of one quad
-            const int i = x * kThreads + tid;
-            if (i >= T * C / 4) return;
-            odd |= !(isfinite(u.x) && isfinite(u.y) && isfinite(u.z) && isfinite(u.w));
-            st4(us + i * 4, u);
-            if (!CHANNEL) st4(u2 + i * 4, make_float4(u.x * after, u.y * after, u.z * after, u.w * after));
-        };
-        cp_wait<1>();                                // this chunk's q and w
-        __syncthreads();                             // (and the state is up to date)
-        if (!SOLVE)
+    };
+    // acc = rows of x . S, a warp's slice of the inner dimension
+    auto state_product = [&](const float* x, const float* S, float (&acc)[RM][RC]) {
 #pragma unroll
-            for (int x = 0; x < NV; ++x) {
-                const int t = (x * kThreads + tid) / (C / 4);
-                put_u(x, make_float4(raw[x].x * vfac[x], raw[x].y * vfac[x], raw[x].z * vfac[x], raw[x].w * vfac[x]), CHANNEL || t >= T ? 1.f : tss[t]);
-            }
-        // products with the state: a warp takes T (or T/2) rows, all columns and a slice of the inner dimension
-        float acc[RM][RC] = {}, accw[SOLVE ? RM : 1][RC] = {};
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int c = 0; c < RC; ++c) acc[i][c] = 0.f;
 #pragma unroll 2
-        for (int k = slice * (DP / KS); k < (slice + 1) * (DP / KS); k += 4) {
+        for (int k = gw * (DP / KS); k < (gw + 1) * (DP / KS); k += 4) {
             float sv[4][RC];
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int g = 0; g < RC / 4; ++g) *reinterpret_cast<float4*>(&sv[j][4 * g]) = ld4(Ss + (k + j) * C + 16 * g + lc * 4);
+                for (int g = 0; g < RC / 4; ++g) *reinterpret_cast<float4*>(&sv[j][4 * g]) = ld4(S + (k + j) * C + 16 * g + lc * 4);
 #pragma unroll
             for (int i = 0; i < RM; ++i) {
-                const float4 qv = ld4(qs + (r0 + lr + 8 * i) * QP + k);
+                const float4 v = ld4(x + (lr + 8 * i) * QP + k);
 #pragma unroll
-                for (int c = 0; c < RC; ++c) acc[i][c] = fmaf(qv.w, sv[3][c], fmaf(qv.z, sv[2][c], fmaf(qv.y, sv[1][c], fmaf(qv.x, sv[0][c], acc[i][c]))));
-                if (SOLVE) {
-                    const float4 wv = ld4(ws + (r0 + lr + 8 * i) * QP + k);
-#pragma unroll
-                    for (int c = 0; c < RC; ++c) accw[i][c] = fmaf(wv.w, sv[3][c], fmaf(wv.z, sv[2][c], fmaf(wv.y, sv[1][c], fmaf(wv.x, sv[0][c], accw[i][c]))));
-                }
+                for (int c = 0; c < RC; ++c) acc[i][c] = fmaf(v.w, sv[3][c], fmaf(v.z, sv[2][c], fmaf(v.y, sv[1][c], fmaf(v.x, sv[0][c], acc[i][c]))));
             }
         }
-        auto put_part = [&](const float (*v)[RC]) {
+    };
+    auto put_part = [&](const float (&v)[RM][RC]) {
 #pragma unroll
-            for (int i = 0; i < RM; ++i)
+        for (int i = 0; i < RM; ++i)
 #pragma unroll
-                for (int g = 0; g < RC / 4; ++g)
-                    st4(part + (slice * T + r0 + lr + 8 * i) * C + 16 * g + lc * 4, make_float4(v[i][4 * g], v[i][4 * g + 1], v[i][4 * g + 2], v[i][4 * g + 3]));
-        };
-        auto sum_part = [&](int x) {                 // the sum over the slices of one quad
-            const int i = x * kThreads + tid;
-            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i < T * C / 4)
+            for (int g = 0; g < RC / 4; ++g)
+                st4(part + (gw * T + lr + 8 * i) * C + 16 * g + lc * 4, make_float4(v[i][4 * g], v[i][4 * g + 1], v[i][4 * g + 2], v[i][4 * g + 3]));
+    };
+    auto sum_part = [&](int x) {                     // the sum over the slices of one quad
+        float4 s = ld4(part + (x * 128 + gt) * 4);
 #pragma unroll
-                for (int z = 0; z < KS; ++z) {
-                    const float4 v = ld4(part + z * T * C + i * 4);
-                    s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
-                }
-            return s;
-        };
-        if (SOLVE) put_part(accw);
-        cp_wait<0>();                                // this chunk's k and P
-        if (SOLVE) {
-            __syncthreads();
-#pragma unroll
-            for (int x = 0; x < NV; ++x) {
-                const int t = (x * kThreads + tid) / (C / 4);
-                const float4 s = sum_part(x);
-                put_u(x, make_float4(raw[x].x - s.x, raw[x].y - s.y, raw[x].z - s.z, raw[x].w - s.w), CHANNEL || t >= T ? 1.f : tss[t]);
-            }
+        for (int z = 1; z < KS; ++z) {
+            const float4 v = ld4(part + z * T * C + (x * 128 + gt) * 4);
+            s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
         }
-        odd = __syncthreads_or(odd);
-        if (next < t_last) {                         // q and w have been read: the next chunk's follow
-            load_qw(next, next_n);
-            load_v(next, next_n);
-        } else {
-            cp_commit();
-        }
-        // what the chunk's own tokens add: P u, a slice of the tokens s per warp; P is zero for s > t
+        return s;
+    };
+    // acc = e^(B_t) acc + P u, a warp's slice of the tokens s; P is zero for s > t
+    auto add_tokens = [&](const float* u, const float* factors, int any_odd, float (&acc)[RM][RC]) {
         if (!CHANNEL)
 #pragma unroll
             for (int i = 0; i < RM; ++i) {
-                const float f = rss[r0 + lr + 8 * i];
+                const float f = factors[lr + 8 * i];
 #pragma unroll
                 for (int c = 0; c < RC; ++c) acc[i][c] *= f;
             }
-        auto add_tokens = [&](bool guarded) {
-#pragma unroll
-            for (int sq = 0; sq < T / KS; sq += 4) {
-                const int s = slice * (T / KS) + sq;
+        auto run = [&](bool guarded) {
+#pragma unroll 1
+            for (int s = gw * (T / KS); s < (gw + 1) * (T / KS); s += 4) {
                 float uv[4][RC];
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
 #pragma unroll
-                    for (int g = 0; g < RC / 4; ++g) *reinterpret_cast<float4*>(&uv[j][4 * g]) = ld4(us + (s + j) * C + 16 * g + lc * 4);
+                    for (int g = 0; g < RC / 4; ++g) *reinterpret_cast<float4*>(&uv[j][4 * g]) = ld4(u + (s + j) * C + 16 * g + lc * 4);
 #pragma unroll
                 for (int i = 0; i < RM; ++i) {
-                    if (r0 + 8 * i + 7 < s) continue;        // rows before these tokens
-                    const int t = r0 + lr + 8 * i;
+                    if (8 * i + 7 < s) continue;     // rows before these tokens
+                    const int t = lr + 8 * i;
                     const float4 pv = ld4(ps + t * PP + s);
                     const float p4[4] = {pv.x, pv.y, pv.z, pv.w};
 #pragma unroll
@@ -296,65 +257,175 @@ chunk_walk_kernel(const WalkArgs a) {
                 }
             }
         };
-        if (odd) add_tokens(true);                   // a token that a row does not see does not touch it, whatever it holds
-        else add_tokens(false);
-        put_part(acc);
-        // the state's update: a warp takes 32 rows, all columns and a slice of the tokens
-        const int dg = warp % (DP / 32), tsl = warp / (DP / 32), row0 = dg * 32 + lr * 4;
-        const float* uu = CHANNEL ? us : u2;
-        float st[4][RC] = {};
-#pragma unroll 4
-        for (int s = tsl * (T / TS); s < (tsl + 1) * (T / TS); ++s) {
-            const float4 kv = ld4(ks + s * QP + row0);
-            const float k4[4] = {kv.x, kv.y, kv.z, kv.w};
-            float uv[RC];
+        if (any_odd) run(true);                      // a token that a row does not see does not touch it, whatever it holds
+        else run(false);
+    };
+    auto put_outputs = [&](int t0, int n) {
+        const float skip = a.skip != nullptr ? a.skip[h] : 0.f;
 #pragma unroll
-            for (int g = 0; g < RC / 4; ++g) *reinterpret_cast<float4*>(&uv[4 * g]) = ld4(uu + s * C + 16 * g + lc * 4);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int c = 0; c < RC; ++c) st[i][c] = fmaf(k4[i], uv[c], st[i][c]);
-        }
-        if (tsl > 0)
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int g = 0; g < RC / 4; ++g)
-                    st4(part2 + ((tsl - 1) * DP + row0 + i) * C + 16 * g + lc * 4, make_float4(st[i][4 * g], st[i][4 * g + 1], st[i][4 * g + 2], st[i][4 * g + 3]));
-        const float total = CHANNEL ? 0.f : rss[n - 1];
-        __syncthreads();                             // k, P, u and the old state have been read; the partial sums are there
-        if (next < t_last) load_kp(next, next_n);
-        else cp_commit();
-#pragma unroll
-        for (int x = 0; x < NV; ++x) {
-            const int i = x * kThreads + tid, t = i / (C / 4), c = (i - t * (C / 4)) * 4;
-            if (i < T * C / 4 && t < n && c0 + c < dv) {
-                const float4 s = sum_part(x);
-                st4(a.o + ((size_t)(t0 + t) * a.H + h) * dv + c0 + c,
-                    make_float4(s.x + skip * raw[x].x, s.y + skip * raw[x].y, s.z + skip * raw[x].z, s.w + skip * raw[x].w));
+        for (int x = 0; x < NQ; ++x) {
+            const int i = x * 128 + gt, t = i / (C / 4), c = (i % (C / 4)) * 4;
+            if (t < n && c0 + c < dv) {
+                float4 s = sum_part(x);
+                if (a.skip != nullptr) {
+                    const float4 v = load4(vb + (size_t)(t0 + t) * a.v_stride + c);
+                    s = make_float4(fmaf(skip, v.x, s.x), fmaf(skip, v.y, s.y), fmaf(skip, v.z, s.z), fmaf(skip, v.w, s.w));
+                }
+                st4(a.o + ((size_t)(t0 + t) * a.H + h) * dv + c0 + c, s);
             }
         }
-        if (tsl == 0)
+    };
+    // to = e^(B_n) from + sum_s k_s u_s^T: a warp takes 64 rows, all columns and a slice of the tokens; 8 rows x RC columns a thread
+    auto update_state = [&](const float* k, const float* u, const float* from, float* to, float total) {
+        const int row0 = (gw % RG) * 64 + lr * 8, slice = gw / RG;
+        float st[8][RC] = {};
+#pragma unroll 4
+        for (int s = slice * (T / TS); s < (slice + 1) * (T / TS); ++s) {
+            const float4 ka = ld4(k + s * QP + row0), kc = ld4(k + s * QP + row0 + 4);
+            const float k8[8] = {ka.x, ka.y, ka.z, ka.w, kc.x, kc.y, kc.z, kc.w};
+            float uv[RC];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int g = 0; g < RC / 4; ++g) *reinterpret_cast<float4*>(&uv[4 * g]) = ld4(u + s * C + 16 * g + lc * 4);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int c = 0; c < RC; ++c) st[i][c] = fmaf(k8[i], uv[c], st[i][c]);
+        }
+        if (slice > 0)
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int g = 0; g < RC / 4; ++g)
+                    st4(part2 + ((slice - 1) * DP + row0 + i) * C + 16 * g + lc * 4, make_float4(st[i][4 * g], st[i][4 * g + 1], st[i][4 * g + 2], st[i][4 * g + 3]));
+        group_sync(group);
+        if (slice == 0)
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
 #pragma unroll
                 for (int g = 0; g < RC / 4; ++g) {
                     const int at = (row0 + i) * C + 16 * g + lc * 4;
                     const float f = CHANNEL ? tots[row0 + i] : total;
-                    float4 s = ld4(Ss + at);
+                    float4 s = ld4(from + at);
                     s = make_float4(fmaf(f, s.x, st[i][4 * g]), fmaf(f, s.y, st[i][4 * g + 1]), fmaf(f, s.z, st[i][4 * g + 2]), fmaf(f, s.w, st[i][4 * g + 3]));
 #pragma unroll
                     for (int z = 0; z < TS - 1; ++z) {
                         const float4 v = ld4(part2 + z * DP * C + at);
                         s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
                     }
-                    st4(Ss + at, s);
+                    st4(to + at, s);
                 }
+    };
+
+    const int first_n = min(T, t_last - t_first);
+    float* last_state = Ss;
+    if (!SOLVE) {
+        if (group == 0) {
+            load_rows(qs, qb, a.qk_stride, t_first, first_n);
+            cp_commit();
+            load_p(t_first, first_n);
+            cp_commit();
+        } else {
+            load_rows(ks, kb, a.qk_stride, t_first, first_n);
+            cp_commit();
+            load_v(t_first, first_n);
+            load_factors(t_first, first_n);
+            put_values(us);
+            if (gt < T) rss[gt] = rfac;
+        }
+        int cur = 0;
+        for (int t0 = t_first; t0 < t_last; t0 += T, cur ^= 1) {
+            const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
+            if (group == 0) cp_wait<1>();            // q (P may still be on its way)
+            else cp_wait<0>();                       // k
+            const int any_odd = __syncthreads_or(odd);       // state, u and factors of this chunk are there as well
+            odd = 0;
+            if (group == 0) {
+                float acc[RM][RC];
+                state_product(qs, Ss + cur * DP * C, acc);
+                cp_wait<0>();
+                group_sync(0);                       // P is there, and q has been read
+                if (next < t_last) load_rows(qs, qb, a.qk_stride, next, next_n);
+                cp_commit();
+                add_tokens(us + cur * T * C, rss + cur * T, any_odd, acc);
+                put_part(acc);
+                group_sync(0);                       // the slices' sums are there, and P has been read
+                if (next < t_last) load_p(next, next_n);
+                cp_commit();
+                put_outputs(t0, n);
+            } else {
+                if (next < t_last) {
+                    load_rows(ks + (cur ^ 1) * T * QP, kb, a.qk_stride, next, next_n);
+                    load_v(next, next_n);
+                    load_factors(next, next_n);
+                }
+                cp_commit();
+                update_state(ks + cur * T * QP, u2, Ss + cur * DP * C, Ss + (cur ^ 1) * DP * C, rss[cur * T + n - 1]);
+                if (next < t_last) {                 // u2 has been read (the barrier inside)
+                    put_values(us + (cur ^ 1) * T * C);
+                    if (gt < T) rss[(cur ^ 1) * T + gt] = rfac;
+                }
+            }
+        }
+        last_state = Ss + cur * DP * C;
+    } else {
+        if (group == 0) {
+            load_rows(ws, wb, (size_t)a.H * d, t_first, first_n);
+            cp_commit();
+            load_rows(ks, kb, a.qk_stride, t_first, first_n);
+            cp_commit();
+            load_v(t_first, first_n);
+        } else {
+            load_rows(qs, qb, a.qk_stride, t_first, first_n);
+            cp_commit();
+            load_p(t_first, first_n);
+            cp_commit();
+        }
+        load_factors(t_first, first_n);
+        for (int t0 = t_first; t0 < t_last; t0 += T) {
+            const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
+            cp_wait<1>();                            // W or q (k and P may still be on their way)
+            __syncthreads();                         // and the state is up to date
+            float acc[RM][RC];
+            odd = 0;
+            if (CHANNEL ? (group == 0 && gt < DP) : (group == 1 && gt < T)) (CHANNEL ? tots : rss)[gt] = rfac;
+            state_product(group == 0 ? ws : qs, Ss, acc);
+            if (group == 0) {
+                put_part(acc);
+                group_sync(0);
+#pragma unroll
+                for (int x = 0; x < NQ; ++x) {
+                    const float4 s = sum_part(x);
+                    put_u(x, make_float4(vreg[x].x - s.x, vreg[x].y - s.y, vreg[x].z - s.z, vreg[x].w - s.w), us);
+                }
+            }
+            cp_wait<0>();
+            const int any_odd = __syncthreads_or(odd);       // u, k and P are there, W and q have been read
+            if (next < t_last) {
+                if (group == 0) load_rows(ws, wb, (size_t)a.H * d, next, next_n);
+                else load_rows(qs, qb, a.qk_stride, next, next_n);
+                if (group == 0) load_v(next, next_n);
+                load_factors(next, next_n);
+            }
+            cp_commit();
+            if (group == 0) {
+                update_state(ks, CHANNEL ? us : u2, Ss, Ss, CHANNEL ? 0.f : rss[n - 1]);
+                if (next < t_last) load_rows(ks, kb, a.qk_stride, next, next_n);       // k has been read (the barrier inside)
+                cp_commit();
+            } else {
+                add_tokens(us, rss, any_odd, acc);
+                put_part(acc);
+                group_sync(1);
+                if (next < t_last) load_p(next, next_n);
+                cp_commit();
+                put_outputs(t0, n);
+            }
+        }
     }
+    cp_wait<0>();
     __syncthreads();
     for (int i = tid; i < DP * C; i += kThreads) {
         const int row = a.s_row == 1 ? i % DP : i / C, c = a.s_row == 1 ? i / DP : i % C;
-        if (row < d && c0 + c < dv) S0[(size_t)row * a.s_row + (size_t)(c0 + c) * a.s_col] = Ss[row * C + c];
+        if (row < d && c0 + c < dv) S0[(size_t)row * a.s_row + (size_t)(c0 + c) * a.s_col] = last_state[row * C + c];
     }
 }
 
