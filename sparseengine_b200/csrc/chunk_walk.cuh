@@ -86,9 +86,9 @@ struct WalkArgs {
     int H, d, dv;
 };
 
-// Two groups of four warps share a chunk's products.  Without a system to solve, group 0 makes the outputs (q S_0, then P u, sums
-// over the slices, stores) while group 1 updates the state into a second buffer and brings the next values: one barrier for
-// all per chunk.  With one, group 0 makes u = U - W S_0 and then the state's update while group 1 makes q S_0 and then the
+// Two groups of four warps share a chunk's products.  Without a system to solve, group 0 makes the outputs (q S_0, then P u, in
+// four slices) while group 1 sums and stores those of the chunk before, updates the state into a second buffer and brings the
+// next values: one barrier for all per chunk, and one at which group 1 only arrives.  With one, group 0 makes u = U - W S_0 and then the state's update while group 1 makes q S_0 and then the
 // outputs: two barriers.  A thread holds T / 8 rows x C / 4 columns of its warp's slice (8 x 8 at best: an FMA costs a quarter of
 // a shared-memory wavefront then, and both units are as busy).  q, k, P and W of the next chunk are copied as soon as the last
 // reader of this one's has passed.
@@ -237,7 +237,7 @@ chunk_walk_kernel(const WalkArgs a) {
             }
         auto run = [&](bool guarded) {
 #pragma unroll 1
-            for (int s = gw * (T / KS); s < (gw + 1) * (T / KS); s += 4) {
+            for (int s = 4 * gw; s < T; s += 4 * KS) {           // dealt out in turn: early tokens have more rows
                 float uv[4][RC];
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
@@ -262,13 +262,20 @@ chunk_walk_kernel(const WalkArgs a) {
     };
     auto put_outputs = [&](int t0, int n) {
         const float skip = a.skip != nullptr ? a.skip[h] : 0.f;
+        float4 raw[NQ];
+        if (!SOLVE && a.skip != nullptr)
+#pragma unroll
+            for (int x = 0; x < NQ; ++x) {
+                const int i = x * 128 + gt, t = i / (C / 4), c = (i % (C / 4)) * 4;
+                raw[x] = t < n && c0 + c < dv ? load4(vb + (size_t)(t0 + t) * a.v_stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
 #pragma unroll
         for (int x = 0; x < NQ; ++x) {
             const int i = x * 128 + gt, t = i / (C / 4), c = (i % (C / 4)) * 4;
             if (t < n && c0 + c < dv) {
                 float4 s = sum_part(x);
-                if (a.skip != nullptr) {
-                    const float4 v = load4(vb + (size_t)(t0 + t) * a.v_stride + c);
+                if (!SOLVE && a.skip != nullptr) {
+                    const float4 v = raw[x];
                     s = make_float4(fmaf(skip, v.x, s.x), fmaf(skip, v.y, s.y), fmaf(skip, v.z, s.z), fmaf(skip, v.w, s.w));
                 }
                 st4(a.o + ((size_t)(t0 + t) * a.H + h) * dv + c0 + c, s);
@@ -322,8 +329,6 @@ chunk_walk_kernel(const WalkArgs a) {
         if (group == 0) {
             load_rows(qs, qb, a.qk_stride, t_first, first_n);
             cp_commit();
-            load_p(t_first, first_n);
-            cp_commit();
         } else {
             load_rows(ks, kb, a.qk_stride, t_first, first_n);
             cp_commit();
@@ -335,30 +340,29 @@ chunk_walk_kernel(const WalkArgs a) {
         int cur = 0;
         for (int t0 = t_first; t0 < t_last; t0 += T, cur ^= 1) {
             const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
-            if (group == 0) cp_wait<1>();            // q (P may still be on its way)
-            else cp_wait<0>();                       // k
+            cp_wait<0>();                            // q, k
             const int any_odd = __syncthreads_or(odd);       // state, u and factors of this chunk are there as well
             odd = 0;
             if (group == 0) {
                 float acc[RM][RC];
                 state_product(qs, Ss + cur * DP * C, acc);
-                cp_wait<0>();
-                group_sync(0);                       // P is there, and q has been read
+                asm volatile("bar.sync 3, 256;" ::: "memory");       // P is there, the last chunk's sums and q have been read
                 if (next < t_last) load_rows(qs, qb, a.qk_stride, next, next_n);
                 cp_commit();
                 add_tokens(us + cur * T * C, rss + cur * T, any_odd, acc);
                 put_part(acc);
-                group_sync(0);                       // the slices' sums are there, and P has been read
-                if (next < t_last) load_p(next, next_n);
-                cp_commit();
-                put_outputs(t0, n);
             } else {
+                load_p(t0, n);
+                cp_commit();
                 if (next < t_last) {
                     load_rows(ks + (cur ^ 1) * T * QP, kb, a.qk_stride, next, next_n);
                     load_v(next, next_n);
                     load_factors(next, next_n);
                 }
                 cp_commit();
+                if (t0 > t_first) put_outputs(t0 - T, T);    // the last chunk's
+                cp_wait<1>();                        // P
+                asm volatile("bar.arrive 3, 256;" ::: "memory");
                 update_state(ks + cur * T * QP, u2, Ss + cur * DP * C, Ss + (cur ^ 1) * DP * C, rss[cur * T + n - 1]);
                 if (next < t_last) {                 // u2 has been read (the barrier inside)
                     put_values(us + (cur ^ 1) * T * C);
@@ -366,6 +370,9 @@ chunk_walk_kernel(const WalkArgs a) {
                 }
             }
         }
+        __syncthreads();
+        const int last = (t_last - t_first - 1) / T * T;
+        if (group == 1) put_outputs(t_first + last, t_last - t_first - last);
         last_state = Ss + cur * DP * C;
     } else {
         if (group == 0) {
