@@ -74,8 +74,9 @@ struct WalkArgs {
     const float* v_scale;          // [tokens][H] a factor on the value rows, or null
     const float* skip;             // per head: o_t += skip * (unscaled) value row, or null
     const float* p;                // [tokens][H][T]
-    const float* rs;               // [tokens][H]: e^(B_t)          (decays per head)
-    const float* ts;               // [tokens][H]: e^(B_n - B_t)
+    const float* rs;               // [tokens][H]: factor on q's products with S_0, e^(B_t) (decays per head)
+    const float* ts;               // [tokens][H]: factor on u where k takes it into the state, e^(B_n - B_t)
+    const float* eb;               // [tokens][H]: e^(B_t)
     const float* tot;              // [places][H][d]: e^(B_n)       (decays per channel: q and k come scaled)
     float* state;
     long long state_stride;
@@ -340,6 +341,7 @@ chunk_walk_kernel(const WalkArgs a) {
         int cur = 0;
         for (int t0 = t_first; t0 < t_last; t0 += T, cur ^= 1) {
             const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
+            const float total = a.eb[(size_t)(t0 + n - 1) * a.H + h];
             cp_wait<0>();                            // q, k
             const int any_odd = __syncthreads_or(odd);       // state, u and factors of this chunk are there as well
             odd = 0;
@@ -363,7 +365,7 @@ chunk_walk_kernel(const WalkArgs a) {
                 if (t0 > t_first) put_outputs(t0 - T, T);    // the last chunk's
                 cp_wait<1>();                        // P
                 asm volatile("bar.arrive 3, 256;" ::: "memory");
-                update_state(ks + cur * T * QP, u2, Ss + cur * DP * C, Ss + (cur ^ 1) * DP * C, rss[cur * T + n - 1]);
+                update_state(ks + cur * T * QP, u2, Ss + cur * DP * C, Ss + (cur ^ 1) * DP * C, total);
                 if (next < t_last) {                 // u2 has been read (the barrier inside)
                     put_values(us + (cur ^ 1) * T * C);
                     if (gt < T) rss[(cur ^ 1) * T + gt] = rfac;
@@ -390,6 +392,7 @@ chunk_walk_kernel(const WalkArgs a) {
         load_factors(t_first, first_n);
         for (int t0 = t_first; t0 < t_last; t0 += T) {
             const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
+            const float total = CHANNEL ? 0.f : a.eb[(size_t)(t0 + n - 1) * a.H + h];
             cp_wait<1>();                            // W or q (k and P may still be on their way)
             __syncthreads();                         // and the state is up to date
             float acc[RM][RC];
@@ -415,7 +418,7 @@ chunk_walk_kernel(const WalkArgs a) {
             }
             cp_commit();
             if (group == 0) {
-                update_state(ks, CHANNEL ? us : u2, Ss, Ss, CHANNEL ? 0.f : rss[n - 1]);
+                update_state(ks, CHANNEL ? us : u2, Ss, Ss, total);
                 if (next < t_last) load_rows(ks, kb, a.qk_stride, next, next_n);       // k has been read (the barrier inside)
                 cp_commit();
             } else {

@@ -672,18 +672,22 @@ def ssm_walk(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, step, y, *, 
     return y
 
 
-def delta_walk(qkv, dec, log_dec, beta, state, step, o, *, heads, kv_heads, head_dim, v_head_dim):
-    """The recurrence of :func:`delta_scan` over prompt portions: one decay per head (``log_dec``, ``dec`` None; chunks of 64
-    tokens) or per head and key channel (``dec``, ``log_dec`` None; chunks of 32)."""
+def delta_walk(qkv, a, proj, b_off: int, dt_bias, a_log, state, step, o, *, heads, kv_heads, head_dim, v_head_dim,
+               unit_eps: float, q_scale: float, per_head: bool = False):
+    """:func:`delta_prep` and :func:`delta_scan` over prompt portions, from the same inputs: chunks of 64 tokens (``per_head``) or
+    of 32.  ``qkv`` stays as it is."""
     tokens = qkv.shape[0]
-    per = 66 + head_dim + v_head_dim if dec is None else 32 + 3 * head_dim + v_head_dim
-    places = 0 if dec is None else (tokens // 32 + step.num_seqs) * heads * head_dim
+    if a.dtype != proj.dtype or a.stride(-1) != 1:
+        raise TypeError("delta_walk: the decay projection must have the projection's type and unit column stride")
+    per = 67 + head_dim + v_head_dim if per_head else 32 + 3 * head_dim + v_head_dim
+    places = 0 if per_head else (tokens // 32 + step.num_seqs) * heads * head_dim
     work = _walk_work(tokens * heads * per + places, qkv.device)
-    _check(_fn("se_delta_walk", "pppp" "pl" "pp" "pp" "iiiiiii" "p")(
-        _ptr(qkv, torch.float32, "qkv"), _ptr(dec, torch.float32, "dec"), _ptr(log_dec, torch.float32, "log_dec"),
-        _ptr(beta, torch.float32, "beta"), _ptr(state, torch.float32, "state"), state.stride(0), _ptr(step.cu_q),
-        _ptr(step.seq_rows), _ptr(o, torch.float32, "o"), work.data_ptr(), tokens, step.num_seqs, heads, kv_heads, head_dim,
-        v_head_dim, sm_count(qkv.device), _stream()), "delta_walk")
+    _check(_fn("se_delta_walk", "ppipii" "pp" "pl" "pp" "pp" "iiiiii" "ff" "iii" "p")(
+        _ptr(qkv, torch.float32, "qkv"), a.data_ptr(), a.stride(0), _rows_ptr(proj, "proj"), proj.stride(0), int(b_off),
+        _ptr(dt_bias, torch.float32, "dt_bias"), _ptr(a_log, torch.float32, "a_log"), _ptr(state, torch.float32, "state"),
+        state.stride(0), _ptr(step.cu_q), _ptr(step.seq_rows), _ptr(o, torch.float32, "o"), work.data_ptr(), tokens, step.num_seqs,
+        heads, kv_heads, head_dim, v_head_dim, float(unit_eps), float(q_scale), int(per_head), sm_count(qkv.device),
+        dtype_code(proj.dtype), _stream()), "delta_walk")
     return o
 
 

@@ -693,8 +693,7 @@ static inline void tile_plan(int rows, int columns, int units, int* nsplit, int*
 // unit_eps), q also times q_scale; dec = exp(-exp(A_log[h]) * softplus(a + dt_bias)); beta =
 // sigmoid(b).  `a` (rows a_pitch apart) is the decay projection: [H*d], one decay per head and key
 // channel, or, with `per_head`, [H], one decay per head (dt_bias likewise), which is written to all
-// of the head's channels (dec may be null then, where only the logarithms are wanted).  `proj` column b_off + h is the
-// beta projection.
+// of the head's channels.  `proj` column b_off + h is the beta projection.
 template <typename T>
 __global__ void delta_prep_kernel(float* qkv, int width, const T* a, int a_pitch, const T* proj, int pitch, int b_off,
                                   const float* __restrict__ dt_bias, const float* __restrict__ a_log,
@@ -710,7 +709,7 @@ __global__ void delta_prep_kernel(float* qkv, int width, const T* a, int a_pitch
         const float f = (hh < G ? q_scale : 1.f) / sqrtf(ss + unit_eps);
         for (int i = lane; i < d; i += 32) v[i] *= f;
     }
-    for (int i = threadIdx.x; dec != nullptr && i < H * d; i += blockDim.x) {
+    for (int i = threadIdx.x; i < H * d; i += blockDim.x) {
         const int h = i / d, j = per_head ? h : i;
         const float rate = expf(a_log[h]);
         dec[(size_t)t * H * d + i] = expf(-rate * softplus_f(to_float(a[(size_t)t * a_pitch + j]) + dt_bias[j]));
@@ -942,7 +941,7 @@ extern "C" int se_delta_prep(float* qkv, const void* a, int a_pitch, const void*
                              cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0 || a_pitch < (per_head ? H : H * d)) return SE_ERR_ARGUMENT;
-    if ((log_dec != nullptr && !per_head) || (dec == nullptr && log_dec == nullptr)) return SE_ERR_ARGUMENT;
+    if (log_dec != nullptr && !per_head) return SE_ERR_ARGUMENT;
     SE_DISPATCH_DTYPE(dtype, T,
         se::delta_prep_kernel<T><<<tokens, 256, 0, stream>>>(qkv, 2 * G * d + H * dv, (const T*)a, a_pitch, (const T*)proj, pitch,
                                                             b_off, dt_bias, a_log, dec, beta, H, G, d, unit_eps, q_scale,

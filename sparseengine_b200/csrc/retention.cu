@@ -671,7 +671,7 @@ static int launch_retention_walk(const float* q32, const float* k32, const void*
         if (rc != 0) return rc;
         WalkArgs a = {};
         a.q = q32; a.k = k32; a.qk_stride = heads * d; a.rep = 1; a.v_stride = proj_stride; a.silu = silu;
-        a.p = p; a.rs = rs; a.ts = ts; a.state = state; a.state_stride = state_stride; a.s_row = dv; a.s_col = 1; a.o = o;
+        a.p = p; a.rs = rs; a.ts = ts; a.eb = rs; a.state = state; a.state_stride = state_stride; a.s_row = dv; a.s_col = 1; a.o = o;
         a.cu_q = cu_q; a.seq_rows = seq_rows; a.H = heads; a.d = d; a.dv = dv;
         const int cols = walk_columns(entries, heads, dv, sms);
         SE_DISPATCH_DTYPE(dtype, T_, {

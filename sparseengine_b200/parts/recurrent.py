@@ -155,29 +155,27 @@ class GatedDeltaMixer(Mixer):
         a, gate = proj[:, self.a_off:self.a_off + self.a_cols], proj[:, self.g_off:self.g_off + self.g_cols]
         if not self.per_head:       # through the low ranks
             a, gate = linear(a, self.a2), linear(gate, self.g2)
-        # Steps with prompt portions run the recurrence in chunks, prepared side by side and walked (csrc/chunk_walk.cuh); so do
-        # not: steps of single tokens and short pieces, and head sizes the chunks do not take.
+        # Steps with prompt portions run the recurrence in chunks, prepared side by side and walked (csrc/chunk_walk.cuh); others
+        # (single tokens, short pieces, head sizes the chunks do not take) prepare q, k, decays and beta, then walk the tokens.
         sizes = dict(heads=s.num_heads, kv_heads=s.num_kv_heads, head_dim=s.head_dim, v_head_dim=s.v_head_dim)
-        long = takes_chunks(self, step, s.num_heads, s.v_head_dim, dev)
-        walk = long and ops.chunk_walk_supported(s.head_dim, s.v_head_dim)
-        # One decay per head and a head size beyond that: chunks of 64 tokens in one kernel, while its (entry, head, 32
-        # columns) blocks do not fill the device (it does about twice the multiply-adds of the walk token by token).
-        chunked = (long and not walk and self.per_head and s.head_dim <= ops.LIMITS["delta_chunk_max_head_dim"]
-                   and step.num_seqs * s.num_heads * (-(-s.v_head_dim // 32)) <= ops.sm_count(dev))
-        log_dec = torch.empty(tokens, s.num_heads, dtype=torch.float32, device=dev) if self.per_head and long else None
-        dec = None
-        if not (self.per_head and (walk or chunked)):
-            dec = torch.empty(tokens, s.num_heads * s.head_dim, dtype=torch.float32, device=dev)
-        beta = torch.empty(tokens, s.num_heads, dtype=torch.float32, device=dev)
-        ops.delta_prep(qkv, a, proj, self.b_off, self.dt_bias, self.a_log, dec, beta, **sizes, unit_eps=s.unit_eps,
-                       q_scale=s.head_dim ** -0.5, per_head=self.per_head, log_dec=log_dec)
+        inputs = dict(unit_eps=s.unit_eps, q_scale=s.head_dim ** -0.5, per_head=self.per_head)
         o = torch.empty(tokens, self.vv, dtype=torch.float32, device=dev)
-        if walk:
-            ops.delta_walk(qkv, dec, log_dec if self.per_head else None, beta, slot.state, step, o, **sizes)
-        elif chunked:
-            ops.delta_chunk(qkv, log_dec, beta, slot.state, step, o, **sizes)
+        long = takes_chunks(self, step, s.num_heads, s.v_head_dim, dev)
+        if long and ops.chunk_walk_supported(s.head_dim, s.v_head_dim):
+            ops.delta_walk(qkv, a, proj, self.b_off, self.dt_bias, self.a_log, slot.state, step, o, **sizes, **inputs)
         else:
-            ops.delta_scan(qkv, dec, beta, slot.state, step, o, **sizes)
+            # One decay per head: chunks of 64 tokens in one kernel, while its (entry, head, 32 columns) blocks do not fill the
+            # device (it does about twice the multiply-adds of the walk token by token).
+            chunked = (long and self.per_head and s.head_dim <= ops.LIMITS["delta_chunk_max_head_dim"]
+                       and step.num_seqs * s.num_heads * (-(-s.v_head_dim // 32)) <= ops.sm_count(dev))
+            log_dec = torch.empty(tokens, s.num_heads, dtype=torch.float32, device=dev) if chunked else None
+            dec = torch.empty(tokens, s.num_heads * s.head_dim, dtype=torch.float32, device=dev)
+            beta = torch.empty(tokens, s.num_heads, dtype=torch.float32, device=dev)
+            ops.delta_prep(qkv, a, proj, self.b_off, self.dt_bias, self.a_log, dec, beta, **sizes, **inputs, log_dec=log_dec)
+            if chunked:
+                ops.delta_chunk(qkv, log_dec, beta, slot.state, step, o, **sizes)
+            else:
+                ops.delta_scan(qkv, dec, beta, slot.state, step, o, **sizes)
         out = torch.empty(tokens, self.vv, dtype=x.dtype, device=dev)
         ops.delta_out(o, gate, self.norm_w, out, heads=s.num_heads, v_head_dim=s.v_head_dim, eps=s.norm_eps,
                       silu=s.gate_activation == "silu")

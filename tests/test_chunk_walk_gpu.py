@@ -59,7 +59,7 @@ def test_chunks_against_the_walk(kind, d, dv, heads, kv_heads, decay):
     first = state.double().clone()
     logs = -(torch.rand(T, heads, d, generator=g, device=DEV) * (30.0 if decay == "fast" else 0.2))
     o = torch.full((T, heads, dv), float("nan"), device=DEV)
-    rep, beta = heads // kv_heads, torch.rand(T, heads, generator=g, device=DEV)
+    rep = heads // kv_heads
     sizes = dict(heads=heads, head_dim=d, v_head_dim=dv)
     column_major = kind != "retention"          # [head][column][row], retention [head][row][column]
     skip = None
@@ -68,8 +68,7 @@ def test_chunks_against_the_walk(kind, d, dv, heads, kv_heads, decay):
         decays = torch.exp(logs[0, :, 0])
         ops.retention_chunk(q.view(T, -1), k.view(T, -1), v, 4, decays, state, step, o.view(T, -1), silu=True, **sizes)
         v = torch.nn.functional.silu(v[:, 4:4 + heads * dv].double()).view(T, heads, dv)
-        keep = decays.double().view(1, heads, 1).expand(T, -1, -1)
-        beta = None
+        keep, beta = decays.double().view(1, heads, 1).expand(T, -1, -1), None
     elif kind == "state space":
         width = heads * dv + 2 * kv_heads * d
         xbc, proj = rnd(T, width), rnd(T, heads + 3)
@@ -81,17 +80,18 @@ def test_chunks_against_the_walk(kind, d, dv, heads, kv_heads, decay):
         q = xbc[:, heads * dv + kv_heads * d:].view(T, kv_heads, d).repeat_interleave(rep, 1)
         v, keep, beta = x * dt[..., None], torch.exp(-torch.exp(a_log.double()) * dt)[..., None], None
     else:
-        qk = torch.nn.functional.normalize(rnd(T, 2 * kv_heads, d), dim=-1)
-        qkv = torch.cat([qk.reshape(T, -1), rnd(T, heads * dv)], 1)
         per_head = kind == "delta, per head"
-        if per_head:
-            logs = logs[..., 0].contiguous()
-        dec = None if per_head else torch.exp(logs).view(T, -1)
-        ops.delta_walk(qkv, dec, logs if per_head else None, beta, state, step, o.view(T, -1), heads=heads, kv_heads=kv_heads, head_dim=d, v_head_dim=dv)
-        q, k = (t.repeat_interleave(rep, 1) for t in (qk[:, :kv_heads], qk[:, kv_heads:]))
+        qkv, proj, cols = rnd(T, 2 * kv_heads * d + heads * dv), rnd(T, heads + 4), heads * (1 if per_head else d)
+        a, bias = rnd(T, cols + (-cols) % 4), rnd(cols) - 1.0
+        a_log = torch.log(torch.rand(heads, generator=g, device=DEV) * (20 if decay == "fast" else 0.5) + 0.05)
+        ops.delta_walk(qkv, a, proj, 2, bias, a_log, state, step, o.view(T, -1), heads=heads, kv_heads=kv_heads, head_dim=d, v_head_dim=dv,
+                       unit_eps=1e-6, q_scale=d ** -0.5, per_head=per_head)
+        qk = qkv[:, :2 * kv_heads * d].double().view(T, 2 * kv_heads, d)
+        qk = qk / torch.sqrt((qk * qk).sum(-1, keepdim=True) + 1e-6)
+        q, k = (t.repeat_interleave(rep, 1) for t in (qk[:, :kv_heads] * d ** -0.5, qk[:, kv_heads:]))
         v = qkv[:, 2 * kv_heads * d:].double().view(T, heads, dv)
-        keep = torch.exp(logs.double())[..., None] if per_head else dec.double().view(T, heads, d)
-        beta = beta.double()
+        steps = torch.nn.functional.softplus(a[:, :cols].double() + bias.double()).view(T, heads, -1)
+        keep, beta = torch.exp(-torch.exp(a_log.double())[:, None] * steps), torch.sigmoid(proj[:, 2:2 + heads].double())
     assert bool(torch.isfinite(o).all())
     for e, n in enumerate(LENS):
         a, b, row = step.cu[e], step.cu[e + 1], step.rows[e]
@@ -117,14 +117,15 @@ def test_later_tokens_do_not_touch_earlier_ones(kind):
     H, d, T = 2, 64, 70
     step = SimpleNamespace(cu_q=torch.tensor([0, T], dtype=torch.int32, device=DEV), seq_rows=torch.zeros(1, dtype=torch.int32, device=DEV), num_seqs=1)
     g = torch.Generator(device=DEV).manual_seed(1)
-    qkv = torch.randn(T, 3 * H * d, generator=g, device=DEV) * 0.1
-    logs, beta = -torch.rand(T, H, generator=g, device=DEV), torch.rand(T, H, generator=g, device=DEV)
-    dec = torch.rand(T, H * d, generator=g, device=DEV) if kind == "per channel" else None
+    qkv, proj = torch.randn(T, 3 * H * d, generator=g, device=DEV), torch.randn(T, H, generator=g, device=DEV)
+    cols = H * (1 if kind == "per head" else d)
+    decay, bias, a_log = torch.randn(T, cols, generator=g, device=DEV), torch.zeros(cols, device=DEV), torch.zeros(H, device=DEV)
     outs = []
     for bad in (False, True):
         if bad:
             qkv[41, 2 * H * d + 3] = float("inf")
         o = torch.empty(T, H * d, device=DEV)
-        ops.delta_walk(qkv, dec, logs if dec is None else None, beta, torch.zeros(1, H * d * d, device=DEV), step, o, heads=H, kv_heads=H, head_dim=d, v_head_dim=d)
+        ops.delta_walk(qkv, decay, proj, 0, bias, a_log, torch.zeros(1, H * d * d, device=DEV), step, o, heads=H, kv_heads=H, head_dim=d, v_head_dim=d,
+                       unit_eps=1e-6, q_scale=0.1, per_head=kind == "per head")
         outs.append(o)
     assert torch.equal(outs[0][:41], outs[1][:41]) and not bool(torch.isfinite(outs[1][41:]).all())
