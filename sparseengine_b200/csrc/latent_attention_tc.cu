@@ -1,0 +1,320 @@
+// Latent attention over prompt portions on 5th-generation tensor cores (bfloat16).
+//
+// The absorbed form has one key/value head: a cached row of rank + rot elements is the key of every head, its first `rank`
+// elements the value.  A query row is one (token, head) pair, token-major, so 128 rows span a few tokens and all their heads.
+// One CTA per (batch entry, 256 query rows): two query tiles of 128 rows share every 64-key tile that is loaded, and a tile of
+// cached rows in shared memory serves both products: S = Q K^T reads it K-major (64 dims per 128-byte row), O += P V reads the
+// first rank / 64 of the same blocks MN-major.  S, P (over its scores) and O are in tensor memory: O of two tiles takes 2 rank
+// columns, which leaves two S buffers per tile up to a rank of 128 and one at 192 (then the two tiles take turns: one's
+// products run while the other's softmax does).
+//
+// The arrangement of warps, barriers and the softmax are those of attention_prefill_tc.cu: two loader warps, one MMA-issuing
+// warp and four softmax warps per query tile, every wait bounded and reported through the error word.
+//
+// What bounds it: at a row of 256 and a rank of 192 a key tile takes a query tile 896 cycles of the tensor pipe
+// (128 x 64 x (256 + 192) multiply-adds) against 512 of the exponential unit.  The mma.sync kernel (latent_attention.cu), which
+// stays for steps of few rows (it splits them along the keys) and for other sizes, ends at a third of the tensor rate.
+#include "common.cuh"
+#include "fa_util.cuh"
+#include "mma_util.cuh"
+
+namespace se {
+namespace lat_tc {
+
+using namespace se::fa;
+using se::mma::cp_async16;
+using se::mma::cp_async_commit;
+using se::mma::smem_u32;
+
+constexpr int kRows = 128, kKeys = 64, kTiles = 2;
+constexpr int kMaxStages = 5;
+constexpr int kLoaderWarp2 = 2 + 4 * kTiles, kMmaWarp2 = kLoaderWarp2 + 1;
+constexpr int kThreads = 32 * (kMmaWarp2 + 1);
+constexpr int kKeyBlock = kKeys * 128;               // [64 keys][64 dims]: rows of 128 bytes
+constexpr int kRowBlock = kRows * 128;               // [128 query rows][64 dims]
+
+struct Bars {
+    uint64_t kv_full[kMaxStages], kv_empty[kMaxStages];
+    uint64_t s_full[kTiles][2], s_empty[kTiles][2];
+    uint64_t p_full[kTiles][2], p_empty[kTiles];
+    uint64_t o_done[kTiles];
+};
+
+// db, rb: blocks of 64 dims of a row and of its latent part; buffers: S buffers per query tile; stages: key tiles in flight
+__global__ void __launch_bounds__(kThreads, 1)
+latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_bfloat16* __restrict__ cache,
+                           const int* __restrict__ table, int table_stride, const int* __restrict__ seq_rows,
+                           const int* __restrict__ cu_q, const int* __restrict__ kv_len, const float* __restrict__ sink,
+                           __nv_bfloat16* __restrict__ out, int heads, int db, int rb, int buffers, int stages, int page_size,
+                           float scale_log2, int window, int num_pages, int* error) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int q_bytes = db * kRowBlock, stage_bytes = db * kKeyBlock, D = db * 64, rank = rb * 64;
+    uint8_t* q_s = smem;                               // [2 tiles][db][128 rows][128 B]
+    uint8_t* kv_s = q_s + kTiles * q_bytes;            // [stages][db][64 keys][128 B]
+    __shared__ __align__(8) Bars bars;
+    __shared__ uint32_t tmem_base_s;
+    __shared__ volatile int abort_s;
+
+    const int entry = blockIdx.y;
+    const int tok0 = cu_q[entry], q_len = cu_q[entry + 1] - tok0;
+    const long long total_rows = (long long)q_len * heads;
+    const long long row_base = (long long)(gridDim.x - 1 - blockIdx.x) * (kTiles * kRows);      // the tiles with the most keys start first
+    if (row_base >= total_rows) return;
+    const int kv_end = kv_len[entry], q_start = kv_end - q_len;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_rows = (int)min((long long)kTiles * kRows, total_rows - row_base);
+    const int first_pos = q_start + (int)(row_base / heads), max_pos = q_start + (int)((row_base + n_rows - 1) / heads);
+    const int k_lo = first_visible(first_pos, window);
+    const int k_begin = (k_lo / kKeys) * kKeys, k_end = max_pos + 1;
+    const int num_tiles = (k_end - k_begin + kKeys - 1) / kKeys;
+
+    auto bar = [&](uint64_t* b) { return smem_u32(b); };
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; ++s) { mbar_init(bar(&bars.kv_full[s]), 32); mbar_init(bar(&bars.kv_empty[s]), kTiles); }
+        for (int x = 0; x < kTiles; ++x) {
+            for (int b = 0; b < 2; ++b) {
+                mbar_init(bar(&bars.s_full[x][b]), 1);
+                mbar_init(bar(&bars.s_empty[x][b]), 4);
+                mbar_init(bar(&bars.p_full[x][b]), 4);
+            }
+            mbar_init(bar(&bars.p_empty[x]), 1);
+            mbar_init(bar(&bars.o_done[x]), 1);
+        }
+        abort_s = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // query rows lie one behind the other; rows beyond the portion's are zeros
+    const __nv_bfloat16* q_rows = qfull + ((size_t)tok0 * heads + (size_t)row_base) * D;
+    for (int i = threadIdx.x; i < kTiles * kRows * db * 8; i += kThreads) {
+        const int r = i / (db * 8), c = i - r * (db * 8);
+        const bool ok = r < n_rows;
+        cp_async16(smem_u32(q_s) + (r >> 7) * q_bytes + (c >> 3) * kRowBlock + sw128(r & 127, c & 7), q_rows + (size_t)(ok ? r : 0) * D + c * 8, ok);
+    }
+    cp_async_commit();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_base_s;
+    // one S buffer: O of tile x in columns 256 x .., its S behind; two: O in 128 x .., the S buffers in 256 + 128 x + 64 b ..
+    auto tmem_o = [&](int x) { return tmem + (uint32_t)((buffers == 1 ? 256 : 128) * x); };
+    auto tmem_s = [&](int x, int b) { return tmem + (uint32_t)(buffers == 1 ? 256 * x + 192 : 256 + 128 * x + 64 * b); };
+
+    if (warp == 0 || warp == kLoaderWarp2) {
+        // ---- loaders: alternate key tiles, as far ahead as stages are free ----------------------
+        const int* row_table = table + (size_t)seq_rows[entry] * table_stride;
+        const int lanes = db > 2 ? 32 : db > 1 ? 16 : 8, c = lane & (lanes - 1), per = 32 / lanes;      // lanes per row, rows per pass
+        auto issue = [&](int tile) {
+            const uint32_t st = smem_u32(kv_s) + (uint32_t)((tile % stages) * stage_bytes);
+            const int base = k_begin + tile * kKeys;
+            // keys outside [k_lo, k_end) are zero-filled, never read (a page the window has left may belong to another
+            // request by now); address 0 marks an entry that names no page of the pool
+            unsigned long long src_row[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int j = min(max(base + 32 * h + lane, k_lo), k_end - 1);
+                const int page = row_table[j / page_size];
+                src_row[h] = page_in_pool(page, num_pages, error, 29)
+                                 ? (unsigned long long)(cache + ((size_t)page * page_size + j % page_size) * D) : 0ull;
+            }
+#pragma unroll 4
+            for (int k = 0; k < kKeys; k += per) {
+                const int r = k + lane / lanes;
+                const unsigned long long a = __shfl_sync(0xffffffffu, src_row[0], r & 31);
+                const unsigned long long b = __shfl_sync(0xffffffffu, src_row[1], r & 31);
+                const unsigned long long row_addr = r < 32 ? a : b;
+                const bool ok = base + r < k_end && base + r >= k_lo && row_addr != 0ull;
+                if (c < db * 8)
+                    cp_async16(st + (uint32_t)((c >> 3) * kKeyBlock) + sw128(r, c & 7),
+                               reinterpret_cast<const __nv_bfloat16*>(ok ? row_addr : (unsigned long long)cache) + c * 8, ok);
+            }
+        };
+        bool ok = true;
+        for (int tile = warp == 0 ? 0 : 1; tile < num_tiles && ok; tile += 2) {
+            if (tile >= stages) ok = mbar_wait(bar(&bars.kv_empty[tile % stages]), ((tile / stages) - 1) & 1, &abort_s);
+            if (!ok) break;
+            issue(tile);
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar(&bars.kv_full[tile % stages])) : "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (!ok) { abort_s = 1; if (lane == 0) atomicCAS(error, 0, 14); }
+    } else if (warp == 1 || warp == kMmaWarp2) {
+        // ---- MMA issuers: one lane per query tile -------------------------------------------------
+        // With two S buffers S(j) goes ahead of P V of tile j - 1; with one, P V of tile j ahead of S(j + 1), which
+        // overwrites P (MMAs of one thread run in their order).
+        if (lane == 0) {
+            const int x = warp == 1 ? 0 : 1;
+            const uint32_t id_s = idesc(kKeys, 0), id_o = idesc(rank, 1);
+            bool ok = true;
+            auto issue_pv = [&](int i) {
+                const int b = i % buffers;
+                if (!mbar_wait(bar(&bars.p_full[x][b]), (i / buffers) & 1, &abort_s)) { ok = false; return; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t va = smem_u32(kv_s) + (uint32_t)((i % stages) * stage_bytes), pa = tmem_s(x, b);
+#pragma unroll
+                for (int kk = 0; kk < kKeys / 16; ++kk)
+                    umma_ts(tmem_o(x), pa + (uint32_t)(kk * 8), desc_mnmajor(va + kk * 2048, kKeyBlock), id_o, (i > 0 || kk > 0) ? 1u : 0u);
+                umma_commit(bar(&bars.p_empty[x]));
+                umma_commit(bar(&bars.kv_empty[i % stages]));
+            };
+            for (int j = 0; j < num_tiles && ok; ++j) {
+                const int b = j % buffers;
+                if (!mbar_wait(bar(&bars.kv_full[j % stages]), (j / stages) & 1, &abort_s)) { ok = false; break; }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the copies were generic-proxy writes
+                if (j >= buffers && !mbar_wait(bar(&bars.s_empty[x][b]), ((j / buffers) - 1) & 1, &abort_s)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t ka = smem_u32(kv_s) + (uint32_t)((j % stages) * stage_bytes), qa = smem_u32(q_s) + (uint32_t)(x * q_bytes);
+                for (int kb = 0; kb < db; ++kb)
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        umma(tmem_s(x, b), desc_kmajor(qa + kb * kRowBlock) + (uint64_t)(kk * 2), desc_kmajor(ka + kb * kKeyBlock) + (uint64_t)(kk * 2),
+                             id_s, (kb > 0 || kk > 0) ? 1u : 0u);
+                umma_commit(bar(&bars.s_full[x][b]));
+                if (j >= buffers - 1) issue_pv(j - (buffers - 1));
+            }
+            if (ok && buffers == 2) issue_pv(num_tiles - 1);
+            if (ok) umma_commit(bar(&bars.o_done[x]));
+            if (!ok) { abort_s = 1; atomicCAS(error, 0, 15); }
+        }
+    } else if (warp < 2 + 4 * kTiles) {
+        // ---- softmax and epilogue: four warps per query tile, one thread per row --------------------
+        const int x = (warp - 2) >> 2, quarter = warp & 3;
+        const int r = x * kRows + quarter * 32 + lane;     // row of the CTA
+        const bool valid = r < n_rows;
+        const long long row = row_base + (valid ? r : n_rows - 1);
+        const int pos = q_start + (int)(row / heads), lo = first_visible(pos, window);
+        const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+        float m_ref = -INFINITY, l = 0.f;                  // reference maximum (log2 units), running sum
+        bool ok = true;
+        for (int j = 0; j < num_tiles && ok; ++j) {
+            const int b = j % buffers;
+            if (!mbar_wait(bar(&bars.s_full[x][b]), (j / buffers) & 1, &abort_s)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint32_t sv[64];
+            tmem_ld32(tmem_s(x, b) + lane_addr, sv);
+            tmem_ld32(tmem_s(x, b) + 32 + lane_addr, sv + 32);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(&bars.s_empty[x][b]));
+            const int key0 = k_begin + j * kKeys;
+            // a tile that every row of the warp sees in full needs no mask (rows ascend with the lane)
+            if (!(key0 + kKeys - 1 <= __shfl_sync(0xffffffffu, pos, 0) && key0 >= __shfl_sync(0xffffffffu, lo, 31))) {
+#pragma unroll
+                for (int c = 0; c < 64; ++c)
+                    if (key0 + c > pos || key0 + c < lo) sv[c] = 0xff800000u;      // -inf
+            }
+            float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int c = 0; c < 64; ++c) m4[c & 3] = fmaxf(m4[c & 3], __uint_as_float(sv[c]));
+            const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * scale_log2;       // scale > 0
+            // the reference maximum moves on the first visible keys or a large jump only
+            float factor = 1.f;
+            bool need = false;
+            if (mx > m_ref + kRescaleThreshold || (m_ref == -INFINITY && mx != -INFINITY)) {
+                factor = m_ref == -INFINITY ? 0.f : exp2f(m_ref - mx);
+                need = m_ref != -INFINITY;
+                m_ref = mx;
+                l *= factor;
+            }
+            if (__any_sync(0xffffffffu, need)) {           // O at rest: P V of the tile before has finished
+                if (j >= 1 && !mbar_wait(bar(&bars.p_empty[x]), (j - 1) & 1, &abort_s)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+                for (int c0 = 0; c0 < rank; c0 += 32) {
+                    uint32_t ov[32];
+                    tmem_ld32(tmem_o(x) + c0 + lane_addr, ov);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) ov[c] = __float_as_uint(__uint_as_float(ov[c]) * (need ? factor : 1.f));
+                    tmem_st32(tmem_o(x) + c0 + lane_addr, ov);
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            }
+            const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref;
+            float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+            uint32_t packed[32];
+#pragma unroll
+            for (int c = 0; c < 32; ++c) {
+                const float p0 = ex2(fmaf(__uint_as_float(sv[2 * c]), scale_log2, neg_m));
+                const float p1 = ex2(fmaf(__uint_as_float(sv[2 * c + 1]), scale_log2, neg_m));
+                sum4[c & 3] += p0 + p1;
+                packed[c] = se::mma::pack_bf16(p0, p1);
+            }
+            tmem_st32(tmem_s(x, b) + lane_addr, packed);   // P over the row's own scores
+            l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(&bars.p_full[x][b]));
+        }
+        if (ok && mbar_wait(bar(&bars.o_done[x]), 0, &abort_s)) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (sink != nullptr) l += exp2f(fmaf(sink[(int)(row % heads)], 1.4426950408889634f, -m_ref));
+            const float inv = 1.f / l;
+            __nv_bfloat16* dst = out + ((size_t)tok0 * heads + (size_t)row) * rank;
+#pragma unroll 1
+            for (int c0 = 0; c0 < rank; c0 += 32) {
+                uint32_t ov[32];
+                tmem_ld32(tmem_o(x) + c0 + lane_addr, ov);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (valid)
+#pragma unroll
+                    for (int c = 0; c < 32; c += 8) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            w[i] = se::mma::pack_bf16(__uint_as_float(ov[c + 2 * i]) * inv, __uint_as_float(ov[c + 2 * i + 1]) * inv);
+                        *reinterpret_cast<uint4*>(dst + c0 + c) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+            }
+        } else {
+            abort_s = 1;
+            atomicCAS(error, 0, 16);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+}  // namespace lat_tc
+}  // namespace se
+
+// A cached row of up to 256 and its latent part of up to 192, both in blocks of 64 (tensor memory holds 2 rank + 128 columns).
+extern "C" int se_latent_attention_tc_supported(int rank, int rot) {
+    return rank > 0 && rank <= 192 && rank % 64 == 0 && rot >= 0 && rot % 64 == 0 && rank + rot <= 256;
+}
+
+// Arguments as se_latent_attention_tiled's (which splits the keys of steps of few rows).
+extern "C" int se_latent_attention_tc(const void* qfull, const void* cache, const int* table, int table_stride, const int* seq_rows,
+                                      const int* cu_q, const int* kv_len, const float* sink, void* out, int entries, int max_q_len,
+                                      int heads, int rank, int rot, int page_size, float scale, int window, int num_pages, int* error,
+                                      cudaStream_t stream) {
+    using namespace se::lat_tc;
+    if (entries <= 0 || max_q_len <= 0) return 0;
+    if (!se_latent_attention_tc_supported(rank, rot) || heads <= 0 || entries > 65535) return SE_ERR_UNSUPPORTED;
+    if (!(scale > 0.f) || page_size <= 0 || window < 0) return SE_ERR_ARGUMENT;
+    if ((reinterpret_cast<uintptr_t>(qfull) | reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) & 15) return SE_ERR_UNSUPPORTED;
+    const long long row_tiles = ((long long)max_q_len * heads + kTiles * kRows - 1) / (kTiles * kRows);
+    if (row_tiles > 0x7fffffffLL) return SE_ERR_UNSUPPORTED;
+    const int db = (rank + rot) / 64, rb = rank / 64, buffers = rank > 128 ? 1 : 2;
+    const int room = 226 * 1024 - kTiles * db * kRowBlock;
+    const int fit = room / (db * kKeyBlock), stages = fit < kMaxStages ? fit : kMaxStages;
+    const size_t smem = (size_t)kTiles * db * kRowBlock + (size_t)stages * db * kKeyBlock + 1024;
+    const cudaError_t e = cudaFuncSetAttribute(latent_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    latent_attention_tc_kernel<<<dim3((unsigned)row_tiles, entries), kThreads, smem, stream>>>(
+        (const __nv_bfloat16*)qfull, (const __nv_bfloat16*)cache, table, table_stride, seq_rows, cu_q, kv_len, sink,
+        (__nv_bfloat16*)out, heads, db, rb, buffers, stages, page_size, scale * 1.4426950408889634f, window, num_pages, error);
+    return (int)cudaGetLastError();
+}

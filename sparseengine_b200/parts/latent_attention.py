@@ -135,6 +135,11 @@ class LatentAttention(Mixer):
 
     def attend_tiled(self, qfull, out_lat, step, slot):
         s = self.spec
+        if ops.latent_takes_tc(step.num_seqs, step.max_q_len, s.num_heads, s.kv_rank, s.rot_dim, ops.sm_count(qfull.device)):
+            ops.latent_attention_tc(qfull, slot.kv, slot.table, step.seq_rows, step.cu_q, step.kv_len, self.sink, out_lat,
+                                    entries=step.num_seqs, max_q_len=step.max_q_len, heads=s.num_heads, rank=s.kv_rank, rot=s.rot_dim,
+                                    page_size=slot.page_size, scale=s.scale, window=s.window)
+            return
         most = step.max_kv_len if s.window is None else min(step.max_kv_len, s.window + step.max_q_len - 1)
         ops.latent_attention_tiled(qfull, slot.kv, slot.table, step.seq_rows, step.cu_q, step.kv_len, self.sink, out_lat,
                                    entries=step.num_seqs, max_q_len=step.max_q_len, heads=s.num_heads, rank=s.kv_rank,
