@@ -28,6 +28,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
     return false;
 }
+// One lane of a converged warp.  What an MMA's issue needs lies in uniform registers; code under a branch that the compiler
+// takes for divergent (lane == 0) moves every operand there for every MMA, about 100 cycles each.  So the issuing warp runs
+// as a whole through warp-uniform loops and only the MMAs are one lane's.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 // rows of 128 bytes, 16-byte chunks XOR-swizzled by (row % 8): the canonical 128-byte-swizzle image
 __device__ __forceinline__ uint32_t sw128(int row, int chunk) { return (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4)); }
 

@@ -8,8 +8,8 @@
 // columns, which leaves two S buffers per tile up to a rank of 128 and one at 192 (then the two tiles take turns: one's
 // products run while the other's softmax does).
 //
-// The arrangement of warps, barriers and the softmax are those of attention_prefill_tc.cu: two loader warps, one MMA-issuing
-// warp and four softmax warps per query tile, every wait bounded and reported through the error word.
+// The arrangement of barriers and the softmax are those of attention_prefill_tc.cu: four softmax warps per query tile, three
+// loader warps, one MMA-issuing warp, every wait bounded and reported through the error word.
 //
 // What bounds it: at a row of 256 and a rank of 192 a key tile takes a query tile 896 cycles of the tensor pipe
 // (128 x 64 x (256 + 192) multiply-adds) against 512 of the exponential unit.  The mma.sync kernel (latent_attention.cu), which
@@ -28,8 +28,9 @@ using se::mma::smem_u32;
 
 constexpr int kRows = 128, kKeys = 64, kTiles = 2;
 constexpr int kMaxStages = 5;
-constexpr int kLoaderWarp2 = 2 + 4 * kTiles, kMmaWarp2 = kLoaderWarp2 + 1;
-constexpr int kThreads = 32 * (kMmaWarp2 + 1);
+constexpr int kLoaders = 3;                          // warp 0 and those behind the softmax warps
+constexpr int kLoaderWarp2 = 2 + 4 * kTiles;
+constexpr int kThreads = 32 * (kLoaderWarp2 + kLoaders - 1);
 constexpr int kKeyBlock = kKeys * 128;               // [64 keys][64 dims]: rows of 128 bytes
 constexpr int kRowBlock = kRows * 128;               // [128 query rows][64 dims]
 
@@ -37,7 +38,7 @@ struct Bars {
     uint64_t kv_full[kMaxStages], kv_empty[kMaxStages];
     uint64_t s_full[kTiles][2], s_empty[kTiles][2];
     uint64_t p_full[kTiles][2], p_empty[kTiles];
-    uint64_t o_done[kTiles];
+    uint64_t o_done[kTiles], q_full[kTiles];
 };
 
 // db, rb: blocks of 64 dims of a row and of its latent part; buffers: S buffers per query tile; stages: key tiles in flight
@@ -55,6 +56,7 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_b
     __shared__ __align__(8) Bars bars;
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_s;
+    __shared__ unsigned long long row_list[kLoaders][kKeys];  // per loader warp: the addresses of a tile's rows
 
     const int entry = blockIdx.y;
     const int tok0 = cu_q[entry], q_len = cu_q[entry + 1] - tok0;
@@ -62,7 +64,7 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_b
     const long long row_base = (long long)(gridDim.x - 1 - blockIdx.x) * (kTiles * kRows);      // the tiles with the most keys start first
     if (row_base >= total_rows) return;
     const int kv_end = kv_len[entry], q_start = kv_end - q_len;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int n_rows = (int)min((long long)kTiles * kRows, total_rows - row_base);
     const int first_pos = q_start + (int)(row_base / heads), max_pos = q_start + (int)((row_base + n_rows - 1) / heads);
     const int k_lo = first_visible(first_pos, window);
@@ -80,6 +82,7 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_b
             }
             mbar_init(bar(&bars.p_empty[x]), 1);
             mbar_init(bar(&bars.o_done[x]), 1);
+            mbar_init(bar(&bars.q_full[x]), 128);            // every thread of the tile's softmax warps
         }
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -88,16 +91,6 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_b
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // query rows lie one behind the other; rows beyond the portion's are zeros
-    const __nv_bfloat16* q_rows = qfull + ((size_t)tok0 * heads + (size_t)row_base) * D;
-    for (int i = threadIdx.x; i < kTiles * kRows * db * 8; i += kThreads) {
-        const int r = i / (db * 8), c = i - r * (db * 8);
-        const bool ok = r < n_rows;
-        cp_async16(smem_u32(q_s) + (r >> 7) * q_bytes + (c >> 3) * kRowBlock + sw128(r & 127, c & 7), q_rows + (size_t)(ok ? r : 0) * D + c * 8, ok);
-    }
-    cp_async_commit();
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -106,82 +99,139 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_b
     auto tmem_o = [&](int x) { return tmem + (uint32_t)((buffers == 1 ? 256 : 128) * x); };
     auto tmem_s = [&](int x, int b) { return tmem + (uint32_t)(buffers == 1 ? 256 * x + 192 : 256 + 128 * x + 64 * b); };
 
-    if (warp == 0 || warp == kLoaderWarp2) {
-        // ---- loaders: alternate key tiles, as far ahead as stages are free ----------------------
+    if (warp == 0 || warp >= kLoaderWarp2) {
+        // ---- loaders: key tiles in turn, as far ahead as stages are free ----------------------
         const int* row_table = table + (size_t)seq_rows[entry] * table_stride;
         const int lanes = db > 2 ? 32 : db > 1 ? 16 : 8, c = lane & (lanes - 1), per = 32 / lanes;      // lanes per row, rows per pass
-        auto issue = [&](int tile) {
-            const uint32_t st = smem_u32(kv_s) + (uint32_t)((tile % stages) * stage_bytes);
-            const int base = k_begin + tile * kKeys;
-            // keys outside [k_lo, k_end) are zero-filled, never read (a page the window has left may belong to another
-            // request by now); address 0 marks an entry that names no page of the pool
-            unsigned long long src_row[2];
+        // Where a tile's rows live: lane l looks two of them up (while the tile before is copied), all 64 addresses go through
+        // shared memory, one broadcast read per row (4,900 cycles a tile and loader; 7,000 with two 64-bit shuffles and a choice
+        // per row).  0: a row that is not read but zero-filled (keys outside
+        // [k_lo, k_end): a page the window has left may belong to another request by now; an entry that names no page).
+        const int tile0 = warp == 0 ? 0 : warp - kLoaderWarp2 + 1;
+        unsigned long long* list = row_list[tile0];
+        unsigned long long mine[2];
+        auto look_up = [&](int tile) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int j = min(max(base + 32 * h + lane, k_lo), k_end - 1);
-                const int page = row_table[j / page_size];
-                src_row[h] = page_in_pool(page, num_pages, error, 29)
-                                 ? (unsigned long long)(cache + ((size_t)page * page_size + j % page_size) * D) : 0ull;
-            }
-#pragma unroll 4
-            for (int k = 0; k < kKeys; k += per) {
-                const int r = k + lane / lanes;
-                const unsigned long long a = __shfl_sync(0xffffffffu, src_row[0], r & 31);
-                const unsigned long long b = __shfl_sync(0xffffffffu, src_row[1], r & 31);
-                const unsigned long long row_addr = r < 32 ? a : b;
-                const bool ok = base + r < k_end && base + r >= k_lo && row_addr != 0ull;
-                if (c < db * 8)
-                    cp_async16(st + (uint32_t)((c >> 3) * kKeyBlock) + sw128(r, c & 7),
-                               reinterpret_cast<const __nv_bfloat16*>(ok ? row_addr : (unsigned long long)cache) + c * 8, ok);
+                const int j = k_begin + tile * kKeys + 32 * h + lane;
+                mine[h] = 0ull;
+                if (j >= k_lo && j < k_end) {
+                    const int page = row_table[j / page_size];
+                    if (page_in_pool(page, num_pages, error, 29))
+                        mine[h] = (unsigned long long)(cache + ((size_t)page * page_size + j % page_size) * D);
+                }
             }
         };
+        const uint32_t c_off = (uint32_t)((c >> 3) * kKeyBlock);
         bool ok = true;
-        for (int tile = warp == 0 ? 0 : 1; tile < num_tiles && ok; tile += 2) {
+        if (tile0 < num_tiles) look_up(tile0);
+        for (int tile = tile0; tile < num_tiles; tile += kLoaders) {
+            __syncwarp();                              // the list of the tile before has been read
+            list[lane] = mine[0];
+            list[32 + lane] = mine[1];
+            __syncwarp();
+            if (tile + kLoaders < num_tiles) look_up(tile + kLoaders);
             if (tile >= stages) ok = mbar_wait(bar(&bars.kv_empty[tile % stages]), ((tile / stages) - 1) & 1, &abort_s);
             if (!ok) break;
-            issue(tile);
+            const uint32_t st = smem_u32(kv_s) + (uint32_t)((tile % stages) * stage_bytes) + c_off;
+            if (c < db * 8) {
+#pragma unroll 8
+                for (int k = 0; k < kKeys; k += per) {
+                    const int r = k + lane / lanes;
+                    const unsigned long long row_addr = list[r];
+                    cp_async16(st + sw128(r, c & 7), reinterpret_cast<const __nv_bfloat16*>(row_addr != 0ull ? row_addr : (unsigned long long)cache) + c * 8,
+                               row_addr != 0ull);
+                }
+            }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar(&bars.kv_full[tile % stages])) : "memory");
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         if (!ok) { abort_s = 1; if (lane == 0) atomicCAS(error, 0, 14); }
-    } else if (warp == 1 || warp == kMmaWarp2) {
-        // ---- MMA issuers: one lane per query tile -------------------------------------------------
-        // With two S buffers S(j) goes ahead of P V of tile j - 1; with one, P V of tile j ahead of S(j + 1), which
-        // overwrites P (MMAs of one thread run in their order).
-        if (lane == 0) {
-            const int x = warp == 1 ? 0 : 1;
-            const uint32_t id_s = idesc(kKeys, 0), id_o = idesc(rank, 1);
-            bool ok = true;
-            auto issue_pv = [&](int i) {
-                const int b = i % buffers;
-                if (!mbar_wait(bar(&bars.p_full[x][b]), (i / buffers) & 1, &abort_s)) { ok = false; return; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t va = smem_u32(kv_s) + (uint32_t)((i % stages) * stage_bytes), pa = tmem_s(x, b);
+    } else if (warp == 1) {
+        // ---- MMA issuer: one lane for both query tiles ---------------------------------------------
+        // With one S buffer P V (j) and S (j + 1) of a tile go out together as its P (j) arrives (MMAs of one thread run in their
+        // order, so P is read before S overwrites it), one tile's after the other's: the tiles' products then lie apart and each
+        // tile's softmax runs beside the other's products.  With two, S (j) goes ahead of P V of tile j - 1.
+        const uint32_t id_s = idesc(kKeys, 0), id_o = idesc(rank, 1);
+        const int tiles = uniform(num_tiles);
+        const uint32_t tm = (uint32_t)uniform((int)tmem);
+        auto o_at = [&](int x) { return tm + (uint32_t)((buffers == 1 ? 256 : 128) * x); };
+        auto s_at = [&](int x, int b) { return tm + (uint32_t)(buffers == 1 ? 256 * x + 192 : 256 + 128 * x + 64 * b); };
+        bool ok = true;
+        auto wait = [&](uint64_t* b, uint32_t parity) { ok = __all_sync(0xffffffffu, mbar_wait(bar(b), parity, &abort_s)); };
+        auto keys_ready = [&](int stage, uint32_t parity) {
+            wait(&bars.kv_full[stage], parity);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");         // the copies were generic-proxy writes
+        };
+        auto issue_pv = [&](int x, int b, int stage, bool first) {
+            const uint64_t v = desc_mnmajor(smem_u32(kv_s) + (uint32_t)(stage * stage_bytes), kKeyBlock);
+            const uint32_t pa = s_at(x, b), o = o_at(x);
 #pragma unroll
-                for (int kk = 0; kk < kKeys / 16; ++kk)
-                    umma_ts(tmem_o(x), pa + (uint32_t)(kk * 8), desc_mnmajor(va + kk * 2048, kKeyBlock), id_o, (i > 0 || kk > 0) ? 1u : 0u);
-                umma_commit(bar(&bars.p_empty[x]));
-                umma_commit(bar(&bars.kv_empty[i % stages]));
-            };
-            for (int j = 0; j < num_tiles && ok; ++j) {
-                const int b = j % buffers;
-                if (!mbar_wait(bar(&bars.kv_full[j % stages]), (j / stages) & 1, &abort_s)) { ok = false; break; }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the copies were generic-proxy writes
-                if (j >= buffers && !mbar_wait(bar(&bars.s_empty[x][b]), ((j / buffers) - 1) & 1, &abort_s)) { ok = false; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t ka = smem_u32(kv_s) + (uint32_t)((j % stages) * stage_bytes), qa = smem_u32(q_s) + (uint32_t)(x * q_bytes);
-                for (int kb = 0; kb < db; ++kb)
+            for (int kk = 0; kk < kKeys / 16; ++kk) umma_ts(o, pa + (uint32_t)(kk * 8), v + (uint64_t)(kk * 128), id_o, (!first || kk > 0) ? 1u : 0u);
+            umma_commit(bar(&bars.p_empty[x]));
+            umma_commit(bar(&bars.kv_empty[stage]));
+        };
+        auto issue_s = [&](int x, int b, int stage) {
+            uint64_t q = desc_kmajor(smem_u32(q_s) + (uint32_t)(x * q_bytes)), k = desc_kmajor(smem_u32(kv_s) + (uint32_t)(stage * stage_bytes));
+            const uint32_t to = s_at(x, b);
+            for (int kb = 0; kb < db; ++kb, q += kRowBlock / 16, k += kKeyBlock / 16)
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        umma(tmem_s(x, b), desc_kmajor(qa + kb * kRowBlock) + (uint64_t)(kk * 2), desc_kmajor(ka + kb * kKeyBlock) + (uint64_t)(kk * 2),
-                             id_s, (kb > 0 || kk > 0) ? 1u : 0u);
-                umma_commit(bar(&bars.s_full[x][b]));
-                if (j >= buffers - 1) issue_pv(j - (buffers - 1));
+                for (int kk = 0; kk < 4; ++kk) umma(to, q + (uint64_t)(kk * 2), k + (uint64_t)(kk * 2), id_s, (kb > 0 || kk > 0) ? 1u : 0u);
+            umma_commit(bar(&bars.s_full[x][b]));
+        };
+        for (int x = 0; x < kTiles && ok; ++x) wait(&bars.q_full[x], 0);
+        int stage = 0;                                       // of tile j
+        uint32_t turn = 0;                                   // how often the stages have gone round, modulo 2
+        if (buffers == 1) {
+            if (ok) keys_ready(0, 0);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (ok && elect_one())
+                for (int x = 0; x < kTiles; ++x) issue_s(x, 0, 0);
+            __syncwarp();
+            for (int j = 0; j < tiles && ok; ++j) {
+                const bool more = j + 1 < tiles;
+                const int next = stage + 1 == stages ? 0 : stage + 1;
+                const uint32_t next_turn = next == 0 ? turn ^ 1 : turn;
+                if (more) keys_ready(next, next_turn);
+                for (int x = 0; x < kTiles && ok; ++x) {
+                    wait(&bars.p_full[x][0], j & 1);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (ok && elect_one()) {
+                        issue_pv(x, 0, stage, j == 0);
+                        if (more) issue_s(x, 0, next);
+                    }
+                    __syncwarp();
+                }
+                stage = next;
+                turn = next_turn;
             }
-            if (ok && buffers == 2) issue_pv(num_tiles - 1);
-            if (ok) umma_commit(bar(&bars.o_done[x]));
-            if (!ok) { abort_s = 1; atomicCAS(error, 0, 15); }
+        } else {
+            int before = 0;                                  // the stage of tile j - 1
+            for (int j = 0; j <= tiles && ok; ++j) {
+                if (j < tiles) keys_ready(stage, turn);
+                for (int x = 0; x < kTiles && ok; ++x) {
+                    if (j < tiles) {
+                        if (j >= 2) wait(&bars.s_empty[x][j & 1], ((j >> 1) - 1) & 1);
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        if (ok && elect_one()) issue_s(x, j & 1, stage);
+                        __syncwarp();
+                    }
+                    if (j >= 1 && ok) {
+                        wait(&bars.p_full[x][(j - 1) & 1], ((j - 1) >> 1) & 1);
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        if (ok && elect_one()) issue_pv(x, (j - 1) & 1, before, j == 1);
+                        __syncwarp();
+                    }
+                }
+                before = stage;
+                stage = stage + 1 == stages ? 0 : stage + 1;
+                if (stage == 0) turn ^= 1;
+            }
         }
+        if (ok && elect_one())
+            for (int x = 0; x < kTiles; ++x) umma_commit(bar(&bars.o_done[x]));
+        if (!ok) { abort_s = 1; if (lane == 0) atomicCAS(error, 0, 15); }
+        __syncwarp();
     } else if (warp < 2 + 4 * kTiles) {
         // ---- softmax and epilogue: four warps per query tile, one thread per row --------------------
         const int x = (warp - 2) >> 2, quarter = warp & 3;
@@ -190,6 +240,18 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_b
         const long long row = row_base + (valid ? r : n_rows - 1);
         const int pos = q_start + (int)(row / heads), lo = first_visible(pos, window);
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+        // The tile's query rows, which lie one behind the other, while the loaders bring the first keys; rows beyond the
+        // portion's are zeros.
+        const int thread = threadIdx.x - 64 - 128 * x;
+        const __nv_bfloat16* q_rows = qfull + ((size_t)tok0 * heads + (size_t)row_base + x * kRows) * D;
+        for (int i = thread; i < kRows * db * 8; i += 128) {
+            const int qr = i / (db * 8), c = i - qr * (db * 8);
+            const bool there = x * kRows + qr < n_rows;
+            cp_async16(smem_u32(q_s) + x * q_bytes + (c >> 3) * kRowBlock + sw128(qr, c & 7), there ? q_rows + (size_t)qr * D + c * 8 : qfull, there);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_arrive(bar(&bars.q_full[x]));
         float m_ref = -INFINITY, l = 0.f;                  // reference maximum (log2 units), running sum
         bool ok = true;
         for (int j = 0; j < num_tiles && ok; ++j) {
