@@ -11,12 +11,17 @@
 // The arrangement of barriers and the softmax are those of attention_prefill_tc.cu: four softmax warps per query tile, three
 // loader warps, one MMA-issuing warp, every wait bounded and reported through the error word.
 //
-// What bounds it: at a row of 256 and a rank of 192 a key tile takes a query tile 896 cycles of the tensor pipe
-// (128 x 64 x (256 + 192) multiply-adds) against 512 of the exponential unit.  The mma.sync kernel (latent_attention.cu), which
-// stays for steps of few rows (it splits them along the keys) and for other sizes, ends at a third of the tensor rate.
+// What bounds it: at a row of 256 and a rank of 192 a key tile takes a query tile 1,150 cycles of the tensor pipe
+// (128 x 64 x (256 + 192) multiply-adds, S at the rate its operands leave shared memory) and each softmax warp about 1,700 beside
+// the other tile's; with one S buffer they follow one another, so a key tile takes the pair 3,700 cycles.  Measured, 32 heads,
+// row 256, rank 192: 8,192 tokens with a window of 1,024 310 us (727 TFLOP/s), four prompts of 2,048 tokens 305, one 79.  The
+// mma.sync kernel (latent_attention.cu) takes 866, 894 and 183: it stays for steps of few rows, which it splits along the keys,
+// and for other sizes.
 #include "common.cuh"
 #include "fa_util.cuh"
 #include "mma_util.cuh"
+#include <cuda.h>
+#include <mutex>
 
 namespace se {
 namespace lat_tc {
@@ -43,7 +48,7 @@ struct Bars {
 
 // db, rb: blocks of 64 dims of a row and of its latent part; buffers: S buffers per query tile; stages: key tiles in flight
 __global__ void __launch_bounds__(kThreads, 1)
-latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_bfloat16* __restrict__ cache,
+latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __nv_bfloat16* __restrict__ cache,
                            const int* __restrict__ table, int table_stride, const int* __restrict__ seq_rows,
                            const int* __restrict__ cu_q, const int* __restrict__ kv_len, const float* __restrict__ sink,
                            __nv_bfloat16* __restrict__ out, int heads, int db, int rb, int buffers, int stages, int page_size,
@@ -82,7 +87,7 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_b
             }
             mbar_init(bar(&bars.p_empty[x]), 1);
             mbar_init(bar(&bars.o_done[x]), 1);
-            mbar_init(bar(&bars.q_full[x]), 128);            // every thread of the tile's softmax warps
+            mbar_init(bar(&bars.q_full[x]), 1);
         }
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -152,6 +157,17 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_b
         // With one S buffer P V (j) and S (j + 1) of a tile go out together as its P (j) arrives (MMAs of one thread run in their
         // order, so P is read before S overwrites it), one tile's after the other's: the tiles' products then lie apart and each
         // tile's softmax runs beside the other's products.  With two, S (j) goes ahead of P V of tile j - 1.
+        // The query tiles first: 128 rows that lie one behind the other, 64 dims at a time.  Rows behind the portion's are other
+        // entries' or beyond the matrix (zeros): they are computed and dropped.
+        if (elect_one())
+            for (int x = 0; x < kTiles; ++x) {
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar(&bars.q_full[x])), "r"(q_bytes) : "memory");
+                for (int kb = 0; kb < db; ++kb)
+                    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                                 ::"r"(smem_u32(q_s) + (uint32_t)(x * q_bytes + kb * kRowBlock)), "l"(&q_map), "r"(bar(&bars.q_full[x])),
+                                 "r"(64 * kb), "r"((int)((long long)tok0 * heads + row_base) + x * kRows) : "memory");
+            }
+        __syncwarp();
         const uint32_t id_s = idesc(kKeys, 0), id_o = idesc(rank, 1);
         const int tiles = uniform(num_tiles);
         const uint32_t tm = (uint32_t)uniform((int)tmem);
@@ -240,18 +256,6 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_b
         const long long row = row_base + (valid ? r : n_rows - 1);
         const int pos = q_start + (int)(row / heads), lo = first_visible(pos, window);
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        // The tile's query rows, which lie one behind the other, while the loaders bring the first keys; rows beyond the
-        // portion's are zeros.
-        const int thread = threadIdx.x - 64 - 128 * x;
-        const __nv_bfloat16* q_rows = qfull + ((size_t)tok0 * heads + (size_t)row_base + x * kRows) * D;
-        for (int i = thread; i < kRows * db * 8; i += 128) {
-            const int qr = i / (db * 8), c = i - qr * (db * 8);
-            const bool there = x * kRows + qr < n_rows;
-            cp_async16(smem_u32(q_s) + x * q_bytes + (c >> 3) * kRowBlock + sw128(qr, c & 7), there ? q_rows + (size_t)qr * D + c * 8 : qfull, there);
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive(bar(&bars.q_full[x]));
         float m_ref = -INFINITY, l = 0.f;                  // reference maximum (log2 units), running sum
         bool ok = true;
         for (int j = 0; j < num_tiles && ok; ++j) {
@@ -320,21 +324,31 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_b
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (sink != nullptr) l += exp2f(fmaf(sink[(int)(row % heads)], 1.4426950408889634f, -m_ref));
             const float inv = 1.f / l;
-            __nv_bfloat16* dst = out + ((size_t)tok0 * heads + (size_t)row) * rank;
+            // A warp's 32 rows go through shared memory (its query tile's, whose last product has been read) and out as one run of
+            // memory: row by row from the threads that hold them they took 11,800 cycles, a seventh of a block's time.
+            uint8_t* stage = q_s + x * q_bytes + quarter * (32 * 2 * rank);
+            const int chunks = rank / 8;                     // 16-byte chunks of a row
 #pragma unroll 1
             for (int c0 = 0; c0 < rank; c0 += 32) {
                 uint32_t ov[32];
                 tmem_ld32(tmem_o(x) + c0 + lane_addr, ov);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (valid)
 #pragma unroll
-                    for (int c = 0; c < 32; c += 8) {
-                        uint32_t w[4];
+                for (int c = 0; c < 32; c += 8) {
+                    uint32_t w[4];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            w[i] = se::mma::pack_bf16(__uint_as_float(ov[c + 2 * i]) * inv, __uint_as_float(ov[c + 2 * i + 1]) * inv);
-                        *reinterpret_cast<uint4*>(dst + c0 + c) = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
+                    for (int i = 0; i < 4; ++i)
+                        w[i] = se::mma::pack_bf16(__uint_as_float(ov[c + 2 * i]) * inv, __uint_as_float(ov[c + 2 * i + 1]) * inv);
+                    *reinterpret_cast<uint4*>(stage + (lane * chunks + (((c0 + c) / 8) ^ (lane & 7))) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            }
+            __syncwarp();
+            const int warp_rows = min(32, n_rows - x * kRows - quarter * 32);
+            uint4* dst = reinterpret_cast<uint4*>(out + ((size_t)tok0 * heads + (size_t)row_base + x * kRows + quarter * 32) * rank);
+#pragma unroll 4
+            for (int i = lane; i < warp_rows * chunks; i += 32) {
+                const int rr = i / chunks, c = i - rr * chunks;
+                dst[i] = *reinterpret_cast<const uint4*>(stage + (rr * chunks + (c ^ (rr & 7))) * 16);
             }
         } else {
             abort_s = 1;
@@ -349,6 +363,22 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ qfull, const __nv_b
     }
 }
 
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static EncodeTiledFn encode_fn() {
+    static EncodeTiledFn fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            fn = (EncodeTiledFn)f;
+    });
+    return fn;
+}
+
 }  // namespace lat_tc
 }  // namespace se
 
@@ -359,8 +389,8 @@ extern "C" int se_latent_attention_tc_supported(int rank, int rot) {
 
 // Arguments as se_latent_attention_tiled's (which splits the keys of steps of few rows).
 extern "C" int se_latent_attention_tc(const void* qfull, const void* cache, const int* table, int table_stride, const int* seq_rows,
-                                      const int* cu_q, const int* kv_len, const float* sink, void* out, int entries, int max_q_len,
-                                      int heads, int rank, int rot, int page_size, float scale, int window, int num_pages, int* error,
+                                      const int* cu_q, const int* kv_len, const float* sink, void* out, int tokens, int entries,
+                                      int max_q_len, int heads, int rank, int rot, int page_size, float scale, int window, int num_pages, int* error,
                                       cudaStream_t stream) {
     using namespace se::lat_tc;
     if (entries <= 0 || max_q_len <= 0) return 0;
@@ -373,10 +403,19 @@ extern "C" int se_latent_attention_tc(const void* qfull, const void* cache, cons
     const int room = 226 * 1024 - kTiles * db * kRowBlock;
     const int fit = room / (db * kKeyBlock), stages = fit < kMaxStages ? fit : kMaxStages;
     const size_t smem = (size_t)kTiles * db * kRowBlock + (size_t)stages * db * kKeyBlock + 1024;
+    const EncodeTiledFn encode = encode_fn();
+    if (encode == nullptr) return (int)cudaErrorNotSupported;
+    CUtensorMap q_map;                                   // [tokens * heads][rank + rot], boxes of 128 rows and 64 dims
+    const cuuint64_t dims[2] = {(cuuint64_t)(db * 64), (cuuint64_t)tokens * heads}, strides[1] = {(cuuint64_t)db * 128};
+    const cuuint32_t box[2] = {64, kRows}, steps[2] = {1, 1};
+    if ((long long)tokens * heads > 0x7fffffffLL - kTiles * kRows) return SE_ERR_UNSUPPORTED;
+    if (encode(&q_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(qfull), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return SE_ERR_ARGUMENT;
     const cudaError_t e = cudaFuncSetAttribute(latent_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     latent_attention_tc_kernel<<<dim3((unsigned)row_tiles, entries), kThreads, smem, stream>>>(
-        (const __nv_bfloat16*)qfull, (const __nv_bfloat16*)cache, table, table_stride, seq_rows, cu_q, kv_len, sink,
+        q_map, (const __nv_bfloat16*)cache, table, table_stride, seq_rows, cu_q, kv_len, sink,
         (__nv_bfloat16*)out, heads, db, rb, buffers, stages, page_size, scale * 1.4426950408889634f, window, num_pages, error);
     return (int)cudaGetLastError();
 }

@@ -530,21 +530,24 @@ def latent_attention_tc_supported(rank: int, rot: int) -> bool:
 
 
 def latent_takes_tc(entries: int, max_q_len: int, heads: int, rank: int, rot: int, sms: Optional[int] = None) -> bool:
-    """Whether a step's latent attention runs on tcgen05 (csrc/latent_attention_tc.cu): sizes it takes, and blocks of 256 rows
-    for a third of the SMs (steps of fewer rows split their keys over the device instead)."""
+    """Whether a step's latent attention runs on tcgen05 (csrc/latent_attention_tc.cu): sizes it takes, an entry that fills half
+    a query tile, and blocks of 256 rows for a fifth of the SMs (steps of fewer rows split their keys over the device instead).
+    Measured, 32 heads, us there and here: 8 blocks over 4,096 keys 52 / 141, 16 blocks 99 / 145, 32 blocks 186 / 149; 64 requests
+    at 2,048 keys that bring 1, 2 and 8 tokens 33 / 46, 38 / 46 and 104 / 47."""
     if sms is None:
         sms = sm_count()
-    return latent_attention_tc_supported(rank, rot) and 3 * entries * -(-max_q_len * heads // 256) >= sms
+    rows = max_q_len * heads
+    return latent_attention_tc_supported(rank, rot) and rows >= 128 and 5 * entries * -(-rows // 256) >= sms
 
 
 def latent_attention_tc(qfull, cache, table, seq_rows, cu_q, kv_len, sink, out, *, entries, max_q_len, heads, rank, rot,
                         page_size, scale, window=None, num_pages=None):
     """:func:`latent_attention_tiled` for steps with prompt portions, on tcgen05."""
-    _check(_fn("se_latent_attention_tc", "pppi" "ppp" "pp" "iiiii" "i" "f" "ii" "p" "p")(
+    _check(_fn("se_latent_attention_tc", "pppi" "ppp" "pp" "iiiiii" "i" "f" "ii" "p" "p")(
         _ptr(qfull, torch.bfloat16, "qfull"), _ptr(cache, torch.bfloat16, "cache"), _ptr(table, torch.int32, "table"),
         table.shape[1], _ptr(seq_rows, torch.int32, "seq_rows"), _ptr(cu_q, torch.int32, "cu_q"),
-        _ptr(kv_len, torch.int32, "kv_len"), _ptr(sink, torch.float32, "sink"), _ptr(out, torch.bfloat16, "out"), entries,
-        max_q_len, heads, rank, rot, page_size, float(scale), int(window or 0),
+        _ptr(kv_len, torch.int32, "kv_len"), _ptr(sink, torch.float32, "sink"), _ptr(out, torch.bfloat16, "out"),
+        qfull.shape[0], entries, max_q_len, heads, rank, rot, page_size, float(scale), int(window or 0),
         cache.shape[0] if num_pages is None else int(num_pages), _ptr(error_word(qfull.device)), _stream()), "latent_attention_tc")
     return out
 

@@ -62,5 +62,5 @@ def test_against_64_bits(rank, rot, heads, window, sinks):
 def test_choice_by_rows():
     from sparseengine_b200.csrc import ops
     assert ops.latent_takes_tc(1, 2048, 32, 192, 64, 148) and ops.latent_takes_tc(4, 512, 16, 128, 64, 148)
-    assert not ops.latent_takes_tc(64, 1, 32, 192, 64, 300) and not ops.latent_takes_tc(1, 64, 32, 192, 64, 148)
+    assert not ops.latent_takes_tc(64, 1, 32, 192, 64, 148) and not ops.latent_takes_tc(1, 64, 32, 192, 64, 148)
     assert not ops.latent_takes_tc(1, 8192, 32, 256, 0, 148) and not ops.latent_takes_tc(1, 8192, 32, 80, 48, 148)
