@@ -727,11 +727,11 @@ def causal_conv(x, c0: int, w, bias, state, conv_off: int, step, out):
     ``step.state_rows``, from element ``conv_off`` on, ``[taps-1, C]``), which are brought up to date."""
     tokens = x.shape[0]
     C, taps = w.shape
-    _check(_fn("se_causal_conv", "pii" "pp" "pli" "ppp" "p" "iiii" "ip")(
+    _check(_fn("se_causal_conv", "pii" "pp" "pli" "ppp" "p" "iiiii" "ip")(
         x.data_ptr(), x.stride(0), int(c0), _ptr(w, torch.float32, "conv weight"), _ptr(bias, torch.float32, "conv bias"),
         _ptr(state, torch.float32, "state"), state.stride(0), int(conv_off), _ptr(step.token_seq), _ptr(step.cu_q),
-        _ptr(step.seq_rows), _ptr(out, torch.float32, "out"), tokens, step.num_seqs, C, taps, dtype_code(x.dtype),
-        _stream()), "causal_conv")
+        _ptr(step.seq_rows), _ptr(out, torch.float32, "out"), tokens, step.num_seqs, C, taps,
+        int(getattr(step, "max_q_len", 0)), dtype_code(x.dtype), _stream()), "causal_conv")
     return out
 
 

@@ -105,8 +105,8 @@ template <> __device__ __forceinline__ void put_four<__nv_bfloat16>(__nv_bfloat1
 template <typename T, int TILE>
 __global__ void __launch_bounds__(128)
 causal_conv4_kernel(const T* x, int pitch, int c0, const float* __restrict__ w, const float* __restrict__ bias,
-                    const float* state, long long state_pitch, int conv_off, const int* __restrict__ token_seq,
-                    const int* __restrict__ cu_q, const int* __restrict__ seq_rows, float* __restrict__ out, int tokens, int C) {
+                    float* state, long long state_pitch, int conv_off, const int* __restrict__ token_seq,
+                    const int* __restrict__ cu_q, const int* __restrict__ seq_rows, float* __restrict__ out, int tokens, int C, int carry) {
     constexpr int kTaps = 4;
     const int t0 = blockIdx.x * TILE, c = (blockIdx.y * 128 + threadIdx.x) * 4;
     if (c >= C) return;
@@ -144,6 +144,11 @@ causal_conv4_kernel(const T* x, int pitch, int c0, const float* __restrict__ w, 
         a.y = b.y + wr[1].x * v[0].y; a.y += wr[1].y * v[1].y; a.y += wr[1].z * v[2].y; a.y += wr[1].w * v[3].y;
         a.z = b.z + wr[2].x * v[0].z; a.z += wr[2].y * v[1].z; a.z += wr[2].z * v[2].z; a.z += wr[2].w * v[3].z;
         a.w = b.w + wr[3].x * v[0].w; a.w += wr[3].y * v[1].w; a.w += wr[3].z * v[2].w; a.w += wr[3].w * v[3].w;
+        if (TILE == 1 && carry) {             // every entry brought one token: its window's last inputs are the new carried ones
+            float* carried = state + (size_t)seq_rows[e] * state_pitch + conv_off + c;
+#pragma unroll
+            for (int j = 0; j < kTaps - 1; ++j) put_four(carried + (size_t)j * C, v[j + 1]);
+        }
         put_four(out + (size_t)t * C + c, make_float4(silu_act<T>(a.x), silu_act<T>(a.y), silu_act<T>(a.z), silu_act<T>(a.w)));
     }
 }
@@ -688,6 +693,165 @@ static inline void tile_plan(int rows, int columns, int units, int* nsplit, int*
     *cols = groups * kTileCols;
 }
 
+// ---- the recurrences a state row per lane group: short pieces and single tokens -------------------
+// A state column (value side) is a run of N or d neighbouring floats: LANES lanes hold it, four floats each, eight columns at a
+// time, so the state moves in 16-byte accesses that are all in flight together and stays in registers over an entry's tokens.  The
+// eight sums over a column are reduced together (lanes trade the sums they do not keep).  A decode step is bound by reading
+// and writing the states once; the tiles above move 4 bytes per access and stage every token in shared memory.
+
+// v[0..7] per lane -> the sum over its group of LANES (8 to 32) lanes of value number `which`, in the lanes that return it
+template <int LANES>
+__device__ __forceinline__ float group_sum8(float (&v)[8], int lane) {
+    int o = LANES / 2;
+#pragma unroll
+    for (int m = 4; m >= 1; m >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < m; ++i) {
+            const float give = up ? v[i] : v[i + m], keep = up ? v[i + m] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+template <int LANES>
+__device__ __forceinline__ int group_which(int lane) {
+    return ((lane & (LANES / 2)) ? 4 : 0) + ((lane & (LANES / 4)) ? 2 : 0) + ((lane & (LANES / 8)) ? 1 : 0);
+}
+template <int LANES>
+__device__ __forceinline__ float group_sum(float v) {
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ float dot4(float4 a, float4 b) { return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x))); }
+
+constexpr int kRowWarps = 4;
+
+// State space, as ssm_scan_tile_kernel; step sizes and decays are worked out here.  grid (entries, H, column groups).
+template <typename T, int LANES>
+__global__ void __launch_bounds__(32 * kRowWarps)
+ssm_rows_kernel(const float* __restrict__ xbc, const T* proj, int pitch, int dt_off, const float* __restrict__ dt_bias,
+                const float* __restrict__ a_log, const float* __restrict__ d_skip, float* state, long long state_pitch,
+                const int* __restrict__ cu_q, const int* __restrict__ seq_rows, float* __restrict__ y, int H, int P, int N, int G) {
+    constexpr int kGroups = 32 / LANES;
+    const int e = blockIdx.x, h = blockIdx.y, g = h / (H / G), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int start = cu_q[e], end = cu_q[e + 1], width = H * P + 2 * G * N;
+    const int c = (lane % LANES) * 4, p0 = ((blockIdx.z * kRowWarps + warp) * kGroups + lane / LANES) * 8;
+    if (start >= end) return;
+    const bool in = c < N;
+    float* Sp = state + (size_t)seq_rows[e] * state_pitch + ((size_t)h * P + p0) * N + c;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 S[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) S[i] = in && p0 + i < P ? four(Sp + (size_t)i * N) : zero;
+    const float rate = expf(a_log[h]), bias = dt_bias[h], skip = d_skip[h];
+    const float* row = xbc + (size_t)start * width;
+    const T* dts = proj + (size_t)start * pitch + dt_off + h;
+    float4 B = in ? four(row + H * P + (size_t)g * N + c) : zero, C = in ? four(row + H * P + (size_t)(G + g) * N + c) : zero;
+    float raw = to_float(*dts);
+    for (int t = start; t < end; ++t) {
+        float x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = p0 + i < P ? row[(size_t)h * P + p0 + i] : 0.f;
+        const float dt = softplus_f(raw + bias), a = expf(-rate * dt);
+        const float4 b = B, cc = C;
+        row += width;
+        dts += pitch;
+        if (t + 1 < end) {                       // the next token's inputs while this one is computed
+            B = in ? four(row + H * P + (size_t)g * N + c) : zero;
+            C = in ? four(row + H * P + (size_t)(G + g) * N + c) : zero;
+            raw = to_float(*dts);
+        }
+        float sums[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float bx = dt * x[i];
+            S[i].x = fmaf(b.x, bx, a * S[i].x);
+            S[i].y = fmaf(b.y, bx, a * S[i].y);
+            S[i].z = fmaf(b.z, bx, a * S[i].z);
+            S[i].w = fmaf(b.w, bx, a * S[i].w);
+            sums[i] = dot4(S[i], cc);
+        }
+        const float sum = group_sum8<LANES>(sums, lane);
+        const int p = p0 + group_which<LANES>(lane);
+        if ((lane & (LANES / 8 - 1)) == 0 && p < P) y[(size_t)t * H * P + (size_t)h * P + p] = sum + skip * (row - width)[(size_t)h * P + p];
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        if (in && p0 + i < P) put_four(Sp + (size_t)i * N, S[i]);
+}
+
+// Gated delta rule, as delta_scan_tile_kernel, from what delta_prep leaves.  A token's two sums per column, (g S)^T k and (g S)^T q,
+// are reduced together: S' = g S + k u^T gives o = (g S)^T q + (k . q) u.
+template <int LANES>
+__global__ void __launch_bounds__(32 * kRowWarps)
+delta_rows_kernel(const float* __restrict__ qkv, const float* __restrict__ dec, const float* __restrict__ beta, float* state,
+                  long long state_pitch, const int* __restrict__ cu_q, const int* __restrict__ seq_rows, float* __restrict__ o,
+                  int H, int G, int d, int dv) {
+    constexpr int kGroups = 32 / LANES;
+    const int e = blockIdx.x, h = blockIdx.y, g = h / (H / G), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int start = cu_q[e], end = cu_q[e + 1], width = 2 * G * d + H * dv;
+    const int c = (lane % LANES) * 4, j0 = ((blockIdx.z * kRowWarps + warp) * kGroups + lane / LANES) * 8;
+    if (start >= end) return;
+    const bool in = c < d;
+    float* Sp = state + (size_t)seq_rows[e] * state_pitch + ((size_t)h * dv + j0) * d + c;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 S[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) S[i] = in && j0 + i < dv ? four(Sp + (size_t)i * d) : zero;
+    const float* row = qkv + (size_t)start * width + (size_t)g * d + c;
+    const float* drow = dec + ((size_t)start * H + h) * d + c;
+    float4 q = in ? four(row) : zero, k = in ? four(row + (size_t)G * d) : zero, gv = in ? four(drow) : zero;
+    const int which = group_which<LANES>(lane), base = lane & ~(LANES - 1);
+    const bool keeper = (lane & (LANES / 8 - 1)) == 0;
+    for (int t = start; t < end; ++t) {
+        const float4 qt = q, kt = k, gt = gv;
+        const float bt = beta[(size_t)t * H + h];
+        const float v = j0 + which < dv ? qkv[(size_t)t * width + 2 * G * d + (size_t)h * dv + j0 + which] : 0.f;
+        row += width;
+        drow += (size_t)H * d;
+        if (t + 1 < end && in) {
+            q = four(row);
+            k = four(row + (size_t)G * d);
+            gv = four(drow);
+        }
+        float rs[8], os[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            S[i].x *= gt.x; S[i].y *= gt.y; S[i].z *= gt.z; S[i].w *= gt.w;
+            rs[i] = dot4(S[i], kt);
+            os[i] = dot4(S[i], qt);
+        }
+        const float r = group_sum8<LANES>(rs, lane), oq = group_sum8<LANES>(os, lane);
+        const float kq = group_sum<LANES>(dot4(kt, qt)), u = bt * (v - r);
+        if (keeper && j0 + which < dv) o[((size_t)t * H + h) * dv + j0 + which] = fmaf(kq, u, oq);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {            // column i's u from a lane that keeps it
+            const int from = base + ((i & 4) ? LANES / 2 : 0) + ((i & 2) ? LANES / 4 : 0) + ((i & 1) ? LANES / 8 : 0);
+            const float ui = __shfl_sync(0xffffffffu, u, from);
+            S[i].x = fmaf(kt.x, ui, S[i].x);
+            S[i].y = fmaf(kt.y, ui, S[i].y);
+            S[i].z = fmaf(kt.z, ui, S[i].z);
+            S[i].w = fmaf(kt.w, ui, S[i].w);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        if (in && j0 + i < dv) put_four(Sp + (size_t)i * d, S[i]);
+}
+
+// Lanes per column for states of `rows` rows, or 0: sizes that stay with the tiles (columns of 20 to 128 floats in fours).
+static inline int row_lanes(int rows) { return rows % 4 || rows <= 16 || rows > 128 ? 0 : rows <= 32 ? 8 : rows <= 64 ? 16 : 32; }
+static inline bool rows_aligned(const void* state, long long pitch, const void* a, const void* b) {
+    return pitch % 4 == 0 && ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
+}
+#define SE_ROW_LANES(lanes, ...)                                   \
+    if ((lanes) == 8) { constexpr int LANES = 8; __VA_ARGS__; }    \
+    else if ((lanes) == 16) { constexpr int LANES = 16; __VA_ARGS__; } \
+    else { constexpr int LANES = 32; __VA_ARGS__; }
+
 // ---- prologue of the delta rule ----------------------------------------------------------------
 // One block per token: q and k heads (in qkv, in place) become unit vectors, x / sqrt(sum x^2 +
 // unit_eps), q also times q_scale; dec = exp(-exp(A_log[h]) * softplus(a + dt_bias)); beta =
@@ -861,8 +1025,9 @@ extern "C" int se_recurrent_max_state_rows() { return se::kMaxStateRows; }
 
 extern "C" int se_causal_conv(const void* x, int pitch, int c0, const float* w, const float* bias, float* state,
                               long long state_pitch, int conv_off, const int* token_seq, const int* cu_q,
-                              const int* seq_rows, float* out, int tokens, int entries, int C, int taps, int dtype,
+                              const int* seq_rows, float* out, int tokens, int entries, int C, int taps, int max_q_len, int dtype,
                               cudaStream_t stream) {
+    // max_q_len: the longest entry's tokens (1: every entry that is not empty has one)
     if (tokens <= 0) return 0;
     if (C <= 0 || taps <= 0 || entries <= 0) return SE_ERR_ARGUMENT;
     const int threads = 128;
@@ -872,20 +1037,21 @@ extern "C" int se_causal_conv(const void* x, int pitch, int c0, const float* w, 
     if (grid.y > 65535 || taps > 64) return SE_ERR_UNSUPPORTED;
     const size_t smem = (size_t)(tile + taps - 1) * 128 * sizeof(float);
     // four channels at a time: four taps, and everything that is read or written on 16 bytes (8 for 16-bit inputs)
+    const int single = max_q_len == 1;
     const bool four = taps == 4 && C % 4 == 0 && pitch % 4 == 0 && c0 % 4 == 0 && state_pitch % 4 == 0 && conv_off % 4 == 0 &&
                       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(bias) |
                         reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     SE_DISPATCH_DTYPE(dtype, T, {
         if (four && tile >= 8)
             se::causal_conv4_kernel<T, 8><<<dim3(se::ceil_div(tokens, 8), se::ceil_div(C, 512)), 128, 0, stream>>>(
-                (const T*)x, pitch, c0, w, bias, state, state_pitch, conv_off, token_seq, cu_q, seq_rows, out, tokens, C);
+                (const T*)x, pitch, c0, w, bias, state, state_pitch, conv_off, token_seq, cu_q, seq_rows, out, tokens, C, 0);
         else if (four)
             se::causal_conv4_kernel<T, 1><<<dim3(tokens, se::ceil_div(C, 512)), 128, 0, stream>>>(
-                (const T*)x, pitch, c0, w, bias, state, state_pitch, conv_off, token_seq, cu_q, seq_rows, out, tokens, C);
+                (const T*)x, pitch, c0, w, bias, state, state_pitch, conv_off, token_seq, cu_q, seq_rows, out, tokens, C, single);
         else
             se::causal_conv_kernel<T><<<grid, threads, smem, stream>>>((const T*)x, pitch, c0, w, bias, state, state_pitch, conv_off,
                                                                        token_seq, cu_q, seq_rows, out, tokens, C, taps, tile);
-        if (taps > 1)
+        if (taps > 1 && !(four && single && tile < 8))
             se::conv_carry_kernel<T><<<grid2, threads, 0, stream>>>((const T*)x, pitch, c0, state, state_pitch, conv_off, cu_q,
                                                                     seq_rows, C, taps);
     });
@@ -901,6 +1067,18 @@ extern "C" int se_ssm_scan(const float* xbc, const void* proj, int pitch, int dt
     if (entries <= 0) return 0;
     if (H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G) return SE_ERR_ARGUMENT;
     if (N > se::kMaxStateRows || H > 65535) return SE_ERR_UNSUPPORTED;
+    const int lanes = se::row_lanes(N);
+    if (lanes != 0 && (H * P) % 4 == 0 && se::rows_aligned(state, state_pitch, xbc, nullptr)) {
+        const int per = se::kRowWarps * (32 / lanes) * 8;
+        const dim3 grid(entries, H, se::ceil_div(P, per));
+        SE_DISPATCH_DTYPE(dtype, T, {
+            SE_ROW_LANES(lanes, {
+                se::ssm_rows_kernel<T, LANES><<<grid, 32 * se::kRowWarps, 0, stream>>>(xbc, (const T*)proj, pitch, dt_off, dt_bias, a_log, d_skip,
+                                                                                   state, state_pitch, cu_q, seq_rows, y, H, P, N, G);
+            });
+        });
+        SE_LAUNCH_CHECK();
+    }
     int regs, nsplit, cols;
     if (N <= se::kTileRows * 32 && steps != nullptr) {
         se::tile_plan(N, P, entries * H, &nsplit, &cols);
@@ -955,6 +1133,15 @@ extern "C" int se_delta_scan(const float* qkv, const float* dec, const float* be
     if (entries <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0) return SE_ERR_ARGUMENT;
     if (d > se::kMaxStateRows || H > 65535) return SE_ERR_UNSUPPORTED;
+    const int lanes = se::row_lanes(d);
+    if (lanes != 0 && dv % 4 == 0 && se::rows_aligned(state, state_pitch, qkv, dec)) {
+        const int per = se::kRowWarps * (32 / lanes) * 8;
+        const dim3 grid(entries, H, se::ceil_div(dv, per));
+        SE_ROW_LANES(lanes, {
+            se::delta_rows_kernel<LANES><<<grid, 32 * se::kRowWarps, 0, stream>>>(qkv, dec, beta, state, state_pitch, cu_q, seq_rows, o, H, G, d, dv);
+        });
+        SE_LAUNCH_CHECK();
+    }
     int regs, nsplit, cols;
     if (d <= se::kTileRows * 32) {
         se::tile_plan(d, dv, entries * H, &nsplit, &cols);

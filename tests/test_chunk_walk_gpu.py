@@ -40,15 +40,17 @@ def _close(got, want, what):
     assert worst < BOUND * most, f"{what}: {worst:.3e} of {most:.3e}"
 
 
-SIZES = [(128, 128, 3, 3), (64, 64, 4, 2), (8, 4, 2, 1), (100, 36, 3, 3), (128, 20, 40, 10), (44, 132, 2, 2)]
+SIZES = [(128, 128, 3, 3), (64, 64, 4, 2), (8, 4, 2, 1), (100, 36, 3, 3), (128, 20, 40, 10), (44, 132, 2, 2), (32, 12, 2, 2)]
 
 
 @pytest.mark.parametrize("decay", ["slow", "fast"])
 @pytest.mark.parametrize("d,dv,heads,kv_heads", SIZES)
-@pytest.mark.parametrize("kind", ["retention", "state space", "delta, per head", "delta, per channel"])
+@pytest.mark.parametrize("kind", ["retention", "state space", "delta, per head", "delta, per channel", "state space, tokens", "delta, tokens"])
 def test_chunks_against_the_walk(kind, d, dv, heads, kv_heads, decay):
-    """``fast``: decays down to e^-30 per token, whose products underflow within a chunk."""
+    """``fast``: decays down to e^-30 per token, whose products underflow within a chunk.  ``tokens``: the kernels that walk token
+    by token, on the same inputs."""
     from sparseengine_b200.csrc import ops
+    tokens = kind.endswith("tokens")
     step = _step([3, 0, 11, 1, 7, 2, 5, 4, 9, 6])
     T, g = step.num_tokens, torch.Generator(device=DEV).manual_seed(d + heads)
 
@@ -69,11 +71,11 @@ def test_chunks_against_the_walk(kind, d, dv, heads, kv_heads, decay):
         ops.retention_chunk(q.view(T, -1), k.view(T, -1), v, 4, decays, state, step, o.view(T, -1), silu=True, **sizes)
         v = torch.nn.functional.silu(v[:, 4:4 + heads * dv].double()).view(T, heads, dv)
         keep, beta = decays.double().view(1, heads, 1).expand(T, -1, -1), None
-    elif kind == "state space":
+    elif kind.startswith("state space"):
         width = heads * dv + 2 * kv_heads * d
         xbc, proj = rnd(T, width), rnd(T, heads + 3)
         bias, a_log, skip = rnd(heads) - 2.0, torch.log(torch.rand(heads, generator=g, device=DEV) * (30 if decay == "fast" else 1) + 0.1), rnd(heads)
-        ops.ssm_walk(xbc, proj, 2, bias, a_log, skip, state, step, o.view(T, -1), heads=heads, head_dim=dv, state_size=d, groups=kv_heads)
+        (ops.ssm_scan if tokens else ops.ssm_walk)(xbc, proj, 2, bias, a_log, skip, state, step, o.view(T, -1), heads=heads, head_dim=dv, state_size=d, groups=kv_heads)
         dt = torch.nn.functional.softplus(proj[:, 2:2 + heads].double() + bias.double())
         x = xbc[:, :heads * dv].double().view(T, heads, dv)
         k = xbc[:, heads * dv:heads * dv + kv_heads * d].view(T, kv_heads, d).repeat_interleave(rep, 1)
@@ -84,8 +86,14 @@ def test_chunks_against_the_walk(kind, d, dv, heads, kv_heads, decay):
         qkv, proj, cols = rnd(T, 2 * kv_heads * d + heads * dv), rnd(T, heads + 4), heads * (1 if per_head else d)
         a, bias = rnd(T, cols + (-cols) % 4), rnd(cols) - 1.0
         a_log = torch.log(torch.rand(heads, generator=g, device=DEV) * (20 if decay == "fast" else 0.5) + 0.05)
-        ops.delta_walk(qkv, a, proj, 2, bias, a_log, state, step, o.view(T, -1), heads=heads, kv_heads=kv_heads, head_dim=d, v_head_dim=dv,
-                       unit_eps=1e-6, q_scale=d ** -0.5, per_head=per_head)
+        delta = dict(heads=heads, kv_heads=kv_heads, head_dim=d, v_head_dim=dv)
+        inputs = dict(unit_eps=1e-6, q_scale=d ** -0.5, per_head=per_head)
+        if tokens:
+            made, dec, b = qkv.clone(), torch.empty(T, heads * d, device=DEV), torch.empty(T, heads, device=DEV)
+            ops.delta_prep(made, a[:, :cols].contiguous(), proj, 2, bias, a_log, dec, b, **delta, **inputs)
+            ops.delta_scan(made, dec, b, state, step, o.view(T, -1), **delta)
+        else:
+            ops.delta_walk(qkv, a, proj, 2, bias, a_log, state, step, o.view(T, -1), **delta, **inputs)
         qk = qkv[:, :2 * kv_heads * d].double().view(T, 2 * kv_heads, d)
         qk = qk / torch.sqrt((qk * qk).sum(-1, keepdim=True) + 1e-6)
         q, k = (t.repeat_interleave(rep, 1) for t in (qk[:, :kv_heads] * d ** -0.5, qk[:, kv_heads:]))

@@ -38,8 +38,7 @@ def test_convolution(C, off, taps, lens, dtype):
     i32 = dict(dtype=torch.int32, device=DEV)
     rows = list(range(len(lens), 0, -1))
     step = SimpleNamespace(token_seq=torch.tensor([e for e, n in enumerate(lens) for _ in range(n)], **i32), cu_q=torch.tensor(cu, **i32),
-                           seq_rows=torch.tensor(rows, **i32), num_seqs=len(lens))
-    step.state_rows = step.seq_rows
+                           seq_rows=torch.tensor(rows, **i32), num_seqs=len(lens), max_q_len=max(lens))
     out = torch.full((T, C), float("nan"), device=DEV)
     ops.causal_conv(x, off, w, b, state, conv_off, step, out)
     for e, n in enumerate(lens):
