@@ -630,29 +630,40 @@ def retention_segment_plan(entries: int, heads: int, v_head_dim: int, max_q_len:
 
 
 def retention_chunk(q32, k32, proj, v_off: int, decay, state, step, o, *, heads, head_dim, v_head_dim, segments=None,
-                    silu: bool = False):
+                    silu: bool = False, qk=None, rotation=None):
     """The same recurrence as :func:`retention_scan` in chunks of 64 tokens (closed form per chunk, 32-bit
-    FMA arithmetic): for steps that bring prompt portions.  By default the chunks are prepared side by side and walked
-    (csrc/chunk_walk.cuh) where the sizes allow it; else, or with ``segments`` (``(per entry, tokens each)``, default by
-    :func:`retention_segment_plan`), one kernel does a chunk at a time."""
+    FMA arithmetic): for steps that bring prompt portions.  With q32 and k32 one kernel does a chunk at a time; ``segments``:
+    ``(per entry, tokens each)``, default by :func:`retention_segment_plan`.  With ``qk`` (and ``q32`` and ``k32`` None): ``(q_off,
+    k_off, k_scale)`` of the projection and ``rotation`` ``(inv_freq, rotary_dim, positions)`` (None: none); the chunks are
+    prepared side by side and walked (csrc/chunk_walk.cuh), where :func:`retention_walk_supported` says so."""
     global launch_count
-    seg_state = work = None
-    max_seg, seg_len = 1, 0
-    if segments is None and chunk_walk_supported(head_dim, v_head_dim, proj.stride(0), int(v_off)) and proj.data_ptr() % 16 == 0:
-        work = _walk_work(q32.shape[0] * heads * 66, q32.device)
+    seg_state = work = inv_freq = positions = None
+    max_seg, seg_len, q_off, k_off, k_scale, rotary_dim, tokens = 1, 0, 0, 0, 1.0, 0, proj.shape[0]
+    if qk is not None:
+        q_off, k_off, k_scale = qk
+        if rotation is not None:
+            inv_freq, rotary_dim, positions = rotation
+        work = _walk_work(tokens * heads * (2 * head_dim + 66), proj.device)
     else:
         max_seg, seg_len = segments if segments is not None else retention_segment_plan(
             step.num_seqs, heads, v_head_dim, step.max_q_len, sm_count(q32.device))
         if max_seg > 1:
             seg_state = torch.empty(step.num_seqs * max_seg * heads * head_dim * v_head_dim, dtype=torch.float32, device=q32.device)
             launch_count += 1
-    _check(_fn("se_retention_chunk", "pp" "pii" "p" "pl" "pp" "p" "iiii" "iipi" "pii" "ip")(
+    _check(_fn("se_retention_chunk", "pp" "pii" "p" "pl" "pp" "p" "iiii" "iipi" "iippif" "pii" "ip")(
         _ptr(q32, torch.float32, "q32"), _ptr(k32, torch.float32, "k32"), proj.data_ptr(), proj.stride(0), int(v_off),
         _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), state.stride(0), _ptr(step.cu_q),
         _ptr(step.seq_rows), _ptr(o, torch.float32, "o"), step.num_seqs, heads, head_dim, v_head_dim, int(max_seg),
-        int(seg_len), _ptr(seg_state), int(silu), _ptr(work), q32.shape[0], sm_count(q32.device), dtype_code(proj.dtype),
-        _stream()), "retention_chunk")
+        int(seg_len), _ptr(seg_state), int(silu), int(q_off), int(k_off), _ptr(inv_freq, torch.float32, "inv_freq"),
+        _ptr(positions, torch.int32, "positions"), int(rotary_dim), float(k_scale), _ptr(work), tokens, sm_count(proj.device),
+        dtype_code(proj.dtype), _stream()), "retention_chunk")
     return o
+
+
+def retention_walk_supported(head_dim: int, v_head_dim: int, rotary_dim: int, proj, *offsets: int) -> bool:
+    """Whether :func:`retention_chunk` takes q and k from the projection ``proj`` with its columns at ``offsets``."""
+    return (rotary_dim % 8 == 0 and chunk_walk_supported(head_dim, v_head_dim, proj.stride(0), *offsets)
+            and proj.data_ptr() % 16 == 0)
 
 
 def retention_out(o, proj, g_off: int, out, *, heads, v_head_dim, eps):

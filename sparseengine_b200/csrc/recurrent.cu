@@ -1067,7 +1067,10 @@ extern "C" int se_ssm_scan(const float* xbc, const void* proj, int pitch, int dt
     if (entries <= 0) return 0;
     if (H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G) return SE_ERR_ARGUMENT;
     if (N > se::kMaxStateRows || H > 65535) return SE_ERR_UNSUPPORTED;
-    const int lanes = se::row_lanes(N);
+    // Short entries: a state column per lane group.  Longer ones, token after token, are a little faster in the tile kernel, whose
+    // chain per token is shorter (64 heads of 64 x 128, us, lane groups / tiles: one entry of 8 tokens 8.5/10.4, of 16 14.5/12.5,
+    // of 64 43/33; four of 16 19.9/22.7; sixty-four of 1 53/99, of 16 255/278, of 32 479/470, of 64 925/853).
+    const int lanes = tokens <= (long long)(entries * (long long)H >= 148 ? 28 : 10) * entries ? se::row_lanes(N) : 0;
     if (lanes != 0 && (H * P) % 4 == 0 && se::rows_aligned(state, state_pitch, xbc, nullptr)) {
         const int per = se::kRowWarps * (32 / lanes) * 8;
         const dim3 grid(entries, H, se::ceil_div(P, per));

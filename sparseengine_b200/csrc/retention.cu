@@ -441,11 +441,33 @@ retention_seg_fix_kernel(const float* __restrict__ q32, const float* __restrict_
 // ---- prompt portions, chunks prepared side by side (chunk_walk.cuh) --------------------------------
 namespace walk {
 
-// Retention: P[t][s] = decay^(t - s) q_t . k_s, rs = decay^(t + 1), ts = decay^(n - 1 - t).
-template <int DP>
+// What the prepare kernel reads: q and k as columns of the projection, rotated over `rotary` of a head's d columns (split halves;
+// 0: not), k times k_scale; with `silu` the activation comes first.
+template <typename T_>
+struct RetentionInputs {
+    const T_* proj;
+    int pitch, q_off, k_off;
+    const float* inv_freq;
+    const int* positions;
+    int rotary, silu;
+    float k_scale;
+};
+
+template <typename T_>
+__device__ __forceinline__ float4 staged4(const T_* src, int silu) {
+    float4 v = load4(src);
+    if (silu) v = make_float4(input_silu<T_>(v.x), input_silu<T_>(v.y), input_silu<T_>(v.z), input_silu<T_>(v.w));
+    return v;
+}
+
+// Retention: P[t][s] = decay^(t - s) q_t . k_s, rs = decay^(t + 1), ts = decay^(n - 1 - t); q and k as the walk reads them.
+// The rotation happens on the way into shared memory: a (chunk, head) works its angles out itself (a sine and a cosine for 128
+// multiply-adds).  Measured, 8,192 tokens of 32 heads of 128: rotated by a kernel of its own first,
+// 69 + 134 us; here 178, and a launch less (2,048 wide, 17 to 64 tokens: a layer's call 92 and 76 us).
+template <int DP, typename T_>
 __global__ void __launch_bounds__(kThreads, 3)
-retention_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ decay,
-                         const int* __restrict__ cu_q, int entries, float* __restrict__ p, float* __restrict__ rs,
+retention_prepare_kernel(const RetentionInputs<T_> in, const float* __restrict__ decay, const int* __restrict__ cu_q, int entries,
+                         float* __restrict__ q, float* __restrict__ k, float* __restrict__ p, float* __restrict__ rs,
                          float* __restrict__ ts, int H, int d) {
     constexpr int T = 64, QP = DP + 4;
     extern __shared__ __align__(16) float sm[];
@@ -455,13 +477,56 @@ retention_prepare_kernel(const float* __restrict__ q, const float* __restrict__ 
     int first, n;
     chunk_of<T>(blockIdx.x, cu_q, entries, first, n);
     if (n <= 0) return;
-    const int h = blockIdx.y;
-    load_tile<T, DP>(qs, q + (size_t)h * d, H * d, first, n, d);
-    load_tile<T, DP>(ks, k + (size_t)h * d, H * d, first, n, d);
-    cp_commit();
+    const int h = blockIdx.y, half = in.rotary / 2, pairs = half / 4, per = pairs + (d - in.rotary) / 4;
+    for (int x = threadIdx.x; x < T * per; x += kThreads) {
+        const int t = x / per, c = x - t * per, i = c < pairs ? c * 4 : in.rotary + (c - pairs) * 4;
+        float4 q0 = {}, q1 = {}, k0 = {}, k1 = {};
+        if (t < n) {
+            const T_* row = in.proj + (size_t)(first + t) * in.pitch + (size_t)h * d + i;
+            const size_t at = ((size_t)(first + t) * H + h) * d + i;
+            q0 = staged4(row + in.q_off, in.silu);
+            k0 = staged4(row + in.k_off, in.silu);
+            if (c < pairs) {
+                q1 = staged4(row + in.q_off + half, in.silu);
+                k1 = staged4(row + in.k_off + half, in.silu);
+                const float pos = (float)in.positions[first + t];
+                const float4 f = ld4(in.inv_freq + i);
+                auto turn = [&](float freq, float& a, float& b, float& e, float& g) {
+                    float sn, cs;
+                    sincosf(pos * freq, &sn, &cs);
+                    const float a0 = a, e0 = e;
+                    a = a0 * cs - b * sn;
+                    b = b * cs + a0 * sn;
+                    e = e0 * cs - g * sn;
+                    g = g * cs + e0 * sn;
+                };
+                turn(f.x, q0.x, q1.x, k0.x, k1.x);
+                turn(f.y, q0.y, q1.y, k0.y, k1.y);
+                turn(f.z, q0.z, q1.z, k0.z, k1.z);
+                turn(f.w, q0.w, q1.w, k0.w, k1.w);
+                k1 = make_float4(k1.x * in.k_scale, k1.y * in.k_scale, k1.z * in.k_scale, k1.w * in.k_scale);
+                st4(q + at + half, q1);
+                st4(k + at + half, k1);
+            }
+            k0 = make_float4(k0.x * in.k_scale, k0.y * in.k_scale, k0.z * in.k_scale, k0.w * in.k_scale);
+            st4(q + at, q0);
+            st4(k + at, k0);
+        }
+        st4(qs + t * QP + i, q0);
+        st4(ks + t * QP + i, k0);
+        if (c < pairs) {
+            st4(qs + t * QP + half + i, q1);
+            st4(ks + t * QP + half + i, k1);
+        }
+    }
+    if (d < DP)
+        for (int x = threadIdx.x; x < T * (DP - d) / 4; x += kThreads) {
+            const int t = x / ((DP - d) / 4), c = d + (x - t * ((DP - d) / 4)) * 4;
+            st4(qs + t * QP + c, make_float4(0.f, 0.f, 0.f, 0.f));
+            st4(ks + t * QP + c, make_float4(0.f, 0.f, 0.f, 0.f));
+        }
     const double g = (double)decay[h];
     if (threadIdx.x <= T) power[threadIdx.x] = (float)pow(g, (double)threadIdx.x);
-    cp_wait<0>();
     __syncthreads();
     if (threadIdx.x < n) {
         rs[(size_t)(first + threadIdx.x) * H + h] = power[threadIdx.x + 1];
@@ -652,30 +717,37 @@ extern "C" int se_retention_scan(const float* q32, const float* k32, const void*
     SE_LAUNCH_CHECK();
 }
 
-static int launch_retention_walk(const float* q32, const float* k32, const void* proj, int proj_stride, int v_off,
-                                 const float* decay, float* state, long long state_stride, const int* cu_q, const int* seq_rows,
-                                 float* o, float* work, int tokens, int entries, int heads, int d, int dv, int sms, int silu,
-                                 int dtype, cudaStream_t stream) {
+static int launch_retention_walk(const void* proj, int proj_stride, int q_off, int k_off, int v_off, const float* inv_freq,
+                                 const int* positions, int rotary, float k_scale, const float* decay, float* state,
+                                 long long state_stride, const int* cu_q, const int* seq_rows, float* o, float* work, int tokens,
+                                 int entries, int heads, int d, int dv, int sms, int silu, int dtype, cudaStream_t stream) {
     using namespace se::walk;
     if (entries <= 0 || tokens <= 0) return 0;
     if (!takes(d, dv) || heads <= 0 || heads > 65535 || dv / 16 >= 65535) return SE_ERR_UNSUPPORTED;
-    if (proj_stride % 4 || v_off % 4 || !aligned(q32) || !aligned(k32) || !aligned(o) || !aligned(work) || (reinterpret_cast<uintptr_t>(proj) & 15))
+    if (rotary < 0 || rotary > d || rotary % 8 || (rotary && (!inv_freq || !positions || !aligned(inv_freq)))) return SE_ERR_UNSUPPORTED;
+    if (proj_stride % 4 || q_off % 4 || k_off % 4 || v_off % 4 || !aligned(o) || !aligned(work) || (reinterpret_cast<uintptr_t>(proj) & 15))
         return SE_ERR_UNSUPPORTED;
-    float* p = work;
-    float* rs = p + (size_t)tokens * heads * 64;
-    float* ts = rs + (size_t)tokens * heads;
+    const size_t rows = (size_t)tokens * heads;
+    float* q = work;
+    float* k = q + rows * d;
+    float* p = k + rows * d;
+    float* rs = p + rows * 64;
+    float* ts = rs + rows;
     const dim3 grid(tokens / 64 + entries, heads);
-    SE_WALK_DIMS(d, {
-        const int rc = launch(retention_prepare_kernel<DP>, grid, 2 * 64 * (DP + 4) * sizeof(float), stream, q32, k32, decay, cu_q,
-                              entries, p, rs, ts, heads, d);
-        if (rc != 0) return rc;
-        WalkArgs a = {};
-        a.q = q32; a.k = k32; a.qk_stride = heads * d; a.rep = 1; a.v_stride = proj_stride; a.silu = silu;
-        a.p = p; a.rs = rs; a.ts = ts; a.eb = rs; a.state = state; a.state_stride = state_stride; a.s_row = dv; a.s_col = 1; a.o = o;
-        a.cu_q = cu_q; a.seq_rows = seq_rows; a.H = heads; a.d = d; a.dv = dv;
-        const int cols = walk_columns(entries, heads, dv, sms);
-        SE_DISPATCH_DTYPE(dtype, T_, {
-            a.v = static_cast<const T_*>(proj) + v_off;
+    WalkArgs a = {};
+    a.q = q; a.k = k; a.qk_stride = heads * d; a.rep = 1; a.v_stride = proj_stride; a.silu = silu;
+    a.p = p; a.rs = rs; a.ts = ts; a.eb = rs; a.state = state; a.state_stride = state_stride; a.s_row = dv; a.s_col = 1; a.o = o;
+    a.cu_q = cu_q; a.seq_rows = seq_rows; a.H = heads; a.d = d; a.dv = dv;
+    const int cols = walk_columns(entries, heads, dv, sms);
+    SE_DISPATCH_DTYPE(dtype, T_, {
+        RetentionInputs<T_> in;
+        in.proj = static_cast<const T_*>(proj); in.pitch = proj_stride; in.q_off = q_off; in.k_off = k_off; in.inv_freq = inv_freq;
+        in.positions = positions; in.rotary = rotary; in.silu = silu; in.k_scale = k_scale;
+        a.v = in.proj + v_off;
+        SE_WALK_DIMS(d, {
+            const int rc = launch(retention_prepare_kernel<DP, T_>, grid, 2 * 64 * (DP + 4) * sizeof(float), stream, in, decay, cu_q,
+                                  entries, q, k, p, rs, ts, heads, d);
+            if (rc != 0) return rc;
             return launch_walk<64, DP, false, false, T_>(a, entries, cols, stream);
         });
     });
@@ -687,12 +759,14 @@ extern "C" int se_retention_chunk_supported(int d) { return d > 0 && d <= 256; }
 extern "C" int se_retention_chunk(const float* q32, const float* k32, const void* proj, int proj_stride, int v_off,
                                   const float* decay, float* state, long long state_stride, const int* cu_q,
                                   const int* seq_rows, float* o, int entries, int heads, int d, int dv, int max_seg,
-                                  int seg_len, float* seg_state, int silu, float* work, int tokens, int sms, int dtype,
+                                  int seg_len, float* seg_state, int silu, int q_off, int k_off, const float* inv_freq,
+                                  const int* positions, int rotary, float k_scale, float* work, int tokens, int sms, int dtype,
                                   cudaStream_t stream) {
-    // work (float [tokens * heads * (64 + 2)]): chunks prepared side by side and walked; else the forms below.
+    // work (float [tokens * heads * (2 d + 64 + 2)]): q and k from the projection's columns q_off and k_off, rotated on the way;
+    // chunks prepared side by side and walked.  Else the forms below, from q32 and k32.
     if (work != nullptr)
-        return launch_retention_walk(q32, k32, proj, proj_stride, v_off, decay, state, state_stride, cu_q, seq_rows, o, work, tokens,
-                                     entries, heads, d, dv, sms, silu, dtype, stream);
+        return launch_retention_walk(proj, proj_stride, q_off, k_off, v_off, inv_freq, positions, rotary, k_scale, decay, state,
+                                     state_stride, cu_q, seq_rows, o, work, tokens, entries, heads, d, dv, sms, silu, dtype, stream);
     // max_seg > 1: the entries' tokens in segments of seg_len (a multiple of 64) that run side by side, joined by
     // the decay's powers (three launches); seg_state: float [entries, max_seg, heads, d, dv].
     if (entries <= 0) return 0;

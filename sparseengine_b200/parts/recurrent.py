@@ -25,15 +25,21 @@ def _check_state_rows(rows: int, what: str) -> None:
                          "column's rows live in the registers of one warp's lanes)")
 
 
-def takes_chunks(mixer, step, heads: int, columns: int, device) -> bool:
-    """Whether a step's recurrence runs in chunks: its longest entry has ``chunk_min_tokens`` tokens, and its entries average
-    ``chunk_min_average`` (a chunk costs a short entry as much as a full one) or do not fill the device.  Measured at a width
-    of 2,048, both mixers of the hybrid design: 64 prompts of 24 to 48 tokens take 0.9 ms more in chunks, four of 750 to 1,500
-    tokens 0.1 (decays per channel) and 0.8 ms (state space) less."""
-    if mixer.chunk_min_tokens is None or step.max_q_len < mixer.chunk_min_tokens:
+def takes_chunks(mixer, step, heads: int, rows: int, columns: int, prepare: float, device) -> bool:
+    """Whether a step's recurrence runs in chunks: by what either form is estimated to take (us), if the longest entry has
+    ``chunk_min_tokens`` tokens.  Token by token: 0.62 per token of the longest entry, or 5.5e-5 per token and state column of 128
+    rows where the device is full.  In chunks: 15 for the launches, 12 + 6.3 per 64 tokens for each block of 32 columns of an
+    entry, ``prepare`` per token and head.  Measured on one B200 (state space of 64 heads, 64 x 128; delta per channel and per head, 16
+    heads of 128 x 128; us token by token / in chunks): one entry of 32 tokens 24/27, 27/29, 25/29, of 64 43/31, 42/31, 41/35; four of
+    64 62/73, 49/60, 47/58, of 128 118/96, 86/86, 87/85; sixty-four of 64 923/1,074, 514/734, 509/708, of 128 1,817/1,414,
+    1,007/1,128, 997/1,030; one of 2,048 about 850/225, 1,000/480, 1,000/245."""
+    longest = step.max_q_len
+    if mixer.chunk_min_tokens is None or longest < mixer.chunk_min_tokens:
         return False
-    return (step.num_tokens >= mixer.chunk_min_average * step.num_seqs
-            or step.num_seqs * heads * -(-columns // 32) <= ops.sm_count(device))
+    walk = max(0.62 * longest, 4.3e-7 * step.num_tokens * heads * columns * rows)
+    share = heads * -(-columns // 32) / ops.sm_count(device)       # of a full device that an entry's blocks are
+    chunks = max(12 + 0.1 * longest, (12 * step.num_seqs + 0.1 * step.num_tokens) * share)
+    return 15 + chunks + prepare * step.num_tokens * heads < walk
 
 
 class StateSpaceMixer(Mixer):
@@ -42,8 +48,9 @@ class StateSpaceMixer(Mixer):
     ``y = S^T C + D x``; ``y * silu(z)`` RMS-normed in ``norm_groups`` parts, times a weight; out
     projection."""
     graph_safe = True
-    chunk_min_tokens = 16        # the longest entry of a step from which the recurrence runs in chunks; None: never
-    chunk_min_average = 64       # ... if the step's entries average this many tokens, or do not fill the device
+    # The longest entry of a step from which the recurrence may run in chunks; None: never.  Below, the launch that chunks take more
+    # costs a small step, which waits for the host, what the kernels save (a layer's call at 64 tokens: 86 us without, 96 with).
+    chunk_min_tokens = 96
 
     def __init__(self, spec, dtype):
         super().__init__(spec, dtype)
@@ -82,7 +89,7 @@ class StateSpaceMixer(Mixer):
         xbc = torch.empty(tokens, self.conv_channels, dtype=torch.float32, device=x.device)
         ops.causal_conv(proj, self.inner, self.conv_w, self.conv_b, slot.state, self.conv_off, step, xbc)
         y = torch.empty(tokens, self.inner, dtype=torch.float32, device=x.device)
-        walk = (takes_chunks(self, step, s.num_heads, s.head_dim, x.device)
+        walk = (takes_chunks(self, step, s.num_heads, s.state_size, s.head_dim, 2e-4, x.device)
                 and ops.chunk_walk_supported(s.state_size, s.head_dim))
         (ops.ssm_walk if walk else ops.ssm_scan)(
             xbc, proj, self.inner + self.conv_channels, self.dt_bias, self.a_log, self.d_skip, slot.state, step, y,
@@ -102,8 +109,9 @@ class GatedDeltaMixer(Mixer):
     with ``a`` a column of the input projection, and the gate ``gate_activation(g)`` with ``g`` columns of
     the input projection (no low ranks)."""
     graph_safe = True
-    chunk_min_tokens = 16        # the longest entry of a step from which the recurrence runs in chunks; None: never
-    chunk_min_average = 64       # ... if the step's entries average this many tokens, or do not fill the device
+    # The longest entry of a step from which the recurrence may run in chunks; None: never.  Below, token by token is as fast (an entry
+    # of 32 tokens: 27 against 29 us).
+    chunk_min_tokens = 48
 
     def __init__(self, spec, dtype):
         super().__init__(spec, dtype)
@@ -111,6 +119,8 @@ class GatedDeltaMixer(Mixer):
         if s.decay_per not in ("channel", "head") or s.gate_activation not in ("sigmoid", "silu"):
             raise ValueError("decay_per is 'channel' or 'head', gate_activation 'sigmoid' or 'silu'")
         self.per_head = s.decay_per == "head"
+        self.sizes = dict(heads=s.num_heads, kv_heads=s.num_kv_heads, head_dim=s.head_dim, v_head_dim=s.v_head_dim)
+        self.inputs = dict(unit_eps=s.unit_eps, q_scale=s.head_dim ** -0.5, per_head=self.per_head)
         ranks = () if self.per_head else (s.decay_rank, s.gate_rank)
         if min(s.num_heads, s.num_kv_heads, s.head_dim, s.v_head_dim, s.conv_taps, s.hidden_size, *ranks) <= 0:
             raise ValueError("the sizes of a gated-delta mixer must be positive")
@@ -157,10 +167,9 @@ class GatedDeltaMixer(Mixer):
             a, gate = linear(a, self.a2), linear(gate, self.g2)
         # Steps with prompt portions run the recurrence in chunks, prepared side by side and walked (csrc/chunk_walk.cuh); others
         # (single tokens, short pieces, head sizes the chunks do not take) prepare q, k, decays and beta, then walk the tokens.
-        sizes = dict(heads=s.num_heads, kv_heads=s.num_kv_heads, head_dim=s.head_dim, v_head_dim=s.v_head_dim)
-        inputs = dict(unit_eps=s.unit_eps, q_scale=s.head_dim ** -0.5, per_head=self.per_head)
+        sizes, inputs = self.sizes, self.inputs
         o = torch.empty(tokens, self.vv, dtype=torch.float32, device=dev)
-        long = takes_chunks(self, step, s.num_heads, s.v_head_dim, dev)
+        long = takes_chunks(self, step, s.num_heads, s.head_dim, s.v_head_dim, 2.1e-3 if self.per_head else 2.5e-3, dev)
         if long and ops.chunk_walk_supported(s.head_dim, s.v_head_dim):
             ops.delta_walk(qkv, a, proj, self.b_off, self.dt_bias, self.a_log, slot.state, step, o, **sizes, **inputs)
         else:
@@ -257,6 +266,12 @@ class RetentionMixer(Mixer):
         sizes = dict(heads=s.num_heads, head_dim=s.head_dim, v_head_dim=s.v_head_dim, silu=silu)
         if not chunked and rotary_dim == 0:      # q and k straight from the projection, as they are staged
             ops.retention_scan(None, None, *args, **sizes, qk=(0, self.qk, self.k_scale))
+        elif (chunked and ops.retention_walk_supported(s.head_dim, s.v_head_dim, rotary_dim, proj, self.qk)
+              # entries of one chunk that fill the device go faster through the kernel that does a chunk at a time (a layer of 32 heads
+              # of 128 x 128, four entries of 17 to 64 tokens: 118 to 135 us against 124 to 143; one entry: 87 against 76)
+              and (step.max_q_len > 64 or step.num_seqs * s.num_heads * (-(-s.v_head_dim // 32)) <= ops.sm_count(dev))):
+            ops.retention_chunk(None, None, *args, **sizes, qk=(0, self.qk, self.k_scale),
+                                rotation=(inv_freq, rotary_dim, step.positions) if rotary_dim else None)
         else:
             q32 = torch.empty(tokens, self.qk, dtype=torch.float32, device=dev)
             k32 = torch.empty(tokens, self.qk, dtype=torch.float32, device=dev)

@@ -66,10 +66,22 @@ def test_chunks_against_the_walk(kind, d, dv, heads, kv_heads, decay):
     column_major = kind != "retention"          # [head][column][row], retention [head][row][column]
     skip = None
     if kind == "retention":
-        q, k, v = rnd(T, heads, d), rnd(T, heads, d) * d ** -0.5, rnd(T, heads * dv + 8).to(torch.bfloat16)
-        decays = torch.exp(logs[0, :, 0])
-        ops.retention_chunk(q.view(T, -1), k.view(T, -1), v, 4, decays, state, step, o.view(T, -1), silu=True, **sizes)
-        v = torch.nn.functional.silu(v[:, 4:4 + heads * dv].double()).view(T, heads, dv)
+        # columns: 4 that nobody reads, k, values, q; rotated where the head size allows the pairs
+        wide, rot = heads * (2 * d + dv) + 8, 16 if d >= 16 else 0
+        proj, decays = rnd(T, wide + -wide % 4).to(torch.bfloat16), torch.exp(logs[0, :, 0])
+        inv, positions = torch.rand(rot // 2, generator=g, device=DEV), torch.arange(T, device=DEV, dtype=torch.int32) * 37 % 101
+        v_off = 4 + heads * d
+        q_off = v_off + heads * dv
+        assert ops.retention_walk_supported(d, dv, rot, proj, q_off, 4, v_off)
+        ops.retention_chunk(None, None, proj, v_off, decays, state, step, o.view(T, -1), silu=True, **sizes,
+                            qk=(q_off, 4, d ** -0.5), rotation=(inv, rot, positions) if rot else None)
+        x = torch.nn.functional.silu(proj.double())
+        q, k = (x[:, f:f + heads * d].reshape(T, heads, d).clone() for f in (q_off, 4))
+        angle = (positions.float()[:, None] * inv).double()[:, None]        # the product in 32-bit, as positions are encoded
+        for z in (q, k):
+            lo, hi = z[..., :rot // 2].clone(), z[..., rot // 2:rot].clone()
+            z[..., :rot // 2], z[..., rot // 2:rot] = lo * angle.cos() - hi * angle.sin(), hi * angle.cos() + lo * angle.sin()
+        k, v = k * d ** -0.5, x[:, v_off:v_off + heads * dv].view(T, heads, dv)
         keep, beta = decays.double().view(1, heads, 1).expand(T, -1, -1), None
     elif kind.startswith("state space"):
         width = heads * dv + 2 * kv_heads * d
