@@ -109,3 +109,36 @@ def test_routed_products(counts, hidden, inter, activation):
     want = part.run_experts(x, ids, weights)
     # sums of at most 260 products of size one in another order
     assert float((got - want).abs().max()) < 4e-6 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("options", [{}, dict(window=37, keep_first=6), dict(softcap=3.0, sink=True)], ids=["plain", "window, kept", "cap, sink"])
+@pytest.mark.parametrize("copies", [1, 8, 64])             # few and many blocks: 16, 8 and 4 warps to a token's keys
+@pytest.mark.parametrize("d,dv,heads,kv_heads", [(128, 128, 6, 1), (132, 68, 2, 2), (20, 140, 4, 2), (256, 256, 4, 1)])
+def test_single_tokens(d, dv, heads, kv_heads, copies, options):
+    """Single tokens that see 1 to 200 keys (groups of four keys, partly empty) against 64-bit sums."""
+    from sparseengine_b200.csrc import ops
+    held, page = [1, 2, 3, 5, 16, 63, 64, 65, 68, 200] * copies, 8
+    b = _batch([1] * len(held), held, page, d)
+    g = torch.Generator(device=DEV).manual_seed(d)
+    cache = torch.randn(b["pages"], page * kv_heads * (d + dv), generator=g, device=DEV)
+    q, out = torch.randn(len(held), heads * d, generator=g, device=DEV), torch.empty(len(held), heads * dv, device=DEV)
+    ops.paged_attention_plain(q, cache, b["table"], b["rows"], b["seq"], b["pos"], out, num_heads=heads, num_kv_heads=kv_heads, head_dim=d,
+                              v_head_dim=dv, page_size=page, scale=d ** -0.5, **options)
+    ops.error_check(DEV)
+    for e in range(10):
+        n = held[e]
+        pages = cache[b["table"][b["rows"][e].long()].long()].double()
+        k = pages[:, :page * kv_heads * d].view(-1, kv_heads, page, d).transpose(1, 2).reshape(-1, kv_heads, d)[:n]
+        v = pages[:, page * kv_heads * d:].view(-1, kv_heads, page, dv).transpose(1, 2).reshape(-1, kv_heads, dv)[:n]
+        k, v = (x.repeat_interleave(heads // kv_heads, 1) for x in (k, v))
+        s = torch.einsum("hd,nhd->hn", q[e].view(heads, d).double(), k) * d ** -0.5
+        if options.get("softcap"):
+            s = 3.0 * torch.tanh(s / 3.0)
+        if options.get("window"):
+            i = torch.arange(n, device=DEV)
+            s = s.masked_fill((i < n - 37) & (i >= 6), float("-inf"))
+        if options.get("sink"):
+            s = torch.cat([s, torch.zeros(heads, 1, dtype=s.dtype, device=DEV)], 1)
+        want = torch.einsum("hn,nhd->hd", torch.softmax(s, 1)[:, :n], v)
+        # sums over at most 256 products and 200 keys of size one; the scores' error enters through the exponential
+        assert float((out[e].view(heads, dv).double() - want).abs().max()) < 4e-6 * max(1.0, float(want.abs().max()))
