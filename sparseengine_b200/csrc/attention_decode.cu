@@ -6,6 +6,11 @@
 // running softmax state in 32-bit and are merged at the end; key splits are merged by a
 // second kernel through their log-sum-exp.
 //
+// With eight warps on an SM it is the warps' own instructions, one behind the other, that bound it before the memory does: so a
+// tile's rows are looked up once, ahead, the copies and ldmatrix reads step by constants, and the output is rescaled only where a
+// maximum moved.  Measured, 64 requests of 1,500 to 3,000 keys, 48 heads over 8 of 128 (590 MB, 89 us at 6.65 TB/s): rows looked
+// up by every thread 181 us, ahead 154, with the rest 125.
+//
 // Arithmetic as in the plain kernel and the reference's split-KV decode
 // (src/sparseengine/kernels/triton/gqa_flash_decoding_stage1.py:69-120,
 // src/sparseengine/kernels/triton/flash_decoding_stage2.py:27-45): scores and softmax in
@@ -28,7 +33,7 @@ namespace se {
 namespace dec {
 
 constexpr int kTileKeys = 64;
-constexpr int kStages = 3;
+constexpr int kStages = 3;       // row_at holds kStages + 1 tiles
 constexpr int kWarps = 4;
 constexpr int kThreads = 32 * kWarps;
 
@@ -78,40 +83,80 @@ attn_decode_kernel(const __nv_bfloat16* q, const __nv_bfloat16* cache,      // w
 
     const int num_tiles = ks < ke ? (ke - ks + kTileKeys - 1) / kTileKeys : 0;
 
-    // Rows [64][DIM] of a tile: a thread copies chunk (tid % chunks) of rows tid / chunks + k * (kThreads / chunks).
-    // The rows' addresses are looked up first (independent loads), so that no table load sits
-    // between the asynchronous copies.  `off`: where the head's rows start in a page; `dim` elements a
-    // row in memory, DIM in the tile.
-    auto load_rows = [&](auto dim_tag, int dim, uint8_t* dst, int base, size_t off) {
-        constexpr int DIM = decltype(dim_tag)::value;
-        constexpr int kChunks = DIM / 8;                 // 16-byte chunks per row
-        constexpr int kRowStep = kThreads / kChunks, kIters = kTileKeys / kRowStep;
-        static_assert(kThreads % kChunks == 0 && kTileKeys % kRowStep == 0, "tile copy mapping");
-        const int c = threadIdx.x % kChunks, r0t = threadIdx.x / kChunks;
-        const bool col_ok = !PAD || c * 8 < dim;
-        const __nv_bfloat16* srcs[kIters];
-        bool page_ok[kIters];
-#pragma unroll
-        for (int k = 0; k < kIters; ++k) {
-            const int j = base + r0t + k * kRowStep;
-            const int jj = key_of(j < ke ? j : ks);      // any valid key: the copy is zero-filled when out of range
-            const int page = row_table[jj / page_size];
-            // an entry that names no page of the pool is not followed: its rows are zero-filled
-            page_ok[k] = page_in_pool(page, num_pages, error, SE_CODE_BAD_PAGE_ATTN_DECODE);
-            srcs[k] = cache + (size_t)(page_ok[k] ? page : 0) * page_elems + off + (size_t)(jj % page_size) * dim + (col_ok ? c * 8 : 0);
+    // Where the rows of the tiles ahead lie (key, value; null: a row of zeros), looked up by one thread per row three tiles before
+    // they are used, so that neither the table's latency nor the divisions by the page size stand between the copies; and whether a
+    // warp's half of a tile has no row of zeros.
+    using RowPtr = unsigned long long;
+    __shared__ __align__(16) ulonglong2 row_at[4][kTileKeys];
+    __shared__ int whole[4][2];
+    struct Place { int page, slot; };
+    auto look = [&](int tile) {
+        const int j = ks + tile * kTileKeys + (int)threadIdx.x;
+        Place p{0, -1};
+        if (threadIdx.x < kTileKeys && tile < num_tiles && j < ke) {
+            const int jj = key_of(j), at = jj / page_size;
+            p.slot = jj - at * page_size;
+            p.page = row_table[at];
         }
+        return p;
+    };
+    auto keep = [&](int tile, Place p) {
+        if (threadIdx.x >= kTileKeys) return;            // two whole warps go on
+        ulonglong2 v = make_ulonglong2(0, 0);
+        // an entry that names no page of the pool is not followed: its rows are zero-filled
+        const bool ok = p.slot >= 0 && page_in_pool(p.page, num_pages, error, SE_CODE_BAD_PAGE_ATTN_DECODE);
+        if (ok) {
+            const __nv_bfloat16* page = cache + (size_t)p.page * page_elems;
+            v = make_ulonglong2((RowPtr)(page + head_off + (size_t)p.slot * d_real), (RowPtr)(page + v_off + (size_t)p.slot * dv_real));
+        }
+        row_at[tile & 3][threadIdx.x] = v;
+        const int all = __all_sync(0xffffffffu, ok);
+        if (lane == 0) whole[tile & 3][warp] = all;
+    };
+    // A tile's rows: a thread copies chunk (tid % chunks) of rows tid / chunks + k * (kThreads / chunks); `dim` elements a row in
+    // memory, DIM in the tile.  The rows step by whole swizzle periods, so a thread's places in the tile are a constant apart.
+    auto copy_row = [&](auto dim_tag, int dim, bool full, uint32_t to, int k, RowPtr row) {
+        constexpr int DIM = decltype(dim_tag)::value;
+        constexpr int kChunks = DIM / 8, kRowStep = kThreads / kChunks;
+        static_assert(kThreads % kChunks == 0 && kTileKeys % kRowStep == 0 && kRowStep % (kChunks < 8 ? kChunks : 8) == 0, "tile copy mapping");
+        const int c = threadIdx.x % kChunks;
+        const bool ok = full || (row != 0 && (!PAD || c * 8 < dim));
+        const RowPtr src = full || ok ? row + c * 16 : (RowPtr)cache;
+        cp_async16(to + k * (kRowStep * DIM * 2), reinterpret_cast<const void*>(src), ok);
+    };
+    auto copy_tile = [&](int tile, uint32_t kbase, bool full) {
+        const ulonglong2* at = row_at[tile & 3];
+        constexpr int kChunksK = D / 8, kChunksV = DV / 8, kStepK = kThreads / kChunksK, kStepV = kThreads / kChunksV;
+        const int rk = threadIdx.x / kChunksK, rv = threadIdx.x / kChunksV;
+        const uint32_t to_k = kbase + tile_off<D>(rk, threadIdx.x % kChunksK);
+        const uint32_t to_v = kbase + kTileBytes + tile_off<DV>(rv, threadIdx.x % kChunksV);
+        if constexpr (D == DV) {
 #pragma unroll
-        for (int k = 0; k < kIters; ++k) {
-            const int r = r0t + k * kRowStep;
-            cp_async16(smem_u32(dst) + tile_off<DIM>(r, c), srcs[k], base + r < ke && page_ok[k] && col_ok);
+            for (int k = 0; k < kTileKeys / kStepK; ++k) {
+                const ulonglong2 row = at[rk + k * kStepK];
+                copy_row(std::integral_constant<int, D>{}, d_real, full, to_k, k, row.x);
+                copy_row(std::integral_constant<int, DV>{}, dv_real, full, to_v, k, row.y);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < kTileKeys / kStepK; ++k) copy_row(std::integral_constant<int, D>{}, d_real, full, to_k, k, at[rk + k * kStepK].x);
+#pragma unroll
+            for (int k = 0; k < kTileKeys / kStepV; ++k) copy_row(std::integral_constant<int, DV>{}, dv_real, full, to_v, k, at[rv + k * kStepV].y);
         }
     };
     auto load_tile = [&](int tile, int stage) {
-        uint8_t* kbase = smem + (size_t)stage * kStageBytes;
-        const int base = ks + tile * kTileKeys;
-        load_rows(std::integral_constant<int, D>{}, d_real, kbase, base, head_off);
-        load_rows(std::integral_constant<int, DV>{}, dv_real, kbase + kTileBytes, base, v_off);
+        const uint32_t kbase = smem_u32(smem) + stage * kStageBytes;
+        if (!PAD && whole[tile & 3][0] && whole[tile & 3][1]) copy_tile(tile, kbase, true);
+        else copy_tile(tile, kbase, false);
     };
+    {
+        Place p[kStages];
+#pragma unroll
+        for (int s = 0; s < kStages; ++s) p[s] = look(s);
+#pragma unroll
+        for (int s = 0; s < kStages; ++s) keep(s, p[s]);
+    }
+    __syncthreads();
 
     // Where the step's inputs are older than the kernel before this one (the one that writes the
     // queries and this step's keys), this kernel is launched as its dependent and may have come
@@ -141,12 +186,18 @@ attn_decode_kernel(const __nv_bfloat16* q, const __nv_bfloat16* cache,      // w
         cp_async_commit();
     }
 
+    // where this lane's ldmatrix rows begin in a tile; two chunks on is an exclusive or with 32 in the swizzled row
+    const int mat = lane >> 3, rr = lane & 7;
+    const uint32_t k_frag = tile_off<D>(warp * 16 + (mat >> 1) * 8 + rr, mat & 1);
+    const uint32_t v_frag = tile_off<DV>(warp * 16 + (mat & 1) * 8 + rr, mat >> 1);
+
     for (int tile = 0; tile < num_tiles; ++tile) {
         cp_async_wait<kStages - 2>();
         __syncthreads();
         // prefetch the tile that reuses the stage everyone has just finished with
         if (tile + kStages - 1 < num_tiles) load_tile(tile + kStages - 1, (tile + kStages - 1) % kStages);
         cp_async_commit();
+        const Place ahead = look(tile + kStages);
 
         const int stage = tile % kStages;
         const uint32_t kaddr = smem_u32(smem + (size_t)stage * kStageBytes);
@@ -158,8 +209,7 @@ attn_decode_kernel(const __nv_bfloat16* q, const __nv_bfloat16* cache,      // w
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
                 uint32_t b0, b1, b2, b3;
-                const int mat = lane >> 3, rr = lane & 7;
-                ldmatrix_x4(kaddr + tile_off<D>(r0 + (mat >> 1) * 8 + rr, 2 * kk + (mat & 1)), b0, b1, b2, b3);
+                ldmatrix_x4(kaddr + (k_frag ^ (kk * 32)), b0, b1, b2, b3);
                 mma_bf16(s[0], qa[kk], b0, b1);
                 mma_bf16(s[1], qa[kk], b2, b3);
             }
@@ -208,20 +258,22 @@ attn_decode_kernel(const __nv_bfloat16* q, const __nv_bfloat16* cache,      // w
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) l_run[h] = l_run[h] * corr[h] + psum[h];
+            if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {       // most tiles move no row's maximum
 #pragma unroll
-            for (int i = 0; i < DV / 8; ++i) {
-                o[i][0] *= corr[0]; o[i][1] *= corr[0];
-                o[i][2] *= corr[1]; o[i][3] *= corr[1];
+                for (int i = 0; i < DV / 8; ++i) {
+                    o[i][0] *= corr[0]; o[i][1] *= corr[0];
+                    o[i][2] *= corr[1]; o[i][3] *= corr[1];
+                }
             }
 #pragma unroll
             for (int n2 = 0; n2 < DV / 16; ++n2) {      // two 8-wide dim tiles per ldmatrix
                 uint32_t b0, b1, b2, b3;
-                const int mat = lane >> 3, rr = lane & 7;
-                ldmatrix_x4_trans(vaddr + tile_off<DV>(r0 + (mat & 1) * 8 + rr, 2 * n2 + (mat >> 1)), b0, b1, b2, b3);
+                ldmatrix_x4_trans(vaddr + (v_frag ^ (n2 * 32)), b0, b1, b2, b3);
                 mma_bf16(o[2 * n2], pa, b0, b1);
                 mma_bf16(o[2 * n2 + 1], pa, b2, b3);
             }
         }
+        keep(tile + kStages, ahead);
     }
     cp_async_wait<0>();
     __syncthreads();
