@@ -81,8 +81,11 @@ KERNEL_TUNING_KEYS = {
     "gemv_max_rows": None,                                              # ... and so do projections of more rows than this
     "router_tensor_core_min_tokens": "split_router_min_tokens",         # prompt steps from this size take router logits from tensor cores
     "moe_pair_min_rows": "pair_min_rows",                               # (token, slot) rows from which experts may run on pairs of SMs
-    "moe_pair_min_rows_per_expert": "pair_min_rows_per_expert",
-    "retention_chunk_min_tokens": "chunk_min_tokens",                   # steps whose longest entry has this many tokens take the chunked recurrence         # ... if the experts that get rows have this many each
+    "moe_pair_min_rows_per_expert": "pair_min_rows_per_expert",         # ... if the experts that get rows have this many each
+    # steps whose longest entry has this many tokens take the chunked recurrence: retention, matrix memory and minGRU, which choose by
+    # that number alone; the state-space mixer and the delta rules, which otherwise estimate what either form takes
+    "retention_chunk_min_tokens": "chunk_min_tokens",
+    "recurrence_chunk_min_tokens": "chunk_min_tokens",
 }
 
 
@@ -109,5 +112,7 @@ def apply_kernel_tuning(model: Model, tuning: dict) -> None:
         for b in model.blocks:
             for part in b.parts().values():
                 for p in (part, *getattr(part, "branches", ())):        # a mixer of mixers: its branches too
-                    if hasattr(p, attr):
+                    if hasattr(p, attr) and getattr(p, "chunk_tuning_key", key) == key:
                         setattr(p, attr, int(value))
+                        if key == "recurrence_chunk_min_tokens":
+                            p.chunks_by_estimate = False

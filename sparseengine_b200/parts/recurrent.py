@@ -27,8 +27,8 @@ def _check_state_rows(rows: int, what: str) -> None:
 
 def takes_chunks(mixer, step, heads: int, rows: int, columns: int, prepare: float, device) -> bool:
     """Whether a step's recurrence runs in chunks: by what either form is estimated to take (us), if the longest entry has
-    ``chunk_min_tokens`` tokens.  Token by token: 0.62 per token of the longest entry, or 5.5e-5 per token and state column of 128
-    rows where the device is full.  In chunks: 15 for the launches, 12 + 6.3 per 64 tokens for each block of 32 columns of an
+    ``chunk_min_tokens`` tokens (by that number alone where ``chunks_by_estimate`` is off).  Token by token: 0.62 per token of the
+    longest entry, or 5.5e-5 per token and state column of 128 rows where the device is full.  In chunks: 15 for the launches, 12 + 6.3 per 64 tokens for each block of 32 columns of an
     entry, ``prepare`` per token and head.  Measured on one B200 (state space of 64 heads, 64 x 128; delta per channel and per head, 16
     heads of 128 x 128; us token by token / in chunks): one entry of 32 tokens 24/27, 27/29, 25/29, of 64 43/31, 42/31, 41/35; four of
     64 62/73, 49/60, 47/58, of 128 118/96, 86/86, 87/85; sixty-four of 64 923/1,074, 514/734, 509/708, of 128 1,817/1,414,
@@ -36,6 +36,8 @@ def takes_chunks(mixer, step, heads: int, rows: int, columns: int, prepare: floa
     longest = step.max_q_len
     if mixer.chunk_min_tokens is None or longest < mixer.chunk_min_tokens:
         return False
+    if not getattr(mixer, "chunks_by_estimate", True):
+        return True
     walk = max(0.62 * longest, 4.3e-7 * step.num_tokens * heads * columns * rows)
     share = heads * -(-columns // 32) / ops.sm_count(device)       # of a full device that an entry's blocks are
     chunks = max(12 + 0.1 * longest, (12 * step.num_seqs + 0.1 * step.num_tokens) * share)
@@ -51,6 +53,7 @@ class StateSpaceMixer(Mixer):
     # The longest entry of a step from which the recurrence may run in chunks; None: never.  Below, the launch that chunks take more
     # costs a small step, which waits for the host, what the kernels save (a layer's call at 64 tokens: 86 us without, 96 with).
     chunk_min_tokens = 96
+    chunk_tuning_key = "recurrence_chunk_min_tokens"     # the engine option that sets it (and switches the estimate off)
 
     def __init__(self, spec, dtype):
         super().__init__(spec, dtype)
@@ -112,6 +115,7 @@ class GatedDeltaMixer(Mixer):
     # The longest entry of a step from which the recurrence may run in chunks; None: never.  Below, token by token is as fast (an entry
     # of 32 tokens: 27 against 29 us).
     chunk_min_tokens = 48
+    chunk_tuning_key = "recurrence_chunk_min_tokens"     # the engine option that sets it (and switches the estimate off)
 
     def __init__(self, spec, dtype):
         super().__init__(spec, dtype)
@@ -202,6 +206,7 @@ class RetentionMixer(Mixer):
     input_projection = "in_proj"
     graph_safe = True
     chunk_min_tokens = 16        # the longest entry of a step from which the chunked kernel runs; None: never
+    chunk_tuning_key = "retention_chunk_min_tokens"
 
     def __init__(self, spec, dtype):
         super().__init__(spec, dtype)
@@ -293,6 +298,7 @@ class MatrixMemoryMixer(Mixer):
     then the maximum per head."""
     graph_safe = True
     chunk_min_tokens = 16        # the longest entry of a step from which the chunked kernel runs; None: never
+    chunk_tuning_key = "retention_chunk_min_tokens"
 
     def __init__(self, spec, dtype):
         super().__init__(spec, dtype)
@@ -351,6 +357,7 @@ class MinGRUMixer(Mixer):
     csrc/min_gru.cu).  The state is one 32-bit row of ``width`` numbers per request."""
     graph_safe = True
     chunk_min_tokens = 8         # the longest entry of a step from which the chunked kernel runs; None: never
+    chunk_tuning_key = "retention_chunk_min_tokens"
 
     def __init__(self, spec, dtype):
         super().__init__(spec, dtype)

@@ -160,3 +160,25 @@ def test_kernel_tuning_options_are_checked_and_reach_the_parts():
     finally:
         linear.GEMV_MAX_ROWS, linear.GEMV_MAX_OUT = before
     assert set(KERNEL_TUNING_KEYS) >= {"router_tensor_core_min_tokens", "moe_pair_min_rows_per_expert"}
+
+
+def test_the_retention_key_leaves_the_other_recurrences_alone():
+    """Each chunk threshold reaches the recurrences that it names, and theirs decides without the estimate."""
+    from types import SimpleNamespace
+
+    from sparseengine_b200.engine.factory import apply_kernel_tuning
+    from sparseengine_b200.parts import recurrent
+    kinds = [recurrent.StateSpaceMixer, recurrent.GatedDeltaMixer, recurrent.RetentionMixer, recurrent.MatrixMemoryMixer, recurrent.MinGRUMixer]
+    parts = [object.__new__(k) for k in kinds]
+    model = SimpleNamespace(blocks=[SimpleNamespace(parts=lambda p=p: {"mixer": p}) for p in parts])
+    before = [k.chunk_min_tokens for k in kinds]
+    apply_kernel_tuning(model, {"retention_chunk_min_tokens": 7})
+    assert [p.chunk_min_tokens for p in parts] == before[:2] + [7, 7, 7]
+    apply_kernel_tuning(model, {"recurrence_chunk_min_tokens": 5})
+    assert [p.chunk_min_tokens for p in parts] == [5, 5, 7, 7, 7]
+    step = SimpleNamespace(max_q_len=5, num_tokens=320, num_seqs=64)
+    for p in parts[:2]:
+        assert recurrent.takes_chunks(p, step, 64, 128, 64, 1.0, "cuda:0")
+        step.max_q_len = 4
+        assert not recurrent.takes_chunks(p, step, 64, 128, 64, 1.0, "cuda:0")
+        step.max_q_len = 5
