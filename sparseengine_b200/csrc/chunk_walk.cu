@@ -5,6 +5,19 @@
 namespace se {
 namespace walk {
 
+// The sum of the lanes' `own` (returned) and, in `before`, that of the lanes below: shifted, not the sum less `own`, so that a
+// lane's infinity or NaN reaches no prefix but those of the lanes above.
+__device__ __forceinline__ double sum_before(double own, int lane, double& before) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double v = __shfl_up_sync(0xffffffffu, own, o);
+        if (lane >= o) own += v;
+    }
+    before = __shfl_up_sync(0xffffffffu, own, 1);
+    if (lane == 0) before = 0.0;
+    return __shfl_sync(0xffffffffu, own, 31);
+}
+
 // State space: one block per (chunk, group of heads that share B and C).  step = softplus(raw + bias), the log decay is
 // -exp(A_log) step; P[t][s] = e^(B_t - B_s) C_t . B_s; the step sizes become the factor on the value rows.
 template <int DP, typename T_>
@@ -42,14 +55,8 @@ ssm_prepare_kernel(const float* __restrict__ xbc, const T_* __restrict__ proj, i
                 step[j] = t < n ? softplus32(to_float(proj[(size_t)(first + t) * pitch + dt_off + h]) + bias) : 0.f;
                 sum[j] = -(double)rate * (double)step[j] + (j ? sum[0] : 0.0);
             }
-            double before = sum[1];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const double v = __shfl_up_sync(0xffffffffu, before, o);
-                if (lane >= o) before += v;
-            }
-            const double last = __shfl_sync(0xffffffffu, before, 31);
-            before -= sum[1];
+            double before;
+            const double last = sum_before(sum[1], lane, before);
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int t = 2 * lane + j;
@@ -153,14 +160,8 @@ delta_head_prepare_kernel(const DeltaInputs<T_> in, float* __restrict__ p, float
             sum[j] = (t < n ? -rate * (double)softplus32(to_float(in.a[row * in.a_pitch + h]) + bias) : 0.0) + (j ? sum[0] : 0.0);
             bt[t] = t < n ? sigmoid32(to_float(in.b[row * in.b_pitch + h])) : 0.f;
         }
-        double before = sum[1];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double v = __shfl_up_sync(0xffffffffu, before, o);
-            if (lane >= o) before += v;
-        }
-        const double last = __shfl_sync(0xffffffffu, before, 31);
-        before -= sum[1];
+        double before;
+        const double last = sum_before(sum[1], lane, before);
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const int t = 2 * lane + j;

@@ -149,3 +149,63 @@ def test_later_tokens_do_not_touch_earlier_ones(kind):
                        unit_eps=1e-6, q_scale=0.1, per_head=kind == "per head")
         outs.append(o)
     assert torch.equal(outs[0][:41], outs[1][:41]) and not bool(torch.isfinite(outs[1][41:]).all())
+
+
+def _one_entry(T):
+    i32 = dict(dtype=torch.int32, device=DEV)
+    return SimpleNamespace(cu_q=torch.tensor([0, T], **i32), seq_rows=torch.zeros(1, **i32), num_seqs=1, max_q_len=T, num_tokens=T)
+
+
+def _inputs(kind, T, H, d):
+    """What a kind of recurrence reads, and where its q, k, v and decay (or step) inputs of head 0 lie."""
+    g = torch.Generator(device=DEV).manual_seed(1)
+    cols = H * (d if kind == "delta, per channel" else 1)
+    x = {"qkv": torch.randn(T, 3 * H * d, generator=g, device=DEV), "decay": torch.randn(T, cols, generator=g, device=DEV),
+         "beta": torch.randn(T, H, generator=g, device=DEV), "bias": torch.zeros(cols, device=DEV), "a_log": torch.zeros(H, device=DEV),
+         "skip": torch.ones(H, device=DEV)}
+    q, k, v = (2 * H * d, H * d, 0) if kind == "state space" else (0, H * d, 2 * H * d)       # there: values, keys, queries
+    return x, {"q": ("qkv", q + 3), "k": ("qkv", k + 3), "v": ("qkv", v + 3), "decay": ("decay", 0)}
+
+
+def _outputs(kind, x, H, d, tokens=False):
+    """Outputs and the state after them, from a state of zeros; ``tokens``: by the kernels that walk token by token."""
+    from sparseengine_b200.csrc import ops
+    T = x["qkv"].shape[0]
+    step, o, state = _one_entry(T), torch.empty(T, H * d, device=DEV), torch.zeros(1, H * d * d, device=DEV)
+    if kind == "state space":
+        (ops.ssm_scan if tokens else ops.ssm_walk)(x["qkv"], x["decay"], 0, x["bias"], x["a_log"], x["skip"], state, step, o, heads=H,
+                                                   head_dim=d, state_size=d, groups=H)
+    elif kind == "retention":
+        ops.retention_chunk(None, None, x["qkv"], 2 * H * d, torch.full((H,), 0.9, device=DEV), state, step, o, heads=H, head_dim=d,
+                            v_head_dim=d, qk=(0, H * d, 1.0))
+    else:
+        sizes = dict(heads=H, kv_heads=H, head_dim=d, v_head_dim=d)
+        inputs = dict(unit_eps=1e-6, q_scale=0.1, per_head=kind == "delta, per head")
+        if tokens:
+            qkv, dec, beta = x["qkv"].clone(), torch.empty(T, H * d, device=DEV), torch.empty(T, H, device=DEV)
+            ops.delta_prep(qkv, x["decay"], x["beta"], 0, x["bias"], x["a_log"], dec, beta, **sizes, **inputs)
+            ops.delta_scan(qkv, dec, beta, state, step, o, **sizes)
+        else:
+            ops.delta_walk(x["qkv"], x["decay"], x["beta"], 0, x["bias"], x["a_log"], state, step, o, **sizes, **inputs)
+    return o, state
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("token", [40, 41, 63])         # the first and the second of a pair of tokens, the last of a chunk
+@pytest.mark.parametrize("where", ["q", "k", "v", "decay"])
+@pytest.mark.parametrize("kind", ["state space", "delta, per head", "delta, per channel", "retention"])
+def test_inputs_that_are_not_finite_stay_with_their_token_and_later_ones(kind, where, token, value):
+    if kind == "retention" and where == "decay":
+        pytest.skip("its decays are constants")
+    H, d, T = 2, 64, 70
+    x, places = _inputs(kind, T, H, d)
+    want, _ = _outputs(kind, x, H, d)
+    name, column = places[where]
+    x[name][token, column] = value
+    got, _ = _outputs(kind, x, H, d)
+    assert torch.equal(got[:token], want[:token])
+    assert torch.equal(got[:, d:], want[:, d:])                  # the other head
+    if where == "q":
+        assert not bool(torch.isfinite(got[token, :d]).any()) and torch.equal(got[token + 1:], want[token + 1:])
+    elif where != "decay" or value != value:                     # an infinite step may be a decay of 0
+        assert not bool(torch.isfinite(got[token:, :d]).all(1).any())
