@@ -5,6 +5,14 @@
 namespace se {
 namespace walk {
 
+// A token's log decay, -rate * step, no further down than -1e4: a decay below e^-104 is 0 in 32-bit, and with an infinite rate or step
+// the sums would be infinite and their differences NaN.  Sums of 64 such terms differ by less than 1e-10 from what they should.  NaN
+// stays NaN.
+__device__ __forceinline__ double log_decay(float rate, float step) {
+    const double v = -(double)rate * (double)step;
+    return v < -1e4 ? -1e4 : v;
+}
+
 // The sum of the lanes' `own` (returned) and, in `before`, that of the lanes below: shifted, not the sum less `own`, so that a
 // lane's infinity or NaN reaches no prefix but those of the lanes above.
 __device__ __forceinline__ double sum_before(double own, int lane, double& before) {
@@ -53,7 +61,7 @@ ssm_prepare_kernel(const float* __restrict__ xbc, const T_* __restrict__ proj, i
             for (int j = 0; j < 2; ++j) {
                 const int t = 2 * lane + j;
                 step[j] = t < n ? softplus32(to_float(proj[(size_t)(first + t) * pitch + dt_off + h]) + bias) : 0.f;
-                sum[j] = -(double)rate * (double)step[j] + (j ? sum[0] : 0.0);
+                sum[j] = (t < n ? log_decay(rate, step[j]) : 0.0) + (j ? sum[0] : 0.0);
             }
             double before;
             const double last = sum_before(sum[1], lane, before);
@@ -150,14 +158,14 @@ delta_head_prepare_kernel(const DeltaInputs<T_> in, float* __restrict__ p, float
     cp_commit();
     float after[2] = {};
     if (warp == 0) {                                 // two neighbouring tokens per lane
-        const double rate = (double)expf(in.a_log[h]);
+        const float rate = expf(in.a_log[h]);
         const float bias = in.dt_bias[h];
         double sum[2];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const int t = 2 * lane + j;
             const size_t row = (size_t)(first + t);
-            sum[j] = (t < n ? -rate * (double)softplus32(to_float(in.a[row * in.a_pitch + h]) + bias) : 0.0) + (j ? sum[0] : 0.0);
+            sum[j] = (t < n ? log_decay(rate, softplus32(to_float(in.a[row * in.a_pitch + h]) + bias)) : 0.0) + (j ? sum[0] : 0.0);
             bt[t] = t < n ? sigmoid32(to_float(in.b[row * in.b_pitch + h])) : 0.f;
         }
         double before;

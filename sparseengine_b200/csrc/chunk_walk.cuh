@@ -13,8 +13,8 @@
 // products per chunk instead of a chain of T dependent steps.
 //
 // What bounds them is the FMA rate (3 to 5 multiply-adds per state element and token); a tensor-core form would need
-// 16-bit or split operands.  Every exponent is a difference of sums of logarithms that is at most 0 (sums in 64-bit) or, for
-// decays per channel, a product of decays of at most T tokens: no term overflows.
+// 16-bit or split operands.  Every exponent is a difference of sums of logarithms that is at most 0 up to the 64-bit sums' rounding
+// (no token's logarithm lies below -1e4) or, for decays per channel, a product of decays of at most T tokens: no term overflows.
 //
 // A step's batch is ragged: entry e owns tokens cu_q[e] .. cu_q[e+1]-1 and state row seq_rows[e].  Chunk c of entry e has the
 // place cu_q[e] / T + e + c among the step's chunks (the places of different entries never meet), so that a block finds its

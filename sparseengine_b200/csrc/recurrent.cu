@@ -880,9 +880,12 @@ __global__ void delta_prep_kernel(float* qkv, int width, const T* a, int a_pitch
     }
     for (int h = threadIdx.x; h < H; h += blockDim.x) {
         beta[(size_t)t * H + h] = sigmoid_f(to_float(proj[(size_t)t * pitch + b_off + h]));
-        // the decays' logarithms (one per head), for the chunked form of the recurrence
-        if (log_dec != nullptr)
-            log_dec[(size_t)t * H + h] = -expf(a_log[h]) * softplus_f(to_float(a[(size_t)t * a_pitch + h]) + dt_bias[h]);
+        // the decays' logarithms (one per head), for the chunked form of the recurrence; a decay below e^-104 is 0 in 32-bit, and
+        // with an infinite rate or step the differences of sums would be NaN
+        if (log_dec != nullptr) {
+            const float v = -expf(a_log[h]) * softplus_f(to_float(a[(size_t)t * a_pitch + h]) + dt_bias[h]);
+            log_dec[(size_t)t * H + h] = v < -1e4f ? -1e4f : v;
+        }
     }
 }
 

@@ -167,8 +167,9 @@ def _inputs(kind, T, H, d):
     return x, {"q": ("qkv", q + 3), "k": ("qkv", k + 3), "v": ("qkv", v + 3), "decay": ("decay", 0)}
 
 
-def _outputs(kind, x, H, d, tokens=False):
-    """Outputs and the state after them, from a state of zeros; ``tokens``: by the kernels that walk token by token."""
+def _outputs(kind, x, H, d, tokens=False, one_kernel=False):
+    """Outputs and the state after them, from a state of zeros; ``tokens``: by the kernels that walk token by token; ``one_kernel``:
+    by the delta rule's other chunked form."""
     from sparseengine_b200.csrc import ops
     T = x["qkv"].shape[0]
     step, o, state = _one_entry(T), torch.empty(T, H * d, device=DEV), torch.zeros(1, H * d * d, device=DEV)
@@ -181,10 +182,14 @@ def _outputs(kind, x, H, d, tokens=False):
     else:
         sizes = dict(heads=H, kv_heads=H, head_dim=d, v_head_dim=d)
         inputs = dict(unit_eps=1e-6, q_scale=0.1, per_head=kind == "delta, per head")
-        if tokens:
+        if tokens or one_kernel:
+            log_dec = torch.empty(T, H, device=DEV) if one_kernel else None
             qkv, dec, beta = x["qkv"].clone(), torch.empty(T, H * d, device=DEV), torch.empty(T, H, device=DEV)
-            ops.delta_prep(qkv, x["decay"], x["beta"], 0, x["bias"], x["a_log"], dec, beta, **sizes, **inputs)
-            ops.delta_scan(qkv, dec, beta, state, step, o, **sizes)
+            ops.delta_prep(qkv, x["decay"], x["beta"], 0, x["bias"], x["a_log"], dec, beta, **sizes, **inputs, log_dec=log_dec)
+            if one_kernel:
+                ops.delta_chunk(qkv, log_dec, beta, state, step, o, **sizes)
+            else:
+                ops.delta_scan(qkv, dec, beta, state, step, o, **sizes)
         else:
             ops.delta_walk(x["qkv"], x["decay"], x["beta"], 0, x["bias"], x["a_log"], state, step, o, **sizes, **inputs)
     return o, state
@@ -209,3 +214,24 @@ def test_inputs_that_are_not_finite_stay_with_their_token_and_later_ones(kind, w
         assert not bool(torch.isfinite(got[token, :d]).any()) and torch.equal(got[token + 1:], want[token + 1:])
     elif where != "decay" or value != value:                     # an infinite step may be a decay of 0
         assert not bool(torch.isfinite(got[token:, :d]).all(1).any())
+
+
+@pytest.mark.parametrize("what", ["rate", "some steps", "all but forgotten"])
+@pytest.mark.parametrize("kind", ["state space", "delta, per head", "delta, per channel", "delta in one kernel"])
+def test_decays_of_zero(kind, what):
+    """Decays that are exactly 0 in 32-bit, from an infinite rate, from infinite steps (the delta rules; a state space takes its step
+    as a factor too) or from rates of e^80: what the kernels give that walk token by token."""
+    H, d, T = 2, 64, 150
+    one_kernel = kind == "delta in one kernel"
+    kind = "delta, per head" if one_kernel else kind
+    x, _ = _inputs(kind, T, H, d)
+    if what == "some steps":
+        if kind == "state space":
+            pytest.skip("outputs are infinite")
+        x["decay"][[0, 17, 40, 41, 64, 149]] = float("inf")
+    else:
+        x["a_log"][1] = 90.0 if what == "rate" else 80.0
+    (got, state), (want, last) = (_outputs(kind, x, H, d, tokens=tokens, one_kernel=one_kernel and not tokens) for tokens in (False, True))
+    assert bool(torch.isfinite(want).all() and torch.isfinite(last).all())
+    _close(got, want.double(), "outputs")
+    _close(state, last.double(), "state")
