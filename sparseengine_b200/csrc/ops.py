@@ -1339,6 +1339,9 @@ def attn_prefill(q, cache, table, seq_rows, cu_q, kv_len, out, *, entries, max_q
     return out
 
 
+F32_TILE_ROWS = 128       # (token, head) rows per tile of the 32-bit prompt-portion kernel (csrc/attention_f32.cu)
+
+
 def attn_prefill_f32_supported(head_dim: int, v_head_dim: int, num_heads: int, num_kv_heads: int) -> bool:
     """What ``se_attn_prefill_f32_supported`` answers (restated, as :func:`attn_decode_supported`)."""
     return (0 < head_dim <= 128 and head_dim % 4 == 0 and 0 < v_head_dim <= 128 and v_head_dim % 4 == 0

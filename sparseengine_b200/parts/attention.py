@@ -217,6 +217,16 @@ class PagedAttention(Mixer):
         return (step.max_q_len >= self.portion_min_tokens
                 and step.num_tokens >= self.portion_min_average * step.num_seqs)
 
+    def takes_f32_tiles(self, q, out, step, slot) -> bool:
+        """Whether a step's 32-bit attention runs on the tiled kernel (csrc/attention_f32.cu): prompt portions as in 16-bit, of sizes
+        it takes, q, out and the cache on 16 bytes (it copies 16 at a time; the plain kernel takes any address, a cache that is a view
+        at an odd offset say), the tiles of the longest entry's rows within the grid."""
+        s = self.spec
+        return (self.use_tensor_cores is not False and q.dtype == torch.float32 and self.takes_portion_kernel(step)
+                and ops.attn_prefill_f32_supported(s.head_dim, s.value_dim, s.num_heads, s.num_kv_heads)
+                and not (q.data_ptr() | out.data_ptr() | slot.kv.data_ptr()) & 15
+                and -(-step.max_q_len * (s.num_heads // s.num_kv_heads) // ops.F32_TILE_ROWS) <= ops.LIMITS["grid_dim_yz"])
+
     use_tensor_cores = None      # False: always the plain kernel
 
     def slopes(self, device):
@@ -251,9 +261,7 @@ class PagedAttention(Mixer):
                    max_q_len=step.max_q_len, num_heads=s.num_heads, num_kv_heads=s.num_kv_heads,
                    head_dim=s.head_dim, page_size=slot.page_size, scale=s.scale, window=s.window, **options)
             return
-        # 32-bit prompt portions: the same hand-over as in 16-bit (a step of single tokens leaves the tiles' rows empty)
-        if (self.use_tensor_cores is not False and q.dtype == torch.float32 and self.takes_portion_kernel(step)
-                and ops.attn_prefill_f32_supported(s.head_dim, s.value_dim, s.num_heads, s.num_kv_heads)):
+        if self.takes_f32_tiles(q, out, step, slot):
             ops.attn_prefill_f32(q, slot.kv, slot.table, step.seq_rows, step.cu_q, step.kv_len, out, entries=step.num_seqs,
                                  max_q_len=step.max_q_len, num_heads=s.num_heads, num_kv_heads=s.num_kv_heads,
                                  head_dim=s.head_dim, page_size=slot.page_size, scale=s.scale, window=s.window, **options)

@@ -142,3 +142,40 @@ def test_single_tokens(d, dv, heads, kv_heads, copies, options):
         want = torch.einsum("hn,nhd->hd", torch.softmax(s, 1)[:, :n], v)
         # sums over at most 256 products and 200 keys of size one; the scores' error enters through the exponential
         assert float((out[e].view(heads, dv).double() - want).abs().max()) < 4e-6 * max(1.0, float(want.abs().max()))
+
+
+def _layer(**sizes):
+    from sparseengine_b200.config.specs import AttentionSpec
+    from sparseengine_b200.parts.base import make_mixer
+    return make_mixer(AttentionSpec(hidden_size=64, scale=0.125, position=None, **sizes), torch.float32)
+
+
+def test_portions_on_odd_addresses_take_the_plain_kernel():
+    """A cache, queries or an output that do not lie on 16 bytes are served as aligned ones are."""
+    from types import SimpleNamespace
+
+    from sparseengine_b200.csrc import ops
+    heads, kv_heads, d, page = 4, 2, 64, 16
+    part = _layer(num_heads=heads, num_kv_heads=kv_heads, head_dim=d)
+    b = _batch([40, 17], [40, 90], page, 1)
+    step = SimpleNamespace(num_tokens=57, num_seqs=2, max_q_len=40, max_kv_len=90, seq_rows=b["rows"], token_seq=b["seq"],
+                           positions=b["pos"], cu_q=b["cu"], kv_len=b["kv"], q_lens=[40, 17], kv_lens=[40, 90])
+    tensors = {"kv": torch.randn(b["pages"], 2, kv_heads, page, d, device=DEV), "q": torch.randn(57, heads * d, device=DEV),
+               "out": torch.empty(57, heads * d, device=DEV)}
+
+    def attend(odd=None):
+        t = dict(tensors)
+        if odd is not None:
+            store = torch.empty(t[odd].numel() + 1, device=DEV)
+            store[1:] = t[odd].flatten()
+            t[odd] = store[1:].view(t[odd].shape)
+        before = ops.calls.get("se_attn_prefill_f32", 0)
+        part.attend(t["q"], t["out"], step, SimpleNamespace(kv=t["kv"], table=b["table"], page_size=page))
+        ops.error_check(DEV)
+        return t["out"].clone(), ops.calls.get("se_attn_prefill_f32", 0) - before
+
+    want, tiled = attend()
+    assert tiled == 1
+    for odd in tensors:
+        got, tiled = attend(odd)
+        assert tiled == 0 and float((got - want).abs().max()) < 4e-6
