@@ -174,7 +174,9 @@ class GatedDeltaMixer(Mixer):
         sizes, inputs = self.sizes, self.inputs
         o = torch.empty(tokens, self.vv, dtype=torch.float32, device=dev)
         long = takes_chunks(self, step, s.num_heads, s.head_dim, s.v_head_dim, 2.1e-3 if self.per_head else 2.5e-3, dev)
-        if long and ops.chunk_walk_supported(s.head_dim, s.v_head_dim):
+        # (decays per channel are read four at a time: a bias bound as a view off 16 bytes goes token by token)
+        if (long and ops.chunk_walk_supported(s.head_dim, s.v_head_dim)
+                and (self.per_head or (self.dt_bias.data_ptr() | a.data_ptr()) % 16 == 0)):
             ops.delta_walk(qkv, a, proj, self.b_off, self.dt_bias, self.a_log, slot.state, step, o, **sizes, **inputs)
         else:
             # One decay per head: chunks of 64 tokens in one kernel, while its (entry, head, 32 columns) blocks do not fill the
@@ -272,6 +274,7 @@ class RetentionMixer(Mixer):
         if not chunked and rotary_dim == 0:      # q and k straight from the projection, as they are staged
             ops.retention_scan(None, None, *args, **sizes, qk=(0, self.qk, self.k_scale))
         elif (chunked and ops.retention_walk_supported(s.head_dim, s.v_head_dim, rotary_dim, proj, self.qk)
+              and (inv_freq is None or inv_freq.data_ptr() % 16 == 0)
               # entries of one chunk that fill the device go faster through the kernel that does a chunk at a time (a layer of 32 heads
               # of 128 x 128, four entries of 17 to 64 tokens: 118 to 135 us against 124 to 143; one entry: 87 against 76)
               and (step.max_q_len > 64 or step.num_seqs * s.num_heads * (-(-s.v_head_dim // 32)) <= ops.sm_count(dev))):

@@ -235,3 +235,42 @@ def test_decays_of_zero(kind, what):
     assert bool(torch.isfinite(want).all() and torch.isfinite(last).all())
     _close(got, want.double(), "outputs")
     _close(state, last.double(), "state")
+
+
+@pytest.mark.parametrize("kind", ["delta", "retention"])
+def test_parameters_off_16_bytes(kind):
+    """A decay bias or rotation frequencies that are views off 16 bytes: what the same numbers give on 16 bytes."""
+    from sparseengine_b200.config.specs import GatedDeltaSpec, RetentionSpec, RotarySpec
+    from sparseengine_b200.csrc import ops
+    from sparseengine_b200.parts.base import LayerSlot, make_mixer
+    from sparseengine_b200.parts.position import as_rotary_args
+    T, width, heads, d = 70, 64, 2, 16
+    if kind == "delta":
+        spec = GatedDeltaSpec(hidden_size=width, num_heads=heads, num_kv_heads=heads, head_dim=d, v_head_dim=d, conv_taps=4, decay_per="channel",
+                              gate_activation="sigmoid", decay_rank=8, gate_rank=8)
+    else:
+        spec = RetentionSpec(hidden_size=width, num_heads=heads, head_dim=d, v_head_dim=d, decays=(0.9, 0.99), position=RotarySpec(rotary_dim=d, theta=1e4))
+    step = _one_entry(T)
+    step.token_seq, step.positions = torch.zeros(T, dtype=torch.int32, device=DEV), torch.arange(T, dtype=torch.int32, device=DEV)
+
+    def odd(t):
+        store = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+        store[1:] = t.flatten()
+        return store[1:].view(t.shape)
+
+    outs, walks = [], []
+    for off in (False, True):
+        part, g = make_mixer(spec, torch.float32), torch.Generator(device=DEV).manual_seed(1)
+        tensors = {n: torch.randn(p.shape, generator=g, device=DEV) * 0.3 for n, p in part.parameters().items()}
+        x = torch.randn(T, width, generator=g, device=DEV)
+        if off and kind == "delta":
+            tensors["dt_bias"] = odd(tensors["dt_bias"])
+        part.bind(tensors)
+        if off and kind == "retention":
+            inv = odd(as_rotary_args(part.position.kernel_args(torch.device(DEV))).inv_freq)
+            part.position.kernel_args = lambda device: (inv, d, 1.0)
+        before = sum(ops.calls.get(n, 0) for n in ("se_delta_walk", "se_retention_prep"))
+        outs.append(part.forward(x, step, LayerSlot(state=torch.zeros(1, *part.state_request().shape, device=DEV))))
+        walks.append(sum(ops.calls.get(n, 0) for n in ("se_delta_walk", "se_retention_prep")) - before)
+    assert walks == ([1, 0] if kind == "delta" else [0, 1])
+    _close(outs[1], outs[0].double(), "outputs")
