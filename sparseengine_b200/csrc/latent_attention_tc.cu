@@ -122,7 +122,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __nv
                 mine[h] = 0ull;
                 if (j >= k_lo && j < k_end) {
                     const int page = row_table[j / page_size];
-                    if (page_in_pool(page, num_pages, error, 29))
+                    if (page_in_pool(page, num_pages, error, SE_CODE_BAD_PAGE_LATENT_TC))
                         mine[h] = (unsigned long long)(cache + ((size_t)page * page_size + j % page_size) * D);
                 }
             }
@@ -151,7 +151,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __nv
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar(&bars.kv_full[tile % stages])) : "memory");
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-        if (!ok) { abort_s = 1; if (lane == 0) atomicCAS(error, 0, 14); }
+        if (!ok) { abort_s = 1; if (lane == 0) atomicCAS(error, 0, 15); }
     } else if (warp == 1) {
         // ---- MMA issuer: one lane for both query tiles ---------------------------------------------
         // With one S buffer P V (j) and S (j + 1) of a tile go out together as its P (j) arrives (MMAs of one thread run in their
@@ -246,7 +246,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __nv
         }
         if (ok && elect_one())
             for (int x = 0; x < kTiles; ++x) umma_commit(bar(&bars.o_done[x]));
-        if (!ok) { abort_s = 1; if (lane == 0) atomicCAS(error, 0, 15); }
+        if (!ok) { abort_s = 1; if (lane == 0) atomicCAS(error, 0, 16); }
         __syncwarp();
     } else if (warp < 2 + 4 * kTiles) {
         // ---- softmax and epilogue: four warps per query tile, one thread per row --------------------
@@ -352,7 +352,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __nv
             }
         } else {
             abort_s = 1;
-            atomicCAS(error, 0, 16);
+            atomicCAS(error, 0, 17);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

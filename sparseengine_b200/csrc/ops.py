@@ -1101,7 +1101,8 @@ _WAIT_ROLES = "a tensor-core kernel timed out waiting on a barrier (role code {c
 _INDEX_CODES = {21: "the q/k preparation kernel", 22: "the plain attention kernel", 23: "the split-key decode attention kernel",
                 24: "the prompt-portion attention kernel", 25: "the tcgen05 prompt-portion attention kernel",
                 26: "the block-table update kernel", 27: "the latent preparation kernel",
-                28: "the latent attention kernel", 29: "the tiled latent attention kernel"}
+                28: "the latent attention kernel", 29: "the tiled latent attention kernel",
+                30: "the tcgen05 latent attention kernel"}
 
 
 def error_text(code: int) -> str:

@@ -59,6 +59,22 @@ def test_against_64_bits(rank, rot, heads, window, sinks):
         assert torch.equal(run(dirty, wrong), out)
 
 
+def test_a_bad_page_names_this_kernel():
+    """An entry that names no page: left out, reported with a code that no other kernel has."""
+    from sparseengine_b200.csrc import ops
+    i32 = dict(dtype=torch.int32, device=DEV)
+    table = torch.tensor([[0, 10 ** 6, 2, 3]], **i32)
+    cache, q = torch.randn(4, 16, 128, device=DEV).to(torch.bfloat16), torch.randn(60, 4, 128, device=DEV).to(torch.bfloat16)
+    out = torch.empty(60, 4, 64, dtype=torch.bfloat16, device=DEV)
+    args = (torch.zeros(1, **i32), torch.tensor([0, 60], **i32), torch.tensor([60], **i32), None, out)
+    sizes = dict(entries=1, max_q_len=60, heads=4, rank=64, rot=64, page_size=16, scale=0.1)
+    for fn, name in ((ops.latent_attention_tc, "the tcgen05 latent"), (ops.latent_attention_tiled, "the tiled latent")):
+        fn(q, cache, table, *args, **sizes)
+        with pytest.raises(RuntimeError, match=name):
+            ops.error_check(DEV)
+    assert bool(torch.isfinite(out).all())
+
+
 def test_choice_by_rows():
     from sparseengine_b200.csrc import ops
     assert ops.latent_takes_tc(1, 2048, 32, 192, 64, 148) and ops.latent_takes_tc(4, 512, 16, 128, 64, 148)
