@@ -6,9 +6,8 @@
 // key once per query row (from L2, 8 bytes per FMA pair) and spends five shuffles per key.  Here a thread keeps 8 rows x 4
 // keys of scores and 8 rows x 4 or 8 columns of the output in registers: three 16-byte shared-memory reads per 32 (scores)
 // and four per 64 (output) FMAs.  Keys arrive while the output of the tile before is summed and values while the scores
-// are (cp.async).  Rows are private to a warp, so the softmax needs no barrier.  A warp owns 16 rows, every other one of them a
-// thread's: a tile that an entry does not fill (a decoding request beside a prompt brings one row per head of its group) costs the
-// arithmetic of its rows, not of 128.  Measured at MiniMax M2's sizes (48 heads
+// are (cp.async).  Rows are private to a warp, so the softmax needs no barrier, and a warp without rows (a decoding request beside a
+// prompt brings one per head of its group) only copies.  Measured at MiniMax M2's sizes (48 heads
 // over 8, head size 128), prompts of 1, 300, 1,024 and 2,047 tokens in one step: 2.3 ms against about 26 ms.
 //
 // Query/key and value head sizes that are multiples of 4 up to 128; the options are the plain kernel's, and so is what a query
@@ -62,9 +61,8 @@ attn_prefill_f32_kernel(const float* __restrict__ q, const float* __restrict__ c
     const int row_base = (int)(gridDim.y - 1 - blockIdx.y) * kRows;      // tiles with the most keys start first
     if (row_base >= total_rows) return;
     const int kv_end = kv_len[entry], q_start = kv_end - q_len;
-    const int tid = threadIdx.x, tc = tid & 15;
-    const int row0 = (tid >> 5) * 16 + ((tid >> 4) & 1);         // this thread's rows: row0 + 2 i
-    const int live = min(8, max(0, (total_rows - row_base - (tid >> 5) * 16 + 1) >> 1));      // a warp's number; the others are left out
+    const int tid = threadIdx.x, tr = tid >> 4, tc = tid & 15;
+    const bool live = row_base + (tid >> 5) * 16 < total_rows;           // this warp has rows
 
     const int last_row = min(row_base + kRows, total_rows) - 1;
     const int k_end = q_start + last_row / group + 1;
@@ -111,11 +109,11 @@ attn_prefill_f32_kernel(const float* __restrict__ q, const float* __restrict__ c
         *reinterpret_cast<float4*>(qs + r * dp + c * 4) = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
     }
 
-    int pos[8], first[8];
+    int pos[8], first[8];                            // this thread's rows tr * 8 + i
     float m[8], l[8], slope[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int row = min(row_base + row0 + 2 * i, total_rows - 1);
+        const int row = min(row_base + tr * 8 + i, total_rows - 1);
         pos[i] = q_start + row / group;
         first[i] = first_visible(pos[i], window);
         slope[i] = opt.slopes != nullptr ? opt.slopes[kvh * group + row % group] : 0.f;
@@ -129,55 +127,51 @@ attn_prefill_f32_kernel(const float* __restrict__ q, const float* __restrict__ c
         const int j0 = tile_key(it);
         cp_wait<1>();                                // this tile's keys (its values may still be on their way)
         __syncthreads();
-        float s[8][4] = {};
-        auto add_scores = [&](auto whole) {
+        if (live) {
+            float s[8][4] = {};
             for (int k = 0; k < d; k += 4) {
                 float4 kv[4];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) kv[c] = *reinterpret_cast<const float4*>(ks + (tc + 16 * c) * dp + k);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    if (!decltype(whole)::value && i >= live) break;
-                    const float4 qv = *reinterpret_cast<const float4*>(qs + (row0 + 2 * i) * dp + k);
+                    const float4 qv = *reinterpret_cast<const float4*>(qs + (tr * 8 + i) * dp + k);
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
                         s[i][c] = fmaf(qv.w, kv[c].w, fmaf(qv.z, kv[c].z, fmaf(qv.y, kv[c].y, fmaf(qv.x, kv[c].x, s[i][c]))));
                 }
             }
-        };
-        if (live == 8) add_scores(std::true_type{});
-        else if (live > 0) add_scores(std::false_type{});
-        int ok[4];
+            int ok[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) ok[c] = key_ok[it & 1][tc + 16 * c];
+            for (int c = 0; c < 4; ++c) ok[c] = key_ok[it & 1][tc + 16 * c];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            if (i >= live) break;
-            float top = -INFINITY;
+            for (int i = 0; i < 8; ++i) {
+                float top = -INFINITY;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int j = j0 + tc + 16 * c;
-                float v = s[i][c];
-                if (opt.softcap > 0.f) v = opt.softcap * tanhf(v / opt.softcap);
-                v -= slope[i] * (float)(pos[i] - j);
-                s[i][c] = ok[c] && j <= pos[i] && (j >= first[i] || j < keep_first) ? v : -INFINITY;
-                top = fmaxf(top, s[i][c]);
+                for (int c = 0; c < 4; ++c) {
+                    const int j = j0 + tc + 16 * c;
+                    float v = s[i][c];
+                    if (opt.softcap > 0.f) v = opt.softcap * tanhf(v / opt.softcap);
+                    v -= slope[i] * (float)(pos[i] - j);
+                    s[i][c] = ok[c] && j <= pos[i] && (j >= first[i] || j < keep_first) ? v : -INFINITY;
+                    top = fmaxf(top, s[i][c]);
+                }
+#pragma unroll
+                for (int x = 8; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
+                const float m_new = fmaxf(m[i], top), base = m_new == -INFINITY ? 0.f : m_new;
+                const float corr = expf(m[i] - base);    // nothing seen so far: exp(-inf) = 0
+                m[i] = m_new;
+                float sum = 0.f;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float p = expf(s[i][c] - base);
+                    sum += p;
+                    ps[(tr * 8 + i) * kPPitch + tc + 16 * c] = p;
+                }
+                l[i] = l[i] * corr + sum;
+#pragma unroll
+                for (int c = 0; c < kCols; ++c) o[i][c] *= corr;
             }
-#pragma unroll
-            for (int x = 8; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
-            const float m_new = fmaxf(m[i], top), base = m_new == -INFINITY ? 0.f : m_new;
-            const float corr = expf(m[i] - base);    // nothing seen so far: exp(-inf) = 0
-            m[i] = m_new;
-            float sum = 0.f;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const float p = expf(s[i][c] - base);
-                sum += p;
-                ps[(row0 + 2 * i) * kPPitch + tc + 16 * c] = p;
-            }
-            l[i] = l[i] * corr + sum;
-#pragma unroll
-            for (int c = 0; c < kCols; ++c) o[i][c] *= corr;
         }
         __syncthreads();                             // all warps are done with the keys
         if (it + 1 < num_tiles) load(it + 1, false);
@@ -189,14 +183,11 @@ attn_prefill_f32_kernel(const float* __restrict__ q, const float* __restrict__ c
             odd |= !(isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w));
         }
         odd = __syncthreads_or(odd);
-        auto add_values = [&](auto guarded, auto whole) {
+        auto add_values = [&](auto guarded) {
             for (int k = 0; k < kKeys; k += 4) {
                 float4 p[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    if (!decltype(whole)::value && i >= live) break;
-                    p[i] = *reinterpret_cast<const float4*>(ps + (row0 + 2 * i) * kPPitch + k);
-                }
+                for (int i = 0; i < 8; ++i) p[i] = *reinterpret_cast<const float4*>(ps + (tr * 8 + i) * kPPitch + k);
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk) {
                     float v[kCols];
@@ -205,7 +196,6 @@ attn_prefill_f32_kernel(const float* __restrict__ q, const float* __restrict__ c
                         *reinterpret_cast<float4*>(v + 4 * g) = *reinterpret_cast<const float4*>(vs + (k + kk) * DVT + g * 64 + tc * 4);
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
-                        if (!decltype(whole)::value && i >= live) break;
                         const float pv = kk == 0 ? p[i].x : kk == 1 ? p[i].y : kk == 2 ? p[i].z : p[i].w;
 #pragma unroll
                         for (int c = 0; c < kCols; ++c)
@@ -214,16 +204,17 @@ attn_prefill_f32_kernel(const float* __restrict__ q, const float* __restrict__ c
                 }
             }
         };
-        if (odd) add_values(std::true_type{}, std::false_type{});
-        else if (live == 8) add_values(std::false_type{}, std::true_type{});
-        else if (live > 0) add_values(std::false_type{}, std::false_type{});
+        if (live) {
+            if (odd) add_values(std::true_type{});
+            else add_values(std::false_type{});
+        }
         __syncthreads();                             // all warps are done with the values
         if (it + 1 < num_tiles) load(it + 1, true);
         else cp_commit();
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int row = row_base + row0 + 2 * i;
+        const int row = row_base + tr * 8 + i;
         float sum = l[i];
 #pragma unroll
         for (int x = 8; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
