@@ -529,15 +529,46 @@ def latent_attention_tc_supported(rank: int, rot: int) -> bool:
     return 0 < rank <= 192 and rank % 64 == 0 and rot >= 0 and rot % 64 == 0 and rank + rot <= 256
 
 
-def latent_takes_tc(entries: int, max_q_len: int, heads: int, rank: int, rot: int, sms: Optional[int] = None) -> bool:
+def latent_takes_tc(entries: int, max_q_len: int, heads: int, rank: int, rot: int, sms: Optional[int] = None, q_lens=None,
+                    kv_lens=None, window: Optional[int] = None) -> bool:
     """Whether a step's latent attention runs on tcgen05 (csrc/latent_attention_tc.cu): sizes it takes, an entry that fills half
-    a query tile, and blocks of 256 rows for a fifth of the SMs (steps of fewer rows split their keys over the device instead).
-    Measured, 32 heads, us there and here: 8 blocks over 4,096 keys 52 / 141, 16 blocks 99 / 145, 32 blocks 186 / 149; 64 requests
-    at 2,048 keys that bring 1, 2 and 8 tokens 33 / 46, 38 / 46 and 104 / 47."""
+    a query tile, and the shorter of the times (us) that the two kernels are estimated to take over the entries' own tokens and keys
+    (``q_lens``, ``kv_lens``; without them every entry is as long as the longest and holds nothing before).  tcgen05: a block per 256
+    rows, 2.1 per 64 keys, one block on an SM, 8 to start and end.  The tiled kernel: a block per 64 rows, its keys split
+    (:func:`latent_split_plan`) where the blocks of the longest entry's rows, times the entries, would not fill the device twice;
+    0.054 per key alone on an SM and 0.067 for each of two, 2 to start and end, 10 (most of it
+    the host's, a launch and two workspaces) and the parts' bytes (32-bit, written and read) at 5 TB/s to join them.  Measured on a B200, 32
+    heads, a layer, us there and here: a portion of 64 tokens beside three decoding requests at 500, 4,000 and 30,000 keys
+    55 / 57, 121 / 168, 625 / 1,012; of 512 beside seven 100 / 79, 296 / 195, 1,765 / 1,058; one of 128 alone at 4,000 keys
+    123 / 166, of 256 206 / 174; 64 requests of which one brings 8 tokens at 4,000 keys 170 / 178."""
     if sms is None:
         sms = sm_count()
-    rows = max_q_len * heads
-    return latent_attention_tc_supported(rank, rot) and rows >= 128 and 5 * entries * -(-rows // 256) >= sms
+    if not latent_attention_tc_supported(rank, rot) or max_q_len * heads < 128:
+        return False
+    q_lens = q_lens or [max_q_len] * entries
+    kv_lens = kv_lens or q_lens
+    tile_keys = latent_tile_keys(max_q_len)
+    most = max(kv_lens) if window is None else min(max(kv_lens), window + max_q_len - 1)
+    splits, per = latent_split_plan(-(-max_q_len * heads // 64), entries, most, sms, tile_keys)
+    wide = wide_keys = wide_last = narrow = narrow_keys = narrow_last = 0
+    for q, kv in zip(q_lens, kv_lens):
+        if q <= 0:
+            continue
+        last = kv if window is None else min(kv, window)           # keys of an entry's last token, of its middle one
+        mean = min(kv - (q - 1) // 2, last)
+        blocks = -(-q * heads // 256)
+        wide += blocks
+        wide_keys += blocks * mean
+        wide_last = max(wide_last, last)
+        each = min(per * tile_keys, last) if splits > 1 else mean
+        blocks = -(-q * heads // 64) * (min(splits, -(-last // each)) if splits > 1 else 1)
+        narrow += blocks
+        narrow_keys += blocks * each
+        narrow_last = max(narrow_last, each if splits > 1 else last)
+    tc = 8 + 2.1 / 64 * max(wide_last, -(-wide // sms) * wide_keys / wide) + 2.1
+    full, rest = divmod(narrow, 2 * sms)
+    tiled = 2 + max(0.054 * narrow_last, (0.067 * full + (0.067 if rest > sms else 0.054 if rest else 0.0)) * narrow_keys / narrow)
+    return tc < tiled + (10 + narrow * 64 * rank * 8 / 5e6 if splits > 1 else 0)
 
 
 def latent_attention_tc(qfull, cache, table, seq_rows, cu_q, kv_len, sink, out, *, entries, max_q_len, heads, rank, rot,

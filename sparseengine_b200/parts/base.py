@@ -85,6 +85,17 @@ class LayerSlot:
     state: Optional[torch.Tensor] = None     # [rows, *StateRequest.shape]
 
 
+def once_per_step(step, key, ask):
+    """``ask()``, asked once per step for all layers that share ``key``: a choice between kernels walks the step's entries on the
+    host."""
+    extras = getattr(step, "extras", None)
+    if extras is None:
+        return ask()
+    if key not in extras:
+        extras[key] = ask()
+    return extras[key]
+
+
 @dataclass
 class StepContext:
     """Device-side description of one step's batch (int32 tensors) plus host copies.

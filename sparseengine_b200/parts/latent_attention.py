@@ -22,7 +22,7 @@ import torch
 
 from ..config.specs import ParamSpec
 from ..csrc import ops
-from .base import KVRequest, Mixer, make_position, register_mixer
+from .base import KVRequest, Mixer, make_position, once_per_step, register_mixer
 from .linear import linear
 from .position import RotaryArgs, as_rotary_args
 
@@ -133,9 +133,19 @@ class LatentAttention(Mixer):
         return (self.use_tensor_cores is not False and dtype == torch.bfloat16 and s.scale > 0
                 and ops.latent_attention_tiled_supported(s.kv_rank, s.rot_dim))
 
+    def takes_tc(self, step, device) -> bool:
+        """``ops.latent_takes_tc`` over the step's own entries, asked once per step for all layers of the same sizes."""
+        s = self.spec
+
+        def ask():
+            kv_lens = step.kv_lens if step.max_kv_bound is None else [step.max_kv_bound] * step.num_seqs
+            return ops.latent_takes_tc(step.num_seqs, step.max_q_len, s.num_heads, s.kv_rank, s.rot_dim, ops.sm_count(device),
+                                       q_lens=step.q_lens, kv_lens=kv_lens, window=s.window)
+        return once_per_step(step, ("latent.takes_tc", s.num_heads, s.kv_rank, s.rot_dim, s.window), ask)
+
     def attend_tiled(self, qfull, out_lat, step, slot):
         s = self.spec
-        if ops.latent_takes_tc(step.num_seqs, step.max_q_len, s.num_heads, s.kv_rank, s.rot_dim, ops.sm_count(qfull.device)):
+        if self.takes_tc(step, qfull.device):
             ops.latent_attention_tc(qfull, slot.kv, slot.table, step.seq_rows, step.cu_q, step.kv_len, self.sink, out_lat,
                                     entries=step.num_seqs, max_q_len=step.max_q_len, heads=s.num_heads, rank=s.kv_rank, rot=s.rot_dim,
                                     page_size=slot.page_size, scale=s.scale, window=s.window)

@@ -1,0 +1,42 @@
+"""Which kernel a step's latent attention takes, by its entries' own tokens and keys (no GPU)."""
+from types import SimpleNamespace
+
+import pytest
+
+from sparseengine_b200.csrc import ops
+
+
+def _takes(lens, held, window=None, heads=32, rank=192, rot=64):
+    return ops.latent_takes_tc(len(lens), max(lens), heads, rank, rot, 148, q_lens=lens, kv_lens=[held + n for n in lens], window=window)
+
+
+@pytest.mark.parametrize("lens,held,window,tc", [
+    # a portion beside decoding requests, which tcgen05 would walk unsplit: measured 121 / 168, 625 / 1,012 and 905 / 1,015 us
+    ([64, 1, 1, 1], 4000, None, False), ([64, 1, 1, 1], 30000, None, False), ([128, 1, 1, 1], 30000, None, False),
+    ([8] + [1] * 31, 30000, None, False), ([64, 1, 1, 1], 4000, 1024, False),
+    # where the tiled kernel does not split either: 296 / 195, 1,765 / 1,058, 254 / 178
+    ([512] + [1] * 7, 4000, None, True), ([512] + [1] * 7, 30000, None, True), ([32] + [1] * 63, 4000, None, True),
+    ([512] + [1] * 7, 4000, 1024, True),
+    # portions alone: 207 / 174, 123 / 166, 1,195 / 411
+    ([256], 4000, None, True), ([128], 4000, None, False), ([2048], 4000, None, True), ([64] * 16, 4000, None, True),
+    ([1] * 64, 4000, None, False)])
+def test_by_entries(lens, held, window, tc):
+    assert _takes(lens, held, window) is tc
+
+
+def test_asked_once_per_step():
+    from sparseengine_b200.config.specs import LatentAttentionSpec
+    from sparseengine_b200.parts.base import make_mixer
+    import torch
+    part = make_mixer(LatentAttentionSpec(hidden_size=64, num_heads=32, head_dim=16, rot_dim=64, v_head_dim=16, q_rank=16, kv_rank=192,
+                                          scale=0.1, position=None), torch.bfloat16)
+    asked = []
+    before, count = ops.latent_takes_tc, ops.sm_count
+    ops.latent_takes_tc, ops.sm_count = lambda *a, **k: asked.append(k["kv_lens"]) or True, lambda device=None: 148
+    try:
+        step = SimpleNamespace(num_seqs=2, max_q_len=5, q_lens=[5, 1], kv_lens=[9, 1], max_kv_bound=None, extras={})
+        assert part.takes_tc(step, "cuda:0") and part.takes_tc(step, "cuda:0") and asked == [[9, 1]]
+        step = SimpleNamespace(num_seqs=2, max_q_len=1, q_lens=[1, 1], kv_lens=[9, 1], max_kv_bound=64, extras={})
+        assert part.takes_tc(step, "cuda:0") and asked[1] == [64, 64]
+    finally:
+        ops.latent_takes_tc, ops.sm_count = before, count
