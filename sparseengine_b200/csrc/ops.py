@@ -1374,6 +1374,35 @@ def attn_prefill(q, cache, table, seq_rows, cu_q, kv_len, out, *, entries, max_q
 F32_TILE_ROWS = 128       # (token, head) rows per tile of the 32-bit prompt-portion kernel (csrc/attention_f32.cu)
 
 
+def attn_f32_tiles_pay(q_lens, kv_lens, num_heads: int, num_kv_heads: int, most: Optional[int] = None, sms: Optional[int] = None) -> bool:
+    """Whether a step's 32-bit attention takes less time in tiles (csrc/attention_f32.cu) than by a block per (token, head)
+    (csrc/attention_plain.cu), as estimated (us) over its entries' tokens and keys; ``most``: keys a query sees at most (a window).
+    Plain: 2.2e-4 per (query head, key) pair.  Tiles: per tile of 128 (token, head) rows and 64 keys 13.5, of which the lookup of
+    the keys' pages is most, and 0.068 per row of the warps that have rows; one block on an SM, so an entry of one token
+    takes two thirds of a full tile's time.  Measured on a B200, a layer, us plain / tiles, 16 heads over 16: a prompt of 600 tokens
+    beside 63 requests of 4,000 keys 9,511 / 7,154, of 160 4,014 / 6,926, of 64 2,355 / 6,282; 600 single tokens of 1,000 keys
+    2,777 / 14,706; 48 heads over 8: 7,613 / 7,673; 32 over 1: 5,048 / 1,331; 48 over 8, a portion of 16 tokens behind 4,000
+    keys 757 / 1,261, of 160 5,567 / 1,421."""
+    sms = sms or sm_count()
+    group = num_heads // num_kv_heads
+    pairs, work, longest = 0.0, 0.0, 0.0
+    for q, kv in zip(q_lens, kv_lens):
+        if q <= 0:
+            continue
+        seen = kv if most is None else min(kv, most)                # keys that the last token sees, that the last tile reads
+        last = kv if most is None else min(kv, most + F32_TILE_ROWS // group)
+        mean = min(kv - (q - 1) / 2, last)
+        pairs += q * min(mean, seen)
+        full, rest = divmod(q * group, F32_TILE_ROWS)
+        rows = F32_TILE_ROWS if full else -(-rest // 16) * 16
+        longest = max(longest, -(-last // 64) * (13.5 + 0.068 * rows))
+        if full:
+            work += full * -(-(mean if full > 1 else last) // 64) * (13.5 + 0.068 * F32_TILE_ROWS)
+        if rest:
+            work += -(-last // 64) * (13.5 + 0.068 * (-(-rest // 16) * 16))
+    return max(longest, num_kv_heads * work / sms) < 2.2e-4 * pairs * num_heads
+
+
 def attn_prefill_f32_supported(head_dim: int, v_head_dim: int, num_heads: int, num_kv_heads: int) -> bool:
     """What ``se_attn_prefill_f32_supported`` answers (restated, as :func:`attn_decode_supported`)."""
     return (0 < head_dim <= 128 and head_dim % 4 == 0 and 0 < v_head_dim <= 128 and v_head_dim % 4 == 0

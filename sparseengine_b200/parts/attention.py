@@ -19,7 +19,7 @@ import torch
 
 from ..config.specs import ParamSpec
 from ..csrc import ops
-from .base import KVRequest, Mixer, make_position, register_mixer
+from .base import KVRequest, Mixer, make_position, once_per_step, register_mixer
 from .linear import linear, pad_rows
 from .position import RotaryArgs, as_rotary_args
 
@@ -218,14 +218,26 @@ class PagedAttention(Mixer):
                 and step.num_tokens >= self.portion_min_average * step.num_seqs)
 
     def takes_f32_tiles(self, q, out, step, slot) -> bool:
-        """Whether a step's 32-bit attention runs on the tiled kernel (csrc/attention_f32.cu): prompt portions as in 16-bit, of sizes
-        it takes, q, out and the cache on 16 bytes (it copies 16 at a time; the plain kernel takes any address, a cache that is a view
-        at an odd offset say), the tiles of the longest entry's rows within the grid."""
+        """Whether a step's 32-bit attention runs on the tiled kernel (csrc/attention_f32.cu): steps with prompt portions, as in 16-bit,
+        if tiles are estimated to take less than a block per (token, head); sizes that it takes, q, out and the cache on 16 bytes (it
+        copies 16 at a time; the plain kernel takes any address, a cache that is a view at an odd offset say), the tiles of the longest
+        entry's rows within the grid."""
         s = self.spec
         return (self.use_tensor_cores is not False and q.dtype == torch.float32 and self.takes_portion_kernel(step)
                 and ops.attn_prefill_f32_supported(s.head_dim, s.value_dim, s.num_heads, s.num_kv_heads)
                 and not (q.data_ptr() | out.data_ptr() | slot.kv.data_ptr()) & 15
-                and -(-step.max_q_len * (s.num_heads // s.num_kv_heads) // ops.F32_TILE_ROWS) <= ops.LIMITS["grid_dim_yz"])
+                and -(-step.max_q_len * (s.num_heads // s.num_kv_heads) // ops.F32_TILE_ROWS) <= ops.LIMITS["grid_dim_yz"]
+                and self.f32_tiles_pay(step, q.device))
+
+    def f32_tiles_pay(self, step, device) -> bool:
+        """``ops.attn_f32_tiles_pay`` over the step's entries, asked once per step for all layers of the same sizes."""
+        s = self.spec
+        most = s.chunk if s.chunk is not None else s.window + s.keep_first if s.window is not None else None
+
+        def ask():
+            kv_lens = step.kv_lens if step.max_kv_bound is None else [step.max_kv_bound] * step.num_seqs
+            return ops.attn_f32_tiles_pay(step.q_lens, kv_lens, s.num_heads, s.num_kv_heads, most, ops.sm_count(device))
+        return once_per_step(step, ("attention.f32_tiles_pay", s.num_heads, s.num_kv_heads, most), ask)
 
     use_tensor_cores = None      # False: always the plain kernel
 

@@ -159,7 +159,8 @@ def test_portions_on_odd_addresses_take_the_plain_kernel():
     part = _layer(num_heads=heads, num_kv_heads=kv_heads, head_dim=d)
     b = _batch([40, 17], [40, 90], page, 1)
     step = SimpleNamespace(num_tokens=57, num_seqs=2, max_q_len=40, max_kv_len=90, seq_rows=b["rows"], token_seq=b["seq"],
-                           positions=b["pos"], cu_q=b["cu"], kv_len=b["kv"], q_lens=[40, 17], kv_lens=[40, 90])
+                           positions=b["pos"], cu_q=b["cu"], kv_len=b["kv"], q_lens=[40, 17], kv_lens=[40, 90], max_kv_bound=None, extras={})
+    part.f32_tiles_pay = lambda step, device: True
     tensors = {"kv": torch.randn(b["pages"], 2, kv_heads, page, d, device=DEV), "q": torch.randn(57, heads * d, device=DEV),
                "out": torch.empty(57, heads * d, device=DEV)}
 
