@@ -780,11 +780,12 @@ def causal_conv(x, c0: int, w, bias, state, conv_off: int, step, out):
 def ssm_scan(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, step, y, *, heads, head_dim, state_size, groups):
     tokens = xbc.shape[0]
     steps = torch.empty(tokens, heads, 2, dtype=torch.float32, device=xbc.device)     # step sizes and decays
-    _check(_fn("se_ssm_scan", "ppii" "ppp" "pl" "pp" "pp" "iiiiii" "ip")(
+    _check(_fn("se_ssm_scan", "ppii" "ppp" "pl" "pp" "pp" "iiiiii" "iiip")(
         _ptr(xbc, torch.float32, "xbc"), proj.data_ptr(), proj.stride(0), int(dt_off), _ptr(dt_bias, torch.float32),
         _ptr(a_log, torch.float32), _ptr(d_skip, torch.float32), _ptr(state, torch.float32, "state"), state.stride(0),
         _ptr(step.cu_q), _ptr(step.seq_rows), _ptr(y, torch.float32, "y"), _ptr(steps), tokens, step.num_seqs, heads,
-        head_dim, state_size, groups, dtype_code(proj.dtype), _stream()), "ssm_scan")
+        head_dim, state_size, groups, int(getattr(step, "max_q_len", 0)) or -(-tokens // step.num_seqs), sm_count(xbc.device),
+        dtype_code(proj.dtype), _stream()), "ssm_scan")
     return y
 
 

@@ -1061,19 +1061,29 @@ extern "C" int se_causal_conv(const void* x, int pitch, int c0, const float* w, 
     SE_LAUNCH_CHECK();
 }
 
+// Whether the state space's tokens are walked with a state column per lane group (1) or in tiles (0), whose chain per token is shorter
+// but which read a state 4 bytes at a time: what either is estimated to take (us) over the longest entry's chain, all tokens and all
+// states.  Measured, 64 heads of 64 x 128, lane groups / tiles: one entry of 8 tokens 8.2/10.3, of 64 43/33; a portion of 64 tokens
+// beside 3 single ones 61/38, beside 15 62/56, beside 31 69/79, of 200 beside 63 221/205, of 90 125/148; 64 entries of 1 53/99, of 17
+// 265/302; 128 of 28 826/841.
+extern "C" int se_ssm_scan_by_lanes(int H, int P, int N, int tokens, int entries, int max_q_len, int sms) {
+    const float size = (float)H * P * N / 524288.f * 148.f / sms, states = size * entries, all = size * tokens;
+    const float lanes = 3.f + .65f * states + fmaxf(fmaxf(.8f, .45f * size) * max_q_len, .19f * all);
+    const float tiles = 6.f + 1.45f * states + fmaxf(fmaxf(.44f, .33f * size) * max_q_len, .182f * all);
+    return lanes <= tiles;
+}
+
 // steps: workspace of 2 * tokens * H floats (step sizes and decays), or null (then the kernel with one
 // column per thread computes them itself)
 extern "C" int se_ssm_scan(const float* xbc, const void* proj, int pitch, int dt_off, const float* dt_bias,
                            const float* a_log, const float* d_skip, float* state, long long state_pitch, const int* cu_q,
                            const int* seq_rows, float* y, float* steps, int tokens, int entries, int H, int P, int N, int G,
-                           int dtype, cudaStream_t stream) {
+                           int max_q_len, int sms, int dtype, cudaStream_t stream) {
+    // max_q_len: the longest entry's tokens; sms: the device's SMs
     if (entries <= 0) return 0;
-    if (H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G) return SE_ERR_ARGUMENT;
+    if (H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G || max_q_len < 1 || sms < 1) return SE_ERR_ARGUMENT;
     if (N > se::kMaxStateRows || H > 65535) return SE_ERR_UNSUPPORTED;
-    // Short entries: a state column per lane group.  Longer ones, token after token, are a little faster in the tile kernel, whose
-    // chain per token is shorter (64 heads of 64 x 128, us, lane groups / tiles: one entry of 8 tokens 8.5/10.4, of 16 14.5/12.5,
-    // of 64 43/33; four of 16 19.9/22.7; sixty-four of 1 53/99, of 16 255/278, of 32 479/470, of 64 925/853).
-    const int lanes = tokens <= (long long)(entries * (long long)H >= 148 ? 28 : 10) * entries ? se::row_lanes(N) : 0;
+    const int lanes = se_ssm_scan_by_lanes(H, P, N, tokens, entries, max_q_len, sms) ? se::row_lanes(N) : 0;
     if (lanes != 0 && (H * P) % 4 == 0 && se::rows_aligned(state, state_pitch, xbc, nullptr)) {
         const int per = se::kRowWarps * (32 / lanes) * 8;
         const dim3 grid(entries, H, se::ceil_div(P, per));

@@ -1,0 +1,30 @@
+"""Which form the state space's token-by-token recurrence takes, by the longest entry and the step's states (no GPU)."""
+import pytest
+
+from sparseengine_b200.csrc import ops
+
+
+@pytest.mark.parametrize("heads,size,lens,lanes", [
+    # portions beside single tokens, measured us lane groups / tiles: 61/38, 62/56, 69/79, 125/148, 221/205, 84/49
+    (64, 128, [64] + [1] * 3, 0), (64, 128, [64] + [1] * 15, 0), (64, 128, [64] + [1] * 31, 1), (64, 128, [90] + [1] * 63, 1),
+    (64, 128, [200] + [1] * 63, 0), (64, 128, [90] + [1] * 3, 0),
+    # 8.2/10.3, 43/33, 53/99, 265/302, and with fewer and more heads 41/29, 12/25, 186/257, 187/135
+    (64, 128, [8], 1), (64, 128, [64], 0), (64, 128, [1] * 64, 1), (64, 128, [17] * 64, 1),
+    (16, 64, [64] + [1] * 7, 0), (16, 64, [1] * 128, 1), (128, 128, [90] + [1] * 63, 1), (128, 128, [200] + [1] * 7, 0)])
+def test_by_the_longest_entry(heads, size, lens, lanes):
+    assert ops.library().se_ssm_scan_by_lanes(heads, 64, size, sum(lens), len(lens), max(lens), 148) == lanes
+
+
+def test_the_launcher_hears_of_the_longest_entry_and_the_device(monkeypatch):
+    from types import SimpleNamespace
+
+    import torch
+    seen = []
+    monkeypatch.setattr(ops, "_fn", lambda name, types: lambda *args: seen.append(args) or 0)
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 99)
+    monkeypatch.setattr(ops, "_stream", lambda: None)
+    monkeypatch.setattr(ops, "_ptr", lambda *args: 0)
+    f, i = torch.zeros(4, 8), torch.zeros(3, dtype=torch.int32)
+    step = SimpleNamespace(cu_q=i, seq_rows=i, num_seqs=2, max_q_len=3)
+    ops.ssm_scan(f, f, 0, f[0], f[0], f[0], f, step, f.clone(), heads=1, head_dim=4, state_size=2, groups=1)
+    assert seen[0][-4:-2] == (3, 99)
