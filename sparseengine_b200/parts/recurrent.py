@@ -14,7 +14,7 @@ import torch
 
 from ..config.specs import ParamSpec
 from ..csrc import ops
-from .base import Mixer, StateRequest, make_position, register_mixer
+from .base import Mixer, StateRequest, make_position, once_per_step, register_mixer
 from .linear import linear, pad_rows
 from .position import as_rotary_args
 
@@ -25,23 +25,34 @@ def _check_state_rows(rows: int, what: str) -> None:
                          "column's rows live in the registers of one warp's lanes)")
 
 
-def takes_chunks(mixer, step, heads: int, rows: int, columns: int, prepare: float, device) -> bool:
+def takes_chunks(mixer, step, heads: int, rows: int, columns: int, prepare: float, device, *, chunk: int = 64, block=(22.0, 4.0),
+                 launches: float = 8.0, token: float = 0.58, walk=None) -> bool:
     """Whether a step's recurrence runs in chunks: by what either form is estimated to take (us), if the longest entry has
-    ``chunk_min_tokens`` tokens (by that number alone where ``chunks_by_estimate`` is off).  Token by token: 0.62 per token of the
-    longest entry, or 5.5e-5 per token and state column of 128 rows where the device is full.  In chunks: 15 for the launches, 12 + 6.3 per 64 tokens for each block of 32 columns of an
-    entry, ``prepare`` per token and head.  Measured on one B200 (state space of 64 heads, 64 x 128; delta per channel and per head, 16
-    heads of 128 x 128; us token by token / in chunks): one entry of 32 tokens 24/27, 27/29, 25/29, of 64 43/31, 42/31, 41/35; four of
-    64 62/73, 49/60, 47/58, of 128 118/96, 86/86, 87/85; sixty-four of 64 923/1,074, 514/734, 509/708, of 128 1,817/1,414,
-    1,007/1,128, 997/1,030; one of 2,048 about 850/225, 1,000/480, 1,000/245."""
+    ``chunk_min_tokens`` tokens (by that number alone where ``chunks_by_estimate`` is off).  ``walk``: token by token, of the longest
+    entry's tokens, the entries and all tokens; by default ``token`` per token of the longest, or 5.9e-5 per token and state column of 128 rows
+    where the device is full.  In chunks: ``launches``, then ``block`` = (an entry's first chunk, each further one) for each block of 32
+    columns, side by side over the device, and ``prepare`` per head and token of the chunks, full or not: single tokens beside a
+    portion cost a block and a chunk each, which is why the entries' own lengths count.  Measured on one B200, a layer (state space
+    of 64 heads, 64 x 128; delta per channel and per head, 16 heads of 128 x 128), us token by token / in chunks: one entry of 48 tokens
+    51/57, 62/57, 57/55, of 128 86/66, 109/64, 100/62, of 2,048 975/349, 1,537/371, 1,416/336; four of 96 135/150, 110/116,
+    100/113, of 192 238/195, 180/164, 177/152; sixty-four of 64 1,099/1,318, 686/908, 693/895; one of 300 beside 7 single tokens
+    190/219, 237/174, 228/166, beside 31 188/588, 244/367, 234/403, of 1,024 beside 31 594/752, 791/546, 753/577."""
     longest = step.max_q_len
     if mixer.chunk_min_tokens is None or longest < mixer.chunk_min_tokens:
         return False
     if not getattr(mixer, "chunks_by_estimate", True):
         return True
-    walk = max(0.62 * longest, 4.3e-7 * step.num_tokens * heads * columns * rows)
-    share = heads * -(-columns // 32) / ops.sm_count(device)       # of a full device that an entry's blocks are
-    chunks = max(12 + 0.1 * longest, (12 * step.num_seqs + 0.1 * step.num_tokens) * share)
-    return 15 + chunks + prepare * step.num_tokens * heads < walk
+    entries, tokens, sms = step.num_seqs, step.num_tokens, ops.sm_count(device)
+    lens = getattr(step, "q_lens", None) or [longest] + [(tokens - longest) // max(1, entries - 1)] * (entries - 1)
+    pieces = sum(-(-n // chunk) for n in lens)
+    if walk is not None:
+        one_by_one = walk(longest, entries, tokens)
+    else:
+        one_by_one = 4 + 0.06 * entries + max(token * longest, 4.5e-7 * 148 / sms * tokens * heads * columns * rows)
+    first, further = block
+    share = heads * -(-columns // 32) / sms                        # of a full device that an entry's blocks are
+    chunks = max(first + further * (-(-longest // chunk) - 1), (first * entries + further * (pieces - entries)) * share)
+    return launches + chunks + prepare * chunk * pieces * heads < one_by_one
 
 
 class StateSpaceMixer(Mixer):
@@ -85,6 +96,19 @@ class StateSpaceMixer(Mixer):
     def state_request(self):
         return StateRequest((self.conv_off + (self.spec.conv_taps - 1) * self.conv_channels,), torch.float32)
 
+    def in_chunks(self, step, device) -> bool:
+        if self.chunk_min_tokens is None or step.max_q_len < self.chunk_min_tokens:
+            return False
+        s = self.spec
+        size = s.num_heads * s.head_dim * s.state_size / 524288 * 148 / ops.sm_count(device)
+
+        def walk(longest, entries, tokens):          # the shorter of csrc/recurrent.cu's two forms, lane groups and tiles
+            return min(3 + 0.65 * size * entries + max(max(0.8, 0.45 * size) * longest, 0.24 * size * tokens),
+                       6 + 1.45 * size * entries + max(max(0.44, 0.33 * size) * longest, 0.23 * size * tokens))
+        return once_per_step(step, ("state_space.in_chunks", s.num_heads, s.state_size, s.head_dim), lambda: (
+            takes_chunks(self, step, s.num_heads, s.state_size, s.head_dim, 2.1e-4, device, block=(19.5, 7.0), launches=17.0, walk=walk)
+            and ops.chunk_walk_supported(s.state_size, s.head_dim)))
+
     def forward(self, x, step, slot):
         s = self.spec
         tokens = x.shape[0]
@@ -92,9 +116,7 @@ class StateSpaceMixer(Mixer):
         xbc = torch.empty(tokens, self.conv_channels, dtype=torch.float32, device=x.device)
         ops.causal_conv(proj, self.inner, self.conv_w, self.conv_b, slot.state, self.conv_off, step, xbc)
         y = torch.empty(tokens, self.inner, dtype=torch.float32, device=x.device)
-        walk = (takes_chunks(self, step, s.num_heads, s.state_size, s.head_dim, 2e-4, x.device)
-                and ops.chunk_walk_supported(s.state_size, s.head_dim))
-        (ops.ssm_walk if walk else ops.ssm_scan)(
+        (ops.ssm_walk if self.in_chunks(step, x.device) else ops.ssm_scan)(
             xbc, proj, self.inner + self.conv_channels, self.dt_bias, self.a_log, self.d_skip, slot.state, step, y,
             heads=s.num_heads, head_dim=s.head_dim, state_size=s.state_size, groups=s.groups)
         gated = torch.empty(tokens, self.inner, dtype=x.dtype, device=x.device)
@@ -160,6 +182,14 @@ class GatedDeltaMixer(Mixer):
     def state_request(self):
         return StateRequest((self.conv_off + (self.spec.conv_taps - 1) * self.conv_channels,), torch.float32)
 
+    def in_chunks(self, step, device) -> bool:
+        if self.chunk_min_tokens is None or step.max_q_len < self.chunk_min_tokens:
+            return False
+        s = self.spec
+        costs = (dict(prepare=1.9e-3) if self.per_head else dict(prepare=2.8e-3, chunk=32, block=(15.0, 3.0), launches=15.0, token=0.63))
+        return once_per_step(step, ("delta.in_chunks", self.per_head, s.num_heads, s.head_dim, s.v_head_dim), lambda: (
+            takes_chunks(self, step, s.num_heads, s.head_dim, s.v_head_dim, device=device, **costs)))
+
     def forward(self, x, step, slot):
         s = self.spec
         tokens, dev = x.shape[0], x.device
@@ -173,7 +203,7 @@ class GatedDeltaMixer(Mixer):
         # (single tokens, short pieces, head sizes the chunks do not take) prepare q, k, decays and beta, then walk the tokens.
         sizes, inputs = self.sizes, self.inputs
         o = torch.empty(tokens, self.vv, dtype=torch.float32, device=dev)
-        long = takes_chunks(self, step, s.num_heads, s.head_dim, s.v_head_dim, 2.1e-3 if self.per_head else 2.5e-3, dev)
+        long = self.in_chunks(step, dev)
         # (decays per channel are read four at a time: a bias bound as a view off 16 bytes goes token by token)
         if (long and ops.chunk_walk_supported(s.head_dim, s.v_head_dim)
                 and (self.per_head or (self.dt_bias.data_ptr() | a.data_ptr()) % 16 == 0)):

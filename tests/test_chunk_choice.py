@@ -1,6 +1,8 @@
 """Which form a recurrence takes, by the step's entries (no GPU)."""
 from types import SimpleNamespace
 
+import pytest
+
 from sparseengine_b200.csrc import ops
 from sparseengine_b200.parts import recurrent
 
@@ -17,3 +19,25 @@ def test_choice(monkeypatch):
     assert not takes([2048], least=None) and not takes([2048], least=4096)
     delta = dict(heads=16, rows=128, columns=128, prepare=2.5e-3)
     assert takes([1500, 1037, 1323, 860], **delta) and not takes([64] * 64, **delta)
+
+
+@pytest.mark.parametrize("lens,state_space,channel,head", [
+    # short pieces beside a portion, a layer, us token by token / in chunks: 188/588, 244/367, 234/403; 594/752, 791/546, 753/577;
+    # 360/422, 425/324, 415/338; 614/1,194, 512/720, 504/814
+    ([300] + [1] * 31, False, False, False), ([1024] + [1] * 31, False, True, True), ([600] + [1] * 15, False, True, True),
+    ([500] + [1] * 63, False, False, False), ([200] + [1] * 15, False, False, False), ([130] + [1] * 3, False, True, True),
+    ([300] + [1] * 7, False, True, True), ([2048] + [1] * 31, True, True, True),
+    # alone and side by side: 86/66, 109/64, 100/62; 238/195, 180/164, 177/152; 2,096/1,886, 1,335/1,457, 1,350/1,391
+    ([128], True, True, True), ([192] * 4, True, True, True), ([128] * 64, True, False, False), ([64] * 64, False, False, False)])
+def test_by_the_entries_own_tokens(monkeypatch, lens, state_space, channel, head):
+    import torch
+
+    from sparseengine_b200.config.specs import GatedDeltaSpec, StateSpaceSpec
+    from sparseengine_b200.parts.base import make_mixer
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    step = SimpleNamespace(max_q_len=max(lens), num_tokens=sum(lens), num_seqs=len(lens), q_lens=lens)
+    delta = dict(hidden_size=64, num_heads=16, num_kv_heads=16, head_dim=128, v_head_dim=128, conv_taps=4)
+    specs = [StateSpaceSpec(hidden_size=64, num_heads=64, head_dim=64, state_size=128, groups=8, conv_taps=4, norm_groups=8),
+             GatedDeltaSpec(**delta, decay_per="channel", gate_activation="sigmoid", decay_rank=8, gate_rank=8),
+             GatedDeltaSpec(**delta, decay_per="head", gate_activation="silu")]
+    assert [make_mixer(s, torch.bfloat16).in_chunks(step, "cuda:0") for s in specs] == [state_space, channel, head]
