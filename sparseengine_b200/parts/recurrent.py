@@ -281,6 +281,25 @@ class RetentionMixer(Mixer):
         s = self.spec
         return StateRequest((s.num_heads * s.head_dim * s.v_head_dim,), torch.float32)
 
+    def in_walk(self, step, device) -> bool:
+        """Whether a step in chunks has them prepared side by side and walked, or goes through the kernel that does a chunk at a time.
+        The walk's blocks take an SM each and 2.5 us more for an entry's first chunk, but 6 less for each further one, or 0.25 a token of
+        the longest entry, which the other kernel takes in segments.  Measured, a layer, us chunk at a time / walk, 16 and 32 heads of
+        128 x 128: one portion of 90 tokens beside 63 single ones 434/491 and 857/983, of 300 515/526 and 968/1,034, of 1,024 838/648
+        and 1,380/1,239, of 90 beside 15 151/127 and 286/301; 64 entries of 96 tokens 1,045/914 and 2,368/2,099; four
+        entries of 17 to 64 tokens, 32 heads, 118 to 135 against 124 to 143 with the host's launches.  Where all blocks run at once
+        the walk is ahead from the first chunk on (one such entry 92 and 76)."""
+        s = self.spec
+
+        def ask():
+            share = s.num_heads * -(-s.v_head_dim // 32) / ops.sm_count(device)        # of a full device that an entry's blocks are
+            if step.num_seqs * share <= 1:
+                return True
+            lens = getattr(step, "q_lens", None) or [step.max_q_len] * step.num_seqs
+            further = sum(-(-n // 64) for n in lens) - len(lens)
+            return step.max_q_len > 64 and 2.5 * step.num_seqs * share < max(0.25 * step.max_q_len, 6 * further * share)
+        return once_per_step(step, ("retention.in_walk", s.num_heads, s.v_head_dim), ask)
+
     def forward(self, x, step, slot, proj=None):
         s = self.spec
         tokens, dev = x.shape[0], x.device
@@ -303,11 +322,8 @@ class RetentionMixer(Mixer):
         sizes = dict(heads=s.num_heads, head_dim=s.head_dim, v_head_dim=s.v_head_dim, silu=silu)
         if not chunked and rotary_dim == 0:      # q and k straight from the projection, as they are staged
             ops.retention_scan(None, None, *args, **sizes, qk=(0, self.qk, self.k_scale))
-        elif (chunked and ops.retention_walk_supported(s.head_dim, s.v_head_dim, rotary_dim, proj, self.qk)
-              and (inv_freq is None or inv_freq.data_ptr() % 16 == 0)
-              # entries of one chunk that fill the device go faster through the kernel that does a chunk at a time (a layer of 32 heads
-              # of 128 x 128, four entries of 17 to 64 tokens: 118 to 135 us against 124 to 143; one entry: 87 against 76)
-              and (step.max_q_len > 64 or step.num_seqs * s.num_heads * (-(-s.v_head_dim // 32)) <= ops.sm_count(dev))):
+        elif (chunked and self.in_walk(step, dev) and ops.retention_walk_supported(s.head_dim, s.v_head_dim, rotary_dim, proj, self.qk)
+              and (inv_freq is None or inv_freq.data_ptr() % 16 == 0)):
             ops.retention_chunk(None, None, *args, **sizes, qk=(0, self.qk, self.k_scale),
                                 rotation=(inv_freq, rotary_dim, step.positions) if rotary_dim else None)
         else:

@@ -41,3 +41,20 @@ def test_by_the_entries_own_tokens(monkeypatch, lens, state_space, channel, head
              GatedDeltaSpec(**delta, decay_per="channel", gate_activation="sigmoid", decay_rank=8, gate_rank=8),
              GatedDeltaSpec(**delta, decay_per="head", gate_activation="silu")]
     assert [make_mixer(s, torch.bfloat16).in_chunks(step, "cuda:0") for s in specs] == [state_space, channel, head]
+
+
+@pytest.mark.parametrize("lens,sixteen,thirty_two", [
+    # a layer, us chunk at a time / walk, 16 and 32 heads: 434/491, 857/983; 484/516, 930/1,022; 631/575, 1,139/1,128; 286/301 at 32
+    ([90] + [1] * 63, False, False), ([150, 150] + [1] * 62, False, False), ([600] + [1] * 63, True, True), ([90] + [1] * 15, True, False),
+    # 1,045/914, 2,368/2,099; 300/260, 682/614; one chunk: 92/76 alone and 118 to 135 / 124 to 143 for four entries of 32 heads
+    ([96] * 64, True, True), ([128] * 16, True, True), ([64], True, True), ([65] * 4, True, True), ([64] * 4, False, False)])
+def test_retention_walk_by_the_entries_own_tokens(monkeypatch, lens, sixteen, thirty_two):
+    import torch
+
+    from sparseengine_b200.config.specs import RetentionSpec
+    from sparseengine_b200.parts.base import make_mixer
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    step = SimpleNamespace(max_q_len=max(lens), num_tokens=sum(lens), num_seqs=len(lens), q_lens=lens)
+    for heads, walk in ((16, sixteen), (32, thirty_two)):
+        part = make_mixer(RetentionSpec(hidden_size=64, num_heads=heads, head_dim=128, v_head_dim=128, decays=(0.9,) * heads, position=None), torch.bfloat16)
+        assert part.in_walk(step, "cuda:0") is walk
