@@ -146,9 +146,11 @@ extern "C" int se_paged_attention_plain(const void* q, const void* cache, const 
                                         const int* seq_rows, const int* token_seq, const int* positions, void* out,
                                         int tokens, int hq, int hkv, int d, int dv, int page_size, float scale, int window,
                                         int num_pages, int* error, float softcap, int sink, const void* gate, int gate_pitch,
-                                        const float* sink_logits, int keep_first, const float* slopes, int gate_per_head, int dtype,
+                                        const float* sink_logits, int keep_first, const float* slopes, int gate_per_head, int sms, int dtype,
                                         cudaStream_t stream) {
+    // sms: the device's SMs
     if (tokens <= 0) return 0;
+    if (sms < 1) return SE_ERR_ARGUMENT;
     if (softcap < 0.f || (gate != nullptr && gate_pitch < (gate_per_head ? hq : hq * dv)) || keep_first < 0) return SE_ERR_ARGUMENT;
     if (sink_logits != nullptr) sink = 1;
     if (window <= 0) keep_first = 0;
@@ -163,10 +165,10 @@ extern "C" int se_paged_attention_plain(const void* q, const void* cache, const 
         scale, window, num_pages, error, softcap, sink, (const T*)gate, gate_pitch, sink_logits, keep_first, slopes, gate_per_head)
     SE_DISPATCH_DTYPE(dtype, T, {
         // as many warps as leave all blocks on the device at once (64 registers a thread; 96 for the wide heads)
-        if (wide && blocks <= 148) SE_PLAIN(8, 16);
+        if (wide && blocks <= sms) SE_PLAIN(8, 16);
         else if (wide) SE_PLAIN(8, 4);
-        else if (blocks <= 148 * 2) SE_PLAIN(4, 16);
-        else if (blocks <= 148 * 4) SE_PLAIN(4, 8);
+        else if (blocks <= 2 * sms) SE_PLAIN(4, 16);
+        else if (blocks <= 4 * sms) SE_PLAIN(4, 8);
         else SE_PLAIN(4, 4);
     });
 #undef SE_PLAIN

@@ -253,7 +253,7 @@ def paged_attention_plain(q, cache, table, seq_rows, token_seq, positions, out, 
         raise ValueError("gate must be a matrix of q's dtype with contiguous rows")
     sink_logits = _sink_logits(sink, num_heads)
     per_head = _gate_per_head(gate, num_heads, int(v_head_dim or head_dim))
-    _check(_fn("se_paged_attention_plain", "pppipppp" "iiiiii" "f" "iip" "fipi" "pip" "iip")(
+    _check(_fn("se_paged_attention_plain", "pppipppp" "iiiiii" "f" "iip" "fipi" "pip" "iiip")(
         _ptr(q, None, "q"), _ptr(cache, dt, "cache"), _ptr(table, torch.int32, "table"), table.shape[1],
         _ptr(seq_rows, torch.int32, "seq_rows"), _ptr(token_seq, torch.int32, "token_seq"),
         _ptr(positions, torch.int32, "positions"), _ptr(out, dt, "out"), tokens, num_heads, num_kv_heads,
@@ -261,7 +261,7 @@ def paged_attention_plain(q, cache, table, seq_rows, token_seq, positions, out, 
         cache.shape[0] if num_pages is None else int(num_pages), _ptr(error_word(q.device)),
         float(softcap or 0.0), _has_sink(sink), gate.data_ptr() if gate is not None else None,
         gate.stride(0) if gate is not None else 0, sink_logits, int(keep_first or 0), _slopes_ptr(slopes, num_heads),
-        per_head, dtype_code(dt), _stream()),
+        per_head, sm_count(q.device), dtype_code(dt), _stream()),
         "paged_attention_plain")
     return out
 

@@ -1,4 +1,4 @@
-"""Which form the state space's token-by-token recurrence takes, by the longest entry and the step's states (no GPU)."""
+"""What launchers are told to choose by: the longest entry, the step's states, the device's SMs (no GPU)."""
 import pytest
 
 from sparseengine_b200.csrc import ops
@@ -15,16 +15,28 @@ def test_by_the_longest_entry(heads, size, lens, lanes):
     assert ops.library().se_ssm_scan_by_lanes(heads, 64, size, sum(lens), len(lens), max(lens), 148) == lanes
 
 
-def test_the_launcher_hears_of_the_longest_entry_and_the_device(monkeypatch):
+@pytest.fixture
+def seen(monkeypatch):
+    """The arguments that launchers are called with, on a device of 99 SMs."""
+    calls = []
+    monkeypatch.setattr(ops, "_fn", lambda name, types: lambda *args: calls.append(args) or 0)
+    for name, value in (("sm_count", 99), ("_stream", None), ("_ptr", 0), ("error_word", None)):
+        monkeypatch.setattr(ops, name, lambda *args, value=value: value)
+    return calls
+
+
+def test_the_scan_hears_of_the_longest_entry_and_the_device(seen):
     from types import SimpleNamespace
 
     import torch
-    seen = []
-    monkeypatch.setattr(ops, "_fn", lambda name, types: lambda *args: seen.append(args) or 0)
-    monkeypatch.setattr(ops, "sm_count", lambda device=None: 99)
-    monkeypatch.setattr(ops, "_stream", lambda: None)
-    monkeypatch.setattr(ops, "_ptr", lambda *args: 0)
     f, i = torch.zeros(4, 8), torch.zeros(3, dtype=torch.int32)
     step = SimpleNamespace(cu_q=i, seq_rows=i, num_seqs=2, max_q_len=3)
     ops.ssm_scan(f, f, 0, f[0], f[0], f[0], f, step, f.clone(), heads=1, head_dim=4, state_size=2, groups=1)
     assert seen[0][-4:-2] == (3, 99)
+
+
+def test_plain_attention_hears_of_the_device(seen):
+    import torch
+    f, i = torch.zeros(4, 8), torch.zeros(4, dtype=torch.int32)
+    ops.paged_attention_plain(f, f, i.view(2, 2), i, i, i, f.clone(), num_heads=2, num_kv_heads=1, head_dim=4, page_size=4, scale=1.0)
+    assert seen[0][-3] == 99
