@@ -13,7 +13,8 @@
 // Query/key and value head sizes that are multiples of 4 up to 128; the options are the plain kernel's, and so is what a query
 // sees (first_visible, keep_first).  Exponentials are expf, the probabilities stay 32-bit.  A block-table entry outside
 // [0, num_pages) is not followed: its key is left out and a code goes to the error word.  A key that a row does not see does
-// not touch it, whatever it holds: where a tile's values are not all finite, products with a zero weight are left out.
+// not touch it, whatever it holds: where a tile's values are not all finite, its products are left out (those of a seen key whose
+// weight underflows to zero are not: there infinity times zero shows, as in the plain kernel).
 #include "common.cuh"
 #include <type_traits>
 
@@ -197,9 +198,11 @@ attn_prefill_f32_kernel(const float* __restrict__ q, const float* __restrict__ c
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const float pv = kk == 0 ? p[i].x : kk == 1 ? p[i].y : kk == 2 ? p[i].z : p[i].w;
+                        const int j = j0 + k + kk;
+                        if (decltype(guarded)::value && !(key_ok[it & 1][k + kk] && j <= pos[i] && (j >= first[i] || j < keep_first))) continue;
 #pragma unroll
                         for (int c = 0; c < kCols; ++c)
-                            if (!decltype(guarded)::value || pv != 0.f) o[i][c] = fmaf(pv, v[c], o[i][c]);
+                            o[i][c] = fmaf(pv, v[c], o[i][c]);
                     }
                 }
             }

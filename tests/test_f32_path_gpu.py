@@ -180,3 +180,25 @@ def test_portions_on_odd_addresses_take_the_plain_kernel():
     for odd in tensors:
         got, tiled = attend(odd)
         assert tiled == 0 and float((got - want).abs().max()) < 4e-6
+
+
+def test_a_seen_key_without_weight_still_shows_what_is_not_finite():
+    """A value of infinity under a weight that underflows to zero gives NaN for the rows that see it, as in the plain kernel."""
+    from sparseengine_b200.csrc import ops
+    b = _batch([150], [150], 16, 1)
+    kv_heads, heads, d = 1, 2, 64
+    cache = torch.randn(b["pages"], 2, kv_heads, 16, d, device=DEV)
+    q = torch.randn(150, heads, d, device=DEV)
+    q[:, :, 0] = 10.0
+    at, slot = int(b["table"][0, 70 // 16]), 70 % 16
+    cache[at, 0, 0, slot] = 0.0
+    cache[at, 0, 0, slot, 0] = -1000.0         # scores of -1,250
+    cache[at, 1, 0, slot, 5] = float("inf")
+    common = dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=d, page_size=16, scale=0.125)
+    want, got = torch.empty(150, heads * d, device=DEV), torch.empty(150, heads * d, device=DEV)
+    ops.paged_attention_plain(q.view(150, -1), cache, b["table"], b["rows"], b["seq"], b["pos"], want, **common)
+    ops.attn_prefill_f32(q.view(150, -1), cache, b["table"], b["rows"], b["cu"], b["kv"], got, entries=1, max_q_len=150, **common)
+    ops.error_check(DEV)
+    bad = ~torch.isfinite(want)
+    assert torch.equal(~torch.isfinite(got), bad) and bool(bad.view(150, heads, d)[70:, :, 5].all()) and int(bad.sum()) == 80 * heads
+    assert float((got - want)[~bad].abs().max()) < 4e-6
