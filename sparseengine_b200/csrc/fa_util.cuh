@@ -28,6 +28,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
     return false;
 }
+// The same whatever else has gone wrong: after a failure, for copies and products that are still in flight.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < kSpin && !mbar_try_wait(bar, parity); ++i) {}
+}
 // One lane of a converged warp.  What an MMA's issue needs lies in uniform registers; code under a branch that the compiler
 // takes for divergent (lane == 0) moves every operand there for every MMA, about 100 cycles each.  So the issuing warp runs
 // as a whole through warp-uniform loops and only the MMAs are one lane's.

@@ -43,7 +43,7 @@ struct Bars {
     uint64_t kv_full[kMaxStages], kv_empty[kMaxStages];
     uint64_t s_full[kTiles][2], s_empty[kTiles][2];
     uint64_t p_full[kTiles][2], p_empty[kTiles];
-    uint64_t o_done[kTiles], q_full[kTiles];
+    uint64_t o_done[kTiles], q_full[kTiles], all_done;
 };
 
 // db, rb: blocks of 64 dims of a row and of its latent part; buffers: S buffers per query tile; stages: key tiles in flight
@@ -89,6 +89,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __nv
             mbar_init(bar(&bars.o_done[x]), 1);
             mbar_init(bar(&bars.q_full[x]), 1);
         }
+        mbar_init(bar(&bars.all_done), 1);
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -246,7 +247,13 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __nv
         }
         if (ok && elect_one())
             for (int x = 0; x < kTiles; ++x) umma_commit(bar(&bars.o_done[x]));
-        if (!ok) { abort_s = 1; if (lane == 0) atomicCAS(error, 0, 16); }
+        if (!ok) {       // a wait ran out: what is on its way into the block's memory ends (or runs out, too) before that is given back
+            abort_s = 1;
+            if (lane == 0) atomicCAS(error, 0, 16);
+            if (elect_one()) umma_commit(bar(&bars.all_done));
+            for (int x = 0; x < kTiles; ++x) mbar_drain(bar(&bars.q_full[x]), 0);
+            mbar_drain(bar(&bars.all_done), 0);
+        }
         __syncwarp();
     } else if (warp < 2 + 4 * kTiles) {
         // ---- softmax and epilogue: four warps per query tile, one thread per row --------------------
