@@ -18,7 +18,7 @@ import sys
 
 import torch
 
-from .kernel_bench import peaks, timed
+from .kernel_bench import design_mixers, peaks, timed
 
 PAGE_SIZE = 16
 VOCAB = 32768
@@ -173,13 +173,15 @@ def _kernels(width: int, tokens_list, pk: dict) -> dict:
     dev = torch.device("cuda:0")
     cfg = hybrid_config(width)
     m2, dl = cfg["layers"][1]["mixer"], cfg["layers"][2]["mixer"]
+    ssm_part, delta_part = design_mixers(cfg, torch.bfloat16)[1:3]
     heads = width // 128
     out = {}
     for tokens, entries in tokens_list:
         per = tokens // entries
         step = SimpleNamespace(token_seq=torch.arange(tokens, device=dev, dtype=torch.int32) // per,
                                cu_q=torch.arange(entries + 1, device=dev, dtype=torch.int32) * per,
-                               seq_rows=torch.arange(entries, device=dev, dtype=torch.int32), num_seqs=entries,
+                               seq_rows=torch.arange(entries, device=dev, dtype=torch.int32), num_seqs=entries, num_tokens=tokens,
+                               max_q_len=per, q_lens=[per] * entries,
                                positions=(torch.arange(tokens, device=dev, dtype=torch.int32) % per) + 2048)
         rec = {}
 
@@ -211,9 +213,10 @@ def _kernels(width: int, tokens_list, pk: dict) -> dict:
         dtb, al, dk = torch.zeros(H, device=dev), torch.zeros(H, device=dev), torch.ones(H, device=dev)
         yy = torch.empty(tokens, inner, device=dev)
         scan_bytes = tokens * (C + inner) * 4 + entries * H * P * N * 8
-        add("ssm_scan", lambda: ops.ssm_scan(xbc, proj, inner + C, dtb, al, dk, state, step, yy, heads=H, head_dim=P,
+        name = "ssm_walk" if ssm_part.in_chunks(step, dev) else "ssm_scan"
+        add(name, lambda: getattr(ops, name)(xbc, proj, inner + C, dtb, al, dk, state, step, yy, heads=H, head_dim=P,
                                              state_size=N, groups=G), scan_bytes, iters=5)
-        rec["ssm_scan"]["us_per_token_of_a_request"] = round(rec["ssm_scan"]["us"] / per, 3)
+        rec[name]["us_per_token_of_a_request"] = round(rec[name]["us"] / per, 3)
         nw, gg = torch.ones(inner, device=dev), torch.empty(tokens, inner, device=dev, dtype=bf)
         add("gated_group_norm", lambda: ops.gated_group_norm(yy, proj, 0, nw, gg, parts=8, eps=1e-6), tokens * inner * 8)
         # gated delta
@@ -227,12 +230,19 @@ def _kernels(width: int, tokens_list, pk: dict) -> dict:
         a = torch.randn(tokens, H * d, device=dev, dtype=bf)
         dec, beta = torch.empty(tokens, H * d, device=dev), torch.empty(tokens, H, device=dev)
         dtb2, al2 = torch.zeros(H * d, device=dev), torch.zeros(H, device=dev)
-        add("delta_prep", lambda: ops.delta_prep(qkv, a, proj2, C, dtb2, al2, dec, beta, heads=H, kv_heads=Gk, head_dim=d,
-                                                 v_head_dim=dv, unit_eps=1e-6, q_scale=d ** -0.5), tokens * (2 * Gk * d * 8 + H * d * 6))
+        sizes, inputs = dict(heads=H, kv_heads=Gk, head_dim=d, v_head_dim=dv), dict(unit_eps=1e-6, q_scale=d ** -0.5)
         oo2 = torch.empty(tokens, H * dv, device=dev)
-        add("delta_scan", lambda: ops.delta_scan(qkv, dec, beta, state2, step, oo2, heads=H, kv_heads=Gk, head_dim=d, v_head_dim=dv),
-            tokens * (C + H * d + H * dv) * 4 + entries * H * d * dv * 8, iters=5)
-        rec["delta_scan"]["us_per_token_of_a_request"] = round(rec["delta_scan"]["us"] / per, 3)
+        if delta_part.in_chunks(step, dev):          # from the same inputs as the two kernels below
+            name, nbytes = "delta_walk", tokens * (C * 4 + H * d * 2 + H * dv * 4)
+            add(name, lambda: ops.delta_walk(qkv, a, proj2, C, dtb2, al2, state2, step, oo2, **sizes, **inputs),
+                nbytes + entries * H * d * dv * 8, iters=5)
+        else:
+            add("delta_prep", lambda: ops.delta_prep(qkv, a, proj2, C, dtb2, al2, dec, beta, **sizes, **inputs),
+                tokens * (2 * Gk * d * 8 + H * d * 6))
+            name = "delta_scan"
+            add(name, lambda: ops.delta_scan(qkv, dec, beta, state2, step, oo2, **sizes),
+                tokens * (C + H * d + H * dv) * 4 + entries * H * d * dv * 8, iters=5)
+        rec[name]["us_per_token_of_a_request"] = round(rec[name]["us"] / per, 3)
         gate, nw2, out2 = torch.randn(tokens, H * dv, device=dev, dtype=bf), torch.ones(dv, device=dev), torch.empty(tokens, H * dv, device=dev, dtype=bf)
         add("delta_out", lambda: ops.delta_out(oo2, gate, nw2, out2, heads=H, v_head_dim=dv, eps=1e-6), tokens * H * dv * 8)
         # query/key preparation (pages written round-robin)

@@ -39,6 +39,14 @@ def peaks() -> dict:
     return out
 
 
+def design_mixers(cfg: dict, dtype) -> list:
+    """The mixers of a design's layers, without weights: the design benches ask them which kernels a step takes."""
+    from .. import models  # noqa: F401  (registers the designs)
+    from ..config.registry import load_model_spec
+    from ..parts.base import make_mixer
+    return [make_mixer(layer.mixer, dtype) for layer in load_model_spec(cfg)[1].layers]
+
+
 def timed(fn, iters: int, warmup: int = 3) -> float:
     """Milliseconds per call.  The calls are captured into one CUDA graph and the graph is
     timed with CUDA events, so that short kernels are not measured by how fast Python can

@@ -70,7 +70,8 @@ def _kernels(width: int, cases, pk: dict) -> dict:
         per = tokens // entries
         step = SimpleNamespace(token_seq=torch.arange(tokens, device=dev, dtype=torch.int32) // per,
                                cu_q=torch.arange(entries + 1, device=dev, dtype=torch.int32) * per,
-                               seq_rows=torch.arange(entries, device=dev, dtype=torch.int32), num_seqs=entries, max_q_len=per,
+                               seq_rows=torch.arange(entries, device=dev, dtype=torch.int32), num_seqs=entries, num_tokens=tokens,
+                               max_q_len=per, q_lens=[per] * entries,
                                positions=(torch.arange(tokens, device=dev, dtype=torch.int32) % per) + held)
         kv_len = torch.full((entries,), held + per, device=dev, dtype=torch.int32)
         rec = {}
@@ -167,10 +168,13 @@ def _attention_kernels(width, tokens, entries, held, step, kv_len, add):
 
 
 def _lightning_kernels(width, tokens, entries, step, add):
+    from ..config.specs import RetentionSpec
     from ..csrc import ops
+    from ..parts.base import make_mixer
     dev, bf = torch.device("cuda:0"), torch.bfloat16
     H, d = max(1, width // 256), 128
     n, per = H * d, tokens // entries
+    part = make_mixer(RetentionSpec(hidden_size=width, num_heads=H, head_dim=d, v_head_dim=d, decays=(0.9,) * H, position=None), bf)
     proj = torch.randn(tokens, 4 * n, device=dev, dtype=bf) * 0.3
     q32, k32 = (torch.randn(tokens, n, device=dev) for _ in range(2))
     decay, state = torch.linspace(0.6, 0.9999, H, device=dev), torch.zeros(entries, H * d * d, device=dev)
@@ -179,10 +183,16 @@ def _lightning_kernels(width, tokens, entries, step, add):
     sizes = dict(heads=H, head_dim=d)
     nbytes = tokens * n * (4 + 8 + 2 + 4) + entries * n * d * 8
     if per > 1:
-        add("retention_prep (silu)", lambda: ops.retention_prep(proj, 0, n, None, step.positions, q32, k32, rotary_dim=0, k_scale=1.0, silu=True, **sizes), tokens * n * 12)
-        add("like: retention_prep (rotation)", lambda: ops.retention_prep(proj, 0, n, inv, step.positions, q32, k32, rotary_dim=d, k_scale=0.09, **sizes), tokens * n * 12)
-        for name, silu in (("retention_chunk (silu)", True), ("like: retention_chunk", False)):
-            add(name, lambda: ops.retention_chunk(q32, k32, proj, 2 * n, decay, state, step, o, v_head_dim=d, silu=silu, **sizes), nbytes, iters=5)
+        if part.in_walk(step, dev):      # q and k from the projection, prepared side by side, walked
+            for name, silu, rotation in (("retention_chunk (walked, silu)", True, None),
+                                         ("like: retention_chunk (walked, rotation)", False, (inv, d, step.positions))):
+                add(name, lambda: ops.retention_chunk(None, None, proj, 2 * n, decay, state, step, o, v_head_dim=d, silu=silu, **sizes,
+                                                      qk=(0, n, 1.0), rotation=rotation), nbytes - 4 * tokens * n, iters=5)
+        else:
+            add("retention_prep (silu)", lambda: ops.retention_prep(proj, 0, n, None, step.positions, q32, k32, rotary_dim=0, k_scale=1.0, silu=True, **sizes), tokens * n * 12)
+            add("like: retention_prep (rotation)", lambda: ops.retention_prep(proj, 0, n, inv, step.positions, q32, k32, rotary_dim=d, k_scale=0.09, **sizes), tokens * n * 12)
+            for name, silu in (("retention_chunk (silu)", True), ("like: retention_chunk", False)):
+                add(name, lambda: ops.retention_chunk(q32, k32, proj, 2 * n, decay, state, step, o, v_head_dim=d, silu=silu, **sizes), nbytes, iters=5)
     else:
         add("retention_scan (silu, straight from the projection)", lambda: ops.retention_scan(
             None, None, proj, 2 * n, decay, state, step, o, v_head_dim=d, silu=True, qk=(0, n, 1.0), **sizes), nbytes, iters=5)

@@ -124,16 +124,23 @@ def _kernels(width: int, cases, pk: dict) -> dict:
         qfull[:, :, :rank].normal_()
         o_lat = torch.empty(tokens, H, rank, device=dev, dtype=bf)
 
-        def tiled(window, sink):
+        def tc(window):          # which of the two a step of these sizes takes
+            return ops.latent_takes_tc(entries, per, H, rank, r, q_lens=[per] * entries, kv_lens=[held + per] * entries, window=window)
+
+        def latent(window, sink):
             most = held + per if window is None else min(held + per, window + per - 1)
+            if tc(window):
+                ops.latent_attention_tc(qfull, cache, btable, step.seq_rows, step.cu_q, kv_len, sink, o_lat, entries=entries,
+                                        max_q_len=per, heads=H, rank=rank, rot=r, page_size=PAGE_SIZE, scale=0.09, window=window)
+                return
             ops.latent_attention_tiled(qfull, cache, btable, step.seq_rows, step.cu_q, kv_len, sink, o_lat, entries=entries,
                                        max_q_len=per, heads=H, rank=rank, rot=r, page_size=PAGE_SIZE, scale=0.09, window=window,
                                        max_keys=most)
-        for name, window, sink in (("latent_attention_tiled (all keys)", None, None),
-                                   ("like: latent_attention_tiled (window, sink)", WINDOW, torch.zeros(H, device=dev))):
+        for name, window, sink in (("{} (all keys)", None, None), ("like: {} (window, sink)", WINDOW, torch.zeros(H, device=dev))):
+            name = name.format("latent_attention_tc" if tc(window) else "latent_attention_tiled")
             seen = sum(min(window or 1 << 30, held + i + 1) for i in range(per)) * entries
             key_rows = entries * (held + per if window is None else min(held + per, window + per - 1))
-            add(name, lambda: tiled(window, sink), nbytes=key_rows * D * 2 + tokens * H * (D + rank) * 2, flops=2.0 * seen * H * (D + rank))
+            add(name, lambda: latent(window, sink), nbytes=key_rows * D * 2 + tokens * H * (D + rank) * 2, flops=2.0 * seen * H * (D + rank))
         heads_out = torch.randn(tokens, H * dv, device=dev, dtype=bf)
         add("sigmoid_gate", lambda: ops.sigmoid_gate_(heads_out, proj[:, cols + D:]), tokens * H * dv * 6)
         # windowed attention with a distance bias
@@ -177,9 +184,13 @@ def _kernels(width: int, cases, pk: dict) -> dict:
         prr = torch.randn(tokens, 2 * qk + 2 * vv, device=dev, dtype=bf) * 0.3
         decay = torch.linspace(0.95, 0.9999, Hr, device=dev)
         rstate, ro = torch.zeros(entries, Hr * dr * dr, device=dev), torch.empty(tokens, vv, device=dev)
-        fn = ops.retention_chunk if per > 1 else ops.retention_scan
-        add("like: " + fn.__name__, lambda: fn(q32, k32, prr, 2 * qk, decay, rstate, step, ro, heads=Hr, head_dim=dr, v_head_dim=dr),
-            tokens * (2 * qk * 4 + vv * 6) + entries * Hr * dr * dr * 8, iters=5)
+        if per > 1:      # q and k from the projection, prepared side by side and walked
+            add("like: retention_chunk", lambda: ops.retention_chunk(None, None, prr, 2 * qk, decay, rstate, step, ro, heads=Hr, head_dim=dr,
+                                                                     v_head_dim=dr, qk=(0, qk, 1.0)),
+                tokens * (2 * qk * 2 + vv * 6) + entries * Hr * dr * dr * 8, iters=5)
+        else:
+            add("like: retention_scan", lambda: ops.retention_scan(q32, k32, prr, 2 * qk, decay, rstate, step, ro, heads=Hr, head_dim=dr,
+                                                                   v_head_dim=dr), tokens * (2 * qk * 4 + vv * 6) + entries * Hr * dr * dr * 8, iters=5)
         # the feed-forward's activation
         up = torch.randn(tokens, 4 * width, device=dev, dtype=bf)
         add("activation (squared relu)", lambda: ops.activation_(up, "relu2"), tokens * 4 * width * 4)

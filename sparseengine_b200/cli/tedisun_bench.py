@@ -21,7 +21,7 @@ import sys
 import torch
 
 from .hybrid_bench import PAGE_SIZE, VOCAB, _parts, _throughput
-from .kernel_bench import peaks, timed
+from .kernel_bench import design_mixers, peaks, timed
 from .zisevik_bench import zisevik_config
 
 WINDOW, KEPT, STREAMS = 1024, 4, 4
@@ -60,12 +60,14 @@ def _kernels(width: int, cases, pk: dict) -> dict:
     cfg = tedisun_config(width)
     dl, pm = cfg["layers"][0]["mixer"], cfg["layers"][1]["mixer"]
     bf = torch.bfloat16
+    delta_part = design_mixers(cfg, bf)[0]
     out = {}
     for tokens, entries, held in cases:
         per = tokens // entries
         step = SimpleNamespace(token_seq=torch.arange(tokens, device=dev, dtype=torch.int32) // per,
                                cu_q=torch.arange(entries + 1, device=dev, dtype=torch.int32) * per,
-                               seq_rows=torch.arange(entries, device=dev, dtype=torch.int32), num_seqs=entries, max_q_len=per,
+                               seq_rows=torch.arange(entries, device=dev, dtype=torch.int32), num_seqs=entries, num_tokens=tokens,
+                               max_q_len=per, q_lens=[per] * entries,
                                positions=(torch.arange(tokens, device=dev, dtype=torch.int32) % per) + held)
         kv_len = torch.full((entries,), held + per, device=dev, dtype=torch.int32)
         rec = {}
@@ -174,8 +176,10 @@ def _kernels(width: int, cases, pk: dict) -> dict:
                                                                v_head_dim=dvm), tokens * (2 * qk * 4 + vv * 6) + entries * Hm * dm * dvm * 8, iters=5)
         rec["like: retention_scan"]["us_per_token_of_a_request"] = round(rec["like: retention_scan"]["us"] / per, 3)
         if per >= 16:
-            add("like: retention_chunk", lambda: ops.retention_chunk(q32, k32, proj_r, 2 * qk, decay, state_r, step, o_r, heads=Hm, head_dim=dm,
-                                                                     v_head_dim=dvm), tokens * (2 * qk * 4 + vv * 6) + entries * Hm * dm * dvm * 8, iters=5)
+            # q and k from the projection, prepared side by side and walked
+            add("like: retention_chunk", lambda: ops.retention_chunk(None, None, proj_r, 2 * qk, decay, state_r, step, o_r, heads=Hm, head_dim=dm,
+                                                                     v_head_dim=dvm, qk=(0, qk, dm ** -0.5)),
+                tokens * (2 * qk * 2 + vv * 6) + entries * Hm * dm * dvm * 8, iters=5)
             rec["like: retention_chunk"]["us_per_token_of_a_request"] = round(rec["like: retention_chunk"]["us"] / per, 3)
         add("like: retention_out", lambda: ops.retention_out(o_r, proj_r, 2 * qk + vv, gm, heads=Hm, v_head_dim=dvm, eps=1e-6), tokens * vv * 8)
         # delta rule: one decay per head (the recurrence is the closest model's own kernel)
@@ -185,19 +189,21 @@ def _kernels(width: int, cases, pk: dict) -> dict:
         qkv = torch.randn(tokens, C, device=dev) * 0.1
         dec, beta = torch.empty(tokens, Hd * dd, device=dev), torch.empty(tokens, Hd, device=dev)
         dtb, alog, nwd = torch.zeros(Hd, device=dev), torch.zeros(Hd, device=dev), torch.ones(dvd, device=dev)
-        add("delta_prep (one decay per head)", lambda: ops.delta_prep(
-            qkv, proj_d[:, C + Hd:C + 2 * Hd], proj_d, C, dtb, alog, dec, beta, heads=Hd, kv_heads=Gd, head_dim=dd, v_head_dim=dvd,
-            unit_eps=1e-6, q_scale=dd ** -0.5, per_head=True), tokens * (2 * Gd * dd * 8 + Hd * dd * 4))
         state_d = torch.zeros(entries, Hd * dd * dvd + 3 * C, device=dev)
         o_d = torch.empty(tokens, Hd * dvd, device=dev)
-        add("delta_scan", lambda: ops.delta_scan(qkv, dec, beta, state_d, step, o_d, heads=Hd, kv_heads=Gd, head_dim=dd, v_head_dim=dvd),
-            tokens * (C + Hd * dd + Hd * dvd) * 4 + entries * Hd * dd * dvd * 8, iters=5)
-        rec["delta_scan"]["us_per_token_of_a_request"] = round(rec["delta_scan"]["us"] / per, 3)
-        if per >= 16:
-            log_dec = torch.rand(tokens, Hd, device=dev) * -0.1
-            add("delta_chunk", lambda: ops.delta_chunk(qkv, log_dec, beta, state_d, step, o_d, heads=Hd, kv_heads=Gd, head_dim=dd,
-                                                       v_head_dim=dvd), tokens * (C + Hd + Hd * dvd) * 4 + entries * Hd * dd * dvd * 8, iters=5)
-            rec["delta_chunk"]["us_per_token_of_a_request"] = round(rec["delta_chunk"]["us"] / per, 3)
+        sizes = dict(heads=Hd, kv_heads=Gd, head_dim=dd, v_head_dim=dvd)
+        inputs = dict(unit_eps=1e-6, q_scale=dd ** -0.5, per_head=True)
+        if delta_part.in_chunks(step, dev):          # from the same inputs as the two kernels below
+            name = "delta_walk (one decay per head)"
+            add(name, lambda: ops.delta_walk(qkv, proj_d[:, C + Hd:C + 2 * Hd], proj_d, C, dtb, alog, state_d, step, o_d, **sizes, **inputs),
+                tokens * (C + Hd + Hd * dvd) * 4 + entries * Hd * dd * dvd * 8, iters=5)
+        else:
+            add("delta_prep (one decay per head)", lambda: ops.delta_prep(
+                qkv, proj_d[:, C + Hd:C + 2 * Hd], proj_d, C, dtb, alog, dec, beta, **sizes, **inputs), tokens * (2 * Gd * dd * 8 + Hd * dd * 4))
+            name = "delta_scan"
+            add(name, lambda: ops.delta_scan(qkv, dec, beta, state_d, step, o_d, **sizes),
+                tokens * (C + Hd * dd + Hd * dvd) * 4 + entries * Hd * dd * dvd * 8, iters=5)
+        rec[name]["us_per_token_of_a_request"] = round(rec[name]["us"] / per, 3)
         out_d = torch.empty(tokens, Hd * dvd, device=dev, dtype=bf)
         add("delta_out (silu gate from the projection)", lambda: ops.delta_out(
             o_d, proj_d[:, C + 2 * Hd:], nwd, out_d, heads=Hd, v_head_dim=dvd, eps=1e-6, silu=True), tokens * Hd * dvd * 8)

@@ -20,7 +20,7 @@ import sys
 import torch
 
 from .hybrid_bench import PAGE_SIZE, VOCAB, _parts, _throughput, hybrid_config
-from .kernel_bench import peaks, timed
+from .kernel_bench import design_mixers, peaks, timed
 
 WINDOW = 1024
 
@@ -56,12 +56,14 @@ def _kernels(width: int, cases, pk: dict) -> dict:
     cfg = zisevik_config(width)
     lat, ret = cfg["layers"][0]["mixer"], cfg["layers"][1]["mixer"]
     bf = torch.bfloat16
+    ret_part = design_mixers(cfg, bf)[1]
     out = {}
     for tokens, entries, held in cases:
         per = tokens // entries
         step = SimpleNamespace(token_seq=torch.arange(tokens, device=dev, dtype=torch.int32) // per,
                                cu_q=torch.arange(entries + 1, device=dev, dtype=torch.int32) * per,
-                               seq_rows=torch.arange(entries, device=dev, dtype=torch.int32), num_seqs=entries, max_q_len=per,
+                               seq_rows=torch.arange(entries, device=dev, dtype=torch.int32), num_seqs=entries, num_tokens=tokens,
+                               max_q_len=per, q_lens=[per] * entries,
                                positions=(torch.arange(tokens, device=dev, dtype=torch.int32) % per) + held)
         kv_len = torch.full((entries,), held + per, device=dev, dtype=torch.int32)
         rec = {}
@@ -105,9 +107,11 @@ def _kernels(width: int, cases, pk: dict) -> dict:
         # keys a query sees: min(window, position + 1)
         seen = sum(min(WINDOW, held + i + 1) for i in range(per)) * entries
         key_rows = entries * min(held + per, WINDOW + per - 1)
-        add("latent_attention_tiled", lambda: ops.latent_attention_tiled(
+        tc = ops.latent_takes_tc(entries, per, H, rank, r, q_lens=[per] * entries, kv_lens=[held + per] * entries, window=WINDOW)
+        most = {} if tc else {"max_keys": min(held + per, WINDOW + per - 1)}
+        add("latent_attention_tc" if tc else "latent_attention_tiled", lambda: (ops.latent_attention_tc if tc else ops.latent_attention_tiled)(
             qfull, cache, table, step.seq_rows, step.cu_q, kv_len, sink, o_lat, entries=entries, max_q_len=per, heads=H, rank=rank,
-            rot=r, page_size=PAGE_SIZE, scale=0.09, window=WINDOW, max_keys=min(held + per, WINDOW + per - 1)),
+            rot=r, page_size=PAGE_SIZE, scale=0.09, window=WINDOW, **most),
             nbytes=key_rows * D * 2 + tokens * H * (D + rank) * 2, flops=2.0 * seen * H * (D + rank))
         if tokens <= 256:
             add("latent_attention_plain", lambda: ops.latent_attention_plain(
@@ -133,22 +137,29 @@ def _kernels(width: int, cases, pk: dict) -> dict:
         proj_r = torch.randn(tokens, 2 * qk + 2 * vv, device=dev, dtype=bf) * 0.3
         inv_r = (1e6 ** (-torch.arange(0, dr, 2, dtype=torch.float32) / dr)).to(dev)
         q32, k32 = torch.empty(tokens, qk, device=dev), torch.empty(tokens, qk, device=dev)
-        add("retention_prep", lambda: ops.retention_prep(proj_r, 0, qk, inv_r, step.positions, q32, k32, heads=Hr, head_dim=dr,
-                                                         rotary_dim=dr, k_scale=dr ** -0.5), tokens * qk * 12)
+        chunked = per >= ret_part.chunk_min_tokens
+        walk = chunked and ret_part.in_walk(step, dev)
+        if not walk:
+            add("retention_prep", lambda: ops.retention_prep(proj_r, 0, qk, inv_r, step.positions, q32, k32, heads=Hr, head_dim=dr,
+                                                             rotary_dim=dr, k_scale=dr ** -0.5), tokens * qk * 12)
         decay = torch.tensor(ret["decay"], device=dev, dtype=torch.float32)
         state = torch.zeros(entries, Hr * dr * dvr, device=dev)
         o_r = torch.empty(tokens, vv, device=dev)
-        add("retention_scan", lambda: ops.retention_scan(q32, k32, proj_r, 2 * qk, decay, state, step, o_r, heads=Hr, head_dim=dr,
-                                                         v_head_dim=dvr), tokens * (2 * qk * 4 + vv * 6) + entries * Hr * dr * dvr * 8, iters=5)
-        rec["retention_scan"]["us_per_token_of_a_request"] = round(rec["retention_scan"]["us"] / per, 3)
-        if per >= 16:
+        sizes = dict(heads=Hr, head_dim=dr, v_head_dim=dvr)
+        moved = tokens * (2 * qk * (2 if walk else 4) + vv * 6) + entries * Hr * dr * dvr * 8
+        if walk:                                     # q and k from the projection, rotated on the way
+            name = "retention_chunk (prepared side by side, walked)"
+            add(name, lambda: ops.retention_chunk(None, None, proj_r, 2 * qk, decay, state, step, o_r, **sizes, qk=(0, qk, dr ** -0.5),
+                                                  rotation=(inv_r, dr, step.positions)), moved, iters=5)
+        else:
+            name = "retention_chunk" if chunked else "retention_scan"
+            add(name, lambda: getattr(ops, name)(q32, k32, proj_r, 2 * qk, decay, state, step, o_r, **sizes), moved, iters=5)
+        rec[name]["us_per_token_of_a_request"] = round(rec[name]["us"] / per, 3)
+        if chunked:
             # 32-bit FMAs of the closed form: scores (half of the 64 x 64 square is used), their product with the
             # values, the old state's part and the new state
             fma = tokens * Hr * (64 * dr * ((dvr + 31) // 32) + 64 * dvr + 2 * dr * dvr)
-            add("retention_chunk", lambda: ops.retention_chunk(q32, k32, proj_r, 2 * qk, decay, state, step, o_r, heads=Hr, head_dim=dr,
-                                                               v_head_dim=dvr), tokens * (2 * qk * 4 + vv * 6) + entries * Hr * dr * dvr * 8, iters=5)
-            rec["retention_chunk"]["us_per_token_of_a_request"] = round(rec["retention_chunk"]["us"] / per, 3)
-            rec["retention_chunk"]["of_fp32_fma_peak"] = round(fma / (rec["retention_chunk"]["us"] * 1e-6) / (148 * 128 * 1.9e9), 3)
+            rec[name]["of_fp32_fma_peak"] = round(fma / (rec[name]["us"] * 1e-6) / (148 * 128 * 1.9e9), 3)
         gated = torch.empty(tokens, vv, device=dev, dtype=bf)
         add("retention_out", lambda: ops.retention_out(o_r, proj_r, 2 * qk + vv, gated, heads=Hr, v_head_dim=dvr, eps=1e-6), tokens * vv * 8)
         # like: the delta rule's recurrence of the closest model, the same state size
