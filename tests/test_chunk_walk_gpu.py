@@ -274,3 +274,26 @@ def test_parameters_off_16_bytes(kind):
         walks.append(sum(ops.calls.get(n, 0) for n in ("se_delta_walk", "se_retention_prep")) - before)
     assert walks == ([1, 0] if kind == "delta" else [0, 1])
     _close(outs[1], outs[0].double(), "outputs")
+
+
+def test_head_sizes_that_the_walk_does_not_take():
+    """A delta rule with one decay per head and a head size that is no multiple of four: a prompt goes through the kernel that does
+    a chunk at a time, and gives what it gives token by token."""
+    from sparseengine_b200.config.specs import GatedDeltaSpec
+    from sparseengine_b200.csrc import ops
+    from sparseengine_b200.parts.base import LayerSlot, make_mixer
+    spec = GatedDeltaSpec(hidden_size=64, num_heads=2, num_kv_heads=1, head_dim=18, v_head_dim=16, conv_taps=3, decay_per="head", gate_activation="silu")
+    T = 150
+    step = _one_entry(T)
+    step.token_seq = torch.zeros(T, dtype=torch.int32, device=DEV)
+    outs, chunks = [], []
+    for least in (None, 48):
+        part, g = make_mixer(spec, torch.float32), torch.Generator(device=DEV).manual_seed(2)
+        part.bind({n: torch.randn(p.shape, generator=g, device=DEV) * 0.3 for n, p in part.parameters().items()})
+        part.chunk_min_tokens = least
+        state, before = torch.zeros(1, *part.state_request().shape, device=DEV), ops.calls.get("se_delta_chunk", 0)
+        outs.append((part.forward(torch.randn(T, 64, generator=g, device=DEV), step, LayerSlot(state=state)), state))
+        chunks.append(ops.calls.get("se_delta_chunk", 0) - before)
+    assert chunks == [0, 1]
+    _close(outs[1][0], outs[0][0].double(), "outputs")
+    _close(outs[1][1], outs[0][1].double(), "state")
