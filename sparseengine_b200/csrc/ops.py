@@ -533,20 +533,21 @@ def latent_takes_tc(entries: int, max_q_len: int, heads: int, rank: int, rot: in
                     kv_lens=None, window: Optional[int] = None) -> bool:
     """Whether a step's latent attention runs on tcgen05 (csrc/latent_attention_tc.cu): sizes it takes, an entry that fills half
     a query tile, and the shorter of the times (us) that the two kernels are estimated to take over the entries' own tokens and keys
-    (``q_lens``, ``kv_lens``; without them every entry is as long as the longest and holds nothing before).  tcgen05: a block per 256
+    (``q_lens``, ``kv_lens``; without them by blocks of 256 rows for a fifth of the SMs, every entry as long as the longest).  tcgen05: a block per 256
     rows, 2.1 per 64 keys, one block on an SM, 8 to start and end.  The tiled kernel: a block per 64 rows, its keys split
     (:func:`latent_split_plan`) where the blocks of the longest entry's rows, times the entries, would not fill the device twice;
-    0.054 per key alone on an SM and 0.067 for each of two, 2 to start and end, 10 (most of it
-    the host's, a launch and two workspaces) and the parts' bytes (32-bit, written and read) at 5 TB/s to join them.  Measured on a B200, 32
-    heads, a layer, us there and here: a portion of 64 tokens beside three decoding requests at 500, 4,000 and 30,000 keys
-    55 / 57, 121 / 168, 625 / 1,012; of 512 beside seven 100 / 79, 296 / 195, 1,765 / 1,058; one of 128 alone at 4,000 keys
-    123 / 166, of 256 206 / 174; 64 requests of which one brings 8 tokens at 4,000 keys 170 / 178."""
+    0.054 per key alone on an SM and 0.067 for each of two, 10 to start and end, 14 and the parts' bytes (32-bit, written and read)
+    at 5 TB/s to join them; of these 10 and 14 the host takes 6 and 10 (it plans the splits, then a launch and two workspaces), for which
+    small steps wait.  Measured on a B200, 32 heads, a layer, us there and here, device time: a portion of 64 tokens
+    beside three decoding requests at 4,000 and 30,000 keys 121 / 168, 625 / 1,012; of 512 beside seven 296 / 195, 1,765 / 1,058; one of 128 alone
+    at 4,000 keys 123 / 166, of 256 206 / 174; a call: one of 64 tokens alone 156 / 151, behind 500 keys 167 / 153, with a window of 1,024
+    beside three requests at 4,000 keys 168 / 153, 8 beside 31 at 4,000 keys 167 / 182."""
     if sms is None:
         sms = sm_count()
     if not latent_attention_tc_supported(rank, rot) or max_q_len * heads < 128:
         return False
-    q_lens = q_lens or [max_q_len] * entries
-    kv_lens = kv_lens or q_lens
+    if not q_lens or not kv_lens:
+        return 5 * entries * -(-max_q_len * heads // 256) >= sms
     tile_keys = latent_tile_keys(max_q_len)
     most = max(kv_lens) if window is None else min(max(kv_lens), window + max_q_len - 1)
     splits, per = latent_split_plan(-(-max_q_len * heads // 64), entries, most, sms, tile_keys)
@@ -567,8 +568,8 @@ def latent_takes_tc(entries: int, max_q_len: int, heads: int, rank: int, rot: in
         narrow_last = max(narrow_last, each if splits > 1 else last)
     tc = 8 + 2.1 / 64 * max(wide_last, -(-wide // sms) * wide_keys / wide) + 2.1
     full, rest = divmod(narrow, 2 * sms)
-    tiled = 2 + max(0.054 * narrow_last, (0.067 * full + (0.067 if rest > sms else 0.054 if rest else 0.0)) * narrow_keys / narrow)
-    return tc < tiled + (10 + narrow * 64 * rank * 8 / 5e6 if splits > 1 else 0)
+    tiled = 10 + max(0.054 * narrow_last, (0.067 * full + (0.067 if rest > sms else 0.054 if rest else 0.0)) * narrow_keys / narrow)
+    return tc < tiled + (14 + narrow * 64 * rank * 8 / 5e6 if splits > 1 else 0)
 
 
 def latent_attention_tc(qfull, cache, table, seq_rows, cu_q, kv_len, sink, out, *, entries, max_q_len, heads, rank, rot,

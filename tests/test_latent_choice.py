@@ -13,7 +13,9 @@ def _takes(lens, held, window=None, heads=32, rank=192, rot=64):
 @pytest.mark.parametrize("lens,held,window,tc", [
     # a portion beside decoding requests, which tcgen05 would walk unsplit: measured 121 / 168, 625 / 1,012 and 905 / 1,015 us
     ([64, 1, 1, 1], 4000, None, False), ([64, 1, 1, 1], 30000, None, False), ([128, 1, 1, 1], 30000, None, False),
-    ([8] + [1] * 31, 30000, None, False), ([64, 1, 1, 1], 4000, 1024, False),
+    ([8] + [1] * 31, 30000, None, False), ([8] + [1] * 31, 4000, None, False),
+    # small steps wait for the host, which the tiled kernel takes longer: a call 168 / 153, 157 / 152, 162 / 151, 167 / 153
+    ([64, 1, 1, 1], 4000, 1024, True), ([64, 1, 1, 1], 0, None, True), ([8] + [1] * 31, 0, None, True), ([64], 500, None, True),
     # where the tiled kernel does not split either: 296 / 195, 1,765 / 1,058, 254 / 178
     ([512] + [1] * 7, 4000, None, True), ([512] + [1] * 7, 30000, None, True), ([32] + [1] * 63, 4000, None, True),
     ([512] + [1] * 7, 4000, 1024, True),
