@@ -1379,9 +1379,9 @@ F32_TILE_ROWS = 128       # (token, head) rows per tile of the 32-bit prompt-por
 def attn_f32_tiles_pay(q_lens, kv_lens, num_heads: int, num_kv_heads: int, most: Optional[int] = None, sms: Optional[int] = None) -> bool:
     """Whether a step's 32-bit attention takes less time in tiles (csrc/attention_f32.cu) than by a block per (token, head)
     (csrc/attention_plain.cu), as estimated (us) over its entries' tokens and keys; ``most``: keys a query sees at most (a window).
-    Plain: 2.2e-4 per (query head, key) pair.  Tiles: per tile of 128 (token, head) rows and 64 keys 13.5, of which the lookup of
-    the keys' pages is most, and 0.068 per row of the warps that have rows; one block on an SM, so an entry of one token
-    takes two thirds of a full tile's time.  Measured on a B200, a layer, us plain / tiles, 16 heads over 16: a prompt of 600 tokens
+    Plain: 2.2e-4 per (query head, key) pair.  Tiles: per tile of 128 (token, head) rows and 64 keys 13.5 whatever
+    the rows (the copies, and one warp's chain) and 0.068 per row of the warps that have rows; one block on an SM, so an entry of one
+    token takes two thirds of a full tile's time.  Measured on a B200, a layer, us plain / tiles, 16 heads over 16: a prompt of 600 tokens
     beside 63 requests of 4,000 keys 9,511 / 7,154, of 160 4,014 / 6,926, of 64 2,355 / 6,282; 600 single tokens of 1,000 keys
     2,777 / 14,706; 48 heads over 8: 7,613 / 7,673; 32 over 1: 5,048 / 1,331; 48 over 8, a portion of 16 tokens behind 4,000
     keys 757 / 1,261, of 160 5,567 / 1,421."""
