@@ -1285,10 +1285,15 @@ _sm_counts: dict = {}
 
 def sm_count(device=None) -> int:
     """Streaming multiprocessors of the device (asked once per device)."""
-    key = torch.cuda.current_device() if device is None or torch.device(device).index is None else torch.device(device).index
-    n = _sm_counts.get(key)
+    n = _sm_counts.get(device) if device is not None else None       # a device that names its index is its own key
     if n is None:
-        n = _sm_counts[key] = torch.cuda.get_device_properties(key).multi_processor_count
+        index = None if device is None else torch.device(device).index
+        key = torch.cuda.current_device() if index is None else index
+        n = _sm_counts.get(key)
+        if n is None:
+            n = _sm_counts[key] = torch.cuda.get_device_properties(key).multi_processor_count
+        if index is not None:
+            _sm_counts[device] = n
     return n
 
 

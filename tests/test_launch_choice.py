@@ -40,3 +40,18 @@ def test_plain_attention_hears_of_the_device(seen):
     f, i = torch.zeros(4, 8), torch.zeros(4, dtype=torch.int32)
     ops.paged_attention_plain(f, f, i.view(2, 2), i, i, i, f.clone(), num_heads=2, num_kv_heads=1, head_dim=4, page_size=4, scale=1.0)
     assert seen[0][-3] == 99
+
+
+def test_sm_counts_are_kept_by_device(monkeypatch):
+    """A device with an index answers from memory; one without goes by the current device each time."""
+    from types import SimpleNamespace
+
+    import torch
+    current, counts = [0], {0: 148, 1: 132}
+    monkeypatch.setattr(ops, "_sm_counts", {})
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[0])
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda key: SimpleNamespace(multi_processor_count=counts[key]))
+    for _ in range(2):
+        assert [ops.sm_count(d) for d in (torch.device("cuda", 1), "cuda:1", 1, torch.device("cuda", 0), "cuda:0")] == [132, 132, 132, 148, 148]
+        for current[0] in (0, 1):
+            assert ops.sm_count() == ops.sm_count("cuda") == ops.sm_count(torch.device("cuda")) == counts[current[0]]
