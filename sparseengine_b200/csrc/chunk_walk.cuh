@@ -12,8 +12,12 @@
 // value columns) that takes the chunks in turn with its slice of the state in shared memory: two or three small matrix
 // products per chunk instead of a chain of T dependent steps.
 //
-// What bounds them is the FMA rate (3 to 5 multiply-adds per state element and token); a tensor-core form would need
-// 16-bit or split operands.  Every exponent is a difference of sums of logarithms that is at most 0 up to the 64-bit sums' rounding
+// What bounds the walk is arithmetic (3 to 5 multiply-adds per state element and token) along a chain of chunks; 16-bit operands would
+// lose what the recurrence has to keep.  With multiply-adds it stood at half their rate, its other half shared-memory reads (8 x 8 outputs
+// a thread, an LDS.128 each four multiply-adds); products in tf32 terms by mma.sync read less.  Measured, multiply-adds / now: state space,
+// 2,048 tokens of 64 heads of 64 columns, 204 / 152 us; retention, 8,192 tokens of 32 heads of 128, 752 / 563; delta rule per channel, 4,670 tokens of
+// 16 heads of 128, 418 / 333; per head, 2,048 tokens, 176 / 134.  Sixteen warps instead of eight: 168, 616, -, 148.  Every exponent is a
+// difference of sums of logarithms that is at most 0 up to the 64-bit sums' rounding
 // (no token's logarithm lies below -1e4) or, for decays per channel, a product of decays of at most T tokens: no term overflows.
 //
 // A step's batch is ragged: entry e owns tokens cu_q[e] .. cu_q[e+1]-1 and state row seq_rows[e].  Chunk c of entry e has the
@@ -21,6 +25,7 @@
 // chunk from the device's arrays alone.
 #pragma once
 #include "common.cuh"
+#include "split_mma.cuh"
 
 namespace se {
 namespace walk {
@@ -49,6 +54,12 @@ __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
     const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
     return make_float4(a.x, a.y, b.x, b.y);
 }
+
+// two of them
+__device__ __forceinline__ float2 load2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 load2(const __nv_bfloat16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
+
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory"); }
 
 // the entry that owns place `slot` among the step's chunks, and the chunk's first token and length (0: nobody's place)
 template <int T>
@@ -87,347 +98,411 @@ struct WalkArgs {
     int H, d, dv;
 };
 
-// Two groups of four warps share a chunk's products.  Without a system to solve, group 0 makes the outputs (q S_0, then P u, in
-// four slices) while group 1 sums and stores those of the chunk before, updates the state into a second buffer and brings the
-// next values: one barrier for all per chunk, and one at which group 1 only arrives.  With one, group 0 makes u = U - W S_0 and then the state's update while group 1 makes q S_0 and then the
-// outputs: two barriers.  A thread holds T / 8 rows x C / 4 columns of its warp's slice (8 x 8 at best: an FMA costs a quarter of
-// a shared-memory wavefront then, and both units are as busy).  q, k, P and W of the next chunk are copied as soon as the last
-// reader of this one's has passed.
+// Two groups of four warps share a chunk's products, all of them on the tensor cores in tf32 terms (split_mma.cuh).  Without a
+// system to solve, group 0 makes the outputs (q S_0, then P u) while group 1 updates the state, which it keeps in registers and
+// hands over through a second buffer, and brings the next values: one barrier per chunk.  With one, group 0 makes
+// u = U - W S_0 and then the state's update while group 1 makes q S_0 and then the outputs: two barriers.  Tiles of q, k, W and P
+// that a warp alone reads are copied by that warp as soon as it has read the last chunk's.  Row pitches are such that no fragment read
+// meets a bank twice: 8 more than a multiple of 32 where rows lie along k (two neighbours per lane), 4 more than a
+// multiple of 16 where columns do.
 template <int T, int DP, int C, bool SOLVE, bool CHANNEL>
 struct WalkShape {
-    static constexpr int kSlices = 4;                                 // of the inner dimension (or the tokens), a warp each
-    static constexpr int kRowGroups = DP / 64;                        // 64 rows of the state per warp ...
-    static constexpr int kTimeSplit = 4 / kRowGroups;                 // ... and a slice of the tokens
-    static constexpr int kQP = DP + 4, kPP = T + 4;
-    static constexpr int kFloats = 3 * T * kQP + T * kPP + (SOLVE ? 2 : 3) * T * C + (SOLVE ? 1 : 2) * DP * C +
-                                   kSlices * T * C + (kTimeSplit - 1) * DP * C + 2 * T + (CHANNEL ? DP : 0);
+    static constexpr int kQP = DP + 8, kKP = DP + 4, kPP = T + 8, kCP = C + 4;
+    static constexpr int kBuffers = SOLVE ? 1 : 2;                    // of k, u and the state
+    static constexpr int kFloats = (SOLVE ? 2 : 1) * T * kQP + kBuffers * T * kKP + T * kPP +
+                                   kBuffers * (CHANNEL ? 1 : 2) * T * kCP + kBuffers * DP * kCP + 2 * T;
+    static constexpr int kBlocks = kFloats * 4 <= 112 * 1024 ? 2 : 1;            // per SM
 };
 
-__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory"); }
-
 template <int T, int DP, int C, bool SOLVE, bool CHANNEL, typename TV>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, WalkShape<T, DP, C, SOLVE, CHANNEL>::kBlocks)
 chunk_walk_kernel(const WalkArgs a) {
     using Shape = WalkShape<T, DP, C, SOLVE, CHANNEL>;
-    constexpr int QP = Shape::kQP, PP = Shape::kPP, KS = Shape::kSlices, TS = Shape::kTimeSplit, RG = Shape::kRowGroups;
-    constexpr int RM = T / 8, RC = C / 4;            // rows and columns of a thread's output tile
-    constexpr int NQ = T * C / 4 / 128;              // quads of the chunk's value columns per thread of a group
+    constexpr int QP = Shape::kQP, KP = Shape::kKP, PP = Shape::kPP, CP = Shape::kCP, NB = Shape::kBuffers;
+    constexpr int WR = T / 16, WC = 4 / WR, NT = C / 8 / WC;          // a warp's outputs: 16 rows, NT tiles of eight columns
+    constexpr int MT = DP / 64, NS = C / 8;                           // a warp's state: MT tiles of 16 rows, all columns
+    constexpr int NQ = T * C / 4 / 128;                               // quads of the chunk's value columns per thread of a group
+    static_assert(SOLVE || T == 64, "without a system a warp has its rows of q and P for itself");
     extern __shared__ __align__(16) float sm[];
     float* qs = sm;                                  // [T][QP]
-    float* ks = qs + T * QP;                         // [T][QP], twice without a system to solve
-    float* ws = ks + T * QP;                         // [T][QP]: W, or the second k
-    float* ps = ws + T * QP;                         // [T][PP]
-    float* us = ps + T * PP;                         // [T][C]: u; twice without a system to solve
-    float* u2 = us + (SOLVE ? 1 : 2) * T * C;        // [T][C]: e^(B_n - B_t) u (decays per head)
-    float* Ss = u2 + T * C;                          // [DP][C]; twice without a system to solve
-    float* part = Ss + (SOLVE ? 1 : 2) * DP * C;     // [KS][T][C]
-    float* part2 = part + KS * T * C;                // [TS - 1][DP][C]
-    float* rss = part2 + (TS - 1) * DP * C;          // [2][T]
-    float* tots = rss + 2 * T;                       // [DP]
+    float* ws = qs + T * QP;                         // [T][QP]: W
+    float* ks = ws + (SOLVE ? T * QP : 0);           // [NB][T][KP]
+    float* ps = ks + NB * T * KP;                    // [T][PP]
+    float* us = ps + T * PP;                         // [NB][T][CP]: u
+    float* u2 = CHANNEL ? us : us + NB * T * CP;     // [NB][T][CP]: e^(B_n - B_t) u (decays per head)
+    float* Ss = u2 + NB * T * CP;                    // [NB][DP][CP]
+    float* rss = Ss + NB * DP * CP;                  // [2][T]
     const int e = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * C;
     const int t_first = a.cu_q[e], t_last = a.cu_q[e + 1];
     if (t_last <= t_first) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lc = lane & 3;
     const int group = warp >> 2, gw = warp & 3, gt = tid & 127;          // the group, and this thread's place in it
     const int d = a.d, dv = a.dv;
+    const int r0 = (gw % WR) * 16 + lr, col0 = (gw / WR) * NT * 8;       // this lane's first row and its warp's first column of outputs
+    const int m0 = gw * MT * 16;                                         // the warp's first row of the state
 
     float* S0 = a.state + (size_t)a.seq_rows[e] * a.state_stride + (size_t)h * d * dv;
     for (int i = tid; i < DP * C; i += kThreads) {   // the faster index in memory runs over neighbouring threads
         const int row = a.s_row == 1 ? i % DP : i / C, c = a.s_row == 1 ? i / DP : i % C;
-        Ss[row * C + c] = row < d && c0 + c < dv ? S0[(size_t)row * a.s_row + (size_t)(c0 + c) * a.s_col] : 0.f;
+        Ss[row * CP + c] = row < d && c0 + c < dv ? S0[(size_t)row * a.s_row + (size_t)(c0 + c) * a.s_col] : 0.f;
     }
 
-    // T rows of d columns to shared memory by one group; rows from n on and columns from d on are zeros
-    auto load_rows = [&](float* tile, const float* src, size_t stride, int t0, int n) {
+    // ROWS x COLS floats from (row0, col0) of a chunk's rows to shared memory by `threads` threads, this one being number `who`; rows
+    // from n on and columns from `most` on are zeros
+    auto load = [&](float* tile, int pitch, const float* src, size_t stride, int t0, int n, int rows, int row0, int cols, int col, int most, int who, int threads) {
 #pragma unroll 4
-        for (int i = gt; i < T * (DP / 4); i += 128) {
-            const int t = i / (DP / 4), c = (i % (DP / 4)) * 4;
-            const bool in = t < n && c < d;
-            cp16(tile + t * QP + c, src + (size_t)(t0 + (in ? t : 0)) * stride + (in ? c : 0), in);
-        }
-    };
-    auto load_p = [&](int t0, int n) {
-#pragma unroll 4
-        for (int i = gt; i < T * (T / 4); i += 128) {
-            const int t = i / (T / 4), c = (i % (T / 4)) * 4;
-            cp16(ps + t * PP + c, a.p + ((size_t)(t0 + (t < n ? t : 0)) * a.H + h) * T + c, t < n);
+        for (int i = who; i < rows * (cols / 4); i += threads) {
+            const int t = row0 + i / (cols / 4), c = col + (i % (cols / 4)) * 4;
+            const bool in = t < n && c < most;
+            cp16(tile + t * pitch + c, src + (size_t)(t0 + (in ? t : 0)) * stride + (in ? c : 0), in);
         }
     };
     const float* qb = a.q + (size_t)(h / a.rep) * d;
     const float* kb = a.k + (size_t)(h / a.rep) * d;
     const float* wb = SOLVE ? a.w + (size_t)h * d : nullptr;
+    const float* pb = a.p + (size_t)h * T;
     const TV* vb = static_cast<const TV*>(a.v) + (size_t)h * dv + c0;
-    // value rows (or U) of a chunk, quad by quad, with the factors that go with their tokens
-    float4 vreg[NQ];
-    float vfac[NQ], tfac[NQ], rfac = 0.f;
-    auto load_v = [&](int t0, int n) {
-#pragma unroll
-        for (int x = 0; x < NQ; ++x) {
-            const int i = x * 128 + gt, t = i / (C / 4), c = (i % (C / 4)) * 4;
-            const bool in = t < n && c0 + c < dv;
-            const size_t at = (size_t)(t0 + t) * a.H + h;
-            vreg[x] = in ? load4(vb + (size_t)(t0 + t) * a.v_stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-            vfac[x] = !SOLVE && in && a.v_scale != nullptr ? a.v_scale[at] : 1.f;
-            tfac[x] = !CHANNEL && in ? a.ts[at] : 1.f;
-        }
+    auto load_k = [&](float* to, int t0, int n) { load(to, KP, kb, a.qk_stride, t0, n, T, 0, DP, 0, d, gt, 128); };
+    auto load_p = [&](int t0, int n) {
+        if (SOLVE) load(ps, PP, pb, (size_t)a.H * T, t0, n, T, 0, T, 0, T, gt, 128);
+        else load(ps, PP, pb, (size_t)a.H * T, t0, n, 16, gw * 16, T, 0, T, lane, 32);
     };
-    auto load_factors = [&](int t0, int n) {         // e^(B_t) of the chunk's tokens, or e^(B_n) of the channels
-        if (!CHANNEL && gt < T) rfac = gt < n ? a.rs[(size_t)(t0 + gt) * a.H + h] : 0.f;
-        if (CHANNEL) rfac = gt < d ? a.tot[((size_t)(t_first / T + e + (t0 - t_first) / T) * a.H + h) * d + gt] : 0.f;
+    auto load_q = [&](int t0, int n) {
+        if (SOLVE) load(qs, QP, qb, a.qk_stride, t0, n, T, 0, DP, 0, d, gt, 128);
+        else load(qs, QP, qb, a.qk_stride, t0, n, 16, gw * 16, DP, 0, d, lane, 32);
     };
-    int odd = 0;                                     // a value that is not finite
-    auto put_u = [&](int x, float4 u, float* to) {   // u and e^(B_n - B_t) u of one quad
-        const int i = x * 128 + gt;
-        odd |= !(isfinite(u.x) && isfinite(u.y) && isfinite(u.z) && isfinite(u.w));
-        st4(to + i * 4, u);
-        if (!CHANNEL) st4(u2 + i * 4, make_float4(u.x * tfac[x], u.y * tfac[x], u.z * tfac[x], u.w * tfac[x]));
-    };
-    auto put_values = [&](float* to) {
+    auto load_w = [&](int t0, int n) { load(ws, QP, wb, (size_t)a.H * d, t0, n, T, 0, DP, 0, d, gt, 128); };
+
+    // rows of x . S
+    auto state_product = [&](const float* x, const float* S, float (&acc)[1][NT][4]) {
 #pragma unroll
-        for (int x = 0; x < NQ; ++x) {
-            float4 v = vreg[x];
-            if (a.silu) v = make_float4(value_silu<TV>(v.x), value_silu<TV>(v.y), value_silu<TV>(v.z), value_silu<TV>(v.w));
-            put_u(x, make_float4(v.x * vfac[x], v.y * vfac[x], v.z * vfac[x], v.w * vfac[x]), to);
-        }
-    };
-    // acc = rows of x . S, a warp's slice of the inner dimension
-    auto state_product = [&](const float* x, const float* S, float (&acc)[RM][RC]) {
+        for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int i = 0; i < RM; ++i)
+            for (int j = 0; j < 4; ++j) acc[0][n][j] = 0.f;
+        const float* xr = x + r0 * QP + 2 * lc;
+        const float* sr = S + 2 * lc * CP + col0 + lr;
+        split::products<1, NT, 4>(acc, DP / 8,
+            [&](int, int s, float (&v)[4]) {
+                const float2 top = *reinterpret_cast<const float2*>(xr + 8 * s), low = *reinterpret_cast<const float2*>(xr + 8 * QP + 8 * s);
+                v[0] = top.x; v[1] = low.x; v[2] = top.y; v[3] = low.y;
+            },
+            [&](int n, int s, float (&v)[2]) { v[0] = sr[8 * s * CP + 8 * n]; v[1] = sr[(8 * s + 1) * CP + 8 * n]; });
+        if (split::odd(acc))
 #pragma unroll
-            for (int c = 0; c < RC; ++c) acc[i][c] = 0.f;
-#pragma unroll 2
-        for (int k = gw * (DP / KS); k < (gw + 1) * (DP / KS); k += 4) {
-            float sv[4][RC];
+            for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int g = 0; g < RC / 4; ++g) *reinterpret_cast<float4*>(&sv[j][4 * g]) = ld4(S + (k + j) * C + 16 * g + lc * 4);
-#pragma unroll
-            for (int i = 0; i < RM; ++i) {
-                const float4 v = ld4(x + (lr + 8 * i) * QP + k);
-#pragma unroll
-                for (int c = 0; c < RC; ++c) acc[i][c] = fmaf(v.w, sv[3][c], fmaf(v.z, sv[2][c], fmaf(v.y, sv[1][c], fmaf(v.x, sv[0][c], acc[i][c]))));
-            }
-        }
-    };
-    auto put_part = [&](const float (&v)[RM][RC]) {
-#pragma unroll
-        for (int i = 0; i < RM; ++i)
-#pragma unroll
-            for (int g = 0; g < RC / 4; ++g)
-                st4(part + (gw * T + lr + 8 * i) * C + 16 * g + lc * 4, make_float4(v[i][4 * g], v[i][4 * g + 1], v[i][4 * g + 2], v[i][4 * g + 3]));
-    };
-    auto sum_part = [&](int x) {                     // the sum over the slices of one quad
-        float4 s = ld4(part + (x * 128 + gt) * 4);
-#pragma unroll
-        for (int z = 1; z < KS; ++z) {
-            const float4 v = ld4(part + z * T * C + (x * 128 + gt) * 4);
-            s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
-        }
-        return s;
-    };
-    // acc = e^(B_t) acc + P u, a warp's slice of the tokens s; P is zero for s > t
-    auto add_tokens = [&](const float* u, const float* factors, int any_odd, float (&acc)[RM][RC]) {
-        if (!CHANNEL)
-#pragma unroll
-            for (int i = 0; i < RM; ++i) {
-                const float f = factors[lr + 8 * i];
-#pragma unroll
-                for (int c = 0; c < RC; ++c) acc[i][c] *= f;
-            }
-        auto run = [&](bool guarded) {
+                for (int j = 0; j < 4; ++j) {
+                    if (isfinite(acc[0][n][j])) continue;
+                    const float* row = x + (r0 + (j >> 1) * 8) * QP;
+                    const float* column = S + col0 + 8 * n + 2 * lc + (j & 1);
+                    float sum = 0.f;
 #pragma unroll 1
-            for (int s = 4 * gw; s < T; s += 4 * KS) {           // dealt out in turn: early tokens have more rows
-                float uv[4][RC];
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int g = 0; g < RC / 4; ++g) *reinterpret_cast<float4*>(&uv[j][4 * g]) = ld4(u + (s + j) * C + 16 * g + lc * 4);
-#pragma unroll
-                for (int i = 0; i < RM; ++i) {
-                    if (8 * i + 7 < s) continue;     // rows before these tokens
-                    const int t = lr + 8 * i;
-                    const float4 pv = ld4(ps + t * PP + s);
-                    const float p4[4] = {pv.x, pv.y, pv.z, pv.w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-#pragma unroll
-                        for (int c = 0; c < RC; ++c)
-                            if (!guarded || s + j <= t) acc[i][c] = fmaf(p4[j], uv[j][c], acc[i][c]);
+                    for (int k = 0; k < DP; ++k) sum = fmaf(row[k], column[k * CP], sum);
+                    acc[0][n][j] = sum;
                 }
-            }
-        };
-        if (any_odd) run(true);                      // a token that a row does not see does not touch it, whatever it holds
-        else run(false);
     };
-    auto put_outputs = [&](int t0, int n) {
-        const float skip = a.skip != nullptr ? a.skip[h] : 0.f;
-        float4 raw[NQ];
-        if (!SOLVE && a.skip != nullptr)
+    // P u; P is zero for s > t
+    auto token_product = [&](const float* u, float (&acc)[1][NT][4]) {
+        const float* pr = ps + r0 * PP + 2 * lc;
+        const float* ur = u + 2 * lc * CP + col0 + lr;
+        auto run = [&](bool finite_only, float (&to)[1][NT][4]) {
 #pragma unroll
-            for (int x = 0; x < NQ; ++x) {
-                const int i = x * 128 + gt, t = i / (C / 4), c = (i % (C / 4)) * 4;
-                raw[x] = t < n && c0 + c < dv ? load4(vb + (size_t)(t0 + t) * a.v_stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+            for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int x = 0; x < NQ; ++x) {
-            const int i = x * 128 + gt, t = i / (C / 4), c = (i % (C / 4)) * 4;
-            if (t < n && c0 + c < dv) {
-                float4 s = sum_part(x);
-                if (!SOLVE && a.skip != nullptr) {
-                    const float4 v = raw[x];
-                    s = make_float4(fmaf(skip, v.x, s.x), fmaf(skip, v.y, s.y), fmaf(skip, v.z, s.z), fmaf(skip, v.w, s.w));
-                }
-                st4(a.o + ((size_t)(t0 + t) * a.H + h) * dv + c0 + c, s);
-            }
-        }
-    };
-    // to = e^(B_n) from + sum_s k_s u_s^T: a warp takes 64 rows, all columns and a slice of the tokens; 8 rows x RC columns a thread
-    auto update_state = [&](const float* k, const float* u, const float* from, float* to, float total) {
-        const int row0 = (gw % RG) * 64 + lr * 8, slice = gw / RG;
-        float st[8][RC] = {};
-#pragma unroll 4
-        for (int s = slice * (T / TS); s < (slice + 1) * (T / TS); ++s) {
-            const float4 ka = ld4(k + s * QP + row0), kc = ld4(k + s * QP + row0 + 4);
-            const float k8[8] = {ka.x, ka.y, ka.z, ka.w, kc.x, kc.y, kc.z, kc.w};
-            float uv[RC];
-#pragma unroll
-            for (int g = 0; g < RC / 4; ++g) *reinterpret_cast<float4*>(&uv[4 * g]) = ld4(u + s * C + 16 * g + lc * 4);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int c = 0; c < RC; ++c) st[i][c] = fmaf(k8[i], uv[c], st[i][c]);
-        }
-        if (slice > 0)
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int g = 0; g < RC / 4; ++g)
-                    st4(part2 + ((slice - 1) * DP + row0 + i) * C + 16 * g + lc * 4, make_float4(st[i][4 * g], st[i][4 * g + 1], st[i][4 * g + 2], st[i][4 * g + 3]));
-        group_sync(group);
-        if (slice == 0)
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int g = 0; g < RC / 4; ++g) {
-                    const int at = (row0 + i) * C + 16 * g + lc * 4;
-                    const float f = CHANNEL ? tots[row0 + i] : total;
-                    float4 s = ld4(from + at);
-                    s = make_float4(fmaf(f, s.x, st[i][4 * g]), fmaf(f, s.y, st[i][4 * g + 1]), fmaf(f, s.z, st[i][4 * g + 2]), fmaf(f, s.w, st[i][4 * g + 3]));
-#pragma unroll
-                    for (int z = 0; z < TS - 1; ++z) {
-                        const float4 v = ld4(part2 + z * DP * C + at);
-                        s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
+                for (int j = 0; j < 4; ++j) to[0][n][j] = 0.f;
+            split::products<1, NT, 2>(to, 2 * (gw % WR) + 2,
+                [&](int, int s, float (&v)[4]) {
+                    const float2 top = *reinterpret_cast<const float2*>(pr + 8 * s), low = *reinterpret_cast<const float2*>(pr + 8 * PP + 8 * s);
+                    v[0] = top.x; v[1] = low.x; v[2] = top.y; v[3] = low.y;
+                },
+                [&](int n, int s, float (&v)[2]) {
+                    v[0] = ur[8 * s * CP + 8 * n];
+                    v[1] = ur[(8 * s + 1) * CP + 8 * n];
+                    if (finite_only) {
+                        if (!isfinite(v[0])) v[0] = 0.f;
+                        if (!isfinite(v[1])) v[1] = 0.f;
                     }
-                    st4(to + at, s);
+                });
+        };
+        run(false, acc);
+        if (split::odd(acc)) {                       // a token that a row does not see does not touch it, whatever it holds
+            float rest[1][NT][4];
+            run(true, rest);
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (isfinite(acc[0][n][j])) continue;
+                    const int t = r0 + (j >> 1) * 8;
+                    const float* column = u + col0 + 8 * n + 2 * lc + (j & 1);
+                    float sum = 0.f;
+#pragma unroll 1
+                    for (int s = 0; s <= t; ++s) sum = fmaf(ps[t * PP + s], column[s * CP], sum);
+                    acc[0][n][j] = isfinite(sum) && isfinite(rest[0][n][j]) ? rest[0][n][j] : sum;
                 }
+        }
+    };
+    // st = e^(B_n) st + sum_s k_s u_s^T over the warp's rows, and the copy that the other products read
+    float st[MT][NS][4];
+    auto get_state = [&](const float* from) {
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int n = 0; n < NS; ++n)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) st[i][n][j] = from[(m0 + 16 * i + lr + (j >> 1) * 8) * CP + 8 * n + 2 * lc + (j & 1)];
+    };
+    auto put_state = [&](float* to) {
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int n = 0; n < NS; ++n)
+#pragma unroll
+                for (int j = 0; j < 4; j += 2)
+                    *reinterpret_cast<float2*>(to + (m0 + 16 * i + lr + j * 4) * CP + 8 * n + 2 * lc) = make_float2(st[i][n][j], st[i][n][j + 1]);
+    };
+    auto update_state = [&](const float* k, const float* u, const float (&total)[MT][2]) {
+        float sum[MT][NS][4] = {};
+        const float* kr = k + 2 * lc * KP + m0 + lr;
+        const float* ur = u + 2 * lc * CP + lr;
+        split::products<MT, NS, 2>(sum, T / 8,
+            [&](int i, int s, float (&v)[4]) {
+                const float* at = kr + 8 * s * KP + 16 * i;
+                v[0] = at[0]; v[1] = at[8]; v[2] = at[KP]; v[3] = at[KP + 8];
+            },
+            [&](int n, int s, float (&v)[2]) { v[0] = ur[8 * s * CP + 8 * n]; v[1] = ur[(8 * s + 1) * CP + 8 * n]; });
+        if (split::odd(sum))
+#pragma unroll
+            for (int i = 0; i < MT; ++i)
+#pragma unroll
+                for (int n = 0; n < NS; ++n)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (isfinite(sum[i][n][j])) continue;
+                        const float* kc = k + m0 + 16 * i + lr + (j >> 1) * 8;
+                        const float* uc = u + 8 * n + 2 * lc + (j & 1);
+                        float x = 0.f;
+#pragma unroll 1
+                        for (int s = 0; s < T; ++s) x = fmaf(kc[s * KP], uc[s * CP], x);
+                        sum[i][n][j] = x;
+                    }
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int n = 0; n < NS; ++n)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) st[i][n][j] = fmaf(total[i][j >> 1], st[i][n][j], sum[i][n][j]);
+    };
+    auto put_outputs = [&](int t0, int n, const float (&acc)[1][NT][4]) {
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {
+            const int t = r0 + 4 * j;
+            if (t >= n) continue;
+#pragma unroll
+            for (int x = 0; x < NT; ++x) {
+                const int c = col0 + 8 * x + 2 * lc;
+                if (c0 + c >= dv) continue;
+                *reinterpret_cast<float2*>(a.o + ((size_t)(t0 + t) * a.H + h) * dv + c0 + c) = make_float2(acc[0][x][j], acc[0][x][j + 1]);
+            }
+        }
     };
 
     const int first_n = min(T, t_last - t_first);
     float* last_state = Ss;
-    if (!SOLVE) {
-        if (group == 0) {
-            load_rows(qs, qb, a.qk_stride, t_first, first_n);
-            cp_commit();
-        } else {
-            load_rows(ks, kb, a.qk_stride, t_first, first_n);
-            cp_commit();
-            load_v(t_first, first_n);
-            load_factors(t_first, first_n);
-            put_values(us);
-            if (gt < T) rss[gt] = rfac;
-        }
-        int cur = 0;
-        for (int t0 = t_first; t0 < t_last; t0 += T, cur ^= 1) {
-            const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
-            const float total = a.eb[(size_t)(t0 + n - 1) * a.H + h];
-            cp_wait<0>();                            // q, k
-            const int any_odd = __syncthreads_or(odd);       // state, u and factors of this chunk are there as well
-            odd = 0;
-            if (group == 0) {
-                float acc[RM][RC];
-                state_product(qs, Ss + cur * DP * C, acc);
-                asm volatile("bar.sync 3, 256;" ::: "memory");       // P is there, the last chunk's sums and q have been read
-                if (next < t_last) load_rows(qs, qb, a.qk_stride, next, next_n);
-                cp_commit();
-                add_tokens(us + cur * T * C, rss + cur * T, any_odd, acc);
-                put_part(acc);
-            } else {
-                load_p(t0, n);
-                cp_commit();
-                if (next < t_last) {
-                    load_rows(ks + (cur ^ 1) * T * QP, kb, a.qk_stride, next, next_n);
-                    load_v(next, next_n);
-                    load_factors(next, next_n);
-                }
-                cp_commit();
-                if (t0 > t_first) put_outputs(t0 - T, T);    // the last chunk's
-                cp_wait<1>();                        // P
-                asm volatile("bar.arrive 3, 256;" ::: "memory");
-                update_state(ks + cur * T * QP, u2, Ss + cur * DP * C, Ss + (cur ^ 1) * DP * C, total);
-                if (next < t_last) {                 // u2 has been read (the barrier inside)
-                    put_values(us + (cur ^ 1) * T * C);
-                    if (gt < T) rss[(cur ^ 1) * T + gt] = rfac;
-                }
+    if constexpr (!SOLVE) {
+        // value rows of a chunk, quad by quad, with the factors that go with their tokens
+        float4 vreg[NQ];
+        float vfac[NQ], tfac[NQ], rfac = 0.f, total = 0.f;
+        auto load_v = [&](int t0, int n) {
+#pragma unroll
+            for (int x = 0; x < NQ; ++x) {
+                const int i = x * 128 + gt, t = i / (C / 4), c = (i % (C / 4)) * 4;
+                const bool in = t < n && c0 + c < dv;
+                const size_t at = (size_t)(t0 + t) * a.H + h;
+                vreg[x] = in ? load4(vb + (size_t)(t0 + t) * a.v_stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                vfac[x] = in && a.v_scale != nullptr ? a.v_scale[at] : 1.f;
+                tfac[x] = in ? a.ts[at] : 1.f;
             }
-        }
-        __syncthreads();
-        const int last = (t_last - t_first - 1) / T * T;
-        if (group == 1) put_outputs(t_first + last, t_last - t_first - last);
-        last_state = Ss + cur * DP * C;
-    } else {
+            if (gt < T) rfac = gt < n ? a.rs[(size_t)(t0 + gt) * a.H + h] : 0.f;
+        };
+        auto put_values = [&](int buffer) {
+#pragma unroll
+            for (int x = 0; x < NQ; ++x) {
+                const int i = x * 128 + gt, at = (buffer * T + i / (C / 4)) * CP + (i % (C / 4)) * 4;
+                float4 v = vreg[x];
+                if (a.silu) v = make_float4(value_silu<TV>(v.x), value_silu<TV>(v.y), value_silu<TV>(v.z), value_silu<TV>(v.w));
+                v = make_float4(v.x * vfac[x], v.y * vfac[x], v.z * vfac[x], v.w * vfac[x]);
+                st4(us + at, v);
+                st4(u2 + at, make_float4(v.x * tfac[x], v.y * tfac[x], v.z * tfac[x], v.w * tfac[x]));
+            }
+            if (gt < T) rss[buffer * T + gt] = rfac;
+        };
         if (group == 0) {
-            load_rows(ws, wb, (size_t)a.H * d, t_first, first_n);
-            cp_commit();
-            load_rows(ks, kb, a.qk_stride, t_first, first_n);
-            cp_commit();
-            load_v(t_first, first_n);
-        } else {
-            load_rows(qs, qb, a.qk_stride, t_first, first_n);
+            load_q(t_first, first_n);
             cp_commit();
             load_p(t_first, first_n);
             cp_commit();
+        } else {
+            load_k(ks, t_first, first_n);
+            cp_commit();
+            load_v(t_first, first_n);
+            put_values(0);
+            total = a.eb[(size_t)(t_first + first_n - 1) * a.H + h];
+            cp_wait<0>();                            // k
         }
-        load_factors(t_first, first_n);
-        for (int t0 = t_first; t0 < t_last; t0 += T) {
+        __syncthreads();                             // state, u and factors of the first chunk
+        if (group == 1) get_state(Ss);
+        const float skip = a.skip != nullptr ? a.skip[h] : 0.f;
+        int cur = 0;
+        for (int t0 = t_first; t0 < t_last; t0 += T, cur ^= 1) {
             const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
-            const float total = CHANNEL ? 0.f : a.eb[(size_t)(t0 + n - 1) * a.H + h];
-            cp_wait<1>();                            // W or q (k and P may still be on their way)
-            __syncthreads();                         // and the state is up to date
-            float acc[RM][RC];
-            odd = 0;
-            if (CHANNEL ? (group == 0 && gt < DP) : (group == 1 && gt < T)) (CHANNEL ? tots : rss)[gt] = rfac;
-            state_product(group == 0 ? ws : qs, Ss, acc);
             if (group == 0) {
-                put_part(acc);
-                group_sync(0);
+                float acc[1][NT][4], sum[1][NT][4];
+                float2 raw[2][NT];                   // the outputs' own values, where they are added
+                if (a.skip != nullptr)
 #pragma unroll
-                for (int x = 0; x < NQ; ++x) {
-                    const float4 s = sum_part(x);
-                    put_u(x, make_float4(vreg[x].x - s.x, vreg[x].y - s.y, vreg[x].z - s.z, vreg[x].w - s.w), us);
+                    for (int j = 0; j < 2; ++j)
+#pragma unroll
+                        for (int x = 0; x < NT; ++x) {
+                            const int t = r0 + 8 * j, c = col0 + 8 * x + 2 * lc;
+                            raw[j][x] = t < n && c0 + c < dv ? load2(vb + (size_t)(t0 + t) * a.v_stride + c) : make_float2(0.f, 0.f);
+                        }
+                cp_wait<1>();                        // q
+                __syncwarp();
+                state_product(qs, Ss + cur * DP * CP, acc);
+                __syncwarp();
+                if (next < t_last) load_q(next, next_n);
+                cp_commit();
+                cp_wait<1>();                        // P
+                __syncwarp();
+                token_product(us + cur * T * CP, sum);
+                __syncwarp();
+                if (next < t_last) load_p(next, next_n);
+                cp_commit();
+#pragma unroll
+                for (int x = 0; x < NT; ++x)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[0][x][j] = fmaf(rss[cur * T + r0 + (j >> 1) * 8], acc[0][x][j], sum[0][x][j]);
+                if (a.skip != nullptr)
+#pragma unroll
+                    for (int x = 0; x < NT; ++x)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) acc[0][x][j] = fmaf(skip, (j & 1) ? raw[j >> 1][x].y : raw[j >> 1][x].x, acc[0][x][j]);
+                put_outputs(t0, n, acc);
+            } else {
+                const float now = total;
+                float totals[MT][2];
+#pragma unroll
+                for (int i = 0; i < MT; ++i) totals[i][0] = totals[i][1] = now;
+                if (next < t_last) {
+                    load_k(ks + (cur ^ 1) * T * KP, next, next_n);
+                    load_v(next, next_n);
+                    total = a.eb[(size_t)(next + next_n - 1) * a.H + h];
+                }
+                cp_commit();
+                update_state(ks + cur * T * KP, u2 + cur * T * CP, totals);
+                put_state(Ss + (cur ^ 1) * DP * CP);
+                if (next < t_last) put_values(cur ^ 1);
+                cp_wait<0>();                        // the next k
+            }
+            __syncthreads();
+        }
+        last_state = Ss + cur * DP * CP;
+    } else {
+        const float* ub = reinterpret_cast<const float*>(vb);
+        float ureg[NT][4], fac[2] = {}, totals[MT][2];
+        auto load_u = [&](int t0, int n) {           // U where the products' sums lie, and the tokens' factors
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) {
+                const int t = r0 + 4 * j;
+#pragma unroll
+                for (int x = 0; x < NT; ++x) {
+                    const int c = col0 + 8 * x + 2 * lc;
+                    const float2 v = t < n && c0 + c < dv ? load2(ub + (size_t)(t0 + t) * a.v_stride + c) : make_float2(0.f, 0.f);
+                    ureg[x][j] = v.x;
+                    ureg[x][j + 1] = v.y;
                 }
             }
-            cp_wait<0>();
-            const int any_odd = __syncthreads_or(odd);       // u, k and P are there, W and q have been read
-            if (next < t_last) {
-                if (group == 0) load_rows(ws, wb, (size_t)a.H * d, next, next_n);
-                else load_rows(qs, qb, a.qk_stride, next, next_n);
-                if (group == 0) load_v(next, next_n);
-                load_factors(next, next_n);
-            }
+        };
+        auto load_factors = [&](const float* from, int t0, int n) {
+            if (!CHANNEL)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) fac[j] = r0 + 8 * j < n ? from[(size_t)(t0 + r0 + 8 * j) * a.H + h] : 0.f;
+        };
+        auto load_totals = [&](int t0, int n) {
+#pragma unroll
+            for (int i = 0; i < MT; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int row = m0 + 16 * i + lr + 8 * j;
+                    totals[i][j] = !CHANNEL ? a.eb[(size_t)(t0 + n - 1) * a.H + h]
+                                   : row < d ? a.tot[((size_t)(t_first / T + e + (t0 - t_first) / T) * a.H + h) * d + row] : 0.f;
+                }
+        };
+        if (group == 0) {
+            load_w(t_first, first_n);
             cp_commit();
+            load_k(ks, t_first, first_n);
+            load_u(t_first, first_n);
+            load_factors(a.ts, t_first, first_n);
+            load_totals(t_first, first_n);
+        } else {
+            load_q(t_first, first_n);
+            cp_commit();
+            load_p(t_first, first_n);
+            load_factors(a.rs, t_first, first_n);
+        }
+        cp_commit();
+        __syncthreads();
+        if (group == 0) get_state(Ss);
+        for (int t0 = t_first; t0 < t_last; t0 += T) {
+            const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
+            cp_wait<1>();                            // W or q (k and P may still be on their way)
+            __syncthreads();                         // and the state is up to date
+            float acc[1][NT][4];
+            state_product(group == 0 ? ws : qs, Ss, acc);
             if (group == 0) {
-                update_state(ks, CHANNEL ? us : u2, Ss, Ss, total);
-                if (next < t_last) load_rows(ks, kb, a.qk_stride, next, next_n);       // k has been read (the barrier inside)
+#pragma unroll
+                for (int x = 0; x < NT; ++x)
+#pragma unroll
+                    for (int j = 0; j < 4; j += 2) {
+                        const float2 u = make_float2(ureg[x][j] - acc[0][x][j], ureg[x][j + 1] - acc[0][x][j + 1]);
+                        const int at = (r0 + 4 * j) * CP + col0 + 8 * x + 2 * lc;
+                        *reinterpret_cast<float2*>(us + at) = u;
+                        if (!CHANNEL) *reinterpret_cast<float2*>(u2 + at) = make_float2(u.x * fac[j >> 1], u.y * fac[j >> 1]);
+                    }
+            }
+            cp_wait<0>();
+            __syncthreads();                         // u, k and P are there, W, q and the state have been read
+            if (group == 0) {
+                if (next < t_last) {
+                    load_w(next, next_n);
+                    load_u(next, next_n);
+                    load_factors(a.ts, next, next_n);
+                }
+                cp_commit();
+                update_state(ks, u2, totals);
+                put_state(Ss);
+                group_sync(0);
+                if (next < t_last) {
+                    load_k(ks, next, next_n);
+                    load_totals(next, next_n);
+                }
                 cp_commit();
             } else {
-                add_tokens(us, rss, any_odd, acc);
-                put_part(acc);
+                float sum[1][NT][4];
+                if (next < t_last) load_q(next, next_n);
+                cp_commit();
+                token_product(us, sum);
                 group_sync(1);
                 if (next < t_last) load_p(next, next_n);
                 cp_commit();
-                put_outputs(t0, n);
+#pragma unroll
+                for (int x = 0; x < NT; ++x)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[0][x][j] = CHANNEL ? acc[0][x][j] + sum[0][x][j] : fmaf(fac[j >> 1], acc[0][x][j], sum[0][x][j]);
+                if (next < t_last) load_factors(a.rs, next, next_n);
+                put_outputs(t0, n, acc);
             }
         }
     }
@@ -435,7 +510,7 @@ chunk_walk_kernel(const WalkArgs a) {
     __syncthreads();
     for (int i = tid; i < DP * C; i += kThreads) {
         const int row = a.s_row == 1 ? i % DP : i / C, c = a.s_row == 1 ? i / DP : i % C;
-        if (row < d && c0 + c < dv) S0[(size_t)row * a.s_row + (size_t)(c0 + c) * a.s_col] = last_state[row * C + c];
+        if (row < d && c0 + c < dv) S0[(size_t)row * a.s_row + (size_t)(c0 + c) * a.s_col] = last_state[row * CP + c];
     }
 }
 
@@ -477,7 +552,6 @@ int launch(void (*kernel)(KArgs...), dim3 grid, size_t smem, cudaStream_t stream
     kernel<<<grid, kThreads, smem, stream>>>(KArgs(args)...);
     return (int)cudaGetLastError();
 }
-
 template <int T, int DP, bool SOLVE, bool CHANNEL, typename TV>
 int launch_walk(const WalkArgs& a, int entries, int cols, cudaStream_t stream) {
     const dim3 grid(entries, a.H, ceil_div(a.dv, cols));
