@@ -292,8 +292,8 @@ __global__ void grouped_gemm_plain_kernel(const T* __restrict__ a, const T* __re
 }
 
 // ---- the same in 32-bit, for widths that are a multiple of 4 ------------------------------------
-// 32-bit operands stay on the CUDA cores (a tensor-core split would lose digits), so a step with many rows is
-// bound by the FMA rate and one with few by streaming the experts' weights.  The kernel above keeps 2 x 4 outputs per
+// A step with many rows is bound by the FMA rate and one with few by streaming the experts' weights.  With many rows and inner
+// dimensions from 512 on the products run on the tensor cores in tf32 terms (gemm_f32_tc.cu); over shorter sums multiply-adds are the more exact.  The kernel above keeps 2 x 4 outputs per
 // thread: one shared-memory read per 1.3 FMAs, which set its pace.
 //
 // Many rows: 128 rows x 128 weight rows per block, 8 x 8 outputs per thread (four 16-byte reads per 64 FMAs), operands

@@ -1242,6 +1242,59 @@ def moe_grouped_gemm_tc(mode: int, a, w, ws: dict, route_w, out, *, experts, max
     return out
 
 
+# ---- 32-bit products on tensor cores in tf32 terms (csrc/gemm_f32_tc.cu) -------------------
+
+F32_TC_TILE_ROWS = 128    # activation rows per tile of the grouped products
+
+
+def gemm_f32_tc_supported(k_dim: int) -> bool:
+    f = library().se_gemm_f32_tc_supported
+    f.restype = _I
+    f.argtypes = [_I]
+    return bool(f(k_dim))
+
+
+# Inner dimensions from which the products in tf32 terms are no further from 64 bits than a chain of multiply-adds: their error is
+# 2.2e-7 to 2.8e-7 of the result's norm at any length, the chain's 1.5e-7 over 64 terms, 4e-7 over 512, 8e-7 over 2,048.
+F32_TC_MIN_INNER = 512
+
+
+def gemm_f32_dense_pays(rows: int, n_out: int, k_dim: int, sms: int) -> bool:
+    """Whether a dense product in tf32 terms is estimated to take less than the library's 32-bit one.  A step of 32 along K takes
+    a block of 128 x 128 outputs 0.5 us with few rows and 0.76 with 128, whatever the other blocks do.  The library's reaches 50
+    TFLOP/s over rows rounded up to 64 at best, and needs 26 ns per term of a sum where it does not split sums (15 with few rows, or
+    too few tiles to go without).  Measured, us, library / this (rows x outputs x inner): 2,048 x 8,192 x 3,072 1,810 / 519;
+    128 x 10,304 x 2,048 147 / 56; 128 x 3,072 x 6,144 179 / 147; 512 x 2,048 x 2,048 86 / 56, 128 rows 40 / 54; 4,096 x 192 x 2,048 86 / 56,
+    1,024 rows 40 / 54; 8 x 8,192 x 3,072 60 / 53.  The very few rows that the library gives to its kernels with split sums (up to
+    7, up to 3 with an inner dimension from 3,072 on) stay there: those sums are the more exact ones (1.2e-7 to 2.5e-7)."""
+    if k_dim < F32_TC_MIN_INNER or rows < (4 if k_dim >= 3072 else 8):
+        return False
+    waves = -(-(-(-rows // 128) * -(-n_out // 128)) // sms)
+    ours = 3.0 + waves * -(-k_dim // 32) * (0.5 + 0.26 * min(rows, 128) / 128)
+    per_term = 0.0 if rows <= 16 else 0.026 if rows > 32 and -(-rows // 128) * -(-n_out // 64) >= 48 else 0.0145
+    return ours < max(2.0 * (-(-rows // 64) * 64) * n_out * k_dim / 50e6, per_term * k_dim)
+
+
+def gemm_f32_dense(x, w, out):
+    """out = x [rows, k] . w [n, k]^T in 32-bit."""
+    rows, k_dim = x.shape
+    _check(_fn("se_gemm_f32_dense", "plppp" "iiii" "p")(
+        _rows_ptr(x, "x", torch.float32), x.stride(0), _ptr(w, torch.float32, "w"), _ptr(out, torch.float32, "out"), _ptr(error_word(x.device)),
+        rows, w.shape[0], k_dim, sm_count(x.device), _stream()), "gemm_f32_dense")
+    return out
+
+
+def gemm_f32_grouped(mode: int, a, w, ws: dict, route_w, out, *, experts, max_tiles, n_out, k_dim, activation=None):
+    """The experts' products of the float32 path over rows in expert order; the tile list in ``ws`` must have been built with
+    ``F32_TC_TILE_ROWS`` rows per tile."""
+    _check(_fn("se_gemm_f32_grouped", "i" "pp" "ppppp" "ppp" "iiiii" "iff" "ip")(
+        mode, _ptr(a, torch.float32, "a"), _ptr(w, torch.float32, "w"), _ptr(ws["sorted"]), _ptr(ws["offsets"]),
+        _ptr(ws["tile_expert"]), _ptr(ws["tile_row0"]), _ptr(ws["num_tiles"]), _ptr(route_w, torch.float32, "route_w"),
+        _ptr(out, torch.float32, "out"), _ptr(error_word(out.device)), a.shape[0], experts, max_tiles, n_out, k_dim, *_glu_args(activation),
+        sm_count(out.device), _stream()), "gemm_f32_grouped")
+    return out
+
+
 PAIR_TILE_ROWS = 256      # activation rows per tile of the kernel that runs on pairs of SMs (csrc/gemm_tc_pair.cu)
 
 

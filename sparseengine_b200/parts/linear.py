@@ -4,9 +4,10 @@ The reference runs these through a library GEMM (``F.linear``:
 src/sparseengine/layers/linear.py:174-191, src/sparseengine/layers/embed_head.py:80), and so
 does this module (cuBLAS through ``torch.matmul``), except for up to 8 rows in bfloat16
 (decode), where the product is a stream over the weights and this library's own kernel
-(csrc/gemv.cu) reads them once at memory speed.  In float32 the reduced-precision
-matrix modes are switched off for the whole process, so a float32 product is a true
-32-bit product.
+(csrc/gemv.cu) reads them once at memory speed, and for float32 products that fill the device
+(csrc/gemm_f32_tc.cu: on the tensor cores in tf32 terms, closer to 64 bits than a chain of multiply-adds).
+Otherwise the reduced-precision matrix modes are switched off for the whole process, so a float32 product
+is a true 32-bit product.
 """
 from __future__ import annotations
 
@@ -32,6 +33,18 @@ GEMV_MAX_ROWS = 8
 GEMV_GLU_MAX_OUT = 65536       # gate and up rows together
 
 
+def _product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    """x . w^T in x's type: in float32 with this library's kernel where it is estimated to be ahead, else the library product."""
+    if (x.dtype == torch.float32 and x.dim() == 2 and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1]
+            and not (x.data_ptr() | w.data_ptr()) & 15 and (out is None or out.is_contiguous() and out.shape == (x.shape[0], w.shape[0]))
+            and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
+            and ops.gemm_f32_tc_supported(x.shape[1]) and ops.gemm_f32_dense_pays(x.shape[0], w.shape[0], x.shape[1], ops.sm_count(x.device))):
+        if out is None:
+            out = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)
+        return ops.gemm_f32_dense(x, w, out)
+    return torch.matmul(x, w.t()) if out is None else torch.matmul(x, w.t(), out=out)
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, activation: str | None = None) -> torch.Tensor:
     """x [rows, in], w [out, in] → [rows, out]; CUDA tensors of one dtype only.  ``activation``: a name of
     ``ops.ACTIVATIONS`` applied to the product (inside this library's few-row kernel, else as a kernel of its own)."""
@@ -46,7 +59,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, ac
         if out is None:
             out = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)
         return ops.gemv(x, w, out, activation)
-    y = torch.matmul(x, w.t()) if out is None else torch.matmul(x, w.t(), out=out)
+    y = _product(x, w, out)
     return y if activation is None else ops.activation_(y, activation)
 
 
@@ -58,7 +71,7 @@ def linear_glu(x: torch.Tensor, w: torch.Tensor, activation=None) -> torch.Tenso
     if (USE_GEMV and x.dtype == torch.bfloat16 and x.is_contiguous() and w.is_contiguous() and x.shape[0] <= GEMV_MAX_ROWS
             and w.shape[0] <= GEMV_GLU_MAX_OUT and ops.gemv_supported(x.shape[0], n, x.shape[1])):
         return ops.gemv_glu(x, w, out, activation)
-    return ops.glu(torch.matmul(x, w.t()), out, activation)
+    return ops.glu(_product(x, w), out, activation)
 
 
 def pad_rows(w: torch.Tensor, multiple: int = 8) -> torch.Tensor:
@@ -74,5 +87,5 @@ def linear32(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     if x.dtype != w.dtype:
         raise TypeError(f"linear32: activation {x.dtype} and weight {w.dtype} differ")
     if x.dtype == torch.float32:
-        return torch.matmul(x, w.t())
+        return _product(x, w)
     return torch.mm(x, w.t(), out_dtype=torch.float32)

@@ -43,8 +43,8 @@ class _RoutedSwiGLU(FeedForward):
             raise ValueError(f"activation {spec.activation!r} needs a positive activation_limit")
         return (spec.activation, float(spec.activation_limit), float(spec.activation_alpha))
 
-    # None: tensor cores whenever the sizes allow (bfloat16, row pitches that TMA takes);
-    # False: always the CUDA-core kernels (the float32 path uses them in any case).
+    # None: tensor cores whenever the sizes allow (row pitches that TMA takes; float32: more than a few rows
+    # per expert and inner dimensions from ops.F32_TC_MIN_INNER on); False: always the CUDA-core kernels.
     use_tensor_cores = None
 
     # Which tensor-core kernel runs the experts.  One CTA per tile (csrc/gemm_tc.cu) streams the
@@ -113,6 +113,10 @@ class _RoutedSwiGLU(FeedForward):
             tile_rows = ops.PAIR_TILE_ROWS if pair else ops.moe_tile_rows_tc(a, self.num_experts)
         else:
             tile_rows = self.plain_tile_rows(x, a)
+        # float32 with more than a few rows per expert: tensor cores in tf32 terms (csrc/gemm_f32_tc.cu)
+        f32_tc = (not tc and self.use_tensor_cores is not False and x.dtype == torch.float32 and tile_rows == ops.F32_TC_TILE_ROWS
+                  and min(self.hidden, self.inter) >= ops.F32_TC_MIN_INNER)
+        sorted_rows = tc or f32_tc
         max_tiles = ops.moe_max_tiles(a, self.num_experts, tile_rows)
         i32 = dict(dtype=torch.int32, device=dev)
         ws = {"counts": torch.empty(self.num_experts, **i32), "rank": torch.empty(a, **i32),
@@ -121,13 +125,13 @@ class _RoutedSwiGLU(FeedForward):
               "sorted": (torch.zeros if self.identity_experts else torch.empty)(a, **i32),
               "inv_pos": torch.empty(a, **i32), "tile_expert": torch.empty(max_tiles, **i32),
               "tile_row0": torch.empty(max_tiles, **i32), "num_tiles": torch.empty(1, **i32)}
-        # the tensor-core GEMM reads the activation rows in expert order
-        xs = torch.empty(a, self.hidden, dtype=x.dtype, device=dev) if tc else None
+        # the tensor-core GEMMs read the activation rows in expert order
+        xs = torch.empty(a, self.hidden, dtype=x.dtype, device=dev) if sorted_rows else None
         if self.route_stats is None:
             self.route_stats = torch.zeros(2, dtype=torch.int64, device=dev)
             self.route_stats_large = torch.zeros(2, dtype=torch.int64, device=dev)
         large = tc and self.pair_min_rows is not None and a >= self.pair_min_rows
-        settled = ops.moe_route_build(ids, self.num_experts, tile_rows, ws, gather=(x, xs, self.top_k) if tc else None,
+        settled = ops.moe_route_build(ids, self.num_experts, tile_rows, ws, gather=(x, xs, self.top_k) if sorted_rows else None,
                                       stats=self.route_stats_large if large else self.route_stats)
         if large:        # what this build counted reaches the host behind this step, for later steps' choice
             if getattr(self, "_large_host", None) is None:
@@ -147,6 +151,11 @@ class _RoutedSwiGLU(FeedForward):
                                     activation=self.activation_args)
             ops.moe_grouped_gemm_tc(1, act, self.w2, ws, weights, y, experts=self.num_experts, max_tiles=max_tiles,
                                     n_out=self.hidden, k_dim=self.inter, nt=tile_rows, lists_settled=True)
+        elif f32_tc:
+            ops.gemm_f32_grouped(0, xs, self.w13, ws, None, act, experts=self.num_experts, max_tiles=max_tiles, n_out=self.inter,
+                                 k_dim=self.hidden, activation=self.activation_args)
+            ops.gemm_f32_grouped(1, act, self.w2, ws, weights, y, experts=self.num_experts, max_tiles=max_tiles, n_out=self.hidden,
+                                 k_dim=self.inter)
         else:
             ops.moe_grouped_gemm_plain(0, x, self.w13, ws, None, act, max_tiles=max_tiles, n_out=self.inter,
                                        k_dim=self.hidden, top_k=self.top_k, activation=self.activation_args,
