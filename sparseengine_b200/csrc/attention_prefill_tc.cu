@@ -202,46 +202,62 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
         asm volatile("cp.async.wait_all;" ::: "memory");
         if (!ok) { abort_s = 1; if (lane == 0) atomicCAS(error, 0, 11); }
     } else if (warp == 1 || warp == kMmaWarp2) {
-        // ---- MMA issuers: one warp (one lane) per query tile ---------------------------------------
+        // ---- MMA issuers: one warp per query tile ---------------------------------------
         // Order for a tile: S(j), then P·V of tile j-1 as its P arrives; S(j+1) is thus issued
         // before the softmax of tile j has finished.  The two issuers share the tensor pipe and
         // do not wait for one another; a K/V stage is free when both have committed its P·V.
-        if (lane == 0) {
-            const int x = warp == 1 ? 0 : 1;
-            const uint32_t id_s = idesc(kKeys, 0), id_o = idesc(D, 1);
-            bool ok = true;
-            auto issue_pv = [&](int i) {
-                if (!mbar_wait(bar(&bars.p_full[x][i & 1]), (i >> 1) & 1, &abort_s)) { ok = false; return; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t va = smem_u32(kv_s) + (i % kStages) * kKVStageBytes + 2 * kHalfBytes;
-                const uint32_t pa = tmem_s(x, i & 1);        // P of tile i lies over the first half of its S buffer
+        // The warp runs as a whole through uniform loops and one elected lane issues (fa_util.cuh): 8,192 tokens behind 16,384 keys 4,145 us,
+        // issued under a divergent branch and with two more shuffles a tile in the softmax 4,206.
+        const int x = warp == 1 ? 0 : 1;
+        const uint32_t id_s = idesc(kKeys, 0), id_o = idesc(D, 1);
+        const int tiles = uniform(num_tiles);
+        const uint32_t tm = (uint32_t)uniform((int)tmem), o_at = tm + 128 * x, s_at = tm + 256 + 128 * x;
+        const uint64_t q_desc = desc_kmajor(smem_u32(q_s) + x * kQBytes);
+        bool ok = true;
+        auto wait = [&](uint64_t* b, uint32_t parity) {
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(b), parity, &abort_s));
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        };
+        auto issue_pv = [&](int i, int stage) {
+            wait(&bars.p_full[x][i & 1], (i >> 1) & 1);
+            if (ok && elect_one()) {
+                const uint64_t v = desc_mnmajor(smem_u32(kv_s) + stage * kKVStageBytes + 2 * kHalfBytes, kHalfBytes);
+                const uint32_t pa = s_at + 64 * (i & 1);     // P of tile i lies over the first half of its S buffer
 #pragma unroll
                 for (int kk = 0; kk < kKeys / 16; ++kk)      // 16 keys per MMA: 8 columns of P, two 8-key groups of V
-                    umma_ts(tmem_o(x), pa + (uint32_t)(kk * 8), desc_mnmajor(va + kk * 2048, kHalfBytes), id_o,
-                            (i > 0 || kk > 0) ? 1u : 0u);
+                    umma_ts(o_at, pa + (uint32_t)(kk * 8), v + (uint64_t)(kk * 128), id_o, (i > 0 || kk > 0) ? 1u : 0u);
                 umma_commit(bar(&bars.p_empty[x]));
-                umma_commit(bar(&bars.kv_empty[i % kStages]));
-            };
-            for (int j = 0; j < num_tiles && ok; ++j) {
-                const int b = j & 1;
-                if (!mbar_wait(bar(&bars.kv_full[j % kStages]), (j / kStages) & 1, &abort_s)) { ok = false; break; }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the copies were generic-proxy writes
-                if (j >= 2 && !mbar_wait(bar(&bars.s_empty[x][b]), ((j >> 1) - 1) & 1, &abort_s)) { ok = false; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t ka = smem_u32(kv_s) + (j % kStages) * kKVStageBytes;
+                umma_commit(bar(&bars.kv_empty[stage]));
+            }
+            __syncwarp();
+        };
+        int stage = 0, before = 0;                           // of tiles j and j - 1
+        uint32_t turn = 0;                                   // how often the stages have gone round, modulo 2
+        for (int j = 0; j < tiles && ok; ++j) {
+            const int b = j & 1;
+            wait(&bars.kv_full[stage], turn);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the copies were generic-proxy writes
+            if (ok && j >= 2) wait(&bars.s_empty[x][b], ((j >> 1) - 1) & 1);
+            if (ok && elect_one()) {
+                const uint64_t k_desc = desc_kmajor(smem_u32(kv_s) + stage * kKVStageBytes);
 #pragma unroll
                 for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
-                        umma(tmem_s(x, b), desc_kmajor(smem_u32(q_s) + x * kQBytes + kb * (kRows * 128)) + (uint64_t)(kk * 2),
-                             desc_kmajor(ka + kb * kHalfBytes) + (uint64_t)(kk * 2), id_s, (kb > 0 || kk > 0) ? 1u : 0u);
+                        umma(s_at + 64 * b, q_desc + (uint64_t)(kb * (kRows * 128 / 16) + kk * 2), k_desc + (uint64_t)(kb * (kHalfBytes / 16) + kk * 2), id_s,
+                             (kb > 0 || kk > 0) ? 1u : 0u);
                 umma_commit(bar(&bars.s_full[x][b]));
-                if (j >= 1) issue_pv(j - 1);
             }
-            if (ok) issue_pv(num_tiles - 1);
-            if (ok) umma_commit(bar(&bars.o_done[x]));
-            if (!ok) { abort_s = 1; atomicCAS(error, 0, 12); }
+            __syncwarp();
+            if (ok && j >= 1) issue_pv(j - 1, before);
+            before = stage;
+            stage = stage + 1 == kStages ? 0 : stage + 1;
+            if (stage == 0) turn ^= 1;
         }
+        if (ok) issue_pv(tiles - 1, before);
+        if (ok && elect_one()) umma_commit(bar(&bars.o_done[x]));
+        __syncwarp();
+        if (!ok && lane == 0) { abort_s = 1; atomicCAS(error, 0, 12); }
     } else if (warp < 2 + 4 * kTiles) {
         // ---- softmax and epilogue: warps 2-5 own query tile 0, warps 6-9 tile 1; one thread per row ----
         const int x = (warp - 2) >> 2;
@@ -255,6 +271,7 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         float m_ref = -INFINITY, l = 0.f;                  // reference maximum (log2 units), running sum
         const float slope = se::mma::raw_slope(opt, kvh * group + rr % group);      // distance bias per token, raw units
+        const int pos_first = __shfl_sync(0xffffffffu, pos, 0), lo_last = __shfl_sync(0xffffffffu, lo, 31);
         bool ok = true;
         for (int j = 0; j < num_tiles && ok; ++j) {
             const int b = j & 1;
@@ -291,8 +308,7 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
             // is seen by every row as far as it holds such keys; in a window's tile a key before the row's window is
             // seen if it is a kept one that no tile of kept keys has brought.
             const bool full = first ? key0 + kKeys <= kept
-                                    : key0 + kKeys - 1 <= __shfl_sync(0xffffffffu, pos, 0) &&
-                                          key0 >= __shfl_sync(0xffffffffu, lo, 31) && key0 >= kept;
+                                    : key0 + kKeys - 1 <= pos_first && key0 >= lo_last && key0 >= kept;
             if (!full) {
 #pragma unroll
                 for (int c = 0; c < 64; ++c) {
