@@ -101,32 +101,39 @@ struct WalkArgs {
 // Two groups of four warps share a chunk's products, all of them on the tensor cores in tf32 terms (split_mma.cuh).  Without a
 // system to solve, group 0 makes the outputs (q S_0, then P u) while group 1 updates the state, which it keeps in registers and
 // hands over through a second buffer, and brings the next values: one barrier per chunk.  With one, group 0 makes
-// u = U - W S_0 and then the state's update while group 1 makes q S_0 and then the outputs: two barriers.  Tiles of q, k, W and P
-// that a warp alone reads are copied by that warp as soon as it has read the last chunk's.  Row pitches are such that no fragment read
+// u = U - W S_0 and then the state's update while group 1 makes q S_0 and then the outputs: two barriers.  With chunks of 64 tokens
+// and 128 state rows (one block per SM) a third group brings tiles and values, a chunk ahead where there is room for two: the copies, a cp.async
+// per 16 bytes, took the other two 1,400 to 2,300 of a chunk's 8,000 to 9,000 cycles.  Elsewhere (two blocks per SM) tiles are copied by the
+// warps that read them, as soon as they have read the last chunk's.  Row pitches are such that no fragment read
 // meets a bank twice: 8 more than a multiple of 32 where rows lie along k (two neighbours per lane), 4 more than a
 // multiple of 16 where columns do.
 template <int T, int DP, int C, bool SOLVE, bool CHANNEL>
 struct WalkShape {
     static constexpr int kQP = DP + 8, kKP = DP + 4, kPP = T + 8, kCP = C + 4;
     static constexpr int kBuffers = SOLVE ? 1 : 2;                    // of k, u and the state
-    static constexpr int kFloats = (SOLVE ? 2 : 1) * T * kQP + kBuffers * T * kKP + T * kPP +
+    static constexpr bool kLoader = T == 64 && DP == 128;             // a group that only loads
+    static constexpr int kThreads = kLoader ? 384 : 256;
+    static constexpr int kAhead = kLoader ? 2 : 1;                    // buffers of q and W
+    static constexpr int kFloats = (SOLVE ? 2 : 1) * kAhead * T * kQP + kBuffers * T * kKP + T * kPP +
                                    kBuffers * (CHANNEL ? 1 : 2) * T * kCP + kBuffers * DP * kCP + 2 * T;
     static constexpr int kBlocks = kFloats * 4 <= 112 * 1024 ? 2 : 1;            // per SM
 };
 
 template <int T, int DP, int C, bool SOLVE, bool CHANNEL, typename TV>
-__global__ void __launch_bounds__(kThreads, WalkShape<T, DP, C, SOLVE, CHANNEL>::kBlocks)
+__global__ void __launch_bounds__(WalkShape<T, DP, C, SOLVE, CHANNEL>::kThreads, WalkShape<T, DP, C, SOLVE, CHANNEL>::kBlocks)
 chunk_walk_kernel(const WalkArgs a) {
     using Shape = WalkShape<T, DP, C, SOLVE, CHANNEL>;
     constexpr int QP = Shape::kQP, KP = Shape::kKP, PP = Shape::kPP, CP = Shape::kCP, NB = Shape::kBuffers;
+    constexpr int QB = Shape::kAhead * T * QP, kThreads = Shape::kThreads;
+    constexpr bool LOADER = Shape::kLoader;
     constexpr int WR = T / 16, WC = 4 / WR, NT = C / 8 / WC;          // a warp's outputs: 16 rows, NT tiles of eight columns
     constexpr int MT = DP / 64, NS = C / 8;                           // a warp's state: MT tiles of 16 rows, all columns
     constexpr int NQ = T * C / 4 / 128;                               // quads of the chunk's value columns per thread of a group
     static_assert(SOLVE || T == 64, "without a system a warp has its rows of q and P for itself");
     extern __shared__ __align__(16) float sm[];
-    float* qs = sm;                                  // [T][QP]
-    float* ws = qs + T * QP;                         // [T][QP]: W
-    float* ks = ws + (SOLVE ? T * QP : 0);           // [NB][T][KP]
+    float* qs = sm;                                  // [T][QP], twice with a loading group
+    float* ws = qs + QB;                             // W: the same
+    float* ks = ws + (SOLVE ? QB : 0);               // [NB][T][KP]
     float* ps = ks + NB * T * KP;                    // [T][PP]
     float* us = ps + T * PP;                         // [NB][T][CP]: u
     float* u2 = CHANNEL ? us : us + NB * T * CP;     // [NB][T][CP]: e^(B_n - B_t) u (decays per head)
@@ -164,14 +171,14 @@ chunk_walk_kernel(const WalkArgs a) {
     const TV* vb = static_cast<const TV*>(a.v) + (size_t)h * dv + c0;
     auto load_k = [&](float* to, int t0, int n) { load(to, KP, kb, a.qk_stride, t0, n, T, 0, DP, 0, d, gt, 128); };
     auto load_p = [&](int t0, int n) {
-        if (SOLVE) load(ps, PP, pb, (size_t)a.H * T, t0, n, T, 0, T, 0, T, gt, 128);
+        if (SOLVE || LOADER) load(ps, PP, pb, (size_t)a.H * T, t0, n, T, 0, T, 0, T, gt, 128);
         else load(ps, PP, pb, (size_t)a.H * T, t0, n, 16, gw * 16, T, 0, T, lane, 32);
     };
-    auto load_q = [&](int t0, int n) {
-        if (SOLVE) load(qs, QP, qb, a.qk_stride, t0, n, T, 0, DP, 0, d, gt, 128);
+    auto load_q = [&](int t0, int n, int buffer = 0) {
+        if (SOLVE || LOADER) load(qs + buffer * T * QP, QP, qb, a.qk_stride, t0, n, T, 0, DP, 0, d, gt, 128);
         else load(qs, QP, qb, a.qk_stride, t0, n, 16, gw * 16, DP, 0, d, lane, 32);
     };
-    auto load_w = [&](int t0, int n) { load(ws, QP, wb, (size_t)a.H * d, t0, n, T, 0, DP, 0, d, gt, 128); };
+    auto load_w = [&](int t0, int n, int buffer = 0) { load(ws + buffer * T * QP, QP, wb, (size_t)a.H * d, t0, n, T, 0, DP, 0, d, gt, 128); };
 
     // rows of x . S
     auto state_product = [&](const float* x, const float* S, float (&acc)[1][NT][4]) {
@@ -337,23 +344,47 @@ chunk_walk_kernel(const WalkArgs a) {
             }
             if (gt < T) rss[buffer * T + gt] = rfac;
         };
-        if (group == 0) {
+        if (group == (LOADER ? 2 : 0)) {
             load_q(t_first, first_n);
             cp_commit();
             load_p(t_first, first_n);
             cp_commit();
-        } else {
+        }
+        if (group == (LOADER ? 2 : 1)) {
             load_k(ks, t_first, first_n);
             cp_commit();
             load_v(t_first, first_n);
             put_values(0);
-            total = a.eb[(size_t)(t_first + first_n - 1) * a.H + h];
-            cp_wait<0>();                            // k
+            cp_wait<0>();                            // k (and, with a loading group, q and P)
         }
+        if (group == 1) total = a.eb[(size_t)(t_first + first_n - 1) * a.H + h];
         __syncthreads();                             // state, u and factors of the first chunk
         if (group == 1) get_state(Ss);
         const float skip = a.skip != nullptr ? a.skip[h] : 0.f;
         int cur = 0;
+        if (LOADER && group == 2) {
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+            for (int t0 = t_first; t0 < t_last; t0 += T, cur ^= 1) {
+                const int next = t0 + T, next_n = min(T, t_last - next);
+                if (t0 > t_first) {
+                    cp_wait<0>();
+                    asm volatile("bar.arrive 4, 256;" ::: "memory");         // this chunk's P is there
+                }
+                if (next < t_last) {
+                    load_q(next, next_n, cur ^ 1);
+                    load_k(ks + (cur ^ 1) * T * KP, next, next_n);
+                    cp_commit();
+                    load_v(next, next_n);
+                    put_values(cur ^ 1);
+                    asm volatile("bar.sync 3, 256;" ::: "memory");           // this chunk's P has been read
+                    load_p(next, next_n);
+                    cp_commit();
+                    cp_wait<1>();                    // the next q and k
+                }
+                __syncthreads();
+            }
+        } else {
+        if (LOADER) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");        // 128 x (2 x 208 + 88): what 384 threads of 168 have
         for (int t0 = t_first; t0 < t_last; t0 += T, cur ^= 1) {
             const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
             if (group == 0) {
@@ -367,18 +398,25 @@ chunk_walk_kernel(const WalkArgs a) {
                             const int t = r0 + 8 * j, c = col0 + 8 * x + 2 * lc;
                             raw[j][x] = t < n && c0 + c < dv ? load2(vb + (size_t)(t0 + t) * a.v_stride + c) : make_float2(0.f, 0.f);
                         }
-                cp_wait<1>();                        // q
-                __syncwarp();
-                state_product(qs, Ss + cur * DP * CP, acc);
-                __syncwarp();
-                if (next < t_last) load_q(next, next_n);
-                cp_commit();
-                cp_wait<1>();                        // P
-                __syncwarp();
-                token_product(us + cur * T * CP, sum);
-                __syncwarp();
-                if (next < t_last) load_p(next, next_n);
-                cp_commit();
+                if constexpr (LOADER) {
+                    state_product(qs + cur * T * QP, Ss + cur * DP * CP, acc);
+                    if (t0 > t_first) asm volatile("bar.sync 4, 256;" ::: "memory");
+                    token_product(us + cur * T * CP, sum);
+                    if (next < t_last) asm volatile("bar.arrive 3, 256;" ::: "memory");
+                } else {
+                    cp_wait<1>();                    // q
+                    __syncwarp();
+                    state_product(qs, Ss + cur * DP * CP, acc);
+                    __syncwarp();
+                    if (next < t_last) load_q(next, next_n);
+                    cp_commit();
+                    cp_wait<1>();                    // P
+                    __syncwarp();
+                    token_product(us + cur * T * CP, sum);
+                    __syncwarp();
+                    if (next < t_last) load_p(next, next_n);
+                    cp_commit();
+                }
 #pragma unroll
                 for (int x = 0; x < NT; ++x)
 #pragma unroll
@@ -395,17 +433,20 @@ chunk_walk_kernel(const WalkArgs a) {
 #pragma unroll
                 for (int i = 0; i < MT; ++i) totals[i][0] = totals[i][1] = now;
                 if (next < t_last) {
-                    load_k(ks + (cur ^ 1) * T * KP, next, next_n);
-                    load_v(next, next_n);
+                    if (!LOADER) {
+                        load_k(ks + (cur ^ 1) * T * KP, next, next_n);
+                        load_v(next, next_n);
+                    }
                     total = a.eb[(size_t)(next + next_n - 1) * a.H + h];
                 }
                 cp_commit();
                 update_state(ks + cur * T * KP, u2 + cur * T * CP, totals);
                 put_state(Ss + (cur ^ 1) * DP * CP);
-                if (next < t_last) put_values(cur ^ 1);
+                if (!LOADER && next < t_last) put_values(cur ^ 1);
                 cp_wait<0>();                        // the next k
             }
             __syncthreads();
+        }
         }
         last_state = Ss + cur * DP * CP;
     } else {
@@ -439,28 +480,55 @@ chunk_walk_kernel(const WalkArgs a) {
                                    : row < d ? a.tot[((size_t)(t_first / T + e + (t0 - t_first) / T) * a.H + h) * d + row] : 0.f;
                 }
         };
-        if (group == 0) {
+        if (LOADER ? group == 2 : group == 0) {
             load_w(t_first, first_n);
+            if (LOADER) load_q(t_first, first_n);
             cp_commit();
             load_k(ks, t_first, first_n);
-            load_u(t_first, first_n);
-            load_factors(a.ts, t_first, first_n);
-            load_totals(t_first, first_n);
-        } else {
+            if (LOADER) load_p(t_first, first_n);
+        } else if (!LOADER) {
             load_q(t_first, first_n);
             cp_commit();
             load_p(t_first, first_n);
-            load_factors(a.rs, t_first, first_n);
         }
         cp_commit();
+        if (group == 0) {
+            load_u(t_first, first_n);
+            load_factors(a.ts, t_first, first_n);
+            load_totals(t_first, first_n);
+        } else if (group == 1) {
+            load_factors(a.rs, t_first, first_n);
+        }
         __syncthreads();
         if (group == 0) get_state(Ss);
-        for (int t0 = t_first; t0 < t_last; t0 += T) {
+        int cur = 0;
+        if (LOADER && group == 2) {
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+            for (int t0 = t_first; t0 < t_last; t0 += T, cur ^= 1) {
+                const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
+                cp_wait<0>();                        // W and q
+                __syncthreads();                     // k and P of the chunk before have been read
+                if (t0 > t_first) {
+                    load_k(ks, t0, n);
+                    load_p(t0, n);
+                }
+                cp_commit();
+                if (next < t_last) {
+                    load_w(next, next_n, cur ^ 1);
+                    load_q(next, next_n, cur ^ 1);
+                }
+                cp_commit();
+                cp_wait<1>();
+                __syncthreads();
+            }
+        } else {
+        if (LOADER) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");        // 128 x (2 x 208 + 88): what 384 threads of 168 have
+        for (int t0 = t_first; t0 < t_last; t0 += T, cur ^= LOADER) {
             const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
             cp_wait<1>();                            // W or q (k and P may still be on their way)
             __syncthreads();                         // and the state is up to date
             float acc[1][NT][4];
-            state_product(group == 0 ? ws : qs, Ss, acc);
+            state_product((group == 0 ? ws : qs) + cur * T * QP, Ss, acc);
             if (group == 0) {
 #pragma unroll
                 for (int x = 0; x < NT; ++x)
@@ -476,26 +544,26 @@ chunk_walk_kernel(const WalkArgs a) {
             __syncthreads();                         // u, k and P are there, W, q and the state have been read
             if (group == 0) {
                 if (next < t_last) {
-                    load_w(next, next_n);
+                    if (!LOADER) load_w(next, next_n);
                     load_u(next, next_n);
                     load_factors(a.ts, next, next_n);
                 }
                 cp_commit();
                 update_state(ks, u2, totals);
                 put_state(Ss);
-                group_sync(0);
+                if (!LOADER) group_sync(0);
                 if (next < t_last) {
-                    load_k(ks, next, next_n);
+                    if (!LOADER) load_k(ks, next, next_n);
                     load_totals(next, next_n);
                 }
                 cp_commit();
             } else {
                 float sum[1][NT][4];
-                if (next < t_last) load_q(next, next_n);
+                if (!LOADER && next < t_last) load_q(next, next_n);
                 cp_commit();
                 token_product(us, sum);
-                group_sync(1);
-                if (next < t_last) load_p(next, next_n);
+                if (!LOADER) group_sync(1);
+                if (!LOADER && next < t_last) load_p(next, next_n);
                 cp_commit();
 #pragma unroll
                 for (int x = 0; x < NT; ++x)
@@ -504,6 +572,7 @@ chunk_walk_kernel(const WalkArgs a) {
                 if (next < t_last) load_factors(a.rs, next, next_n);
                 put_outputs(t0, n, acc);
             }
+        }
         }
     }
     cp_wait<0>();
@@ -546,18 +615,26 @@ __device__ __forceinline__ void row_products(const float* x, const float* y, int
 
 // ---- launches ------------------------------------------------------------------------------------
 template <typename... KArgs, typename... Args>
-int launch(void (*kernel)(KArgs...), dim3 grid, size_t smem, cudaStream_t stream, Args... args) {
+int launch_threads(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    kernel<<<grid, kThreads, smem, stream>>>(KArgs(args)...);
+    kernel<<<grid, threads, smem, stream>>>(KArgs(args)...);
     return (int)cudaGetLastError();
+}
+template <typename... KArgs, typename... Args>
+int launch(void (*kernel)(KArgs...), dim3 grid, size_t smem, cudaStream_t stream, Args... args) {
+    return launch_threads(kernel, grid, kThreads, smem, stream, args...);
+}
+template <int T, int DP, int C, bool SOLVE, bool CHANNEL, typename TV>
+int launch_walk_columns(const WalkArgs& a, int entries, cudaStream_t stream) {
+    using Shape = WalkShape<T, DP, C, SOLVE, CHANNEL>;
+    return launch_threads(chunk_walk_kernel<T, DP, C, SOLVE, CHANNEL, TV>, dim3(entries, a.H, ceil_div(a.dv, C)), Shape::kThreads,
+                          Shape::kFloats * sizeof(float), stream, a);
 }
 template <int T, int DP, bool SOLVE, bool CHANNEL, typename TV>
 int launch_walk(const WalkArgs& a, int entries, int cols, cudaStream_t stream) {
-    const dim3 grid(entries, a.H, ceil_div(a.dv, cols));
-    if (cols == 16)
-        return launch(chunk_walk_kernel<T, DP, 16, SOLVE, CHANNEL, TV>, grid, WalkShape<T, DP, 16, SOLVE, CHANNEL>::kFloats * sizeof(float), stream, a);
-    return launch(chunk_walk_kernel<T, DP, 32, SOLVE, CHANNEL, TV>, grid, WalkShape<T, DP, 32, SOLVE, CHANNEL>::kFloats * sizeof(float), stream, a);
+    if (cols == 16) return launch_walk_columns<T, DP, 16, SOLVE, CHANNEL, TV>(a, entries, stream);
+    return launch_walk_columns<T, DP, 32, SOLVE, CHANNEL, TV>(a, entries, stream);
 }
 
 // Value columns per block: 32 while the blocks then fill the device, 16 (twice the blocks, which each read q and k) else.
