@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(kThreads, 3)
 ssm_prepare_kernel(const float* __restrict__ xbc, const T_* __restrict__ proj, int pitch, int dt_off, const float* __restrict__ dt_bias,
                    const float* __restrict__ a_log, const int* __restrict__ cu_q, int entries, float* __restrict__ p,
                    float* __restrict__ rs, float* __restrict__ ts, float* __restrict__ steps, int H, int P, int N, int G) {
-    constexpr int T = 64, QP = DP + 4;
+    constexpr int T = 64, QP = DP + 8;
     extern __shared__ __align__(16) float sm[];
     float* qs = sm;                                  // C
     float* ks = qs + T * QP;                         // B
@@ -42,14 +42,15 @@ ssm_prepare_kernel(const float* __restrict__ xbc, const T_* __restrict__ proj, i
     chunk_of<T>(blockIdx.x, cu_q, entries, first, n);
     if (n <= 0) return;
     const int g = blockIdx.y, rep = H / G, width = H * P + 2 * G * N;
-    load_tile<T, DP>(ks, xbc + H * P + (size_t)g * N, width, first, n, N);
-    load_tile<T, DP>(qs, xbc + H * P + (size_t)(G + g) * N, width, first, n, N);
+    load_tile<T, DP, 8>(ks, xbc + H * P + (size_t)g * N, width, first, n, N);
+    load_tile<T, DP, 8>(qs, xbc + H * P + (size_t)(G + g) * N, width, first, n, N);
     cp_commit();
     cp_wait<0>();
     __syncthreads();
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float acc[4][4] = {};
-    row_products<DP, 4>(qs, ks, ty, tx, acc);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float* const x[1] = {qs};
+    triangle_products<DP, 1>(x, ks, warp, lane, [&](const auto& acc, int r0, int n0, int zeros) {
+    constexpr int NT = sizeof(acc[0]) / sizeof(acc[0][0]);
     for (int h0 = 0; h0 < rep; h0 += 8) {
         __syncthreads();                             // the sums of the eight heads before have been read
         if (h0 + warp < rep) {                       // a warp per head, two neighbouring tokens per lane
@@ -82,18 +83,22 @@ ssm_prepare_kernel(const float* __restrict__ xbc, const T_* __restrict__ proj, i
         for (int hh = 0; hh < min(8, rep - h0); ++hh) {
             const int h = g * rep + h0 + hh;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int t = ty + 16 * i;
+            for (int j = 0; j < 4; j += 2) {
+                const int t = r0 + 4 * j;
                 if (t >= n) continue;
                 const double bt = sums[hh][t];
+                float* row = p + ((size_t)(first + t) * H + h) * T;
 #pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const int s = tx + 16 * b;
-                    p[((size_t)(first + t) * H + h) * T + s] = s <= t ? acc[i][b] * expf((float)(bt - sums[hh][s])) : 0.f;
+                for (int x = 0; x < NT; ++x) {
+                    const int s = n0 + 8 * x;
+                    *reinterpret_cast<float2*>(row + s) = make_float2(s <= t ? acc[0][x][j] * expf((float)(bt - sums[hh][s])) : 0.f,
+                                                                      s < t ? acc[0][x][j + 1] * expf((float)(bt - sums[hh][s + 1])) : 0.f);
                 }
+                for (int s = zeros; s < T; s += 16) *reinterpret_cast<float2*>(row + s) = make_float2(0.f, 0.f);
             }
         }
     }
+    });
 }
 
 // x[t] -= sum_{s < t} A[t][s] x[s]: forward substitution, one column per thread; at [s][t] transposed
@@ -141,7 +146,7 @@ template <int DP, typename T_>
 __global__ void __launch_bounds__(kThreads, 2)
 delta_head_prepare_kernel(const DeltaInputs<T_> in, float* __restrict__ p, float* __restrict__ w, float* __restrict__ u,
                           float* __restrict__ rs, float* __restrict__ ts, float* __restrict__ eb_out) {
-    constexpr int T = 64, QP = DP + 4, HB = 32;
+    constexpr int T = 64, QP = DP + 8, HB = 32;
     const int H = in.H, G = in.G, d = in.d, dv = in.dv;
     extern __shared__ __align__(16) float sm[];
     float* ks = sm;
@@ -153,8 +158,8 @@ delta_head_prepare_kernel(const DeltaInputs<T_> in, float* __restrict__ p, float
     chunk_of<T>(blockIdx.x, in.cu_q, in.entries, first, n);
     if (n <= 0) return;
     const int h = blockIdx.y, g = h / (H / G), width = 2 * G * d + H * dv, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    load_tile<T, DP>(qs, in.qkv + (size_t)g * d, width, first, n, d);
-    load_tile<T, DP>(ks, in.qkv + (size_t)(G + g) * d, width, first, n, d);
+    load_tile<T, DP, 8>(qs, in.qkv + (size_t)g * d, width, first, n, d);
+    load_tile<T, DP, 8>(ks, in.qkv + (size_t)(G + g) * d, width, first, n, d);
     cp_commit();
     float after[2] = {};
     if (warp == 0) {                                 // two neighbouring tokens per lane
@@ -200,37 +205,34 @@ delta_head_prepare_kernel(const DeltaInputs<T_> in, float* __restrict__ p, float
                 eb_out[at_] = eb[t];
             }
         }
-    {
-        const int ty = tid >> 4, tx = tid & 15;
-        float kk[4][4] = {}, qk[4][4] = {};
-#pragma unroll 2
-        for (int k = 0; k < DP; k += 4) {
-            float4 yv[4];
+    const float* const x[2] = {ks, qs};
+    triangle_products<DP, 2>(x, ks, warp, lane, [&](const auto& acc, int r0, int n0, int zeros) {
+        constexpr int NT = sizeof(acc[0]) / sizeof(acc[0][0]);
 #pragma unroll
-            for (int b = 0; b < 4; ++b) yv[b] = ld4(ks + (tx + 16 * b) * QP + k);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 kv = ld4(ks + (ty + 16 * i) * QP + k), qv = ld4(qs + (ty + 16 * i) * QP + k);
-#pragma unroll
-                for (int b = 0; b <= i; ++b) {       // tiles beyond the diagonal are zero
-                    kk[i][b] = fma4(kv, yv[b], kk[i][b]);
-                    qk[i][b] = fma4(qv, yv[b], qk[i][b]);
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int t = ty + 16 * i;
+        for (int j = 0; j < 4; j += 2) {
+            const int t = r0 + 4 * j;
             const float ft = bt[t] * fk[t];
+            float* row = p + ((size_t)(first + t) * H + h) * T;
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int s = tx + 16 * b;
-                const float f = s <= t ? expf((float)(sums[t] - sums[s])) * fk[s] : 0.f;
-                at[s * (T + 4) + t] = s < t ? ft * f * kk[i][b] : 0.f;
-                if (t < n) p[((size_t)(first + t) * H + h) * T + s] = s <= t ? fq[t] * f * qk[i][b] : 0.f;
+            for (int x = 0; x < NT; ++x) {
+                const int s0 = n0 + 8 * x;
+                float2 pv;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int s = s0 + i;
+                    const float f = s <= t ? expf((float)(sums[t] - sums[s])) * fk[s] : 0.f;
+                    at[s * (T + 4) + t] = s < t ? ft * f * acc[0][x][j + i] : 0.f;
+                    (i ? pv.y : pv.x) = s <= t ? fq[t] * f * acc[1][x][j + i] : 0.f;
+                }
+                if (t < n) *reinterpret_cast<float2*>(row + s0) = pv;
+            }
+            for (int s = zeros; s < T; s += 16) {
+                at[s * (T + 4) + t] = 0.f;
+                at[(s + 1) * (T + 4) + t] = 0.f;
+                if (t < n) *reinterpret_cast<float2*>(row + s) = make_float2(0.f, 0.f);
             }
         }
-    }
+    });
     __syncthreads();                                 // A is there, q has been read
     for (int c = tid; c < d + dv; c += kThreads) {
         float* dst = c < d ? w + ((size_t)first * H + h) * d + c : u + ((size_t)first * H + h) * dv + (c - d);
@@ -321,8 +323,8 @@ delta_channel_prepare_kernel(const DeltaInputs<T_> in, float* __restrict__ p, fl
     chunk_of<T>(blockIdx.x, in.cu_q, in.entries, first, n);
     if (n <= 0) return;
     const int h = blockIdx.y, g = h / (H / G), width = 2 * G * d + H * dv, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    load_tile<T, DP>(qs, in.qkv + (size_t)g * d, width, first, n, d);
-    load_tile<T, DP>(ks, in.qkv + (size_t)(G + g) * d, width, first, n, d);
+    load_tile<T, DP, 4>(qs, in.qkv + (size_t)g * d, width, first, n, d);
+    load_tile<T, DP, 4>(ks, in.qkv + (size_t)(G + g) * d, width, first, n, d);
     cp_commit();
     const float rate = expf(in.a_log[h]);
 #pragma unroll 4
@@ -512,7 +514,7 @@ extern "C" int se_ssm_walk(const float* xbc, const void* proj, int pitch, int dt
     SE_WALK_DIMS(N, {
         int rc = 0;
         SE_DISPATCH_DTYPE(dtype, T_, {
-            rc = launch(ssm_prepare_kernel<DP, T_>, dim3(tokens / 64 + entries, G), 2 * 64 * (DP + 4) * sizeof(float), stream, xbc,
+            rc = launch(ssm_prepare_kernel<DP, T_>, dim3(tokens / 64 + entries, G), 2 * 64 * (DP + 8) * sizeof(float), stream, xbc,
                         (const T_*)proj, pitch, dt_off, dt_bias, a_log, cu_q, entries, p, rs, ts, steps, H, P, N, G);
         });
         if (rc != 0) return rc;
@@ -554,9 +556,9 @@ extern "C" int se_delta_walk(const float* qkv, const void* in_a, int a_pitch, co
                 float* rs = p + rows * 64;
                 float* ts = rs + rows;
                 float* eb = ts + rows;
-                const int tile = 64 * (DP + 4) > 32 * kThreads ? 64 * (DP + 4) : 32 * kThreads;
+                const int tile = 64 * (DP + 8) > 32 * kThreads ? 64 * (DP + 8) : 32 * kThreads;
                 const int rc = launch(delta_head_prepare_kernel<DP, T_>, dim3(tokens / 64 + entries, H),
-                                      (64 * (DP + 4) + 64 * 68 + tile) * sizeof(float), stream, in, p, w, u, rs, ts, eb);
+                                      (64 * (DP + 8) + 64 * 68 + tile) * sizeof(float), stream, in, p, w, u, rs, ts, eb);
                 if (rc != 0) return rc;
                 a.q = qkv; a.k = qkv + G * d; a.qk_stride = 2 * G * d + H * dv; a.rep = H / G; a.p = p; a.rs = rs; a.ts = ts; a.eb = eb;
                 return launch_walk<64, DP, true, false, float>(a, entries, cols, stream);

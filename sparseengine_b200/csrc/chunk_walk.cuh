@@ -15,8 +15,8 @@
 // What bounds the walk is arithmetic (3 to 5 multiply-adds per state element and token) along a chain of chunks; 16-bit operands would
 // lose what the recurrence has to keep.  With multiply-adds it stood at half their rate, its other half shared-memory reads (8 x 8 outputs
 // a thread, an LDS.128 each four multiply-adds); products in tf32 terms by mma.sync read less.  Measured, multiply-adds / now: state space,
-// 2,048 tokens of 64 heads of 64 columns, 204 / 152 us; retention, 8,192 tokens of 32 heads of 128, 752 / 563; delta rule per channel, 4,670 tokens of
-// 16 heads of 128, 418 / 333; per head, 2,048 tokens, 176 / 134.  Sixteen warps instead of eight: 168, 616, -, 148.  Every exponent is a
+// 2,048 tokens of 64 heads of 64 columns, 204 / 150 us; retention, 8,192 tokens of 32 heads of 128, 752 / 541; delta rule per channel, 4,670 tokens of
+// 16 heads of 128, 418 / 333; per head, 2,048 tokens, 176 / 123.  Sixteen warps at the products instead of eight, all loading for themselves: 168, 616, -, 148 (eight: 152, 563, 333, 134).  Every exponent is a
 // difference of sums of logarithms that is at most 0 up to the 64-bit sums' rounding
 // (no token's logarithm lies below -1e4) or, for decays per channel, a product of decays of at most T tokens: no term overflows.
 //
@@ -584,10 +584,10 @@ chunk_walk_kernel(const WalkArgs a) {
 }
 
 // ---- what the walk needs, per chunk ---------------------------------------------------------------
-// rows r of `src` (element (first + r) * stride + c) into tile [T][QP]; rows from n on and columns from d to DP are zeros
-template <int T, int DP>
+// rows r of `src` (element (first + r) * stride + c) into tile [T][DP + PAD]; rows from n on and columns from d to DP are zeros
+template <int T, int DP, int PAD>
 __device__ __forceinline__ void load_tile(float* tile, const float* src, int stride, int first, int n, int d) {
-    constexpr int QP = DP + 4;
+    constexpr int QP = DP + PAD;
     for (int i = threadIdx.x; i < T * (DP / 4); i += kThreads) {
         const int t = i / (DP / 4), c = (i - t * (DP / 4)) * 4;
         const bool in = t < n && c < d;
@@ -595,21 +595,51 @@ __device__ __forceinline__ void load_tile(float* tile, const float* src, int str
     }
 }
 
-// acc[a][b] += rows (ty * M + a) of x . rows (tx * M + b) of y, over DP columns
-template <int DP, int M>
-__device__ __forceinline__ void row_products(const float* x, const float* y, int ty, int tx, float (*acc)[M]) {
-    constexpr int QP = DP + 4;
-#pragma unroll 4
-    for (int k = 0; k < DP; k += 4) {
-        float4 yv[M];
+// Products of 64 rows x[i] (MT matrices) with 64 rows y over DP columns, rows DP + 8 floats apart, where the row of y is not after the
+// row of x: eight warps share out the tiles of 16 x 8 on and below the diagonal, ten to each scheduler's two.  use(acc, r0, n0,
+// first zero column): acc[i][n] holds (row r0, columns n0 + 8 n and the one after it), then the same of row r0 + 8.  Multiply-adds on
+// 4 x 4 outputs a thread were bound by their reads from shared memory.
+template <int DP, int MT, int NT, typename Use>
+__device__ __forceinline__ void triangle_tiles(const float* const (&x)[MT], const float* y, int block, int half, int lane, Use use) {
+    constexpr int QP = DP + 8;
+    const int lr = lane >> 2, lc = lane & 3, r0 = block * 16 + lr, n0 = half * NT * 8;
+    const float* yr = y + (n0 + lr) * QP + 2 * lc;
+    float acc[MT][NT][4] = {};
+    split::products<MT, NT, 2>(acc, DP / 8,
+        [&](int i, int s, float (&v)[4]) {
+            const float* at = x[i] + r0 * QP + 2 * lc + 8 * s;
+            const float2 top = *reinterpret_cast<const float2*>(at), low = *reinterpret_cast<const float2*>(at + 8 * QP);
+            v[0] = top.x; v[1] = low.x; v[2] = top.y; v[3] = low.y;
+        },
+        [&](int n, int s, float (&v)[2]) {
+            const float2 w = *reinterpret_cast<const float2*>(yr + 8 * n * QP + 8 * s);
+            v[0] = w.x; v[1] = w.y;
+        });
+    if (split::odd(acc))
 #pragma unroll
-        for (int b = 0; b < M; ++b) yv[b] = ld4(y + (tx + 16 * b) * QP + k);
+        for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int i = 0; i < M; ++i) {
-            const float4 xv = ld4(x + (ty + 16 * i) * QP + k);
+            for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int b = 0; b < M; ++b) acc[i][b] = fma4(xv, yv[b], acc[i][b]);
-        }
+                for (int j = 0; j < 4; ++j) {
+                    if (isfinite(acc[i][n][j])) continue;
+                    const float* row = x[i] + (r0 + (j >> 1) * 8) * QP;
+                    const float* other = y + (n0 + 8 * n + 2 * lc + (j & 1)) * QP;
+                    float sum = 0.f;
+#pragma unroll 1
+                    for (int k = 0; k < DP; ++k) sum = fmaf(row[k], other[k], sum);
+                    acc[i][n][j] = sum;
+                }
+    use(acc, r0, n0 + 2 * lc, (block + 1) * 16 + half * 8 + 2 * lc);
+}
+template <int DP, int MT, typename Use>
+__device__ __forceinline__ void triangle_products(const float* const (&x)[MT], const float* y, int warp, int lane, Use use) {
+    const int half = warp & 1;
+    switch (warp >> 1) {
+        case 0: triangle_tiles<DP, MT, 4>(x, y, 3, half, lane, use); break;
+        case 1: triangle_tiles<DP, MT, 3>(x, y, 2, half, lane, use); break;
+        case 2: triangle_tiles<DP, MT, 1>(x, y, 0, half, lane, use); break;
+        default: triangle_tiles<DP, MT, 2>(x, y, 1, half, lane, use);
     }
 }
 

@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 3)
 retention_prepare_kernel(const RetentionInputs<T_> in, const float* __restrict__ decay, const int* __restrict__ cu_q, int entries,
                          float* __restrict__ q, float* __restrict__ k, float* __restrict__ p, float* __restrict__ rs,
                          float* __restrict__ ts, int H, int d) {
-    constexpr int T = 64, QP = DP + 4;
+    constexpr int T = 64, QP = DP + 8;
     extern __shared__ __align__(16) float sm[];
     float* qs = sm;
     float* ks = qs + T * QP;
@@ -532,19 +532,22 @@ retention_prepare_kernel(const RetentionInputs<T_> in, const float* __restrict__
         rs[(size_t)(first + threadIdx.x) * H + h] = power[threadIdx.x + 1];
         ts[(size_t)(first + threadIdx.x) * H + h] = power[n - 1 - threadIdx.x];
     }
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    float acc[4][4] = {};
-    row_products<DP, 4>(qs, ks, ty, tx, acc);
+    const float* const x[1] = {qs};
+    triangle_products<DP, 1>(x, ks, threadIdx.x >> 5, threadIdx.x & 31, [&](const auto& acc, int r0, int n0, int zeros) {
+        constexpr int NT = sizeof(acc[0]) / sizeof(acc[0][0]);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t = ty + 16 * i;
-        if (t >= n) continue;
+        for (int j = 0; j < 4; j += 2) {
+            const int t = r0 + 4 * j;
+            if (t >= n) continue;
+            float* row = p + ((size_t)(first + t) * H + h) * T;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int s = tx + 16 * b;
-            p[((size_t)(first + t) * H + h) * T + s] = s <= t ? acc[i][b] * power[t - s] : 0.f;
+            for (int x = 0; x < NT; ++x) {
+                const int s = n0 + 8 * x;
+                *reinterpret_cast<float2*>(row + s) = make_float2(s <= t ? acc[0][x][j] * power[t - s] : 0.f, s < t ? acc[0][x][j + 1] * power[t - s - 1] : 0.f);
+            }
+            for (int s = zeros; s < T; s += 16) *reinterpret_cast<float2*>(row + s) = make_float2(0.f, 0.f);
         }
-    }
+    });
 }
 
 }  // namespace walk
@@ -745,7 +748,7 @@ static int launch_retention_walk(const void* proj, int proj_stride, int q_off, i
         in.positions = positions; in.rotary = rotary; in.silu = silu; in.k_scale = k_scale;
         a.v = in.proj + v_off;
         SE_WALK_DIMS(d, {
-            const int rc = launch(retention_prepare_kernel<DP, T_>, grid, 2 * 64 * (DP + 4) * sizeof(float), stream, in, decay, cu_q,
+            const int rc = launch(retention_prepare_kernel<DP, T_>, grid, 2 * 64 * (DP + 8) * sizeof(float), stream, in, decay, cu_q,
                                   entries, q, k, p, rs, ts, heads, d);
             if (rc != 0) return rc;
             return launch_walk<64, DP, false, false, T_>(a, entries, cols, stream);
