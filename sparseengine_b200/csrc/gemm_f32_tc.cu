@@ -4,7 +4,7 @@
 // stay 32-bit in memory and are split on their way: TMA brings 128 weight rows (the M side) and up to 128 activation rows (the N side),
 // 32 values along K each; other warps cut the weights into hi, the nearest tf32 value, and the rest and put both into tensor memory,
 // from where they are the A operand, and put the activations' rest beside them in shared memory (their hi needs no copy: the
-// tensor cores read the upper 19 bits).  Activations split by a kernel ahead took as long (2,048 rows by 8,192 x 3,072 weights: 513 us, 520 so;
+// tensor cores read the upper 19 bits).  Activations split by a kernel ahead took as long (2,048 rows by 8,192 x 3,072 weights: 513 us, 520 so then;
 // the library 1,810) and a workspace of twice their size.
 //
 // The tensor cores cut sums off instead of rounding them, which a long sum shows: 2.5e-7 of the result per 32 products.  So hi hi
@@ -25,6 +25,7 @@
 #include <cuda.h>
 
 #include <mutex>
+#include <type_traits>
 
 namespace se {
 namespace f32tc {
@@ -189,30 +190,58 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             ok = __all_sync(0xffffffffu, mbar_wait(bar(b), parity, &abort_s));
             return ok;
         };
+        auto wait_step = [&](int it, int kb, int chunk) {
+            if (kb % kChunk == 0 && chunk >= 2) wait(&bars.sum_empty[chunk & 1], ((chunk >> 1) - 1) & 1);
+            if (ok) wait(&bars.split_full[it & 1], (it >> 1) & 1);          // who arrives there has seen the copies land
+        };
         for (int i = blockIdx.x; i < last && ok; i += gridDim.x, ++done) {
-            const uint32_t id = instr(max(16, (fa::uniform(item_of<MODE>(p, i, tiles).valid) + 15) & ~15));
+            const int valid = fa::uniform(item_of<MODE>(p, i, tiles).valid);
+            const uint32_t id = instr(max(16, (valid + 15) & ~15));
+            // With more than 64 activation rows the waits of a step come between the two halves of the products of the step before it, which
+            // run meanwhile (the tensor cores hold some five products ahead, less than the waits take).  Few rows make short
+            // products, whose buffers are better freed early, and so are those of the experts' first product, whose weights come from
+            // memory.  2,048 rows by 8,192 x 3,072 weights 511 -> 479 us; experts of 105 rows, first product 3,682 (3,760 so), second 1,811 -> 1,780.
+            const bool apart = MODE != GATE_UP && valid > 64;
             if (done > 0) wait(&bars.low_empty, (done - 1) & 1);
+            if (ok) wait_step(it, 0, chunk);
             for (int kb = 0; kb < num_kb && ok; ++kb, ++it) {
                 const int s = it % kStages, x = it & 1, b = chunk & 1;
                 const bool first = kb % kChunk == 0, ends = kb % kChunk == kChunk - 1 || kb == num_kb - 1;
-                if (first && chunk >= 2) wait(&bars.sum_empty[b], ((chunk >> 1) - 1) & 1);
-                if (ok) wait(&bars.split_full[x], (it >> 1) & 1);          // who arrives there has seen the copies land
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t at = smem_addr(smem) + s * kStageBytes, wh = tm + kSplit + x * 2 * kK, wl = wh + kK, to = tm + b * kN;
                 const uint64_t bh = fa::desc_kmajor(at + kTile), bl = fa::desc_kmajor(at + 2 * kTile);
-                if (ok && fa::elect_one()) {
+                auto half = [&](int k0) {
 #pragma unroll
-                    for (int k = 0; k < kK / 8; ++k) {           // steps of 8: 32 bytes along K, 8 columns of A
+                    for (int k = k0; k < k0 + kK / 16; ++k) {    // steps of 8: 32 bytes along K, 8 columns of A
                         multiply(to, wh + 8 * k, bh + 2 * k, id, !first || k != 0);
                         multiply(tm + kLow, wl + 8 * k, bh + 2 * k, id, kb != 0 || k != 0);
                         multiply(tm + kLow, wh + 8 * k, bl + 2 * k, id, 1);
                     }
+                };
+                auto free = [&]() {
                     fa::umma_commit(bar(&bars.empty[s]));
                     fa::umma_commit(bar(&bars.split_empty[x]));
                     if (ends) fa::umma_commit(bar(&bars.sum_full[b]));
-                }
-                __syncwarp();
+                };
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 chunk += ends;
+                if (apart) {
+                    if (fa::elect_one()) half(0);
+                    __syncwarp();
+                    if (kb + 1 < num_kb) wait_step(it + 1, kb + 1, chunk);
+                    if (fa::elect_one()) {                       // also after a failed wait: what waits for this step ends
+                        half(kK / 16);
+                        free();
+                    }
+                    __syncwarp();
+                } else {
+                    if (fa::elect_one()) {
+                        half(0);
+                        half(kK / 16);
+                        free();
+                    }
+                    __syncwarp();
+                    if (kb + 1 < num_kb) wait_step(it + 1, kb + 1, chunk);
+                }
             }
         }
         if (!ok && lane == 0) { abort_s = 1; atomicCAS(p.error, 0, kErrorCode); }
@@ -343,23 +372,45 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
                 for (int c = 0; c < kN / 2; ++c) put[c * 64] = up ? sum[c] : sum[kN / 2 + c];
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (n < p.n_out) {
+                // Eight rows at a time, every value computed and only the stores guarded: row by row behind a branch, an item's epilogue took
+                // 35,000 cycles of its 145,000, and the products wait for it once both sums are full.
+                const int rows = t.valid - (up ? kN / 2 : 0);        // of this thread's half
+                float* o = p.out + (size_t)(t.row0 + (up ? kN / 2 : 0)) * p.n_out + n;
+                auto store = [&](auto kind) {
 #pragma unroll
-                    for (int c = 0; c < kN / 2; ++c) {
-                        const int row = up ? kN / 2 + c : c;
-                        if (row >= t.valid) continue;
-                        const float own = up ? sum[kN / 2 + c] : sum[c], other = get[c * 64];
-                        p.out[(size_t)(t.row0 + row) * p.n_out + n] =
-                            glu_value<float>(up ? other : own, up ? own : other, p.act_kind, p.act_limit, p.act_alpha);
+                    for (int c0 = 0; c0 < kN / 2; c0 += 8) {
+                        if (c0 >= rows) break;
+                        float v[8];
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            const float own = up ? sum[kN / 2 + c0 + c] : sum[c0 + c], other = get[(c0 + c) * 64];
+                            v[c] = glu_value<float>(up ? other : own, up ? own : other, decltype(kind)::value, p.act_limit, p.act_alpha);
+                        }
+#pragma unroll
+                        for (int c = 0; c < 8; ++c)
+                            if (c0 + c < rows && n < p.n_out) o[(size_t)(c0 + c) * p.n_out] = v[c];
                     }
-                }
+                };
+                if (p.act_kind == SE_GLU_SILU) store(std::integral_constant<int, SE_GLU_SILU>{});
+                else if (p.act_kind == SE_GLU_CLAMPED) store(std::integral_constant<int, SE_GLU_CLAMPED>{});
+                else store(std::integral_constant<int, SE_GLU_GELU>{});
             } else {
                 const int n = t.n0 + quarter * 32 + lane;
-                if (n < p.n_out) {
-                    float* o = p.out + (size_t)t.row0 * p.n_out + n;
+                float* o = p.out + (size_t)t.row0 * p.n_out + n;
 #pragma unroll
-                    for (int c = 0; c < kN; ++c)
-                        if (c < t.valid) o[(size_t)c * p.n_out] = MODE == DOWN ? sum[c] * route_s[done & 1][c] : sum[c];
+                for (int c0 = 0; c0 < kN; c0 += 8) {
+                    if (c0 >= t.valid) break;
+                    if (MODE == DOWN)
+#pragma unroll
+                        for (int c = c0; c < c0 + 8; ++c) sum[c] *= route_s[done & 1][c];
+                    if (c0 + 8 <= t.valid && t.n0 + kM <= p.n_out) {
+#pragma unroll
+                        for (int c = c0; c < c0 + 8; ++c) o[(size_t)c * p.n_out] = sum[c];
+                    } else {
+#pragma unroll
+                        for (int c = c0; c < c0 + 8; ++c)
+                            if (c < t.valid && n < p.n_out) o[(size_t)c * p.n_out] = sum[c];
+                    }
                 }
             }
         }

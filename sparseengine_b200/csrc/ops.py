@@ -1261,16 +1261,16 @@ F32_TC_MIN_INNER = 512
 
 def gemm_f32_dense_pays(rows: int, n_out: int, k_dim: int, sms: int) -> bool:
     """Whether a dense product in tf32 terms is estimated to take less than the library's 32-bit one.  A step of 32 along K takes
-    a block of 128 x 128 outputs 0.5 us with few rows and 0.76 with 128, whatever the other blocks do.  The library's reaches 50
+    a block of 128 x 128 outputs 0.5 us with few rows and 0.71 with 128, whatever the other blocks do.  The library's reaches 50
     TFLOP/s over rows rounded up to 64 at best, and needs 26 ns per term of a sum where it does not split sums (15 with few rows, or
-    too few tiles to go without).  Measured, us, library / this (rows x outputs x inner): 2,048 x 8,192 x 3,072 1,810 / 519;
-    128 x 10,304 x 2,048 147 / 56; 128 x 3,072 x 6,144 179 / 147; 512 x 2,048 x 2,048 86 / 56, 128 rows 40 / 54; 4,096 x 192 x 2,048 86 / 56,
-    1,024 rows 40 / 54; 8 x 8,192 x 3,072 60 / 53.  The very few rows that the library gives to its kernels with split sums (up to
+    too few tiles to go without).  Measured, us, library / this (rows x outputs x inner): 2,048 x 8,192 x 3,072 1,810 / 479;
+    128 x 10,304 x 2,048 147 / 52; 128 x 3,072 x 6,144 179 / 135; 512 x 2,048 x 2,048 86 / 51, 128 rows 40 / 50; 4,096 x 192 x 2,048 86 / 51,
+    1,024 rows 40 / 50; 8 x 8,192 x 3,072 60 / 53.  The very few rows that the library gives to its kernels with split sums (up to
     7, up to 3 with an inner dimension from 3,072 on) stay there: those sums are the more exact ones (1.2e-7 to 2.5e-7)."""
     if k_dim < F32_TC_MIN_INNER or rows < (4 if k_dim >= 3072 else 8):
         return False
     waves = -(-(-(-rows // 128) * -(-n_out // 128)) // sms)
-    ours = 3.0 + waves * -(-k_dim // 32) * (0.5 + 0.26 * min(rows, 128) / 128)
+    ours = 3.0 + waves * -(-k_dim // 32) * (0.5 + 0.21 * min(rows, 128) / 128)
     per_term = 0.0 if rows <= 16 else 0.026 if rows > 32 and -(-rows // 128) * -(-n_out // 64) >= 48 else 0.0145
     return ours < max(2.0 * (-(-rows // 64) * 64) * n_out * k_dim / 50e6, per_term * k_dim)
 
