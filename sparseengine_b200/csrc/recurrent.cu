@@ -998,6 +998,42 @@ __global__ void gated_group_norm4_kernel(const float* __restrict__ y, const T* p
     }
 }
 
+// The same with a warp per (token, part), for parts of up to 512 columns: no barriers, whose waits took a fifth of the time (2,048
+// tokens of 8 parts of 512: 23 and 17.5 us).
+template <typename T>
+__global__ void __launch_bounds__(256)
+gated_group_norm_warp_kernel(const float* __restrict__ y, const T* proj, int pitch, int z_off, const float* __restrict__ w,
+                             T* __restrict__ out, int inner, int parts, int rows, float eps) {
+    const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= rows) return;
+    const int t = r / parts, n = inner / parts, base = (r - t * parts) * n;
+    const float* yr = y + (size_t)t * inner + base;
+    const T* zr = proj + (size_t)t * pitch + z_off + base;
+    constexpr int kQuads = 4;
+    float4 v[kQuads], z[kQuads];
+#pragma unroll
+    for (int k = 0; k < kQuads; ++k) {
+        const int i = (k * 32 + lane) * 4;
+        v[k] = i < n ? four(yr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        z[k] = i < n ? four(zr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < kQuads; ++k) {
+        v[k] = make_float4(v[k].x * silu_f(z[k].x), v[k].y * silu_f(z[k].y), v[k].z * silu_f(z[k].z), v[k].w * silu_f(z[k].w));
+        ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
+    }
+    const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)n + eps);
+#pragma unroll
+    for (int k = 0; k < kQuads; ++k) {
+        const int i = (k * 32 + lane) * 4;
+        if (i < n) {
+            const float4 wv = four(w + base + i);
+            put_four(out + (size_t)t * inner + base + i, make_float4(v[k].x * inv * wv.x, v[k].y * inv * wv.y, v[k].z * inv * wv.z, v[k].w * inv * wv.w));
+        }
+    }
+}
+
 // rows of the key/state side a recurrence kernel takes (32 registers x 16 lanes)
 constexpr int kMaxStateRows = 512;
 
@@ -1209,7 +1245,14 @@ extern "C" int se_gated_group_norm(const float* y, const void* proj, int pitch, 
     const int n = inner / parts, keep = n * (int)sizeof(float) <= 40 * 1024;
     if (n % 4 == 0 && n <= 4096 && pitch % 4 == 0 && z_off % 4 == 0 &&
         ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
-        const int block = n <= 128 ? 32 : n <= 256 ? 64 : n <= 1024 ? 128 : 256;
+        const long long rows = (long long)tokens * parts;
+        if (n <= 512 && rows <= 0x7fffffffLL) {
+            SE_DISPATCH_DTYPE(dtype, T,
+                se::gated_group_norm_warp_kernel<T><<<(int)((rows + 7) / 8), 256, 0, stream>>>(y, (const T*)proj, pitch, z_off, w, (T*)out, inner,
+                                                                                             parts, (int)rows, eps));
+            SE_LAUNCH_CHECK();
+        }
+        const int block = n <= 1024 ? 128 : 256;
         SE_DISPATCH_DTYPE(dtype, T,
             se::gated_group_norm4_kernel<T><<<dim3(tokens, parts), block, 0, stream>>>(y, (const T*)proj, pitch, z_off, w, (T*)out, inner,
                                                                                      parts, eps));
