@@ -523,7 +523,7 @@ extern "C" int se_ssm_walk(const float* xbc, const void* proj, int pitch, int dt
         a.v = xbc; a.v_stride = a.qk_stride; a.v_scale = steps; a.skip = d_skip;
         a.p = p; a.rs = rs; a.ts = ts; a.eb = rs; a.state = state; a.state_stride = state_stride; a.s_row = 1; a.s_col = N; a.o = y;
         a.cu_q = cu_q; a.seq_rows = seq_rows; a.H = H; a.d = N; a.dv = P;
-        return launch_walk<64, DP, false, false, float>(a, entries, walk_columns(entries, H, P, sms), stream);
+        return launch_walk<64, DP, false, false, false, false, float>(a, entries, walk_columns(entries, H, P, sms), stream);
     });
 }
 
@@ -561,7 +561,7 @@ extern "C" int se_delta_walk(const float* qkv, const void* in_a, int a_pitch, co
                                       (64 * (DP + 8) + 64 * 68 + tile) * sizeof(float), stream, in, p, w, u, rs, ts, eb);
                 if (rc != 0) return rc;
                 a.q = qkv; a.k = qkv + G * d; a.qk_stride = 2 * G * d + H * dv; a.rep = H / G; a.p = p; a.rs = rs; a.ts = ts; a.eb = eb;
-                return launch_walk<64, DP, true, false, float>(a, entries, cols, stream);
+                return launch_walk<64, DP, true, false, false, false, float>(a, entries, cols, stream);
             }
             float* qt = u + rows * dv;
             float* kt = qt + rows * d;
@@ -571,7 +571,7 @@ extern "C" int se_delta_walk(const float* qkv, const void* in_a, int a_pitch, co
                                   (3 * 32 * (DP + 4) + 2 * 32 * 36 + 2 * DP) * sizeof(float), stream, in, p, w, u, qt, kt, tot);
             if (rc != 0) return rc;
             a.q = qt; a.k = kt; a.qk_stride = H * d; a.rep = 1; a.p = p; a.tot = tot;
-            return launch_walk<32, DP, true, true, float>(a, entries, cols, stream);
+            return launch_walk<32, DP, true, true, true, false, float>(a, entries, cols, stream);
         });
     });
 }

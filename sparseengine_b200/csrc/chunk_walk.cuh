@@ -15,7 +15,7 @@
 // What bounds the walk is arithmetic (3 to 5 multiply-adds per state element and token) along a chain of chunks; 16-bit operands would
 // lose what the recurrence has to keep.  With multiply-adds it stood at half their rate, its other half shared-memory reads (8 x 8 outputs
 // a thread, an LDS.128 each four multiply-adds); products in tf32 terms by mma.sync read less.  Measured, multiply-adds / now: state space,
-// 2,048 tokens of 64 heads of 64 columns, 204 / 150 us; retention, 8,192 tokens of 32 heads of 128, 752 / 541; delta rule per channel, 4,670 tokens of
+// 2,048 tokens of 64 heads of 64 columns, 204 / 150 us; retention, 8,192 tokens of 32 heads of 128, 752 / 456; delta rule per channel, 4,670 tokens of
 // 16 heads of 128, 418 / 333; per head, 2,048 tokens, 176 / 123.  Sixteen warps at the products instead of eight, all loading for themselves: 168, 616, -, 148 (eight: 152, 563, 333, 134).  Every exponent is a
 // difference of sums of logarithms that is at most 0 up to the 64-bit sums' rounding
 // (no token's logarithm lies below -1e4) or, for decays per channel, a product of decays of at most T tokens: no term overflows.
@@ -86,7 +86,7 @@ struct WalkArgs {
     const float* skip;             // per head: o_t += skip * (unscaled) value row, or null
     const float* p;                // [tokens][H][T]
     const float* rs;               // [tokens][H]: factor on q's products with S_0, e^(B_t) (decays per head)
-    const float* ts;               // [tokens][H]: factor on u where k takes it into the state, e^(B_n - B_t)
+    const float* ts;               // [tokens][H]: factor on u where k takes it into the state, e^(B_n - B_t); not where k comes scaled
     const float* eb;               // [tokens][H]: e^(B_t)
     const float* tot;              // [places][H][d]: e^(B_n)       (decays per channel: q and k come scaled)
     float* state;
@@ -107,7 +107,7 @@ struct WalkArgs {
 // warps that read them, as soon as they have read the last chunk's.  Row pitches are such that no fragment read
 // meets a bank twice: 8 more than a multiple of 32 where rows lie along k (two neighbours per lane), 4 more than a
 // multiple of 16 where columns do.
-template <int T, int DP, int C, bool SOLVE, bool CHANNEL>
+template <int T, int DP, int C, bool SOLVE, bool SCALED>
 struct WalkShape {
     static constexpr int kQP = DP + 8, kKP = DP + 4, kPP = T + 8, kCP = C + 4;
     static constexpr int kBuffers = SOLVE ? 1 : 2;                    // of k, u and the state
@@ -115,14 +115,16 @@ struct WalkShape {
     static constexpr int kThreads = kLoader ? 384 : 256;
     static constexpr int kAhead = kLoader ? 2 : 1;                    // buffers of q and W
     static constexpr int kFloats = (SOLVE ? 2 : 1) * kAhead * T * kQP + kBuffers * T * kKP + T * kPP +
-                                   kBuffers * (CHANNEL ? 1 : 2) * T * kCP + kBuffers * DP * kCP + 2 * T;
+                                   kBuffers * (SCALED ? 1 : 2) * T * kCP + kBuffers * DP * kCP + 2 * T;
     static constexpr int kBlocks = kFloats * 4 <= 112 * 1024 ? 2 : 1;            // per SM
 };
 
-template <int T, int DP, int C, bool SOLVE, bool CHANNEL, typename TV>
-__global__ void __launch_bounds__(WalkShape<T, DP, C, SOLVE, CHANNEL>::kThreads, WalkShape<T, DP, C, SOLVE, CHANNEL>::kBlocks)
+// CHANNEL: a decay per key channel; SCALED: k comes as e^(B_n - B_t) k; EXACT: the value rows are 16-bit numbers and nothing else, so
+// that products with them need two terms (retention of 8,192 tokens of 32 heads: 541 and 456 us).
+template <int T, int DP, int C, bool SOLVE, bool CHANNEL, bool SCALED, bool EXACT, typename TV>
+__global__ void __launch_bounds__(WalkShape<T, DP, C, SOLVE, SCALED>::kThreads, WalkShape<T, DP, C, SOLVE, SCALED>::kBlocks)
 chunk_walk_kernel(const WalkArgs a) {
-    using Shape = WalkShape<T, DP, C, SOLVE, CHANNEL>;
+    using Shape = WalkShape<T, DP, C, SOLVE, SCALED>;
     constexpr int QP = Shape::kQP, KP = Shape::kKP, PP = Shape::kPP, CP = Shape::kCP, NB = Shape::kBuffers;
     constexpr int QB = Shape::kAhead * T * QP, kThreads = Shape::kThreads;
     constexpr bool LOADER = Shape::kLoader;
@@ -136,7 +138,7 @@ chunk_walk_kernel(const WalkArgs a) {
     float* ks = ws + (SOLVE ? QB : 0);               // [NB][T][KP]
     float* ps = ks + NB * T * KP;                    // [T][PP]
     float* us = ps + T * PP;                         // [NB][T][CP]: u
-    float* u2 = CHANNEL ? us : us + NB * T * CP;     // [NB][T][CP]: e^(B_n - B_t) u (decays per head)
+    float* u2 = SCALED ? us : us + NB * T * CP;      // [NB][T][CP]: e^(B_n - B_t) u, where k does not come with that factor
     float* Ss = u2 + NB * T * CP;                    // [NB][DP][CP]
     float* rss = Ss + NB * DP * CP;                  // [2][T]
     const int e = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * C;
@@ -217,7 +219,7 @@ chunk_walk_kernel(const WalkArgs a) {
             for (int n = 0; n < NT; ++n)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) to[0][n][j] = 0.f;
-            split::products<1, NT, 2>(to, 2 * (gw % WR) + 2,
+            split::products<1, NT, 2, EXACT>(to, 2 * (gw % WR) + 2,
                 [&](int, int s, float (&v)[4]) {
                     const float2 top = *reinterpret_cast<const float2*>(pr + 8 * s), low = *reinterpret_cast<const float2*>(pr + 8 * PP + 8 * s);
                     v[0] = top.x; v[1] = low.x; v[2] = top.y; v[3] = low.y;
@@ -272,7 +274,7 @@ chunk_walk_kernel(const WalkArgs a) {
         float sum[MT][NS][4] = {};
         const float* kr = k + 2 * lc * KP + m0 + lr;
         const float* ur = u + 2 * lc * CP + lr;
-        split::products<MT, NS, 2>(sum, T / 8,
+        split::products<MT, NS, 2, EXACT>(sum, T / 8,
             [&](int i, int s, float (&v)[4]) {
                 const float* at = kr + 8 * s * KP + 16 * i;
                 v[0] = at[0]; v[1] = at[8]; v[2] = at[KP]; v[3] = at[KP + 8];
@@ -328,7 +330,7 @@ chunk_walk_kernel(const WalkArgs a) {
                 const size_t at = (size_t)(t0 + t) * a.H + h;
                 vreg[x] = in ? load4(vb + (size_t)(t0 + t) * a.v_stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
                 vfac[x] = in && a.v_scale != nullptr ? a.v_scale[at] : 1.f;
-                tfac[x] = in ? a.ts[at] : 1.f;
+                tfac[x] = !SCALED && in ? a.ts[at] : 1.f;
             }
             if (gt < T) rfac = gt < n ? a.rs[(size_t)(t0 + gt) * a.H + h] : 0.f;
         };
@@ -340,7 +342,7 @@ chunk_walk_kernel(const WalkArgs a) {
                 if (a.silu) v = make_float4(value_silu<TV>(v.x), value_silu<TV>(v.y), value_silu<TV>(v.z), value_silu<TV>(v.w));
                 v = make_float4(v.x * vfac[x], v.y * vfac[x], v.z * vfac[x], v.w * vfac[x]);
                 st4(us + at, v);
-                st4(u2 + at, make_float4(v.x * tfac[x], v.y * tfac[x], v.z * tfac[x], v.w * tfac[x]));
+                if (!SCALED) st4(u2 + at, make_float4(v.x * tfac[x], v.y * tfac[x], v.z * tfac[x], v.w * tfac[x]));
             }
             if (gt < T) rss[buffer * T + gt] = rfac;
         };
@@ -494,7 +496,7 @@ chunk_walk_kernel(const WalkArgs a) {
         cp_commit();
         if (group == 0) {
             load_u(t_first, first_n);
-            load_factors(a.ts, t_first, first_n);
+            if (!SCALED) load_factors(a.ts, t_first, first_n);
             load_totals(t_first, first_n);
         } else if (group == 1) {
             load_factors(a.rs, t_first, first_n);
@@ -537,7 +539,7 @@ chunk_walk_kernel(const WalkArgs a) {
                         const float2 u = make_float2(ureg[x][j] - acc[0][x][j], ureg[x][j + 1] - acc[0][x][j + 1]);
                         const int at = (r0 + 4 * j) * CP + col0 + 8 * x + 2 * lc;
                         *reinterpret_cast<float2*>(us + at) = u;
-                        if (!CHANNEL) *reinterpret_cast<float2*>(u2 + at) = make_float2(u.x * fac[j >> 1], u.y * fac[j >> 1]);
+                        if (!SCALED) *reinterpret_cast<float2*>(u2 + at) = make_float2(u.x * fac[j >> 1], u.y * fac[j >> 1]);
                     }
             }
             cp_wait<0>();
@@ -546,7 +548,7 @@ chunk_walk_kernel(const WalkArgs a) {
                 if (next < t_last) {
                     if (!LOADER) load_w(next, next_n);
                     load_u(next, next_n);
-                    load_factors(a.ts, next, next_n);
+                    if (!SCALED) load_factors(a.ts, next, next_n);
                 }
                 cp_commit();
                 update_state(ks, u2, totals);
@@ -655,16 +657,16 @@ template <typename... KArgs, typename... Args>
 int launch(void (*kernel)(KArgs...), dim3 grid, size_t smem, cudaStream_t stream, Args... args) {
     return launch_threads(kernel, grid, kThreads, smem, stream, args...);
 }
-template <int T, int DP, int C, bool SOLVE, bool CHANNEL, typename TV>
+template <int T, int DP, int C, bool SOLVE, bool CHANNEL, bool SCALED, bool EXACT, typename TV>
 int launch_walk_columns(const WalkArgs& a, int entries, cudaStream_t stream) {
-    using Shape = WalkShape<T, DP, C, SOLVE, CHANNEL>;
-    return launch_threads(chunk_walk_kernel<T, DP, C, SOLVE, CHANNEL, TV>, dim3(entries, a.H, ceil_div(a.dv, C)), Shape::kThreads,
+    using Shape = WalkShape<T, DP, C, SOLVE, SCALED>;
+    return launch_threads(chunk_walk_kernel<T, DP, C, SOLVE, CHANNEL, SCALED, EXACT, TV>, dim3(entries, a.H, ceil_div(a.dv, C)), Shape::kThreads,
                           Shape::kFloats * sizeof(float), stream, a);
 }
-template <int T, int DP, bool SOLVE, bool CHANNEL, typename TV>
+template <int T, int DP, bool SOLVE, bool CHANNEL, bool SCALED, bool EXACT, typename TV>
 int launch_walk(const WalkArgs& a, int entries, int cols, cudaStream_t stream) {
-    if (cols == 16) return launch_walk_columns<T, DP, 16, SOLVE, CHANNEL, TV>(a, entries, stream);
-    return launch_walk_columns<T, DP, 32, SOLVE, CHANNEL, TV>(a, entries, stream);
+    if (cols == 16) return launch_walk_columns<T, DP, 16, SOLVE, CHANNEL, SCALED, EXACT, TV>(a, entries, stream);
+    return launch_walk_columns<T, DP, 32, SOLVE, CHANNEL, SCALED, EXACT, TV>(a, entries, stream);
 }
 
 // Value columns per block: 32 while the blocks then fill the device, 16 (twice the blocks, which each read q and k) else.

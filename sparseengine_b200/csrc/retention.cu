@@ -460,15 +460,14 @@ __device__ __forceinline__ float4 staged4(const T_* src, int silu) {
     return v;
 }
 
-// Retention: P[t][s] = decay^(t - s) q_t . k_s, rs = decay^(t + 1), ts = decay^(n - 1 - t); q and k as the walk reads them.
+// Retention: P[t][s] = decay^(t - s) q_t . k_s, rs = decay^(t + 1); q and k as the walk reads them, k times decay^(n - 1 - t).
 // The rotation happens on the way into shared memory: a (chunk, head) works its angles out itself (a sine and a cosine for 128
 // multiply-adds).  Measured, 8,192 tokens of 32 heads of 128: rotated by a kernel of its own first,
-// 69 + 134 us; here 178, and a launch less (2,048 wide, 17 to 64 tokens: a layer's call 92 and 76 us).
+// 69 + 134 us; here 178 (165 with the products in tf32 terms), and a launch less (2,048 wide, 17 to 64 tokens: a layer's call 92 and 76 us).
 template <int DP, typename T_>
 __global__ void __launch_bounds__(kThreads, 3)
 retention_prepare_kernel(const RetentionInputs<T_> in, const float* __restrict__ decay, const int* __restrict__ cu_q, int entries,
-                         float* __restrict__ q, float* __restrict__ k, float* __restrict__ p, float* __restrict__ rs,
-                         float* __restrict__ ts, int H, int d) {
+                         float* __restrict__ q, float* __restrict__ k, float* __restrict__ p, float* __restrict__ rs, int H, int d) {
     constexpr int T = 64, QP = DP + 8;
     extern __shared__ __align__(16) float sm[];
     float* qs = sm;
@@ -478,12 +477,16 @@ retention_prepare_kernel(const RetentionInputs<T_> in, const float* __restrict__
     chunk_of<T>(blockIdx.x, cu_q, entries, first, n);
     if (n <= 0) return;
     const int h = blockIdx.y, half = in.rotary / 2, pairs = half / 4, per = pairs + (d - in.rotary) / 4;
+    const double g = (double)decay[h];
+    if (threadIdx.x <= T) power[threadIdx.x] = (float)pow(g, (double)threadIdx.x);
+    __syncthreads();
     for (int x = threadIdx.x; x < T * per; x += kThreads) {
         const int t = x / per, c = x - t * per, i = c < pairs ? c * 4 : in.rotary + (c - pairs) * 4;
         float4 q0 = {}, q1 = {}, k0 = {}, k1 = {};
         if (t < n) {
             const T_* row = in.proj + (size_t)(first + t) * in.pitch + (size_t)h * d + i;
             const size_t at = ((size_t)(first + t) * H + h) * d + i;
+            const float left = power[n - 1 - t];
             q0 = staged4(row + in.q_off, in.silu);
             k0 = staged4(row + in.k_off, in.silu);
             if (c < pairs) {
@@ -506,11 +509,11 @@ retention_prepare_kernel(const RetentionInputs<T_> in, const float* __restrict__
                 turn(f.w, q0.w, q1.w, k0.w, k1.w);
                 k1 = make_float4(k1.x * in.k_scale, k1.y * in.k_scale, k1.z * in.k_scale, k1.w * in.k_scale);
                 st4(q + at + half, q1);
-                st4(k + at + half, k1);
+                st4(k + at + half, make_float4(k1.x * left, k1.y * left, k1.z * left, k1.w * left));
             }
             k0 = make_float4(k0.x * in.k_scale, k0.y * in.k_scale, k0.z * in.k_scale, k0.w * in.k_scale);
             st4(q + at, q0);
-            st4(k + at, k0);
+            st4(k + at, make_float4(k0.x * left, k0.y * left, k0.z * left, k0.w * left));
         }
         st4(qs + t * QP + i, q0);
         st4(ks + t * QP + i, k0);
@@ -525,12 +528,9 @@ retention_prepare_kernel(const RetentionInputs<T_> in, const float* __restrict__
             st4(qs + t * QP + c, make_float4(0.f, 0.f, 0.f, 0.f));
             st4(ks + t * QP + c, make_float4(0.f, 0.f, 0.f, 0.f));
         }
-    const double g = (double)decay[h];
-    if (threadIdx.x <= T) power[threadIdx.x] = (float)pow(g, (double)threadIdx.x);
     __syncthreads();
     if (threadIdx.x < n) {
         rs[(size_t)(first + threadIdx.x) * H + h] = power[threadIdx.x + 1];
-        ts[(size_t)(first + threadIdx.x) * H + h] = power[n - 1 - threadIdx.x];
     }
     const float* const x[1] = {qs};
     triangle_products<DP, 1>(x, ks, threadIdx.x >> 5, threadIdx.x & 31, [&](const auto& acc, int r0, int n0, int zeros) {
@@ -735,11 +735,10 @@ static int launch_retention_walk(const void* proj, int proj_stride, int q_off, i
     float* k = q + rows * d;
     float* p = k + rows * d;
     float* rs = p + rows * 64;
-    float* ts = rs + rows;
     const dim3 grid(tokens / 64 + entries, heads);
     WalkArgs a = {};
     a.q = q; a.k = k; a.qk_stride = heads * d; a.rep = 1; a.v_stride = proj_stride; a.silu = silu;
-    a.p = p; a.rs = rs; a.ts = ts; a.eb = rs; a.state = state; a.state_stride = state_stride; a.s_row = dv; a.s_col = 1; a.o = o;
+    a.p = p; a.rs = rs; a.eb = rs; a.state = state; a.state_stride = state_stride; a.s_row = dv; a.s_col = 1; a.o = o;
     a.cu_q = cu_q; a.seq_rows = seq_rows; a.H = heads; a.d = d; a.dv = dv;
     const int cols = walk_columns(entries, heads, dv, sms);
     SE_DISPATCH_DTYPE(dtype, T_, {
@@ -749,9 +748,11 @@ static int launch_retention_walk(const void* proj, int proj_stride, int q_off, i
         a.v = in.proj + v_off;
         SE_WALK_DIMS(d, {
             const int rc = launch(retention_prepare_kernel<DP, T_>, grid, 2 * 64 * (DP + 8) * sizeof(float), stream, in, decay, cu_q,
-                                  entries, q, k, p, rs, ts, heads, d);
+                                  entries, q, k, p, rs, heads, d);
             if (rc != 0) return rc;
-            return launch_walk<64, DP, false, false, T_>(a, entries, cols, stream);
+            // 16-bit value rows as they are have no lower term
+            if (sizeof(T_) == 2 && !silu) return launch_walk<64, DP, false, false, true, sizeof(T_) == 2, T_>(a, entries, cols, stream);
+            return launch_walk<64, DP, false, false, true, false, T_>(a, entries, cols, stream);
         });
     });
 }

@@ -34,8 +34,8 @@ __device__ __forceinline__ void mma_start(float (&d)[4], const uint32_t (&a)[4],
 // values of tile row i: (row lane / 4, first k), (row + 8, first k), (row, second k), (row + 8, second k); b(n, step, v) its two of
 // tile column n: (first k, column lane / 4), (second k, the same).  Which two of the step's eight k are a lane's is the callers' choice:
 // 2 (lane % 4) and the one after it, so that rows along k are read two at a time.  acc[i][n] holds (row lane / 4, columns 2 (lane % 4)
-// and the one after it), then the same of row + 8.
-template <int MT, int NT, int UNROLL, typename A, typename B>
+// and the one after it), then the same of row + 8.  EXACT: b's values are tf32 values themselves (16-bit inputs): two terms.
+template <int MT, int NT, int UNROLL, bool EXACT = false, typename A, typename B>
 __device__ __forceinline__ void products(float (&acc)[MT][NT][4], int steps, A a, B b) {
     float low[MT][NT][4] = {};
 #pragma unroll UNROLL
@@ -52,8 +52,13 @@ __device__ __forceinline__ void products(float (&acc)[MT][NT][4], int steps, A a
         for (int n = 0; n < NT; ++n) {
             float v[2];
             b(n, s, v);
-            halves(v[0], bh[n][0], bl[n][0]);
-            halves(v[1], bh[n][1], bl[n][1]);
+            if (EXACT) {
+                bh[n][0] = __float_as_uint(v[0]);
+                bh[n][1] = __float_as_uint(v[1]);
+            } else {
+                halves(v[0], bh[n][0], bl[n][0]);
+                halves(v[1], bh[n][1], bl[n][1]);
+            }
         }
         float big[MT][NT][4];
 #pragma unroll
@@ -64,10 +69,11 @@ __device__ __forceinline__ void products(float (&acc)[MT][NT][4], int steps, A a
         for (int i = 0; i < MT; ++i)
 #pragma unroll
             for (int n = 0; n < NT; ++n) mma_add(low[i][n], al[i], bh[n]);
+        if (!EXACT)
 #pragma unroll
-        for (int i = 0; i < MT; ++i)
+            for (int i = 0; i < MT; ++i)
 #pragma unroll
-            for (int n = 0; n < NT; ++n) mma_add(low[i][n], ah[i], bl[n]);
+                for (int n = 0; n < NT; ++n) mma_add(low[i][n], ah[i], bl[n]);
 #pragma unroll
         for (int i = 0; i < MT; ++i)
 #pragma unroll
