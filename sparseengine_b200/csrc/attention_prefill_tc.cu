@@ -65,6 +65,9 @@ struct Bars {
                                                          // wait for p_empty may be phases behind it, so the end has a barrier of its own)
 };
 
+// The n lowest bits (none below 0, all from 32 on).
+__device__ __forceinline__ uint32_t low_bits(int n) { return n >= 32 ? 0xffffffffu : (1u << max(n, 0)) - 1u; }
+
 __global__ void __launch_bounds__(kThreads, 1)
 attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
                        const int* __restrict__ table, int table_stride, const int* __restrict__ seq_rows,
@@ -106,6 +109,15 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
     const int kept_tiles = (kept + kKeys - 1) / kKeys;
     const int num_tiles = kept_tiles + (k_end - k_begin + kKeys - 1) / kKeys;
 
+    // The tiles [j0, j1) that some row of query tile x sees: with few query heads to a KV head its 128 rows see up to
+    // two tiles fewer than the CTA's 256 at either end, and a tile without rows sees none.
+    auto seen_tiles = [&](int x, int& j0, int& j1) {
+        const int row0 = row_base + x * kRows, row1 = min(row0 + kRows, total_rows) - 1;
+        if (row0 > row1) { j0 = j1 = 0; return; }
+        j0 = keep_first > 0 ? 0 : (first_visible(q_start + row0 / group, window) - k_begin) / kKeys;
+        j1 = kept_tiles + (q_start + row1 / group + 1 - k_begin + kKeys - 1) / kKeys;
+    };
+
     auto bar = [&](uint64_t* b) { return smem_u32(b); };
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(bar(&bars.kv_full[s]), 32); mbar_init(bar(&bars.kv_empty[s]), kTiles); }   // full: every lane of the tile's loader warp; empty: both query tiles' MMAs
@@ -126,8 +138,8 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // Q tiles: every thread copies chunks; rows beyond the portion's rows are zero-filled
-    for (int i = threadIdx.x; i < kTiles * kRows * 16; i += kThreads) {
+    // Q tiles: the softmax warps copy chunks, and the first K/V tiles are fetched meanwhile; rows beyond the portion's rows are zero-filled
+    for (int i = threadIdx.x - 64; i < kTiles * kRows * 16 && warp >= 2 && warp < kLoaderWarp2; i += 32 * 4 * kTiles) {
         const int r = i >> 4, c = i & 15;                  // r: 0..255 over both tiles
         const int row = row_base + r;
         const bool ok = row < total_rows;
@@ -136,11 +148,14 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
         cp_async16(smem_u32(q_s) + (r >> 7) * kQBytes + (c >> 3) * (kRows * 128) + sw128(r & 127, c & 7), src, ok);
     }
     cp_async_commit();
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    __syncthreads();                                       // barriers and tensor memory
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp != 0 && warp != kLoaderWarp2) {               // Q, for all that compute
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(kThreads - 64) : "memory");
+    }
     const uint32_t tmem = tmem_base_s;
     // tensor memory: O of tile x in columns 128 x .. 128 x + 127; S buffer b of tile x in 256 + 128 x + 64 b ..
     auto tmem_o = [&](int x) { return tmem + (uint32_t)(128 * x); };
@@ -211,6 +226,10 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
         const int x = warp == 1 ? 0 : 1;
         const uint32_t id_s = idesc(kKeys, 0), id_o = idesc(D, 1);
         const int tiles = uniform(num_tiles);
+        int j0, j1;
+        seen_tiles(x, j0, j1);
+        j0 = uniform(j0);
+        j1 = uniform(j1);
         const uint32_t tm = (uint32_t)uniform((int)tmem), o_at = tm + 128 * x, s_at = tm + 256 + 128 * x;
         const uint64_t q_desc = desc_kmajor(smem_u32(q_s) + x * kQBytes);
         bool ok = true;
@@ -234,10 +253,18 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
         int stage = 0, before = 0;                           // of tiles j and j - 1
         uint32_t turn = 0;                                   // how often the stages have gone round, modulo 2
         for (int j = 0; j < tiles && ok; ++j) {
-            const int b = j & 1;
+            const int i = j - j0, b = i & 1;                 // S, P and their barriers count the query tile's own tiles
             wait(&bars.kv_full[stage], turn);
+            if (j < j0 || j >= j1) {                         // not seen: the stage goes back (its last turn has ended, for it is full)
+                if (ok && j == j1 && i > 0) issue_pv(i - 1, before);
+                if (ok && elect_one()) mbar_arrive(bar(&bars.kv_empty[stage]));
+                __syncwarp();
+                stage = stage + 1 == kStages ? 0 : stage + 1;
+                if (stage == 0) turn ^= 1;
+                continue;
+            }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the copies were generic-proxy writes
-            if (ok && j >= 2) wait(&bars.s_empty[x][b], ((j >> 1) - 1) & 1);
+            if (ok && i >= 2) wait(&bars.s_empty[x][b], ((i >> 1) - 1) & 1);
             if (ok && elect_one()) {
                 const uint64_t k_desc = desc_kmajor(smem_u32(kv_s) + stage * kKVStageBytes);
 #pragma unroll
@@ -249,12 +276,12 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
                 umma_commit(bar(&bars.s_full[x][b]));
             }
             __syncwarp();
-            if (ok && j >= 1) issue_pv(j - 1, before);
+            if (ok && i >= 1) issue_pv(i - 1, before);
             before = stage;
             stage = stage + 1 == kStages ? 0 : stage + 1;
             if (stage == 0) turn ^= 1;
         }
-        if (ok) issue_pv(tiles - 1, before);
+        if (ok && j1 == tiles && j1 > j0) issue_pv(j1 - j0 - 1, before);
         if (ok && elect_one()) umma_commit(bar(&bars.o_done[x]));
         __syncwarp();
         if (!ok && lane == 0) { abort_s = 1; atomicCAS(error, 0, 12); }
@@ -273,9 +300,11 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
         const float slope = se::mma::raw_slope(opt, kvh * group + rr % group);      // distance bias per token, raw units
         const int pos_first = __shfl_sync(0xffffffffu, pos, 0), lo_last = __shfl_sync(0xffffffffu, lo, 31);
         bool ok = true;
-        for (int j = 0; j < num_tiles && ok; ++j) {
-            const int b = j & 1;
-            if (!mbar_wait(bar(&bars.s_full[x][b]), (j >> 1) & 1, &abort_s)) { ok = false; break; }
+        int j0, j1;
+        seen_tiles(x, j0, j1);
+        for (int j = j0; j < j1 && ok; ++j) {
+            const int i = j - j0, b = i & 1;
+            if (!mbar_wait(bar(&bars.s_full[x][b]), (i >> 1) & 1, &abort_s)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             uint32_t sv[64];
             tmem_ld32(tmem_s(x, b) + lane_addr, sv);
@@ -310,10 +339,15 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
             const bool full = first ? key0 + kKeys <= kept
                                     : key0 + kKeys - 1 <= pos_first && key0 >= lo_last && key0 >= kept;
             if (!full) {
+                // a bit per key, so that a key costs a test and a select: compared key by key a tile took 1.7 us more than a full one
+                const int shown = first ? kept - key0 : pos + 1 - key0;
 #pragma unroll
-                for (int c = 0; c < 64; ++c) {
-                    const int key = key0 + c;
-                    if (first ? key >= kept : (key > pos || (key < lo && key >= keep_first) || key < kept)) sv[c] = 0xff800000u;      // -inf
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t bits = low_bits(shown - 32 * h);
+                    if (!first) bits &= (~low_bits(lo - key0 - 32 * h) | low_bits(keep_first - key0 - 32 * h)) & ~low_bits(kept - key0 - 32 * h);
+#pragma unroll
+                    for (int c = 0; c < 32; ++c)
+                        if (!(bits & (1u << c))) sv[32 * h + c] = 0xff800000u;      // -inf
                 }
             }
             float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains instead of one of 64
@@ -339,7 +373,7 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
                 // O must be at rest: P·V of the previous tile has finished.  (Only then: a warp whose
                 // rows keep their reference maximum runs on, up to a tile ahead of the others, which
                 // is why P's barrier exists once per S buffer.)
-                if (j >= 1 && !mbar_wait(bar(&bars.p_empty[x]), (j - 1) & 1, &abort_s)) { ok = false; break; }
+                if (i >= 1 && !mbar_wait(bar(&bars.p_empty[x]), (i - 1) & 1, &abort_s)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
                 for (int c0 = 0; c0 < D; c0 += 32) {
