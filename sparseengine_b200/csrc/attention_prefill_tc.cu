@@ -34,9 +34,15 @@
 // special-function operations per score for the cap, an add and a multiply-add per score for a distance
 // bias, one term in the last sum for the sink, and one load and exponential per output element for the gate.  Arithmetic as the reference's prefill kernel
 // (src/sparseengine/kernels/triton/context_flashattention_nopad.py:92-127).
+//
+// With PARTS the same kernel runs latent attention over keys and values that were formed per head from the latents (heads of 64
+// unrotated and 64 rotated dims, values of 64): a key's first half comes from a product's rows, its second, which all heads share, from
+// the latents' rows, and no page is looked up.
 #include "common.cuh"
 #include "fa_util.cuh"
 #include "mma_util.cuh"
+
+#include <initializer_list>
 
 namespace se {
 namespace fa {
@@ -65,15 +71,27 @@ struct Bars {
                                                          // wait for p_empty may be phases behind it, so the end has a barrier of its own)
 };
 
+// Where keys and values formed per head lie: rows of the keys that the entries see, each entry's from the first key that its first token
+// sees on, entry after entry.
+struct Parts {
+    int q_pitch;
+    const __nv_bfloat16* kv;       // [rows][kv_pitch]: heads' 64 key dims, from v_off on their 64 value dims
+    int kv_pitch, v_off;
+    const __nv_bfloat16* rot;      // [rows][rot_pitch]: the shared 64 rotated dims
+    int rot_pitch;
+};
+
 // The n lowest bits (none below 0, all from 32 on).
 __device__ __forceinline__ uint32_t low_bits(int n) { return n >= 32 ? 0xffffffffu : (1u << max(n, 0)) - 1u; }
 
+template <bool PARTS>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
                        const int* __restrict__ table, int table_stride, const int* __restrict__ seq_rows,
                        const int* __restrict__ cu_q, const int* __restrict__ kv_len, __nv_bfloat16* __restrict__ out,
                        int* error, int hq, int hkv, int page_size, float scale_log2, int window, int num_pages,
-                       const se::mma::SoftmaxOptions opt) {
+                       const se::mma::SoftmaxOptions opt, const Parts parts) {
+    constexpr int DV = PARTS ? 64 : D;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* q_s = smem;                               // [2 tiles][2 halves][128 rows][128 B]
@@ -144,7 +162,8 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
         const int row = row_base + r;
         const bool ok = row < total_rows;
         const int rr = ok ? row : total_rows - 1;
-        const __nv_bfloat16* src = q + ((size_t)(tok0 + rr / group) * hq + kvh * group + rr % group) * D + c * 8;
+        const __nv_bfloat16* src = (PARTS ? q + (size_t)(tok0 + rr) * parts.q_pitch + kvh * D
+                                          : q + ((size_t)(tok0 + rr / group) * hq + kvh * group + rr % group) * D) + c * 8;
         cp_async16(smem_u32(q_s) + (r >> 7) * kQBytes + (c >> 3) * (kRows * 128) + sw128(r & 127, c & 7), src, ok);
     }
     cp_async_commit();
@@ -161,7 +180,7 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
     auto tmem_o = [&](int x) { return tmem + (uint32_t)(128 * x); };
     auto tmem_s = [&](int x, int b) { return tmem + (uint32_t)(256 + 128 * x + 64 * b); };
 
-    const int* row_table = table + (size_t)seq_rows[entry] * table_stride;
+    const int* row_table = PARTS ? nullptr : table + (size_t)seq_rows[entry] * table_stride;
     const size_t page_elems = (size_t)2 * hkv * page_size * D;
     const size_t head_off = (size_t)kvh * page_size * D;
     const size_t v_off = (size_t)hkv * page_size * D;
@@ -172,11 +191,33 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
         // Lane l looks up where keys base+l and base+32+l live (two independent table loads per
         // lane and tile); the copy loop gets each row's address by shuffle, so no load sits
         // between the asynchronous copies.
+        int rows_before = 0;                             // PARTS: the rows of the entries before this one
+        if constexpr (PARTS) {
+            for (int e = lane; e < entry; e += 32) rows_before += kv_len[e] - first_visible(kv_len[e] - (cu_q[e + 1] - cu_q[e]), window);
+            rows_before = __reduce_add_sync(0xffffffffu, rows_before) - first_visible(q_start, window);
+        }
         auto issue = [&](int tile) {
             uint8_t* st = kv_s + (size_t)(tile % kStages) * kKVStageBytes;
             const bool first = tile < kept_tiles;
             const int base = first ? tile * kKeys : k_begin + (tile - kept_tiles) * kKeys;
             const int k_lo = first ? 0 : k_lo_window, k_end = first ? kept : k_end_window;      // the keys of this tile that are read
+            if constexpr (PARTS) {                   // zero-filled outside [k_lo, k_end), as below
+                const int c = lane & 7;
+                const size_t row0 = (size_t)(rows_before + base);
+                const __nv_bfloat16* kv = parts.kv + kvh * 64 + c * 8;
+                const __nv_bfloat16* rot = parts.rot + c * 8;
+#pragma unroll 4
+                for (int k = 0; k < kKeys / 4; ++k) {
+                    const int r = 4 * k + (lane >> 3);
+                    const bool ok = base + r < k_end && base + r >= k_lo;
+                    const size_t row = ok ? row0 + r : 0;
+                    const uint32_t off = sw128(r, c);
+                    cp_async16(smem_u32(st) + off, kv + row * parts.kv_pitch, ok);
+                    cp_async16(smem_u32(st) + kHalfBytes + off, rot + row * parts.rot_pitch, ok);
+                    cp_async16(smem_u32(st) + 2 * kHalfBytes + off, kv + row * parts.kv_pitch + parts.v_off, ok);
+                }
+                return;
+            }
             // Keys outside [k_lo, k_end) are zero-filled, never read: a page the window has left
             // behind may belong to another request by now.  An entry that names no page of the pool
             // is not followed either (address 0 marks its row; a code goes to the error word).
@@ -224,7 +265,7 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
         // The warp runs as a whole through uniform loops and one elected lane issues (fa_util.cuh): 8,192 tokens behind 16,384 keys 4,145 us,
         // issued under a divergent branch and with two more shuffles a tile in the softmax 4,206.
         const int x = warp == 1 ? 0 : 1;
-        const uint32_t id_s = idesc(kKeys, 0), id_o = idesc(D, 1);
+        const uint32_t id_s = idesc(kKeys, 0), id_o = idesc(DV, 1);
         const int tiles = uniform(num_tiles);
         int j0, j1;
         seen_tiles(x, j0, j1);
@@ -376,7 +417,7 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
                 if (i >= 1 && !mbar_wait(bar(&bars.p_empty[x]), (i - 1) & 1, &abort_s)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-                for (int c0 = 0; c0 < D; c0 += 32) {
+                for (int c0 = 0; c0 < DV; c0 += 32) {
                     uint32_t ov[32];
                     tmem_ld32(tmem_o(x) + c0 + lane_addr, ov);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -415,14 +456,14 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
             // the sink's term 2^(0 - m): it grows beyond the type only where the keys hold nothing (the output is 0 then)
             if (opt.sink) l += exp2f(se::mma::sink_log2(opt, kvh * group + rr % group) - m_ref);
             const float inv = 1.f / l;
-            __nv_bfloat16* dst = out + ((size_t)(tok0 + rr / group) * hq + kvh * group + rr % group) * D;
+            __nv_bfloat16* dst = out + ((size_t)(tok0 + rr / group) * hq + kvh * group + rr % group) * DV;
             const bool gate_vec = opt.gate != nullptr && !opt.gate_per_head && se::mma::gate_rows_aligned(opt, 16);
             const __nv_bfloat16* gp = opt.gate != nullptr
                 ? se::mma::gate_of(opt, tok0 + rr / group, kvh * group + rr % group, D) : nullptr;
             const float inv_gated = gp != nullptr && opt.gate_per_head ? se::mma::gated(inv, gp) : inv;     // one gate per head: in the factor
             const bool gate_each = gp != nullptr && !opt.gate_per_head;
 #pragma unroll 1
-            for (int c0 = 0; c0 < D; c0 += 32) {
+            for (int c0 = 0; c0 < DV; c0 += 32) {
                 uint32_t ov[32];
                 tmem_ld32(tmem_o(x) + c0 + lane_addr, ov);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -488,7 +529,7 @@ extern "C" int se_attn_prefill_tc(const void* q, const void* cache, const int* t
     const size_t smem = (size_t)kTiles * kQBytes + kStages * kKVStageBytes + 1024;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
@@ -496,8 +537,32 @@ extern "C" int se_attn_prefill_tc(const void* q, const void* cache, const int* t
     const int row_tiles = se::ceil_div(max_q_len * group, kTiles * kRows);
     if (row_tiles > 65535) return SE_ERR_UNSUPPORTED;
     dim3 grid(hkv, row_tiles, entries);
-    attn_prefill_tc_kernel<<<grid, kThreads, smem, stream>>>(
+    attn_prefill_tc_kernel<false><<<grid, kThreads, smem, stream>>>(
         (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, table, table_stride, seq_rows, cu_q, kv_len,
-        (__nv_bfloat16*)out, error, hq, hkv, page_size, scale * 1.4426950408889634f, window, num_pages, opt);
+        (__nv_bfloat16*)out, error, hq, hkv, page_size, scale * 1.4426950408889634f, window, num_pages, opt, Parts{});
+    return (int)cudaGetLastError();
+}
+
+// Latent attention over keys and values formed per head: heads of 64 unrotated and 64 rotated dims (q's rows: heads x 128, already
+// rotated), values of 64 (the pointers as struct Parts has them); out [tokens][heads][64].  window: 0 none, else the keys a token sees.
+extern "C" int se_attn_prefill_tc_parts(const void* q, int q_pitch, const void* kv, int kv_pitch, int v_off, const void* rot,
+                                        int rot_pitch, const int* cu_q, const int* kv_len, const float* sink_logits, void* out,
+                                        int* error, int entries, int max_q_len, int heads, float scale, int window, cudaStream_t stream) {
+    using namespace se::fa;
+    if (entries <= 0 || max_q_len <= 0) return 0;
+    if (heads <= 0 || heads > 65535 || entries > 65535 || q_pitch % 8 || kv_pitch % 8 || v_off % 8 || rot_pitch % 8) return SE_ERR_UNSUPPORTED;
+    if (!(scale > 0.f) || window < 0) return SE_ERR_ARGUMENT;
+    for (const void* x : {q, kv, rot, (const void*)out})
+        if (reinterpret_cast<uintptr_t>(x) & 15) return SE_ERR_UNSUPPORTED;
+    const se::mma::SoftmaxOptions opt{0.f, 0.f, sink_logits != nullptr, nullptr, 0, sink_logits, 0, nullptr, 1.f / scale, 0};
+    const Parts parts{q_pitch, (const __nv_bfloat16*)kv, kv_pitch, v_off, (const __nv_bfloat16*)rot, rot_pitch};
+    const size_t smem = (size_t)kTiles * kQBytes + kStages * kKVStageBytes + 1024;
+    const cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    const int row_tiles = se::ceil_div(max_q_len, kTiles * kRows);
+    if (row_tiles > 65535) return SE_ERR_UNSUPPORTED;
+    attn_prefill_tc_kernel<true><<<dim3(heads, row_tiles, entries), kThreads, smem, stream>>>(
+        (const __nv_bfloat16*)q, nullptr, nullptr, 0, nullptr, cu_q, kv_len, (__nv_bfloat16*)out, error, heads, heads, 1,
+        scale * 1.4426950408889634f, window, 0, opt, parts);
     return (int)cudaGetLastError();
 }

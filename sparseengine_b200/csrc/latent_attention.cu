@@ -330,13 +330,14 @@ __global__ void latent_q_rotate_kernel(const __nv_bfloat16* q, int q_pitch, int 
                                        int rotary_dim, int interleaved, const int* __restrict__ positions,
                                        __nv_bfloat16* qfull, int heads, int rank, int rot) {
     extern __shared__ float cs_sn[];
+    const size_t out_pitch = qfull == q ? q_pitch : heads * (rank + rot);
     grid_dependency_trigger();
     grid_dependency_wait();
     const int t = blockIdx.x, half = rotary_dim / 2;
     for (int k = threadIdx.x; k < half; k += blockDim.x)
         sincosf((float)positions[t] * inv_freq[k], &cs_sn[half + k], &cs_sn[k]);
     __syncthreads();
-    rotate_queries<true>(q + (size_t)t * q_pitch, d, qfull + (size_t)t * heads * (rank + rot), heads, rank, rot, rotary_dim, interleaved,
+    rotate_queries<true>(q + (size_t)t * q_pitch, d, qfull + (size_t)t * out_pitch, heads, rank, rot, rotary_dim, interleaved,
                    cs_sn, cs_sn + half);
 }
 
@@ -645,12 +646,13 @@ extern "C" int se_latent_attention_tiled_supported(int rank, int rot) {
     return rank > 0 && rot >= 0 && rank % 16 == 0 && rot % 16 == 0 && rank + rot <= 256;
 }
 
+// qfull may be q itself (rank the unrotated dims): rotated in place, rows q_pitch apart.
 extern "C" int se_latent_q_rotate(const void* q, int q_pitch, int d, const float* inv_freq, int rotary_dim, int interleaved,
                                   const int* positions, void* qfull, int tokens, int heads, int rank, int rot,
                                   cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (heads <= 0 || rank <= 0 || rot < 0 || rotary_dim < 0 || rotary_dim > rot || (rotary_dim & 1) || d < 0 ||
-        q_pitch < heads * (d + rot))
+        q_pitch < heads * (d + rot) || (qfull == q && rank != d))
         return SE_ERR_ARGUMENT;
     if (rank + rot > se_latent_max_row()) return SE_ERR_UNSUPPORTED;
     cudaError_t e = SE_LAUNCH_DEPENDENT("lat", se::lat::latent_q_rotate_kernel, dim3(tokens), dim3(256),

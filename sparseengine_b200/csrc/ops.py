@@ -490,12 +490,12 @@ def latent_attention_tiled_supported(rank: int, rot: int) -> bool:
 
 def latent_q_rotate(q, inv_freq, positions, qfull, *, heads, head_dim, rank, rot, rotary_dim, pairing: str = "split_half"):
     """``qfull[t, h, rank:] = rotated part of q[t, h]`` (bfloat16): the query rows of the tiled kernel, whose first
-    ``rank`` dims a matrix product writes.  ``q``'s rows may be a view with a pitch."""
+    ``rank`` dims a matrix product writes.  ``q``'s rows may be a view with a pitch.  ``qfull`` may be ``q`` itself (``rank`` its unrotated dims)."""
     tokens = q.shape[0]
     _check(_fn("se_latent_q_rotate", "piipii" "pp" "iiii" "p")(
         _rows_ptr(q, "q", torch.bfloat16), q.stride(0), head_dim, _ptr(inv_freq, torch.float32, "inv_freq"), rotary_dim,
-        _interleaved(pairing), _ptr(positions, torch.int32, "positions"), _ptr(qfull, torch.bfloat16, "qfull"), tokens, heads,
-        rank, rot, _stream()), "latent_q_rotate")
+        _interleaved(pairing), _ptr(positions, torch.int32, "positions"),
+        q.data_ptr() if qfull is q else _ptr(qfull, torch.bfloat16, "qfull"), tokens, heads, rank, rot, _stream()), "latent_q_rotate")
     return qfull
 
 
@@ -548,6 +548,12 @@ def latent_takes_tc(entries: int, max_q_len: int, heads: int, rank: int, rot: in
         return False
     if not q_lens or not kv_lens:
         return 5 * entries * -(-max_q_len * heads // 256) >= sms
+    tc, tiled = latent_times(entries, max_q_len, heads, rank, sms, q_lens, kv_lens, window)
+    return tc < tiled
+
+
+def latent_times(entries: int, max_q_len: int, heads: int, rank: int, sms: int, q_lens, kv_lens, window: Optional[int]):
+    """The times (us) that the tcgen05 and the tiled latent attention are estimated to take (:func:`latent_takes_tc`)."""
     tile_keys = latent_tile_keys(max_q_len)
     most = max(kv_lens) if window is None else min(max(kv_lens), window + max_q_len - 1)
     splits, per = latent_split_plan(-(-max_q_len * heads // 64), entries, most, sms, tile_keys)
@@ -569,7 +575,67 @@ def latent_takes_tc(entries: int, max_q_len: int, heads: int, rank: int, rot: in
     tc = 8 + 2.1 / 64 * max(wide_last, -(-wide // sms) * wide_keys / wide) + 2.1
     full, rest = divmod(narrow, 2 * sms)
     tiled = 10 + max(0.054 * narrow_last, (0.067 * full + (0.067 if rest > sms else 0.054 if rest else 0.0)) * narrow_keys / narrow)
-    return tc < tiled + (14 + narrow * 64 * rank * 8 / 5e6 if splits > 1 else 0)
+    return tc, tiled + (14 + narrow * 64 * rank * 8 / 5e6 if splits > 1 else 0)
+
+
+# Most bytes that keys and values formed per head may take for a step.
+LATENT_HEADS_MAX_BYTES = 256 << 20
+
+
+def latent_seen_keys(q_lens, kv_lens, window: Optional[int]) -> list:
+    """How many cached rows each entry sees: from the first key that its first token sees on."""
+    return [kv if window is None else min(kv, q + window - 1) for q, kv in zip(q_lens, kv_lens)]
+
+
+def latent_takes_heads(max_q_len: int, heads: int, rank: int, sms: int, q_lens, kv_lens, window: Optional[int]) -> bool:
+    """Whether a step's latent attention forms keys and values per head (heads of 64 + 64 dims, values of 64) instead of taking the queries
+    into the latent's space: a score and its sum then take 192 multiply-adds instead of 448, for two products over the rows that
+    the entries see.  A block takes 256 tokens of a head, 1.2 us per 64 keys, 8 to start and end; the products reach 700 TFLOP/s and
+    5 TB/s and take 12 for their launches and the gathered rows.  Against it the shorter of :func:`latent_times` and the two
+    products that take queries and sums from and to the latent's space.  Device us of a layer,
+    in the latent's space / per head: 32 heads, window 1,024: 8,192 tokens 524 / 391, 256 47.5 / 43.6; no window: 4,096 tokens 392 / 271,
+    300 behind 4,000 keys 176 / 130; 64 heads: 4 x 500 behind 500 217 / 197, 64 behind 100 55.0 / 54.8 (stays)."""
+    seen = latent_seen_keys(q_lens, kv_lens, window)
+    total, tokens = sum(seen), sum(q_lens)
+    if max_q_len < 32 or total * heads * 256 > LATENT_HEADS_MAX_BYTES:
+        return False
+    blocks = keys = last = 0
+    for q, kv, n in zip(q_lens, kv_lens, seen):
+        if q <= 0:
+            continue
+        b = heads * -(-q // 256)
+        most = min(kv, n, n if window is None else window + min(q, 256) - 1)
+        blocks += b
+        keys += b * (most if window is not None and kv - q >= window else max(most // 2, most - q // 2))
+        last = max(last, most)
+    formed = 8 + 1.2 / 64 * max(last, -(-blocks // sms) * keys / blocks) + 12 + total * heads * (rank * 256 / 7e8 + 512 / 5e6)
+    tc, tiled = latent_times(len(q_lens), max_q_len, heads, rank, sms, q_lens, kv_lens, window)
+    if not max_q_len * heads >= 128:
+        tc = tiled
+    return formed < min(tc, tiled) + 6 + tokens * heads * rank * 8 / 5e6
+
+
+def latent_attention_heads(q, cache, table, seq_rows, cu_q, kv_len, sink, uk, uv, *, rows, most_keys, entries, max_q_len, heads, rank,
+                           page_size, scale, window=None, num_pages=None):
+    """Latent attention over keys and values formed per head (heads of 64 + 64 dims, values of 64): ``q`` [tokens, heads * 128] with its
+    rotated dims rotated, ``uk`` and ``uv`` [heads * 64, rank]; ``rows`` cached rows are seen by all entries, ``most_keys`` by one.
+    Returns [tokens, heads * 64]."""
+    dev, bf16, row, n = q.device, torch.bfloat16, cache.shape[-1], heads * 64
+    work = torch.empty(rows * (row + 2 * n), dtype=bf16, device=dev)          # the rows, keys, values
+    lat, error, cu, kv = work.data_ptr(), _ptr(error_word(dev)), _ptr(cu_q, torch.int32, "cu_q"), _ptr(kv_len, torch.int32, "kv_len")
+    _check(_fn("se_latent_gather", "ppi" "ppp" "pp" "iiiiii" "p")(
+        _ptr(cache, bf16, "cache"), _ptr(table, torch.int32, "table"), table.shape[1], _ptr(seq_rows, torch.int32, "seq_rows"), cu, kv, lat,
+        error, entries, most_keys, row, page_size, int(window or 0), cache.shape[0] if num_pages is None else int(num_pages), _stream()),
+        "latent_gather")
+    seen = work.as_strided((rows, rank), (row, 1))
+    for i, w in enumerate((uk, uv)):
+        torch.mm(seen, w.t(), out=work.as_strided((rows, n), (n, 1), rows * (row + i * n)))
+    out = torch.empty(q.shape[0], n, dtype=bf16, device=dev)
+    _check(_fn("se_attn_prefill_tc_parts", "pi" "pii" "pi" "ppp" "pp" "iii" "fi" "p")(
+        _rows_ptr(q, "q", bf16), q.stride(0), lat + 2 * rows * row, n, rows * n, lat + 2 * rank, row, cu, kv,
+        _ptr(sink, torch.float32, "sink"), out.data_ptr(), error, entries, max_q_len, heads, float(scale), int(window or 0), _stream()),
+        "latent_attention_heads")
+    return out
 
 
 def latent_attention_tc(qfull, cache, table, seq_rows, cu_q, kv_len, sink, out, *, entries, max_q_len, heads, rank, rot,

@@ -89,6 +89,8 @@ class LatentAttention(Mixer):
             rope = RotaryArgs(None, 0)
         proj = linear(x, self.down if s.q_rank else self.in_proj)
         tiled = self.takes_tiles(x.dtype)
+        formed = self.takes_heads(step, dev) if tiled else None
+        tiled = tiled and formed is None
         qfull = torch.empty(tokens, H, rank + r, dtype=x.dtype, device=dev) if tiled else None
         cq = torch.empty(tokens, s.q_rank, dtype=x.dtype, device=dev) if s.q_rank else None
         q = proj[:, :self.q_cols]                                            # [tokens, H * (d + r)]
@@ -102,6 +104,11 @@ class LatentAttention(Mixer):
             if tiled:
                 ops.latent_q_rotate(q, rope.inv_freq, step.positions, qfull, heads=H, head_dim=d, rank=rank, rot=r,
                                     rotary_dim=rope.rotary_dim, pairing=rope.pairing)
+        if formed is not None:
+            heads_out = self.attend_heads(q, rope, step, slot, formed)
+            if s.output_gate:
+                ops.sigmoid_gate_(heads_out, proj[:, self.g_off:])
+            return linear(heads_out, self.o)
         # the unrotated queries in the latent's space: [H, tokens, d] x [H, d, rank], in the tiled kernel's query rows
         # or 32-bit
         q_plain, uk = q.unflatten(1, (H, d + r))[:, :, :d].transpose(0, 1), self.uk.view(H, d, rank)
@@ -142,6 +149,29 @@ class LatentAttention(Mixer):
             return ops.latent_takes_tc(step.num_seqs, step.max_q_len, s.num_heads, s.kv_rank, s.rot_dim, ops.sm_count(device),
                                        q_lens=step.q_lens, kv_lens=kv_lens, window=s.window)
         return once_per_step(step, ("latent.takes_tc", s.num_heads, s.kv_rank, s.rot_dim, s.window), ask)
+
+    def takes_heads(self, step, device):
+        """``ops.latent_takes_heads`` over the step's own entries, asked once per step for all layers of the same sizes: how many cached
+        rows the entries see, and the most that one sees, or None.  Steps that are captured know bounds only."""
+        s = self.spec
+        if (s.head_dim, s.rot_dim, s.v_head_dim) != (64, 64, 64) or s.kv_rank % 8 or step.max_kv_bound is not None or not step.q_lens:
+            return None
+
+        def ask():
+            if not ops.latent_takes_heads(step.max_q_len, s.num_heads, s.kv_rank, ops.sm_count(device), step.q_lens, step.kv_lens, s.window):
+                return None
+            seen = ops.latent_seen_keys(step.q_lens, step.kv_lens, s.window)
+            return sum(seen), max(seen)
+        return once_per_step(step, ("latent.takes_heads", s.num_heads, s.kv_rank, s.window), ask)
+
+    def attend_heads(self, q, rope, step, slot, formed):
+        """Keys and values formed per head from the rows that the step sees (``formed``: takes_heads'): [tokens, H * v_head_dim]."""
+        s = self.spec
+        ops.latent_q_rotate(q, rope.inv_freq, step.positions, q, heads=s.num_heads, head_dim=s.head_dim, rank=s.head_dim, rot=s.rot_dim,
+                            rotary_dim=rope.rotary_dim, pairing=rope.pairing)
+        return ops.latent_attention_heads(q, slot.kv, slot.table, step.seq_rows, step.cu_q, step.kv_len, self.sink, self.uk, self.uv,
+                                          rows=formed[0], most_keys=formed[1], entries=step.num_seqs, max_q_len=step.max_q_len,
+                                          heads=s.num_heads, rank=s.kv_rank, page_size=slot.page_size, scale=s.scale, window=s.window)
 
     def attend_tiled(self, qfull, out_lat, step, slot):
         s = self.spec

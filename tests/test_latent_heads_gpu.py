@@ -1,0 +1,68 @@
+"""Latent attention over keys and values formed per head against 64-bit softmax: query tiles that are full, nearly empty and empty, entries that
+follow held rows, windows that end inside key tiles and leave whole tiles to one of a block's two query tiles, pages that must not be read."""
+import pytest
+import torch
+
+DEV = "cuda:0"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,window,sinks", [(1, None, False), (3, 1, True), (2, 64, False), (5, 100, True), (2, 700, False), (32, None, True)])
+def test_against_64_bits(heads, window, sinks):
+    from sparseengine_b200.csrc import ops
+    rank, page, D = 192, 16, 256
+    g = torch.Generator(device=DEV).manual_seed(heads + (window or 0))
+    q_lens, kv_lens = [257, 1, 128, 255, 17, 600], [257, 64, 129, 900, 17, 1000]
+    entries, tokens = len(q_lens), sum(q_lens)
+    most = -(-max(kv_lens) // page)
+    table = torch.randperm(entries * most, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(entries, most).to(DEV)
+    rows = torch.tensor([3, 0, 5, 4, 1, 2], dtype=torch.int32, device=DEV)
+    cache = (torch.randn(entries * most, page, D, generator=g, device=DEV) * 0.7).to(torch.bfloat16)
+    uk, uv = ((torch.randn(heads * 64, rank, generator=g, device=DEV) * rank ** -0.5).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(tokens, heads * 128 + 8, generator=g, device=DEV).to(torch.bfloat16)[:, :heads * 128]      # rows at a pitch
+    sink = torch.linspace(-6.0, 4.0, heads, device=DEV) if sinks else None
+    cu = [0]
+    for n in q_lens:
+        cu.append(cu[-1] + n)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    cu_d, kv_d, scale = torch.tensor(cu, **i32), torch.tensor(kv_lens, **i32), 128 ** -0.5 * 2.0
+    seen = ops.latent_seen_keys(q_lens, kv_lens, window)
+
+    def run(cache, table):
+        out = ops.latent_attention_heads(q, cache, table, rows, cu_d, kv_d, sink, uk, uv, rows=sum(seen), most_keys=max(seen), entries=entries,
+                                         max_q_len=max(q_lens), heads=heads, rank=rank, page_size=page, scale=scale, window=window)
+        ops.error_check(DEV)
+        return out.view(tokens, heads, 64)
+
+    out = run(cache, table)
+    want = torch.empty(tokens, heads, 64, dtype=torch.float64, device=DEV)
+    for e, (n, m) in enumerate(zip(q_lens, kv_lens)):
+        at0 = m - seen[e]
+        lat = cache[table[int(rows[e])].long()].reshape(-1, D)[at0:m]
+        k, v = (torch.mm(lat[:, :rank], w.t()).double().view(-1, heads, 64) for w in (uk, uv))        # rounded to 16 bits there too
+        k = torch.cat([k, lat[:, None, rank:].double().expand(-1, heads, -1)], -1)
+        qs = q[cu[e]:cu[e + 1]].view(n, heads, 128).double()
+        pos, at = torch.arange(m - n, m, device=DEV)[:, None], torch.arange(at0, m, device=DEV)[None]
+        s = torch.einsum("thd,khd->thk", qs, k) * scale
+        s = s.masked_fill(((at > pos) | (at <= pos - window) if window else at > pos)[:, None], float("-inf"))
+        if sinks:
+            s = torch.cat([s, sink.double()[None, :, None].expand(n, -1, 1)], -1)
+        want[cu[e]:cu[e + 1]] = torch.einsum("thk,khd->thd", torch.softmax(s, -1)[..., :seen[e]], v)
+    # weights rounded to 16 bits (2^-9 of their sum's size), the result rounded once
+    assert float((out.double() - want).abs().max()) < 8e-3 * float(want.abs().max())
+    if window:          # what lies before every query's window may be anybody's
+        dirty, wrong = cache.clone(), table.clone()
+        for e, n in enumerate(seen):
+            for i in range((kv_lens[e] - n) // page):
+                dirty[int(table[int(rows[e]), i])] = float("inf")
+                wrong[int(rows[e]), i] = 10 ** 6
+        assert torch.equal(run(dirty, wrong), out)
+
+
+def test_choice():
+    from sparseengine_b200.csrc import ops
+    assert ops.latent_seen_keys([5, 1, 8], [5, 90, 20], 10) == [5, 10, 17] and ops.latent_seen_keys([5], [90], None) == [90]
+    take = lambda q, kv, window=None, heads=32: ops.latent_takes_heads(max(q), heads, 192, 148, q, kv, window)
+    assert take([8192], [8192], 1024) and take([1000], [5000]) and take([500] * 4, [1000] * 4, 1024, 64)
+    assert not take([1] * 64, [3000] * 64) and not take([31], [31])            # single tokens: the expansion is never paid back
+    assert not take([64], [200000], None, 64)                                 # the keys and values would take more than their bound
