@@ -76,6 +76,13 @@ def test_gated_group_norm(parts, n, off, dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("parts,n,off", [(1, 4, 0), (3, 508, 4), (1, 512, 0), (7, 512, 8), (1, 516, 4)])
+def test_gated_group_norm_by_warps(parts, n, off, dtype):
+    """Around the 512 columns that a warp takes, with warps of the last block that have no part."""
+    test_gated_group_norm(parts, n, off, dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads,d,rot,off,silu", [(1, 16, 16, 0, False), (3, 24, 16, 8, True), (40, 128, 128, 0, False), (2, 128, 64, 8, True),
                                                   (2, 20, 16, 0, False), (2, 32, 24, 0, True), (2, 32, 32, 4, False)])
 def test_retention_preparation_and_output(heads, d, rot, off, silu, dtype):
