@@ -543,7 +543,6 @@ extern "C" int se_delta_walk(const float* qkv, const void* in_a, int a_pitch, co
     WalkArgs a = {};
     a.state = state; a.state_stride = state_stride; a.s_row = 1; a.s_col = d; a.o = o; a.cu_q = cu_q; a.seq_rows = seq_rows;
     a.H = H; a.d = d; a.dv = dv;
-    const int cols = walk_columns(entries, H, dv, sms);
     float* w = work;
     float* u = w + rows * d;
     a.w = w; a.v = u; a.v_stride = H * dv;
@@ -561,7 +560,7 @@ extern "C" int se_delta_walk(const float* qkv, const void* in_a, int a_pitch, co
                                       (64 * (DP + 8) + 64 * 68 + tile) * sizeof(float), stream, in, p, w, u, rs, ts, eb);
                 if (rc != 0) return rc;
                 a.q = qkv; a.k = qkv + G * d; a.qk_stride = 2 * G * d + H * dv; a.rep = H / G; a.p = p; a.rs = rs; a.ts = ts; a.eb = eb;
-                return launch_walk<64, DP, true, false, false, false, float>(a, entries, cols, stream);
+                return launch_walk<64, DP, true, false, false, false, float>(a, entries, walk_columns(entries, H, dv, sms), stream);
             }
             float* qt = u + rows * dv;
             float* kt = qt + rows * d;
@@ -571,7 +570,9 @@ extern "C" int se_delta_walk(const float* qkv, const void* in_a, int a_pitch, co
                                   (3 * 32 * (DP + 4) + 2 * 32 * 36 + 2 * DP) * sizeof(float), stream, in, p, w, u, qt, kt, tot);
             if (rc != 0) return rc;
             a.q = qt; a.k = kt; a.qk_stride = H * d; a.rep = 1; a.p = p; a.tot = tot;
-            return launch_walk<32, DP, true, true, true, false, float>(a, entries, cols, stream);
+            // Chunks of 32 tokens leave two blocks an SM: 16 columns are ahead also where there are many (16 heads, walk in us by columns,
+            // 16 / 32: two entries of 1,558 tokens 305 / 352, three of 1,500 467 / 487, four of 1,500 511 / 523).
+            return launch_walk_columns<32, DP, 16, true, true, true, false, float>(a, entries, stream);
         });
     });
 }
