@@ -570,8 +570,8 @@ extern "C" int se_delta_walk(const float* qkv, const void* in_a, int a_pitch, co
                                   (3 * 32 * (DP + 4) + 2 * 32 * 36 + 2 * DP) * sizeof(float), stream, in, p, w, u, qt, kt, tot);
             if (rc != 0) return rc;
             a.q = qt; a.k = kt; a.qk_stride = H * d; a.rep = 1; a.p = p; a.tot = tot;
-            // Chunks of 32 tokens leave two blocks an SM: 16 columns are ahead also where there are many (16 heads, walk in us by columns,
-            // 16 / 32: two entries of 1,558 tokens 305 / 352, three of 1,500 467 / 487, four of 1,500 511 / 523).
+            // Chunks of 32 tokens leave two blocks an SM: 16 columns are ahead also where there are many (16 heads, walk alone in us by columns,
+            // 16 / 32: two entries of 1,558 tokens 201 / 248, three of 1,500 311 / 331, four of 1,500 320 / 335; eight of 700 the same).
             return launch_walk_columns<32, DP, 16, true, true, true, false, float>(a, entries, stream);
         });
     });
