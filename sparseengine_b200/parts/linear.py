@@ -34,8 +34,8 @@ GEMV_GLU_MAX_OUT = 65536       # gate and up rows together
 
 
 def _product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """x . w^T in x's type: in float32 with this library's kernel where it is estimated to be ahead, else the library product."""
-    if (x.dtype == torch.float32 and x.dim() == 2 and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1]
+    """x . w^T in float32: with this library's kernel where it is estimated to be ahead, else the library product."""
+    if (x.dim() == 2 and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1]
             and not (x.data_ptr() | w.data_ptr()) & 15 and (out is None or out.is_contiguous() and out.shape == (x.shape[0], w.shape[0]))
             and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
             and ops.gemm_f32_tc_supported(x.shape[1]) and ops.gemm_f32_dense_pays(x.shape[0], w.shape[0], x.shape[1], ops.sm_count(x.device))):
@@ -59,7 +59,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, ac
         if out is None:
             out = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)
         return ops.gemv(x, w, out, activation)
-    y = _product(x, w, out)
+    if x.dtype == torch.float32:
+        y = _product(x, w, out)
+    else:
+        y = torch.matmul(x, w.t()) if out is None else torch.matmul(x, w.t(), out=out)
     return y if activation is None else ops.activation_(y, activation)
 
 
@@ -71,7 +74,7 @@ def linear_glu(x: torch.Tensor, w: torch.Tensor, activation=None) -> torch.Tenso
     if (USE_GEMV and x.dtype == torch.bfloat16 and x.is_contiguous() and w.is_contiguous() and x.shape[0] <= GEMV_MAX_ROWS
             and w.shape[0] <= GEMV_GLU_MAX_OUT and ops.gemv_supported(x.shape[0], n, x.shape[1])):
         return ops.gemv_glu(x, w, out, activation)
-    return ops.glu(_product(x, w), out, activation)
+    return ops.glu(_product(x, w) if x.dtype == torch.float32 else torch.matmul(x, w.t()), out, activation)
 
 
 def pad_rows(w: torch.Tensor, multiple: int = 8) -> torch.Tensor:
