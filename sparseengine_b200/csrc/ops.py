@@ -1344,6 +1344,8 @@ def gemm_f32_dense_pays(rows: int, n_out: int, k_dim: int, sms: int) -> bool:
 def gemm_f32_dense(x, w, out):
     """out = x [rows, k] . w [n, k]^T in 32-bit."""
     rows, k_dim = x.shape
+    if w.dim() != 2 or w.shape[1] != k_dim or out.shape != (rows, w.shape[0]):
+        raise ValueError(f"gemm_f32_dense: x {tuple(x.shape)}, w {tuple(w.shape)} and out {tuple(out.shape)} do not fit together")
     _check(_fn("se_gemm_f32_dense", "plppp" "iiii" "p")(
         _rows_ptr(x, "x", torch.float32), x.stride(0), _ptr(w, torch.float32, "w"), _ptr(out, torch.float32, "out"), _ptr(error_word(x.device)),
         rows, w.shape[0], k_dim, sm_count(x.device), _stream()), "gemm_f32_dense")

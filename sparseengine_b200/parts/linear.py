@@ -33,11 +33,17 @@ GEMV_MAX_ROWS = 8
 GEMV_GLU_MAX_OUT = 65536       # gate and up rows together
 
 
+def _kernel_reads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None) -> bool:
+    """Whether the float32 kernel can read and write these: matrices whose inner sizes agree (the library product refuses what does not
+    fit together; the kernel has only pointers), rows on 16-byte boundaries, a whole result."""
+    return (x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1] and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 4 == 0
+            and x.stride(0) >= x.shape[1] and not (x.data_ptr() | w.data_ptr()) & 15
+            and (out is None or out.is_contiguous() and out.shape == (x.shape[0], w.shape[0])))
+
+
 def _product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """x . w^T in float32: with this library's kernel where it is estimated to be ahead, else the library product."""
-    if (x.dim() == 2 and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1]
-            and not (x.data_ptr() | w.data_ptr()) & 15 and (out is None or out.is_contiguous() and out.shape == (x.shape[0], w.shape[0]))
-            and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
+    if (_kernel_reads(x, w, out) and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
             and ops.gemm_f32_tc_supported(x.shape[1]) and ops.gemm_f32_dense_pays(x.shape[0], w.shape[0], x.shape[1], ops.sm_count(x.device))):
         if out is None:
             out = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)

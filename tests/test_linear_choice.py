@@ -1,0 +1,41 @@
+"""Which float32 projections this library's kernel takes and which go on to the library product (no GPU: the kernel is a stand-in)."""
+import pytest
+import torch
+
+from sparseengine_b200.csrc import ops
+from sparseengine_b200.parts import linear as module
+from sparseengine_b200.parts.linear import linear32
+
+
+@pytest.fixture
+def taken(monkeypatch):
+    """The sizes that reached the kernel; every size pays."""
+    seen = []
+
+    def dense(x, w, out):
+        seen.append((tuple(x.shape), tuple(w.shape)))
+        return out.zero_()
+
+    monkeypatch.setattr(ops, "gemm_f32_dense", dense)
+    monkeypatch.setattr(ops, "gemm_f32_tc_supported", lambda k: True)
+    monkeypatch.setattr(ops, "gemm_f32_dense_pays", lambda *sizes: True)
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    monkeypatch.setattr(module, "_kernel_reaches", lambda *tensors: True, raising=False)
+    return seen
+
+
+def test_sizes_that_do_not_fit_together_are_refused(taken):
+    x = torch.randn(16, 32)
+    for w in (torch.randn(8, 28), torch.randn(8, 36), torch.randn(4, 8, 32)):
+        with pytest.raises(RuntimeError):
+            linear32(x, w)
+    assert linear32(x, torch.randn(32)).shape == (16,)          # a vector is a product with a vector, not 32 rows of weights
+    assert not taken
+    assert linear32(x, torch.randn(8, 32)).shape == (16, 8) and taken == [((16, 32), (8, 32))]
+
+
+def test_binding_refuses_sizes_that_do_not_fit_together():
+    x = torch.randn(16, 32)
+    for w, out in ((torch.randn(8, 28), torch.empty(16, 8)), (torch.randn(8, 32), torch.empty(16, 4)), (torch.randn(32), torch.empty(16, 32))):
+        with pytest.raises(ValueError, match="fit together"):
+            ops.gemm_f32_dense(x, w, out)
