@@ -41,9 +41,17 @@ def _kernel_reads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None) ->
             and (out is None or out.is_contiguous() and out.shape == (x.shape[0], w.shape[0])))
 
 
+def _kernel_reaches(*tensors: torch.Tensor) -> bool:
+    """Whether dense tensors all lie on the current CUDA device, whose stream the kernel is launched on.  The library product takes others too: all on
+    the CPU or on another device, sparse weights, views whose sign is still to be applied."""
+    here = tensors[0].device
+    return (here.type == "cuda" and here.index == torch.cuda.current_device()
+            and all(t.device == here and t.layout is torch.strided and not t.is_neg() for t in tensors))
+
+
 def _product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """x . w^T in float32: with this library's kernel where it is estimated to be ahead, else the library product."""
-    if (_kernel_reads(x, w, out) and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
+    if (_kernel_reaches(x, w, *(() if out is None else (out,))) and _kernel_reads(x, w, out) and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
             and ops.gemm_f32_tc_supported(x.shape[1]) and ops.gemm_f32_dense_pays(x.shape[0], w.shape[0], x.shape[1], ops.sm_count(x.device))):
         if out is None:
             out = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)

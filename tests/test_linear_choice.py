@@ -20,11 +20,16 @@ def taken(monkeypatch):
     monkeypatch.setattr(ops, "gemm_f32_tc_supported", lambda k: True)
     monkeypatch.setattr(ops, "gemm_f32_dense_pays", lambda *sizes: True)
     monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
-    monkeypatch.setattr(module, "_kernel_reaches", lambda *tensors: True, raising=False)
     return seen
 
 
-def test_sizes_that_do_not_fit_together_are_refused(taken):
+@pytest.fixture
+def reached(monkeypatch):
+    """The CPU's tensors count as the device's."""
+    monkeypatch.setattr(module, "_kernel_reaches", lambda *tensors: True)
+
+
+def test_sizes_that_do_not_fit_together_are_refused(taken, reached):
     x = torch.randn(16, 32)
     for w in (torch.randn(8, 28), torch.randn(8, 36), torch.randn(4, 8, 32)):
         with pytest.raises(RuntimeError):
@@ -39,3 +44,14 @@ def test_binding_refuses_sizes_that_do_not_fit_together():
     for w, out in ((torch.randn(8, 28), torch.empty(16, 8)), (torch.randn(8, 32), torch.empty(16, 4)), (torch.randn(32), torch.empty(16, 32))):
         with pytest.raises(ValueError, match="fit together"):
             ops.gemm_f32_dense(x, w, out)
+
+
+def test_tensors_elsewhere_go_to_the_library_product(taken, monkeypatch):
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    x, w = torch.randn(16, 32), torch.randn(8, 32)
+    assert torch.equal(linear32(x, w), x @ w.t())
+    assert torch.equal(linear32(x, w.to_sparse()), x @ w.t())
+    assert not taken
+    cuda, other = (type("T", (), dict(device=torch.device("cuda", i), layout=torch.strided, is_neg=lambda self: False))() for i in (0, 1))
+    assert module._kernel_reaches(cuda, cuda) and not module._kernel_reaches(other, other) and not module._kernel_reaches(cuda, other)
+    assert not module._kernel_reaches(cuda, w)
