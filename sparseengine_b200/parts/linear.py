@@ -12,6 +12,7 @@ is a true 32-bit product.
 from __future__ import annotations
 
 import torch
+from torch.autograd.forward_ad import unpack_dual
 
 from ..csrc import ops
 
@@ -33,6 +34,19 @@ GEMV_MAX_ROWS = 8
 GEMV_GLU_MAX_OUT = 65536       # gate and up rows together
 
 
+def _only_values(*tensors: torch.Tensor) -> bool:
+    """Whether the product's values are all that is asked for.  The kernel is called past torch's dispatcher, so gradients, forward-mode tangents,
+    vmap and torch.func, tracing, dispatch modes, subclasses and autocast would not see it."""
+    if torch._C._len_torch_dispatch_stack() or torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling():
+        return False
+    grad = torch.is_grad_enabled()
+    for t in tensors:
+        if (type(t) not in (torch.Tensor, torch.nn.Parameter) or grad and t.requires_grad or torch._C._functorch.is_functorch_wrapped_tensor(t)
+                or unpack_dual(t).tangent is not None):
+            return False
+    return True
+
+
 def _kernel_reads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None) -> bool:
     """Whether the float32 kernel can read and write these: matrices whose inner sizes agree (the library product refuses what does not
     fit together; the kernel has only pointers), rows on 16-byte boundaries, a whole result."""
@@ -51,8 +65,9 @@ def _kernel_reaches(*tensors: torch.Tensor) -> bool:
 
 def _product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """x . w^T in float32: with this library's kernel where it is estimated to be ahead, else the library product."""
-    if (_kernel_reaches(x, w, *(() if out is None else (out,))) and _kernel_reads(x, w, out) and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
-            and ops.gemm_f32_tc_supported(x.shape[1]) and ops.gemm_f32_dense_pays(x.shape[0], w.shape[0], x.shape[1], ops.sm_count(x.device))):
+    tensors = (x, w) if out is None else (x, w, out)
+    if (_only_values(*tensors) and _kernel_reaches(*tensors) and _kernel_reads(x, w, out) and ops.gemm_f32_tc_supported(x.shape[1])
+            and ops.gemm_f32_dense_pays(x.shape[0], w.shape[0], x.shape[1], ops.sm_count(x.device))):
         if out is None:
             out = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)
         return ops.gemm_f32_dense(x, w, out)

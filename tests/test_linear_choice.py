@@ -55,3 +55,34 @@ def test_tensors_elsewhere_go_to_the_library_product(taken, monkeypatch):
     cuda, other = (type("T", (), dict(device=torch.device("cuda", i), layout=torch.strided, is_neg=lambda self: False))() for i in (0, 1))
     assert module._kernel_reaches(cuda, cuda) and not module._kernel_reaches(other, other) and not module._kernel_reaches(cuda, other)
     assert not module._kernel_reaches(cuda, w)
+
+
+def test_what_sees_the_product_sees_it(taken, reached, monkeypatch):
+    """Gradients, tangents, vmap, torch.func, tracing, dispatch modes, subclasses and autocast: the library product is one that they know."""
+    import torch.autograd.forward_ad as fwd
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils.flop_counter import FlopCounterMode
+    x, w = torch.randn(16, 32), torch.randn(8, 32)
+    want = x @ w.t()
+    with fwd.dual_level():
+        y, tangent = fwd.unpack_dual(linear32(fwd.make_dual(x, 2 * x), w))
+        assert torch.equal(y, want) and torch.equal(tangent, 2 * want)
+    assert torch.allclose(torch.vmap(lambda r: linear32(r, w))(x.expand(3, 16, 32)), want.expand(3, 16, 8))
+    assert torch.allclose(torch.func.jvp(lambda r: linear32(r, w), (x,), (x,))[1], want)
+    assert torch.equal(torch.func.grad(lambda r: linear32(r, w).sum())(x), torch.autograd.functional.jacobian(lambda r: (r @ w.t()).sum(), x))
+    assert torch.equal(make_fx(linear32)(x, w)(2 * x, w), 2 * x @ w.t())
+    assert torch.equal(torch.jit.trace(linear32, (x, w), check_trace=False)(2 * x, w), 2 * x @ w.t())
+    with FlopCounterMode(display=False) as count:
+        linear32(x, w)
+    assert count.get_total_flops() == 2 * 16 * 8 * 32
+    z = x.clone().requires_grad_()
+    assert linear32(z, w).requires_grad and linear32(x, torch.nn.Parameter(w)).requires_grad
+    with monkeypatch.context() as m:            # (autocast itself is off without a GPU)
+        m.setattr(torch, "is_autocast_enabled", lambda kind: kind == "cuda")
+        linear32(x, w)
+    linear32(x.as_subclass(type("Sub", (torch.Tensor,), {})), w)
+    assert not taken
+    with torch.no_grad():
+        linear32(z, torch.nn.Parameter(w))
+    linear32(x, w)
+    assert len(taken) == 2
