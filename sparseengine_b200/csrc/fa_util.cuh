@@ -32,6 +32,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
     for (uint32_t i = 0; i < kSpin && !mbar_try_wait(bar, parity); ++i) {}
 }
+// Warps that share a buffer meet at an mbarrier that counts one arrival each, for the n-th time (from 0) since its start.  A bar.sync would
+// have no bound: after a failed wait elsewhere one warp can give up while another, whose wait was answered in time, waits for it.
+__device__ __forceinline__ bool warps_meet(uint32_t bar, uint32_t n, volatile int* abort_flag) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+    return __all_sync(0xffffffffu, mbar_wait(bar, n & 1, abort_flag));
+}
 // One lane of a converged warp.  What an MMA's issue needs lies in uniform registers; code under a branch that the compiler
 // takes for divergent (lane == 0) moves every operand there for every MMA, about 100 cycles each.  So the issuing warp runs
 // as a whole through warp-uniform loops and only the MMAs are one lane's.

@@ -120,7 +120,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     float* exchange = reinterpret_cast<float*>(smem + kStages * kStageBytes);
     struct Bars {
-        uint64_t full[kStages], empty[kStages], split_full[2], split_empty[2], sum_full[2], sum_empty[2], low_empty, all_done;
+        uint64_t full[kStages], empty[kStages], split_full[2], split_empty[2], sum_full[2], sum_empty[2], low_empty, meet, all_done;
     };
     __shared__ __align__(8) Bars bars;
     __shared__ float route_s[2][kN];
@@ -138,6 +138,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             mbar_init(bar(&bars.sum_empty[b]), 4);
         }
         mbar_init(bar(&bars.low_empty), 4);
+        mbar_init(bar(&bars.meet), 4);
         mbar_init(bar(&bars.all_done), 1);
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -320,12 +321,13 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int quarter = warp & 3, et = threadIdx.x - 384;
         const uint32_t from = tmem + ((uint32_t)(quarter * 32) << 16);
         const int chunks = ceil_div(num_kb, kChunk);
-        int chunk = 0, done = 0;
+        int chunk = 0, done = 0, met = 0;
+        auto meet = [&]() { return ok = fa::warps_meet(bar(&bars.meet), met++, &abort_s); };
         for (int i = blockIdx.x; i < items && ok; i += gridDim.x, ++done) {
             const Item t = item_of<MODE>(p, i, tiles);
             if (MODE == DOWN) {
                 route_s[done & 1][et] = et < t.valid ? p.route_w[p.sorted[t.row0 + et]] : 0.f;
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (!meet()) break;
             }
             float sum[kN];
 #pragma unroll
@@ -368,10 +370,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 const int f = (quarter & 1) * 32 + lane, n = t.n0 + f;
                 float* put = exchange + (up ? 0 : (kN / 2) * 64) + f;
                 const float* get = exchange + (up ? (kN / 2) * 64 : 0) + f;
-                asm volatile("bar.sync 1, 128;" ::: "memory");   // the last item's values have been read
+                if (!meet()) break;                  // the last item's values have been read
 #pragma unroll
                 for (int c = 0; c < kN / 2; ++c) put[c * 64] = up ? sum[c] : sum[kN / 2 + c];
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (!meet()) break;
                 // Eight rows at a time, every value computed and only the stores guarded: row by row behind a branch, an item's epilogue took
                 // 35,000 cycles of its 145,000, and the products wait for it once both sums are full.
                 const int rows = t.valid - (up ? kN / 2 : 0);        // of this thread's half

@@ -1341,25 +1341,25 @@ def gemm_f32_dense_pays(rows: int, n_out: int, k_dim: int, sms: int) -> bool:
     return ours < max(2.0 * (-(-rows // 64) * 64) * n_out * k_dim / 50e6, per_term * k_dim)
 
 
-def gemm_f32_dense(x, w, out):
-    """out = x [rows, k] . w [n, k]^T in 32-bit."""
+def gemm_f32_dense(x, w, out, sms=None):
+    """out = x [rows, k] . w [n, k]^T in 32-bit, on ``sms`` blocks (None: one per SM)."""
     rows, k_dim = x.shape
     if w.dim() != 2 or w.shape[1] != k_dim or out.shape != (rows, w.shape[0]):
         raise ValueError(f"gemm_f32_dense: x {tuple(x.shape)}, w {tuple(w.shape)} and out {tuple(out.shape)} do not fit together")
     _check(_fn("se_gemm_f32_dense", "plppp" "iiii" "p")(
         _rows_ptr(x, "x", torch.float32), x.stride(0), _ptr(w, torch.float32, "w"), _ptr(out, torch.float32, "out"), _ptr(error_word(x.device)),
-        rows, w.shape[0], k_dim, sm_count(x.device), _stream()), "gemm_f32_dense")
+        rows, w.shape[0], k_dim, sms or sm_count(x.device), _stream()), "gemm_f32_dense")
     return out
 
 
-def gemm_f32_grouped(mode: int, a, w, ws: dict, route_w, out, *, experts, max_tiles, n_out, k_dim, activation=None):
-    """The experts' products of the float32 path over rows in expert order; the tile list in ``ws`` must have been built with
-    ``F32_TC_TILE_ROWS`` rows per tile."""
+def gemm_f32_grouped(mode: int, a, w, ws: dict, route_w, out, *, experts, max_tiles, n_out, k_dim, activation=None, sms=None):
+    """The experts' products of the float32 path over rows in expert order, on ``sms`` blocks (None: one per SM); the tile list in
+    ``ws`` must have been built with ``F32_TC_TILE_ROWS`` rows per tile."""
     _check(_fn("se_gemm_f32_grouped", "i" "pp" "ppppp" "ppp" "iiiii" "iff" "ip")(
         mode, _ptr(a, torch.float32, "a"), _ptr(w, torch.float32, "w"), _ptr(ws["sorted"]), _ptr(ws["offsets"]),
         _ptr(ws["tile_expert"]), _ptr(ws["tile_row0"]), _ptr(ws["num_tiles"]), _ptr(route_w, torch.float32, "route_w"),
         _ptr(out, torch.float32, "out"), _ptr(error_word(out.device)), a.shape[0], experts, max_tiles, n_out, k_dim, *_glu_args(activation),
-        sm_count(out.device), _stream()), "gemm_f32_grouped")
+        sms or sm_count(out.device), _stream()), "gemm_f32_grouped")
     return out
 
 

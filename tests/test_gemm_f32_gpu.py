@@ -28,6 +28,24 @@ def test_dense(rows, n, k):
     ops.error_check(DEV)
 
 
+@pytest.mark.parametrize("sms", [1, 2, 3])
+@pytest.mark.parametrize("k", [36, 68, 516, 1100])
+@pytest.mark.parametrize("rows,n", [(191, 700), (150, 1100), (64, 520), (300, 260)])
+def test_dense_item_after_item(rows, n, k, sms):
+    """Few blocks, so that each takes several items in turn: last tiles of 22 to 63 rows after full ones, odd numbers of steps (k 36, 68, 516, 1100: 2, 3,
+    17 and 35) and of sums (1, 2, 9 and 18)."""
+    from sparseengine_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(rows + n + k)
+    x, w = torch.randn(rows, k, generator=g, device=DEV), torch.randn(n, k, generator=g, device=DEV)
+    out = torch.full((rows, n), float("nan"), device=DEV)
+    ops.gemm_f32_dense(x, w, out, sms=sms)
+    assert bool(((out.double() - x.double() @ w.double().t()).abs() <= _bound(x, w)).all())
+    whole = torch.empty_like(out)
+    ops.gemm_f32_dense(x, w, whole)
+    assert torch.equal(out, whole)              # an item's sums do not depend on the items before it
+    ops.error_check(DEV)
+
+
 def test_dense_ends_of_the_range():
     """Infinities, NaN and the largest values come out as multiply-adds leave them."""
     from sparseengine_b200.csrc import ops
@@ -76,6 +94,17 @@ def test_routed_products(counts, hidden, inter, activation):
     # two sums of at most 1,028 products of size one each (results of size one), some 1e-6 off in either order
     assert float((got - want).abs().max()) < 2e-5 * max(1.0, float(want.abs().max()))
     ops.error_check(DEV)
+
+
+@pytest.mark.parametrize("sms", [1, 3])
+def test_routed_products_item_after_item(sms, monkeypatch):
+    """Few blocks: tiles of 1 to 128 rows of an expert in turn, products issued apart and joined, gate and up rows and routing weights of item
+    after item through the same buffers."""
+    from sparseengine_b200.csrc import ops
+    whole = ops.gemm_f32_grouped
+    monkeypatch.setattr(ops, "gemm_f32_grouped", lambda *a, **kw: whole(*a, sms=sms, **kw))
+    test_routed_products([1, 128, 5, 65, 0, 64, 200, 17, 66, 3], 516, 548, None)
+    test_routed_products([300, 5], 640, 1028, ("gelu_tanh", 0.0, 0.0))
 
 
 def test_projections_take_it():
