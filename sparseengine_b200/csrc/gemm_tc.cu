@@ -27,6 +27,7 @@
 // were measured there and gained nothing) times one tile of activation rows, which the NA
 // accumulators share.
 #include "common.cuh"
+#include "fa_util.cuh"
 #include "glu.cuh"
 
 #include <cuda.h>
@@ -198,7 +199,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t stage_bytes = NA * kTileABytes + nt * kBlockK * 2;
-    __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 4 + 2 * kSchedSlots];
+    __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 4 + 2 * kSchedSlots + 1];
     __shared__ __align__(16) uint4 sched_s[kSchedSlots];
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_s;
@@ -208,6 +209,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     const uint32_t acc_full0 = smem_u32(&bars[2 * kMaxStages]), acc_empty0 = smem_u32(&bars[2 * kMaxStages + 2]);
     const uint32_t sched_full0 = smem_u32(&bars[2 * kMaxStages + 4]);
     const uint32_t sched_empty0 = smem_u32(&bars[2 * kMaxStages + 4 + kSchedSlots]);
+    const uint32_t meet = smem_u32(&bars[2 * kMaxStages + 4 + 2 * kSchedSlots]);     // of the epilogue warps (fa_util.cuh)
     const uint32_t sched0 = smem_u32(&sched_s[0]);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -230,6 +232,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             mbar_init(sched_full0 + 8 * q, 1);
             mbar_init(sched_empty0 + 8 * q, 5);     // the MMA thread and the four epilogue warps
         }
+        mbar_init(meet, 4);
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -255,7 +258,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     // role: 0 the loader (it frees nothing), 1 a single thread, 2 a whole warp
     auto next_item = [&](int j, int role) -> bool {
         const int q = j % kSchedSlots;
-        if (!mbar_wait(sched_full0 + 8 * q, (j / kSchedSlots) & 1, &abort_s)) {
+        bool ok = mbar_wait(sched_full0 + 8 * q, (j / kSchedSlots) & 1, &abort_s);
+        if (role == 2) ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
             abort_s = 1;
             atomicCAS(p.error, 0, 5);
             return false;
@@ -444,9 +449,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                 const int valid = min(nt, row_end - row0);
                 if (MODE == MODE_DOWN) {
                     for (int e = et; e < nt; e += 128) route_s[b][e] = e < valid ? p.route_w[p.sorted[row0 + e]] : 0.f;
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
                 }
-                if (!mbar_wait(acc_full0 + 8 * b, (used / bufs) & 1, &abort_s)) {
+                if ((MODE == MODE_DOWN && !fa::warps_meet(meet, used, &abort_s)) ||
+                    !__all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * b, (used / bufs) & 1, &abort_s))) {
                     abort_s = 1;
                     atomicCAS(p.error, 0, 3);
                     break;

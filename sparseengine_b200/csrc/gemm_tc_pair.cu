@@ -26,6 +26,7 @@
 // CTAs of a pair leave together.  Arithmetic and rounding points are those of gemm_tc.cu
 // (src/sparseengine/kernels/triton/moe.py:557-563,726-732,1374-1440).
 #include "common.cuh"
+#include "fa_util.cuh"
 #include "glu.cuh"
 
 #include <cuda.h>
@@ -168,7 +169,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t bars[2 * kStages + 4];
+    __shared__ __align__(8) uint64_t bars[2 * kStages + 5];
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_s;
     __shared__ float route_s[2][kTileN];
@@ -176,6 +177,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     __shared__ __align__(16) __nv_bfloat16 xch_s[2][2][kXchCols][MODE == MODE_GATE_UP ? kCtaFeatures : 1];
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kStages]);
     const uint32_t acc_full0 = smem_u32(&bars[2 * kStages]), acc_empty0 = smem_u32(&bars[2 * kStages + 2]);
+    const uint32_t meet = smem_u32(&bars[2 * kStages + 4]);      // of this CTA's epilogue warps (fa_util.cuh)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -187,6 +189,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             mbar_init(acc_full0 + 8 * b, 1);      // the pair's MMA commit
             mbar_init(acc_empty0 + 8 * b, 8);     // four epilogue warps of each CTA (used in the leader)
         }
+        mbar_init(meet, 4);
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -295,13 +298,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             const int b = used & 1;
             if (MODE == MODE_DOWN) {
                 for (int e = et; e < kTileN; e += 128) route_s[b][e] = e < valid ? p.route_w[p.sorted[row0 + e]] : 0.f;
-                asm volatile("bar.sync 1, 128;" ::: "memory");
             }
-            if (!mbar_wait(acc_full0 + 8 * b, (used >> 1) & 1, &abort_s)) {
-                abort_s = 1;
-                atomicCAS(p.error, 0, 3);
-                break;
-            }
+            bool ok = MODE != MODE_DOWN || fa::warps_meet(meet, used, &abort_s);
+            ok = ok && __all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * b, (used >> 1) & 1, &abort_s));
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * kTileN);
             if (MODE == MODE_GATE_UP) {
@@ -314,15 +313,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 const int n = nb * kItemFeatures + (int)rank * kCtaFeatures + f;
                 const int j0 = is_up ? kXchCols / 2 : 0;                     // this thread's columns of a chunk
                 // `chunk` runs on across items: the two exchange buffers alternate without a gap
-                for (int c0 = 0; c0 < valid; c0 += kXchCols, ++chunk) {      // uniform over the 128 threads
+                for (int c0 = 0; c0 < valid && ok; c0 += kXchCols, ++chunk) {        // uniform over the 128 threads
                     uint32_t v[32];
                     tmem_ld32(taddr + c0, v);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     auto mine = xch_s[chunk & 1][is_up ? 1 : 0];
 #pragma unroll
                     for (int j = 0; j < kXchCols; ++j) mine[j][f] = __float2bfloat16_rn(__uint_as_float(v[j]));
-                    asm volatile("bar.sync 1, 128;" ::: "memory");           // both halves of this chunk are there
-                    if (n < p.n_out) {
+                    ok = fa::warps_meet(meet, chunk, &abort_s);              // both halves of this chunk are there
+                    if (ok && n < p.n_out) {
                         const auto gs = xch_s[chunk & 1][0];
                         const auto us = xch_s[chunk & 1][1];
 #pragma unroll
@@ -346,7 +345,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 }
             } else {
                 const int n = nb * kItemFeatures + (int)rank * kCtaFeatures + et;
-                for (int c0 = 0; c0 < valid; c0 += 32) {
+                for (int c0 = 0; c0 < valid && ok; c0 += 32) {
                     uint32_t v[32];
                     tmem_ld32(taddr + c0, v);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -359,6 +358,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                         }
                     }
                 }
+            }
+            if (!ok) {
+                abort_s = 1;
+                atomicCAS(p.error, 0, 3);
+                break;
             }
             // this warp has read its lanes of buffer b: tell the leader's MMA thread
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
