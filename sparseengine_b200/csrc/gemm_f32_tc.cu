@@ -299,7 +299,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 fa::tmem_st32(to, hi);
                 fa::tmem_st32(to + kK, lo);
-                if (__any_sync(0xffffffffu, !isfinite((rest[0] + rest[1]) + (rest[2] + rest[3]))))
+                if (__any_sync(0xffffffffu, !isfinite((rest[0] + rest[1]) + (rest[2] + rest[3])))) {
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");         // stores to one place have no order of their own
 #pragma unroll 1
                     for (int j = 0; j < kK; ++j) {               // a value without a finite nearest tf32 value: cut off, or kept as it is
                         const uint32_t v = lds4(tile + sw128(row, j / 4) + (j & 3) * 4), h = (v + 0x1000u) & 0xffffe000u;
@@ -309,6 +310,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(to + j), "r"(upper) : "memory");
                         asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(to + kK + j), "r"(rest_of) : "memory");
                     }
+                }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
