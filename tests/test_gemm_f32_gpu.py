@@ -67,6 +67,23 @@ def test_dense_ends_of_the_range():
     ops.error_check(DEV)
 
 
+def test_dense_nan_of_any_bits():
+    """A NaN may have its set bits among those that the tensor cores cut off, or be negative, in an activation and in a weight."""
+    from sparseengine_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(2)
+    x, w = torch.randn(140, 256, generator=g, device=DEV), torch.randn(300, 256, generator=g, device=DEV)
+    bits = torch.tensor([0x7f800001, 0x7f801fff, 0x7fffffff, -0x7fffff], dtype=torch.int32, device=DEV).view(torch.float32)     # the last: 0xff800001
+    x[torch.tensor([2, 40, 77, 139]), torch.tensor([0, 31, 32, 255])] = bits
+    w[torch.tensor([0, 64, 130, 299]), torch.tensor([255, 3, 64, 31])] = bits
+    out = torch.empty(140, 300, device=DEV)
+    ops.gemm_f32_dense(x, w, out)
+    want = x.double() @ w.double().t()
+    assert torch.equal(out.isnan(), want.isnan()) and not bool(out.isinf().any())
+    finite = ~want.isnan()
+    assert bool(((out.double() - want).abs() <= _bound(x, w))[finite].all())
+    ops.error_check(DEV)
+
+
 @pytest.mark.parametrize("activation", [None, ("clamped_swiglu", 2.0, 1.3), ("gelu_tanh", 0.0, 0.0)], ids=["silu", "clamped", "gelu"])
 @pytest.mark.parametrize("counts,hidden,inter", [([127, 128, 129, 0, 1, 31, 33, 97], 512, 516), ([300, 5], 640, 1028), ([64, 63, 65], 1024, 512)])
 def test_routed_products(counts, hidden, inter, activation):
