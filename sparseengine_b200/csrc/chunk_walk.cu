@@ -50,54 +50,54 @@ ssm_prepare_kernel(const float* __restrict__ xbc, const T_* __restrict__ proj, i
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float* const x[1] = {qs};
     triangle_products<DP, 1>(x, ks, warp, lane, [&](const auto& acc, int r0, int n0, int zeros) {
-    constexpr int NT = sizeof(acc[0]) / sizeof(acc[0][0]);
-    for (int h0 = 0; h0 < rep; h0 += 8) {
-        __syncthreads();                             // the sums of the eight heads before have been read
-        if (h0 + warp < rep) {                       // a warp per head, two neighbouring tokens per lane
-            const int h = g * rep + h0 + warp;
-            const float rate = expf(a_log[h]), bias = dt_bias[h];
-            float step[2];
-            double sum[2];
+        constexpr int NT = sizeof(acc[0]) / sizeof(acc[0][0]);
+        for (int h0 = 0; h0 < rep; h0 += 8) {
+            roles_sync<kThreads>();                  // the sums of the eight heads before have been read
+            if (h0 + warp < rep) {                   // a warp per head, two neighbouring tokens per lane
+                const int h = g * rep + h0 + warp;
+                const float rate = expf(a_log[h]), bias = dt_bias[h];
+                float step[2];
+                double sum[2];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int t = 2 * lane + j;
-                step[j] = t < n ? softplus32(to_float(proj[(size_t)(first + t) * pitch + dt_off + h]) + bias) : 0.f;
-                sum[j] = (t < n ? log_decay(rate, step[j]) : 0.0) + (j ? sum[0] : 0.0);
+                for (int j = 0; j < 2; ++j) {
+                    const int t = 2 * lane + j;
+                    step[j] = t < n ? softplus32(to_float(proj[(size_t)(first + t) * pitch + dt_off + h]) + bias) : 0.f;
+                    sum[j] = (t < n ? log_decay(rate, step[j]) : 0.0) + (j ? sum[0] : 0.0);
+                }
+                double before;
+                const double last = sum_before(sum[1], lane, before);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int t = 2 * lane + j;
+                    const double b = before + sum[j];
+                    sums[warp][t] = b;
+                    if (t < n) {
+                        const size_t at = (size_t)(first + t) * H + h;
+                        rs[at] = expf((float)b);
+                        ts[at] = expf((float)(last - b));
+                        steps[at] = step[j];
+                    }
+                }
             }
-            double before;
-            const double last = sum_before(sum[1], lane, before);
+            roles_sync<kThreads>();
+            for (int hh = 0; hh < min(8, rep - h0); ++hh) {
+                const int h = g * rep + h0 + hh;
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int t = 2 * lane + j;
-                const double b = before + sum[j];
-                sums[warp][t] = b;
-                if (t < n) {
-                    const size_t at = (size_t)(first + t) * H + h;
-                    rs[at] = expf((float)b);
-                    ts[at] = expf((float)(last - b));
-                    steps[at] = step[j];
+                for (int j = 0; j < 4; j += 2) {
+                    const int t = r0 + 4 * j;
+                    if (t >= n) continue;
+                    const double bt = sums[hh][t];
+                    float* row = p + ((size_t)(first + t) * H + h) * T;
+#pragma unroll
+                    for (int x = 0; x < NT; ++x) {
+                        const int s = n0 + 8 * x;
+                        *reinterpret_cast<float2*>(row + s) = make_float2(s <= t ? acc[0][x][j] * expf((float)(bt - sums[hh][s])) : 0.f,
+                                                                          s < t ? acc[0][x][j + 1] * expf((float)(bt - sums[hh][s + 1])) : 0.f);
+                    }
+                    for (int s = zeros; s < T; s += 16) *reinterpret_cast<float2*>(row + s) = make_float2(0.f, 0.f);
                 }
             }
         }
-        __syncthreads();
-        for (int hh = 0; hh < min(8, rep - h0); ++hh) {
-            const int h = g * rep + h0 + hh;
-#pragma unroll
-            for (int j = 0; j < 4; j += 2) {
-                const int t = r0 + 4 * j;
-                if (t >= n) continue;
-                const double bt = sums[hh][t];
-                float* row = p + ((size_t)(first + t) * H + h) * T;
-#pragma unroll
-                for (int x = 0; x < NT; ++x) {
-                    const int s = n0 + 8 * x;
-                    *reinterpret_cast<float2*>(row + s) = make_float2(s <= t ? acc[0][x][j] * expf((float)(bt - sums[hh][s])) : 0.f,
-                                                                      s < t ? acc[0][x][j + 1] * expf((float)(bt - sums[hh][s + 1])) : 0.f);
-                }
-                for (int s = zeros; s < T; s += 16) *reinterpret_cast<float2*>(row + s) = make_float2(0.f, 0.f);
-            }
-        }
-    }
     });
 }
 

@@ -61,6 +61,10 @@ __device__ __forceinline__ float2 load2(const __nv_bfloat16* p) { return __bfloa
 
 __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory"); }
 
+// A meeting of `THREADS` threads whose warps come from different places in the code (roles, branches that a whole warp takes): the numbered barrier counts
+// arrivals from wherever they come, which __syncthreads() does not promise.
+template <int THREADS> __device__ __forceinline__ void roles_sync() { asm volatile("bar.sync 5, %0;" ::"n"(THREADS) : "memory"); }
+
 // the entry that owns place `slot` among the step's chunks, and the chunk's first token and length (0: nobody's place)
 template <int T>
 __device__ __forceinline__ int chunk_of(int slot, const int* cu_q, int entries, int& first, int& n) {
@@ -383,7 +387,7 @@ chunk_walk_kernel(const WalkArgs a) {
                     cp_commit();
                     cp_wait<1>();                    // the next q and k
                 }
-                __syncthreads();
+                roles_sync<kThreads>();
             }
         } else {
         if (LOADER) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");        // 128 x (2 x 208 + 88): what 384 threads of 168 have
@@ -447,7 +451,7 @@ chunk_walk_kernel(const WalkArgs a) {
                 if (!LOADER && next < t_last) put_values(cur ^ 1);
                 cp_wait<0>();                        // the next k
             }
-            __syncthreads();
+            roles_sync<kThreads>();
         }
         }
         last_state = Ss + cur * DP * CP;
@@ -509,7 +513,7 @@ chunk_walk_kernel(const WalkArgs a) {
             for (int t0 = t_first; t0 < t_last; t0 += T, cur ^= 1) {
                 const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
                 cp_wait<0>();                        // W and q
-                __syncthreads();                     // k and P of the chunk before have been read
+                roles_sync<kThreads>();              // k and P of the chunk before have been read
                 if (t0 > t_first) {
                     load_k(ks, t0, n);
                     load_p(t0, n);
@@ -521,14 +525,14 @@ chunk_walk_kernel(const WalkArgs a) {
                 }
                 cp_commit();
                 cp_wait<1>();
-                __syncthreads();
+                roles_sync<kThreads>();
             }
         } else {
         if (LOADER) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");        // 128 x (2 x 208 + 88): what 384 threads of 168 have
         for (int t0 = t_first; t0 < t_last; t0 += T, cur ^= LOADER) {
             const int n = min(T, t_last - t0), next = t0 + T, next_n = min(T, t_last - next);
             cp_wait<1>();                            // W or q (k and P may still be on their way)
-            __syncthreads();                         // and the state is up to date
+            roles_sync<kThreads>();                  // and the state is up to date
             float acc[1][NT][4];
             state_product((group == 0 ? ws : qs) + cur * T * QP, Ss, acc);
             if (group == 0) {
@@ -543,7 +547,7 @@ chunk_walk_kernel(const WalkArgs a) {
                     }
             }
             cp_wait<0>();
-            __syncthreads();                         // u, k and P are there, W, q and the state have been read
+            roles_sync<kThreads>();                  // u, k and P are there, W, q and the state have been read
             if (group == 0) {
                 if (next < t_last) {
                     if (!LOADER) load_w(next, next_n);
