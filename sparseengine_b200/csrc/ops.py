@@ -610,7 +610,7 @@ def latent_takes_heads(max_q_len: int, heads: int, rank: int, sms: int, q_lens, 
         last = max(last, most)
     formed = 8 + 1.2 / 64 * max(last, -(-blocks // sms) * keys / blocks) + 12 + total * heads * (rank * 256 / 7e8 + 512 / 5e6)
     tc, tiled = latent_times(len(q_lens), max_q_len, heads, rank, sms, q_lens, kv_lens, window)
-    if not max_q_len * heads >= 128:
+    if not latent_attention_tc_supported(rank, 64) or max_q_len * heads < 128:          # as latent_takes_tc: the tiled kernel runs then
         tc = tiled
     return formed < min(tc, tiled) + 6 + tokens * heads * rank * 8 / 5e6
 

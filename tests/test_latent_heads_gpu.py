@@ -66,3 +66,12 @@ def test_choice():
     assert take([8192], [8192], 1024) and take([1000], [5000]) and take([500] * 4, [1000] * 4, 1024, 64)
     assert not take([1] * 64, [3000] * 64) and not take([31], [31])            # single tokens: the expansion is never paid back
     assert not take([64], [200000], None, 64)                                 # the keys and values would take more than their bound
+
+
+def test_choice_compares_with_the_kernel_that_would_run():
+    """A latent of 176 is not for the tcgen05 kernel, whose estimate kept steps from the keys per head though the tiled kernel would have run."""
+    from sparseengine_b200.csrc import ops
+    assert ops.latent_attention_tiled_supported(176, 64) and not ops.latent_attention_tc_supported(176, 64)
+    take = lambda q, kv, window=None, heads=16, rank=176: ops.latent_takes_heads(max(q), heads, rank, 148, q, kv, window)
+    assert take([64] * 4, [1064] * 4, 1024) and take([100], [100]) and not take([64] * 4, [1064] * 4, 1024, rank=192)
+    assert not take([32], [32], heads=2)
