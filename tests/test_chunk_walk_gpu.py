@@ -40,15 +40,17 @@ def _close(got, want, what):
     assert worst < BOUND * most, f"{what}: {worst:.3e} of {most:.3e}"
 
 
-SIZES = [(128, 128, 3, 3), (64, 64, 4, 2), (8, 4, 2, 1), (100, 36, 3, 3), (128, 20, 40, 10), (44, 132, 2, 2), (32, 12, 2, 2)]
+# the last: 32 value columns a block with up to 64 rows
+SIZES = [(128, 128, 3, 3), (64, 64, 4, 2), (8, 4, 2, 1), (100, 36, 3, 3), (128, 20, 40, 10), (44, 132, 2, 2), (32, 12, 2, 2), (64, 64, 8, 4)]
 
 
 @pytest.mark.parametrize("decay", ["slow", "fast"])
 @pytest.mark.parametrize("d,dv,heads,kv_heads", SIZES)
-@pytest.mark.parametrize("kind", ["retention", "state space", "delta, per head", "delta, per channel", "state space, tokens", "delta, tokens"])
+@pytest.mark.parametrize("kind", ["retention", "retention, 16-bit values", "state space", "delta, per head", "delta, per channel", "state space, tokens",
+                                  "delta, tokens"])
 def test_chunks_against_the_walk(kind, d, dv, heads, kv_heads, decay):
     """``fast``: decays down to e^-30 per token, whose products underflow within a chunk.  ``tokens``: the kernels that walk token
-    by token, on the same inputs."""
+    by token, on the same inputs.  ``16-bit values``: as the projection leaves them, whose products need no lower term; with an activation they do."""
     from sparseengine_b200.csrc import ops
     tokens = kind.endswith("tokens")
     step = _step([3, 0, 11, 1, 7, 2, 5, 4, 9, 6])
@@ -63,9 +65,10 @@ def test_chunks_against_the_walk(kind, d, dv, heads, kv_heads, decay):
     o = torch.full((T, heads, dv), float("nan"), device=DEV)
     rep = heads // kv_heads
     sizes = dict(heads=heads, head_dim=d, v_head_dim=dv)
-    column_major = kind != "retention"          # [head][column][row], retention [head][row][column]
+    column_major = not kind.startswith("retention")          # [head][column][row], retention [head][row][column]
     skip = None
-    if kind == "retention":
+    if not column_major:
+        silu = kind == "retention"
         # columns: 4 that nobody reads, k, values, q; rotated where the head size allows the pairs
         wide, rot = heads * (2 * d + dv) + 8, 16 if d >= 16 else 0
         proj, decays = rnd(T, wide + -wide % 4).to(torch.bfloat16), torch.exp(logs[0, :, 0])
@@ -73,9 +76,9 @@ def test_chunks_against_the_walk(kind, d, dv, heads, kv_heads, decay):
         v_off = 4 + heads * d
         q_off = v_off + heads * dv
         assert ops.retention_walk_supported(d, dv, rot, proj, q_off, 4, v_off)
-        ops.retention_chunk(None, None, proj, v_off, decays, state, step, o.view(T, -1), silu=True, **sizes,
+        ops.retention_chunk(None, None, proj, v_off, decays, state, step, o.view(T, -1), silu=silu, **sizes,
                             qk=(q_off, 4, d ** -0.5), rotation=(inv, rot, positions) if rot else None)
-        x = torch.nn.functional.silu(proj.double())
+        x = torch.nn.functional.silu(proj.double()) if silu else proj.double()
         q, k = (x[:, f:f + heads * d].reshape(T, heads, d).clone() for f in (q_off, 4))
         angle = (positions.float()[:, None] * inv).double()[:, None]        # the product in 32-bit, as positions are encoded
         for z in (q, k):
@@ -176,8 +179,9 @@ def _outputs(kind, x, H, d, tokens=False, one_kernel=False):
     if kind == "state space":
         (ops.ssm_scan if tokens else ops.ssm_walk)(x["qkv"], x["decay"], 0, x["bias"], x["a_log"], x["skip"], state, step, o, heads=H,
                                                    head_dim=d, state_size=d, groups=H)
-    elif kind == "retention":
-        ops.retention_chunk(None, None, x["qkv"], 2 * H * d, torch.full((H,), 0.9, device=DEV), state, step, o, heads=H, head_dim=d,
+    elif kind.startswith("retention"):
+        qkv = x["qkv"].to(torch.bfloat16) if kind.endswith("16-bit values") else x["qkv"]
+        ops.retention_chunk(None, None, qkv, 2 * H * d, torch.full((H,), 0.9, device=DEV), state, step, o, heads=H, head_dim=d,
                             v_head_dim=d, qk=(0, H * d, 1.0))
     else:
         sizes = dict(heads=H, kv_heads=H, head_dim=d, v_head_dim=d)
@@ -198,9 +202,9 @@ def _outputs(kind, x, H, d, tokens=False, one_kernel=False):
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
 @pytest.mark.parametrize("token", [40, 41, 63])         # the first and the second of a pair of tokens, the last of a chunk
 @pytest.mark.parametrize("where", ["q", "k", "v", "decay"])
-@pytest.mark.parametrize("kind", ["state space", "delta, per head", "delta, per channel", "retention"])
+@pytest.mark.parametrize("kind", ["state space", "delta, per head", "delta, per channel", "retention", "retention, 16-bit values"])
 def test_inputs_that_are_not_finite_stay_with_their_token_and_later_ones(kind, where, token, value):
-    if kind == "retention" and where == "decay":
+    if kind.startswith("retention") and where == "decay":
         pytest.skip("its decays are constants")
     H, d, T = 2, 64, 70
     x, places = _inputs(kind, T, H, d)
