@@ -152,9 +152,11 @@ class LatentAttention(Mixer):
 
     def takes_heads(self, step, device):
         """``ops.latent_takes_heads`` over the step's own entries, asked once per step for all layers of the same sizes: how many cached
-        rows the entries see, and the most that one sees, or None.  Steps that are captured know bounds only."""
+        rows the entries see, and the most that one sees, or None.  Those numbers size the workspace, so steps that are captured, which may be
+        replayed with other lengths on the device, stay in the latent's space, whose kernels read the lengths there alone."""
         s = self.spec
-        if (s.head_dim, s.rot_dim, s.v_head_dim) != (64, 64, 64) or s.kv_rank % 8 or step.max_kv_bound is not None or not step.q_lens:
+        if ((s.head_dim, s.rot_dim, s.v_head_dim) != (64, 64, 64) or s.kv_rank % 8 or step.max_kv_bound is not None or not step.q_lens
+                or torch.cuda.is_initialized() and torch.cuda.is_current_stream_capturing()):
             return None
 
         def ask():

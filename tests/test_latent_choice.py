@@ -42,3 +42,21 @@ def test_asked_once_per_step():
         assert part.takes_tc(step, "cuda:0") and asked[1] == [64, 64]
     finally:
         ops.latent_takes_tc, ops.sm_count = before, count
+
+
+def test_captured_steps_stay_in_the_latent_space(monkeypatch):
+    """Keys per head take a workspace for the lengths that the host knows, a replayed graph may meet others: also where the same step has
+    run before."""
+    from sparseengine_b200.config.specs import LatentAttentionSpec
+    from sparseengine_b200.parts.base import make_mixer
+    import torch
+    part = make_mixer(LatentAttentionSpec(hidden_size=64, num_heads=32, head_dim=64, rot_dim=64, v_head_dim=64, q_rank=16, kv_rank=192,
+                                          scale=0.1, position=None), torch.bfloat16)
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    step = SimpleNamespace(num_seqs=1, max_q_len=2048, q_lens=[2048], kv_lens=[2500], max_kv_bound=None, extras={})
+    assert part.takes_heads(step, "cuda:0") == (2500, 2500)
+    monkeypatch.setattr(torch.cuda, "is_initialized", lambda: True)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    assert part.takes_heads(step, "cuda:0") is None
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    assert part.takes_heads(step, "cuda:0") == (2500, 2500)

@@ -59,6 +59,64 @@ def test_against_64_bits(heads, window, sinks):
         assert torch.equal(run(dirty, wrong), out)
 
 
+def _mixer_step(lens, held, pages_per=None):
+    from sparseengine_b200.parts.base import StepContext
+    n, total, cu = len(lens), sum(lens), [0]
+    for t in lens:
+        cu.append(cu[-1] + t)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    kv = [h + t for h, t in zip(held, lens)]
+    return StepContext(num_tokens=total, num_seqs=n, token_ids=torch.zeros(total, **i32),
+                       positions=torch.tensor([h + i for h, t in zip(held, lens) for i in range(t)], **i32),
+                       token_seq=torch.tensor([j for j, t in enumerate(lens) for _ in range(t)], **i32),
+                       seq_rows=torch.arange(n, **i32), cu_q=torch.tensor(cu, **i32), kv_len=torch.tensor(kv, **i32), q_lens=list(lens),
+                       q_starts=list(held), kv_lens=kv, rows=list(range(n)), dtype=torch.bfloat16)
+
+
+def _mixer(**options):
+    from sparseengine_b200.config.specs import LatentAttentionSpec, RotarySpec
+    from sparseengine_b200.parts.base import make_mixer
+    part = make_mixer(LatentAttentionSpec(**dict(dict(hidden_size=256, num_heads=4, head_dim=64, rot_dim=64, v_head_dim=64, q_rank=128, kv_rank=192,
+                                                      scale=128 ** -0.5, sink=True, position=RotarySpec(rotary_dim=64, theta=1e4)), **options)), torch.bfloat16)
+    g = torch.Generator(device=DEV).manual_seed(3)
+    part.bind({n: (torch.randn(p.shape, generator=g, device=DEV) * (0.5 if "sink" in n else 0.06) + float("norm" in n)).to(
+        torch.float32 if p.dtype == "float32" else torch.bfloat16) for n, p in part.parameters().items()})
+    return part
+
+
+@pytest.mark.gpu
+def test_captured_portion_replayed_with_other_lengths(monkeypatch):
+    """A graph of a prompt portion is replayed behind more held keys than it was captured with."""
+    from sparseengine_b200.csrc import ops
+    from sparseengine_b200.parts.base import LayerSlot
+    monkeypatch.setattr(ops, "latent_takes_heads", lambda *a, **k: True)
+    part, lens = _mixer(), [70]
+    g = torch.Generator(device=DEV).manual_seed(4)
+    x = torch.randn(70, 256, generator=g, device=DEV).to(torch.bfloat16)
+    cache = torch.randn(80, 16, 256, generator=g, device=DEV).to(torch.bfloat16)
+    slot = LayerSlot(kv=cache, table=torch.randperm(80, generator=torch.Generator().manual_seed(5)).to(torch.int32).view(1, 80).to(DEV), page_size=16)
+    step, later = _mixer_step(lens, [30]), _mixer_step(lens, [1000])
+    before = ops.calls.get("se_latent_gather", 0)
+    part.forward(x, step, slot)
+    want = part.forward(x, later, slot).clone()
+    assert ops.calls.get("se_latent_gather", 0) == before + 2
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        part.forward(x, step, slot)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = part.forward(x, step, slot)
+    step.positions.copy_(later.positions)
+    step.kv_len.copy_(later.kv_len)
+    graph.replay()
+    torch.cuda.synchronize()
+    ops.error_check(DEV)
+    # two forms of the same attention, each with 16-bit weights and intermediate vectors
+    assert float((out.double() - want.double()).norm()) < 2e-2 * float(want.double().norm())
+
+
 def test_choice():
     from sparseengine_b200.csrc import ops
     assert ops.latent_seen_keys([5, 1, 8], [5, 90, 20], 10) == [5, 10, 17] and ops.latent_seen_keys([5], [90], None) == [90]
