@@ -78,7 +78,7 @@ struct Parts {
     const __nv_bfloat16* kv;       // [rows][kv_pitch]: heads' 64 key dims, from v_off on their 64 value dims
     int kv_pitch, v_off;
     const __nv_bfloat16* rot;      // [rows][rot_pitch]: the shared 64 rotated dims
-    int rot_pitch;
+    int rot_pitch, rows;
 };
 
 // The n lowest bits (none below 0, all from 32 on).
@@ -201,7 +201,7 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
             const bool first = tile < kept_tiles;
             const int base = first ? tile * kKeys : k_begin + (tile - kept_tiles) * kKeys;
             const int k_lo = first ? 0 : k_lo_window, k_end = first ? kept : k_end_window;      // the keys of this tile that are read
-            if constexpr (PARTS) {                   // zero-filled outside [k_lo, k_end), as below
+            if constexpr (PARTS) {                   // zero-filled outside [k_lo, k_end), as below, and beyond the last row
                 const int c = lane & 7;
                 const size_t row0 = (size_t)(rows_before + base);
                 const __nv_bfloat16* kv = parts.kv + kvh * 64 + c * 8;
@@ -209,7 +209,7 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
 #pragma unroll 4
                 for (int k = 0; k < kKeys / 4; ++k) {
                     const int r = 4 * k + (lane >> 3);
-                    const bool ok = base + r < k_end && base + r >= k_lo;
+                    const bool ok = base + r < k_end && base + r >= k_lo && rows_before + base + r < parts.rows;
                     const size_t row = ok ? row0 + r : 0;
                     const uint32_t off = sw128(r, c);
                     cp_async16(smem_u32(st) + off, kv + row * parts.kv_pitch, ok);
@@ -546,7 +546,7 @@ extern "C" int se_attn_prefill_tc(const void* q, const void* cache, const int* t
 // Latent attention over keys and values formed per head: heads of 64 unrotated and 64 rotated dims (q's rows: heads x 128, already
 // rotated), values of 64 (the pointers as struct Parts has them); out [tokens][heads][64].  window: 0 none, else the keys a token sees.
 extern "C" int se_attn_prefill_tc_parts(const void* q, int q_pitch, const void* kv, int kv_pitch, int v_off, const void* rot,
-                                        int rot_pitch, const int* cu_q, const int* kv_len, const float* sink_logits, void* out,
+                                        int rot_pitch, int rows, const int* cu_q, const int* kv_len, const float* sink_logits, void* out,
                                         int* error, int entries, int max_q_len, int heads, float scale, int window, cudaStream_t stream) {
     using namespace se::fa;
     if (entries <= 0 || max_q_len <= 0) return 0;
@@ -555,7 +555,7 @@ extern "C" int se_attn_prefill_tc_parts(const void* q, int q_pitch, const void* 
     for (const void* x : {q, kv, rot, (const void*)out})
         if (reinterpret_cast<uintptr_t>(x) & 15) return SE_ERR_UNSUPPORTED;
     const se::mma::SoftmaxOptions opt{0.f, 0.f, sink_logits != nullptr, nullptr, 0, sink_logits, 0, nullptr, 1.f / scale, 0};
-    const Parts parts{q_pitch, (const __nv_bfloat16*)kv, kv_pitch, v_off, (const __nv_bfloat16*)rot, rot_pitch};
+    const Parts parts{q_pitch, (const __nv_bfloat16*)kv, kv_pitch, v_off, (const __nv_bfloat16*)rot, rot_pitch, rows};
     const size_t smem = (size_t)kTiles * kQBytes + kStages * kKVStageBytes + 1024;
     const cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;

@@ -129,6 +129,7 @@ __host__ __device__ __forceinline__ int first_visible(int pos, int window) {
 #define SE_CODE_BAD_TABLE_UPDATE 26
 // 27 to 29: the latent preparation and the two older latent attention kernels (latent_attention.cu)
 #define SE_CODE_BAD_PAGE_LATENT_TC 30
+#define SE_CODE_LATENT_ROWS 31       // an entry sees more cached rows than the workspace was made for
 
 // True if block-table entry `page` names a page of a pool of `num_pages`; otherwise the code
 // goes to the error word (if there is one) and the caller leaves the page alone.

@@ -390,8 +390,8 @@ static EncodeTiledFn encode_fn() {
 // between them: what a product that forms keys and values per head reads.  A warp per row, blocks of 32 rows.
 __global__ void __launch_bounds__(256)
 latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ table, int table_stride, const int* __restrict__ seq_rows,
-                     const int* __restrict__ cu_q, const int* __restrict__ kv_len, __nv_bfloat16* __restrict__ out, int row,
-                     int page_size, int window, int num_pages, int* error) {
+                     const int* __restrict__ cu_q, const int* __restrict__ kv_len, __nv_bfloat16* __restrict__ out, int rows,
+                     int row, int page_size, int window, int num_pages, int* error) {
     __shared__ int sums[8];
     const int e = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto first_of = [&](int x) { return first_visible(kv_len[x] - (cu_q[x + 1] - cu_q[x]), window); };
@@ -404,8 +404,10 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restr
 #pragma unroll
     for (int x = 0; x < 8; ++x) before += sums[x];
     const int first = first_of(e), n = kv_len[e] - first;
+    // the workspace is as large as the lengths that the host knows: beyond its end, or beyond the grid's, nothing is written
+    if (threadIdx.x == 0 && blockIdx.x == 0 && (before + n > rows || n > (int)gridDim.x * 32)) atomicCAS(error, 0, SE_CODE_LATENT_ROWS);
     const int* pages = table + (size_t)seq_rows[e] * table_stride;
-    for (int i = blockIdx.x * 32 + warp; i < min(n, (int)(blockIdx.x + 1) * 32); i += 8) {
+    for (int i = blockIdx.x * 32 + warp; i < min(min(n, rows - before), (int)(blockIdx.x + 1) * 32); i += 8) {
         const int j = first + i, page = pages[j / page_size];
         const bool there = page_in_pool(page, num_pages, error, SE_CODE_BAD_PAGE_LATENT_TC);
         const __nv_bfloat16* src = cache + ((size_t)(there ? page : 0) * page_size + j % page_size) * row;
@@ -455,14 +457,15 @@ extern "C" int se_latent_attention_tc(const void* qfull, const void* cache, cons
     return (int)cudaGetLastError();
 }
 
-// out [rows][row]: the cached rows (row elements, a multiple of 8) that the entries see; most_keys: the most that one entry sees.
+// out [rows][row]: the cached rows (row elements, a multiple of 8) that the entries see; most_keys: the most that one entry sees.  Lengths on the device that
+// go beyond either leave a code in the error word.
 extern "C" int se_latent_gather(const void* cache, const int* table, int table_stride, const int* seq_rows, const int* cu_q, const int* kv_len,
-                                void* out, int* error, int entries, int most_keys, int row, int page_size, int window, int num_pages,
-                                cudaStream_t stream) {
+                                void* out, int* error, int entries, int most_keys, int rows, int row, int page_size, int window,
+                                int num_pages, cudaStream_t stream) {
     if (entries <= 0 || most_keys <= 0) return 0;
-    if (row <= 0 || row % 8 || page_size <= 0 || entries > 65535 || ((reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) & 15))
+    if (rows < 0 || row <= 0 || row % 8 || page_size <= 0 || entries > 65535 || ((reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) & 15))
         return SE_ERR_UNSUPPORTED;
     se::lat_tc::latent_gather_kernel<<<dim3(se::ceil_div(most_keys, 32), entries), 256, 0, stream>>>(
-        (const __nv_bfloat16*)cache, table, table_stride, seq_rows, cu_q, kv_len, (__nv_bfloat16*)out, row, page_size, window, num_pages, error);
+        (const __nv_bfloat16*)cache, table, table_stride, seq_rows, cu_q, kv_len, (__nv_bfloat16*)out, rows, row, page_size, window, num_pages, error);
     SE_LAUNCH_CHECK();
 }

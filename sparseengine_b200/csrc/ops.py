@@ -623,16 +623,16 @@ def latent_attention_heads(q, cache, table, seq_rows, cu_q, kv_len, sink, uk, uv
     dev, bf16, row, n = q.device, torch.bfloat16, cache.shape[-1], heads * 64
     work = torch.empty(rows * (row + 2 * n), dtype=bf16, device=dev)          # the rows, keys, values
     lat, error, cu, kv = work.data_ptr(), _ptr(error_word(dev)), _ptr(cu_q, torch.int32, "cu_q"), _ptr(kv_len, torch.int32, "kv_len")
-    _check(_fn("se_latent_gather", "ppi" "ppp" "pp" "iiiiii" "p")(
+    _check(_fn("se_latent_gather", "ppi" "ppp" "pp" "iiiiiii" "p")(
         _ptr(cache, bf16, "cache"), _ptr(table, torch.int32, "table"), table.shape[1], _ptr(seq_rows, torch.int32, "seq_rows"), cu, kv, lat,
-        error, entries, most_keys, row, page_size, int(window or 0), cache.shape[0] if num_pages is None else int(num_pages), _stream()),
+        error, entries, most_keys, rows, row, page_size, int(window or 0), cache.shape[0] if num_pages is None else int(num_pages), _stream()),
         "latent_gather")
     seen = work.as_strided((rows, rank), (row, 1))
     for i, w in enumerate((uk, uv)):
         torch.mm(seen, w.t(), out=work.as_strided((rows, n), (n, 1), rows * (row + i * n)))
     out = torch.empty(q.shape[0], n, dtype=bf16, device=dev)
-    _check(_fn("se_attn_prefill_tc_parts", "pi" "pii" "pi" "ppp" "pp" "iii" "fi" "p")(
-        _rows_ptr(q, "q", bf16), q.stride(0), lat + 2 * rows * row, n, rows * n, lat + 2 * rank, row, cu, kv,
+    _check(_fn("se_attn_prefill_tc_parts", "pi" "pii" "pii" "ppp" "pp" "iii" "fi" "p")(
+        _rows_ptr(q, "q", bf16), q.stride(0), lat + 2 * rows * row, n, rows * n, lat + 2 * rank, row, rows, cu, kv,
         _ptr(sink, torch.float32, "sink"), out.data_ptr(), error, entries, max_q_len, heads, float(scale), int(window or 0), _stream()),
         "latent_attention_heads")
     return out
@@ -1205,6 +1205,9 @@ _INDEX_CODES = {21: "the q/k preparation kernel", 22: "the plain attention kerne
 
 
 def error_text(code: int) -> str:
+    if code == 31:
+        return ("the latent attention over keys per head met lengths on the device beyond those that it was planned for (code 31); "
+                "the rows beyond were left out, the step's results are not valid")
     if code in _INDEX_CODES:
         return (f"{_INDEX_CODES[code]} was given a block-table entry outside its page pool (code {code}); "
                 "the access was skipped, the step's results are not valid")

@@ -117,6 +117,32 @@ def test_captured_portion_replayed_with_other_lengths(monkeypatch):
     assert float((out.double() - want.double()).norm()) < 2e-2 * float(want.double().norm())
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows_short,keys_short", [(1, 0), (300, 0), (0, 40), (561, 468)])
+def test_lengths_beyond_the_planned_ones(rows_short, keys_short):
+    """Lengths on the device that go beyond what the workspace and the grid were made for are reported and their rows left alone."""
+    from sparseengine_b200.csrc import ops
+    heads, rank, lens, kv = 2, 192, [64, 100], [500, 61 + 100]
+    g = torch.Generator(device=DEV).manual_seed(6)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    cache = torch.randn(64, 16, 256, generator=g, device=DEV).to(torch.bfloat16)
+    uk, uv = ((torch.randn(heads * 64, rank, generator=g, device=DEV) * 0.07).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(sum(lens), heads * 128, generator=g, device=DEV).to(torch.bfloat16)
+    table = torch.arange(64, **i32).view(2, 32)
+
+    def run(rows, most):
+        return ops.latent_attention_heads(q, cache, table, torch.tensor([0, 1], **i32), torch.tensor([0, 64, 164], **i32), torch.tensor(kv, **i32), None, uk, uv,
+                                          rows=rows, most_keys=most, entries=2, max_q_len=100, heads=heads, rank=rank, page_size=16, scale=0.1)
+
+    want = run(661, 500)
+    ops.error_check(DEV)
+    got = run(661 - rows_short, 500 - keys_short)
+    with pytest.raises(RuntimeError, match="code 31"):
+        ops.error_check(DEV)
+    if rows_short == 1:                                 # the first entry's rows are all there
+        assert torch.equal(got[:64], want[:64])
+
+
 def test_choice():
     from sparseengine_b200.csrc import ops
     assert ops.latent_seen_keys([5, 1, 8], [5, 90, 20], 10) == [5, 10, 17] and ops.latent_seen_keys([5], [90], None) == [90]
