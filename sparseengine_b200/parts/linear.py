@@ -63,10 +63,10 @@ def _kernel_reaches(*tensors: torch.Tensor) -> bool:
             and all(t.device == here and t.layout is torch.strided and not t.is_neg() for t in tensors))
 
 
-def _product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """x . w^T in float32: with this library's kernel where it is estimated to be ahead, else the library product."""
+def _product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, f32_terms: bool = True) -> torch.Tensor:
+    """x . w^T in float32: with this library's kernel where it is estimated to be ahead, else (and without ``f32_terms``) the library product."""
     tensors = (x, w) if out is None else (x, w, out)
-    if (_only_values(*tensors) and _kernel_reaches(*tensors) and _kernel_reads(x, w, out) and ops.gemm_f32_tc_supported(x.shape[1])
+    if (f32_terms and _only_values(*tensors) and _kernel_reaches(*tensors) and _kernel_reads(x, w, out) and ops.gemm_f32_tc_supported(x.shape[1])
             and ops.gemm_f32_dense_pays(x.shape[0], w.shape[0], x.shape[1], ops.sm_count(x.device))):
         if out is None:
             out = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)
@@ -74,9 +74,11 @@ def _product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) 
     return torch.matmul(x, w.t()) if out is None else torch.matmul(x, w.t(), out=out)
 
 
-def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, activation: str | None = None) -> torch.Tensor:
+def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, activation: str | None = None, *,
+           f32_terms: bool = True) -> torch.Tensor:
     """x [rows, in], w [out, in] → [rows, out]; CUDA tensors of one dtype only.  ``activation``: a name of
-    ``ops.ACTIVATIONS`` applied to the product (inside this library's few-row kernel, else as a kernel of its own)."""
+    ``ops.ACTIVATIONS`` applied to the product (inside this library's few-row kernel, else as a kernel of its own).
+    ``f32_terms``: float32 products may be taken in tf32 terms (False: multiply-adds of the whole numbers, always)."""
     if not (x.is_cuda and w.is_cuda):
         raise ValueError("linear needs CUDA tensors (there is no CPU path)")
     if x.dtype != w.dtype:
@@ -89,21 +91,22 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, ac
             out = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)
         return ops.gemv(x, w, out, activation)
     if x.dtype == torch.float32:
-        y = _product(x, w, out)
+        y = _product(x, w, out, f32_terms)
     else:
         y = torch.matmul(x, w.t()) if out is None else torch.matmul(x, w.t(), out=out)
     return y if activation is None else ops.activation_(y, activation)
 
 
-def linear_glu(x: torch.Tensor, w: torch.Tensor, activation=None) -> torch.Tensor:
+def linear_glu(x: torch.Tensor, w: torch.Tensor, activation=None, *, f32_terms: bool = True) -> torch.Tensor:
     """The gated activation of x [rows, in] . w [2n, in]^T (gate rows, then up rows) -> [rows, n]: inside this library's
-    few-row kernel, else as a kernel of its own after the library product.  ``activation`` as ``ops.glu``'s."""
+    few-row kernel, else as a kernel of its own after the library product.  ``activation`` as ``ops.glu``'s, ``f32_terms`` as
+    :func:`linear`'s."""
     n = w.shape[0] // 2
     out = torch.empty(x.shape[0], n, dtype=x.dtype, device=x.device)
     if (USE_GEMV and x.dtype == torch.bfloat16 and x.is_contiguous() and w.is_contiguous() and x.shape[0] <= GEMV_MAX_ROWS
             and w.shape[0] <= GEMV_GLU_MAX_OUT and ops.gemv_supported(x.shape[0], n, x.shape[1])):
         return ops.gemv_glu(x, w, out, activation)
-    return ops.glu(_product(x, w) if x.dtype == torch.float32 else torch.matmul(x, w.t()), out, activation)
+    return ops.glu(_product(x, w, None, f32_terms) if x.dtype == torch.float32 else torch.matmul(x, w.t()), out, activation)
 
 
 def pad_rows(w: torch.Tensor, multiple: int = 8) -> torch.Tensor:
@@ -113,11 +116,11 @@ def pad_rows(w: torch.Tensor, multiple: int = 8) -> torch.Tensor:
     return torch.cat([w, w.new_zeros(extra, *w.shape[1:])], 0) if extra else w
 
 
-def linear32(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def linear32(x: torch.Tensor, w: torch.Tensor, *, f32_terms: bool = True) -> torch.Tensor:
     """x [rows, in] . w [out, in]^T with the result left in 32-bit (not rounded to the activation type):
-    a product whose output joins a 32-bit residual stream."""
+    a product whose output joins a 32-bit residual stream.  ``f32_terms`` as :func:`linear`'s."""
     if x.dtype != w.dtype:
         raise TypeError(f"linear32: activation {x.dtype} and weight {w.dtype} differ")
     if x.dtype == torch.float32:
-        return _product(x, w)
+        return _product(x, w, None, f32_terms)
     return torch.mm(x, w.t(), out_dtype=torch.float32)

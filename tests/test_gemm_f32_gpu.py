@@ -130,11 +130,11 @@ def test_projections_take_it():
     from sparseengine_b200.parts.linear import linear
     x, w = torch.randn(1024, 2052, device=DEV), torch.randn(2048, 2048, device=DEV)
 
-    def calls(a, b):
+    def calls(a, b, **options):
         before = ops.calls.get("se_gemm_f32_dense", 0)
-        y = linear(a, b)
+        y = linear(a, b, **options)
         assert bool(((y.double() - a.double() @ b.double().t()).abs() <= 4 * _bound(a, b)).all())
         return ops.calls.get("se_gemm_f32_dense", 0) - before
 
-    assert calls(x[:, :2048], w) == 1 and calls(x[:, 4:], w) == 1
+    assert calls(x[:, :2048], w) == 1 and calls(x[:, 4:], w) == 1 and calls(x[:, 4:], w, f32_terms=False) == 0
     assert calls(x[:, 1:2049], w) == 0 and calls(x[:3, :2048], w) == 0 and calls(x[:, :64], w[:, :64].contiguous()) == 0

@@ -70,7 +70,7 @@ def test_what_sees_the_product_sees_it(taken, reached, monkeypatch):
     assert torch.allclose(torch.vmap(lambda r: linear32(r, w))(x.expand(3, 16, 32)), want.expand(3, 16, 8))
     assert torch.allclose(torch.func.jvp(lambda r: linear32(r, w), (x,), (x,))[1], want)
     assert torch.equal(torch.func.grad(lambda r: linear32(r, w).sum())(x), torch.autograd.functional.jacobian(lambda r: (r @ w.t()).sum(), x))
-    assert torch.equal(make_fx(linear32)(x, w)(2 * x, w), 2 * x @ w.t())
+    assert torch.equal(make_fx(lambda a, b: linear32(a, b))(x, w)(2 * x, w), 2 * x @ w.t())
     assert torch.equal(torch.jit.trace(linear32, (x, w), check_trace=False)(2 * x, w), 2 * x @ w.t())
     with FlopCounterMode(display=False) as count:
         linear32(x, w)
@@ -86,3 +86,10 @@ def test_what_sees_the_product_sees_it(taken, reached, monkeypatch):
         linear32(z, torch.nn.Parameter(w))
     linear32(x, w)
     assert len(taken) == 2
+
+
+def test_the_caller_may_have_the_library_product(taken, reached):
+    x, w = torch.randn(16, 32), torch.randn(8, 32)
+    assert torch.equal(linear32(x, w, f32_terms=False), x @ w.t()) and not taken
+    linear32(x, w)
+    assert len(taken) == 1
