@@ -59,7 +59,7 @@ def test_against_64_bits(heads, window, sinks):
         assert torch.equal(run(dirty, wrong), out)
 
 
-def _mixer_step(lens, held, pages_per=None):
+def _mixer_step(lens, held):
     from sparseengine_b200.parts.base import StepContext
     n, total, cu = len(lens), sum(lens), [0]
     for t in lens:
@@ -82,6 +82,115 @@ def _mixer(**options):
     part.bind({n: (torch.randn(p.shape, generator=g, device=DEV) * (0.5 if "sink" in n else 0.06) + float("norm" in n)).to(
         torch.float32 if p.dtype == "float32" else torch.bfloat16) for n, p in part.parameters().items()})
     return part
+
+
+def _mixer64(part, x, step, cache, table):
+    """The mixer in 64 bits: cache [pages, 16, row] as it was before the step."""
+    from sparseengine_b200.parts.position import as_rotary_args
+    s, H = part.spec, part.spec.num_heads
+    inv, split = as_rotary_args(part.position.kernel_args(torch.device(DEV))).inv_freq.double(), s.position.pairing == "split_half"
+    angle = step.positions.double()[:, None] * inv
+
+    def norm(t, w):
+        return t / torch.sqrt((t * t).mean(-1, keepdim=True) + s.norm_eps) * w.double()
+
+    def turn(t):                # [tokens, ..., 64]
+        cs, sn = (f(angle).view(-1, *[1] * (t.dim() - 2), 32) for f in (torch.cos, torch.sin))
+        a, b = (t[..., :32], t[..., 32:]) if split else (t[..., 0::2], t[..., 1::2])
+        a, b = a * cs - b * sn, b * cs + a * sn
+        return torch.cat([a, b], -1) if split else torch.stack([a, b], -1).flatten(-2)
+
+    proj = x.double() @ (part.down if s.q_rank else part.in_proj).double().t()
+    q = norm(proj[:, :s.q_rank], part.q_norm) @ part.uq.double().t() if s.q_rank else proj[:, :H * 128]
+    q = q.view(-1, H, 128)
+    q = torch.cat([q[..., :64], turn(q[..., 64:])], -1)
+    lat = proj[:, s.q_rank or H * 128:]
+    new = torch.cat([norm(lat[:, :s.kv_rank], part.kv_norm), turn(lat[:, s.kv_rank:s.kv_rank + 64])], -1)
+    out, at = [], 0
+    for e, (n, kv) in enumerate(zip(step.q_lens, step.kv_lens)):
+        rows = torch.cat([cache[table[e].long()].reshape(-1, cache.shape[-1])[:kv - n].double(), new[at:at + n]])
+        k, v = ((rows[:, :s.kv_rank] @ w.double().t()).view(kv, H, 64) for w in (part.uk, part.uv))
+        k = torch.cat([k, rows[:, None, s.kv_rank:].expand(-1, H, -1)], -1)
+        pos, key = torch.arange(kv - n, kv, device=DEV)[:, None], torch.arange(kv, device=DEV)[None]
+        hidden = (key > pos) | (key <= pos - s.window) if s.window else key > pos
+        score = (torch.einsum("thd,khd->thk", q[at:at + n], k) * s.scale).masked_fill(hidden[:, None], float("-inf"))
+        if s.sink:
+            score = torch.cat([score, part.sink.double()[None, :, None].expand(n, -1, 1)], -1)
+        out.append(torch.einsum("thk,khd->thd", torch.softmax(score, -1)[..., :kv], v).flatten(1))
+        at += n
+    out = torch.cat(out)
+    if s.output_gate:
+        out = out * torch.sigmoid(proj[:, part.g_off:])
+    return out @ part.o.double().t()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pairing", ["split_half", "interleaved"])
+@pytest.mark.parametrize("options", [dict(), dict(q_rank=0, output_gate=True, sink=False), dict(q_rank=0, window=100), dict(q_rank=0, output_gate=True, kv_rank=80)],
+                         ids=["query latent", "direct, gated", "direct, window", "direct, gated, short latent"])
+def test_mixer_against_64_bits(options, pairing, monkeypatch):
+    """The whole mixer in this form: queries rotated in place, which without a query latent are columns of the projection beside the gate's."""
+    from sparseengine_b200.config.specs import RotarySpec
+    from sparseengine_b200.csrc import ops
+    from sparseengine_b200.parts.base import LayerSlot
+    monkeypatch.setattr(ops, "latent_takes_heads", lambda *a, **k: True)
+    part = _mixer(position=RotarySpec(rotary_dim=64, theta=1e4, pairing=pairing), **options)
+    step, row = _mixer_step([257, 1, 70], [0, 64, 500]), part.spec.kv_rank + 64
+    g = torch.Generator(device=DEV).manual_seed(8)
+    x = torch.randn(328, 256, generator=g, device=DEV).to(torch.bfloat16)
+    cache = torch.randn(120, 16, row, generator=g, device=DEV).to(torch.bfloat16)
+    table = torch.randperm(120, generator=torch.Generator().manual_seed(9)).to(torch.int32)[:108].view(3, 36).contiguous().to(DEV)
+    want = _mixer64(part, x, step, cache.clone(), table)
+    before = ops.calls.get("se_latent_gather", 0)
+    got = part.forward(x, step, LayerSlot(kv=cache, table=table, page_size=16))
+    assert ops.calls.get("se_latent_gather", 0) == before + 1
+    ops.error_check(DEV)
+    # nine roundings to 16 bits one after another (projection, norm, queries, rotation, keys or values, weights, sums, gate, result), each 2^-9 / sqrt(3)
+    # of its vector on average; scores of order one pass theirs on once more: sqrt(2 * 9) * 1.13e-3 = 4.8e-3, three times that
+    assert float((got.double() - want).norm()) < 1.5e-2 * float(want.norm())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pairing", ["split_half", "interleaved"])
+@pytest.mark.parametrize("heads,d,rot,rotary,more", [(4, 64, 64, 64, 0), (3, 64, 64, 64, 24), (40, 16, 32, 32, 8), (3, 20, 24, 24, 0), (2, 64, 64, 32, 8), (5, 7, 6, 4, 3)])
+def test_queries_rotated_in_place(heads, d, rot, rotary, more, pairing):
+    """The same numbers as into another matrix, and nothing else of the rows (views with ``more`` columns behind) touched."""
+    from sparseengine_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(10)
+    wide = torch.randn(37, heads * (d + rot) + more, generator=g, device=DEV).to(torch.bfloat16)
+    inv, positions = torch.rand(rotary // 2, generator=g, device=DEV), torch.arange(37, dtype=torch.int32, device=DEV) * 13
+    sizes = dict(heads=heads, head_dim=d, rank=d, rot=rot, rotary_dim=rotary, pairing=pairing)
+    apart, want = torch.zeros(37, heads, d + rot, dtype=torch.bfloat16, device=DEV), wide.clone()
+    ops.latent_q_rotate(wide[:, :heads * (d + rot)], inv, positions, apart, **sizes)
+    want[:, :heads * (d + rot)].view(37, heads, d + rot)[..., d:] = apart[..., d:]
+    assert not torch.equal(want, wide)
+    q = wide[:, :heads * (d + rot)]
+    ops.latent_q_rotate(q, inv, positions, q, **sizes)
+    assert torch.equal(wide, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("page", [-1, 64, 10 ** 6])
+def test_pages_outside_the_pool(page):
+    """A table entry in the gathered range that names no page: reported, its rows zeros, the other entry's outputs as they were."""
+    from sparseengine_b200.csrc import ops
+    g, i32 = torch.Generator(device=DEV).manual_seed(11), dict(dtype=torch.int32, device=DEV)
+    cache = torch.randn(64, 16, 256, generator=g, device=DEV).to(torch.bfloat16)
+    uk, uv = ((torch.randn(128, 192, generator=g, device=DEV) * 0.07).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(164, 256, generator=g, device=DEV).to(torch.bfloat16)
+
+    def run(cache, table):
+        return ops.latent_attention_heads(q, cache, table, torch.tensor([0, 1], **i32), torch.tensor([0, 64, 164], **i32), torch.tensor([300, 100], **i32),
+                                          None, uk, uv, rows=400, most_keys=300, entries=2, max_q_len=100, heads=2, rank=192, page_size=16, scale=0.1)
+
+    table, blank = torch.arange(64, **i32).view(2, 32), cache.clone()
+    blank[5] = 0
+    want = run(blank, table)
+    table[0, 5] = page
+    got = run(cache, table)
+    with pytest.raises(RuntimeError, match="code 30"):
+        ops.error_check(DEV)
+    assert torch.equal(got, want)
 
 
 @pytest.mark.gpu
