@@ -12,11 +12,13 @@
 // value columns) that takes the chunks in turn with its slice of the state in shared memory: two or three small matrix
 // products per chunk instead of a chain of T dependent steps.
 //
-// What bounds the walk is arithmetic (3 to 5 multiply-adds per state element and token) along a chain of chunks; 16-bit operands would
+// What bounds the walk is the chain of a chunk: products, the split of their operands, barriers, the state through shared memory.  The tensor pipe is busy
+// 43 % of the time (state space), instructions issue in 49 % of the cycles; 16-bit operands would
 // lose what the recurrence has to keep.  With multiply-adds it stood at half their rate, its other half shared-memory reads (8 x 8 outputs
 // a thread, an LDS.128 each four multiply-adds); products in tf32 terms by mma.sync read less.  Measured, multiply-adds / now: state space,
-// 2,048 tokens of 64 heads of 64 columns, 204 / 150 us; retention, 8,192 tokens of 32 heads of 128, 752 / 456; delta rule per channel, 4,670 tokens of
-// 16 heads of 128, 418 / 333; per head, 2,048 tokens, 176 / 123.  Sixteen warps at the products instead of eight, all loading for themselves: 168, 616, -, 148 (eight: 152, 563, 333, 134).  Every exponent is a
+// 2,048 tokens of 64 heads of 64 columns, 204 / 151 us; retention, 8,192 tokens of 32 heads of 128, 752 / 456; delta rule per channel, 4,670 tokens of
+// 16 heads of 128, 418 / 322; per head, 2,048 tokens, 176 / 122.  Sixteen warps at the products instead of eight, all loading for themselves: 168, 616, -, 148
+// (eight: 152, 563, 333 with 32 value columns, 134).  Every exponent is a
 // difference of sums of logarithms that is at most 0 up to the 64-bit sums' rounding
 // (no token's logarithm lies below -1e4) or, for decays per channel, a product of decays of at most T tokens: no term overflows.
 //

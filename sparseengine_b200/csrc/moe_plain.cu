@@ -600,6 +600,9 @@ extern "C" int se_moe_plain_tile_rows() { return se::kBM; }
 // Rows per tile that the 32-bit grouped products take for a step of `assignments` rows over `experts` experts, whose
 // products have inner dimensions k0 and k1: 8 (weights streamed past a few rows) while an expert has about four rows or
 // fewer and eight rows of the wider operand fit in shared memory, 128 beyond; 0: widths that only the general kernel takes.
+// Against the tiles on tensor cores (gemm_f32_tc.cu) the two meet between five and six rows.  Expert layer, us streamed / tiles: 256 experts of 3,072 x 1,536,
+// 2 rows 2,015 / 2,781, 4 2,848 / 3,360, 5 3,179 / 3,366, 6 3,533 / 3,410, 8 4,189 / 3,363, 16 7,287 / 3,434; 32 of 2,048 x 1,024, 4 rows 222 / 256,
+// 6 259 / 262, 8 299 / 260.
 extern "C" int se_moe_f32_tile_rows(int assignments, int experts, int k0, int k1) {
     if (k0 <= 0 || k1 <= 0 || (k0 & 3) || (k1 & 3)) return 0;
     const int k = k0 > k1 ? k0 : k1;

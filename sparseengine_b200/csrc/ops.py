@@ -729,11 +729,12 @@ def retention_segment_plan(entries: int, heads: int, v_head_dim: int, max_q_len:
 
 def retention_chunk(q32, k32, proj, v_off: int, decay, state, step, o, *, heads, head_dim, v_head_dim, segments=None,
                     silu: bool = False, qk=None, rotation=None):
-    """The same recurrence as :func:`retention_scan` in chunks of 64 tokens (closed form per chunk, 32-bit
-    FMA arithmetic): for steps that bring prompt portions.  With q32 and k32 one kernel does a chunk at a time; ``segments``:
+    """The same recurrence as :func:`retention_scan` in chunks of 64 tokens (closed form per chunk): for steps that bring prompt
+    portions.  With q32 and k32 one kernel does a chunk at a time in 32-bit multiply-adds; ``segments``:
     ``(per entry, tokens each)``, default by :func:`retention_segment_plan`.  With ``qk`` (and ``q32`` and ``k32`` None): ``(q_off,
     k_off, k_scale)`` of the projection and ``rotation`` ``(inv_freq, rotary_dim, positions)`` (None: none); the chunks are
-    prepared side by side and walked (csrc/chunk_walk.cuh), where :func:`retention_walk_supported` says so."""
+    prepared side by side and walked, 32-bit values as products of tf32 terms (csrc/chunk_walk.cuh), where
+    :func:`retention_walk_supported` says so."""
     global launch_count
     seg_state = work = inv_freq = positions = None
     max_seg, seg_len, q_off, k_off, k_scale, rotary_dim, tokens = 1, 0, 0, 0, 1.0, 0, proj.shape[0]
@@ -1335,7 +1336,9 @@ def gemm_f32_dense_pays(rows: int, n_out: int, k_dim: int, sms: int) -> bool:
     too few tiles to go without).  Measured, us, library / this (rows x outputs x inner): 2,048 x 8,192 x 3,072 1,810 / 479;
     128 x 10,304 x 2,048 147 / 52; 128 x 3,072 x 6,144 179 / 135; 512 x 2,048 x 2,048 86 / 51, 128 rows 40 / 50; 4,096 x 192 x 2,048 86 / 51,
     1,024 rows 40 / 50; 8 x 8,192 x 3,072 60 / 53.  The very few rows that the library gives to its kernels with split sums (up to
-    7, up to 3 with an inner dimension from 3,072 on) stay there: those sums are the more exact ones (1.2e-7 to 2.5e-7)."""
+    7, up to 3 with an inner dimension from 3,072 on) stay there: those sums are the more exact ones (1.2e-7 to 2.5e-7).
+    Up to 8 rows the library still splits most sums; terms of either sign, error over the result's norm 3.1e-7 and more, here 2.4e-7 to 2.6e-7;
+    terms of one sign 1.0e-7 to 1.5e-7, here 2.7e-7 to 2.9e-7.  From 9 rows on it is 3.3e-7 to 1.6e-6 for either, here 2.1e-7 to 3.2e-7."""
     if k_dim < F32_TC_MIN_INNER or rows < (4 if k_dim >= 3072 else 8):
         return False
     waves = -(-(-(-rows // 128) * -(-n_out // 128)) // sms)

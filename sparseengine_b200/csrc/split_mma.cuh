@@ -1,10 +1,15 @@
 // Products of 32-bit values with mma.sync in tf32 terms: an operand is the sum of two tf32 values (11 bits of mantissa each, hi the
-// nearest one, lo what is left), and hi hi + lo hi + hi lo leaves out terms of 2^-24 of a product.  The tensor cores cut off what does
+// nearest one, lo what is left, of which they read 11 of its up to 12 bits), and hi hi + lo hi + hi lo leaves out lo lo, up to 2^-22 of a product.  The
+// tensor cores cut off what does
 // not fit when they add to an accumulator instead of rounding it, so that long sums there come out too small: the large products are
 // summed by m16n8k8 steps that start from zero and are then added in 32-bit; the small ones have an accumulator of their own,
 // where what is cut off does not count.  Measured against 64 bits, sums of 32 / 128 products of normal values, error over the result's
 // norm: 1.0e-7 / 1.2e-7; one chain of multiply-adds 1.0e-7 / 2.0e-7, four chains 0.7e-7 / 1.1e-7, one accumulator for all three
-// terms 2.5e-7 / 9.1e-7.
+// terms 2.5e-7 / 9.1e-7.  The walks that use them (chunk_walk.cuh; 70, 700 and 3,000 tokens), with chains of multiply-adds / now, 1e-7: outputs of
+// the state space 1.00, 1.06, 1.29 / 0.95, 0.94, 1.01, its state 1.18, 1.22, 0.90 / 1.42, 1.43, 1.15; retention 2.09, 1.98, 2.56 / 1.71, 1.80, 2.33,
+// state 1.11, 1.54, 2.57 / 1.15, 1.40, 2.39; delta rule per head 2.14, 2.22, 2.43 / 1.87, 1.93, 2.14, state 1.83, 2.07, 2.39 / 1.89, 2.14, 2.31; per
+// channel 1.55, 1.56, 2.11 / 1.67, 1.69, 2.17, state 2.24, 2.25, 3.19 / 2.30, 2.31, 3.24.  Whole mixers in float32, whose projections count for more: outputs
+// 1.5e-6 to 4.5e-6 / 0.4e-6 to 4.1e-6, states 0.8e-6 to 3.7e-6 / 0.2e-6 to 3.6e-6, none larger than before.
 //
 // What it buys is shared-memory reads, not arithmetic: mma.sync takes 8.4 cycles of a quarter SM for 1,024 products and, on this
 // part, multiply-adds and integer instructions wait for it (0.65 to 1 cycle more for each), so three terms cost 25 cycles where
