@@ -1,0 +1,173 @@
+// Linear recurrences over prompt portions by chunks of 128 tokens on tcgen05, side by side: what the chunks' kernels share.
+//
+// The walk (chunk_walk.cuh) takes a head's chunks one after another, outputs and all.  Only the state has to go that way, and of it
+// only e^(B_n) S + (what the chunk adds), which needs no product with the state.  So here one kernel forms what chunks add
+// (sum_s e^(B_n - B_s) k_s u_s^T, rows of the state = the M side), the states at the chunks' starts follow by multiply-adds, and another kernel
+// makes the outputs e^(B_t) q_t . S_0 + sum_s P[t][s] u_s of every chunk by itself (tokens = the M side).
+//
+// Everything is 32-bit and multiplied as such: a value is cut into three bfloat16 terms of 8 bits each, which together are the value (`cut`), and of the
+// nine products of terms the six down to 2^-16 are summed, the smallest first, in 32-bit tensor memory; what is left out is below 2^-23
+// of a product.  Values that were 16-bit are a term themselves.  bfloat16 has twice tf32's rate and half its steps into the accumulator, and an operand
+// takes 96 KB for 128 x 128 values instead of 128.
+//
+// What is not finite leaves its outputs not finite, and those of earlier tokens too (their weights for it are 0): a tile with such an output is done
+// again token by token.
+#pragma once
+#include "chunk_walk.cuh"
+#include "fa_util.cuh"
+
+namespace se {
+namespace tiles {
+
+using walk::chunk_of;
+using walk::ld4;
+
+constexpr int kT = 128, kD = 128, kThreads = 512;
+constexpr int kHalf = 128 * 128;                     // bytes of [128 rows][64 bfloat16], a swizzled 128 bytes each
+constexpr int kTerm = 2 * kHalf;                     // a term of a 128 x 128 operand
+constexpr int kErrorCode = 19;
+
+// x = its upper 8 bits of mantissa + the next 8 + the last 8, each a bfloat16; of a pair, x in the lower half
+__device__ __forceinline__ void cut(float x, float y, uint32_t (&t)[3]) {
+    uint32_t a = __float_as_uint(x), b = __float_as_uint(y);
+    t[0] = __byte_perm(a, b, 0x7632);
+    x -= __uint_as_float(a & 0xffff0000u);
+    y -= __uint_as_float(b & 0xffff0000u);
+    a = __float_as_uint(x);
+    b = __float_as_uint(y);
+    t[1] = __byte_perm(a, b, 0x7632);
+    x -= __uint_as_float(a & 0xffff0000u);
+    y -= __uint_as_float(b & 0xffff0000u);
+    t[2] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+}
+
+// kind::f16 of bfloat16 operands, 32-bit sums, M = 128
+__device__ __forceinline__ uint32_t instr(int n, bool a_mn, bool b_mn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+}
+// An operand in shared memory: terms `term` bytes apart.  K-major: halves of 64 along K `half` bytes apart, rows of 128 bytes; MN-major: rows along K, groups of 64
+// along M or N `half` bytes apart.  The descriptor of step k of 16.
+template <bool MN>
+__device__ __forceinline__ uint64_t step_desc(uint32_t at, uint32_t half, int k) {
+    return MN ? fa::desc_mnmajor(at, half) + (uint64_t)(128 * k) : fa::desc_kmajor(at + (k >> 2) * half) + (uint64_t)(2 * (k & 3));
+}
+// d = A . B over K = 128 in terms, the smallest products first.  One lane of a warp-uniform branch.
+template <bool A_MN, bool B_MN, int B_TERMS>
+__device__ __forceinline__ void product(uint32_t d, uint32_t a, uint32_t a_half, uint32_t a_term, uint32_t b, uint32_t b_half, uint32_t b_term, uint32_t id) {
+    uint32_t started = 0;
+#pragma unroll
+    for (int sum = 2; sum >= 0; --sum)
+#pragma unroll
+        for (int j = 0; j <= sum && j < B_TERMS; ++j)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                fa::umma(d, step_desc<A_MN>(a + (sum - j) * a_term, a_half, k), step_desc<B_MN>(b + j * b_term, b_half, k), id, started);
+                started = 1;
+            }
+}
+// The same with A in tensor memory, terms of 64 columns; ADD: to what d holds
+template <bool B_MN, int B_TERMS, bool ADD = false>
+__device__ __forceinline__ void product_ts(uint32_t d, uint32_t a, uint32_t b, uint32_t b_half, uint32_t b_term, uint32_t id) {
+    uint32_t started = ADD;
+#pragma unroll
+    for (int sum = 2; sum >= 0; --sum)
+#pragma unroll
+        for (int j = 0; j <= sum && j < B_TERMS; ++j)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                fa::umma_ts(d, a + (sum - j) * 64 + 8 * k, step_desc<B_MN>(b + j * b_term, b_half, k), id, started);
+                started = 1;
+            }
+}
+
+__device__ __forceinline__ void st4(uint32_t addr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
+__device__ __forceinline__ void st8(uint32_t addr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void st16(uint32_t addr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+                   "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void ld8(uint32_t addr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ld16(uint32_t addr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                   "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void sts8(uint32_t at, uint32_t x, uint32_t y) {
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool fill) {      // 16 bytes, or zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(fill ? 16 : 0) : "memory");
+}
+
+// Four neighbours along a row in three terms, to an operand at `at` (a row is 64 bfloat16, quad = the four's place among its sixteen)
+__device__ __forceinline__ void put4(uint32_t at, uint32_t term, int row, int quad, float4 v) {
+    uint32_t a[3], b[3];
+    cut(v.x, v.y, a);
+    cut(v.z, v.w, b);
+    at += fa::sw128(row, quad >> 1) + (quad & 1) * 8;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) sts8(at + i * term, a[i], b[i]);
+}
+
+// Tensor memory, one barrier for the products of a block (each committed and waited for in turn) and the end of both.
+struct Shared {
+    uint64_t done, last;
+    uint32_t tmem;
+    volatile int abort_flag;
+};
+__device__ __forceinline__ uint32_t begin(Shared& s) {
+    if (threadIdx.x == 0) {
+        fa::mbar_init(smem_u32(&s.done), 1);
+        fa::mbar_init(smem_u32(&s.last), 1);
+        s.abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&s.tmem)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    return s.tmem;
+}
+__device__ __forceinline__ void end(Shared& s) {
+    const uint32_t tmem = s.tmem;
+    fence_before();
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        fence_after();
+        if (fa::elect_one()) fa::umma_commit(smem_u32(&s.last));           // what was issued ends before its memory is given back
+        __syncwarp();
+        fa::mbar_drain(smem_u32(&s.last), 0);
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+    }
+}
+// Until the products committed `n`-th (from 0) are there; the same answer in every thread.  A wait that runs out is reported.
+__device__ __forceinline__ bool products_done(Shared& s, uint32_t n, int* error) {
+    const bool ok = fa::mbar_wait(smem_u32(&s.done), n & 1, &s.abort_flag);
+    if (__syncthreads_and(ok)) {
+        fence_after();
+        return true;
+    }
+    if (threadIdx.x == 0) atomicCAS(error, 0, kErrorCode);
+    return false;
+}
+
+}  // namespace tiles
+}  // namespace se

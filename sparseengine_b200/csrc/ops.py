@@ -26,7 +26,7 @@ _fns: dict = {}
 
 # Kernels launched through these bindings since the process started (a launcher that
 # starts two kernels counts two).  Benchmarks read the difference around a timed region.
-KERNELS_PER_CALL = {"se_attn_decode": 2, "se_router": 2, "se_causal_conv": 2, "se_ssm_scan": 2, "se_retention_chunk": 2, "se_ssm_walk": 2, "se_delta_walk": 2}   # upper bounds per call
+KERNELS_PER_CALL = {"se_attn_decode": 2, "se_router": 2, "se_causal_conv": 2, "se_ssm_scan": 2, "se_retention_chunk": 2, "se_ssm_walk": 2, "se_delta_walk": 2, "se_retention_tiles": 4}   # upper bounds per call
 launch_count = 0
 calls: dict = {}     # launcher name -> times called (tests check which kernels a path took)
 
@@ -763,6 +763,42 @@ def retention_walk_supported(head_dim: int, v_head_dim: int, rotary_dim: int, pr
     """Whether :func:`retention_chunk` takes q and k from the projection ``proj`` with its columns at ``offsets``."""
     return (rotary_dim % 8 == 0 and chunk_walk_supported(head_dim, v_head_dim, proj.stride(0), *offsets)
             and proj.data_ptr() % 16 == 0)
+
+
+def retention_tiles_supported(head_dim: int, v_head_dim: int, rotary_dim: int, proj, state, *offsets: int) -> bool:
+    """Whether :func:`retention_tiles` takes the projection ``proj`` with its columns at ``offsets`` (what
+    ``se_retention_tiles_supported`` answers, restated, and the rows' alignment)."""
+    return (head_dim == 128 and v_head_dim == 128 and rotary_dim in (0, 128) and proj.dtype == torch.bfloat16
+            and proj.stride(0) % 8 == 0 and proj.data_ptr() % 16 == 0 and not any(n % 8 for n in offsets)
+            and state.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0)
+
+
+def retention_tiles_plan(step, tokens: int, heads: int, rotary_dim: int, device) -> tuple:
+    """(segments, chunks of a segment, floats of workspace) of :func:`retention_tiles`: an entry's chunks in as many segments,
+    summed side by side, as fill the device."""
+    n, chunks = step.num_seqs, -(-step.max_q_len // 128)
+    per = -(-chunks // max(1, min(chunks, sm_count(device) // (heads * n))))
+    segments = -(-chunks // per)
+    states = (tokens // 128 + n + (n * segments if segments > 1 else 0)) * heads * 128 * 128
+    return segments, per, states + heads * (130 + per) + 4 + (tokens * 128 if rotary_dim else 0)
+
+
+def retention_tiles(proj, q_off: int, k_off: int, v_off: int, g_off: int, k_scale: float, rotation, decay, state, step, *, heads, head_dim,
+                    v_head_dim, eps: float = 0.0, out=None, o=None):
+    """The recurrence of :func:`retention_chunk` from the projection's columns, in chunks of 128 tokens side by side on tcgen05
+    (csrc/retention_tiles.cu), where :func:`retention_tiles_supported`: into ``out``, normed and gated as by :func:`retention_out`,
+    or into ``o`` as it is."""
+    dev, tokens, n = proj.device, proj.shape[0], step.num_seqs
+    inv_freq, rotary_dim, positions = rotation if rotation is not None else (None, 0, None)
+    segments, per, floats = retention_tiles_plan(step, tokens, heads, rotary_dim, dev)
+    work = _walk_work(floats, dev)
+    _check(_fn("se_retention_tiles", "piiiii" "ppif" "ppl" "pp" "ppf" "pp" "iiiii" "iiip")(
+        _rows_ptr(proj, "proj", torch.bfloat16), proj.stride(0), int(q_off), int(k_off), int(v_off), int(g_off),
+        _ptr(inv_freq, torch.float32, "inv_freq"), _ptr(positions, torch.int32, "positions"), int(rotary_dim), float(k_scale),
+        _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), state.stride(0), _ptr(step.cu_q), _ptr(step.seq_rows),
+        _ptr(out, torch.bfloat16, "out"), _ptr(o, torch.float32, "o"), float(eps), work.data_ptr(), _ptr(error_word(dev)),
+        tokens, n, heads, head_dim, v_head_dim, segments, per, sm_count(dev), _stream()), "retention_tiles")
+    return out if out is not None else o
 
 
 def retention_out(o, proj, g_off: int, out, *, heads, v_head_dim, eps):

@@ -1,0 +1,569 @@
+// Retention over prompt portions by chunks of 128 tokens side by side (chunk_tiles.cuh), bfloat16 activations, heads of 128 x 128:
+//
+//     o_t = g^(t+1) q_t . S_0 + sum_{s <= t} g^(t-s) (q_t . k_s) v_s,      S = g^n S_0 + sum_s g^(n-1-s) k_s v_s^T
+//
+// Three kernels after one that works out angles and powers once for all heads: `states` (a block per head and segment of an entry's chunks) leaves the
+// state at each chunk's start, `join` (where an entry has several segments) the states at the segments' starts, `outputs` (a block per chunk and head)
+// the rest: q and k turned on their way from the projection, both products with q, the decays, P v, and where the mixer norms each head the norm and the gate.
+//
+// Measured, 8,192 tokens of 32 heads (the walk, its preparation and the norm: 675 us): 330 = angles 4 + states 73 + join 4 + outputs 247; 2,048 tokens of 16
+// heads 147 and 62; four entries of 100 tokens, 32 heads, 54 and 37.  Errors against 64 bits over the result's norm: outputs 2.0e-7 to 2.7e-7 (the walk 1.4e-7 to 2.1e-7), states
+// 0.8e-7 to 1.5e-7 (0.8e-7 to 2.2e-7), where 16-bit inputs and outputs leave 4e-3.
+#include "chunk_tiles.cuh"
+
+namespace se {
+namespace tiles {
+
+struct Retention {
+    const __nv_bfloat16* proj;
+    int pitch, q_off, k_off, v_off, g_off;
+    const float2* turn;            // [tokens][64] cosine and sine, or null: q and k as they are
+    const float* powers;           // [H][powers_pitch]: g^0 .. g^128, then g^(128 j) for j = 0 ..
+    int powers_pitch;
+    float* states;                 // [places][H][128 columns][128 rows]: at a chunk's start, from its segment's start on
+    float* starts;                 // [entries * segments][H][128][128]: what a segment leaves by itself, then the state at its start
+    int segments, seg_chunks;      // per entry at most; chunks of a segment
+    float* state;
+    long long state_stride;
+    const int* cu_q;
+    const int* seq_rows;
+    int entries, H, places;
+    float k_scale, eps;
+    __nv_bfloat16* out;            // [tokens][H * 128] after norm and gate, or null:
+    float* o;                      // [tokens][H * 128]
+    int* error;
+};
+
+__global__ void __launch_bounds__(256)
+retention_tables_kernel(float2* __restrict__ turn, const int* __restrict__ positions, const float* __restrict__ inv_freq, int tokens, int turn_blocks,
+                        float* __restrict__ powers, int pitch, const float* __restrict__ decay) {
+    if ((int)blockIdx.x < turn_blocks) {
+        const int x = blockIdx.x * 256 + threadIdx.x;
+        if (x >= tokens * 64) return;
+        float s, c;
+        sincosf((float)positions[x >> 6] * inv_freq[x & 63], &s, &c);
+        turn[x] = make_float2(c, s);
+        return;
+    }
+    const int h = blockIdx.x - turn_blocks;
+    const double g = (double)decay[h];
+    for (int i = threadIdx.x; i < pitch; i += 256) powers[(size_t)h * pitch + i] = (float)pow(g, (double)(i <= kT ? i : (i - kT - 1) * kT));
+}
+
+// a pair of a row turned by its angle
+__device__ __forceinline__ void rotate(float2 cs, float& a, float& b) {
+    const float a0 = a;
+    a = a0 * cs.x - b * cs.y;
+    b = b * cs.x + a0 * cs.y;
+}
+// element d of a token's q or k row (columns from `off` on), turned
+__device__ __forceinline__ float column_of(const Retention& p, int off, size_t token, int h, int d) {
+    const __nv_bfloat16* row = p.proj + token * p.pitch + off + (size_t)h * kD;
+    float lo = __bfloat162float(row[d & 63]), hi = __bfloat162float(row[64 + (d & 63)]);
+    if (p.turn != nullptr) rotate(p.turn[token * 64 + (d & 63)], lo, hi);
+    return d < 64 ? lo : hi;
+}
+__device__ __forceinline__ float key_of(const Retention& p, size_t token, int h, int d) { return column_of(p, p.k_off, token, h, d) * p.k_scale; }
+// four pairs of columns of a row turned (two pairs a float4) and cut: to the row's place in the halves of an operand
+__device__ __forceinline__ void put_pairs(uint32_t at, int row, int quad, uint2 lo, uint2 hi, float4 c0, float4 c1, float f) {
+    float x[4] = {__uint_as_float(lo.x << 16), __uint_as_float(lo.x & 0xffff0000u), __uint_as_float(lo.y << 16), __uint_as_float(lo.y & 0xffff0000u)};
+    float y[4] = {__uint_as_float(hi.x << 16), __uint_as_float(hi.x & 0xffff0000u), __uint_as_float(hi.y << 16), __uint_as_float(hi.y & 0xffff0000u)};
+    rotate(make_float2(c0.x, c0.y), x[0], y[0]);
+    rotate(make_float2(c0.z, c0.w), x[1], y[1]);
+    rotate(make_float2(c1.x, c1.y), x[2], y[2]);
+    rotate(make_float2(c1.z, c1.w), x[3], y[3]);
+    put4(at, kTerm, row, quad, make_float4(x[0] * f, x[1] * f, x[2] * f, x[3] * f));
+    put4(at + kHalf, kTerm, row, quad, make_float4(y[0] * f, y[1] * f, y[2] * f, y[3] * f));
+}
+// k's rows of a chunk in three terms, each times `factor(row)`: two rows a warp at a time, four pairs of columns a lane
+template <typename Factor>
+__device__ __forceinline__ void put_keys(const Retention& p, uint32_t at, int first, int n, int h, Factor factor) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = lane & 15;
+    const __nv_bfloat16* k = p.proj + p.k_off + (size_t)h * kD + 4 * quad;
+    uint2 lo[4], hi[4];
+    float4 cs[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = 32 * i + 2 * warp + (lane >> 4);
+        const size_t row = (size_t)first + t;
+        lo[i] = hi[i] = make_uint2(0, 0);
+        cs[i][0] = cs[i][1] = make_float4(1.f, 0.f, 1.f, 0.f);
+        if (t < n) {
+            lo[i] = *reinterpret_cast<const uint2*>(k + row * p.pitch);
+            hi[i] = *reinterpret_cast<const uint2*>(k + row * p.pitch + 64);
+            if (p.turn != nullptr) {
+                const float4* c = reinterpret_cast<const float4*>(p.turn + row * 64 + 4 * quad);
+                cs[i][0] = c[0];
+                cs[i][1] = c[1];
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = 32 * i + 2 * warp + (lane >> 4);
+        put_pairs(at, t, quad, lo[i], hi[i], cs[i][0], cs[i][1], factor(t) * p.k_scale);
+    }
+}
+// a head's rows as they are, columns from `off` on: [128 tokens][64 columns], twice
+__device__ __forceinline__ void fetch_rows(const Retention& p, uint32_t at, int off, int first, int n, int h) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int x = i * kThreads + threadIdx.x, t = x >> 4, c = x & 15;
+        const bool in = t < n;
+        cp16(at + (c >> 3) * kHalf + fa::sw128(t, c & 7), p.proj + (size_t)(first + (in ? t : 0)) * p.pitch + off + (size_t)h * kD + c * 8, in);
+    }
+}
+
+// Bound by a chunk's steps one after another (loads and cuts of k, products, the state's update; 4.6 us a chunk, the tensor pipe 18 % busy): 128 rows of the
+// state by 128 columns in registers, a row and 32 columns a thread.  As many segments as fill the device, because the alternative, what every chunk adds and a
+// scan over it, reads and writes the states (134 MB for 8,192 tokens of 32 heads) once more.
+__global__ void __launch_bounds__(kThreads, 1)
+retention_states_kernel(const Retention p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u, keys = base, values = base + 3 * kTerm;
+    __shared__ Shared sh;
+    __shared__ float power[kT + 1];
+    const int e = blockIdx.x / p.segments, seg = blockIdx.x - e * p.segments, h = blockIdx.y;
+    const int t_first = p.cu_q[e], t_last = p.cu_q[e + 1];
+    const int c0 = seg * p.seg_chunks, c1 = min(c0 + p.seg_chunks, ceil_div(t_last - t_first, kT));
+    if (c0 >= c1) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = (warp & 3) * 32 + lane, col = (warp >> 2) * 32;
+    for (int i = threadIdx.x; i <= kT; i += kThreads) power[i] = p.powers[(size_t)h * p.powers_pitch + i];
+    const uint32_t tmem = begin(sh);
+    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + col;
+    float S[32];
+    float* own = p.state + (size_t)p.seq_rows[e] * p.state_stride + ((size_t)h * kD + row) * kD + col;
+#pragma unroll
+    for (int c = 0; c < 32; c += 4) {
+        const float4 v = seg == 0 ? ld4(own + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        S[c] = v.x; S[c + 1] = v.y; S[c + 2] = v.z; S[c + 3] = v.w;
+    }
+    auto store = [&](float* to) {                    // [column][row]
+#pragma unroll
+        for (int c = 0; c < 32; ++c) to[(size_t)(col + c) * kD + row] = S[c];
+    };
+    uint32_t round = 0;
+    for (int c = c0; c < c1; ++c, ++round) {
+        const int first = t_first + c * kT, n = min(kT, t_last - first);
+        fetch_rows(p, values, p.v_off, first, n, h);
+        walk::cp_commit();
+        put_keys(p, keys, first, n, h, [&](int t) { return t < n ? power[n - 1 - t] : 0.f; });
+        walk::cp_wait<0>();
+        fence_smem();
+        fence_before();                              // the last chunk's sums have been read
+        __syncthreads();
+        if (warp == 0) {
+            fence_after();
+            if (fa::elect_one()) {
+                product<true, true, 1>(tmem, keys, kHalf, kTerm, values, kHalf, kTerm, instr(kD, true, true));
+                fa::umma_commit(smem_u32(&sh.done));
+            }
+            __syncwarp();
+        }
+        store(p.states + ((size_t)(t_first / kT + e + c) * p.H + h) * (kD * kD));
+        if (!products_done(sh, round, p.error)) break;
+        uint32_t v[32];
+        fa::tmem_ld32(mine, v);
+        wait_ld();
+        float z = 0.f;
+#pragma unroll
+        for (int x = 0; x < 32; ++x) z = fmaf(__uint_as_float(v[x]), 0.f, z);
+        const float total = power[n];
+        if (!__syncthreads_or(z != 0.f)) {
+#pragma unroll
+            for (int x = 0; x < 32; ++x) S[x] = fmaf(total, S[x], __uint_as_float(v[x]));
+        } else {
+#pragma unroll 1
+            for (int t = 0; t < n; ++t) {
+                const float k = key_of(p, (size_t)first + t, h, row);
+                const __nv_bfloat16* vr = p.proj + (size_t)(first + t) * p.pitch + p.v_off + (size_t)h * kD + col;
+#pragma unroll
+                for (int x = 0; x < 32; ++x) S[x] = fmaf(power[1], S[x], k * __bfloat162float(vr[x]));
+            }
+        }
+    }
+    if (p.segments > 1) store(p.starts + ((size_t)blockIdx.x * p.H + h) * (kD * kD));
+    else
+#pragma unroll
+        for (int c = 0; c < 32; c += 4) *reinterpret_cast<float4*>(own + c) = make_float4(S[c], S[c + 1], S[c + 2], S[c + 3]);
+    end(sh);
+}
+
+// A segment's end by itself -> the state at its start; the last one goes back to the entry's row.  32 x 32 elements a block.
+__global__ void __launch_bounds__(256)
+retention_join_kernel(const Retention p) {
+    __shared__ float turned[32][33];
+    const int e = blockIdx.z, h = blockIdx.y, c0 = (blockIdx.x >> 2) * 32, r0 = (blockIdx.x & 3) * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int len = p.cu_q[e + 1] - p.cu_q[e], chunks = ceil_div(len, kT);
+    if (len <= 0) return;
+    const float* power = p.powers + (size_t)h * p.powers_pitch;
+    float S[4] = {};
+    const int most = min(p.segments, ceil_div(chunks, p.seg_chunks));
+    for (int seg0 = 0; seg0 < most; seg0 += 4) {     // four segments asked for together
+        float left[4][4];
+        float* at = p.starts + ((size_t)(e * p.segments + seg0) * p.H + h) * (kD * kD) + r0 + tx;
+        const size_t step = (size_t)p.H * kD * kD;
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) left[x][i] = seg0 + x < most ? at[x * step + (size_t)(c0 + ty + 8 * i) * kD] : 0.f;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            if (seg0 + x >= most) break;
+            const int tokens = min(len - (seg0 + x) * p.seg_chunks * kT, p.seg_chunks * kT);
+            const float f = power[kT + 1 + tokens / kT] * power[tokens % kT];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (seg0 + x) at[x * step + (size_t)(c0 + ty + 8 * i) * kD] = S[i];
+                S[i] = seg0 + x ? fmaf(f, S[i], left[x][i]) : left[x][i];
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) turned[ty + 8 * i][tx] = S[i];
+    __syncthreads();
+    float* own = p.state + (size_t)p.seq_rows[e] * p.state_stride + (size_t)h * kD * kD;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) own[(size_t)(r0 + ty + 8 * i) * kD + c0 + tx] = turned[tx][ty + 8 * i];
+}
+
+// A block takes chunks in turn.  The next chunk's q, k and angles are fetched into room that this one's products have left (the state's terms, the last of
+// k's) while its weights are made and P v runs; the state comes into registers meanwhile.  Bound by the steps of a chunk, 17 us, one after another: the
+// products take 8,000 cycles of 33,000, instructions issue in 30 %.  Measured, 8,192 tokens of 32 heads: 247 us; q and angles row by row from memory 292;
+// a warp group per operand, which leaves 64 to 112 registers a thread and spills, 253 to 288; a warp that only issues products, 112 registers, 274.
+//   columns of tensor memory: q's terms, then P's 0-191; scores, then P v 192-319; what the state gives 320-447
+__global__ void __launch_bounds__(kThreads, 1)
+retention_outputs_kernel(const Retention p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u, keys = base, state = base + 3 * kTerm, values = base + 6 * kTerm;
+    const uint32_t raw_k = keys + 2 * kTerm, raw_q = state, angles = state + kTerm;       // angles: [128][64] cosines and sines, 16-byte pieces of a row in the order of its last three bits
+    uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
+    float* plain = reinterpret_cast<float*>(sm);                                          // for the form token by token
+    float (*squares)[kT] = reinterpret_cast<float (*)[kT]>(sm + 2 * kTerm - 4 * kT * 4);  // at the end of k's second term
+    __shared__ Shared sh;
+    __shared__ float power[kT + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp >> 2, row = (warp & 3) * 32 + lane, col = part * 32, quad = lane & 15;
+    const uint32_t tmem = (uint32_t)fa::uniform((int)begin(sh));
+    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16), scores = 192, old = 320;
+    const bool issuer = fa::uniform(warp) == 0;
+    uint32_t round = 0;
+    int last_h = -1;
+    bool ok = true;
+    struct Item { int e, h, first, n, place, seg, inner; };      // inner: the chunk's number in its segment
+    __shared__ Item items[2];                        // this item and the next one, n = 0 after the last
+    int at = blockIdx.x;
+    auto find = [&](Item& t) {                       // by one thread
+        t.n = 0;
+        for (; at < p.places * p.H && t.n <= 0; at += gridDim.x) {
+            const int place = at / p.H;
+            int first, n;
+            const int e = chunk_of<kT>(place, p.cu_q, p.entries, first, n);
+            if (n <= 0) continue;
+            const int chunk = place - p.cu_q[e] / kT - e, seg = chunk / p.seg_chunks;
+            if (seg < p.segments) t = Item{e, at - place * p.H, first, n, place, seg, chunk - seg * p.seg_chunks};     // (else an entry longer than the host knew)
+        }
+        t.n = max(t.n, 0);
+    };
+    auto fetch = [&](const Item& t) {
+        fetch_rows(p, raw_k, p.k_off, t.first, t.n, t.h);
+        fetch_rows(p, raw_q, p.q_off, t.first, t.n, t.h);
+        if (p.turn != nullptr)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int x = i * kThreads + threadIdx.x, r = x >> 5, c = x & 31;
+                cp16(angles + r * 512 + ((c ^ (r & 7)) << 4), p.turn + (size_t)(t.first + min(r, t.n - 1)) * 64 + 2 * c, true);
+            }
+        walk::cp_commit();
+    };
+    auto angle = [&](int r, int c) {                 // of pairs 2 c and 2 c + 1 of row r
+        return p.turn != nullptr ? *reinterpret_cast<const float4*>(sm + 4 * kTerm + r * 512 + ((c ^ (r & 7)) << 4)) : make_float4(1.f, 0.f, 1.f, 0.f);
+    };
+    if (threadIdx.x == 32) find(items[0]);
+    __syncthreads();
+    if (items[0].n > 0) fetch(items[0]);
+    for (uint32_t j = 0; items[j & 1].n > 0; ++j) {
+        const Item& t = items[j & 1];
+        const Item& next = items[(j & 1) ^ 1];
+        const int first = t.first, n = t.n, h = t.h;
+        const bool in = row < n;
+        if (h != last_h) {                           // (read last before the barriers of the item before)
+            for (int i = threadIdx.x; i <= kT; i += kThreads) power[i] = p.powers[(size_t)h * p.powers_pitch + i];
+            last_h = h;
+        }
+        const float* S = p.states + ((size_t)t.place * p.H + h) * (kD * kD);
+        const float* S_seg = t.seg > 0 ? p.starts + ((size_t)(t.e * p.segments + t.seg) * p.H + h) * (kD * kD) : nullptr;
+        const float lead = p.powers[(size_t)h * p.powers_pitch + kT + 1 + t.inner];
+        float4 own_S[4];                             // the state at the chunk's start: a column of it per warp at a time, half of them ahead
+#pragma unroll
+        for (int i = 0; i < 4; ++i) own_S[i] = ld4(S + (size_t)(16 * i + warp) * kD + 4 * lane);
+        walk::cp_wait<0>();
+        __syncthreads();                             // k, q and angles are there
+        fetch_rows(p, values, p.v_off, first, n, h);
+        walk::cp_commit();
+        {
+            uint2 lo[4], hi[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = 32 * i + 2 * warp + (lane >> 4);
+                const uint8_t* from = sm + 2 * kTerm + fa::sw128(r, quad >> 1) + (quad & 1) * 8;
+                lo[i] = *reinterpret_cast<const uint2*>(from);
+                hi[i] = *reinterpret_cast<const uint2*>(from + kHalf);
+            }
+            __syncthreads();                         // before the last of k's terms takes its place
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = 32 * i + 2 * warp + (lane >> 4);
+                put_pairs(keys, r, quad, lo[i], hi[i], angle(r, 2 * quad), angle(r, 2 * quad + 1), p.k_scale);
+            }
+        }
+        // q: a row and 16 pairs of columns a thread, to tensor memory
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const uint8_t* from = sm + 3 * kTerm + fa::sw128(row, part * 2 + x);
+            const uint4 a = *reinterpret_cast<const uint4*>(from), b = *reinterpret_cast<const uint4*>(from + kHalf);
+            const uint32_t a4[4] = {a.x, a.y, a.z, a.w}, b4[4] = {b.x, b.y, b.z, b.w};
+            uint32_t lo[3][4], hi[3][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float a0 = __uint_as_float(a4[j] << 16), a1 = __uint_as_float(a4[j] & 0xffff0000u), b0 = __uint_as_float(b4[j] << 16), b1 = __uint_as_float(b4[j] & 0xffff0000u);
+                const float4 cs = angle(row, part * 8 + 4 * x + j);
+                rotate(make_float2(cs.x, cs.y), a0, b0);
+                rotate(make_float2(cs.z, cs.w), a1, b1);
+                uint32_t w[3];
+                cut(a0, a1, w);
+#pragma unroll
+                for (int y = 0; y < 3; ++y) lo[y][j] = w[y];
+                cut(b0, b1, w);
+#pragma unroll
+                for (int y = 0; y < 3; ++y) hi[y][j] = w[y];
+            }
+#pragma unroll
+            for (int y = 0; y < 3; ++y) {
+                st4(mine + y * 64 + part * 8 + 4 * x, lo[y]);
+                st4(mine + y * 64 + 32 + part * 8 + 4 * x, hi[y]);
+            }
+        }
+        wait_st();
+        fence_smem();
+        fence_before();
+        __syncthreads();                             // q and the angles have been read
+        if (issuer) {
+            fence_after();
+            if (fa::elect_one()) {
+                product_ts<false, 3>(tmem + scores, tmem, keys, kHalf, kTerm, instr(kT, false, false));
+                fa::umma_commit(smem_u32(&sh.done));
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) {
+            float4 seg[4];
+            if (i > 0)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) own_S[j] = ld4(S + (size_t)(16 * (i + j) + warp) * kD + 4 * lane);
+            if (S_seg != nullptr)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) seg[j] = ld4(S_seg + (size_t)(16 * (i + j) + warp) * kD + 4 * lane);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float4 v = own_S[j];
+                if (S_seg != nullptr) v = make_float4(fmaf(lead, seg[j].x, v.x), fmaf(lead, seg[j].y, v.y), fmaf(lead, seg[j].z, v.z), fmaf(lead, seg[j].w, v.w));
+                put4(state + (lane >> 4) * kHalf, kTerm, 16 * (i + j) + warp, quad, v);
+            }
+        }
+        walk::cp_wait<0>();
+        fence_smem();
+        __syncthreads();
+        if (issuer) {                                // (one barrier: the scores' end is waited for before this one's is committed)
+            if (fa::elect_one()) product_ts<false, 3>(tmem + old, tmem, state, kHalf, kTerm, instr(kD, false, false));
+            __syncwarp();
+        }
+        if (threadIdx.x == 32) find(items[(j & 1) ^ 1]);
+        if (!(ok = products_done(sh, round++, p.error))) break;
+        if (issuer) {
+            if (fa::elect_one()) fa::umma_commit(smem_u32(&sh.done));
+            __syncwarp();
+        }
+        {
+            uint32_t v[32], w[3][8];
+            if (col <= (row | 31)) {
+                fa::tmem_ld32(mine + scores + col, v);
+                wait_ld();
+            }
+            fence_before();
+            auto weights = [&](int half) {
+#pragma unroll
+                for (int x = 0; x < 16; x += 2) {    // (the table's index is one of its own also where it is not used)
+                    const int s = col + 16 * half + x;
+                    const float fa_ = power[(row - s) & 127], fb = power[(row - s - 1) & 127];
+                    const float a = s <= row ? __uint_as_float(v[16 * half + x]) * fa_ : 0.f, b = s < row ? __uint_as_float(v[16 * half + x + 1]) * fb : 0.f;
+                    uint32_t c[3];
+                    cut(a, b, c);
+#pragma unroll
+                    for (int y = 0; y < 3; ++y) w[y][x / 2] = c[y];
+                }
+            };
+            weights(0);
+            if (!(ok = products_done(sh, round++, p.error))) break;          // q's terms give way
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                if (half) weights(1);
+#pragma unroll
+                for (int y = 0; y < 3; ++y) st8(mine + y * 64 + part * 16 + 8 * half, w[y]);
+            }
+        }
+        wait_st();
+        fence_before();
+        __syncthreads();
+        if (issuer) {
+            fence_after();
+            if (fa::elect_one()) {
+                product_ts<true, 1>(tmem + scores, tmem, values, kHalf, kTerm, instr(kD, false, true));
+                fa::umma_commit(smem_u32(&sh.done));
+            }
+            __syncwarp();
+        }
+        if (next.n > 0) fetch(next);
+        const size_t out_at = ((size_t)(first + row) * p.H + h) * kD + col;
+        const uint4* gate = reinterpret_cast<const uint4*>(p.proj + (size_t)(first + (in ? row : 0)) * p.pitch + p.g_off + (size_t)h * kD + col);
+        uint4 gates[4];
+        if (p.out != nullptr)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) gates[x] = gate[x];
+        float o[32];
+        const float f = power[row + 1];
+        {
+            uint32_t v[32];
+            fa::tmem_ld32(mine + old + col, v);
+            wait_ld();
+#pragma unroll
+            for (int x = 0; x < 32; ++x) o[x] = f * __uint_as_float(v[x]);
+        }
+        if (!(ok = products_done(sh, round++, p.error))) break;
+        float z = 0.f, sum = 0.f;
+        {
+            uint32_t v[32];
+            fa::tmem_ld32(mine + scores + col, v);
+            wait_ld();
+#pragma unroll
+            for (int x = 0; x < 32; ++x) {
+                o[x] += __uint_as_float(v[x]);
+                z = fmaf(o[x], 0.f, z);
+                sum = fmaf(o[x], o[x], sum);
+            }
+        }
+        squares[part][row] = sum;
+        fence_before();
+        if (__syncthreads_or(z != 0.f)) {            // token by token: a column of the state and 32 rows a thread
+            walk::cp_wait<0>();                      // what has been fetched for the next chunk is fetched again afterwards
+            __syncthreads();
+            float* qs = plain;                       // [128][128]
+            float* ks = qs + kT * kD;
+            float* os = ks + kT * kD;
+            float* sums = os + kT * kD;              // [2][4][128]
+#pragma unroll 1
+            for (int x = threadIdx.x; x < kT * kD; x += kThreads) {
+                qs[x] = x / kD < n ? column_of(p, p.q_off, (size_t)first + x / kD, h, x % kD) : 0.f;
+                ks[x] = x / kD < n ? key_of(p, (size_t)first + x / kD, h, x % kD) : 0.f;
+            }
+            const int c = threadIdx.x & 127, r0 = (threadIdx.x >> 7) * 32;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                o[j] = S[(size_t)c * kD + r0 + j];
+                if (S_seg != nullptr) o[j] = fmaf(lead, S_seg[(size_t)c * kD + r0 + j], o[j]);
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (int i = 0; i < n; ++i) {
+                const float v = __bfloat162float(p.proj[(size_t)(first + i) * p.pitch + p.v_off + (size_t)h * kD + c]);
+                float x = 0.f;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    o[j] = fmaf(power[1], o[j], ks[i * kD + r0 + j] * v);
+                    x = fmaf(qs[i * kD + r0 + j], o[j], x);
+                }
+                float* to = sums + (i & 1) * 4 * kD;
+                to[(r0 / 32) * kD + c] = x;
+                __syncthreads();
+                if (r0 == 0) os[i * kD + c] = (to[c] + to[kD + c]) + (to[2 * kD + c] + to[3 * kD + c]);
+            }
+            __syncthreads();
+            sum = 0.f;
+#pragma unroll
+            for (int x = 0; x < 32; ++x) {
+                o[x] = in ? os[row * kD + col + x] : 0.f;
+                sum = fmaf(o[x], o[x], sum);
+            }
+            __syncthreads();
+            squares[part][row] = sum;
+            __syncthreads();
+            if (next.n > 0) fetch(next);
+        }
+        if (in && p.out == nullptr) {
+#pragma unroll
+            for (int x = 0; x < 32; x += 8) store8(p.o + out_at + x, o + x);
+        } else if (in) {
+            const float inv = 1.0f / sqrtf(((squares[0][row] + squares[1][row]) + (squares[2][row] + squares[3][row])) / (float)kD + p.eps);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const uint32_t g4[4] = {gates[x].x, gates[x].y, gates[x].z, gates[x].w};
+                float u[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float g = __uint_as_float(i & 1 ? g4[i / 2] & 0xffff0000u : g4[i / 2] << 16);
+                    u[i] = o[8 * x + i] * inv * __fdividef(g, 1.f + __expf(-g));
+                }
+                store8(p.out + out_at + 8 * x, u);
+            }
+        }
+    }
+    walk::cp_wait<0>();
+    end(sh);
+}
+
+static bool aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+}  // namespace tiles
+}  // namespace se
+
+using namespace se::tiles;
+
+// 1 for what the kernels below take: heads of 128 x 128, all of a head's columns turned or none
+extern "C" int se_retention_tiles_supported(int d, int dv, int rotary) { return d == kD && dv == kD && (rotary == 0 || rotary == kD); }
+
+// work: float [(tokens / 128 + entries) * heads * 128 * 128 (the chunks' states) + (segments > 1 ? entries * segments : 0) * heads * 128 * 128
+// + heads * (130 + seg_chunks) rounded up to 4 + (rotary ? tokens * 128 : 0)].  An entry's chunks in `segments` of seg_chunks (all of the longest entry's).
+// out: after norm and gate (columns from g_off on), or null: o.
+extern "C" int se_retention_tiles(const void* proj, int pitch, int q_off, int k_off, int v_off, int g_off, const float* inv_freq, const int* positions,
+                                  int rotary, float k_scale, const float* decay, float* state, long long state_stride, const int* cu_q,
+                                  const int* seq_rows, void* out, float* o, float eps, float* work, int* error, int tokens, int entries, int heads, int d,
+                                  int dv, int segments, int seg_chunks, int sms, cudaStream_t stream) {
+    if (entries <= 0 || tokens <= 0) return 0;
+    if (!se_retention_tiles_supported(d, dv, rotary) || heads <= 0 || heads > 65535 || entries > 65535) return SE_ERR_UNSUPPORTED;
+    if (segments < 1 || seg_chunks < 1 || (out == nullptr) == (o == nullptr) || (rotary && (inv_freq == nullptr || positions == nullptr))) return SE_ERR_ARGUMENT;
+    if (pitch % 8 || q_off % 8 || k_off % 8 || v_off % 8 || g_off % 8 || state_stride % 4 || !aligned(proj) || !aligned(work) || !aligned(state) ||
+        (out != nullptr && !aligned(out)) || (o != nullptr && !aligned(o)))
+        return SE_ERR_UNSUPPORTED;
+    const long long places = tokens / kT + entries;
+    if (places * heads > 0x7fffffffLL || (long long)entries * segments > 0x7fffffffLL || (long long)tokens * 64 > 0x7fffffffLL - 256) return SE_ERR_UNSUPPORTED;
+    Retention p = {};
+    p.proj = (const __nv_bfloat16*)proj; p.pitch = pitch; p.q_off = q_off; p.k_off = k_off; p.v_off = v_off; p.g_off = g_off;
+    p.states = work;
+    p.starts = p.states + (size_t)places * heads * kD * kD;
+    p.powers_pitch = kT + 2 + seg_chunks;
+    float* powers = p.starts + (segments > 1 ? (size_t)entries * segments * heads * kD * kD : 0);
+    float2* turn = reinterpret_cast<float2*>(powers + ((size_t)heads * p.powers_pitch + 3) / 4 * 4);
+    p.powers = powers; p.turn = rotary ? turn : nullptr;
+    p.segments = segments; p.seg_chunks = seg_chunks; p.state = state; p.state_stride = state_stride; p.cu_q = cu_q; p.seq_rows = seq_rows;
+    p.entries = entries; p.H = heads; p.places = (int)places; p.k_scale = k_scale; p.eps = eps; p.out = (__nv_bfloat16*)out; p.o = o; p.error = error;
+    const int turn_blocks = rotary ? (tokens * 64 + 255) / 256 : 0, states_smem = 4 * kTerm + 1024, outputs_smem = 7 * kTerm + 1024;
+    retention_tables_kernel<<<turn_blocks + heads, 256, 0, stream>>>(turn, positions, inv_freq, tokens, turn_blocks, powers, p.powers_pitch, decay);
+    cudaError_t e = cudaFuncSetAttribute(retention_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, states_smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(retention_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, outputs_smem);
+    if (e != cudaSuccess) return (int)e;
+    retention_states_kernel<<<dim3(entries * segments, heads), kThreads, states_smem, stream>>>(p);
+    if (segments > 1) retention_join_kernel<<<dim3(16, heads, entries), 256, 0, stream>>>(p);
+    const long long items = places * heads;
+    retention_outputs_kernel<<<(int)(items < sms ? items : sms), kThreads, outputs_smem, stream>>>(p);
+    SE_LAUNCH_CHECK();
+}

@@ -300,6 +300,15 @@ class RetentionMixer(Mixer):
             return step.max_q_len > 64 and 2.5 * step.num_seqs * share < max(0.25 * step.max_q_len, 6 * further * share)
         return once_per_step(step, ("retention.in_walk", s.num_heads, s.v_head_dim), ask)
 
+    def in_tiles(self, step, tokens: int, rotary_dim: int, device) -> bool:
+        """Whether a step in chunks that csrc/retention_tiles.cu takes (bfloat16, heads of 128 x 128) goes there: it is ahead or level from 17 tokens
+        on, beside whatever single tokens (a layer's call, us before / now, 16 and 32 heads: one portion of 17 tokens 103/87 and 75/74, of 128
+        101/86 and 79/80, of 512 80/67 and 132/113, of 8,192 774/400 and 1,534/1,207; 90 tokens beside 63 single ones 444/221 and
+        878/407; 64 entries of 96 719/440 and 1,754/1,172), as long as its workspace, 64 KB per head and entry or 128 tokens, is no
+        larger than that of the other forms or 256 MB."""
+        heads = self.spec.num_heads
+        return ops.retention_tiles_plan(step, tokens, heads, rotary_dim, device)[2] <= max(1 << 26, tokens * heads * 322)
+
     def forward(self, x, step, slot, proj=None):
         s = self.spec
         tokens, dev = x.shape[0], x.device
@@ -318,6 +327,16 @@ class RetentionMixer(Mixer):
         # a step with a prompt portion takes the recurrence in chunks of 64 tokens (closed form per chunk);
         # steps of single tokens and of short pieces walk it token by token
         chunked = self.chunk_min_tokens is not None and step.max_q_len >= self.chunk_min_tokens
+        if (chunked and not silu and ops.retention_tiles_supported(s.head_dim, s.v_head_dim, rotary_dim, proj, slot.state, self.qk, self.vv)
+                and self.in_tiles(step, tokens, rotary_dim, dev)):
+            out = torch.empty(tokens, self.vv, dtype=x.dtype, device=dev)
+            normed = s.output_norm == "per_head"
+            ops.retention_tiles(proj, 0, self.qk, 2 * self.qk, 2 * self.qk + self.vv, self.k_scale,
+                                (inv_freq, rotary_dim, step.positions) if rotary_dim else None, self._decay, slot.state, step, heads=s.num_heads,
+                                head_dim=s.head_dim, v_head_dim=s.v_head_dim, eps=s.norm_eps, **({"out": out} if normed else {"o": o}))
+            if not normed:
+                ops.retention_out_joint(o, proj, 2 * self.qk + self.vv, self.norm_w, out, eps=s.norm_eps)
+            return linear(out, self.o)
         args = (proj, 2 * self.qk, self._decay, slot.state, step, o)
         sizes = dict(heads=s.num_heads, head_dim=s.head_dim, v_head_dim=s.v_head_dim, silu=silu)
         if not chunked and rotary_dim == 0:      # q and k straight from the projection, as they are staged

@@ -1,0 +1,102 @@
+"""Linear recurrences by chunks of 128 tokens side by side (csrc/chunk_tiles.cuh) against 64-bit walks token by token, from non-zero states, with entries that
+end on, before and behind the chunks' edges."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from test_chunk_walk_gpu import _close, _walk64
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _step(lens):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    rows = [(3 * i + 1) % (len(lens) + 2) for i in range(len(lens))] if len(lens) % 3 != 1 else list(range(len(lens)))
+    return SimpleNamespace(cu_q=torch.tensor(cu, **i32), seq_rows=torch.tensor(rows, **i32), num_seqs=len(lens), num_tokens=cu[-1],
+                           max_q_len=max(lens), cu=cu, rows=rows)
+
+
+def _retention(lens, heads, rotary, decay, bad=None, out=False):
+    from sparseengine_b200.csrc import ops
+    d, step = 128, _step(lens)
+    T, g = step.num_tokens, torch.Generator(device=DEV).manual_seed(heads)
+    proj = torch.randn(T, 8 + 4 * heads * d, generator=g, device=DEV).to(torch.bfloat16)      # v, 8 columns that nobody reads, k, q, gate
+    v_off, k_off, q_off, g_off = 0, heads * d + 8, 2 * heads * d + 8, 3 * heads * d + 8
+    decays = torch.exp(-torch.rand(heads, generator=g, device=DEV) * (20.0 if decay == "fast" else 0.03))
+    state = torch.randn(len(lens) + 2, heads * d * d + 4, generator=g, device=DEV)
+    inv, positions = torch.rand(64, generator=g, device=DEV), torch.arange(T, device=DEV, dtype=torch.int32) * 37 % 101
+    if bad is not None:
+        proj[bad[0], {"q": q_off, "k": k_off, "v": v_off}[bad[1]] + 5] = bad[2]
+    first = state.clone()
+    assert ops.retention_tiles_supported(d, d, rotary, proj, state, q_off, k_off, v_off, g_off)
+    to = dict(out=torch.empty(T, heads * d, dtype=torch.bfloat16, device=DEV)) if out else dict(o=torch.full((T, heads * d), float("nan"), device=DEV))
+    got = ops.retention_tiles(proj, q_off, k_off, v_off, g_off, d ** -0.5, (inv, rotary, positions) if rotary else None, decays, state, step,
+                              heads=heads, head_dim=d, v_head_dim=d, eps=1e-6, **to)
+    ops.error_check(DEV)
+    q, k, v = (proj[:, f:f + heads * d].double().view(T, heads, d) for f in (q_off, k_off, v_off))
+    if rotary:
+        a = (positions.float()[:, None] * inv).double()[:, None]
+        q, k = (torch.cat([x[..., :64] * a.cos() - x[..., 64:] * a.sin(), x[..., 64:] * a.cos() + x[..., :64] * a.sin()], -1) for x in (q, k))
+    return step, got, first, state, (q, k * d ** -0.5, v, decays.double().view(1, heads, 1).expand(T, -1, -1)), proj[:, g_off:]
+
+
+@pytest.mark.parametrize("decay", ["slow", "fast"])
+@pytest.mark.parametrize("rotary", [0, 128])
+@pytest.mark.parametrize("lens,heads", [([1, 127, 128, 129, 0, 300, 64, 17], 3), ([1500], 2), ([257], 40)])       # the second: several segments of chunks
+def test_retention_against_the_walk(lens, heads, rotary, decay):
+    step, o, first, state, inputs, _ = _retention(lens, heads, rotary, decay)
+    d = 128
+    for e, n in enumerate(lens):
+        a, b, row = step.cu[e], step.cu[e + 1], step.rows[e]
+        if n == 0:
+            assert torch.equal(state[row], first[row])
+            continue
+        want, S = _walk64(*(x[a:b] for x in inputs), first[row, :heads * d * d].double().view(heads, d, d))
+        _close(o[a:b].view(n, heads, d), want, f"outputs of {n} tokens")
+        _close(state[row, :heads * d * d].view(heads, d, d), S, f"state after {n} tokens")
+    others = [r for r in range(len(lens) + 2) if r not in step.rows]
+    assert torch.equal(state[others], first[others]) and torch.equal(state[:, heads * d * d:], first[:, heads * d * d:])
+
+
+def test_retention_with_norm_and_gate():
+    _, o, _, _, _, gate = _retention([200, 5], 2, 128, "slow")
+    _, y, _, _, _, _ = _retention([200, 5], 2, 128, "slow", out=True)
+    o = o.double().view(-1, 2, 128)
+    want = (o / torch.sqrt((o * o).mean(-1, keepdim=True) + 1e-6)).view(-1, 256) * torch.nn.functional.silu(gate.double())
+    # rounded to the nearest of 8 bits: half a step is at most 2^-8 of the value; the 32-bit value before it 1e-5 (the gate's fast exponential and quotient)
+    assert bool(((y.double() - want).abs() <= want.abs() * (2.0 ** -8 + 1e-5) + 1e-30).all())
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["q", "k", "v"])
+@pytest.mark.parametrize("out", [False, True])
+def test_retention_inputs_that_are_not_finite_stay_with_their_token_and_later_ones(where, value, out):
+    """Token 150 of 400: the second of four chunks, head 0 of two."""
+    lens, t = [400], 150
+    _, want, _, s_want, _, _ = _retention(lens, 2, 128, "slow", out=out)
+    _, got, _, s_got, _, _ = _retention(lens, 2, 128, "slow", bad=(t, where, value), out=out)
+    want, got = want.float(), got.float()
+    # its chunk is done again token by token: another order of the same sums, within a step of what is stored
+    near = dict(rtol=2.0 ** -7 if out else 1e-4, atol=1e-4)
+    assert torch.equal(got[:128], want[:128]) and torch.equal(got[:, 128:], want[:, 128:])
+    torch.testing.assert_close(got[128:t], want[128:t], **near)
+    if where == "q":
+        assert not bool(torch.isfinite(got[t, :128]).any())
+        torch.testing.assert_close(got[t + 1:], want[t + 1:], **near)
+        assert torch.equal(s_got, s_want)
+    else:
+        assert not bool(torch.isfinite(got[t:, :128]).all(1).any()) and not bool(torch.isfinite(s_got[0, :128 * 128]).all())
+        assert torch.equal(s_got[0, 128 * 128:], s_want[0, 128 * 128:])
+
+
+def test_retention_mixer_keeps_to_the_other_forms_beyond_its_workspace():
+    from sparseengine_b200.config.specs import RetentionSpec
+    from sparseengine_b200.parts.base import make_mixer
+    part = make_mixer(RetentionSpec(hidden_size=64, num_heads=32, head_dim=128, v_head_dim=128, decays=(0.9,) * 32, position=None), torch.bfloat16)
+    few, many = (SimpleNamespace(num_seqs=n, max_q_len=20) for n in (64, 512))
+    assert part.in_tiles(few, 20 + 63, 0, DEV) and not part.in_tiles(many, 20 + 511, 0, DEV)
