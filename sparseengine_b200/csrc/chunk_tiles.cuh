@@ -133,7 +133,7 @@ struct Shared {
 __device__ __forceinline__ uint32_t begin(Shared& s) {
     if (threadIdx.x == 0) {
         fa::mbar_init(smem_u32(&s.done), 1);
-        fa::mbar_init(smem_u32(&s.last), 1);
+        fa::mbar_init(smem_u32(&s.last), 2);
         s.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -150,10 +150,12 @@ __device__ __forceinline__ void end(Shared& s) {
     const uint32_t tmem = s.tmem;
     fence_before();
     __syncthreads();
+    if (threadIdx.x < 64) {                          // what the first two warps issued ends before its memory is given back
+        if (fa::elect_one()) fa::umma_commit(smem_u32(&s.last));
+        __syncwarp();
+    }
     if (threadIdx.x < 32) {
         fence_after();
-        if (fa::elect_one()) fa::umma_commit(smem_u32(&s.last));           // what was issued ends before its memory is given back
-        __syncwarp();
         fa::mbar_drain(smem_u32(&s.last), 0);
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
     }

@@ -5,27 +5,6 @@
 namespace se {
 namespace walk {
 
-// A token's log decay, -rate * step, no further down than -1e4: a decay below e^-104 is 0 in 32-bit, and with an infinite rate or step
-// the sums would be infinite and their differences NaN.  Sums of 64 such terms differ by less than 1e-10 from what they should.  NaN
-// stays NaN.
-__device__ __forceinline__ double log_decay(float rate, float step) {
-    const double v = -(double)rate * (double)step;
-    return v < -1e4 ? -1e4 : v;
-}
-
-// The sum of the lanes' `own` (returned) and, in `before`, that of the lanes below: shifted, not the sum less `own`, so that a
-// lane's infinity or NaN reaches no prefix but those of the lanes above.
-__device__ __forceinline__ double sum_before(double own, int lane, double& before) {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double v = __shfl_up_sync(0xffffffffu, own, o);
-        if (lane >= o) own += v;
-    }
-    before = __shfl_up_sync(0xffffffffu, own, 1);
-    if (lane == 0) before = 0.0;
-    return __shfl_sync(0xffffffffu, own, 31);
-}
-
 // State space: one block per (chunk, group of heads that share B and C).  step = softplus(raw + bias), the log decay is
 // -exp(A_log) step; P[t][s] = e^(B_t - B_s) C_t . B_s; the step sizes become the factor on the value rows.
 template <int DP, typename T_>

@@ -26,7 +26,7 @@ _fns: dict = {}
 
 # Kernels launched through these bindings since the process started (a launcher that
 # starts two kernels counts two).  Benchmarks read the difference around a timed region.
-KERNELS_PER_CALL = {"se_attn_decode": 2, "se_router": 2, "se_causal_conv": 2, "se_ssm_scan": 2, "se_retention_chunk": 2, "se_ssm_walk": 2, "se_delta_walk": 2, "se_retention_tiles": 4}   # upper bounds per call
+KERNELS_PER_CALL = {"se_attn_decode": 2, "se_router": 2, "se_causal_conv": 2, "se_ssm_scan": 2, "se_retention_chunk": 2, "se_ssm_walk": 2, "se_delta_walk": 2, "se_retention_tiles": 4, "se_ssm_tiles": 3}   # upper bounds per call
 launch_count = 0
 calls: dict = {}     # launcher name -> times called (tests check which kernels a path took)
 
@@ -843,6 +843,24 @@ def ssm_walk(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, step, y, *, 
         _ptr(state, torch.float32, "state"), state.stride(0), _ptr(step.cu_q), _ptr(step.seq_rows), _ptr(y, torch.float32, "y"),
         work.data_ptr(), tokens, step.num_seqs, heads, head_dim, state_size, groups, sm_count(xbc.device), dtype_code(proj.dtype),
         _stream()), "ssm_walk")
+    return y
+
+
+def ssm_tiles_supported(state_size: int, head_dim: int, proj, state) -> bool:
+    """Whether :func:`ssm_tiles` takes these sizes (what ``se_ssm_tiles_supported`` answers, restated) and the state's rows."""
+    return state_size == 128 and head_dim == 64 and proj.dtype == torch.bfloat16 and state.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0
+
+
+def ssm_tiles(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, step, y, *, heads, head_dim, state_size, groups):
+    """The recurrence of :func:`ssm_walk` in chunks of 128 tokens side by side on tcgen05 (csrc/ssm_tiles.cu)."""
+    tokens, n = xbc.shape[0], step.num_seqs
+    work = _walk_work((tokens // 128 + n) * heads * (head_dim * state_size + 1), xbc.device)
+    _check(_fn("se_ssm_tiles", "ppii" "ppp" "pl" "pp" "ppp" "iiiiiiii" "p")(
+        _ptr(xbc, torch.float32, "xbc"), _rows_ptr(proj, "proj"), proj.stride(0), int(dt_off),
+        _ptr(dt_bias, torch.float32, "dt_bias"), _ptr(a_log, torch.float32, "a_log"), _ptr(d_skip, torch.float32, "d_skip"),
+        _ptr(state, torch.float32, "state"), state.stride(0), _ptr(step.cu_q), _ptr(step.seq_rows), _ptr(y, torch.float32, "y"),
+        work.data_ptr(), _ptr(error_word(xbc.device)), tokens, n, heads, head_dim, state_size, groups, sm_count(xbc.device), dtype_code(proj.dtype),
+        _stream()), "ssm_tiles")
     return y
 
 

@@ -1,0 +1,426 @@
+// The state-space recurrence over prompt portions by chunks of 128 tokens side by side (chunk_tiles.cuh), for states of 128 rows and heads of 64 columns
+// beside bfloat16 activations:
+//
+//     y_t = e^(B_t) C_t . S_0 + sum_{s <= t} e^(B_t - B_s) (C_t . B_s) u_s + D x_t,     S = e^(B_n) S_0 + sum_s e^(B_n - B_s) B_s u_s^T,     u = step x
+//
+// (B_t the sum of the log decays up to and with token t.)  A group's heads share C and B: a block takes up to eight of them and a chunk, cuts C and B into terms once
+// and forms C B^T once.  Three kernels: `states` leaves what each chunk adds, `scan` turns that into the states at the chunks' starts, `outputs` does
+// the rest.
+#include "chunk_tiles.cuh"
+
+namespace se {
+namespace tiles {
+
+constexpr int kV = 64, kHeads = 8;                   // columns of a head's state; heads that a block takes at most
+constexpr int kSTerm = kV * 256, kSHalf = kV * 128;  // bytes of a term of the state (rows along its columns), of half of one
+constexpr int kUTerm = kT * 128;                     // of the values: rows are tokens
+
+template <typename T_>
+struct StateSpace {
+    const float* xbc;              // [tokens][H * 64 + 2 G * 128]: values, B, C
+    const T_* proj;                // steps' columns from dt_off on
+    int pitch, dt_off;
+    const float* dt_bias;
+    const float* a_log;
+    const float* d_skip;
+    float* states;                 // [places][H][64][128]: what a chunk adds, then the state at its start
+    float* totals;                 // [places][H]: e^(B_n)
+    float* state;
+    long long state_stride;
+    const int* cu_q;
+    const int* seq_rows;
+    float* y;
+    int entries, H, G, blocks, per;        // blocks per group of heads, heads per block
+    int* error;
+};
+
+struct Tables { float hi[kHeads][kT], lo[kHeads][kT], step[kHeads][kT]; };
+
+// B_t of a block's heads as two 32-bit parts, and the steps (0 where there is no token), a warp per head and four tokens a lane
+template <typename T_>
+__device__ __forceinline__ void fill_tables(const StateSpace<T_>& p, Tables& s, int h0, int heads, int first, int n) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp >= heads) return;
+    const int h = h0 + warp;
+    const float rate = expf(p.a_log[h]), bias = p.dt_bias[h];
+    float step[4];
+    double sum[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int t = 4 * lane + j;
+        step[j] = t < n ? walk::softplus32(to_float(p.proj[(size_t)(first + t) * p.pitch + p.dt_off + h]) + bias) : 0.f;
+        sum[j] = (t < n ? walk::log_decay(rate, step[j]) : 0.0) + (j ? sum[j - 1] : 0.0);
+    }
+    double before;
+    walk::sum_before(sum[3], lane, before);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int t = 4 * lane + j;
+        const double b = before + sum[j];
+        const float hi = (float)b;
+        s.hi[warp][t] = hi;
+        s.lo[warp][t] = (float)(b - (double)hi);
+        s.step[warp][t] = step[j];
+    }
+}
+// e^(B_t - B_s)
+__device__ __forceinline__ float decay_between(const Tables& s, int h, int t, int t0) { return expf((s.hi[h][t] - s.hi[h][t0]) + (s.lo[h][t] - s.lo[h][t0])); }
+
+// B's or C's rows of a chunk in three terms: a row per warp at a time
+__device__ __forceinline__ void put_rows(uint32_t at, const float* src, size_t stride, int n) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = 16 * i + warp < n ? ld4(src + (size_t)(16 * i + warp) * stride + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) put4(at + (lane >> 4) * kHalf, kTerm, 16 * i + warp, lane & 15, v[i]);
+}
+// A head's values: two rows a warp at a time, four columns a lane
+__device__ __forceinline__ void fetch_rows(float4 (&v)[4], const float* src, size_t stride, int n) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = 32 * i + 2 * warp + (lane >> 4);
+        v[i] = t < n ? ld4(src + (size_t)t * stride + 4 * (lane & 15)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+template <typename Factor>
+__device__ __forceinline__ void put_values(uint32_t at, const float4 (&v)[4], Factor factor) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = 32 * i + 2 * warp + (lane >> 4);
+        const float f = factor(t);
+        put4(at, kUTerm, t, lane & 15, make_float4(v[i].x * f, v[i].y * f, v[i].z * f, v[i].w * f));
+    }
+}
+
+// What each chunk adds to its heads' states: rows of the state = the M side, B's rows as they lie.  A head's values are cut while the products of the head before run.
+template <typename T_>
+__global__ void __launch_bounds__(kThreads, 1)
+ssm_states_kernel(const StateSpace<T_> p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u, keys = base, values = base + 3 * kTerm;
+    Tables& tab = *reinterpret_cast<Tables*>(smem_raw + (base - smem_u32(smem_raw)) + 3 * kTerm + 6 * kUTerm);
+    __shared__ Shared sh;
+    __shared__ __align__(8) uint64_t done[2];
+    int first, n;
+    chunk_of<kT>(blockIdx.x, p.cu_q, p.entries, first, n);
+    if (n <= 0) return;
+    const int rep = p.H / p.G, g = blockIdx.y / p.blocks, h0 = g * rep + (blockIdx.y - g * p.blocks) * p.per, heads = min(p.per, (g + 1) * rep - h0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = (warp & 3) * 32 + lane, col = (warp >> 2) * 16;
+    const size_t width = (size_t)p.H * kV + 2 * (size_t)p.G * kD;
+    const float* x = p.xbc + (size_t)first * width;
+    const float* b = x + (size_t)p.H * kV + (size_t)g * kD;
+    if (threadIdx.x < 2) fa::mbar_init(smem_u32(&done[threadIdx.x]), 1);
+    const uint32_t tmem = (uint32_t)fa::uniform((int)begin(sh));
+    const int role = fa::uniform(warp);
+    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + col;
+    float4 v[4];
+    fetch_rows(v, x + (size_t)h0 * kV, width, n);
+    fill_tables(p, tab, h0, heads, first, n);
+    put_rows(keys, b, width, n);
+    __syncthreads();
+    bool ok = true;
+    for (int i = 0; i <= heads && ok; ++i) {         // head i's products are issued, head i - 1's sums stored
+        if (i < heads) {
+            put_values(values + (i & 1) * 3 * kUTerm, v, [&](int t) { return t < n ? decay_between(tab, i, n - 1, t) * tab.step[i][t] : 0.f; });
+            fence_smem();
+            fence_before();
+            __syncthreads();
+            if (role == (i & 1)) {
+                fence_after();
+                if (fa::elect_one()) {
+                    product<true, true, 3>(tmem + (i & 1) * kV, keys, kHalf, kTerm, values + (i & 1) * 3 * kUTerm, 0, kUTerm, instr(kV, true, true));
+                    fa::umma_commit(smem_u32(&done[i & 1]));
+                }
+                __syncwarp();
+            }
+            if (i + 1 < heads) fetch_rows(v, x + (size_t)(h0 + i + 1) * kV, width, n);
+        }
+        if (i > 0) {
+            const int h = h0 + i - 1;
+            ok = __syncthreads_and(fa::mbar_wait(smem_u32(&done[(i - 1) & 1]), ((i - 1) >> 1) & 1, &sh.abort_flag));
+            fence_after();
+            if (!ok) {
+                if (threadIdx.x == 0) atomicCAS(p.error, 0, kErrorCode);
+                break;
+            }
+            uint32_t w[16];
+            ld16(mine + ((i - 1) & 1) * kV, w);
+            wait_ld();
+            float sum[16], z = 0.f;
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                sum[c] = __uint_as_float(w[c]);
+                z = fmaf(sum[c], 0.f, z);
+            }
+            if (__any_sync(0xffffffffu, z != 0.f)) {
+#pragma unroll
+                for (int c = 0; c < 16; ++c) sum[c] = 0.f;
+#pragma unroll 1
+                for (int t = 0; t < n; ++t) {
+                    const float k = b[(size_t)t * width + row], f = decay_between(tab, i - 1, n - 1, t) * tab.step[i - 1][t];
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) sum[c] = fmaf(k, x[(size_t)t * width + (size_t)h * kV + col + c] * f, sum[c]);
+                }
+            }
+            float* to = p.states + ((size_t)blockIdx.x * p.H + h) * (kV * kD) + row;
+#pragma unroll
+            for (int c = 0; c < 16; ++c) to[(size_t)(col + c) * kD] = sum[c];
+            if (threadIdx.x == 0) p.totals[(size_t)blockIdx.x * p.H + h] = expf(tab.hi[i - 1][n - 1] + tab.lo[i - 1][n - 1]);
+        }
+    }
+    end(sh);
+}
+
+// What chunks add -> the states at their starts; the last one goes back to the entry's row.  Four elements a thread; four chunks asked for together.
+template <typename T_>
+__global__ void __launch_bounds__(256)
+ssm_scan_kernel(const StateSpace<T_> p) {
+    const int e = blockIdx.z, h = blockIdx.y, i = (blockIdx.x * 256 + threadIdx.x) * 4;
+    const int t0 = p.cu_q[e], chunks = ceil_div(p.cu_q[e + 1] - t0, kT);
+    if (chunks <= 0) return;
+    float* own = p.state + (size_t)p.seq_rows[e] * p.state_stride + (size_t)h * kV * kD + i;
+    const size_t place = (size_t)(t0 / kT + e);
+    float4 S = ld4(own);
+    for (int c0 = 0; c0 < chunks; c0 += 4) {
+        float4 add[4];
+        float f[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const size_t at = (place + min(c0 + c, chunks - 1)) * p.H + h;
+            add[c] = ld4(p.states + at * (kV * kD) + i);
+            f[c] = p.totals[at];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (c0 + c >= chunks) break;
+            walk::st4(p.states + ((place + c0 + c) * p.H + h) * (kV * kD) + i, S);
+            S = make_float4(fmaf(f[c], S.x, add[c].x), fmaf(f[c], S.y, add[c].y), fmaf(f[c], S.z, add[c].z), fmaf(f[c], S.w, add[c].w));
+        }
+    }
+    walk::st4(own, S);
+}
+
+// Bound by a head's steps one after another (some 17,000 cycles, of which its products take 3,800 and shared memory gives them 128 bytes a cycle).  Each warp's weights are eight
+// columns of every 32, so that all share the exponents of the diagonal (32 columns a warp, and one warp of four with all of them: 87 us, 77 so); two warps issue, because
+// a warp is held by the products it issues (one for both 116 and 87).
+// Columns of tensor memory: C B^T 0-127, P's terms 128-319, what the state gives 320-447 (two heads in turn), P u 448-511.  While a head's P u is summed the next
+// head's state is cut and its product with C queued behind.
+template <typename T_>
+__global__ void __launch_bounds__(kThreads, 1)
+ssm_outputs_kernel(const StateSpace<T_> p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u, queries = base, keys = base + 3 * kTerm, state = keys, values = keys + 3 * kSTerm;
+    Tables& tab = *reinterpret_cast<Tables*>(smem_raw + (base - smem_u32(smem_raw)) + 6 * kTerm);
+    __shared__ Shared sh;
+    __shared__ __align__(8) uint64_t state_done;
+    int first, n;
+    chunk_of<kT>(blockIdx.x, p.cu_q, p.entries, first, n);
+    if (n <= 0) return;
+    const int rep = p.H / p.G, g = blockIdx.y / p.blocks, h0 = g * rep + (blockIdx.y - g * p.blocks) * p.per, heads = min(p.per, (g + 1) * rep - h0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp >> 2, row = (warp & 3) * 32 + lane, vcol = part * 16;
+    const size_t width = (size_t)p.H * kV + 2 * (size_t)p.G * kD;
+    const float* x = p.xbc + (size_t)first * width;
+    const float* b = x + (size_t)p.H * kV + (size_t)g * kD;
+    const float* c = b + (size_t)p.G * kD;
+    const float* S = p.states + (size_t)blockIdx.x * p.H * (kV * kD);
+    if (threadIdx.x == 0) fa::mbar_init(smem_u32(&state_done), 1);
+    const uint32_t tmem = (uint32_t)fa::uniform((int)begin(sh));
+    const int role = fa::uniform(warp);              // 0 issues P u, 1 what the state gives
+    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16), weights = 128, old = 320, sums = 448;
+    uint32_t round = 0;
+    bool ok = true;
+    float4 uv[4];
+    auto put_state = [&](int i) {                    // a column of it per warp at a time
+        float4 sv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sv[j] = ld4(S + ((size_t)(h0 + i) * kV + 16 * j + warp) * kD + 4 * lane);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) put4(state + (lane >> 4) * kSHalf, kSTerm, 16 * j + warp, lane & 15, sv[j]);
+    };
+    auto issue_state = [&](int i) {
+        if (role == 1) {
+            fence_after();
+            if (fa::elect_one()) {
+                product<false, false, 3>(tmem + old + (i & 1) * kV, queries, kHalf, kTerm, state, kSHalf, kSTerm, instr(kV, false, false));
+                fa::umma_commit(smem_u32(&state_done));
+            }
+            __syncwarp();
+        }
+    };
+    fill_tables(p, tab, h0, heads, first, n);
+    put_rows(queries, c, width, n);
+    put_rows(keys, b, width, n);
+    fence_smem();
+    __syncthreads();
+    if (role == 0) {
+        if (fa::elect_one()) {
+            product<false, false, 3>(tmem, queries, kHalf, kTerm, keys, kHalf, kTerm, instr(kT, false, false));
+            fa::umma_commit(smem_u32(&sh.done));
+        }
+        __syncwarp();
+    }
+    fetch_rows(uv, x + (size_t)h0 * kV, width, n);
+    ok = products_done(sh, round++, p.error);        // B's terms give way to the first head's state and values
+    if (ok) {
+        put_state(0);
+        fence_smem();
+        __syncthreads();
+        issue_state(0);
+    }
+    for (int i = 0; i < heads && ok; ++i) {
+        const int h = h0 + i;
+        // P of this head: the block on the diagonal by its own exponents, those before it by e^(B_t - B_r) e^(B_r - B_s), r the block's first token
+        put_values(values, uv, [&](int t) { return tab.step[i][t]; });
+        const int block = warp & 3, r = 32 * block;  // rows r .. r + 31; a warp's columns are eight of each block of 32
+        const float f = decay_between(tab, i, row, r);
+        const float before = lane < 8 * block ? decay_between(tab, i, r, 32 * (lane >> 3) + 8 * part + (lane & 7)) : 0.f;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            uint32_t w[3][4] = {};
+            if (x <= block) {
+                uint32_t v[8];
+                ld8(mine + 32 * x + 8 * part, v);
+                wait_ld();
+                float e[8];
+                if (x < block) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) e[j] = __uint_as_float(v[j]) * (f * __shfl_sync(0xffffffffu, before, 8 * x + j));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const int s = 8 * part + j;
+                        const float d = decay_between(tab, i, row, r + s);
+                        e[j] = s <= lane ? __uint_as_float(v[j]) * d : 0.f;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t t3[3];
+                    cut(e[2 * j], e[2 * j + 1], t3);
+#pragma unroll
+                    for (int y = 0; y < 3; ++y) w[y][j] = t3[y];
+                }
+            }
+#pragma unroll
+            for (int y = 0; y < 3; ++y) st4(mine + weights + y * 64 + 16 * x + 4 * part, w[y]);
+        }
+        wait_st();
+        fence_smem();
+        fence_before();
+        // the state's product is there: its terms may give way
+        ok = __syncthreads_and(fa::mbar_wait(smem_u32(&state_done), i & 1, &sh.abort_flag));
+        if (!ok) {
+            if (threadIdx.x == 0) atomicCAS(p.error, 0, kErrorCode);
+            break;
+        }
+        fence_after();
+        if (role == 0) {
+            if (fa::elect_one()) {
+                product_ts<true, 3>(tmem + sums, tmem + weights, values, 0, kUTerm, instr(kV, false, true));
+                fa::umma_commit(smem_u32(&sh.done));
+            }
+            __syncwarp();
+        }
+        if (i + 1 < heads) {
+            put_state(i + 1);
+            fence_smem();
+            __syncthreads();
+            issue_state(i + 1);
+            fetch_rows(uv, x + (size_t)(h + 1) * kV, width, n);
+        }
+        const float skip = p.d_skip[h];
+        float4 own[4];                               // the row's values
+        if (row < n)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) own[j] = ld4(x + (size_t)row * width + (size_t)h * kV + vcol + 4 * j);
+        uint32_t u[16], o[16];
+        ld16(mine + old + (i & 1) * kV + vcol, u);
+        wait_ld();
+        if (!(ok = products_done(sh, round++, p.error))) break;
+        ld16(mine + sums + vcol, o);
+        wait_ld();
+        fence_before();
+        const float lead = expf(tab.hi[i][row] + tab.lo[i][row]);
+        float z = 0.f, y[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            y[j] = fmaf(lead, __uint_as_float(u[j]), __uint_as_float(o[j]));
+            z = fmaf(y[j], 0.f, z);
+        }
+        float* to = p.y + ((size_t)first * p.H + h) * kV;
+        if (!__syncthreads_or(z != 0.f && row < n)) {
+            if (row < n)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    walk::st4(to + (size_t)row * p.H * kV + vcol + 4 * j, make_float4(fmaf(skip, own[j].x, y[4 * j]), fmaf(skip, own[j].y, y[4 * j + 1]),
+                                                                                fmaf(skip, own[j].z, y[4 * j + 2]), fmaf(skip, own[j].w, y[4 * j + 3])));
+        } else {                                     // token by token: a column of the state and 16 rows a thread
+            const int v0 = threadIdx.x >> 3, d0 = (threadIdx.x & 7) * 16;
+            float s[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) s[j] = S[((size_t)h * kV + v0) * kD + d0 + j];
+#pragma unroll 1
+            for (int t = 0; t < n; ++t) {
+                const float xv = x[(size_t)t * width + (size_t)h * kV + v0], uv1 = xv * tab.step[i][t];
+                const float keep = t ? decay_between(tab, i, t, t - 1) : expf(tab.hi[i][0] + tab.lo[i][0]);
+                float sum = 0.f;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    s[j] = fmaf(keep, s[j], b[(size_t)t * width + d0 + j] * uv1);
+                    sum = fmaf(c[(size_t)t * width + d0 + j], s[j], sum);
+                }
+#pragma unroll
+                for (int m = 1; m < 8; m <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+                if (d0 == 0) to[(size_t)t * p.H * kV + v0] = fmaf(skip, xv, sum);
+            }
+        }
+    }
+    end(sh);
+}
+
+template <typename T_>
+static int launch_ssm(const StateSpace<T_>& p, int places, cudaStream_t stream) {
+    const int states_smem = 3 * kTerm + 6 * kUTerm + (int)sizeof(Tables) + 1024, outputs_smem = 6 * kTerm + (int)sizeof(Tables) + 1024;
+    cudaError_t e = cudaFuncSetAttribute(ssm_states_kernel<T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, states_smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(ssm_outputs_kernel<T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, outputs_smem);
+    if (e != cudaSuccess) return (int)e;
+    const dim3 grid(places, p.G * p.blocks);
+    ssm_states_kernel<T_><<<grid, kThreads, states_smem, stream>>>(p);
+    ssm_scan_kernel<T_><<<dim3(kV * kD / 1024, p.H, p.entries), 256, 0, stream>>>(p);
+    ssm_outputs_kernel<T_><<<grid, kThreads, outputs_smem, stream>>>(p);
+    SE_LAUNCH_CHECK();
+}
+
+}  // namespace tiles
+}  // namespace se
+
+using namespace se::tiles;
+
+extern "C" int se_ssm_tiles_supported(int state_size, int head_dim) { return state_size == kD && head_dim == kV; }
+
+// Arguments as se_ssm_walk's.  work: float [(tokens / 128 + entries) * H * (64 * 128 + 1)].
+extern "C" int se_ssm_tiles(const float* xbc, const void* proj, int pitch, int dt_off, const float* dt_bias, const float* a_log, const float* d_skip,
+                            float* state, long long state_stride, const int* cu_q, const int* seq_rows, float* y, float* work, int* error, int tokens,
+                            int entries, int H, int P, int N, int G, int sms, int dtype, cudaStream_t stream) {
+    if (entries <= 0 || tokens <= 0) return 0;
+    if (H <= 0 || G <= 0 || H % G) return SE_ERR_ARGUMENT;
+    const long long places = tokens / kT + entries;
+    // heads a block: as many as leave a block for each SM, eight at most (C and B are cut and multiplied once per block)
+    int per = H / G < kHeads ? H / G : kHeads;
+    while (per > 1 && places * G * ((H / G + per - 1) / per) < sms * 3 / 4) per = (per + 1) / 2;
+    const int blocks = (H / G + per - 1) / per;
+    auto aligned = [](const void* a) { return (reinterpret_cast<uintptr_t>(a) & 15) == 0; };
+    if (!se_ssm_tiles_supported(N, P) || H > 65535 || (long long)G * blocks > 65535 || entries > 65535 || places > 0x7fffffffLL || state_stride % 4 ||
+        !aligned(xbc) || !aligned(state) || !aligned(y) || !aligned(work))
+        return SE_ERR_UNSUPPORTED;
+    SE_DISPATCH_DTYPE(dtype, T_, {
+        StateSpace<T_> p;
+        p.xbc = xbc; p.proj = (const T_*)proj; p.pitch = pitch; p.dt_off = dt_off; p.dt_bias = dt_bias; p.a_log = a_log; p.d_skip = d_skip;
+        p.states = work; p.totals = work + (size_t)places * H * (kV * kD); p.state = state; p.state_stride = state_stride; p.cu_q = cu_q; p.seq_rows = seq_rows;
+        p.y = y; p.entries = entries; p.H = H; p.G = G; p.blocks = blocks; p.per = per; p.error = error;
+        return launch_ssm<T_>(p, (int)places, stream);
+    });
+}

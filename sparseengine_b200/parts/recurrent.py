@@ -96,18 +96,42 @@ class StateSpaceMixer(Mixer):
     def state_request(self):
         return StateRequest((self.conv_off + (self.spec.conv_taps - 1) * self.conv_channels,), torch.float32)
 
+    def token_by_token(self, longest: int, entries: int, tokens: int, sms: int) -> float:
+        """Estimated us of the shorter of csrc/recurrent.cu's two forms, lane groups and tiles."""
+        s = self.spec
+        size = s.num_heads * s.head_dim * s.state_size / 524288 * 148 / sms
+        return min(3 + 0.65 * size * entries + max(max(0.8, 0.45 * size) * longest, 0.24 * size * tokens),
+                   6 + 1.45 * size * entries + max(max(0.44, 0.33 * size) * longest, 0.23 * size * tokens))
+
     def in_chunks(self, step, device) -> bool:
         if self.chunk_min_tokens is None or step.max_q_len < self.chunk_min_tokens:
             return False
-        s = self.spec
-        size = s.num_heads * s.head_dim * s.state_size / 524288 * 148 / ops.sm_count(device)
-
-        def walk(longest, entries, tokens):          # the shorter of csrc/recurrent.cu's two forms, lane groups and tiles
-            return min(3 + 0.65 * size * entries + max(max(0.8, 0.45 * size) * longest, 0.24 * size * tokens),
-                       6 + 1.45 * size * entries + max(max(0.44, 0.33 * size) * longest, 0.23 * size * tokens))
+        s, sms = self.spec, ops.sm_count(device)
         return once_per_step(step, ("state_space.in_chunks", s.num_heads, s.state_size, s.head_dim), lambda: (
-            takes_chunks(self, step, s.num_heads, s.state_size, s.head_dim, 2.1e-4, device, block=(19.5, 7.0), launches=17.0, walk=walk)
+            takes_chunks(self, step, s.num_heads, s.state_size, s.head_dim, 2.1e-4, device, block=(19.5, 7.0), launches=17.0,
+                         walk=lambda longest, entries, tokens: self.token_by_token(longest, entries, tokens, sms))
             and ops.chunk_walk_supported(s.state_size, s.head_dim)))
+
+    def in_tiles(self, step, device) -> bool:
+        """Whether a step that csrc/ssm_tiles.cu takes (bfloat16, states of 128 rows, heads of 64 columns) goes there: by estimates of it
+        and of the form token by token.  A block takes a chunk of 128 tokens, full or not, and up to eight of a group's heads: 13 us each and 10 for what
+        they share.  Measured, a layer of 64 heads in 8 groups, us before / now: one entry of 110 tokens 92/89, of 128 94/90, of 512 124/109, of 2,048 298/247; four of 40
+        87/92, of 60 108/90, of 300 233/209; sixty-four of 20 400/524, of 40 749/605, of 96 1,719/830; one of 300 beside 15 single tokens 218/179,
+        beside 31 249/284, of 1,024 beside 63 662/531.  Few heads over few tokens stay in chunks of 64 (8 heads of 256 tokens 27, here 33).  The chunks' states
+        take 32 KB per head and chunk: no more than 256 MB, or than the other chunks' workspace."""
+        if self.chunk_min_tokens is None or not getattr(self, "chunks_by_estimate", True):
+            return False
+
+        def ask():
+            s, sms = self.spec, ops.sm_count(device)
+            longest, entries, tokens = step.max_q_len, step.num_seqs, step.num_tokens
+            if s.num_heads * longest <= 2048 or (tokens // 128 + entries) * s.num_heads * 8193 > max(1 << 26, tokens * s.num_heads * 67):
+                return False
+            lens = getattr(step, "q_lens", None) or [longest] + [(tokens - longest) // max(1, entries - 1)] * (entries - 1)
+            per = min(8, s.num_heads // s.groups)
+            blocks = sum(-(-n // 128) for n in lens) * s.groups * -(-(s.num_heads // s.groups) // per)
+            return 35 + blocks * (10 + 13 * per) / sms < self.token_by_token(longest, entries, tokens, sms)
+        return once_per_step(step, ("state_space.in_tiles", self.spec.num_heads, self.spec.groups, self.spec.state_size, self.spec.head_dim), ask)
 
     def forward(self, x, step, slot):
         s = self.spec
@@ -116,7 +140,8 @@ class StateSpaceMixer(Mixer):
         xbc = torch.empty(tokens, self.conv_channels, dtype=torch.float32, device=x.device)
         ops.causal_conv(proj, self.inner, self.conv_w, self.conv_b, slot.state, self.conv_off, step, xbc)
         y = torch.empty(tokens, self.inner, dtype=torch.float32, device=x.device)
-        (ops.ssm_walk if self.in_chunks(step, x.device) else ops.ssm_scan)(
+        tiles = ops.ssm_tiles_supported(s.state_size, s.head_dim, proj, slot.state) and self.in_tiles(step, x.device)
+        (ops.ssm_tiles if tiles else ops.ssm_walk if self.in_chunks(step, x.device) else ops.ssm_scan)(
             xbc, proj, self.inner + self.conv_channels, self.dt_bias, self.a_log, self.d_skip, slot.state, step, y,
             heads=s.num_heads, head_dim=s.head_dim, state_size=s.state_size, groups=s.groups)
         gated = torch.empty(tokens, self.inner, dtype=x.dtype, device=x.device)

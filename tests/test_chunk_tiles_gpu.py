@@ -100,3 +100,82 @@ def test_retention_mixer_keeps_to_the_other_forms_beyond_its_workspace():
     part = make_mixer(RetentionSpec(hidden_size=64, num_heads=32, head_dim=128, v_head_dim=128, decays=(0.9,) * 32, position=None), torch.bfloat16)
     few, many = (SimpleNamespace(num_seqs=n, max_q_len=20) for n in (64, 512))
     assert part.in_tiles(few, 20 + 63, 0, DEV) and not part.in_tiles(many, 20 + 511, 0, DEV)
+
+
+def _state_space(lens, heads, groups, decay, bad=None):
+    from sparseengine_b200.csrc import ops
+    P, N, step = 64, 128, _step(lens)
+    T, g = step.num_tokens, torch.Generator(device=DEV).manual_seed(heads)
+    xbc = torch.randn(T, heads * P + 2 * groups * N, generator=g, device=DEV)
+    proj = torch.randn(T, heads + 5, generator=g, device=DEV).to(torch.bfloat16)
+    bias, skip = torch.randn(heads, generator=g, device=DEV) - 2.0, torch.randn(heads, generator=g, device=DEV)
+    a_log = torch.log(torch.rand(heads, generator=g, device=DEV) * (30 if decay == "fast" else 1) + 0.1)
+    state = torch.randn(len(lens) + 2, heads * P * N + 4, generator=g, device=DEV)
+    if bad is not None:
+        t, where, value = bad
+        if where == "dt":
+            proj[t, 3] = value
+        else:
+            xbc[t, {"v": 5, "k": heads * P + 5, "q": heads * P + groups * N + 5}[where]] = value
+    first, y = state.clone(), torch.full((T, heads * P), float("nan"), device=DEV)
+    assert ops.ssm_tiles_supported(N, P, proj, state)
+    ops.ssm_tiles(xbc, proj, 3, bias, a_log, skip, state, step, y, heads=heads, head_dim=P, state_size=N, groups=groups)
+    ops.error_check(DEV)
+    dt = torch.nn.functional.softplus(proj[:, 3:3 + heads].double() + bias.double())
+    x, rep = xbc[:, :heads * P].double().view(T, heads, P), heads // groups
+    k, q = (c.double().reshape(T, groups, N).repeat_interleave(rep, 1) for c in xbc[:, heads * P:].split(groups * N, 1))
+    return step, y, first, state, (q, k, x * dt[..., None], torch.exp(-torch.exp(a_log.double()) * dt)[..., None]), skip.double()[:, None] * x
+
+
+# heads a block: one, five of a group of nine, eight and three more
+@pytest.mark.parametrize("decay", ["slow", "fast"])
+@pytest.mark.parametrize("lens,heads,groups", [([1, 127, 128, 129, 0, 300, 64, 17], 4, 4), ([513], 18, 2), ([130] * 64, 11, 1)])
+def test_state_space_against_the_walk(lens, heads, groups, decay):
+    step, y, first, state, inputs, add = _state_space(lens, heads, groups, decay)
+    P, N = 64, 128
+    for e, n in enumerate(lens):
+        a, b, row = step.cu[e], step.cu[e + 1], step.rows[e]
+        if n == 0:
+            assert torch.equal(state[row], first[row])
+            continue
+        if e > 8:                                    # 64 equal ones: the first few and the last
+            if e != len(lens) - 1:
+                continue
+        want, S = _walk64(*(x[a:b] for x in inputs), first[row, :heads * P * N].double().view(heads, P, N).transpose(1, 2))
+        _close(y[a:b].view(n, heads, P), want + add[a:b], f"outputs of {n} tokens")
+        _close(state[row, :heads * P * N].view(heads, P, N).transpose(1, 2), S, f"state after {n} tokens")
+    others = [r for r in range(len(lens) + 2) if r not in step.rows]
+    assert torch.equal(state[others], first[others]) and torch.equal(state[:, heads * P * N:], first[:, heads * P * N:])
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["q", "k", "v", "dt"])
+def test_state_space_inputs_that_are_not_finite_stay_with_their_token_and_later_ones(where, value):
+    """Token 150 of 400: the second of four chunks, the first of two groups of two heads (of v and dt its first head)."""
+    t, P = 150, 64
+    _, want, _, s_want, _, _ = _state_space([400], 4, 2, "slow")
+    _, got, _, s_got, _, _ = _state_space([400], 4, 2, "slow", bad=(t, where, value))
+    own = P if where in ("v", "dt") else 2 * P       # columns that it may reach
+    near = dict(rtol=1e-4, atol=1e-4)                # its chunk is done again token by token: another order of the same sums
+    assert torch.equal(got[:128], want[:128]) and torch.equal(got[:, own:], want[:, own:])
+    torch.testing.assert_close(got[128:t], want[128:t], **near)
+    if where == "q":
+        assert not bool(torch.isfinite(got[t, :own]).any())
+        torch.testing.assert_close(got[t + 1:], want[t + 1:], **near)
+        assert torch.equal(s_got, s_want)
+    elif where != "dt" or value != value:            # an infinite step may be a decay of 0
+        assert not bool(torch.isfinite(got[t:, :own]).all(1).any()) and not bool(torch.isfinite(s_got[0, :own * 128]).all())
+        assert torch.equal(s_got[0, own * 128:], s_want[0, own * 128:])
+
+
+def test_state_space_mixer_chooses_by_both_estimates():
+    from sparseengine_b200.config.specs import StateSpaceSpec
+    from sparseengine_b200.parts.base import make_mixer
+    part = make_mixer(StateSpaceSpec(hidden_size=64, num_heads=64, head_dim=64, state_size=128, groups=8, conv_taps=4, norm_groups=8), torch.bfloat16)
+
+    def asked(lens):
+        return part.in_tiles(SimpleNamespace(num_seqs=len(lens), max_q_len=max(lens), num_tokens=sum(lens), q_lens=lens), DEV)
+    assert asked([2048]) and asked([60] * 4) and asked([40] * 64) and not asked([20] * 64) and not asked([90] + [1] * 63)
+    assert not asked([17]) and not asked([100] * 200)        # the last: its states would take 419 MB
+    part.chunk_min_tokens = None
+    assert not asked([2048])
