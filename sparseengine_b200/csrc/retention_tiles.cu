@@ -6,8 +6,8 @@
 // state at each chunk's start, `join` (where an entry has several segments) the states at the segments' starts, `outputs` (a block per chunk and head)
 // the rest: q and k turned on their way from the projection, both products with q, the decays, P v, and where the mixer norms each head the norm and the gate.
 //
-// Measured, 8,192 tokens of 32 heads (the walk, its preparation and the norm: 675 us): 330 = angles 4 + states 73 + join 4 + outputs 247; 2,048 tokens of 16
-// heads 147 and 62; four entries of 100 tokens, 32 heads, 54 and 37.  Errors against 64 bits over the result's norm: outputs 2.0e-7 to 2.7e-7 (the walk 1.4e-7 to 2.1e-7), states
+// Measured, 8,192 tokens of 32 heads (the walk, its preparation and the norm: 675 us): 322 = angles 4 + states 73 + join 4 + outputs 232; 2,048 tokens of 16
+// heads 147 and 60; four entries of 100 tokens, 32 heads, 54 and 39.  Errors against 64 bits over the result's norm: outputs 2.0e-7 to 2.7e-7 (the walk 1.4e-7 to 2.1e-7), states
 // 0.8e-7 to 1.5e-7 (0.8e-7 to 2.2e-7), where 16-bit inputs and outputs leave 4e-3.
 #include "chunk_tiles.cuh"
 
@@ -75,35 +75,6 @@ __device__ __forceinline__ void put_pairs(uint32_t at, int row, int quad, uint2 
     put4(at, kTerm, row, quad, make_float4(x[0] * f, x[1] * f, x[2] * f, x[3] * f));
     put4(at + kHalf, kTerm, row, quad, make_float4(y[0] * f, y[1] * f, y[2] * f, y[3] * f));
 }
-// k's rows of a chunk in three terms, each times `factor(row)`: two rows a warp at a time, four pairs of columns a lane
-template <typename Factor>
-__device__ __forceinline__ void put_keys(const Retention& p, uint32_t at, int first, int n, int h, Factor factor) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = lane & 15;
-    const __nv_bfloat16* k = p.proj + p.k_off + (size_t)h * kD + 4 * quad;
-    uint2 lo[4], hi[4];
-    float4 cs[4][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t = 32 * i + 2 * warp + (lane >> 4);
-        const size_t row = (size_t)first + t;
-        lo[i] = hi[i] = make_uint2(0, 0);
-        cs[i][0] = cs[i][1] = make_float4(1.f, 0.f, 1.f, 0.f);
-        if (t < n) {
-            lo[i] = *reinterpret_cast<const uint2*>(k + row * p.pitch);
-            hi[i] = *reinterpret_cast<const uint2*>(k + row * p.pitch + 64);
-            if (p.turn != nullptr) {
-                const float4* c = reinterpret_cast<const float4*>(p.turn + row * 64 + 4 * quad);
-                cs[i][0] = c[0];
-                cs[i][1] = c[1];
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t = 32 * i + 2 * warp + (lane >> 4);
-        put_pairs(at, t, quad, lo[i], hi[i], cs[i][0], cs[i][1], factor(t) * p.k_scale);
-    }
-}
 // a head's rows as they are, columns from `off` on: [128 tokens][64 columns], twice
 __device__ __forceinline__ void fetch_rows(const Retention& p, uint32_t at, int off, int first, int n, int h) {
 #pragma unroll
@@ -114,13 +85,28 @@ __device__ __forceinline__ void fetch_rows(const Retention& p, uint32_t at, int 
     }
 }
 
-// Bound by a chunk's steps one after another (loads and cuts of k, products, the state's update; 4.6 us a chunk, the tensor pipe 18 % busy): 128 rows of the
-// state by 128 columns in registers, a row and 32 columns a thread.  As many segments as fill the device, because the alternative, what every chunk adds and a
+// a chunk's angles: [128][64] cosines and sines, 16-byte pieces of a row in the order of its last three bits
+__device__ __forceinline__ void fetch_angles(const Retention& p, uint32_t at, int first, int n) {
+    if (p.turn == nullptr) return;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int x = i * kThreads + threadIdx.x, r = x >> 5, c = x & 31;
+        cp16(at + r * 512 + ((c ^ (r & 7)) << 4), p.turn + (size_t)(first + min(r, n - 1)) * 64 + 2 * c, true);
+    }
+}
+// of pairs 2 c and 2 c + 1 of row r
+__device__ __forceinline__ float4 angle_at(const Retention& p, const uint8_t* angles, int r, int c) {
+    return p.turn != nullptr ? *reinterpret_cast<const float4*>(angles + r * 512 + ((c ^ (r & 7)) << 4)) : make_float4(1.f, 0.f, 1.f, 0.f);
+}
+
+// Bound by a chunk's steps one after another (cuts of k 3,000 cycles, products 2,200 beside copies and stores of 3,000, the state's update 600; 4.6 us a chunk, the tensor pipe 18 % busy): 128 rows of the
+// state by 128 columns in registers, a row and 32 columns a thread.  The next chunk's k and angles are fetched while this one's products run.  As many segments as fill the device, because the alternative, what every chunk adds and a
 // scan over it, reads and writes the states (134 MB for 8,192 tokens of 32 heads) once more.
 __global__ void __launch_bounds__(kThreads, 1)
 retention_states_kernel(const Retention p) {
     extern __shared__ uint8_t smem_raw[];
-    const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u, keys = base, values = base + 3 * kTerm;
+    const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u, keys = base, values = base + 3 * kTerm, raw = base + 4 * kTerm, angles = base + 5 * kTerm;
+    const uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
     __shared__ Shared sh;
     __shared__ float power[kT + 1];
     const int e = blockIdx.x / p.segments, seg = blockIdx.x - e * p.segments, h = blockIdx.y;
@@ -129,7 +115,11 @@ retention_states_kernel(const Retention p) {
     if (c0 >= c1) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = (warp & 3) * 32 + lane, col = (warp >> 2) * 32;
     for (int i = threadIdx.x; i <= kT; i += kThreads) power[i] = p.powers[(size_t)h * p.powers_pitch + i];
-    const uint32_t tmem = begin(sh);
+    fetch_rows(p, raw, p.k_off, t_first + c0 * kT, min(kT, t_last - t_first - c0 * kT), h);
+    fetch_angles(p, angles, t_first + c0 * kT, min(kT, t_last - t_first - c0 * kT));
+    walk::cp_commit();
+    const uint32_t tmem = (uint32_t)fa::uniform((int)begin(sh));
+    const bool issuer = fa::uniform(warp) == 0;
     const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + col;
     float S[32];
     float* own = p.state + (size_t)p.seq_rows[e] * p.state_stride + ((size_t)h * kD + row) * kD + col;
@@ -145,20 +135,33 @@ retention_states_kernel(const Retention p) {
     uint32_t round = 0;
     for (int c = c0; c < c1; ++c, ++round) {
         const int first = t_first + c * kT, n = min(kT, t_last - first);
+        walk::cp_wait<0>();
+        __syncthreads();                             // k and angles are there
         fetch_rows(p, values, p.v_off, first, n, h);
         walk::cp_commit();
-        put_keys(p, keys, first, n, h, [&](int t) { return t < n ? power[n - 1 - t] : 0.f; });
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = 32 * i + 2 * warp + (lane >> 4), quad = lane & 15;
+            const uint8_t* from = sm + 4 * kTerm + fa::sw128(t, quad >> 1) + (quad & 1) * 8;
+            put_pairs(keys, t, quad, *reinterpret_cast<const uint2*>(from), *reinterpret_cast<const uint2*>(from + kHalf),
+                      angle_at(p, sm + 5 * kTerm, t, 2 * quad), angle_at(p, sm + 5 * kTerm, t, 2 * quad + 1), t < n ? power[n - 1 - t] * p.k_scale : 0.f);
+        }
         walk::cp_wait<0>();
         fence_smem();
         fence_before();                              // the last chunk's sums have been read
         __syncthreads();
-        if (warp == 0) {
+        if (issuer) {
             fence_after();
             if (fa::elect_one()) {
                 product<true, true, 1>(tmem, keys, kHalf, kTerm, values, kHalf, kTerm, instr(kD, true, true));
                 fa::umma_commit(smem_u32(&sh.done));
             }
             __syncwarp();
+        }
+        if (c + 1 < c1) {
+            fetch_rows(p, raw, p.k_off, first + kT, min(kT, t_last - first - kT), h);
+            fetch_angles(p, angles, first + kT, min(kT, t_last - first - kT));
+            walk::cp_commit();
         }
         store(p.states + ((size_t)(t_first / kT + e + c) * p.H + h) * (kD * kD));
         if (!products_done(sh, round, p.error)) break;
@@ -182,6 +185,7 @@ retention_states_kernel(const Retention p) {
             }
         }
     }
+    walk::cp_wait<0>();
     if (p.segments > 1) store(p.starts + ((size_t)blockIdx.x * p.H + h) * (kD * kD));
     else
 #pragma unroll
@@ -228,18 +232,18 @@ retention_join_kernel(const Retention p) {
 }
 
 // A block takes chunks in turn.  The next chunk's q, k and angles are fetched into room that this one's products have left (the state's terms, the last of
-// k's) while its weights are made and P v runs; the state comes into registers meanwhile.  Bound by the steps of a chunk, 17 us, one after another: the
-// products take 8,000 cycles of 33,000, instructions issue in 30 %.  Measured, 8,192 tokens of 32 heads: 247 us; q and angles row by row from memory 292;
-// a warp group per operand, which leaves 64 to 112 registers a thread and spills, 253 to 288; a warp that only issues products, 112 registers, 274.
+// k's) while its weights are made and P v runs; the state comes into registers meanwhile.  Bound by the steps of a chunk, 16 us, one after another: the
+// products take 8,000 cycles of 32,000, instructions issue in 30 %.  Measured, 8,192 tokens of 32 heads: 232 us; q and angles row by row from memory and outputs and gates a row a
+// thread 292, the latter alone 240; a warp group per operand, which leaves 64 to 112 registers a thread and spills, 253 to 288; a warp that only issues products, 112 registers, 274.
 //   columns of tensor memory: q's terms, then P's 0-191; scores, then P v 192-319; what the state gives 320-447
 __global__ void __launch_bounds__(kThreads, 1)
 retention_outputs_kernel(const Retention p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u, keys = base, state = base + 3 * kTerm, values = base + 6 * kTerm;
-    const uint32_t raw_k = keys + 2 * kTerm, raw_q = state, angles = state + kTerm;       // angles: [128][64] cosines and sines, 16-byte pieces of a row in the order of its last three bits
+    const uint32_t raw_k = keys + 2 * kTerm, raw_q = state, angles = state + kTerm;
     uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
     float* plain = reinterpret_cast<float*>(sm);                                          // for the form token by token
-    float (*squares)[kT] = reinterpret_cast<float (*)[kT]>(sm + 2 * kTerm - 4 * kT * 4);  // at the end of k's second term
+    float (*squares)[kT] = reinterpret_cast<float (*)[kT]>(sm + 6 * kTerm);               // where the values have been read
     __shared__ Shared sh;
     __shared__ float power[kT + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp >> 2, row = (warp & 3) * 32 + lane, col = part * 32, quad = lane & 15;
@@ -267,17 +271,10 @@ retention_outputs_kernel(const Retention p) {
     auto fetch = [&](const Item& t) {
         fetch_rows(p, raw_k, p.k_off, t.first, t.n, t.h);
         fetch_rows(p, raw_q, p.q_off, t.first, t.n, t.h);
-        if (p.turn != nullptr)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int x = i * kThreads + threadIdx.x, r = x >> 5, c = x & 31;
-                cp16(angles + r * 512 + ((c ^ (r & 7)) << 4), p.turn + (size_t)(t.first + min(r, t.n - 1)) * 64 + 2 * c, true);
-            }
+        fetch_angles(p, angles, t.first, t.n);
         walk::cp_commit();
     };
-    auto angle = [&](int r, int c) {                 // of pairs 2 c and 2 c + 1 of row r
-        return p.turn != nullptr ? *reinterpret_cast<const float4*>(sm + 4 * kTerm + r * 512 + ((c ^ (r & 7)) << 4)) : make_float4(1.f, 0.f, 1.f, 0.f);
-    };
+    auto angle = [&](int r, int c) { return angle_at(p, sm + 4 * kTerm, r, c); };
     if (threadIdx.x == 32) find(items[0]);
     __syncthreads();
     if (items[0].n > 0) fetch(items[0]);
@@ -385,18 +382,18 @@ retention_outputs_kernel(const Retention p) {
             __syncwarp();
         }
         {
-            uint32_t v[32], w[3][8];
-            if (col <= (row | 31)) {
-                fa::tmem_ld32(mine + scores + col, v);
-                wait_ld();
-            }
-            fence_before();
+            uint32_t w[3][8];
             auto weights = [&](int half) {
+                uint32_t v[16];
+                if (col + 16 * half <= (row | 31)) {
+                    ld16(mine + scores + col + 16 * half, v);
+                    wait_ld();
+                }
 #pragma unroll
                 for (int x = 0; x < 16; x += 2) {    // (the table's index is one of its own also where it is not used)
                     const int s = col + 16 * half + x;
                     const float fa_ = power[(row - s) & 127], fb = power[(row - s - 1) & 127];
-                    const float a = s <= row ? __uint_as_float(v[16 * half + x]) * fa_ : 0.f, b = s < row ? __uint_as_float(v[16 * half + x + 1]) * fb : 0.f;
+                    const float a = s <= row ? __uint_as_float(v[x]) * fa_ : 0.f, b = s < row ? __uint_as_float(v[x + 1]) * fb : 0.f;
                     uint32_t c[3];
                     cut(a, b, c);
 #pragma unroll
@@ -424,32 +421,36 @@ retention_outputs_kernel(const Retention p) {
             __syncwarp();
         }
         if (next.n > 0) fetch(next);
-        const size_t out_at = ((size_t)(first + row) * p.H + h) * kD + col;
-        const uint4* gate = reinterpret_cast<const uint4*>(p.proj + (size_t)(first + (in ? row : 0)) * p.pitch + p.g_off + (size_t)h * kD + col);
+        // the gates as the outputs are stored: 16 bytes of a row a thread, two rows a warp
         uint4 gates[4];
         if (p.out != nullptr)
 #pragma unroll
-            for (int x = 0; x < 4; ++x) gates[x] = gate[x];
+            for (int i = 0; i < 4; ++i) {
+                const int r = 32 * i + 2 * warp + (lane >> 4);
+                gates[i] = *reinterpret_cast<const uint4*>(p.proj + (size_t)(first + min(r, n - 1)) * p.pitch + p.g_off + (size_t)h * kD + 8 * quad);
+            }
         float o[32];
         const float f = power[row + 1];
-        {
-            uint32_t v[32];
-            fa::tmem_ld32(mine + old + col, v);
+#pragma unroll
+        for (int y = 0; y < 32; y += 16) {
+            uint32_t v[16];
+            ld16(mine + old + col + y, v);
             wait_ld();
 #pragma unroll
-            for (int x = 0; x < 32; ++x) o[x] = f * __uint_as_float(v[x]);
+            for (int x = 0; x < 16; ++x) o[y + x] = f * __uint_as_float(v[x]);
         }
         if (!(ok = products_done(sh, round++, p.error))) break;
         float z = 0.f, sum = 0.f;
-        {
-            uint32_t v[32];
-            fa::tmem_ld32(mine + scores + col, v);
+#pragma unroll
+        for (int y = 0; y < 32; y += 16) {
+            uint32_t v[16];
+            ld16(mine + scores + col + y, v);
             wait_ld();
 #pragma unroll
-            for (int x = 0; x < 32; ++x) {
-                o[x] += __uint_as_float(v[x]);
-                z = fmaf(o[x], 0.f, z);
-                sum = fmaf(o[x], o[x], sum);
+            for (int x = 0; x < 16; ++x) {
+                o[y + x] += __uint_as_float(v[x]);
+                z = fmaf(o[y + x], 0.f, z);
+                sum = fmaf(o[y + x], o[y + x], sum);
             }
         }
         squares[part][row] = sum;
@@ -499,22 +500,31 @@ retention_outputs_kernel(const Retention p) {
             __syncthreads();
             if (next.n > 0) fetch(next);
         }
-        if (in && p.out == nullptr) {
+        // through shared memory (where k's first two terms were), so that neighbouring threads store neighbours
 #pragma unroll
-            for (int x = 0; x < 32; x += 8) store8(p.o + out_at + x, o + x);
-        } else if (in) {
-            const float inv = 1.0f / sqrtf(((squares[0][row] + squares[1][row]) + (squares[2][row] + squares[3][row])) / (float)kD + p.eps);
+        for (int x = 0; x < 8; ++x)
+            *reinterpret_cast<float4*>(sm + row * 512 + (((8 * part + x) ^ (row & 7)) << 4)) = make_float4(o[4 * x], o[4 * x + 1], o[4 * x + 2], o[4 * x + 3]);
+        __syncthreads();
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const uint32_t g4[4] = {gates[x].x, gates[x].y, gates[x].z, gates[x].w};
-                float u[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float g = __uint_as_float(i & 1 ? g4[i / 2] & 0xffff0000u : g4[i / 2] << 16);
-                    u[i] = o[8 * x + i] * inv * __fdividef(g, 1.f + __expf(-g));
-                }
-                store8(p.out + out_at + 8 * x, u);
+        for (int i = 0; i < 4; ++i) {
+            const int r = 32 * i + 2 * warp + (lane >> 4);
+            if (r >= n) continue;
+            const float4 a = *reinterpret_cast<const float4*>(sm + r * 512 + (((2 * quad) ^ (r & 7)) << 4));
+            const float4 b = *reinterpret_cast<const float4*>(sm + r * 512 + (((2 * quad + 1) ^ (r & 7)) << 4));
+            float y[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            const size_t to = ((size_t)(first + r) * p.H + h) * kD + 8 * quad;
+            if (p.out == nullptr) {
+                store8(p.o + to, y);
+                continue;
             }
+            const float inv = 1.0f / sqrtf(((squares[0][r] + squares[1][r]) + (squares[2][r] + squares[3][r])) / (float)kD + p.eps);
+            const uint32_t g4[4] = {gates[i].x, gates[i].y, gates[i].z, gates[i].w};
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+                const float g = __uint_as_float(x & 1 ? g4[x / 2] & 0xffff0000u : g4[x / 2] << 16);
+                y[x] = y[x] * inv * __fdividef(g, 1.f + __expf(-g));
+            }
+            store8(p.out + to, y);
         }
     }
     walk::cp_wait<0>();
@@ -556,7 +566,7 @@ extern "C" int se_retention_tiles(const void* proj, int pitch, int q_off, int k_
     p.powers = powers; p.turn = rotary ? turn : nullptr;
     p.segments = segments; p.seg_chunks = seg_chunks; p.state = state; p.state_stride = state_stride; p.cu_q = cu_q; p.seq_rows = seq_rows;
     p.entries = entries; p.H = heads; p.places = (int)places; p.k_scale = k_scale; p.eps = eps; p.out = (__nv_bfloat16*)out; p.o = o; p.error = error;
-    const int turn_blocks = rotary ? (tokens * 64 + 255) / 256 : 0, states_smem = 4 * kTerm + 1024, outputs_smem = 7 * kTerm + 1024;
+    const int turn_blocks = rotary ? (tokens * 64 + 255) / 256 : 0, states_smem = 7 * kTerm + 1024, outputs_smem = 7 * kTerm + 1024;
     retention_tables_kernel<<<turn_blocks + heads, 256, 0, stream>>>(turn, positions, inv_freq, tokens, turn_blocks, powers, p.powers_pitch, decay);
     cudaError_t e = cudaFuncSetAttribute(retention_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, states_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(retention_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, outputs_smem);

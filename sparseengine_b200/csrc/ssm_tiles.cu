@@ -203,9 +203,9 @@ ssm_scan_kernel(const StateSpace<T_> p) {
     walk::st4(own, S);
 }
 
-// Bound by a head's steps one after another (some 17,000 cycles, of which its products take 3,800 and shared memory gives them 128 bytes a cycle).  Each warp's weights are eight
+// Bound by a head's steps one after another (some 14,000 cycles, of which its products take 3,800 and shared memory gives them 128 bytes a cycle).  Each warp's weights are eight
 // columns of every 32, so that all share the exponents of the diagonal (32 columns a warp, and one warp of four with all of them: 87 us, 77 so); two warps issue, because
-// a warp is held by the products it issues (one for both 116 and 87).
+// a warp is held by the products it issues (one for both 116, two 87); outputs leave through shared memory (a row a thread 77, 63 so).
 // Columns of tensor memory: C B^T 0-127, P's terms 128-319, what the state gives 320-447 (two heads in turn), P u 448-511.  While a head's P u is summed the next
 // head's state is cut and its product with C queued behind.
 template <typename T_>
@@ -332,10 +332,8 @@ ssm_outputs_kernel(const StateSpace<T_> p) {
             fetch_rows(uv, x + (size_t)(h + 1) * kV, width, n);
         }
         const float skip = p.d_skip[h];
-        float4 own[4];                               // the row's values
-        if (row < n)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) own[j] = ld4(x + (size_t)row * width + (size_t)h * kV + vcol + 4 * j);
+        float4 own[4];                               // the values as they are
+        fetch_rows(own, x + (size_t)h * kV, width, n);
         uint32_t u[16], o[16];
         ld16(mine + old + (i & 1) * kV + vcol, u);
         wait_ld();
@@ -352,11 +350,20 @@ ssm_outputs_kernel(const StateSpace<T_> p) {
         }
         float* to = p.y + ((size_t)first * p.H + h) * kV;
         if (!__syncthreads_or(z != 0.f && row < n)) {
-            if (row < n)
+            // through shared memory (the values have been read), so that neighbouring threads store neighbours
+            uint8_t* rows = smem_raw + (values - smem_u32(smem_raw));
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    walk::st4(to + (size_t)row * p.H * kV + vcol + 4 * j, make_float4(fmaf(skip, own[j].x, y[4 * j]), fmaf(skip, own[j].y, y[4 * j + 1]),
-                                                                                fmaf(skip, own[j].z, y[4 * j + 2]), fmaf(skip, own[j].w, y[4 * j + 3])));
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<float4*>(rows + row * 256 + (((4 * part + j) ^ (row & 7)) << 4)) = make_float4(y[4 * j], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int r = 32 * j + 2 * warp + (lane >> 4), q = lane & 15;
+                const float4 v = *reinterpret_cast<const float4*>(rows + r * 256 + ((q ^ (r & 7)) << 4));
+                if (r < n)
+                    walk::st4(to + (size_t)r * p.H * kV + 4 * q, make_float4(fmaf(skip, own[j].x, v.x), fmaf(skip, own[j].y, v.y), fmaf(skip, own[j].z, v.z), fmaf(skip, own[j].w, v.w)));
+            }
+            __syncthreads();                         // before the next head's values
         } else {                                     // token by token: a column of the state and 16 rows a thread
             const int v0 = threadIdx.x >> 3, d0 = (threadIdx.x & 7) * 16;
             float s[16];

@@ -115,9 +115,9 @@ class StateSpaceMixer(Mixer):
     def in_tiles(self, step, device) -> bool:
         """Whether a step that csrc/ssm_tiles.cu takes (bfloat16, states of 128 rows, heads of 64 columns) goes there: by estimates of it
         and of the form token by token.  A block takes a chunk of 128 tokens, full or not, and up to eight of a group's heads: 13 us each and 10 for what
-        they share.  Measured, a layer of 64 heads in 8 groups, us before / now: one entry of 110 tokens 92/89, of 128 94/90, of 512 124/109, of 2,048 298/247; four of 40
-        87/92, of 60 108/90, of 300 233/209; sixty-four of 20 400/524, of 40 749/605, of 96 1,719/830; one of 300 beside 15 single tokens 218/179,
-        beside 31 249/284, of 1,024 beside 63 662/531.  Few heads over few tokens stay in chunks of 64 (8 heads of 256 tokens 27, here 33).  The chunks' states
+        they share.  Measured, a layer of 64 heads in 8 groups, us before / now: one entry of 110 tokens 91/88, of 128 94/90, of 512 124/105, of 2,048 298/233; four of 40
+        90/92, of 60 109/90, of 300 232/203; sixty-four of 20 401/527, of 40 750/606, of 96 1,722/816; one of 300 beside 15 single tokens 217/167,
+        beside 31 251/272, of 1,024 beside 63 657/521.  Few heads over few tokens stay in chunks of 64 (8 heads of 256 tokens 26, here 29).  The chunks' states
         take 32 KB per head and chunk: no more than 256 MB, or than the other chunks' workspace."""
         if self.chunk_min_tokens is None or not getattr(self, "chunks_by_estimate", True):
             return False
