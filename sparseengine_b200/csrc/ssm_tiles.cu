@@ -85,25 +85,25 @@ __device__ __forceinline__ void fetch_rows(float4 (&v)[4], const float* src, siz
     }
 }
 template <typename Factor>
-__device__ __forceinline__ void put_values(uint32_t at, const float4 (&v)[4], Factor factor) {
+__device__ __forceinline__ void put_values(uint32_t at, uint32_t term, const float4 (&v)[4], Factor factor) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int t = 32 * i + 2 * warp + (lane >> 4);
         const float f = factor(t);
-        put4(at, kUTerm, t, lane & 15, make_float4(v[i].x * f, v[i].y * f, v[i].z * f, v[i].w * f));
+        put4(at, term, t, lane & 15, make_float4(v[i].x * f, v[i].y * f, v[i].z * f, v[i].w * f));
     }
 }
 
-// What each chunk adds to its heads' states: rows of the state = the M side, B's rows as they lie.  A head's values are cut while the products of the head before run.
+// What each chunk adds to its heads' states: rows of the state = the M side, B's rows as they lie, two heads' columns the N side (one at a time, N = 64, shared memory
+// holds the products up: 32 us, 27 so).  A pair's sums are stored while the next pair's products run.
 template <typename T_>
 __global__ void __launch_bounds__(kThreads, 1)
 ssm_states_kernel(const StateSpace<T_> p) {
     extern __shared__ uint8_t smem_raw[];
-    const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u, keys = base, values = base + 3 * kTerm;
+    const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u, keys = base, values = base + 3 * kTerm;       // values: terms of two heads' columns side by side
     Tables& tab = *reinterpret_cast<Tables*>(smem_raw + (base - smem_u32(smem_raw)) + 3 * kTerm + 6 * kUTerm);
     __shared__ Shared sh;
-    __shared__ __align__(8) uint64_t done[2];
     int first, n;
     chunk_of<kT>(blockIdx.x, p.cu_q, p.entries, first, n);
     if (n <= 0) return;
@@ -112,42 +112,47 @@ ssm_states_kernel(const StateSpace<T_> p) {
     const size_t width = (size_t)p.H * kV + 2 * (size_t)p.G * kD;
     const float* x = p.xbc + (size_t)first * width;
     const float* b = x + (size_t)p.H * kV + (size_t)g * kD;
-    if (threadIdx.x < 2) fa::mbar_init(smem_u32(&done[threadIdx.x]), 1);
     const uint32_t tmem = (uint32_t)fa::uniform((int)begin(sh));
-    const int role = fa::uniform(warp);
+    const bool issuer = fa::uniform(warp) == 0;
     const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + col;
-    float4 v[4];
-    fetch_rows(v, x + (size_t)h0 * kV, width, n);
+    float4 v[2][4];
+    auto fetch = [&](int i) {
+        fetch_rows(v[0], x + (size_t)(h0 + i) * kV, width, n);
+        if (i + 1 < heads) fetch_rows(v[1], x + (size_t)(h0 + i + 1) * kV, width, n);
+    };
+    fetch(0);
     fill_tables(p, tab, h0, heads, first, n);
     put_rows(keys, b, width, n);
     __syncthreads();
+    const int pairs = (heads + 1) / 2;
     bool ok = true;
-    for (int i = 0; i <= heads && ok; ++i) {         // head i's products are issued, head i - 1's sums stored
-        if (i < heads) {
-            put_values(values + (i & 1) * 3 * kUTerm, v, [&](int t) { return t < n ? decay_between(tab, i, n - 1, t) * tab.step[i][t] : 0.f; });
+    for (int i = 0; i <= pairs && ok; ++i) {         // pair i's products are issued, pair i - 1's sums stored
+        if (i > 0 && !(ok = products_done(sh, i - 1, p.error))) break;
+        if (i < pairs) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if (2 * i + j < heads)
+                    put_values(values + j * kUTerm, 2 * kUTerm, v[j], [&](int t) { return t < n ? decay_between(tab, 2 * i + j, n - 1, t) * tab.step[2 * i + j][t] : 0.f; });
             fence_smem();
             fence_before();
             __syncthreads();
-            if (role == (i & 1)) {
+            if (issuer) {
                 fence_after();
                 if (fa::elect_one()) {
-                    product<true, true, 3>(tmem + (i & 1) * kV, keys, kHalf, kTerm, values + (i & 1) * 3 * kUTerm, 0, kUTerm, instr(kV, true, true));
-                    fa::umma_commit(smem_u32(&done[i & 1]));
+                    product<true, true, 3>(tmem + (i & 1) * 2 * kV, keys, kHalf, kTerm, values, kUTerm, 2 * kUTerm, instr(2 * i + 1 < heads ? 2 * kV : kV, true, true));
+                    fa::umma_commit(smem_u32(&sh.done));
                 }
                 __syncwarp();
             }
-            if (i + 1 < heads) fetch_rows(v, x + (size_t)(h0 + i + 1) * kV, width, n);
+            if (i + 1 < pairs) fetch(2 * i + 2);
         }
-        if (i > 0) {
-            const int h = h0 + i - 1;
-            ok = __syncthreads_and(fa::mbar_wait(smem_u32(&done[(i - 1) & 1]), ((i - 1) >> 1) & 1, &sh.abort_flag));
-            fence_after();
-            if (!ok) {
-                if (threadIdx.x == 0) atomicCAS(p.error, 0, kErrorCode);
-                break;
-            }
+        if (i == 0) continue;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int own = 2 * (i - 1) + j, h = h0 + own;
+            if (own >= heads) break;
             uint32_t w[16];
-            ld16(mine + ((i - 1) & 1) * kV, w);
+            ld16(mine + ((i - 1) & 1) * 2 * kV + j * kV, w);
             wait_ld();
             float sum[16], z = 0.f;
 #pragma unroll
@@ -160,7 +165,7 @@ ssm_states_kernel(const StateSpace<T_> p) {
                 for (int c = 0; c < 16; ++c) sum[c] = 0.f;
 #pragma unroll 1
                 for (int t = 0; t < n; ++t) {
-                    const float k = b[(size_t)t * width + row], f = decay_between(tab, i - 1, n - 1, t) * tab.step[i - 1][t];
+                    const float k = b[(size_t)t * width + row], f = decay_between(tab, own, n - 1, t) * tab.step[own][t];
 #pragma unroll
                     for (int c = 0; c < 16; ++c) sum[c] = fmaf(k, x[(size_t)t * width + (size_t)h * kV + col + c] * f, sum[c]);
                 }
@@ -168,7 +173,7 @@ ssm_states_kernel(const StateSpace<T_> p) {
             float* to = p.states + ((size_t)blockIdx.x * p.H + h) * (kV * kD) + row;
 #pragma unroll
             for (int c = 0; c < 16; ++c) to[(size_t)(col + c) * kD] = sum[c];
-            if (threadIdx.x == 0) p.totals[(size_t)blockIdx.x * p.H + h] = expf(tab.hi[i - 1][n - 1] + tab.lo[i - 1][n - 1]);
+            if (threadIdx.x == 0) p.totals[(size_t)blockIdx.x * p.H + h] = expf(tab.hi[own][n - 1] + tab.lo[own][n - 1]);
         }
     }
     end(sh);
@@ -273,7 +278,7 @@ ssm_outputs_kernel(const StateSpace<T_> p) {
     for (int i = 0; i < heads && ok; ++i) {
         const int h = h0 + i;
         // P of this head: the block on the diagonal by its own exponents, those before it by e^(B_t - B_r) e^(B_r - B_s), r the block's first token
-        put_values(values, uv, [&](int t) { return tab.step[i][t]; });
+        put_values(values, kUTerm, uv, [&](int t) { return tab.step[i][t]; });
         const int block = warp & 3, r = 32 * block;  // rows r .. r + 31; a warp's columns are eight of each block of 32
         const float f = decay_between(tab, i, row, r);
         const float before = lane < 8 * block ? decay_between(tab, i, r, 32 * (lane >> 3) + 8 * part + (lane & 7)) : 0.f;
