@@ -197,6 +197,7 @@ retention_states_kernel(const Retention p) {
 __global__ void __launch_bounds__(256)
 retention_join_kernel(const Retention p) {
     __shared__ float turned[32][33];
+    grid_dependency_trigger();                       // the outputs' kernel may fetch its first chunk
     const int e = blockIdx.z, h = blockIdx.y, c0 = (blockIdx.x >> 2) * 32, r0 = (blockIdx.x & 3) * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int len = p.cu_q[e + 1] - p.cu_q[e], chunks = ceil_div(len, kT);
     if (len <= 0) return;
@@ -278,6 +279,7 @@ retention_outputs_kernel(const Retention p) {
     if (threadIdx.x == 32) find(items[0]);
     __syncthreads();
     if (items[0].n > 0) fetch(items[0]);
+    grid_dependency_wait();                          // the states at the chunks' and the segments' starts (angles and powers are older than the kernel before this one)
     for (uint32_t j = 0; items[j & 1].n > 0; ++j) {
         const Item& t = items[j & 1];
         const Item& next = items[(j & 1) ^ 1];
@@ -574,6 +576,6 @@ extern "C" int se_retention_tiles(const void* proj, int pitch, int q_off, int k_
     retention_states_kernel<<<dim3(entries * segments, heads), kThreads, states_smem, stream>>>(p);
     if (segments > 1) retention_join_kernel<<<dim3(16, heads, entries), 256, 0, stream>>>(p);
     const long long items = places * heads;
-    retention_outputs_kernel<<<(int)(items < sms ? items : sms), kThreads, outputs_smem, stream>>>(p);
-    SE_LAUNCH_CHECK();
+    if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
+    return (int)SE_LAUNCH_DEPENDENT_IF(segments > 1, "ret", retention_outputs_kernel, dim3((unsigned)(items < sms ? items : sms)), dim3(kThreads), (size_t)outputs_smem, stream, p);
 }

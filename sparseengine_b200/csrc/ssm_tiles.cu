@@ -183,6 +183,7 @@ ssm_states_kernel(const StateSpace<T_> p) {
 template <typename T_>
 __global__ void __launch_bounds__(256)
 ssm_scan_kernel(const StateSpace<T_> p) {
+    grid_dependency_trigger();                       // the outputs' kernel may start: it has C B^T to form first
     const int e = blockIdx.z, h = blockIdx.y, i = (blockIdx.x * 256 + threadIdx.x) * 4;
     const int t0 = p.cu_q[e], chunks = ceil_div(p.cu_q[e + 1] - t0, kT);
     if (chunks <= 0) return;
@@ -269,6 +270,7 @@ ssm_outputs_kernel(const StateSpace<T_> p) {
     }
     fetch_rows(uv, x + (size_t)h0 * kV, width, n);
     ok = products_done(sh, round++, p.error);        // B's terms give way to the first head's state and values
+    grid_dependency_wait();                          // the states at the chunks' starts
     if (ok) {
         put_state(0);
         fence_smem();
@@ -402,8 +404,8 @@ static int launch_ssm(const StateSpace<T_>& p, int places, cudaStream_t stream) 
     const dim3 grid(places, p.G * p.blocks);
     ssm_states_kernel<T_><<<grid, kThreads, states_smem, stream>>>(p);
     ssm_scan_kernel<T_><<<dim3(kV * kD / 1024, p.H, p.entries), 256, 0, stream>>>(p);
-    ssm_outputs_kernel<T_><<<grid, kThreads, outputs_smem, stream>>>(p);
-    SE_LAUNCH_CHECK();
+    if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
+    return (int)SE_LAUNCH_DEPENDENT("ssm", ssm_outputs_kernel<T_>, grid, dim3(kThreads), (size_t)outputs_smem, stream, p);
 }
 
 }  // namespace tiles
