@@ -161,8 +161,9 @@ __device__ __forceinline__ void end(Shared& s) {
     }
 }
 // Until the products committed `n`-th (from 0) are there; the same answer in every thread.  A wait that runs out is reported.
-__device__ __forceinline__ bool products_done(Shared& s, uint32_t n, int* error) {
-    const bool ok = fa::mbar_wait(smem_u32(&s.done), n & 1, &s.abort_flag);
+// `so_far`: false in a thread whose earlier wait by itself ran out.
+__device__ __forceinline__ bool products_done(Shared& s, uint32_t n, int* error, bool so_far = true) {
+    const bool ok = so_far && fa::mbar_wait(smem_u32(&s.done), n & 1, &s.abort_flag);
     if (__syncthreads_and(ok)) {
         fence_after();
         return true;

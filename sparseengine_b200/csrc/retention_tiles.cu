@@ -6,8 +6,8 @@
 // state at each chunk's start, `join` (where an entry has several segments) the states at the segments' starts, `outputs` (a block per chunk and head)
 // the rest: q and k turned on their way from the projection, both products with q, the decays, P v, and where the mixer norms each head the norm and the gate.
 //
-// Measured, 8,192 tokens of 32 heads (the walk, its preparation and the norm: 675 us): 322 = angles 4 + states 73 + join 4 + outputs 232; 2,048 tokens of 16
-// heads 147 and 60; four entries of 100 tokens, 32 heads, 54 and 39.  Errors against 64 bits over the result's norm: outputs 2.0e-7 to 2.7e-7 (the walk 1.4e-7 to 2.1e-7), states
+// Measured, 8,192 tokens of 32 heads (the walk, its preparation and the norm: 675 us): 311 = angles 4 + states 73 + join 4 + outputs 224; 2,048 tokens of 16
+// heads 147 and 56; four entries of 100 tokens, 32 heads, 54 and 39.  Errors against 64 bits over the result's norm: outputs 2.0e-7 to 2.7e-7 (the walk 1.4e-7 to 2.1e-7), states
 // 0.8e-7 to 1.5e-7 (0.8e-7 to 2.2e-7), where 16-bit inputs and outputs leave 4e-3.
 #include "chunk_tiles.cuh"
 
@@ -234,7 +234,8 @@ retention_join_kernel(const Retention p) {
 
 // A block takes chunks in turn.  The next chunk's q, k and angles are fetched into room that this one's products have left (the state's terms, the last of
 // k's) while its weights are made and P v runs; the state comes into registers meanwhile.  Bound by the steps of a chunk, 16 us, one after another: the
-// products take 8,000 cycles of 32,000, instructions issue in 30 %.  Measured, 8,192 tokens of 32 heads: 232 us; q and angles row by row from memory and outputs and gates a row a
+// products take 8,000 cycles of 30,000, instructions issue in 30 %; a warp is held by the products that it issues, so warp 0 cuts no part of the state (all sixteen: 232 us).
+// Measured, 8,192 tokens of 32 heads: 224 us; q and angles row by row from memory and outputs and gates a row a
 // thread 292, the latter alone 240; a warp group per operand, which leaves 64 to 112 registers a thread and spills, 253 to 288; a warp that only issues products, 112 registers, 274.
 //   columns of tensor memory: q's terms, then P's 0-191; scores, then P v 192-319; what the state gives 320-447
 __global__ void __launch_bounds__(kThreads, 1)
@@ -246,8 +247,10 @@ retention_outputs_kernel(const Retention p) {
     float* plain = reinterpret_cast<float*>(sm);                                          // for the form token by token
     float (*squares)[kT] = reinterpret_cast<float (*)[kT]>(sm + 6 * kTerm);               // where the values have been read
     __shared__ Shared sh;
+    __shared__ __align__(8) uint64_t scores_done;
     __shared__ float power[kT + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp >> 2, row = (warp & 3) * 32 + lane, col = part * 32, quad = lane & 15;
+    if (threadIdx.x == 0) fa::mbar_init(smem_u32(&scores_done), 1);
     const uint32_t tmem = (uint32_t)fa::uniform((int)begin(sh));
     const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16), scores = 192, old = 320;
     const bool issuer = fa::uniform(warp) == 0;
@@ -292,9 +295,11 @@ retention_outputs_kernel(const Retention p) {
         const float* S = p.states + ((size_t)t.place * p.H + h) * (kD * kD);
         const float* S_seg = t.seg > 0 ? p.starts + ((size_t)(t.e * p.segments + t.seg) * p.H + h) * (kD * kD) : nullptr;
         const float lead = p.powers[(size_t)h * p.powers_pitch + kT + 1 + t.inner];
-        float4 own_S[4];                             // the state at the chunk's start: a column of it per warp at a time, half of them ahead
+        // the state at the chunk's start: a column of it per warp at a time, four of them ahead; none for the warp that issues, which the scores' products hold
+        constexpr int kOthers = kThreads / 32 - 1;
+        float4 own_S[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) own_S[i] = ld4(S + (size_t)(16 * i + warp) * kD + 4 * lane);
+        for (int i = 0; i < 4; ++i) own_S[i] = issuer ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4(S + (size_t)(kOthers * i + warp - 1) * kD + 4 * lane);
         walk::cp_wait<0>();
         __syncthreads();                             // k, q and angles are there
         fetch_rows(p, values, p.v_off, first, n, h);
@@ -350,39 +355,44 @@ retention_outputs_kernel(const Retention p) {
             fence_after();
             if (fa::elect_one()) {
                 product_ts<false, 3>(tmem + scores, tmem, keys, kHalf, kTerm, instr(kT, false, false));
-                fa::umma_commit(smem_u32(&sh.done));
+                fa::umma_commit(smem_u32(&scores_done));
             }
             __syncwarp();
-        }
+        } else {
 #pragma unroll
-        for (int i = 0; i < 8; i += 4) {
-            float4 seg[4];
-            if (i > 0)
+            for (int i = 0; i < 12; i += 4) {
+                float4 seg[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) own_S[j] = ld4(S + (size_t)(16 * (i + j) + warp) * kD + 4 * lane);
-            if (S_seg != nullptr)
+                for (int j = 0; j < 4; ++j) {
+                    const int c = kOthers * (i + j) + warp - 1;
+                    if (c >= kD) continue;
+                    if (i > 0) own_S[j] = ld4(S + (size_t)c * kD + 4 * lane);
+                    if (S_seg != nullptr) seg[j] = ld4(S_seg + (size_t)c * kD + 4 * lane);
+                }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) seg[j] = ld4(S_seg + (size_t)(16 * (i + j) + warp) * kD + 4 * lane);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float4 v = own_S[j];
-                if (S_seg != nullptr) v = make_float4(fmaf(lead, seg[j].x, v.x), fmaf(lead, seg[j].y, v.y), fmaf(lead, seg[j].z, v.z), fmaf(lead, seg[j].w, v.w));
-                put4(state + (lane >> 4) * kHalf, kTerm, 16 * (i + j) + warp, quad, v);
+                for (int j = 0; j < 4; ++j) {
+                    const int c = kOthers * (i + j) + warp - 1;
+                    if (c >= kD) continue;
+                    float4 v = own_S[j];
+                    if (S_seg != nullptr) v = make_float4(fmaf(lead, seg[j].x, v.x), fmaf(lead, seg[j].y, v.y), fmaf(lead, seg[j].z, v.z), fmaf(lead, seg[j].w, v.w));
+                    put4(state + (lane >> 4) * kHalf, kTerm, c, quad, v);
+                }
             }
         }
         walk::cp_wait<0>();
         fence_smem();
         __syncthreads();
-        if (issuer) {                                // (one barrier: the scores' end is waited for before this one's is committed)
-            if (fa::elect_one()) product_ts<false, 3>(tmem + old, tmem, state, kHalf, kTerm, instr(kD, false, false));
+        if (issuer) {
+            if (fa::elect_one()) {
+                product_ts<false, 3>(tmem + old, tmem, state, kHalf, kTerm, instr(kD, false, false));
+                fa::umma_commit(smem_u32(&sh.done));
+            }
             __syncwarp();
         }
         if (threadIdx.x == 32) find(items[(j & 1) ^ 1]);
-        if (!(ok = products_done(sh, round++, p.error))) break;
-        if (issuer) {
-            if (fa::elect_one()) fa::umma_commit(smem_u32(&sh.done));
-            __syncwarp();
-        }
+        // the scores, warp by warp: the others need not wait for the one that issues (a wait that ran out shows in the next one)
+        ok = fa::mbar_wait(smem_u32(&scores_done), j & 1, &sh.abort_flag);
+        fence_after();
         {
             uint32_t w[3][8];
             auto weights = [&](int half) {
@@ -403,7 +413,7 @@ retention_outputs_kernel(const Retention p) {
                 }
             };
             weights(0);
-            if (!(ok = products_done(sh, round++, p.error))) break;          // q's terms give way
+            if (!(ok = products_done(sh, round++, p.error, ok))) break;      // q's terms give way
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
                 if (half) weights(1);
