@@ -22,7 +22,7 @@ struct Retention {
     int powers_pitch;
     float* states;                 // [places][H][128 columns][128 rows]: at a chunk's start, from its segment's start on
     float* starts;                 // [entries * segments][H][128][128]: what a segment leaves by itself, then the state at its start
-    int segments, seg_chunks;      // per entry at most; chunks of a segment
+    int segments, seg_chunks;      // per entry at most; chunks of a segment (the last one takes what is left: a captured step may meet longer entries)
     float* state;
     long long state_stride;
     const int* cu_q;
@@ -48,6 +48,12 @@ retention_tables_kernel(float2* __restrict__ turn, const int* __restrict__ posit
     const int h = blockIdx.x - turn_blocks;
     const double g = (double)decay[h];
     for (int i = threadIdx.x; i < pitch; i += 256) powers[(size_t)h * pitch + i] = (float)pow(g, (double)(i <= kT ? i : (i - kT - 1) * kT));
+}
+
+// g^(128 j) of a head
+__device__ __forceinline__ float chunks_power(const Retention& p, int h, int j) {
+    const float* power = p.powers + (size_t)h * p.powers_pitch;
+    return j <= p.seg_chunks ? power[kT + 1 + j] : (float)pow((double)power[1], (double)j * kT);
 }
 
 // a pair of a row turned by its angle
@@ -111,7 +117,7 @@ retention_states_kernel(const Retention p) {
     __shared__ float power[kT + 1];
     const int e = blockIdx.x / p.segments, seg = blockIdx.x - e * p.segments, h = blockIdx.y;
     const int t_first = p.cu_q[e], t_last = p.cu_q[e + 1];
-    const int c0 = seg * p.seg_chunks, c1 = min(c0 + p.seg_chunks, ceil_div(t_last - t_first, kT));
+    const int chunks = ceil_div(t_last - t_first, kT), c0 = seg * p.seg_chunks, c1 = seg == p.segments - 1 ? chunks : min(c0 + p.seg_chunks, chunks);
     if (c0 >= c1) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = (warp & 3) * 32 + lane, col = (warp >> 2) * 32;
     for (int i = threadIdx.x; i <= kT; i += kThreads) power[i] = p.powers[(size_t)h * p.powers_pitch + i];
@@ -215,8 +221,8 @@ retention_join_kernel(const Retention p) {
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
             if (seg0 + x >= most) break;
-            const int tokens = min(len - (seg0 + x) * p.seg_chunks * kT, p.seg_chunks * kT);
-            const float f = power[kT + 1 + tokens / kT] * power[tokens % kT];
+            const int rest = len - (seg0 + x) * p.seg_chunks * kT, tokens = seg0 + x == p.segments - 1 ? rest : min(rest, p.seg_chunks * kT);
+            const float f = chunks_power(p, h, tokens / kT) * power[tokens % kT];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 if (seg0 + x) at[x * step + (size_t)(c0 + ty + 8 * i) * kD] = S[i];
@@ -267,8 +273,8 @@ retention_outputs_kernel(const Retention p) {
             int first, n;
             const int e = chunk_of<kT>(place, p.cu_q, p.entries, first, n);
             if (n <= 0) continue;
-            const int chunk = place - p.cu_q[e] / kT - e, seg = chunk / p.seg_chunks;
-            if (seg < p.segments) t = Item{e, at - place * p.H, first, n, place, seg, chunk - seg * p.seg_chunks};     // (else an entry longer than the host knew)
+            const int chunk = place - p.cu_q[e] / kT - e, seg = min(chunk / p.seg_chunks, p.segments - 1);
+            t = Item{e, at - place * p.H, first, n, place, seg, chunk - seg * p.seg_chunks};
         }
         t.n = max(t.n, 0);
     };
@@ -294,7 +300,7 @@ retention_outputs_kernel(const Retention p) {
         }
         const float* S = p.states + ((size_t)t.place * p.H + h) * (kD * kD);
         const float* S_seg = t.seg > 0 ? p.starts + ((size_t)(t.e * p.segments + t.seg) * p.H + h) * (kD * kD) : nullptr;
-        const float lead = p.powers[(size_t)h * p.powers_pitch + kT + 1 + t.inner];
+        const float lead = S_seg != nullptr ? chunks_power(p, h, t.inner) : 0.f;
         // the state at the chunk's start: a column of it per warp at a time, four of them ahead; none for the warp that issues, which the scores' products hold
         constexpr int kOthers = kThreads / 32 - 1;
         float4 own_S[4];

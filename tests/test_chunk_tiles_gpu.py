@@ -21,9 +21,10 @@ def _step(lens):
                            max_q_len=max(lens), cu=cu, rows=rows)
 
 
-def _retention(lens, heads, rotary, decay, bad=None, out=False):
+def _retention(lens, heads, rotary, decay, bad=None, out=False, known=None):
     from sparseengine_b200.csrc import ops
     d, step = 128, _step(lens)
+    step.max_q_len = known or step.max_q_len
     T, g = step.num_tokens, torch.Generator(device=DEV).manual_seed(heads)
     proj = torch.randn(T, 8 + 4 * heads * d, generator=g, device=DEV).to(torch.bfloat16)      # v, 8 columns that nobody reads, k, q, gate
     v_off, k_off, q_off, g_off = 0, heads * d + 8, 2 * heads * d + 8, 3 * heads * d + 8
@@ -61,6 +62,17 @@ def test_retention_against_the_walk(lens, heads, rotary, decay):
         _close(state[row, :heads * d * d].view(heads, d, d), S, f"state after {n} tokens")
     others = [r for r in range(len(lens) + 2) if r not in step.rows]
     assert torch.equal(state[others], first[others]) and torch.equal(state[:, heads * d * d:], first[:, heads * d * d:])
+
+
+@pytest.mark.parametrize("lens,known", [([1500, 40], 300), ([900], 60)])
+def test_retention_of_entries_longer_than_the_host_knows(lens, known):
+    """What a captured step meets when it is replayed with the same tokens in other entries."""
+    step, o, first, state, inputs, _ = _retention(lens, 2, 128, "slow", known=known)
+    for e, n in enumerate(lens):
+        a, b, row = step.cu[e], step.cu[e + 1], step.rows[e]
+        want, S = _walk64(*(x[a:b] for x in inputs), first[row, :2 * 128 * 128].double().view(2, 128, 128))
+        _close(o[a:b].view(n, 2, 128), want, f"outputs of {n} tokens")
+        _close(state[row, :2 * 128 * 128].view(2, 128, 128), S, f"state after {n} tokens")
 
 
 def test_retention_with_norm_and_gate():
