@@ -11,6 +11,7 @@
 // makes P and where needed W and U (and per-channel decays' scaled q and k); and a `walk` kernel per (request, head, tile of
 // value columns) that takes the chunks in turn with its slice of the state in shared memory: two or three small matrix
 // products per chunk instead of a chain of T dependent steps.
+// (State spaces and retention beside bfloat16 activations have a form whose outputs are no part of the chain: chunk_tiles.cuh.)
 //
 // What bounds the walk is the chain of a chunk: products, the split of their operands, barriers, the state through shared memory.  The tensor pipe is busy
 // 43 % of the time (state space), instructions issue in 49 % of the cycles; 16-bit operands would
