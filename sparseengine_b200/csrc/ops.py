@@ -855,12 +855,11 @@ def ssm_tiles(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, step, y, *,
     """The recurrence of :func:`ssm_walk` in chunks of 128 tokens side by side on tcgen05 (csrc/ssm_tiles.cu)."""
     tokens, n = xbc.shape[0], step.num_seqs
     work = _walk_work((tokens // 128 + n) * heads * (head_dim * state_size + 1), xbc.device)
-    _check(_fn("se_ssm_tiles", "ppii" "ppp" "pl" "pp" "ppp" "iiiiiiii" "p")(
-        _ptr(xbc, torch.float32, "xbc"), _rows_ptr(proj, "proj"), proj.stride(0), int(dt_off),
+    _check(_fn("se_ssm_tiles", "ppii" "ppp" "pl" "pp" "ppp" "iiiiiii" "p")(
+        _ptr(xbc, torch.float32, "xbc"), _rows_ptr(proj, "proj", torch.bfloat16), proj.stride(0), int(dt_off),
         _ptr(dt_bias, torch.float32, "dt_bias"), _ptr(a_log, torch.float32, "a_log"), _ptr(d_skip, torch.float32, "d_skip"),
         _ptr(state, torch.float32, "state"), state.stride(0), _ptr(step.cu_q), _ptr(step.seq_rows), _ptr(y, torch.float32, "y"),
-        work.data_ptr(), _ptr(error_word(xbc.device)), tokens, n, heads, head_dim, state_size, groups, sm_count(xbc.device), dtype_code(proj.dtype),
-        _stream()), "ssm_tiles")
+        work.data_ptr(), _ptr(error_word(xbc.device)), tokens, n, heads, head_dim, state_size, groups, sm_count(xbc.device), _stream()), "ssm_tiles")
     return y
 
 

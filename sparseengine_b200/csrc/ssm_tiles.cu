@@ -15,10 +15,9 @@ constexpr int kV = 64, kHeads = 8;                   // columns of a head's stat
 constexpr int kSTerm = kV * 256, kSHalf = kV * 128;  // bytes of a term of the state (rows along its columns), of half of one
 constexpr int kUTerm = kT * 128;                     // of the values: rows are tokens
 
-template <typename T_>
 struct StateSpace {
     const float* xbc;              // [tokens][H * 64 + 2 G * 128]: values, B, C
-    const T_* proj;                // steps' columns from dt_off on
+    const __nv_bfloat16* proj;                // steps' columns from dt_off on
     int pitch, dt_off;
     const float* dt_bias;
     const float* a_log;
@@ -37,8 +36,7 @@ struct StateSpace {
 struct Tables { float hi[kHeads][kT], lo[kHeads][kT], step[kHeads][kT]; };
 
 // B_t of a block's heads as two 32-bit parts, and the steps (0 where there is no token), a warp per head and four tokens a lane
-template <typename T_>
-__device__ __forceinline__ void fill_tables(const StateSpace<T_>& p, Tables& s, int h0, int heads, int first, int n) {
+__device__ __forceinline__ void fill_tables(const StateSpace& p, Tables& s, int h0, int heads, int first, int n) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp >= heads) return;
     const int h = h0 + warp;
@@ -97,9 +95,8 @@ __device__ __forceinline__ void put_values(uint32_t at, uint32_t term, const flo
 
 // What each chunk adds to its heads' states: rows of the state = the M side, B's rows as they lie, two heads' columns the N side (one at a time, N = 64, shared memory
 // holds the products up: 32 us, 27 so).  A pair's sums are stored while the next pair's products run.
-template <typename T_>
 __global__ void __launch_bounds__(kThreads, 1)
-ssm_states_kernel(const StateSpace<T_> p) {
+ssm_states_kernel(const StateSpace p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u, keys = base, values = base + 3 * kTerm;       // values: terms of two heads' columns side by side
     Tables& tab = *reinterpret_cast<Tables*>(smem_raw + (base - smem_u32(smem_raw)) + 3 * kTerm + 6 * kUTerm);
@@ -180,9 +177,8 @@ ssm_states_kernel(const StateSpace<T_> p) {
 }
 
 // What chunks add -> the states at their starts; the last one goes back to the entry's row.  Four elements a thread; four chunks asked for together.
-template <typename T_>
 __global__ void __launch_bounds__(256)
-ssm_scan_kernel(const StateSpace<T_> p) {
+ssm_scan_kernel(const StateSpace p) {
     grid_dependency_trigger();                       // the outputs' kernel may start: it has C B^T to form first
     const int e = blockIdx.z, h = blockIdx.y, i = (blockIdx.x * 256 + threadIdx.x) * 4;
     const int t0 = p.cu_q[e], chunks = ceil_div(p.cu_q[e + 1] - t0, kT);
@@ -214,9 +210,8 @@ ssm_scan_kernel(const StateSpace<T_> p) {
 // a warp is held by the products it issues (one for both 116, two 87); outputs leave through shared memory (a row a thread 77, 63 so).
 // Columns of tensor memory: C B^T 0-127, P's terms 128-319, what the state gives 320-447 (two heads in turn), P u 448-511.  While a head's P u is summed the next
 // head's state is cut and its product with C queued behind.
-template <typename T_>
 __global__ void __launch_bounds__(kThreads, 1)
-ssm_outputs_kernel(const StateSpace<T_> p) {
+ssm_outputs_kernel(const StateSpace p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u, queries = base, keys = base + 3 * kTerm, state = keys, values = keys + 3 * kSTerm;
     Tables& tab = *reinterpret_cast<Tables*>(smem_raw + (base - smem_u32(smem_raw)) + 6 * kTerm);
@@ -224,7 +219,10 @@ ssm_outputs_kernel(const StateSpace<T_> p) {
     __shared__ __align__(8) uint64_t state_done;
     int first, n;
     chunk_of<kT>(blockIdx.x, p.cu_q, p.entries, first, n);
-    if (n <= 0) return;
+    if (n <= 0) {
+        grid_dependency_wait();                      // nothing of this kernel ends before the one ahead
+        return;
+    }
     const int rep = p.H / p.G, g = blockIdx.y / p.blocks, h0 = g * rep + (blockIdx.y - g * p.blocks) * p.per, heads = min(p.per, (g + 1) * rep - h0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp >> 2, row = (warp & 3) * 32 + lane, vcol = part * 16;
     const size_t width = (size_t)p.H * kV + 2 * (size_t)p.G * kD;
@@ -395,17 +393,16 @@ ssm_outputs_kernel(const StateSpace<T_> p) {
     end(sh);
 }
 
-template <typename T_>
-static int launch_ssm(const StateSpace<T_>& p, int places, cudaStream_t stream) {
+static int launch_ssm(const StateSpace& p, int places, cudaStream_t stream) {
     const int states_smem = 3 * kTerm + 6 * kUTerm + (int)sizeof(Tables) + 1024, outputs_smem = 6 * kTerm + (int)sizeof(Tables) + 1024;
-    cudaError_t e = cudaFuncSetAttribute(ssm_states_kernel<T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, states_smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(ssm_outputs_kernel<T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, outputs_smem);
+    cudaError_t e = cudaFuncSetAttribute(ssm_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, states_smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(ssm_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, outputs_smem);
     if (e != cudaSuccess) return (int)e;
     const dim3 grid(places, p.G * p.blocks);
-    ssm_states_kernel<T_><<<grid, kThreads, states_smem, stream>>>(p);
-    ssm_scan_kernel<T_><<<dim3(kV * kD / 1024, p.H, p.entries), 256, 0, stream>>>(p);
+    ssm_states_kernel<<<grid, kThreads, states_smem, stream>>>(p);
+    ssm_scan_kernel<<<dim3(kV * kD / 1024, p.H, p.entries), 256, 0, stream>>>(p);
     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
-    return (int)SE_LAUNCH_DEPENDENT("ssm", ssm_outputs_kernel<T_>, grid, dim3(kThreads), (size_t)outputs_smem, stream, p);
+    return (int)SE_LAUNCH_DEPENDENT("ssm", ssm_outputs_kernel, grid, dim3(kThreads), (size_t)outputs_smem, stream, p);
 }
 
 }  // namespace tiles
@@ -415,10 +412,10 @@ using namespace se::tiles;
 
 extern "C" int se_ssm_tiles_supported(int state_size, int head_dim) { return state_size == kD && head_dim == kV; }
 
-// Arguments as se_ssm_walk's.  work: float [(tokens / 128 + entries) * H * (64 * 128 + 1)].
+// Arguments as se_ssm_walk's, proj bfloat16.  work: float [(tokens / 128 + entries) * H * (64 * 128 + 1)].
 extern "C" int se_ssm_tiles(const float* xbc, const void* proj, int pitch, int dt_off, const float* dt_bias, const float* a_log, const float* d_skip,
                             float* state, long long state_stride, const int* cu_q, const int* seq_rows, float* y, float* work, int* error, int tokens,
-                            int entries, int H, int P, int N, int G, int sms, int dtype, cudaStream_t stream) {
+                            int entries, int H, int P, int N, int G, int sms, cudaStream_t stream) {
     if (entries <= 0 || tokens <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G) return SE_ERR_ARGUMENT;
     const long long places = tokens / kT + entries;
@@ -430,11 +427,9 @@ extern "C" int se_ssm_tiles(const float* xbc, const void* proj, int pitch, int d
     if (!se_ssm_tiles_supported(N, P) || H > 65535 || (long long)G * blocks > 65535 || entries > 65535 || places > 0x7fffffffLL || state_stride % 4 ||
         !aligned(xbc) || !aligned(state) || !aligned(y) || !aligned(work))
         return SE_ERR_UNSUPPORTED;
-    SE_DISPATCH_DTYPE(dtype, T_, {
-        StateSpace<T_> p;
-        p.xbc = xbc; p.proj = (const T_*)proj; p.pitch = pitch; p.dt_off = dt_off; p.dt_bias = dt_bias; p.a_log = a_log; p.d_skip = d_skip;
-        p.states = work; p.totals = work + (size_t)places * H * (kV * kD); p.state = state; p.state_stride = state_stride; p.cu_q = cu_q; p.seq_rows = seq_rows;
-        p.y = y; p.entries = entries; p.H = H; p.G = G; p.blocks = blocks; p.per = per; p.error = error;
-        return launch_ssm<T_>(p, (int)places, stream);
-    });
+    StateSpace p;
+    p.xbc = xbc; p.proj = (const __nv_bfloat16*)proj; p.pitch = pitch; p.dt_off = dt_off; p.dt_bias = dt_bias; p.a_log = a_log; p.d_skip = d_skip;
+    p.states = work; p.totals = work + (size_t)places * H * (kV * kD); p.state = state; p.state_stride = state_stride; p.cu_q = cu_q; p.seq_rows = seq_rows;
+    p.y = y; p.entries = entries; p.H = H; p.G = G; p.blocks = blocks; p.per = per; p.error = error;
+    return launch_ssm(p, (int)places, stream);
 }
