@@ -65,10 +65,10 @@ __device__ __forceinline__ void product(uint32_t d, uint32_t a, uint32_t a_half,
                 started = 1;
             }
 }
-// The same with A in tensor memory, terms of 64 columns; ADD: to what d holds
-template <bool B_MN, int B_TERMS, bool ADD = false>
+// The same with A in tensor memory, terms of 64 columns
+template <bool B_MN, int B_TERMS>
 __device__ __forceinline__ void product_ts(uint32_t d, uint32_t a, uint32_t b, uint32_t b_half, uint32_t b_term, uint32_t id) {
-    uint32_t started = ADD;
+    uint32_t started = 0;
 #pragma unroll
     for (int sum = 2; sum >= 0; --sum)
 #pragma unroll
@@ -119,7 +119,8 @@ __device__ __forceinline__ void put4(uint32_t at, uint32_t term, int row, int qu
     for (int i = 0; i < 3; ++i) sts8(at + i * term, a[i], b[i]);
 }
 
-// Tensor memory, one barrier for the products of a block (each committed and waited for in turn) and the end of both.
+// Tensor memory, one barrier for the products of a block (each committed and waited for in turn) and the end of both.  abort_flag: a wait has run out,
+// the others need not run to their limit.
 struct Shared {
     uint64_t done, last;
     uint32_t tmem;
@@ -133,6 +134,7 @@ __device__ __forceinline__ uint32_t begin(Shared& s) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (threadIdx.x < 32) {
+        __syncwarp();                                // its first lane comes from the branch above, the instruction is the whole warp's
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&s.tmem)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -152,13 +154,21 @@ __device__ __forceinline__ void end(Shared& s) {
     if (threadIdx.x < 32) {
         fence_after();
         fa::mbar_drain(smem_u32(&s.last), 0);
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
     }
+}
+// Until `bar` is in phase `n` (from 0); the same answer in every lane of a warp, whose lanes are together again afterwards: what reads tensor memory next
+// is the whole warp's instruction.
+__device__ __forceinline__ bool warp_wait(Shared& s, uint64_t& bar, uint32_t n) {
+    const bool ok = __all_sync(0xffffffffu, fa::mbar_wait(smem_u32(&bar), n & 1, &s.abort_flag));
+    if (!ok) s.abort_flag = 1;
+    return ok;
 }
 // Until the products committed `n`-th (from 0) are there; the same answer in every thread.  A wait that runs out is reported.
 // `so_far`: false in a thread whose earlier wait by itself ran out.
 __device__ __forceinline__ bool products_done(Shared& s, uint32_t n, int* error, bool so_far = true) {
-    const bool ok = so_far && fa::mbar_wait(smem_u32(&s.done), n & 1, &s.abort_flag);
+    const bool ok = warp_wait(s, s.done, n) && so_far;
     if (__syncthreads_and(ok)) {
         fence_after();
         return true;

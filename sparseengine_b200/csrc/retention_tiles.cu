@@ -396,8 +396,9 @@ retention_outputs_kernel(const Retention p) {
             __syncwarp();
         }
         if (threadIdx.x == 32) find(items[(j & 1) ^ 1]);
+        __syncwarp();
         // the scores, warp by warp: the others need not wait for the one that issues (a wait that ran out shows in the next one)
-        ok = fa::mbar_wait(smem_u32(&scores_done), j & 1, &sh.abort_flag);
+        ok = warp_wait(sh, scores_done, j);
         fence_after();
         {
             uint32_t w[3][8];

@@ -316,7 +316,7 @@ ssm_outputs_kernel(const StateSpace p) {
         fence_smem();
         fence_before();
         // the state's product is there: its terms may give way
-        ok = __syncthreads_and(fa::mbar_wait(smem_u32(&state_done), i & 1, &sh.abort_flag));
+        ok = __syncthreads_and(warp_wait(sh, state_done, i));
         if (!ok) {
             if (threadIdx.x == 0) atomicCAS(p.error, 0, kErrorCode);
             break;
