@@ -6,9 +6,8 @@
 // state at each chunk's start, `join` (where an entry has several segments) the states at the segments' starts, `outputs` (a block per chunk and head)
 // the rest: q and k turned on their way from the projection, both products with q, the decays, P v, and where the mixer norms each head the norm and the gate.
 //
-// Measured, 8,192 tokens of 32 heads (the walk, its preparation and the norm: 675 us): 311 = angles 4 + states 73 + join 4 + outputs 224; 2,048 tokens of 16
-// heads 147 and 56; four entries of 100 tokens, 32 heads, 54 and 39.  Errors against 64 bits over the result's norm: outputs 2.0e-7 to 2.7e-7 (the walk 1.4e-7 to 2.1e-7), states
-// 0.8e-7 to 1.5e-7 (0.8e-7 to 2.2e-7), where 16-bit inputs and outputs leave 4e-3.
+// Measured, 8,192 tokens of 32 heads (the walk, its preparation and the norm: 676 us): 302, of them angles 4, states 74, join 6, outputs 214, starts and ends 4; 2,048 tokens of 16
+// heads 147 and 59; four entries of 100 tokens, 32 heads, 54 and 39.  Errors: chunk_tiles.cuh; 16-bit inputs and outputs leave 4e-3.
 #include "chunk_tiles.cuh"
 
 namespace se {
@@ -159,7 +158,7 @@ retention_states_kernel(const Retention p) {
         if (issuer) {
             fence_after();
             if (fa::elect_one()) {
-                product<true, true, 1>(tmem, keys, kHalf, kTerm, values, kHalf, kTerm, instr(kD, true, true));
+                product<true, true, 1>(tmem, tmem + kD, keys, kHalf, kTerm, values, kHalf, kTerm, instr(kD, true, true));
                 fa::umma_commit(smem_u32(&sh.done));
             }
             __syncwarp();
@@ -171,16 +170,15 @@ retention_states_kernel(const Retention p) {
         }
         store(p.states + ((size_t)(t_first / kT + e + c) * p.H + h) * (kD * kD));
         if (!products_done(sh, round, p.error)) break;
-        uint32_t v[32];
-        fa::tmem_ld32(mine, v);
-        wait_ld();
-        float z = 0.f;
+        float v[32], z = 0.f;
+        ld_sum16(mine, mine + kD, v);
+        ld_sum16(mine + 16, mine + kD + 16, v + 16);
 #pragma unroll
-        for (int x = 0; x < 32; ++x) z = fmaf(__uint_as_float(v[x]), 0.f, z);
+        for (int x = 0; x < 32; ++x) z = fmaf(v[x], 0.f, z);
         const float total = power[n];
         if (!__syncthreads_or(z != 0.f)) {
 #pragma unroll
-            for (int x = 0; x < 32; ++x) S[x] = fmaf(total, S[x], __uint_as_float(v[x]));
+            for (int x = 0; x < 32; ++x) S[x] = fmaf(total, S[x], v[x]);
         } else {
 #pragma unroll 1
             for (int t = 0; t < n; ++t) {
@@ -240,10 +238,10 @@ retention_join_kernel(const Retention p) {
 
 // A block takes chunks in turn.  The next chunk's q, k and angles are fetched into room that this one's products have left (the state's terms, the last of
 // k's) while its weights are made and P v runs; the state comes into registers meanwhile.  Bound by the steps of a chunk, 16 us, one after another: the
-// products take 8,000 cycles of 30,000, instructions issue in 30 %; a warp is held by the products that it issues, so warp 0 cuts no part of the state (all sixteen: 232 us).
-// Measured, 8,192 tokens of 32 heads: 224 us; q and angles row by row from memory and outputs and gates a row a
+// products take 8,000 cycles of 30,000, instructions issue in 30 %; a warp is held by the products that it issues, so warp 0 cuts no part of the state (all sixteen: 232 us, 224 without it).
+// Measured, 8,192 tokens of 32 heads: 214 us.  While products had one part (224): q and angles row by row from memory and outputs and gates a row a
 // thread 292, the latter alone 240; a warp group per operand, which leaves 64 to 112 registers a thread and spills, 253 to 288; a warp that only issues products, 112 registers, 274.
-//   columns of tensor memory: q's terms, then P's 0-191; scores, then P v 192-319; what the state gives 320-447
+//   columns of tensor memory: q's terms, then P's 0-191; a product's two parts 192-447: the scores, what the state gives, P v in turn
 __global__ void __launch_bounds__(kThreads, 1)
 retention_outputs_kernel(const Retention p) {
     extern __shared__ uint8_t smem_raw[];
@@ -258,7 +256,7 @@ retention_outputs_kernel(const Retention p) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp >> 2, row = (warp & 3) * 32 + lane, col = part * 32, quad = lane & 15;
     if (threadIdx.x == 0) fa::mbar_init(smem_u32(&scores_done), 1);
     const uint32_t tmem = (uint32_t)fa::uniform((int)begin(sh));
-    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16), scores = 192, old = 320;
+    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16), one = 192, two = 320;
     const bool issuer = fa::uniform(warp) == 0;
     uint32_t round = 0;
     int last_h = -1;
@@ -360,7 +358,7 @@ retention_outputs_kernel(const Retention p) {
         if (issuer) {
             fence_after();
             if (fa::elect_one()) {
-                product_ts<false, 3>(tmem + scores, tmem, keys, kHalf, kTerm, instr(kT, false, false));
+                product_ts<false, 3>(tmem + one, tmem + two, tmem, keys, kHalf, kTerm, instr(kT, false, false));
                 fa::umma_commit(smem_u32(&scores_done));
             }
             __syncwarp();
@@ -385,34 +383,35 @@ retention_outputs_kernel(const Retention p) {
                 }
             }
         }
+        // the scores give way to what the state gives (a wait that ran out shows in the next one)
+        ok = warp_wait(sh, scores_done, j);
+        fence_after();
+        float v[32];
+#pragma unroll
+        for (int x = 0; x < 32; x += 16)
+            if (col + x <= (row | 31)) ld_sum16(mine + one + col + x, mine + two + col + x, v + x);
         walk::cp_wait<0>();
         fence_smem();
+        fence_before();
         __syncthreads();
         if (issuer) {
+            fence_after();
             if (fa::elect_one()) {
-                product_ts<false, 3>(tmem + old, tmem, state, kHalf, kTerm, instr(kD, false, false));
+                product_ts<false, 3>(tmem + one, tmem + two, tmem, state, kHalf, kTerm, instr(kD, false, false));
                 fa::umma_commit(smem_u32(&sh.done));
             }
             __syncwarp();
         }
         if (threadIdx.x == 32) find(items[(j & 1) ^ 1]);
         __syncwarp();
-        // the scores, warp by warp: the others need not wait for the one that issues (a wait that ran out shows in the next one)
-        ok = warp_wait(sh, scores_done, j);
-        fence_after();
         {
             uint32_t w[3][8];
             auto weights = [&](int half) {
-                uint32_t v[16];
-                if (col + 16 * half <= (row | 31)) {
-                    ld16(mine + scores + col + 16 * half, v);
-                    wait_ld();
-                }
 #pragma unroll
                 for (int x = 0; x < 16; x += 2) {    // (the table's index is one of its own also where it is not used)
                     const int s = col + 16 * half + x;
                     const float fa_ = power[(row - s) & 127], fb = power[(row - s - 1) & 127];
-                    const float a = s <= row ? __uint_as_float(v[x]) * fa_ : 0.f, b = s < row ? __uint_as_float(v[x + 1]) * fb : 0.f;
+                    const float a = s <= row ? v[16 * half + x] * fa_ : 0.f, b = s < row ? v[16 * half + x + 1] * fb : 0.f;
                     uint32_t c[3];
                     cut(a, b, c);
 #pragma unroll
@@ -428,13 +427,21 @@ retention_outputs_kernel(const Retention p) {
                 for (int y = 0; y < 3; ++y) st8(mine + y * 64 + part * 16 + 8 * half, w[y]);
             }
         }
+        float o[32];
+        const float f = power[row + 1];
+#pragma unroll
+        for (int y = 0; y < 32; y += 16) {           // what the state gives, before P v takes its place
+            ld_sum16(mine + one + col + y, mine + two + col + y, o + y);
+#pragma unroll
+            for (int x = 0; x < 16; ++x) o[y + x] *= f;
+        }
         wait_st();
         fence_before();
         __syncthreads();
         if (issuer) {
             fence_after();
             if (fa::elect_one()) {
-                product_ts<true, 1>(tmem + scores, tmem, values, kHalf, kTerm, instr(kD, false, true));
+                product_ts<true, 1>(tmem + one, tmem + two, tmem, values, kHalf, kTerm, instr(kD, false, true));
                 fa::umma_commit(smem_u32(&sh.done));
             }
             __syncwarp();
@@ -448,26 +455,15 @@ retention_outputs_kernel(const Retention p) {
                 const int r = 32 * i + 2 * warp + (lane >> 4);
                 gates[i] = *reinterpret_cast<const uint4*>(p.proj + (size_t)(first + min(r, n - 1)) * p.pitch + p.g_off + (size_t)h * kD + 8 * quad);
             }
-        float o[32];
-        const float f = power[row + 1];
-#pragma unroll
-        for (int y = 0; y < 32; y += 16) {
-            uint32_t v[16];
-            ld16(mine + old + col + y, v);
-            wait_ld();
-#pragma unroll
-            for (int x = 0; x < 16; ++x) o[y + x] = f * __uint_as_float(v[x]);
-        }
         if (!(ok = products_done(sh, round++, p.error))) break;
         float z = 0.f, sum = 0.f;
 #pragma unroll
         for (int y = 0; y < 32; y += 16) {
-            uint32_t v[16];
-            ld16(mine + scores + col + y, v);
-            wait_ld();
+            float own[16];
+            ld_sum16(mine + one + col + y, mine + two + col + y, own);
 #pragma unroll
             for (int x = 0; x < 16; ++x) {
-                o[y + x] += __uint_as_float(v[x]);
+                o[y + x] += own[x];
                 z = fmaf(o[y + x], 0.f, z);
                 sum = fmaf(o[y + x], o[y + x], sum);
             }

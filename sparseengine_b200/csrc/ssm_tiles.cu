@@ -136,7 +136,7 @@ ssm_states_kernel(const StateSpace p) {
             if (issuer) {
                 fence_after();
                 if (fa::elect_one()) {
-                    product<true, true, 3>(tmem + (i & 1) * 2 * kV, keys, kHalf, kTerm, values, kUTerm, 2 * kUTerm, instr(2 * i + 1 < heads ? 2 * kV : kV, true, true));
+                    product<true, true, 3>(tmem + (i & 1) * 4 * kV, tmem + (i & 1) * 4 * kV + 2 * kV, keys, kHalf, kTerm, values, kUTerm, 2 * kUTerm, instr(2 * i + 1 < heads ? 2 * kV : kV, true, true));
                     fa::umma_commit(smem_u32(&sh.done));
                 }
                 __syncwarp();
@@ -148,15 +148,10 @@ ssm_states_kernel(const StateSpace p) {
         for (int j = 0; j < 2; ++j) {
             const int own = 2 * (i - 1) + j, h = h0 + own;
             if (own >= heads) break;
-            uint32_t w[16];
-            ld16(mine + ((i - 1) & 1) * 2 * kV + j * kV, w);
-            wait_ld();
             float sum[16], z = 0.f;
+            ld_sum16(mine + ((i - 1) & 1) * 4 * kV + j * kV, mine + ((i - 1) & 1) * 4 * kV + 2 * kV + j * kV, sum);
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                sum[c] = __uint_as_float(w[c]);
-                z = fmaf(sum[c], 0.f, z);
-            }
+            for (int c = 0; c < 16; ++c) z = fmaf(sum[c], 0.f, z);
             if (__any_sync(0xffffffffu, z != 0.f)) {
 #pragma unroll
                 for (int c = 0; c < 16; ++c) sum[c] = 0.f;
@@ -207,9 +202,10 @@ ssm_scan_kernel(const StateSpace p) {
 
 // Bound by a head's steps one after another (some 14,000 cycles, of which its products take 3,800 and shared memory gives them 128 bytes a cycle).  Each warp's weights are eight
 // columns of every 32, so that all share the exponents of the diagonal (32 columns a warp, and one warp of four with all of them: 87 us, 77 so); two warps issue, because
-// a warp is held by the products it issues (one for both 116, two 87); outputs leave through shared memory (a row a thread 77, 63 so).
-// Columns of tensor memory: C B^T 0-127, P's terms 128-319, what the state gives 320-447 (two heads in turn), P u 448-511.  While a head's P u is summed the next
-// head's state is cut and its product with C queued behind.
+// a warp is held by the products it issues (one for both 116, two 87); outputs leave through shared memory (a row a thread 77, 63 so; 67 with
+// products in two parts).
+// Columns of tensor memory: C B^T 0-127, P's terms 128-319, what the state gives in two parts 320-383 and 384-447, P u 384-447 and 448-511.  While a head's P u
+// is summed the next head's state is cut and the first part of its product with C queued behind, the second part once P u has been read.
 __global__ void __launch_bounds__(kThreads, 1)
 ssm_outputs_kernel(const StateSpace p) {
     extern __shared__ uint8_t smem_raw[];
@@ -233,7 +229,7 @@ ssm_outputs_kernel(const StateSpace p) {
     if (threadIdx.x == 0) fa::mbar_init(smem_u32(&state_done), 1);
     const uint32_t tmem = (uint32_t)fa::uniform((int)begin(sh));
     const int role = fa::uniform(warp);              // 0 issues P u, 1 what the state gives
-    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16), weights = 128, old = 320, sums = 448;
+    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16), weights = 128, old = 320, shared = 384, sums = 448;
     uint32_t round = 0;
     bool ok = true;
     float4 uv[4];
@@ -244,12 +240,16 @@ ssm_outputs_kernel(const StateSpace p) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) put4(state + (lane >> 4) * kSHalf, kSTerm, 16 * j + warp, lane & 15, sv[j]);
     };
-    auto issue_state = [&](int i) {
+    auto issue_state = [&](int half) {
         if (role == 1) {
             fence_after();
             if (fa::elect_one()) {
-                product<false, false, 3>(tmem + old + (i & 1) * kV, queries, kHalf, kTerm, state, kSHalf, kSTerm, instr(kV, false, false));
-                fa::umma_commit(smem_u32(&state_done));
+                if (half == 0)
+                    product_first<false, false, 3>(tmem + old, queries, kHalf, kTerm, state, kSHalf, kSTerm, instr(kV, false, false));
+                else {
+                    product_second<false, false>(tmem + shared, queries, kHalf, state, kSHalf, instr(kV, false, false));
+                    fa::umma_commit(smem_u32(&state_done));
+                }
             }
             __syncwarp();
         }
@@ -261,7 +261,7 @@ ssm_outputs_kernel(const StateSpace p) {
     __syncthreads();
     if (role == 0) {
         if (fa::elect_one()) {
-            product<false, false, 3>(tmem, queries, kHalf, kTerm, keys, kHalf, kTerm, instr(kT, false, false));
+            product<false, false, 3>(tmem, tmem + weights, queries, kHalf, kTerm, keys, kHalf, kTerm, instr(kT, false, false));
             fa::umma_commit(smem_u32(&sh.done));
         }
         __syncwarp();
@@ -270,10 +270,23 @@ ssm_outputs_kernel(const StateSpace p) {
     ok = products_done(sh, round++, p.error);        // B's terms give way to the first head's state and values
     grid_dependency_wait();                          // the states at the chunks' starts
     if (ok) {
+        if (part <= (warp & 3)) {                    // both parts of C B^T together, where tokens see others (a warp's 32 columns)
+#pragma unroll
+            for (int x = 0; x < 32; x += 16) {
+                float v[16];
+                ld_sum16(mine + 32 * part + x, mine + weights + 32 * part + x, v);
+                st8(mine + 32 * part + x, reinterpret_cast<uint32_t*>(v));
+                st8(mine + 32 * part + x + 8, reinterpret_cast<uint32_t*>(v + 8));
+            }
+            wait_st();
+        }
         put_state(0);
         fence_smem();
+        fence_before();
         __syncthreads();
+        fence_after();
         issue_state(0);
+        issue_state(1);
     }
     for (int i = 0; i < heads && ok; ++i) {
         const int h = h0 + i;
@@ -312,11 +325,15 @@ ssm_outputs_kernel(const StateSpace p) {
 #pragma unroll
             for (int y = 0; y < 3; ++y) st4(mine + weights + y * 64 + 16 * x + 4 * part, w[y]);
         }
+        // the state's product is there: its terms may give way, its columns to P u
+        ok = warp_wait(sh, state_done, i);
+        fence_after();
+        float u[16];
+        ld_sum16(mine + old + vcol, mine + shared + vcol, u);
         wait_st();
         fence_smem();
         fence_before();
-        // the state's product is there: its terms may give way
-        ok = __syncthreads_and(warp_wait(sh, state_done, i));
+        ok = __syncthreads_and(ok);
         if (!ok) {
             if (threadIdx.x == 0) atomicCAS(p.error, 0, kErrorCode);
             break;
@@ -324,7 +341,7 @@ ssm_outputs_kernel(const StateSpace p) {
         fence_after();
         if (role == 0) {
             if (fa::elect_one()) {
-                product_ts<true, 3>(tmem + sums, tmem + weights, values, 0, kUTerm, instr(kV, false, true));
+                product_ts<true, 3>(tmem + shared, tmem + sums, tmem + weights, values, 0, kUTerm, instr(kV, false, true));
                 fa::umma_commit(smem_u32(&sh.done));
             }
             __syncwarp();
@@ -333,28 +350,27 @@ ssm_outputs_kernel(const StateSpace p) {
             put_state(i + 1);
             fence_smem();
             __syncthreads();
-            issue_state(i + 1);
+            issue_state(0);
             fetch_rows(uv, x + (size_t)(h + 1) * kV, width, n);
         }
         const float skip = p.d_skip[h];
         float4 own[4];                               // the values as they are
         fetch_rows(own, x + (size_t)h * kV, width, n);
-        uint32_t u[16], o[16];
-        ld16(mine + old + (i & 1) * kV + vcol, u);
-        wait_ld();
         if (!(ok = products_done(sh, round++, p.error))) break;
-        ld16(mine + sums + vcol, o);
-        wait_ld();
+        float o[16];
+        ld_sum16(mine + shared + vcol, mine + sums + vcol, o);
         fence_before();
         const float lead = expf(tab.hi[i][row] + tab.lo[i][row]);
         float z = 0.f, y[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            y[j] = fmaf(lead, __uint_as_float(u[j]), __uint_as_float(o[j]));
+            y[j] = fmaf(lead, u[j], o[j]);
             z = fmaf(y[j], 0.f, z);
         }
         float* to = p.y + ((size_t)first * p.H + h) * kV;
-        if (!__syncthreads_or(z != 0.f && row < n)) {
+        const bool finite = !__syncthreads_or(z != 0.f && row < n);
+        if (i + 1 < heads) issue_state(1);
+        if (finite) {
             // through shared memory (the values have been read), so that neighbouring threads store neighbours
             uint8_t* rows = smem_raw + (values - smem_u32(smem_raw));
 #pragma unroll

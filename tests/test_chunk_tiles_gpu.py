@@ -21,7 +21,8 @@ def _step(lens):
                            max_q_len=max(lens), cu=cu, rows=rows)
 
 
-def _retention(lens, heads, rotary, decay, bad=None, out=False, known=None):
+def _retention(lens, heads, rotary, decay, bad=None, out=False, known=None, positive=False, walk=False):
+    """``walk``: by the chunks of 64 tokens one after another (csrc/retention.cu) instead."""
     from sparseengine_b200.csrc import ops
     d, step = 128, _step(lens)
     step.max_q_len = known or step.max_q_len
@@ -31,13 +32,20 @@ def _retention(lens, heads, rotary, decay, bad=None, out=False, known=None):
     decays = torch.exp(-torch.rand(heads, generator=g, device=DEV) * (20.0 if decay == "fast" else 0.03))
     state = torch.randn(len(lens) + 2, heads * d * d + 4, generator=g, device=DEV)
     inv, positions = torch.rand(64, generator=g, device=DEV), torch.arange(T, device=DEV, dtype=torch.int32) * 37 % 101
+    if positive:
+        proj, state = proj.abs(), state.abs()
     if bad is not None:
         proj[bad[0], {"q": q_off, "k": k_off, "v": v_off}[bad[1]] + 5] = bad[2]
     first = state.clone()
     assert ops.retention_tiles_supported(d, d, rotary, proj, state, q_off, k_off, v_off, g_off)
     to = dict(out=torch.empty(T, heads * d, dtype=torch.bfloat16, device=DEV)) if out else dict(o=torch.full((T, heads * d), float("nan"), device=DEV))
-    got = ops.retention_tiles(proj, q_off, k_off, v_off, g_off, d ** -0.5, (inv, rotary, positions) if rotary else None, decays, state, step,
-                              heads=heads, head_dim=d, v_head_dim=d, eps=1e-6, **to)
+    rotation = (inv, rotary, positions) if rotary else None
+    if walk:
+        got = ops.retention_chunk(None, None, proj, v_off, decays, state, step, to["o"], heads=heads, head_dim=d, v_head_dim=d,
+                                  qk=(q_off, k_off, d ** -0.5), rotation=rotation)
+    else:
+        got = ops.retention_tiles(proj, q_off, k_off, v_off, g_off, d ** -0.5, rotation, decays, state, step, heads=heads, head_dim=d, v_head_dim=d,
+                                  eps=1e-6, **to)
     ops.error_check(DEV)
     q, k, v = (proj[:, f:f + heads * d].double().view(T, heads, d) for f in (q_off, k_off, v_off))
     if rotary:
@@ -62,6 +70,28 @@ def test_retention_against_the_walk(lens, heads, rotary, decay):
         _close(state[row, :heads * d * d].view(heads, d, d), S, f"state after {n} tokens")
     others = [r for r in range(len(lens) + 2) if r not in step.rows]
     assert torch.equal(state[others], first[others]) and torch.equal(state[:, heads * d * d:], first[:, heads * d * d:])
+
+
+def _norm_error(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+# Values of one sign: a step of tensor memory cuts off up to a unit of the 24th bit of the sum so far, always towards zero: half on average, of sums that are
+# half of the last one on average.  Four steps in either part of a product, two products behind one another: 8 x 2^-26, and what 32-bit rounding leaves.
+ONE_SIGN = 1.5e-7
+
+
+@pytest.mark.parametrize("positive", [False, True])
+@pytest.mark.parametrize("rotary", [0, 128])
+@pytest.mark.parametrize("n", [128, 700])
+def test_retention_is_as_exact_as_the_walk(n, rotary, positive):
+    errors = []
+    for walk in (False, True):
+        _, o, first, state, inputs, _ = _retention([n], 4, rotary, "slow", positive=positive, walk=walk)
+        want, S = _walk64(*inputs, first[0, :4 * 128 * 128].double().view(4, 128, 128))
+        errors.append((_norm_error(o.view(n, 4, 128), want), _norm_error(state[0, :4 * 128 * 128].view(4, 128, 128), S)))
+    for here, walked in zip(*errors):
+        assert here <= (max(walked, ONE_SIGN) if positive else walked), errors
 
 
 @pytest.mark.parametrize("lens,known", [([1500, 40], 300), ([900], 60)])
@@ -114,7 +144,7 @@ def test_retention_mixer_keeps_to_the_other_forms_beyond_its_workspace():
     assert part.in_tiles(few, 20 + 63, 0, DEV) and not part.in_tiles(many, 20 + 511, 0, DEV)
 
 
-def _state_space(lens, heads, groups, decay, bad=None):
+def _state_space(lens, heads, groups, decay, bad=None, positive=False, walk=False):
     from sparseengine_b200.csrc import ops
     P, N, step = 64, 128, _step(lens)
     T, g = step.num_tokens, torch.Generator(device=DEV).manual_seed(heads)
@@ -123,6 +153,8 @@ def _state_space(lens, heads, groups, decay, bad=None):
     bias, skip = torch.randn(heads, generator=g, device=DEV) - 2.0, torch.randn(heads, generator=g, device=DEV)
     a_log = torch.log(torch.rand(heads, generator=g, device=DEV) * (30 if decay == "fast" else 1) + 0.1)
     state = torch.randn(len(lens) + 2, heads * P * N + 4, generator=g, device=DEV)
+    if positive:
+        xbc, skip, state = xbc.abs(), skip.abs(), state.abs()
     if bad is not None:
         t, where, value = bad
         if where == "dt":
@@ -131,7 +163,7 @@ def _state_space(lens, heads, groups, decay, bad=None):
             xbc[t, {"v": 5, "k": heads * P + 5, "q": heads * P + groups * N + 5}[where]] = value
     first, y = state.clone(), torch.full((T, heads * P), float("nan"), device=DEV)
     assert ops.ssm_tiles_supported(N, P, proj, state)
-    ops.ssm_tiles(xbc, proj, 3, bias, a_log, skip, state, step, y, heads=heads, head_dim=P, state_size=N, groups=groups)
+    (ops.ssm_walk if walk else ops.ssm_tiles)(xbc, proj, 3, bias, a_log, skip, state, step, y, heads=heads, head_dim=P, state_size=N, groups=groups)
     ops.error_check(DEV)
     dt = torch.nn.functional.softplus(proj[:, 3:3 + heads].double() + bias.double())
     x, rep = xbc[:, :heads * P].double().view(T, heads, P), heads // groups
@@ -158,6 +190,19 @@ def test_state_space_against_the_walk(lens, heads, groups, decay):
         _close(state[row, :heads * P * N].view(heads, P, N).transpose(1, 2), S, f"state after {n} tokens")
     others = [r for r in range(len(lens) + 2) if r not in step.rows]
     assert torch.equal(state[others], first[others]) and torch.equal(state[:, heads * P * N:], first[:, heads * P * N:])
+
+
+@pytest.mark.parametrize("positive", [False, True])
+@pytest.mark.parametrize("decay", ["slow", "fast"])
+@pytest.mark.parametrize("n", [128, 700])
+def test_state_space_is_as_exact_as_the_walk(n, decay, positive):
+    errors = []
+    for walk in (False, True):
+        _, y, first, state, inputs, add = _state_space([n], 4, 2, decay, positive=positive, walk=walk)
+        want, S = _walk64(*inputs, first[0, :4 * 64 * 128].double().view(4, 64, 128).transpose(1, 2))
+        errors.append((_norm_error(y.view(n, 4, 64), want + add), _norm_error(state[0, :4 * 64 * 128].view(4, 64, 128).transpose(1, 2), S)))
+    for here, walked in zip(*errors):
+        assert here <= (max(walked, ONE_SIGN) if positive else walked), errors
 
 
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
