@@ -9,7 +9,7 @@
 // With eight warps on an SM it is the warps' own instructions, one behind the other, that bound it before the memory does: so a
 // tile's rows are looked up once, ahead, the copies and ldmatrix reads step by constants, and the output is rescaled only where a
 // maximum moved.  Measured, 64 requests of 1,500 to 3,000 keys, 48 heads over 8 of 128 (590 MB, 89 us at 6.65 TB/s): rows looked
-// up by every thread 181 us, ahead 154, with the rest 125, with the longest requests' blocks first 118.
+// up by every thread 181 us, ahead 154, with the rest 125.
 //
 // Arithmetic as in the plain kernel and the reference's split-KV decode
 // (src/sparseengine/kernels/triton/gqa_flash_decoding_stage1.py:69-120,
@@ -36,31 +36,10 @@ constexpr int kTileKeys = 64;
 constexpr int kStages = 3;       // row_at holds kStages + 1 tiles
 constexpr int kWarps = 4;
 constexpr int kThreads = 32 * kWarps;
-constexpr int kSorted = 256;     // the most query tokens that are taken in the order of their keys
 
 using namespace se::mma;
 
-// The query token with the `place`-th most visible keys (the earlier one of equals first), by the whole block.  Where there are more blocks than run at once, the
-// last ones to start set the end: 64 requests of 1,500 to 3,000 keys over 8 KV heads, two blocks an SM, are done after 92 tiles' time in the requests' order and
-// after 74 with the longest first (67 if all blocks ended together).
-__device__ __forceinline__ int longest_first(const int* positions, int tokens, int place, int window, int keep_first) {
-    __shared__ int seen[kSorted], found;
-    for (int t = threadIdx.x; t < tokens; t += kThreads) {
-        const int pos = positions[t], lo = first_visible(pos, window);
-        seen[t] = min(keep_first, lo) + pos + 1 - lo;
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < tokens; t += kThreads) {
-        const int own = seen[t];
-        int before = 0;
-        for (int u = 0; u < tokens; ++u) before += seen[u] > own || (seen[u] == own && u < t);
-        if (before == place) found = t;
-    }
-    __syncthreads();
-    return found;
-}
-
-template <int D, int DV, bool PAD, bool SORTED>
+template <int D, int DV, bool PAD>
 __global__ void __launch_bounds__(kThreads)
 attn_decode_kernel(const __nv_bfloat16* q, const __nv_bfloat16* cache,      // written by the kernel before this one: no __restrict__ (see the wait below)
                    const int* __restrict__ table, int table_stride, const int* __restrict__ seq_rows,
@@ -74,12 +53,10 @@ attn_decode_kernel(const __nv_bfloat16* q, const __nv_bfloat16* cache,      // w
     constexpr int kStageBytes = kTileKeys * (D + DV) * 2;    // a K tile and a V tile
     extern __shared__ __align__(128) uint8_t smem[];
 
-    // SORTED: all of a token's blocks follow one another, the longest token's first
-    const int t = SORTED ? longest_first(positions, gridDim.x, (blockIdx.x + gridDim.x * blockIdx.y) / gridDim.y, window, opt.keep_first) : (int)blockIdx.x;
-    const unsigned y = SORTED ? (blockIdx.x + gridDim.x * blockIdx.y) % gridDim.y : blockIdx.y;
+    const int t = blockIdx.x;
     const int group = hq / hkv;
     const int gtiles = (group + 15) / 16;
-    const int kvh = y / gtiles, gt = y % gtiles;
+    const int kvh = blockIdx.y / gtiles, gt = blockIdx.y % gtiles;
     const int split = blockIdx.z;
     const int rows_valid = min(16, group - gt * 16);
     const int head0 = kvh * group + gt * 16;
@@ -382,7 +359,7 @@ template <int D, int DV, bool PAD>
 static int launch(const void* q, const void* cache, const int* table, int table_stride, const int* seq_rows,
                   const int* token_seq, const int* positions, void* out, float* part_o, float* part_ml, int tokens,
                   int hq, int hkv, int page_size, float scale, int window, int splits, int keys_per_split,
-                  int num_pages, int* error, int settled, int sorted, const SoftmaxOptions& opt, int d, int dv, cudaStream_t stream) {
+                  int num_pages, int* error, int settled, const SoftmaxOptions& opt, int d, int dv, cudaStream_t stream) {
     const int group = hq / hkv;
     const int gtiles = (group + 15) / 16;
     const size_t stage_smem = (size_t)kStages * kTileKeys * (D + DV) * 2;
@@ -390,15 +367,13 @@ static int launch(const void* q, const void* cache, const int* table, int table_
     const size_t smem = stage_smem > merge_smem ? stage_smem : merge_smem;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D, DV, PAD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_decode_kernel<D, DV, PAD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D, DV, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
     dim3 grid(tokens, hkv * gtiles, splits);
-    const auto kernel = sorted && splits == 1 && tokens <= kSorted ? attn_decode_kernel<D, DV, PAD, true> : attn_decode_kernel<D, DV, PAD, false>;
     cudaError_t e = SE_LAUNCH_DEPENDENT_IF(
-        settled != 0, "attn", kernel, grid, dim3(kThreads), smem, stream, (const __nv_bfloat16*)q,
+        settled != 0, "attn", attn_decode_kernel<D, DV, PAD>, grid, dim3(kThreads), smem, stream, (const __nv_bfloat16*)q,
         (const __nv_bfloat16*)cache, table, table_stride, seq_rows, token_seq, positions, (__nv_bfloat16*)out, part_o,
         part_ml, hq, hkv, page_size, scale * 1.4426950408889634f, window, splits, keys_per_split, num_pages, error, opt, d, dv);
     if (e == cudaSuccess) e = cudaGetLastError();
@@ -427,14 +402,13 @@ extern "C" int se_attn_decode_value_dim_supported(int v_head_dim) {
 // launched just before this one began (they are inputs of the step, and that kernel is the one
 // that writes the queries and the step's keys).  The attention kernel is then launched as that
 // kernel's dependent and reads them while it may still run; else it is launched the ordinary way.
-// sorted: CTAs start in the order of their tokens' keys, the longest first (one split and at most 256 tokens; else as they come).
 // softcap (0: none), sink, gate (nullptr: none) and gate_pitch: the softmax's options, as the plain kernel's.
 extern "C" int se_attn_decode(const void* q, const void* cache, const int* table, int table_stride,
                               const int* seq_rows, const int* token_seq, const int* positions, void* out,
                               float* part_o, float* part_ml, int tokens, int hq, int hkv, int head_dim, int v_head_dim,
                               int page_size, float scale, int window, int splits, int keys_per_split, int num_pages,
                               int* error, int settled, float softcap, int sink, const void* gate, int gate_pitch,
-                              const float* sink_logits, int keep_first, const float* slopes, int gate_per_head, int sorted,
+                              const float* sink_logits, int keep_first, const float* slopes, int gate_per_head,
                               cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (!se_attn_decode_supported(head_dim, hq, hkv) || !se_attn_decode_value_dim_supported(v_head_dim) || splits < 1 ||
@@ -452,7 +426,7 @@ extern "C" int se_attn_decode(const void* q, const void* cache, const int* table
 #define SE_DECODE_LAUNCH(DQ, DVAL, PAD)                                                                                 \
     return se::dec::launch<DQ, DVAL, PAD>(q, cache, table, table_stride, seq_rows, token_seq, positions, out, part_o,   \
                                           part_ml, tokens, hq, hkv, page_size, scale, window, splits, keys_per_split,   \
-                                          num_pages, error, settled, sorted, opt, head_dim, v_head_dim, stream)
+                                          num_pages, error, settled, opt, head_dim, v_head_dim, stream)
 #define SE_DECODE_CASE(DQ, DVAL)                                                                                        \
     if (dt == DQ && dvt == DVAL) {                                                                                      \
         if (pad) SE_DECODE_LAUNCH(DQ, DVAL, true);                                                                      \

@@ -1502,13 +1502,6 @@ def attn_decode_plan(tokens: int, num_heads: int, num_kv_heads: int, max_keys: i
     return splits, per_tiles * 64
 
 
-def attn_decode_sorted(tokens: int, num_heads: int, num_kv_heads: int, max_keys: int, splits: int, sms: int) -> bool:
-    """Whether the CTAs of a decode step start with the longest contexts: where there are more than run at once, and keys enough to pay for the
-    sorting that each does for itself (64 requests, a layer's call in us, as they come / sorted: up to 1,000 keys 84/84, 2,000 119/115, 3,000
-    155/148)."""
-    return splits == 1 and tokens <= 256 and max_keys >= 1500 and tokens * num_kv_heads * -(-num_heads // num_kv_heads // 16) > 2 * sms
-
-
 def _softmax_options(q, gate, num_heads, v_head_dim, softcap, sink, keep_first, slopes):
     """The tail of the tensor-core attention kernels' arguments: cap, sink, gate pointer, gate pitch, the learned
     sink's logits, the count of first keys that stay visible, the distance bias's slopes, and whether the gate has one
@@ -1540,14 +1533,14 @@ def attn_decode(q, cache, table, seq_rows, token_seq, positions, out, *, num_hea
     if splits > 1:
         part_o = torch.empty(tokens * num_heads * splits * dv, dtype=torch.float32, device=q.device)
         part_ml = torch.empty(tokens * num_heads * splits * 2, dtype=torch.float32, device=q.device)
-    _check(_fn("se_attn_decode", "pppipppppp" "iiiiii" "f" "iii" "ip" "i" "fipi" "pipi" "ip")(
+    _check(_fn("se_attn_decode", "pppipppppp" "iiiiii" "f" "iii" "ip" "i" "fipi" "pipi" "p")(
         _ptr(q, torch.bfloat16, "q"), _ptr(cache, torch.bfloat16, "cache"), _ptr(table, torch.int32, "table"),
         table.shape[1], _ptr(seq_rows, torch.int32, "seq_rows"), _ptr(token_seq, torch.int32, "token_seq"),
         _ptr(positions, torch.int32, "positions"), _ptr(out, torch.bfloat16, "out"), _ptr(part_o), _ptr(part_ml),
         tokens, num_heads, num_kv_heads, head_dim, dv, page_size, float(scale), _visible_arg(window, chunk), splits, per,
         cache.shape[0] if num_pages is None else int(num_pages), _ptr(error_word(q.device)),
         int(bool(step_inputs_settled)), *_softmax_options(q, gate, num_heads, dv, softcap, sink, keep_first or 0, slopes),
-        int(attn_decode_sorted(tokens, num_heads, num_kv_heads, max_keys, splits, sm_count(q.device))), _stream()), "attn_decode")
+        _stream()), "attn_decode")
     return out
 
 
