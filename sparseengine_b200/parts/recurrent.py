@@ -326,13 +326,19 @@ class RetentionMixer(Mixer):
         return once_per_step(step, ("retention.in_walk", s.num_heads, s.v_head_dim), ask)
 
     def in_tiles(self, step, tokens: int, rotary_dim: int, device) -> bool:
-        """Whether a step in chunks that csrc/retention_tiles.cu takes (bfloat16, heads of 128 x 128) goes there: it is ahead or level from 17 tokens
-        on, beside whatever single tokens (a layer's call, us before / now, 16 and 32 heads: one portion of 17 tokens 103/87 and 75/74, of 128
-        101/86 and 79/80, of 512 80/67 and 132/113, of 8,192 774/400 and 1,534/1,207; 90 tokens beside 63 single ones 444/221 and
-        878/407; 64 entries of 96 719/440 and 1,754/1,172), as long as its workspace, 64 KB per head and entry or 128 tokens, is no
-        larger than that of the other forms or 256 MB."""
-        heads = self.spec.num_heads
-        return ops.retention_tiles_plan(step, tokens, heads, rotary_dim, device)[2] <= max(1 << 26, tokens * heads * 322)
+        """Whether a step in chunks that csrc/retention_tiles.cu takes (bfloat16, heads of 128 x 128) goes there.  Not where all of the walk's
+        blocks run at once and its longest chain is four chunks: each of the two kernels takes some 15 us for a chunk, the walk and its preparation
+        7 to 14 and 4 more a chunk.  Measured, device us of a layer without its projections, the other forms / here: 4, 8, 16 and 32 heads, one
+        portion of 17 tokens 25/45, 25/41, 27/43, 33/45, of 128 30/41, 31/41, 33/43, 41/45, of 200 35/39, 37/41, 39/43, 48/48, of
+        257 39/42, 41/40, 44/45, 56/51, of 1,024 72/41, 76/46, 84/50, 123/80; 17 tokens beside 15 single ones 43/46, 71/45, 117/78, 213/125, 90 beside 63
+        86/76, 226/122, 425/221, 823/400; two entries of 40 27/41, 27/41, 33/43, 52/45, sixty-four of 96 156/98, 296/171, 574/301, 1,115/569.
+        (A whole layer's call of 128 tokens and 16 heads, waited for: 89/100; calls one behind the other, where the host is what takes the time, 77/70.)
+        And as long as its workspace, 64 KB per head and entry or 128 tokens, is no larger than that of the other forms or 256 MB."""
+        s = self.spec
+        if step.max_q_len <= 256 and step.num_seqs * s.num_heads * -(-s.v_head_dim // 32) <= ops.sm_count(device):
+            return False
+        return once_per_step(step, ("retention.in_tiles", s.num_heads, rotary_dim), lambda: (
+            ops.retention_tiles_plan(step, tokens, s.num_heads, rotary_dim, device)[2] <= max(1 << 26, tokens * s.num_heads * 322)))
 
     def forward(self, x, step, slot, proj=None):
         s = self.spec
@@ -352,8 +358,8 @@ class RetentionMixer(Mixer):
         # a step with a prompt portion takes the recurrence in chunks of 64 tokens (closed form per chunk);
         # steps of single tokens and of short pieces walk it token by token
         chunked = self.chunk_min_tokens is not None and step.max_q_len >= self.chunk_min_tokens
-        if (chunked and not silu and ops.retention_tiles_supported(s.head_dim, s.v_head_dim, rotary_dim, proj, slot.state, self.qk, self.vv)
-                and self.in_tiles(step, tokens, rotary_dim, dev)):
+        if (chunked and not silu and self.in_tiles(step, tokens, rotary_dim, dev)
+                and ops.retention_tiles_supported(s.head_dim, s.v_head_dim, rotary_dim, proj, slot.state, self.qk, self.vv)):
             out = torch.empty(tokens, self.vv, dtype=x.dtype, device=dev)
             normed = s.output_norm == "per_head"
             ops.retention_tiles(proj, 0, self.qk, 2 * self.qk, 2 * self.qk + self.vv, self.k_scale,

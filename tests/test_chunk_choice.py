@@ -58,3 +58,18 @@ def test_retention_walk_by_the_entries_own_tokens(monkeypatch, lens, sixteen, th
     for heads, walk in ((16, sixteen), (32, thirty_two)):
         part = make_mixer(RetentionSpec(hidden_size=64, num_heads=heads, head_dim=128, v_head_dim=128, decays=(0.9,) * heads, position=None), torch.bfloat16)
         assert part.in_walk(step, "cuda:0") is walk
+
+
+@pytest.mark.parametrize("lens,heads,tiles", [
+    # device us of a layer without its projections, the walk / chunks side by side: 27/43, 33/43, 41/45, 41/46; 44/45, 56/51, 56/53, 52/45, 45/47, 117/78
+    ([17], 16, False), ([128], 16, False), ([128], 32, False), ([130] * 2, 16, False), ([256], 32, False), ([90] + [1] * 3, 8, False),
+    ([257], 16, True), ([257], 32, True), ([17], 64, True), ([40] * 2, 32, True), ([17] * 4, 16, True), ([17] + [1] * 15, 16, True), ([8192], 32, True)])
+def test_retention_tiles_where_the_walk_is_not_ahead(monkeypatch, lens, heads, tiles):
+    import torch
+
+    from sparseengine_b200.config.specs import RetentionSpec
+    from sparseengine_b200.parts.base import make_mixer
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    part = make_mixer(RetentionSpec(hidden_size=64, num_heads=heads, head_dim=128, v_head_dim=128, decays=(0.9,) * heads, position=None), torch.bfloat16)
+    step = SimpleNamespace(max_q_len=max(lens), num_tokens=sum(lens), num_seqs=len(lens), q_lens=lens)
+    assert part.in_tiles(step, sum(lens), 0, "cuda:0") is tiles
