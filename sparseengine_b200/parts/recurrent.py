@@ -354,7 +354,6 @@ class RetentionMixer(Mixer):
         if proj is None:
             proj = linear(x, self.in_proj)
         silu = s.activation == "silu"
-        o = torch.empty(tokens, self.vv, dtype=torch.float32, device=dev)
         # a step with a prompt portion takes the recurrence in chunks of 64 tokens (closed form per chunk);
         # steps of single tokens and of short pieces walk it token by token
         chunked = self.chunk_min_tokens is not None and step.max_q_len >= self.chunk_min_tokens
@@ -362,12 +361,14 @@ class RetentionMixer(Mixer):
                 and ops.retention_tiles_supported(s.head_dim, s.v_head_dim, rotary_dim, proj, slot.state, self.qk, self.vv)):
             out = torch.empty(tokens, self.vv, dtype=x.dtype, device=dev)
             normed = s.output_norm == "per_head"
+            o = None if normed else torch.empty(tokens, self.vv, dtype=torch.float32, device=dev)
             ops.retention_tiles(proj, 0, self.qk, 2 * self.qk, 2 * self.qk + self.vv, self.k_scale,
                                 (inv_freq, rotary_dim, step.positions) if rotary_dim else None, self._decay, slot.state, step, heads=s.num_heads,
                                 head_dim=s.head_dim, v_head_dim=s.v_head_dim, eps=s.norm_eps, **({"out": out} if normed else {"o": o}))
             if not normed:
                 ops.retention_out_joint(o, proj, 2 * self.qk + self.vv, self.norm_w, out, eps=s.norm_eps)
             return linear(out, self.o)
+        o = torch.empty(tokens, self.vv, dtype=torch.float32, device=dev)
         args = (proj, 2 * self.qk, self._decay, slot.state, step, o)
         sizes = dict(heads=s.num_heads, head_dim=s.head_dim, v_head_dim=s.v_head_dim, silu=silu)
         if not chunked and rotary_dim == 0:      # q and k straight from the projection, as they are staged

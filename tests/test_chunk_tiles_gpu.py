@@ -144,6 +144,40 @@ def test_retention_mixer_keeps_to_the_other_forms_beyond_its_workspace():
     assert part.in_tiles(few, 20 + 63, 0, DEV) and not part.in_tiles(many, 20 + 511, 0, DEV)
 
 
+@pytest.mark.parametrize("norm", ["per_head", "joint"])
+def test_retention_mixer_through_the_chunks(norm):
+    """Both output norms against the other forms; and beside what the step needs nothing as large as 32-bit outputs is held where the kernel norms them."""
+    from sparseengine_b200.config.specs import RetentionSpec
+    from sparseengine_b200.csrc import ops
+    from sparseengine_b200.parts.base import LayerSlot, make_mixer
+    heads, T, width = 4, 8192, 64
+    part = make_mixer(RetentionSpec(hidden_size=width, num_heads=heads, head_dim=128, v_head_dim=128, decays=(0.99,) * heads, position=None, output_norm=norm),
+                      torch.bfloat16)
+    g = torch.Generator(device=DEV).manual_seed(1)
+    part.bind({name: (torch.randn(*p.shape, generator=g, device=DEV) * 0.05).to(torch.bfloat16) for name, p in part.parameters().items()})
+    x, step, ys = torch.randn(T, width, generator=g, device=DEV).to(torch.bfloat16), _step([T]), []
+    step.positions = torch.arange(T, dtype=torch.int32, device=DEV)
+    for least in (16, None):                         # the chunks side by side; token by token
+        part.chunk_min_tokens = least
+        slot = LayerSlot(state=torch.zeros(3, heads * 128 * 128, device=DEV))
+        for _ in range(2):                           # the second call's memory: what the library keeps is there
+            slot.state.zero_()
+            before, calls = torch.cuda.memory_allocated(), ops.calls.get("se_retention_tiles", 0)
+            torch.cuda.reset_peak_memory_stats()
+            y = part.forward(x, step, slot)
+            held = torch.cuda.max_memory_allocated() - before
+        assert ops.calls.get("se_retention_tiles", 0) - calls == (least is not None)
+        if least is not None and norm == "per_head":
+            vv = heads * 128
+            needed = T * 4 * vv * 2 + T * vv * 2 + 4 * ops.retention_tiles_plan(step, T, heads, 0, DEV)[2] + T * width * 2
+            assert held < needed + T * vv * 2, (held, needed)        # columns, outputs after the norm, workspace, result; no 32-bit outputs
+        ys.append((y.double(), slot.state[0].double()))
+    ops.error_check(DEV)
+    # outputs after the norm are 16-bit in both, rounded at different values at times: 2^-8 of a value, in sums over 512 of either sign
+    assert float((ys[0][0] - ys[1][0]).norm() / ys[1][0].norm()) < 2.0 ** -8
+    assert float((ys[0][1] - ys[1][1]).norm() / ys[1][1].norm()) < 1e-6
+
+
 def _state_space(lens, heads, groups, decay, bad=None, positive=False, walk=False):
     from sparseengine_b200.csrc import ops
     P, N, step = 64, 128, _step(lens)
