@@ -851,15 +851,31 @@ def ssm_tiles_supported(state_size: int, head_dim: int, proj, state) -> bool:
     return state_size == 128 and head_dim == 64 and proj.dtype == torch.bfloat16 and state.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0
 
 
-def ssm_tiles(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, step, y, *, heads, head_dim, state_size, groups):
-    """The recurrence of :func:`ssm_walk` in chunks of 128 tokens side by side on tcgen05 (csrc/ssm_tiles.cu)."""
+def ssm_tiles_plan(chunks: int, heads: int, groups: int, sms: int) -> tuple:
+    """(estimated us, heads of a group that a block takes) of :func:`ssm_tiles` over ``chunks`` chunks of 128 tokens: 13 us a head and 10 for what a block's
+    heads share, times the rounds that its blocks take, a last one of few blocks counted half (measured, device us of a layer of 64 heads in 8 groups: 257 tokens, 192
+    blocks of one head 72, 96 of two 60; 4,096 tokens, 512 blocks of four 346, 256 of eight 310)."""
+    rep = heads // groups
+
+    def cost(per):
+        rounds = chunks * groups * -(-rep // per) / sms
+        return max(1.0, (rounds + -(-rounds // 1)) / 2) * (10 + 13 * per), -per
+    us, per = min(cost(per) for per in range(1, min(8, rep) + 1))
+    return us, -per
+
+
+def ssm_tiles(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, step, y, *, heads, head_dim, state_size, groups, heads_per_block=None):
+    """The recurrence of :func:`ssm_walk` in chunks of 128 tokens side by side on tcgen05 (csrc/ssm_tiles.cu).  ``heads_per_block``: of
+    :func:`ssm_tiles_plan`; the same results with any."""
     tokens, n = xbc.shape[0], step.num_seqs
-    work = _walk_work((tokens // 128 + n) * heads * (head_dim * state_size + 1), xbc.device)
+    places = tokens // 128 + n
+    per = heads_per_block or ssm_tiles_plan(places, heads, groups, sm_count(xbc.device))[1]
+    work = _walk_work(places * heads * (head_dim * state_size + 1), xbc.device)
     _check(_fn("se_ssm_tiles", "ppii" "ppp" "pl" "pp" "ppp" "iiiiiii" "p")(
         _ptr(xbc, torch.float32, "xbc"), _rows_ptr(proj, "proj", torch.bfloat16), proj.stride(0), int(dt_off),
         _ptr(dt_bias, torch.float32, "dt_bias"), _ptr(a_log, torch.float32, "a_log"), _ptr(d_skip, torch.float32, "d_skip"),
         _ptr(state, torch.float32, "state"), state.stride(0), _ptr(step.cu_q), _ptr(step.seq_rows), _ptr(y, torch.float32, "y"),
-        work.data_ptr(), _ptr(error_word(xbc.device)), tokens, n, heads, head_dim, state_size, groups, sm_count(xbc.device), _stream()), "ssm_tiles")
+        work.data_ptr(), _ptr(error_word(xbc.device)), tokens, n, heads, head_dim, state_size, groups, int(per), _stream()), "ssm_tiles")
     return y
 
 

@@ -428,16 +428,14 @@ using namespace se::tiles;
 
 extern "C" int se_ssm_tiles_supported(int state_size, int head_dim) { return state_size == kD && head_dim == kV; }
 
-// Arguments as se_ssm_walk's, proj bfloat16.  work: float [(tokens / 128 + entries) * H * (64 * 128 + 1)].
+// Arguments as se_ssm_walk's, proj bfloat16.  work: float [(tokens / 128 + entries) * H * (64 * 128 + 1)].  per: heads of a group that a block takes at most (C and B are
+// cut and multiplied once per block).
 extern "C" int se_ssm_tiles(const float* xbc, const void* proj, int pitch, int dt_off, const float* dt_bias, const float* a_log, const float* d_skip,
                             float* state, long long state_stride, const int* cu_q, const int* seq_rows, float* y, float* work, int* error, int tokens,
-                            int entries, int H, int P, int N, int G, int sms, cudaStream_t stream) {
+                            int entries, int H, int P, int N, int G, int per, cudaStream_t stream) {
     if (entries <= 0 || tokens <= 0) return 0;
-    if (H <= 0 || G <= 0 || H % G) return SE_ERR_ARGUMENT;
+    if (H <= 0 || G <= 0 || H % G || per < 1 || per > kHeads) return SE_ERR_ARGUMENT;
     const long long places = tokens / kT + entries;
-    // heads a block: as many as leave a block for each SM, eight at most (C and B are cut and multiplied once per block)
-    int per = H / G < kHeads ? H / G : kHeads;
-    while (per > 1 && places * G * ((H / G + per - 1) / per) < sms * 3 / 4) per = (per + 1) / 2;
     const int blocks = (H / G + per - 1) / per;
     auto aligned = [](const void* a) { return (reinterpret_cast<uintptr_t>(a) & 15) == 0; };
     if (!se_ssm_tiles_supported(N, P) || H > 65535 || (long long)G * blocks > 65535 || entries > 65535 || places > 0x7fffffffLL || state_stride % 4 ||

@@ -61,10 +61,11 @@ class StateSpaceMixer(Mixer):
     ``y = S^T C + D x``; ``y * silu(z)`` RMS-normed in ``norm_groups`` parts, times a weight; out
     projection."""
     graph_safe = True
-    # The longest entry of a step from which the recurrence may run in chunks; None: never.  Below, the launch that chunks take more
-    # costs a small step, which waits for the host, what the kernels save (a layer's call at 64 tokens: 86 us without, 96 with).
+    # The longest entry of a step from which the recurrence may run in chunks of 64 one after another; None: in no chunks at all.  Below, the launch that
+    # they take more costs a small step, which waits for the host, what the kernels save (a layer's call at 64 tokens: 86 us without, 96
+    # with).  Chunks side by side (`in_tiles`) go by estimates alone.
     chunk_min_tokens = 96
-    chunk_tuning_key = "recurrence_chunk_min_tokens"     # the engine option that sets it (and switches the estimate off)
+    chunk_tuning_key = "recurrence_chunk_min_tokens"     # the engine option that sets it (and switches the estimates off, and chunks side by side)
 
     def __init__(self, spec, dtype):
         super().__init__(spec, dtype)
@@ -112,25 +113,37 @@ class StateSpaceMixer(Mixer):
                          walk=lambda longest, entries, tokens: self.token_by_token(longest, entries, tokens, sms))
             and ops.chunk_walk_supported(s.state_size, s.head_dim)))
 
-    def in_tiles(self, step, device) -> bool:
-        """Whether a step that csrc/ssm_tiles.cu takes (bfloat16, states of 128 rows, heads of 64 columns) goes there: by estimates of it
-        and of the form token by token.  A block takes a chunk of 128 tokens, full or not, and up to eight of a group's heads: 13 us each and 10 for what
-        they share.  Measured, a layer of 64 heads in 8 groups, us before / now: one entry of 110 tokens 91/88, of 128 94/90, of 512 124/105, of 2,048 298/233; four of 40
-        90/92, of 60 109/90, of 300 232/203; sixty-four of 20 401/527, of 40 750/606, of 96 1,722/816; one of 300 beside 15 single tokens 217/167,
-        beside 31 251/272, of 1,024 beside 63 657/521.  Few heads over few tokens stay in chunks of 64 (8 heads of 256 tokens 26, here 29).  The chunks' states
-        take 32 KB per head and chunk: no more than 256 MB, or than the other chunks' workspace."""
-        if self.chunk_min_tokens is None or not getattr(self, "chunks_by_estimate", True):
-            return False
+    def in_tiles(self, step, device) -> int:
+        """Heads that a block takes (true) of a step that csrc/ssm_tiles.cu takes (bfloat16, states of 128 rows, heads of 64 columns) and that goes there; else 0.
+        By estimates of it, of the form token by token and of chunks of 64 one after another (where those would be next), which read C and B once per head and take
+        4 us a chunk where their blocks leave half of the device idle, else 7.  Measured, device us of a layer, the other forms (s, w) / here: 64 heads in 8
+        groups, one entry of 90 tokens s 66/48, of 128 w 52/49, of 257 66/60, of 512 84/67, of 4,096 437/317, four of 96 s 117/80, of 130 w 153/88, sixteen of 40 s 185/139, sixty-four of 96
+        s 1,529/616, 300 beside 15 single tokens w 188/139, 1,024 beside 63 s 611/465; 32 heads in 8, 128 tokens w 42/46, 200 49/47, 512 64/54,
+        in one group 128 w 65/45; 16 heads in 8, two entries of 130 w 43/47, 1,024 tokens w 90/58; 8 heads in 8, 200 w 45/45, 257 w 46/46, 1,024 w 90/56.
+        The chunks' states take 32 KB per head and chunk: no more than 256 MB, or than the other chunks' workspace."""
+        least = self.chunk_min_tokens
+        if least is None or step.max_q_len < 17 or not getattr(self, "chunks_by_estimate", True):
+            return 0
 
         def ask():
             s, sms = self.spec, ops.sm_count(device)
             longest, entries, tokens = step.max_q_len, step.num_seqs, step.num_tokens
-            if s.num_heads * longest <= 2048 or (tokens // 128 + entries) * s.num_heads * 8193 > max(1 << 26, tokens * s.num_heads * 67):
-                return False
+            if (tokens // 128 + entries) * s.num_heads * 8193 > max(1 << 26, tokens * s.num_heads * 67):
+                return 0
             lens = getattr(step, "q_lens", None) or [longest] + [(tokens - longest) // max(1, entries - 1)] * (entries - 1)
-            per = min(8, s.num_heads // s.groups)
-            blocks = sum(-(-n // 128) for n in lens) * s.groups * -(-(s.num_heads // s.groups) // per)
-            return 35 + blocks * (10 + 13 * per) / sms < self.token_by_token(longest, entries, tokens, sms)
+            chunks, rep = sum(-(-n // 128) for n in lens), s.num_heads // s.groups
+            us, per = ops.ssm_tiles_plan(chunks, s.num_heads, s.groups, sms)
+            most = min(8, rep)
+            shared_out = 35 + chunks * s.groups * -(-rep // most) * (10 + 13 * most) / sms
+            if s.num_heads * longest <= 2048 or shared_out >= self.token_by_token(longest, entries, tokens, sms):
+                return 0
+            if not self.in_chunks(step, device):
+                return per
+            share = s.num_heads * -(-s.head_dim // 32) / sms
+            first, further = (19.5, 7.0) if share > 0.5 else (17.0, 4.2)
+            pieces = sum(-(-n // 64) for n in lens)
+            walk = max(first + further * (-(-longest // 64) - 1), (first * entries + further * (pieces - entries)) * share)
+            return per if 26 + us < 17 + walk + 2.1e-4 * 64 * pieces * s.num_heads + 0.8 * rep else 0
         return once_per_step(step, ("state_space.in_tiles", self.spec.num_heads, self.spec.groups, self.spec.state_size, self.spec.head_dim), ask)
 
     def forward(self, x, step, slot):
@@ -140,10 +153,13 @@ class StateSpaceMixer(Mixer):
         xbc = torch.empty(tokens, self.conv_channels, dtype=torch.float32, device=x.device)
         ops.causal_conv(proj, self.inner, self.conv_w, self.conv_b, slot.state, self.conv_off, step, xbc)
         y = torch.empty(tokens, self.inner, dtype=torch.float32, device=x.device)
-        tiles = ops.ssm_tiles_supported(s.state_size, s.head_dim, proj, slot.state) and self.in_tiles(step, x.device)
-        (ops.ssm_tiles if tiles else ops.ssm_walk if self.in_chunks(step, x.device) else ops.ssm_scan)(
-            xbc, proj, self.inner + self.conv_channels, self.dt_bias, self.a_log, self.d_skip, slot.state, step, y,
-            heads=s.num_heads, head_dim=s.head_dim, state_size=s.state_size, groups=s.groups)
+        args = (xbc, proj, self.inner + self.conv_channels, self.dt_bias, self.a_log, self.d_skip, slot.state, step, y)
+        sizes = dict(heads=s.num_heads, head_dim=s.head_dim, state_size=s.state_size, groups=s.groups)
+        per = self.in_tiles(step, x.device)
+        if per and ops.ssm_tiles_supported(s.state_size, s.head_dim, proj, slot.state):
+            ops.ssm_tiles(*args, **sizes, heads_per_block=per)
+        else:
+            (ops.ssm_walk if self.in_chunks(step, x.device) else ops.ssm_scan)(*args, **sizes)
         gated = torch.empty(tokens, self.inner, dtype=x.dtype, device=x.device)
         ops.gated_group_norm(y, proj, 0, self.norm_w, gated, parts=s.norm_groups, eps=s.norm_eps)
         return linear(gated, self.o)

@@ -73,3 +73,30 @@ def test_retention_tiles_where_the_walk_is_not_ahead(monkeypatch, lens, heads, t
     part = make_mixer(RetentionSpec(hidden_size=64, num_heads=heads, head_dim=128, v_head_dim=128, decays=(0.9,) * heads, position=None), torch.bfloat16)
     step = SimpleNamespace(max_q_len=max(lens), num_tokens=sum(lens), num_seqs=len(lens), q_lens=lens)
     assert part.in_tiles(step, sum(lens), 0, "cuda:0") is tiles
+
+
+def _state_space(heads, groups):
+    import torch
+
+    from sparseengine_b200.config.specs import StateSpaceSpec
+    from sparseengine_b200.parts.base import make_mixer
+    return make_mixer(StateSpaceSpec(hidden_size=64, num_heads=heads, head_dim=64, state_size=128, groups=groups, conv_taps=4, norm_groups=groups), torch.bfloat16)
+
+
+@pytest.mark.parametrize("lens,heads,groups,tiles", [
+    # device us of a layer, the walk / chunks side by side: 42/46, 45/47, 43/47; 52/49, 65/45, 66/60, 84/67, 90/58
+    ([128], 32, 8, False), ([96] * 2, 32, 8, False), ([130] * 2, 16, 8, False), ([128], 64, 8, True), ([128], 32, 1, True), ([257], 64, 8, True),
+    ([512], 64, 8, True), ([1024], 16, 8, True),
+    # token by token / side by side: 66/48, 185/138; 94/92 by tokens
+    ([90], 64, 8, True), ([40] * 16, 64, 8, True), ([17] * 16, 64, 8, False)])
+def test_state_space_tiles_by_all_three_estimates(monkeypatch, lens, heads, groups, tiles):
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    step = SimpleNamespace(max_q_len=max(lens), num_tokens=sum(lens), num_seqs=len(lens), q_lens=lens)
+    assert bool(_state_space(heads, groups).in_tiles(step, "cuda:0")) is tiles
+
+
+def test_state_space_heads_a_block():
+    heads = lambda *a: ops.ssm_tiles_plan(*a, 148)[1]      # noqa: E731
+    # 257 tokens 72 us a layer with one head, 60 with two; 4,096 346 with four, 310 with eight; one block per SM and head at 128
+    assert heads(3, 64, 8) == 2 and heads(32, 64, 8) == 8 and heads(1, 64, 8) == 1 and heads(95, 64, 8) == 8
+    assert heads(10000, 11, 1) <= 8 and heads(1, 3, 3) == 1 and heads(50, 18, 2) <= 8
