@@ -82,8 +82,9 @@ KERNEL_TUNING_KEYS = {
     "router_tensor_core_min_tokens": "split_router_min_tokens",         # prompt steps from this size take router logits from tensor cores
     "moe_pair_min_rows": "pair_min_rows",                               # (token, slot) rows from which experts may run on pairs of SMs
     "moe_pair_min_rows_per_expert": "pair_min_rows_per_expert",         # ... if the experts that get rows have this many each
-    # steps whose longest entry has this many tokens take the chunked recurrence: retention, matrix memory and minGRU, which choose by
-    # that number alone; the state-space mixer and the delta rules, which otherwise estimate what either form takes
+    # steps whose longest entry has this many tokens take the recurrence in chunks: retention, matrix memory and minGRU, which choose by
+    # that number alone; the state-space mixer and the delta rules, which otherwise estimate what chunks and single tokens take
+    # (between its forms of chunks retention chooses by the step's sizes, the state-space mixer by estimates, also with the option)
     "retention_chunk_min_tokens": "chunk_min_tokens",
     "recurrence_chunk_min_tokens": "chunk_min_tokens",
 }

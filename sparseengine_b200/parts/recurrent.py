@@ -65,7 +65,9 @@ class StateSpaceMixer(Mixer):
     # they take more costs a small step, which waits for the host, what the kernels save (a layer's call at 64 tokens: 86 us without, 96
     # with).  Chunks side by side (`in_tiles`) go by estimates alone.
     chunk_min_tokens = 96
-    chunk_tuning_key = "recurrence_chunk_min_tokens"     # the engine option that sets it (and switches the estimates off, and chunks side by side)
+    # the engine option that sets it and switches the estimate off that chunks take less time than tokens one by one: either form of chunks is then taken
+    # from that many tokens on, the one that is estimated to take less time
+    chunk_tuning_key = "recurrence_chunk_min_tokens"
 
     def __init__(self, spec, dtype):
         super().__init__(spec, dtype)
@@ -122,7 +124,7 @@ class StateSpaceMixer(Mixer):
         in one group 128 w 65/45; 16 heads in 8, two entries of 130 w 43/47, 1,024 tokens w 90/58; 8 heads in 8, 200 w 45/45, 257 w 46/46, 1,024 w 90/56.
         The chunks' states take 32 KB per head and chunk: no more than 256 MB, or than the other chunks' workspace."""
         least = self.chunk_min_tokens
-        if least is None or step.max_q_len < 17 or not getattr(self, "chunks_by_estimate", True):
+        if least is None or step.max_q_len < min(least, 17):
             return 0
 
         def ask():
@@ -133,12 +135,15 @@ class StateSpaceMixer(Mixer):
             lens = getattr(step, "q_lens", None) or [longest] + [(tokens - longest) // max(1, entries - 1)] * (entries - 1)
             chunks, rep = sum(-(-n // 128) for n in lens), s.num_heads // s.groups
             us, per = ops.ssm_tiles_plan(chunks, s.num_heads, s.groups, sms)
-            most = min(8, rep)
-            shared_out = 35 + chunks * s.groups * -(-rep // most) * (10 + 13 * most) / sms
-            if s.num_heads * longest <= 2048 or shared_out >= self.token_by_token(longest, entries, tokens, sms):
+            if getattr(self, "chunks_by_estimate", True):
+                most = min(8, rep)
+                shared_out = 35 + chunks * s.groups * -(-rep // most) * (10 + 13 * most) / sms
+                if s.num_heads * longest <= 2048 or shared_out >= self.token_by_token(longest, entries, tokens, sms):
+                    return 0
+                if not self.in_chunks(step, device):
+                    return per
+            elif longest < least:
                 return 0
-            if not self.in_chunks(step, device):
-                return per
             share = s.num_heads * -(-s.head_dim // 32) / sms
             first, further = (19.5, 7.0) if share > 0.5 else (17.0, 4.2)
             pieces = sum(-(-n // 64) for n in lens)

@@ -95,6 +95,22 @@ def test_state_space_tiles_by_all_three_estimates(monkeypatch, lens, heads, grou
     assert bool(_state_space(heads, groups).in_tiles(step, "cuda:0")) is tiles
 
 
+def test_state_space_chunks_from_a_number_of_tokens_on(monkeypatch):
+    """What the engine's option sets: both forms of chunks from that many tokens on, whichever is estimated shorter."""
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    wide, narrow = _state_space(64, 8), _state_space(8, 8)
+    wide.chunk_min_tokens, wide.chunks_by_estimate = 40, False
+    narrow.chunk_min_tokens, narrow.chunks_by_estimate = 5, False
+
+    def forms(part, lens):
+        step = SimpleNamespace(max_q_len=max(lens), num_tokens=sum(lens), num_seqs=len(lens), q_lens=lens)
+        return bool(part.in_tiles(step, "cuda:0")), part.in_chunks(step, "cuda:0")
+    assert forms(wide, [2048]) == (True, True) and forms(wide, [40] * 4) == (True, True) and forms(wide, [39] * 400) == (False, False)
+    assert forms(narrow, [5]) == (False, True) and forms(narrow, [4]) == (False, False) and forms(narrow, [1024]) == (True, True)
+    wide.chunk_min_tokens = None
+    assert forms(wide, [2048]) == (False, False)
+
+
 def test_state_space_heads_a_block():
     heads = lambda *a: ops.ssm_tiles_plan(*a, 148)[1]      # noqa: E731
     # 257 tokens 72 us a layer with one head, 60 with two; 4,096 346 with four, 310 with eight; one block per SM and head at 128
