@@ -136,6 +136,45 @@ def test_retention_inputs_that_are_not_finite_stay_with_their_token_and_later_on
         assert torch.equal(s_got[0, 128 * 128:], s_want[0, 128 * 128:])
 
 
+# more items (chunks and heads) than two for each SM: a block's loop goes on to other chunks of other heads, past places without a token
+MANY = [([2500], 16), ([130, 0, 257, 1, 64] * 5, 16)]
+
+
+@pytest.mark.parametrize("lens,heads", MANY)
+def test_retention_blocks_of_several_items(lens, heads):
+    from sparseengine_b200.csrc import ops
+    assert (sum(lens) // 128 + len(lens)) * heads > 2 * ops.sm_count(DEV)
+    step, o, first, state, inputs, gate = _retention(lens, heads, 128, "slow")
+    for e, n in enumerate(lens):
+        a, b, row = step.cu[e], step.cu[e + 1], step.rows[e]
+        if n == 0:
+            assert torch.equal(state[row], first[row])
+            continue
+        want, S = _walk64(*(x[a:b] for x in inputs), first[row, :heads * 128 * 128].double().view(heads, 128, 128))
+        _close(o[a:b].view(n, heads, 128), want, f"outputs of {n} tokens")
+        _close(state[row, :heads * 128 * 128].view(heads, 128, 128), S, f"state after {n} tokens")
+    _, y, _, state2, _, _ = _retention(lens, heads, 128, "slow", out=True)
+    assert torch.equal(state2, state)
+    o = o.double().view(-1, heads, 128)
+    want = (o / torch.sqrt((o * o).mean(-1, keepdim=True) + 1e-6)).view(len(o), -1) * torch.nn.functional.silu(gate.double())
+    assert bool(((y.double() - want).abs() <= want.abs() * (2.0 ** -8 + 1e-5) + 1e-30).all())       # as in the test of norm and gate
+
+
+@pytest.mark.parametrize("where", ["q", "k", "v"])
+@pytest.mark.parametrize("out", [False, True])
+def test_retention_goes_on_behind_a_chunk_that_is_done_again(where, out):
+    """Token 150 of 2,500, head 0 of 16: the block that does its chunk again has fetched another chunk of another head meanwhile, which it fetches again."""
+    (lens, heads), t = MANY[0], 150
+    _, want, _, s_want, _, _ = _retention(lens, heads, 128, "slow", out=out)
+    _, got, _, s_got, _, _ = _retention(lens, heads, 128, "slow", bad=(t, where, float("nan")), out=out)
+    assert torch.equal(got[:, 128:], want[:, 128:]) and torch.equal(s_got[:, 128 * 128:], s_want[:, 128 * 128:])
+    assert torch.equal(got[:128, :128], want[:128, :128]) and not bool(torch.isfinite(got[t, :128].float()).all())
+    if where == "q":
+        assert torch.equal(got[256:, :128], want[256:, :128]) and torch.equal(s_got, s_want)
+    else:
+        assert not bool(torch.isfinite(got[t:, :128].float()).all(1).any())
+
+
 def test_retention_mixer_keeps_to_the_other_forms_beyond_its_workspace():
     from sparseengine_b200.config.specs import RetentionSpec
     from sparseengine_b200.parts.base import make_mixer
@@ -178,7 +217,7 @@ def test_retention_mixer_through_the_chunks(norm):
     assert float((ys[0][1] - ys[1][1]).norm() / ys[1][1].norm()) < 1e-6
 
 
-def _state_space(lens, heads, groups, decay, bad=None, positive=False, walk=False):
+def _state_space(lens, heads, groups, decay, bad=None, positive=False, walk=False, per=None):
     from sparseengine_b200.csrc import ops
     P, N, step = 64, 128, _step(lens)
     T, g = step.num_tokens, torch.Generator(device=DEV).manual_seed(heads)
@@ -197,7 +236,8 @@ def _state_space(lens, heads, groups, decay, bad=None, positive=False, walk=Fals
             xbc[t, {"v": 5, "k": heads * P + 5, "q": heads * P + groups * N + 5}[where]] = value
     first, y = state.clone(), torch.full((T, heads * P), float("nan"), device=DEV)
     assert ops.ssm_tiles_supported(N, P, proj, state)
-    (ops.ssm_walk if walk else ops.ssm_tiles)(xbc, proj, 3, bias, a_log, skip, state, step, y, heads=heads, head_dim=P, state_size=N, groups=groups)
+    (ops.ssm_walk if walk else ops.ssm_tiles)(xbc, proj, 3, bias, a_log, skip, state, step, y, heads=heads, head_dim=P, state_size=N, groups=groups,
+                                                **({} if walk else {"heads_per_block": per}))
     ops.error_check(DEV)
     dt = torch.nn.functional.softplus(proj[:, 3:3 + heads].double() + bias.double())
     x, rep = xbc[:, :heads * P].double().view(T, heads, P), heads // groups
@@ -224,6 +264,13 @@ def test_state_space_against_the_walk(lens, heads, groups, decay):
         _close(state[row, :heads * P * N].view(heads, P, N).transpose(1, 2), S, f"state after {n} tokens")
     others = [r for r in range(len(lens) + 2) if r not in step.rows]
     assert torch.equal(state[others], first[others]) and torch.equal(state[:, heads * P * N:], first[:, heads * P * N:])
+
+
+@pytest.mark.parametrize("lens,heads,groups", [([130, 1, 0, 300], 11, 1), ([200], 12, 3)])
+def test_state_space_is_the_same_with_any_number_of_heads_a_block(lens, heads, groups):
+    runs = [_state_space(lens, heads, groups, "slow", per=per) for per in (None, 1, 3, 8)]
+    for _, y, _, state, _, _ in runs[1:]:
+        assert torch.equal(y, runs[0][1]) and torch.equal(state, runs[0][3])
 
 
 @pytest.mark.parametrize("positive", [False, True])
@@ -254,7 +301,7 @@ def test_state_space_inputs_that_are_not_finite_stay_with_their_token_and_later_
         assert not bool(torch.isfinite(got[t, :own]).any())
         torch.testing.assert_close(got[t + 1:], want[t + 1:], **near)
         assert torch.equal(s_got, s_want)
-    elif where != "dt" or value != value:            # an infinite step may be a decay of 0
+    else:                                            # also of an infinite step, whose decay is 0: what the token adds is not finite
         assert not bool(torch.isfinite(got[t:, :own]).all(1).any()) and not bool(torch.isfinite(s_got[0, :own * 128]).all())
         assert torch.equal(s_got[0, own * 128:], s_want[0, own * 128:])
 
