@@ -213,7 +213,8 @@ def _kernels(width: int, tokens_list, pk: dict) -> dict:
         dtb, al, dk = torch.zeros(H, device=dev), torch.zeros(H, device=dev), torch.ones(H, device=dev)
         yy = torch.empty(tokens, inner, device=dev)
         scan_bytes = tokens * (C + inner) * 4 + entries * H * P * N * 8
-        name = "ssm_walk" if ssm_part.in_chunks(step, dev) else "ssm_scan"
+        tiles = ssm_part.in_tiles(step, dev) and ops.ssm_tiles_supported(N, P, proj, state)
+        name = "ssm_tiles" if tiles else "ssm_walk" if ssm_part.in_chunks(step, dev) else "ssm_scan"
         add(name, lambda: getattr(ops, name)(xbc, proj, inner + C, dtb, al, dk, state, step, yy, heads=H, head_dim=P,
                                              state_size=N, groups=G), scan_bytes, iters=5)
         rec[name]["us_per_token_of_a_request"] = round(rec[name]["us"] / per, 3)

@@ -138,16 +138,22 @@ def _kernels(width: int, cases, pk: dict) -> dict:
         inv_r = (1e6 ** (-torch.arange(0, dr, 2, dtype=torch.float32) / dr)).to(dev)
         q32, k32 = torch.empty(tokens, qk, device=dev), torch.empty(tokens, qk, device=dev)
         chunked = per >= ret_part.chunk_min_tokens
-        walk = chunked and ret_part.in_walk(step, dev)
-        if not walk:
-            add("retention_prep", lambda: ops.retention_prep(proj_r, 0, qk, inv_r, step.positions, q32, k32, heads=Hr, head_dim=dr,
-                                                             rotary_dim=dr, k_scale=dr ** -0.5), tokens * qk * 12)
         decay = torch.tensor(ret["decay"], device=dev, dtype=torch.float32)
         state = torch.zeros(entries, Hr * dr * dvr, device=dev)
-        o_r = torch.empty(tokens, vv, device=dev)
+        o_r, gated = torch.empty(tokens, vv, device=dev), torch.empty(tokens, vv, device=dev, dtype=bf)
+        tiles = (chunked and ret_part.in_tiles(step, tokens, dr, dev)
+                 and ops.retention_tiles_supported(dr, dvr, dr, proj_r, state, 0, qk, 2 * qk, 2 * qk + vv))
+        walk = chunked and not tiles and ret_part.in_walk(step, dev)
+        if not (tiles or walk):
+            add("retention_prep", lambda: ops.retention_prep(proj_r, 0, qk, inv_r, step.positions, q32, k32, heads=Hr, head_dim=dr,
+                                                             rotary_dim=dr, k_scale=dr ** -0.5), tokens * qk * 12)
         sizes = dict(heads=Hr, head_dim=dr, v_head_dim=dvr)
-        moved = tokens * (2 * qk * (2 if walk else 4) + vv * 6) + entries * Hr * dr * dvr * 8
-        if walk:                                     # q and k from the projection, rotated on the way
+        moved = tokens * (2 * qk * (4 if not (tiles or walk) else 2) + vv * 6) + entries * Hr * dr * dvr * 8
+        if tiles:                                    # the same, with the norm and the gate
+            name = "retention_tiles (chunks side by side, with norm and gate)"
+            add(name, lambda: ops.retention_tiles(proj_r, 0, qk, 2 * qk, 2 * qk + vv, dr ** -0.5, (inv_r, dr, step.positions), decay, state, step, **sizes,
+                                                  eps=1e-6, out=gated), moved, iters=5)
+        elif walk:                                   # q and k from the projection, rotated on the way
             name = "retention_chunk (prepared side by side, walked)"
             add(name, lambda: ops.retention_chunk(None, None, proj_r, 2 * qk, decay, state, step, o_r, **sizes, qk=(0, qk, dr ** -0.5),
                                                   rotation=(inv_r, dr, step.positions)), moved, iters=5)
@@ -155,13 +161,13 @@ def _kernels(width: int, cases, pk: dict) -> dict:
             name = "retention_chunk" if chunked else "retention_scan"
             add(name, lambda: getattr(ops, name)(q32, k32, proj_r, 2 * qk, decay, state, step, o_r, **sizes), moved, iters=5)
         rec[name]["us_per_token_of_a_request"] = round(rec[name]["us"] / per, 3)
-        if chunked:
+        if chunked and not tiles:
             # 32-bit FMAs of the closed form: scores (half of the 64 x 64 square is used), their product with the
             # values, the old state's part and the new state
             fma = tokens * Hr * (64 * dr * ((dvr + 31) // 32) + 64 * dvr + 2 * dr * dvr)
             rec[name]["of_fp32_fma_peak"] = round(fma / (rec[name]["us"] * 1e-6) / (148 * 128 * 1.9e9), 3)
-        gated = torch.empty(tokens, vv, device=dev, dtype=bf)
-        add("retention_out", lambda: ops.retention_out(o_r, proj_r, 2 * qk + vv, gated, heads=Hr, v_head_dim=dvr, eps=1e-6), tokens * vv * 8)
+        if not tiles:
+            add("retention_out", lambda: ops.retention_out(o_r, proj_r, 2 * qk + vv, gated, heads=Hr, v_head_dim=dvr, eps=1e-6), tokens * vv * 8)
         # like: the delta rule's recurrence of the closest model, the same state size
         C = 2 * qk + vv
         qkv = torch.randn(tokens, C, device=dev) * 0.1
