@@ -348,16 +348,20 @@ class RetentionMixer(Mixer):
 
     def in_tiles(self, step, tokens: int, rotary_dim: int, device) -> bool:
         """Whether a step in chunks that csrc/retention_tiles.cu takes (bfloat16, heads of 128 x 128) goes there.  Not where all of the walk's
-        blocks run at once and its longest chain is four chunks: each of the two kernels takes some 15 us for a chunk, the walk and its preparation
-        7 to 14 and 4 more a chunk.  Measured, device us of a layer without its projections, the other forms / here: 4, 8, 16 and 32 heads, one
+        blocks run at once and its longest chain is three chunks: each of the two kernels takes some 15 us for a chunk, the walk and its preparation
+        7 to 14 and 4 more a chunk; unless it is the host that takes the time (one launch instead of three), which it is until the projections' weights
+        take the device as long as 100 MB do.  Measured, device us of a layer without its projections, the other forms / here: 4, 8, 16 and 32 heads, one
         portion of 17 tokens 25/45, 25/41, 27/43, 33/45, of 128 30/41, 31/41, 33/43, 41/45, of 200 35/39, 37/41, 39/43, 48/48, of
         257 39/42, 41/40, 44/45, 56/51, of 1,024 72/41, 76/46, 84/50, 123/80; 17 tokens beside 15 single ones 43/46, 71/45, 117/78, 213/125, 90 beside 63
-        86/76, 226/122, 425/221, 823/400; two entries of 40 27/41, 27/41, 33/43, 52/45, sixty-four of 96 156/98, 296/171, 574/301, 1,115/569.
-        (A whole layer's call of 128 tokens and 16 heads, waited for: 89/100; calls one behind the other, where the host is what takes the time, 77/70.)
+        86/76, 226/122, 425/221, 823/400; two entries of 40 27/41, 27/41, 33/43, 52/45, sixty-four of 96 156/98, 296/171, 574/301, 1,115/569.  Whole layers over
+        17 tokens, 16 heads of 2,048 (42 MB): on the device 31/45, calls one behind the other 73/60, a call waited for 83/93; 24 of 3,072 (94 MB) 47/60, 71/69,
+        86/99; 24 of 4,096 (126 MB) 56/70, 71/78, 87/99; 32 of 4,096 (168 MB) 61/73, 72/79, 89/98, over 128 tokens 70/77, 78/84, 99/104, over 250 84/84, 92/90, 112/109.
         And as long as its workspace, 64 KB per head and entry or 128 tokens, is no larger than that of the other forms or 256 MB."""
         s = self.spec
-        if step.max_q_len <= 256 and step.num_seqs * s.num_heads * -(-s.v_head_dim // 32) <= ops.sm_count(device):
-            return False
+        if step.max_q_len <= 192 and step.num_seqs * s.num_heads * -(-s.v_head_dim // 32) <= ops.sm_count(device):
+            weights = 2 * s.hidden_size * (2 * self.qk + 3 * self.vv)
+            if weights > 100e6 or torch.cuda.is_initialized() and torch.cuda.is_current_stream_capturing():
+                return False
         return once_per_step(step, ("retention.in_tiles", s.num_heads, rotary_dim), lambda: (
             ops.retention_tiles_plan(step, tokens, s.num_heads, rotary_dim, device)[2] <= max(1 << 26, tokens * s.num_heads * 322)))
 

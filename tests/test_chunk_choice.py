@@ -60,19 +60,26 @@ def test_retention_walk_by_the_entries_own_tokens(monkeypatch, lens, sixteen, th
         assert part.in_walk(step, "cuda:0") is walk
 
 
-@pytest.mark.parametrize("lens,heads,tiles", [
-    # device us of a layer without its projections, the walk / chunks side by side: 27/43, 33/43, 41/45, 41/46; 44/45, 56/51, 56/53, 52/45, 45/47, 117/78
-    ([17], 16, False), ([128], 16, False), ([128], 32, False), ([130] * 2, 16, False), ([256], 32, False), ([90] + [1] * 3, 8, False),
-    ([257], 16, True), ([257], 32, True), ([17], 64, True), ([40] * 2, 32, True), ([17] * 4, 16, True), ([17] + [1] * 15, 16, True), ([8192], 32, True)])
-def test_retention_tiles_where_the_walk_is_not_ahead(monkeypatch, lens, heads, tiles):
+@pytest.mark.parametrize("lens,heads,hidden,tiles", [
+    # device us of a layer without its projections, the walk / chunks side by side: 33/45, 41/45; 56/51, 56/53, 52/45; 44/45, 45/47, 117/78
+    ([17], 32, 4096, False), ([128], 32, 4096, False), ([192], 32, 4096, False), ([257], 32, 4096, True), ([17], 64, 8192, True), ([40] * 2, 32, 4096, True),
+    ([257], 16, 8192, True), ([17] * 4, 16, 8192, True), ([17] + [1] * 15, 16, 8192, True), ([8192], 32, 4096, True), ([130] * 2, 16, 8192, False),
+    # calls one behind the other: 73/60, 72/60, 71/69; 71/78
+    ([17], 16, 2048, True), ([17], 32, 2048, True), ([17], 24, 3072, True), ([17], 24, 4096, False)])
+def test_retention_tiles_where_the_walk_is_not_ahead(monkeypatch, lens, heads, hidden, tiles):
     import torch
 
     from sparseengine_b200.config.specs import RetentionSpec
     from sparseengine_b200.parts.base import make_mixer
     monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
-    part = make_mixer(RetentionSpec(hidden_size=64, num_heads=heads, head_dim=128, v_head_dim=128, decays=(0.9,) * heads, position=None), torch.bfloat16)
+    part = make_mixer(RetentionSpec(hidden_size=hidden, num_heads=heads, head_dim=128, v_head_dim=128, decays=(0.9,) * heads, position=None), torch.bfloat16)
     step = SimpleNamespace(max_q_len=max(lens), num_tokens=sum(lens), num_seqs=len(lens), q_lens=lens)
     assert part.in_tiles(step, sum(lens), 0, "cuda:0") is tiles
+    # a captured step does not wait for the host
+    if max(lens) <= 192 and len(lens) * heads * 4 <= 148:
+        monkeypatch.setattr(torch.cuda, "is_initialized", lambda: True)
+        monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+        assert not part.in_tiles(step, sum(lens), 0, "cuda:0")
 
 
 def _state_space(heads, groups):
