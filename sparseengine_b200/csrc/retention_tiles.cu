@@ -237,8 +237,8 @@ retention_join_kernel(const Retention p) {
 }
 
 // A block takes chunks in turn.  The next chunk's q, k and angles are fetched into room that this one's products have left (the state's terms, the last of
-// k's) while its weights are made and P v runs; the state comes into registers meanwhile.  Bound by the steps of a chunk, 16 us, one after another: the
-// products take 8,000 cycles of 30,000, instructions issue in 30 %; a warp is held by the products that it issues, so warp 0 cuts no part of the state (all sixteen: 232 us, 224 without it).
+// k's) while its weights are made and P v runs; the state comes into registers meanwhile.  Bound by the steps of a chunk, 15 us, one after another: the
+// products take 8,000 cycles of 29,000, instructions issue in 47 %; a warp is held by the products that it issues, so warp 0 cuts no part of the state (all sixteen: 232 us, 224 without it).
 // Measured, 8,192 tokens of 32 heads: 214 us.  While products had one part (224): q and angles row by row from memory and outputs and gates a row a
 // thread 292, the latter alone 240; a warp group per operand, which leaves 64 to 112 registers a thread and spills, 253 to 288; a warp that only issues products, 112 registers, 274.
 //   columns of tensor memory: q's terms, then P's 0-191; a product's two parts 192-447: the scores, what the state gives, P v in turn
